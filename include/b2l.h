@@ -209,6 +209,12 @@ int b2l_q8_gemv(const void* x, const void* w_tiled, const void* cb, const void* 
                 b2l_stream_t stream);
 int b2l_q8_outlier_mask(const void* x, int ldx, int M, int K, float threshold, void* mask,
                         b2l_stream_t stream);
+/* The same for M activation rows at once (csrc/q8_gemm.cu: tcgen05 kind::i8), outlier columns shared by the batch; reads CB in the
+ * checkpoint's layout.  K % 128 == 0, K <= 12288; x, cb and workspace 16-byte aligned; workspace of
+ * b2l_q8_linear_workspace_bytes(M, K) bytes. */
+size_t b2l_q8_linear_workspace_bytes(int M, int K);
+int b2l_q8_linear(const void* x, int ldx, const void* cb, const void* scb, void* y, int ldy,
+                  void* workspace, int M, int N, int K, float threshold, b2l_stream_t stream);
 
 /* generate.py:68-75 up to the probabilities: probs = softmax(where(l < kth, -inf, l)) with
  * l = logits / temperature (bf16, rounded like ATen does on the GPU) and kth the top_k-th

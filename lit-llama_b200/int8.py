@@ -102,7 +102,15 @@ class Linear8bitLt(torch.nn.Module):
         M, K, N = x2.shape[0], self.in_features, self.out_features
         y = torch.empty((M, N), device=x.device, dtype=x.dtype)
         lib = L.lib()
-        cb, scb, wt = self.weight.data, self.weight.SCB, self.tiled()
+        cb, scb = self.weight.data, self.weight.SCB
+        if M > 1 and cb.data_ptr() % 16 == 0:        # all rows in one product: the weight is read once (TMA wants 16-byte aligned rows)
+            ws = torch.empty(lib.b2l_q8_linear_workspace_bytes(M, K), dtype=torch.uint8, device=x.device)
+            L.check(lib.b2l_q8_linear(x2.data_ptr(), K, cb.data_ptr(), scb.data_ptr(), y.data_ptr(), N, ws.data_ptr(), M, N, K, self.threshold,
+                                      L.stream_ptr()), "b2l_q8_linear")
+            if self.bias is not None:
+                y = y + self.bias.to(y.dtype)
+            return y.reshape(*shape[:-1], N)
+        wt = self.tiled()
         mask = None
         if M > 1:  # outlier columns are a property of the whole batch (any row over the threshold)
             mask = torch.empty((K + 31) // 32, dtype=torch.int32, device=x.device)

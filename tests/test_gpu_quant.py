@@ -362,6 +362,33 @@ def test_int8_linear_vs_oracle(dev, N, K, M, outliers):
     assert (y - exact).norm() / exact.norm() < 3e-2  # the int8 scheme itself is ~1% accurate
 
 
+@pytest.mark.parametrize("M,N,K,outliers", [(2, 48, 128, 0), (16, 130, 256, 1), (17, 128, 1024, 3), (33, 4096, 4096, 5), (137, 11008, 4096, 6), (256, 300, 12288, 2),
+                                            (257, 272, 1024, 40), (5, 512, 512, 512)])
+def test_int8_rows_at_once_equal_single_rows(dev, M, N, K, outliers):
+    """All rows in one product (token tiles of 16..256, K split over clusters of 1..8) give the bits of the single-row kernel under the
+    batch's outlier mask: the contraction is integer and the roundings are the same, so there is no tolerance."""
+    from lit_llama_b200 import _lib as L
+
+    lib, g = L.lib(), torch.Generator().manual_seed(M + N + K)
+    cb = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(dev)
+    scb = (torch.rand(N, generator=g) * 0.1 + 0.01).to(dev)
+    x = torch.randn(M, K, generator=g).clamp_(-5, 5)
+    for i in range(outliers):
+        x[i % M, (37 * i + 11) % K] = (-1) ** i * (7.5 + i)
+    x = x.bfloat16().to(dev)
+    tiled = torch.empty(lib.b2l_q8_tiled_bytes(N, K), dtype=torch.uint8, device=dev)
+    mask = torch.empty(K // 32, dtype=torch.int32, device=dev)
+    want, got = torch.empty(M, N, dtype=torch.bfloat16, device=dev), torch.empty(M, N, dtype=torch.bfloat16, device=dev)
+    L.check(lib.b2l_q8_tile(cb.data_ptr(), tiled.data_ptr(), N, K, L.stream_ptr()), "tile")
+    L.check(lib.b2l_q8_outlier_mask(x.data_ptr(), K, M, K, 6.0, mask.data_ptr(), L.stream_ptr()), "mask")
+    for m in range(M):
+        L.check(lib.b2l_q8_gemv(x[m].data_ptr(), tiled.data_ptr(), cb.data_ptr(), scb.data_ptr(), mask.data_ptr(), want[m].data_ptr(), N, K, 6.0, 0,
+                                L.stream_ptr()), "gemv")
+    ws = torch.empty(lib.b2l_q8_linear_workspace_bytes(M, K), dtype=torch.uint8, device=dev)
+    L.check(lib.b2l_q8_linear(x.data_ptr(), K, cb.data_ptr(), scb.data_ptr(), got.data_ptr(), N, ws.data_ptr(), M, N, K, 6.0, L.stream_ptr()), "linear")
+    assert torch.equal(want, got), int((want != got).sum())
+
+
 @pytest.mark.parametrize("n", [4096, 8192, 130])
 def test_tp_allreduce_single_rank_is_identity(dev, n):
     """b2l_tp_allreduce with world = 1 (no peers): the multi-CTA indexing, the in-place path and the epoch words that
