@@ -15,6 +15,7 @@
 // entries; each map is a softmax attention of its own and is handled as a head of its own ("virtual head" h = real
 // head * maps + map) that reads key map (h % maps) of its key/value head and that head's values.  The maps' outputs are
 // stored side by side; combining them (for instance the difference of two maps) is the caller's next kernel.
+#include "attn_tc.cuh"
 #include "seq_common.cuh"
 
 namespace b2l {
@@ -636,6 +637,74 @@ static int launch_tile(const b2l_seq_attn_args* a, cudaStream_t s, int cache_slo
   return 0;
 }
 
+// ---- prompt portions with bf16 keys and values: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, 1), the tiles with the
+// most keys first.
+struct LocalProb {
+  b2l_seq_attn_args a;
+  int DK, DV, stages, split8;
+  float scale, softcap;
+  struct Tile {
+    int h, gk, gv, kh, t_first, rows, pos0, j_begin, j_end;
+    const __nv_bfloat16 *kn, *vn, *ck, *cv;
+  };
+  struct Row { const __nv_bfloat16 *ka, *kb, *v; };
+  __device__ __forceinline__ Tile tile() const {
+    Tile t;
+    t.h = blockIdx.x;
+    kv_heads_of(a, t.h, t.gk, t.gv);
+    t.kh = a.kv_heads * (a.maps > 1 ? a.maps : 1);
+    t.t_first = ((int)gridDim.y - 1 - (int)blockIdx.y) * atc::ROWS;
+    t.rows = min(atc::ROWS, a.T - t.t_first);
+    const int slot = a.meta[0];
+    t.pos0 = a.meta[1];
+    t.j_begin = first_visible(a, t.pos0 + t.t_first);
+    t.j_end = t.pos0 + t.t_first + t.rows;
+    t.kn = (const __nv_bfloat16*)a.k_new;
+    t.vn = (const __nv_bfloat16*)a.v_new;
+    t.ck = (const __nv_bfloat16*)a.cache_k + (size_t)slot * a.block * t.kh * a.K;
+    t.cv = (const __nv_bfloat16*)a.cache_v + (size_t)slot * a.block * a.kv_heads * a.V;
+    return t;
+  }
+  __device__ __forceinline__ Row row(const Tile& t, int j) const {
+    Row r;
+    const int e = j % a.block;
+    r.ka = j >= t.pos0 ? t.kn + ((size_t)(j - t.pos0) * t.kh + t.gk) * a.K : t.ck + ((size_t)e * t.kh + t.gk) * a.K;
+    r.kb = nullptr;
+    r.v = j >= t.pos0 ? t.vn + (size_t)(j - t.pos0) * a.ldv + (size_t)t.gv * a.V : t.cv + ((size_t)e * a.kv_heads + t.gv) * a.V;
+    return r;
+  }
+  __device__ __forceinline__ void query(const Tile& t, int r, int c, float (&x)[8]) const {
+    const float4* q = reinterpret_cast<const float4*>(a.q + ((size_t)(t.t_first + r) * a.heads + t.h) * a.K + 8 * c);
+    const float4 u = q[0], v = q[1];
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+  }
+  __device__ __forceinline__ void range(const Tile& t, int r, int& lo, int& hi) const {
+    hi = t.pos0 + t.t_first + r;
+    lo = first_visible(a, hi);
+  }
+  __device__ __forceinline__ float sink(const Tile&) const { return a.has_sink ? 0.f : -INFINITY; }
+  __device__ __forceinline__ bool partial(const Tile&) const { return false; }
+  __device__ __forceinline__ void store_ml(const Tile&, int, float, float) const {}
+  __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[16]) const {}
+  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
+    const int tt = t.t_first + r;
+    const __nv_bfloat16* gate = (const __nv_bfloat16*)a.gate + (size_t)tt * a.ldg;
+    const float f = a.out_mult * ((a.gate && !a.gate_per_channel) ? sigmoid_f(ld_act(gate, t.h)) : 1.f);
+    const size_t o = (size_t)tt * a.ldo + (size_t)t.h * a.V + c0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      st_out<__nv_bfloat16>(a, o + i, x[i] * f * ((a.gate && a.gate_per_channel) ? sigmoid_f(ld_act(gate, (size_t)t.h * a.V + c0 + i)) : 1.f));
+  }
+};
+
+static DynSmemCache g_local_tc_smem;
+
+static int launch_local_tc(const b2l_seq_attn_args* a, cudaStream_t s) {
+  const atc::Layout l = atc::layout(3, a->K, a->V);
+  LocalProb p{*a, a->K, a->V, l.stages, 1 << 20, a->scale, a->softcap};
+  return atc::launch<LocalProb, 3, 3>(p, dim3((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS)), l.smem, g_local_tc_smem, s);
+}
+
 // ring[p % block] <- token p for the portion's tokens in the block of its last token (block-local) or for its last
 // `block` tokens (sliding window).
 template <typename act_t>
@@ -753,7 +822,11 @@ extern "C" int b2l_seq_block_attention(const b2l_seq_attn_args* a, b2l_stream_t 
   const bool gate_ok = !(a->gate && a->gate_per_channel) || (((uintptr_t)a->gate % 16) == 0 && (a->ldg * esz) % 16 == 0);
   const bool tile = !split && a->T >= 16 && al && (a->K * esz) % 16 == 0 && (a->V * esz) % 16 == 0 && a->V % 4 == 0 && a->V <= 128 &&
                     (a->ldv * esz) % 16 == 0 && gate_ok && tile_smem <= 200 * 1024;
-  if (tile) {
+  // bf16 keys and values of sizes the MMA takes (16 entries per step): tensor cores; else the f32 tiles
+  const bool tens = tile && a->T >= 64 && a->act_dtype == B2L_BF16 && a->K % 16 == 0 && a->K <= atc::MAX_DK && a->V % 16 == 0 && (a->T + atc::ROWS - 1) / atc::ROWS <= 65535;
+  if (tens) {
+    if (int rc = launch_local_tc(a, s)) return rc;
+  } else if (tile) {
     const int vc = (a->V + 31) / 32;
     int rc = 0;
     if (a->act_dtype == B2L_BF16)

@@ -10,8 +10,10 @@
 // Softmax has one learned sink per head in the denominator (exp(sink_h), no key, no value) when a sink is given.  With
 // a window a row sees its own position and the window - 1 before it; a CTA then walks only the keys between the first
 // key of its first row and the last key of its last row.  Scores, weights and accumulators are f32.
+#include <algorithm>
 #include <climits>
 
+#include "attn_tc.cuh"
 #include "seq_common.cuh"
 
 namespace b2l {
@@ -505,6 +507,89 @@ __global__ void seq_head_gate_kernel(const act_t* __restrict__ in, long long ld_
   }
 }
 
+// ---- the expanded form of a prompt portion in bf16: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, key splits), the tiles
+// with the most keys first.
+struct LatentProb {
+  b2l_seq_latent_attn_args a;
+  int DK, DV, stages, split8;
+  float scale, softcap;
+  struct Tile {
+    int h, t_first, rows, pos0, j_begin, j_end;
+    const __nv_bfloat16 *key_a, *key_b;
+  };
+  struct Row { const __nv_bfloat16 *ka, *kb, *v; };
+  __device__ __forceinline__ Tile tile() const {
+    Tile t;
+    t.h = blockIdx.x;
+    t.t_first = ((int)gridDim.y - 1 - (int)blockIdx.y) * atc::ROWS;
+    t.rows = min(atc::ROWS, a.T - t.t_first);
+    const int slot = a.meta[0];
+    t.pos0 = a.meta[1];
+    const int end = t.pos0 + t.t_first + t.rows, begin = a.window > 0 ? max(0, t.pos0 + t.t_first - a.window + 1) : 0;
+    int per = (end - begin + (int)gridDim.z - 1) / (int)gridDim.z;
+    per = (per + atc::KEYS - 1) / atc::KEYS * atc::KEYS;
+    t.j_begin = min(end, begin + (int)blockIdx.z * per);
+    t.j_end = min(end, t.j_begin + per);
+    t.key_a = reinterpret_cast<const __nv_bfloat16*>(a.key_a) + (long long)slot * a.slot_stride_a + (long long)t.h * a.hska;
+    t.key_b = reinterpret_cast<const __nv_bfloat16*>(a.key_b) + (long long)slot * a.slot_stride_b;
+    return t;
+  }
+  __device__ __forceinline__ Row row(const Tile& t, int j) const {
+    Row r;
+    r.v = t.key_a + (long long)j * a.ldka;
+    r.ka = r.v + a.score_off;
+    r.kb = t.key_b + (long long)j * a.ldkb;
+    return r;
+  }
+  __device__ __forceinline__ void query(const Tile& t, int r, int c, float (&x)[8]) const {
+    const long long tt = t.t_first + r;
+    const float* p = c < split8 ? a.q_a + tt * a.ldqa_t + t.h * a.ldqa_h + 8 * c : a.q_b + tt * a.ldqb_t + t.h * a.ldqb_h + 8 * (c - split8);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = p[e];
+  }
+  __device__ __forceinline__ void range(const Tile& t, int r, int& lo, int& hi) const {
+    hi = min(t.pos0 + t.t_first + r, t.j_end - 1);
+    lo = a.window > 0 ? max(0, t.pos0 + t.t_first + r - a.window + 1) : 0;
+  }
+  __device__ __forceinline__ float sink(const Tile& t) const { return a.sink ? a.sink[t.h] : -INFINITY; }
+  __device__ __forceinline__ bool partial(const Tile&) const { return gridDim.z > 1; }
+  __device__ __forceinline__ float* part(const Tile& t, int r) const {
+    return a.work + ((size_t)blockIdx.z * a.T * a.heads + (size_t)(t.t_first + r) * a.heads + t.h) * (size_t)(a.vdim + 2);
+  }
+  __device__ __forceinline__ void store_ml(const Tile& t, int r, float m, float l) const {
+    part(t, r)[0] = m;
+    part(t, r)[1] = l;
+  }
+  __device__ __forceinline__ void store_part(const Tile& t, int r, int c0, const float (&x)[16]) const {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) part(t, r)[2 + c0 + i] = x[i];
+  }
+  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
+    const int tt = t.t_first + r;
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)tt * a.ldo + (size_t)t.h * a.vdim + c0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) st_act(o, i, x[i] * (a.gate ? sigmoid_f(a.gate[(size_t)tt * a.ldg + (size_t)t.h * a.vdim + c0 + i]) : 1.f));
+  }
+};
+
+static DynSmemCache g_lat_tc_smem;
+
+// The form the tensor-core kernel takes: a key group per head, bf16, 16-byte pieces everywhere, a portion worth a row tile.
+static bool latent_tc(const b2l_seq_latent_attn_args* a) {
+  const int dn = a->n_a - a->score_off, dk = dn + a->n_b;
+  auto m8 = [](long long v) { return v % 8 == 0; };
+  return a->act_dtype == B2L_BF16 && a->heads_per_group == 1 && !a->partial && a->T >= 32 && dk % 16 == 0 && dk <= atc::MAX_DK && a->vdim % 16 == 0 &&
+         a->vdim <= atc::MAX_DV && dn > 0 && m8(dn) && m8(a->score_off) && m8(a->ldka) && m8(a->hska) && m8(a->slot_stride_a) && al16(a->key_a) &&
+         (a->n_b == 0 || (m8(a->ldkb) && m8(a->slot_stride_b) && al16(a->key_b))) && (a->T + atc::ROWS - 1) / atc::ROWS <= 65535;
+}
+
+static int launch_latent_tc(const b2l_seq_latent_attn_args* a, int splits, cudaStream_t st) {
+  const int dn = a->n_a - a->score_off, dk = dn + a->n_b;
+  const atc::Layout l = atc::layout(3, dk, a->vdim);
+  LatentProb p{*a, dk, a->vdim, l.stages, dn / 8, a->scale, 0.f};
+  return atc::launch<LatentProb, 3, 3>(p, dim3((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS), (unsigned)splits), l.smem, g_lat_tc_smem, st);
+}
+
 static DynSmemCache g_lat_smem[8];
 
 template <typename act_t, int VI>
@@ -588,21 +673,27 @@ extern "C" int b2l_seq_latent_attention(const b2l_seq_latent_attn_args* a, b2l_s
   const size_t smem = sizeof(float) * ((size_t)Kp * LAT_LDK + (size_t)row_warps * LAT_RW * Qp + (size_t)row_warps * LAT_RW * LAT_BN);
   B2L_CHECK_SUPPORTED(smem <= 220 * 1024, "b2l_seq_latent_attention: key size %d needs %zu bytes of shared memory", Kall, smem);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = 0;
-  B2L_SEQ_DISPATCH(a->act_dtype, {
+  int rc = 0, splits = a->splits;
+  if (latent_tc(a)) {                                  // as many of the caller's key splits as leave one CTA per SM
+    const int ctas = a->heads * ((a->T + atc::ROWS - 1) / atc::ROWS);
+    splits = std::max(1, std::min(splits, sm_count() / ctas));
+    rc = launch_latent_tc(a, splits, st);
+  } else {
+   B2L_SEQ_DISPATCH(a->act_dtype, {
     const int base = sizeof(act_t) == 2 ? 0 : 4;
     if (a->vdim <= 64) rc = launch_latent<act_t, 2>(*a, row_warps, smem, base + 0, st);
     else if (a->vdim <= 128) rc = launch_latent<act_t, 4>(*a, row_warps, smem, base + 1, st);
     else if (a->vdim <= 256) rc = launch_latent<act_t, 8>(*a, row_warps, smem, base + 2, st);
     else rc = launch_latent<act_t, 16>(*a, row_warps, smem, base + 3, st);
-  });
+   });
+  }
   if (rc != 0) return rc;
   B2L_LAUNCH_CHECK("seq_latent_attention_kernel");
-  if (a->splits > 1 && !a->partial) {
+  if (splits > 1 && !a->partial) {
     const int R = a->T * a->heads;
     B2L_SEQ_DISPATCH(a->act_dtype, {
-      seq_latent_combine_kernel<act_t><<<R, a->vdim > 128 ? 256 : 128, sizeof(float) * a->splits, st>>>(a->work, a->sink, a->gate, a->ldg, (act_t*)a->out, a->ldo, R, a->heads,
-                                                                                                                a->vdim, a->splits);
+      seq_latent_combine_kernel<act_t><<<R, a->vdim > 128 ? 256 : 128, sizeof(float) * splits, st>>>(a->work, a->sink, a->gate, a->ldg, (act_t*)a->out, a->ldo, R, a->heads,
+                                                                                                             a->vdim, splits);
     });
     B2L_LAUNCH_CHECK("seq_latent_combine_kernel");
   }
