@@ -4,17 +4,27 @@
 // every softmax weight (NP = 3): the products of the parts with bf16 keys or values are exact, the tensor core adds them in f32, so
 // the result is that of an f32 kernel up to the order of the sums.  Three bf16 MMAs cost 3 / 16 of what one f32 FMA costs on the CUDA cores.
 //
-//   warps 0..7   softmax: a thread owns one row (tensor-memory lane) and half of a tile's keys; scores by tcgen05.ld, maxima of the two
-//                halves through shared memory, weights back to tensor memory as the A operand of the second product.  The reference
-//                maximum of a row moves only when it is exceeded by more than 8 (weights reach e^8; nothing is rounded by that), so the
-//                output accumulator is rescaled a few times per row instead of once per tile.
-//   warps 8, 9   keys, warps 10, 11 values: rows gathered from the fresh projections or the cache ring by 16-byte cp.async into 128-byte
-//                swizzled rows (keys K-major, values MN-major for the second product), two or three stages
-//   warp 12      issues the MMAs: S(t+2) = Q K^T goes behind O += P(t) V, so the tensor pipe works while tile t+1 is exponentiated
-// Tensor memory: S 2 x 64 columns, O 128, P 2 x 3 x 32.  One CTA per SM.
+//   warp 0       issues the MMAs: S(t+2) = Q K^T goes behind O += P(t) V
+//   warps 1, 2   keys, warps 3, 12 values, into 128-byte swizzled rows (keys K-major, values MN-major for the second product), two or three
+//                stages.  Tiles of 64 consecutive rows (the fresh projections, an expanded latent) come by tiled TMA copies; tiles that touch
+//                the cache ring or end early by 16-byte cp.async, which arrive on the stage's barrier by themselves but take 3000 cycles
+//                to issue, twice what the rest of a tile takes
+//   warps 4..7   softmax of the even tiles, warps 8..11 of the odd ones: a thread owns one row (tensor-memory lane) of a tile.  The two
+//                groups are half a period apart, so one exponentiates while the other waits for tensor memory.  A row's reference maximum
+//                travels from tile to tile through shared memory and moves only when it is exceeded by more than 8 (weights reach e^8;
+//                nothing is rounded by that), so the output accumulator is rescaled a few times per row instead of once per tile.
+// Tensor memory: 2 x 96 columns for a tile's scores (the upper 64) and, behind the reader, its weights (24 columns per 16 keys: three
+// parts of 8); O 128; the rest holds query parts (all three
+// of a 128-entry head, two of a 192-entry one, the third stays in shared memory): with the query in shared memory an N = 64 MMA
+// reads 6 KB in its 48 cycles, which is all of the shared-memory bandwidth, and everything else on the SM waited for it.  One CTA per SM.
 //
-// Bound by the softmax warps and the tensor pipe alike: per 128 x 64 tile 1536 tensor cycles (head size 128) and about 20 instructions
-// per score on the CUDA cores.  The f32 kernel on the CUDA cores ran at 9-19 TFLOP/s.
+// All roles' loops together stay under the 12 KB or so that an instruction cache next to the schedulers holds: with the softmax written out
+// over 64 keys (26 KB) every role ran into instruction fetches (2.7 stalled warps per issued instruction) and an MMA took 120 cycles to
+// issue.  So a tile is taken in four steps of 16 keys, read from tensor memory once for the maximum and once for the weights.
+//
+// A 128 x 64 tile of head size 128 is 24 MMAs of 32 cycles and 12 of 64; it takes 2640 (3000 cycles of copies, then 5250 of softmax and issue
+// in the first form), bound by the issuing warp's waits between the two products.  Layer of width 2048, 2048 tokens, window 1024:
+// 811 us on the CUDA cores (9-19 TFLOP/s), 204 us so; latent layer 1555 -> 203 us.
 #pragma once
 #include "tc_common.cuh"
 
@@ -24,52 +34,62 @@ namespace atc {
 using namespace tc;
 
 constexpr int ROWS = 128, KEYS = 64;
-constexpr int SOFT_WARPS = 8, THREADS = 32 * (SOFT_WARPS + 5);
+constexpr int K_THREADS = 64, V_THREADS = 64, THREADS = 416;
 constexpr int Q_ATOM = ROWS * 128, K_ATOM = KEYS * 128;      // bytes of 64 columns of a query / key / value tile
-constexpr uint32_t COL_S = 0, COL_O = 128, COL_P = 256;
+constexpr uint32_t REGION = 96, S_AT = 32, COL_O = 192, COL_Q = 320;      // tile parity b: region at 96 b, scores at + 32, weights over them
 constexpr int MAX_DK = 192, MAX_DV = 128;
+constexpr int CONTROL = 3072;                                // barriers, tensor-memory address, row maxima
 
 __host__ __device__ inline int atoms(int d) { return (d + 63) / 64; }
-constexpr int CONTROL = 3072;                                // barriers, tensor-memory address, row maxima
-struct Layout { int stages; size_t smem; };
+struct Layout { int stages, q_tmem; size_t smem; };
 static inline Layout layout(int nq, int dk, int dv) {
   Layout l;
-  const size_t q = (size_t)nq * atoms(dk) * Q_ATOM, st = (size_t)(atoms(dk) + atoms(dv)) * K_ATOM;
+  l.q_tmem = (512 - (int)COL_Q) / (dk / 2);                  // query parts in tensor memory, the others in shared memory
+  if (l.q_tmem > nq) l.q_tmem = nq;
+  const size_t q = (size_t)(nq - l.q_tmem) * atoms(dk) * Q_ATOM, st = (size_t)(atoms(dk) + atoms(dv)) * K_ATOM;
   l.stages = CONTROL + q + 3 * st <= 227 * 1024 ? 3 : 2;
-  l.smem = CONTROL + q + l.stages * st;                    // head sizes 192 and 128: all of the 227 KB
-  if (l.smem < 120 * 1024) l.smem = 120 * 1024;            // one CTA per SM: each takes all of tensor memory
+  l.smem = CONTROL + q + l.stages * st;
+  if (l.smem < 120 * 1024) l.smem = 120 * 1024;              // one CTA per SM: each takes all of tensor memory
   return l;
 }
 
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void st_zero16(uint32_t dst) { asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0) : "memory"); }
-__device__ __forceinline__ void bar_named(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-
-__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+// 16 bytes, or zeros where `in` is false
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+// one arrival on the barrier when the thread's copies so far have landed
+__device__ __forceinline__ void cp_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void bar_named(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_named_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// The whole warp runs the issuing loop (descriptors stay in uniform registers); `lead` is set in the one lane that issues.
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+               "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
+               : "memory");
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+               "r"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
+               : "memory");
 }
 // MN-major operand, 128-byte swizzle: rows of 64 consecutive MN entries, one row per k; `lbo` bytes to the next 64 entries
 __device__ __forceinline__ uint64_t desc_mn(uint32_t addr, uint32_t lbo) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-#define B2L_R16(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7]), \
-                      "=r"(r[o + 8]), "=r"(r[o + 9]), "=r"(r[o + 10]), "=r"(r[o + 11]), "=r"(r[o + 12]), "=r"(r[o + 13]), "=r"(r[o + 14]), "=r"(r[o + 15])
-__device__ __forceinline__ void tmem_ld32(uint32_t a, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
-      "%25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : B2L_R16(r, 0), B2L_R16(r, 16)
-      : "r"(a)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-#undef B2L_R16
 __device__ __forceinline__ void tmem_st16(uint32_t a, const uint32_t (&r)[16]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(a), "r"(r[0]), "r"(r[1]),
                "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t a, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]),
+               "r"(r[6]), "r"(r[7])
                : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -81,33 +101,37 @@ __device__ __forceinline__ float rest(float x) { return x - __uint_as_float(__fl
 // Prob: what a family's attention is made of.  Members, all __device__:
 //   Tile tile()                           blockIdx -> {first row, rows, [j_begin, j_end) keys, ...}; per-CTA values in Prob::Tile
 //   Row row(tile, j)                      pointers of key j: ka (score entries 0 .. split8*8), kb (the rest), v
+//   bool bulk(tile, j0, ra, rb, rv)       keys j0 .. j0+63 are rows ra.. of map_a (64-column boxes from column tile.xa; the columns from
+//                                         split8*8 on: rows rb.. of map_b from tile.xb) and values rows rv.. of map_v from tile.xv
 //   void query(tile, r, c, float x[8])    query entries 8c .. 8c+7 of row r
 //   void range(tile, r, lo, hi)           keys lo .. hi are visible to row r
 //   float sink(tile)                      score of the sink, -inf without one
 //   bool partial(tile); void store_part(tile, r, c0, x[16]); void store_ml(tile, r, m, l)
 //   void store(tile, r, c0, x[16])        normalised outputs c0 .. c0+15
-// and the host-visible ints DK, DV, stages, split8, floats scale, softcap.
-template <class Prob, int NQ, int NP>
+// and the tensor maps, the host-visible ints DK, DV, stages, split8, q_tmem, floats scale, softcap.
+template <class Prob, int NQ, int NP, bool CAP>
 __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_constant__ Prob pr) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  float (&s_max)[2][2][ROWS] = *reinterpret_cast<float (*)[2][2][ROWS]>(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + sizeof(s_max));      // 18
+  float* s_ref = reinterpret_cast<float*>(smem_raw);         // [ROWS] a row's reference maximum after the latest tile
+  float* s_end = s_ref + ROWS;                               // [2][ROWS] maximum and sum of the other group at the end
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 18
   uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 18);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages;
-  const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + NQ * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
+  const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages, nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
+  const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
   const uint32_t b0 = smem_u32(bars);
   const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 112, pv_done = b0 + 128;
   uint32_t dead = (sq & 1023u) ? 1u : 0u;                    // swizzle atoms need 1024-byte alignment (shared memory starts on one)
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) {
-      mbar_init(k_full + 8 * i, 2); mbar_init(k_empty + 8 * i, 1);
-      mbar_init(v_full + 8 * i, 2); mbar_init(v_empty + 8 * i, 1);
+      mbar_init(k_full + 8 * i, K_THREADS); mbar_init(k_empty + 8 * i, 1);
+      mbar_init(v_full + 8 * i, V_THREADS); mbar_init(v_empty + 8 * i, 1);
     }
-    for (int i = 0; i < 2; ++i) { mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, SOFT_WARPS); mbar_init(pv_done + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, 4); mbar_init(pv_done + 8 * i, 1); }
     mbar_init_fence();
   }
-  if (warp == SOFT_WARPS + 4) tmem_alloc(smem_u32(&tmem_slot), 512);
+  if (tid < ROWS) s_ref[tid] = -INFINITY;
+  if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 512);
   fence_before();
   __syncthreads();
   fence_after();
@@ -115,138 +139,223 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   const typename Prob::Tile tl = pr.tile();
   const int n = (tl.j_end - tl.j_begin + KEYS - 1) / KEYS;
 
-  if (warp >= SOFT_WARPS && warp < SOFT_WARPS + 4) {
-    // ===================== keys (two warps) and values (two warps) =====================
-    const bool keys = warp < SOFT_WARPS + 2;
-    const int lt = tid - 32 * (keys ? SOFT_WARPS : SOFT_WARPS + 2), r0 = lt >> 3, c0 = lt & 7;
-    const int chunks = (keys ? pr.DK : pr.DV) / 8;
-    const uint32_t base = keys ? sk : sv, stage = (uint32_t)(keys ? ka : va) * K_ATOM, full = keys ? k_full : v_full, empty = keys ? k_empty : v_empty;
-    for (int t = 0; t < n; ++t) {
-      const int st = t % nst;
-      if (t >= nst) mbar_wait(empty + 8 * st, (uint32_t)(t / nst - 1) & 1u, dead);
-      const uint32_t dst0 = base + st * stage;
-#pragma unroll 2
-      for (int i = 0; i < KEYS / 8; ++i) {
-        const int r = r0 + 8 * i, j = tl.j_begin + t * KEYS + r;
-        const uint32_t dst = dst0 + r * 128 + ((c0 ^ (r & 7)) << 4);
-        if (j < tl.j_end) {
-          const typename Prob::Row row = pr.row(tl, j);
-          for (int c = c0; c < chunks; c += 8)
-            cp16(dst + (c >> 3) * K_ATOM, keys ? (c < pr.split8 ? row.ka + c * 8 : row.kb + (c - pr.split8) * 8) : row.v + c * 8);
-        } else {
-          for (int c = c0; c < chunks; c += 8) st_zero16(dst + (c >> 3) * K_ATOM);
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(full + 8 * st);
-    }
-  } else if (warp == SOFT_WARPS + 4) {
+  if (warp == 0) {
     // ===================== MMA issue =====================
-    bar_named(9, 32 * (SOFT_WARPS + 1));                     // the query tile is in shared memory
-    if (lane == 0) {
+    bar_named(9, 32 + 2 * ROWS);                             // the queries are in place
+    {
+      const uint32_t lead = elect_lane();
       fence_after();
       const uint32_t id_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KEYS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
       const uint32_t id_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(pr.DV >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
-      const int ks = pr.DK / 16;
+      const int full = pr.DK / 64, odd = pr.DK / 16 % 4;      // steps of 16 entries: four per 64, and the rest
+      auto copied = [&](int t) {                             // cp.async writes through the generic proxy; the fence costs some 300 cycles
+        int ra, rb, rv;
+        if (!pr.bulk(tl, tl.j_begin + t * KEYS, ra, rb, rv)) fence_proxy_async();
+      };
+      int k_st = 0, v_st = 0;                                // stages and their phases, counted instead of divided out
+      uint32_t k_ph = 0, v_ph = 0;
       auto score = [&](int t) {
-        const int st = t % nst;
-        mbar_wait(k_full + 8 * st, (uint32_t)(t / nst) & 1u, dead);
+        const int st = k_st;
+        mbar_wait(k_full + 8 * st, k_ph, dead);
+        if (++k_st == nst) { k_st = 0; k_ph ^= 1u; }
         if (dead) return;
+        copied(t);
         fence_after();
-        const uint32_t kb = sk + st * ka * K_ATOM;
+        const uint32_t kb = sk + st * ka * K_ATOM, d = tmem + REGION * (t & 1) + S_AT;
+        const uint64_t kd0 = desc_sw128(kb);
+        uint32_t acc = 0;
 #pragma unroll 1
         for (int s = NQ - 1; s >= 0; --s) {                  // the smallest parts first
-          const uint32_t qb = sq + s * ka * Q_ATOM;
-          for (int k = 0; k < ks; ++k)
-            mma_ss(tmem + COL_S + 64 * (t & 1), desc_sw128(qb + (k >> 2) * Q_ATOM) + 2 * (k & 3), desc_sw128(kb + (k >> 2) * K_ATOM) + 2 * (k & 3), id_s,
-                   (s < NQ - 1 || k > 0) ? 1u : 0u);
+          uint64_t kd = kd0;
+          if (s >= nsm) {
+            uint32_t qa = tmem + COL_Q + (s - nsm) * (pr.DK / 2);
+#pragma unroll 1
+            for (int a = 0; a < full; ++a, qa += 32, kd += K_ATOM >> 4) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mma_ts(d, qa + 8 * k, kd + 2 * k, id_s, k > 0 ? 1u : acc, lead);
+              acc = 1;
+            }
+#pragma unroll 1
+            for (int k = 0; k < odd; ++k, acc = 1) mma_ts(d, qa + 8 * k, kd + 2 * k, id_s, acc, lead);
+          } else {
+            uint64_t qd = desc_sw128(sq + s * ka * Q_ATOM);
+#pragma unroll 1
+            for (int a = 0; a < full; ++a, qd += Q_ATOM >> 4, kd += K_ATOM >> 4) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mma_ss(d, qd + 2 * k, kd + 2 * k, id_s, k > 0 ? 1u : acc, lead);
+              acc = 1;
+            }
+#pragma unroll 1
+            for (int k = 0; k < odd; ++k, acc = 1) mma_ss(d, qd + 2 * k, kd + 2 * k, id_s, acc, lead);
+          }
         }
-        commit(s_full + 8 * (t & 1));
-        commit(k_empty + 8 * st);
+        if (lead) {
+          commit(s_full + 8 * (t & 1));
+          commit(k_empty + 8 * st);
+        }
+        __syncwarp();
       };
       if (n > 0) score(0);                                   // an empty key split has no tile
       if (n > 1) score(1);
       for (int t = 0; t < n && !dead; ++t) {
-        const int st = t % nst;
+        const int st = v_st;
+        mbar_wait(v_full + 8 * st, v_ph, dead);
+        if (++v_st == nst) { v_st = 0; v_ph ^= 1u; }
         mbar_wait(p_full + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, dead);
-        mbar_wait(v_full + 8 * st, (uint32_t)(t / nst) & 1u, dead);
         if (dead) break;
+        copied(t);
         fence_after();
-        const uint32_t vb = sv + st * va * K_ATOM, pc = tmem + COL_P + 96 * (t & 1);
+        const uint64_t vd = desc_mn(sv + st * va * K_ATOM, K_ATOM);
+        const uint32_t pc = tmem + REGION * (t & 1);
+#pragma unroll 1
+        for (int q = NP - 1; q >= 0; --q)
 #pragma unroll
-        for (int s = NP - 1; s >= 0; --s)
-#pragma unroll
-          for (int k = 0; k < KEYS / 16; ++k)
-            mma_ts(tmem + COL_O, pc + 32 * s + 8 * k, desc_mn(vb + k * 16 * 128, K_ATOM), id_o, (t > 0 || s < NP - 1 || k > 0) ? 1u : 0u);
-        commit(v_empty + 8 * st);
-        commit(pv_done + 8 * (t & 1));
-        if (t + 2 < n) score(t + 2);                         // its scores' buffer was read before the weights of tile t arrived
+          for (int k = 0; k < KEYS / 16; ++k) mma_ts(tmem + COL_O, pc + 24 * k + 8 * q, vd + k * (16 * 128 / 16), id_o, (t > 0 || q < NP - 1 || k > 0) ? 1u : 0u, lead);
+        if (lead) {
+          commit(v_empty + 8 * st);
+          commit(pv_done + 8 * (t & 1));
+        }
+        __syncwarp();
+        if (t + 2 < n) score(t + 2);                         // over the weights of tile t, which the MMAs before it have read
       }
     }
     __syncwarp();
+  } else if (warp < 4 || warp == 12) {
+    // ===================== keys and values, two warps each =====================
+    const bool keys = warp < 3;
+    const int lt = keys ? tid - 32 : (warp == 12 ? 32 : 0) + lane, r0 = lt >> 3, c0 = lt & 7;
+    const int chunks = (keys ? pr.DK : pr.DV) / 8;
+    const uint32_t base = keys ? sk : sv, stage = (uint32_t)(keys ? ka : va) * K_ATOM, full = keys ? k_full : v_full, empty = keys ? k_empty : v_empty;
+    int st = -1;
+    uint32_t phase = 0;                                      // parity of the stage's previous use
+    for (int t = 0; t < n; ++t) {
+      if (++st == nst) { st = 0; phase ^= t > nst ? 1u : 0u; }
+      if (t >= nst) mbar_wait(empty + 8 * st, phase, dead);
+      const uint32_t dst0 = base + st * stage;
+      const int j0 = tl.j_begin + t * KEYS;
+      int row_a, row_b, row_v;
+      if (pr.bulk(tl, j0, row_a, row_b, row_v)) {            // 64 consecutive rows: a tiled copy per 64 columns
+        if (lt == 0) {
+          mbar_expect_tx(full + 8 * st, stage);
+          if (keys) {
+            for (int a = 0; a < ka; ++a) {
+              if (8 * a < pr.split8) tma_load_2d(dst0 + a * K_ATOM, &pr.map_a, tl.xa + 64 * a, row_a, full + 8 * st);
+              else tma_load_2d(dst0 + a * K_ATOM, &pr.map_b, tl.xb + 64 * a - 8 * pr.split8, row_b, full + 8 * st);
+            }
+          } else {
+            for (int a = 0; a < va; ++a) tma_load_2d(dst0 + a * K_ATOM, &pr.map_v, tl.xv + 64 * a, row_v, full + 8 * st);
+          }
+        } else {
+          mbar_arrive(full + 8 * st);
+        }
+        continue;
+      }
+#pragma unroll 2
+      for (int i = 0; i < KEYS / 8; ++i) {
+        const int r = r0 + 8 * i, j = j0 + r;
+        const bool in = j < tl.j_end;
+        const uint32_t dst = dst0 + r * 128 + ((c0 ^ (r & 7)) << 4);
+        const typename Prob::Row row = pr.row(tl, in ? j : tl.j_begin);
+#pragma unroll
+        for (int a = 0; a < MAX_DK / 64; ++a) {
+          const int c = c0 + 8 * a;
+          if (c < chunks) cp16(dst + a * K_ATOM, keys ? (c < pr.split8 ? row.ka + c * 8 : row.kb + (c - pr.split8) * 8) : row.v + c * 8, in);
+        }
+      }
+      cp_arrive(full + 8 * st);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");         // no copy outlives its thread
   } else {
     // ===================== queries, softmax, output =====================
-    const int qtr = warp & 3, half = warp >> 2, r = qtr * 32 + lane;
-    for (int i = tid; i < ROWS * (pr.DK / 8); i += 32 * SOFT_WARPS) {
-      const int rr = i / (pr.DK / 8), c = i - rr * (pr.DK / 8);
-      float x[8];
+    const int qtr = warp & 3, b = (warp >> 2) - 1, r = qtr * 32 + lane;      // b: the parity of the group's tiles
+    const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
+    for (int g = b; g < pr.DK / 16; g += 2) {                // the groups take turns with 16 entries of a row
+      float x[16];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] = 0.f;
-      if (rr < tl.rows) pr.query(tl, rr, c, x);
-      const uint32_t dst = sq + (c >> 3) * Q_ATOM + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
+      for (int e = 0; e < 16; ++e) x[e] = 0.f;
+      if (r < tl.rows) {
+        pr.query(tl, r, 2 * g, *reinterpret_cast<float (*)[8]>(x));
+        pr.query(tl, r, 2 * g + 1, *reinterpret_cast<float (*)[8]>(x + 8));
+      }
+      __syncwarp();
 #pragma unroll
       for (int s = 0; s < NQ; ++s) {
-        const uint32_t w0 = hi_pair(x[0], x[1]), w1 = hi_pair(x[2], x[3]), w2 = hi_pair(x[4], x[5]), w3 = hi_pair(x[6], x[7]);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + s * ka * Q_ATOM), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+        uint32_t w[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = fabsf(x[e]) < INFINITY ? rest(x[e]) : 0.f;
+        for (int e = 0; e < 8; ++e) w[e] = hi_pair(x[2 * e], x[2 * e + 1]);
+        if (s >= nsm) {
+          tmem_st8(tmem + lane_at + COL_Q + (s - nsm) * (pr.DK / 2) + 8 * g, w);
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = 2 * g + h;
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sq + (s * ka + (c >> 3)) * Q_ATOM + r * 128 + (((c & 7) ^ (r & 7)) << 4)), "r"(w[4 * h]),
+                         "r"(w[4 * h + 1]), "r"(w[4 * h + 2]), "r"(w[4 * h + 3]) : "memory");
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[e] = fabsf(x[e]) < INFINITY ? rest(x[e]) : 0.f;
       }
     }
+    tmem_wait_st();
+    fence_before();
     fence_proxy_async();
-    bar_named(9, 32 * (SOFT_WARPS + 1));
+    bar_named(9, 32 + 2 * ROWS);
 
     int lo, hi;
     pr.range(tl, r, lo, hi);
     if (r >= tl.rows) { lo = 1; hi = 0; }
-    const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
-    float m = -INFINITY, l = 0.f;
-    for (int t = 0; t < n; ++t) {
-      const int b = t & 1;
+    float m = -INFINITY, l = 0.f;                            // reference maximum, and the sum over this group's tiles relative to it
+    for (int t = b; t < n; t += 2) {
       mbar_wait(s_full + 8 * b, (uint32_t)(t >> 1) & 1u, dead);
       fence_after();
-      uint32_t sr[32];
-      tmem_ld32(tmem + lane_at + COL_S + 64 * b + 32 * half, sr);
-      float s[32], mx = -INFINITY;
-      const int at = tl.j_begin + t * KEYS + 32 * half, first = lo - at, last = hi - at;      // keys first .. last of these 32 are seen
+      const uint32_t reg = tmem + lane_at + REGION * b;
+      const int at = tl.j_begin + t * KEYS, first = lo - at, last = hi - at;      // keys first .. last of these 64 are seen
+      const bool cut = __any_sync(0xffffffffu, first > 0 || last < KEYS - 1);
+      float mx = -INFINITY;
+#pragma unroll 1
+      for (int c = 0; c < KEYS / 16; ++c) {
+        uint32_t u[16];
+        tmem_ld16(reg + S_AT + 16 * c, u);
+        float s[16];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) s[i] = __uint_as_float(sr[i]) * pr.scale;
-      if (pr.softcap > 0.f) {
+        for (int i = 0; i < 16; ++i) s[i] = __uint_as_float(u[i]) * pr.scale;
+        if (CAP) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) s[i] = pr.softcap * tanhf(s[i] / pr.softcap);
+          for (int i = 0; i < 16; ++i) s[i] = pr.softcap * tanhf(s[i] / pr.softcap);
+        }
+        if (cut) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) s[i] = (16 * c + i >= first && 16 * c + i <= last) ? s[i] : -INFINITY;
+        }
+        if (CAP || cut) {                                    // the weights are taken from what is left here
+#pragma unroll
+          for (int i = 0; i < 16; ++i) u[i] = __float_as_uint(s[i]);
+          tmem_st16(reg + S_AT + 16 * c, u);
+        }
+        float m2[2] = {mx, s[0]};
+#pragma unroll
+        for (int i = 1; i < 16; ++i) m2[i & 1] = fmaxf(m2[i & 1], s[i]);
+        mx = fmaxf(m2[0], m2[1]);
       }
-      if (first > 0 || last < 31) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) s[i] = (i >= first && i <= last) ? s[i] : -INFINITY;
+      const float scale = (CAP || cut) ? 1.f : pr.scale;
+      if (CAP || cut) tmem_wait_st();
+      // the row's reference after tile t - 1, from the other group; this tile's goes to it (barriers 1..4 even -> odd, 5..8 odd -> even)
+      if (t > 0) bar_named(1 + 4 * (b ^ 1) + qtr, 64);
+      const float ref = s_ref[r];
+      const bool up = mx > ref + 8.f;                        // also the first key a row sees (ref = -inf)
+      const float now = up ? mx : ref;
+      if (up) s_ref[r] = now;
+      if (t + 1 < n) bar_named_arrive(1 + 4 * b + qtr, 64);
+      if (m != now) {
+        l *= m == -INFINITY ? 0.f : expf(m - now);
+        m = now;
       }
-#pragma unroll
-      for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
-      s_max[b][half][r] = mx;
-      bar_named(1 + qtr, 64);
-      mx = fmaxf(mx, s_max[b][half ^ 1][r]);
-      if (t >= 2) mbar_wait(pv_done + 8 * b, (uint32_t)((t >> 1) - 1) & 1u, dead);            // P[b] has been read
-      float f = 1.f;
-      if (mx > m + 8.f) {                                   // also the first key a row sees (m = -inf)
-        f = m == -INFINITY ? 1.f : expf(m - mx);            // nothing has been added to a row that has seen no key
-        m = mx;
-      }
-      l *= f;
-      if (__any_sync(0xffffffffu, f != 1.f)) {              // t > 0 here
+      const float f = (up && ref != -INFINITY) ? expf(ref - now) : 1.f;      // nothing was added to a row that saw no key
+      if (__any_sync(0xffffffffu, f != 1.f)) {               // t > 0 here; the scores of this tile came after PV(t - 2)
         mbar_wait(pv_done + 8 * (b ^ 1), (uint32_t)((t - 1) >> 1) & 1u, dead);
         fence_after();
-        for (int g = half; g < pr.DV / 16; g += 2) {
+        for (int g = 0; g < pr.DV / 16; ++g) {
           uint32_t o[16];
           tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
 #pragma unroll
@@ -254,41 +363,57 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
           tmem_st16(tmem + lane_at + COL_O + 16 * g, o);
         }
       }
-      float sum = 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        s[i] = s[i] == -INFINITY ? 0.f : expf(s[i] - m);
-        sum += s[i];
-      }
-      l += sum;
-#pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        uint32_t w[16];
+      const float mm = m == -INFINITY ? 0.f : m;             // a row that has seen no key: every score is -inf, every weight 0
+      float sum[2] = {0.f, 0.f};
+#pragma unroll 1
+      for (int c = 0; c < KEYS / 16; ++c) {
+        uint32_t u[16];
+        tmem_ld16(reg + S_AT + 16 * c, u);
+        float s[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          w[i] = hi_pair(s[2 * i], s[2 * i + 1]);
-          s[2 * i] = rest(s[2 * i]);
-          s[2 * i + 1] = rest(s[2 * i + 1]);
+          s[i] = expf(__uint_as_float(u[i]) * scale - mm);
+          sum[i & 1] += s[i];
         }
-        tmem_st16(tmem + lane_at + COL_P + 96 * b + 32 * q + 16 * half, w);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          uint32_t w[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            w[i] = hi_pair(s[2 * i], s[2 * i + 1]);
+            if (q + 1 < NP) { s[2 * i] = rest(s[2 * i]); s[2 * i + 1] = rest(s[2 * i + 1]); }
+          }
+          tmem_st8(reg + 24 * c + 8 * q, w);
+        }
       }
+      l += sum[0] + sum[1];
       tmem_wait_st();
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full + 8 * b);
     }
-    s_max[n & 1][half][r] = l;                               // the buffer of tile n - 2: both warps are past it
-    bar_named(1 + qtr, 64);
-    l = s_max[n & 1][0][r] + s_max[n & 1][1][r];
+    // the even group ends with the sum of both (relative to the last reference); each group stores every other 16 columns
     if (n > 0) mbar_wait(pv_done + 8 * ((n - 1) & 1), (uint32_t)((n - 1) >> 1) & 1u, dead);
     fence_after();
+    if (b == 1) { s_end[r] = m; s_end[ROWS + r] = l; }
+    bar_named(10, 2 * ROWS);
+    const float ref = s_ref[r];
+    float* tot = s_end;                                      // [ROWS]: the sum, for both groups
+    if (b == 0) {
+      const float m1 = s_end[r], l1 = s_end[ROWS + r];
+      l = (m == -INFINITY ? 0.f : l * expf(m - ref)) + (m1 == -INFINITY ? 0.f : l1 * expf(m1 - ref));
+      tot[r] = l;
+    }
+    bar_named(10, 2 * ROWS);
+    l = tot[r];
+    m = ref;
     const bool part = pr.partial(tl), live = r < tl.rows;
     const float sink = pr.sink(tl), M = fmaxf(m, sink);
     const float e = m == -INFINITY ? 0.f : expf(m - M);
     float inv = e / (l * e + (sink == -INFINITY ? 0.f : expf(sink - M)));
     if (dead) inv = l = __int_as_float(0x7fc00000);
-    if (part && live && half == 0) pr.store_ml(tl, r, m, l);
-    for (int g = half; g < pr.DV / 16; g += 2) {
+    if (part && live && b == 0) pr.store_ml(tl, r, m, l);
+    for (int g = b; g < pr.DV / 16; g += 2) {
       uint32_t o[16];
       __syncwarp();
       tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
@@ -303,13 +428,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   }
   fence_before();
   __syncthreads();
-  if (warp == SOFT_WARPS + 4) tmem_dealloc(tmem, 512);
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-template <class Prob, int NQ, int NP>
+template <class Prob, int NQ, int NP, bool CAP>
 static int launch(const Prob& p, dim3 grid, size_t smem, DynSmemCache& cache, cudaStream_t st) {
-  if (int rc = ensure_dyn_smem(attn_tc_kernel<Prob, NQ, NP>, smem, cache)) return rc;
-  attn_tc_kernel<Prob, NQ, NP><<<grid, THREADS, smem, st>>>(p);
+  if (int rc = ensure_dyn_smem(attn_tc_kernel<Prob, NQ, NP, CAP>, smem, cache)) return rc;
+  attn_tc_kernel<Prob, NQ, NP, CAP><<<grid, THREADS, smem, st>>>(p);
   B2L_LAUNCH_CHECK("attn_tc_kernel");
   return 0;
 }

@@ -640,38 +640,54 @@ static int launch_tile(const b2l_seq_attn_args* a, cudaStream_t s, int cache_slo
 // ---- prompt portions with bf16 keys and values: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, 1), the tiles with the
 // most keys first.
 struct LocalProb {
+  CUtensorMap map_a, map_b, map_v;
   b2l_seq_attn_args a;
-  int DK, DV, stages, split8;
+  int DK, DV, stages, split8, q_tmem;
   float scale, softcap;
   struct Tile {
-    int h, gk, gv, kh, t_first, rows, pos0, j_begin, j_end;
+    int h, t_first, rows, pos0, j_begin, j_end, ring0, sk, sv, xa, xb, xv;
     const __nv_bfloat16 *kn, *vn, *ck, *cv;
   };
   struct Row { const __nv_bfloat16 *ka, *kb, *v; };
   __device__ __forceinline__ Tile tile() const {
     Tile t;
     t.h = blockIdx.x;
-    kv_heads_of(a, t.h, t.gk, t.gv);
-    t.kh = a.kv_heads * (a.maps > 1 ? a.maps : 1);
+    int gk, gv;
+    kv_heads_of(a, t.h, gk, gv);
+    t.sk = a.kv_heads * (a.maps > 1 ? a.maps : 1) * a.K;
+    t.sv = a.kv_heads * a.V;
     t.t_first = ((int)gridDim.y - 1 - (int)blockIdx.y) * atc::ROWS;
     t.rows = min(atc::ROWS, a.T - t.t_first);
     const int slot = a.meta[0];
     t.pos0 = a.meta[1];
     t.j_begin = first_visible(a, t.pos0 + t.t_first);
     t.j_end = t.pos0 + t.t_first + t.rows;
-    t.kn = (const __nv_bfloat16*)a.k_new;
-    t.vn = (const __nv_bfloat16*)a.v_new;
-    t.ck = (const __nv_bfloat16*)a.cache_k + (size_t)slot * a.block * t.kh * a.K;
-    t.cv = (const __nv_bfloat16*)a.cache_v + (size_t)slot * a.block * a.kv_heads * a.V;
+    t.ring0 = t.j_begin / a.block * a.block;
+    t.xa = gk * a.K;
+    t.xb = 0;
+    t.xv = gv * a.V;
+    t.kn = (const __nv_bfloat16*)a.k_new + (size_t)gk * a.K;
+    t.vn = (const __nv_bfloat16*)a.v_new + (size_t)gv * a.V;
+    t.ck = (const __nv_bfloat16*)a.cache_k + (size_t)slot * a.block * t.sk + (size_t)gk * a.K;
+    t.cv = (const __nv_bfloat16*)a.cache_v + (size_t)slot * a.block * t.sv + (size_t)gv * a.V;
     return t;
   }
   __device__ __forceinline__ Row row(const Tile& t, int j) const {
     Row r;
-    const int e = j % a.block;
-    r.ka = j >= t.pos0 ? t.kn + ((size_t)(j - t.pos0) * t.kh + t.gk) * a.K : t.ck + ((size_t)e * t.kh + t.gk) * a.K;
+    // cached keys lie less than a ring before the portion: one turn past ring0 at most
+    const bool fresh = j >= t.pos0;
+    int e = j - t.ring0;
+    if (e >= a.block) e -= a.block;
+    if (fresh) e = j - t.pos0;
+    r.ka = (fresh ? t.kn : t.ck) + (long long)e * t.sk;
     r.kb = nullptr;
-    r.v = j >= t.pos0 ? t.vn + (size_t)(j - t.pos0) * a.ldv + (size_t)t.gv * a.V : t.cv + ((size_t)e * a.kv_heads + t.gv) * a.V;
+    r.v = (fresh ? t.vn : t.cv) + (long long)e * (fresh ? a.ldv : t.sv);
     return r;
+  }
+  __device__ __forceinline__ bool bulk(const Tile& t, int j0, int& ra, int& rb, int& rv) const {
+    ra = rv = j0 - t.pos0;                                    // rows past the portion's last read as zeros
+    rb = 0;
+    return j0 >= t.pos0;
   }
   __device__ __forceinline__ void query(const Tile& t, int r, int c, float (&x)[8]) const {
     const float4* q = reinterpret_cast<const float4*>(a.q + ((size_t)(t.t_first + r) * a.heads + t.h) * a.K + 8 * c);
@@ -697,12 +713,19 @@ struct LocalProb {
   }
 };
 
-static DynSmemCache g_local_tc_smem;
+static DynSmemCache g_local_tc_smem[2];
 
 static int launch_local_tc(const b2l_seq_attn_args* a, cudaStream_t s) {
   const atc::Layout l = atc::layout(3, a->K, a->V);
-  LocalProb p{*a, a->K, a->V, l.stages, 1 << 20, a->scale, a->softcap};
-  return atc::launch<LocalProb, 3, 3>(p, dim3((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS)), l.smem, g_local_tc_smem, s);
+  LocalProb p;
+  const int sk = a->kv_heads * (a->maps > 1 ? a->maps : 1) * a->K;
+  if (int rc = tc::map_sw128(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->k_new, a->T, sk, sk, 64, atc::KEYS)) return rc;
+  if (int rc = tc::map_sw128(&p.map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->v_new, a->T, (long long)a->kv_heads * a->V, a->ldv, 64, atc::KEYS)) return rc;
+  p.map_b = p.map_a;
+  p.a = *a; p.DK = a->K; p.DV = a->V; p.stages = l.stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = a->softcap;
+  const dim3 grid((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS));
+  return a->softcap > 0.f ? atc::launch<LocalProb, 3, 3, true>(p, grid, l.smem, g_local_tc_smem[1], s)
+                          : atc::launch<LocalProb, 3, 3, false>(p, grid, l.smem, g_local_tc_smem[0], s);
 }
 
 // ring[p % block] <- token p for the portion's tokens in the block of its last token (block-local) or for its last

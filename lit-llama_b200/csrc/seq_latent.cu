@@ -510,11 +510,12 @@ __global__ void seq_head_gate_kernel(const act_t* __restrict__ in, long long ld_
 // ---- the expanded form of a prompt portion in bf16: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, key splits), the tiles
 // with the most keys first.
 struct LatentProb {
+  CUtensorMap map_a, map_b, map_v;
   b2l_seq_latent_attn_args a;
-  int DK, DV, stages, split8;
+  int DK, DV, stages, split8, q_tmem, tiled;
   float scale, softcap;
   struct Tile {
-    int h, t_first, rows, pos0, j_begin, j_end;
+    int h, t_first, rows, pos0, j_begin, j_end, xa, xb, xv, row_b;
     const __nv_bfloat16 *key_a, *key_b;
   };
   struct Row { const __nv_bfloat16 *ka, *kb, *v; };
@@ -530,6 +531,10 @@ struct LatentProb {
     per = (per + atc::KEYS - 1) / atc::KEYS * atc::KEYS;
     t.j_begin = min(end, begin + (int)blockIdx.z * per);
     t.j_end = min(end, t.j_begin + per);
+    t.xv = (int)(t.h * a.hska);
+    t.xa = t.xv + a.score_off;
+    t.xb = 0;
+    t.row_b = a.n_b > 0 ? (int)(slot * (a.slot_stride_b / a.ldkb)) : 0;
     t.key_a = reinterpret_cast<const __nv_bfloat16*>(a.key_a) + (long long)slot * a.slot_stride_a + (long long)t.h * a.hska;
     t.key_b = reinterpret_cast<const __nv_bfloat16*>(a.key_b) + (long long)slot * a.slot_stride_b;
     return t;
@@ -540,6 +545,11 @@ struct LatentProb {
     r.ka = r.v + a.score_off;
     r.kb = t.key_b + (long long)j * a.ldkb;
     return r;
+  }
+  __device__ __forceinline__ bool bulk(const Tile& t, int j0, int& ra, int& rb, int& rv) const {
+    ra = rv = j0;
+    rb = j0 + t.row_b;
+    return tiled && j0 + atc::KEYS <= t.j_end;                // the maps do not know where the rows end
   }
   __device__ __forceinline__ void query(const Tile& t, int r, int c, float (&x)[8]) const {
     const long long tt = t.t_first + r;
@@ -586,8 +596,20 @@ static bool latent_tc(const b2l_seq_latent_attn_args* a) {
 static int launch_latent_tc(const b2l_seq_latent_attn_args* a, int splits, cudaStream_t st) {
   const int dn = a->n_a - a->score_off, dk = dn + a->n_b;
   const atc::Layout l = atc::layout(3, dk, a->vdim);
-  LatentProb p{*a, dk, a->vdim, l.stages, dn / 8, a->scale, 0.f};
-  return atc::launch<LatentProb, 3, 3>(p, dim3((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS), (unsigned)splits), l.smem, g_lat_tc_smem, st);
+  LatentProb p;
+  p.a = *a; p.DK = dk; p.DV = a->vdim; p.stages = l.stages; p.split8 = dn / 8; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = 0.f;
+  // tiled copies: rows of one slot's keys counted from position 0 (only rows of visible positions are read), whole 64-column steps per part.
+  // The shared part lies in the slot that the device names: its rows are reached through the map only when the rows of all slots follow one
+  // another, and then from slot 0's first.
+  p.tiled = a->slot_stride_a == 0 && (a->n_b == 0 || (dn % 64 == 0 && a->slot_stride_b % a->ldkb == 0));
+  if (p.tiled) {
+    const long long rows = 1LL << 31;
+    if (int rc = tc::map_sw128(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->key_a, rows, (a->heads - 1) * a->hska + a->n_a, a->ldka, 64, atc::KEYS)) return rc;
+    p.map_v = p.map_b = p.map_a;
+    if (a->n_b > 0)
+      if (int rc = tc::map_sw128(&p.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->key_b, rows, a->n_b, a->ldkb, 64, atc::KEYS)) return rc;
+  }
+  return atc::launch<LatentProb, 3, 3, false>(p, dim3((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS), (unsigned)splits), l.smem, g_lat_tc_smem, st);
 }
 
 static DynSmemCache g_lat_smem[8];
