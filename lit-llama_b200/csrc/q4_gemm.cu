@@ -1,264 +1,269 @@
-// Prefill-shaped int4 weight-only GEMM on the 5th-generation tensor cores: y[M, N] = x[M, K] . dequant(W)[N, K]^T
-// for M > 16 (prompt processing, no-cache forward, evaluation; BASELINE.json configs[3] prefill 8 x 512).
+// Prompt-shaped int4 weight-only GEMM on the 5th-generation tensor cores: y[M, N] = x[M, K] . dequant(W)[N, K]^T for M > 16 (prompt
+// processing, no-cache forward, evaluation).
 //
-// Replaces ColBlockQuantizedLinear.forward (lit_llama/quantization.py:413-423) and the Triton kernel
-// linear_kernel_4bit_weight (quantization.py:187-333: tiles up to 256 x 256, dequantise inside the tile loop) for
-// 4-bit weights with one (scale, zero) per output row.  Round 1 sent this shape to a dequantise + library GEMM.
+// Replaces ColBlockQuantizedLinear.forward (lit_llama/quantization.py:413-423) and the Triton kernel linear_kernel_4bit_weight
+// (quantization.py:187-333: tiles up to 256 x 256, dequantise inside the tile loop) for 4-bit weights with one (scale, zero) per row.
 //
-// One CTA computes a 256 (tokens) x 256 (output features) tile of y over the full K:
-//   warp 0, one elected lane: tcgen05.mma.cta_group::1.kind::f16 (bf16 x bf16 -> fp32), M = 128, N = 256, K = 16,
-//       both operands from shared memory (K-major canonical core-matrix layout, no swizzle), two accumulators
-//       (token rows 0..127 and 128..255) of 256 columns each = all 512 columns of tensor memory;
-//       tcgen05.commit releases a stage to the producers and finally hands the accumulators to the epilogue;
-//   warps 1..8 (256 threads = the 256 weight rows of the tile), per 64-wide k stage:
-//       * the activation tile [256 tokens][64 k]: ONE tensor-map TMA copy (cp.async.bulk.tensor.3d) per stage.  x is
-//         described to the TMA unit as a 3-D tensor (8 elements = 16 B | M rows, stride ldx | K/8 chunks, stride 16 B),
-//         so a box of 8 x 256 x 8 lands in shared memory as [k chunk][row][16 B] -- exactly the no-swizzle
-//         K-major core-matrix order tcgen05 reads; rows beyond M are zero-filled by the TMA unit;
-//       * two LDG.128 of packed levels per thread (load-time tiling b2l_q4_tile: a row's 32 levels of a k slab in
-//         16 bytes, nibble order chosen so that (w >> 4s) & 0x000f000f | 0x43004300 IS the bf16 pair
-//         (128 + level[k], 128 + level[k+1])), dequantised with the reference's own rounding:
-//         level = v - 128 (exact), level - zero (bf16), * scale (bf16) -- bit-identical to get_weight
-//         (quantization.py:392-411), so the GEMM sees exactly the matrix the reference's dense branch multiplies;
-//       * 16-byte st.shared of 8 consecutive k of a row = one row of a core matrix; fence.proxy.async; mbarrier arrive;
-//   afterwards the same 8 warps are the epilogue: tcgen05.ld 32x32b (a warp reaches the TMEM lanes of its
-//   warp_id % 4 quarter), fp32 -> bf16, 32-byte stores.
-// The dequantisation costs the 8 producer warps ~400 issue cycles per stage against 1024 tensor-pipe cycles
-// (8 MMAs of 128 x 256 x 16), so the tensor pipe is the bound; a 4-deep ring (64 KB per stage) hides the loads.
-#include <cuda.h>   // CUtensorMap and its enums only: the encoder is fetched with cudaGetDriverEntryPoint (no libcuda link)
-
-#include <cstdlib>
-
-#include "b2l_common.cuh"
+// A CTA computes 128 output features x `bt` tokens (16..256), the WEIGHT as the 128-row operand in tensor memory:
+//   warp 0       TMA: per 64-wide k stage the 4 KB of packed levels (load-time tiling b2l_q4_tile: contiguous) and the activation tile
+//                [bt tokens][64 k] as one 128-byte swizzled box, on one mbarrier; rows beyond M are zero-filled by the TMA unit
+//   warps 4..11  two groups, alternate stages: a thread owns one weight row: LDS.128 of 32 levels, nibble order chosen so that
+//                (w >> 4s) & 0x000f000f | 0x43004300 IS the bf16 pair (128 + level[k], 128 + level[k+1]), then level - zero and * scale with
+//                get_weight's own bf16 roundings (quantization.py:392-411), so the product sees exactly the matrix the reference's dense
+//                branch multiplies; tcgen05.st into one of four tensor-memory buffers of 32 columns
+//   warp 1       tcgen05.mma.cta_group::1.kind::f16, A from tensor memory, B from shared memory, M 128, N bt, K 16
+//   afterwards the eight dequantising warps are the epilogue: tcgen05.ld, bf16, a warp writes 32 neighbouring features per token.
+//
+// Why this form: with both operands in shared memory a 256 x 256 tile moves 160 bytes per cycle through it (dequantised weights written
+// and read, activations written and read) where 128 fit, and held the tensor pipe at 42 % (4096 x 5120 -> 5120: 291 us on the device);
+// a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice.  With the weight in tensor memory 128 bytes
+// per cycle remain for wide tiles, and a tile's height follows the prompt.  Where tiles are few a cluster of up to 8 CTAs splits K
+// and adds its f32 sums through distributed shared memory in rank order (the result does not depend on timing).
+#include "tc_common.cuh"
 
 namespace b2l {
 namespace q4gm {
 
-// NACC = accumulators = 128-token row groups per CTA: 2 (256 x 256 tile) for large problems; 1 (128 x 256) when the
-// 256-row tiling would leave the last wave of CTAs mostly empty (e.g. N = 5120, M = 4096: 320 tiles on 148 SMs)
-constexpr int BN = 256, BK = 64;
-constexpr int B_BYTES = BN * BK * 2;           // 32 KB: [8 k-columns][256 rows][16 B]
-constexpr int NPROD = 256;                     // producer threads = weight rows of the tile
-constexpr int NTHREADS = 32 + NPROD;
-constexpr int LBO_B = BN * 16;                 // bytes between adjacent 8-k columns of the weight operand
-constexpr int SBO = 128;                       // bytes between adjacent 8-row groups
-template <int NACC> struct Cfg {
-  static constexpr int BM = 128 * NACC;
-  static constexpr int A_BYTES = BM * BK * 2;  // [8 k-columns][BM rows][16 B]
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int NSTAGE = NACC == 2 ? 3 : 4;
-  static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + 256;
-  static constexpr int LBO_A = BM * 16;
-};
+using namespace tc;
+
+constexpr int BN = 128, BK = 64;
+constexpr int W_BYTES = BN * BK / 2;           // packed levels of a stage
+constexpr int NTHREADS = 384, GROUPS = 2;
+constexpr int NA = 4, A_COLS = BK / 2, COL_ACC = NA * A_COLS;      // tensor memory: four weight buffers, then the accumulator
+constexpr int MAX_STAGES = 8;
 
 struct Params {
-  CUtensorMap xmap;        // 3-D view of x (see above); must stay the first member (64-byte alignment)
-  const __nv_bfloat16* x; int ldx;
+  CUtensorMap xmap;        // x as 2-D, boxes of 64 columns x bt rows; must stay the first member (64-byte alignment)
   const uint8_t* qwt;      // b2l_q4_tile layout: [N/128 tiles][K/32 slabs][128 rows][16 B]
   const void* scales; const void* zeros; int szdt;
   __nv_bfloat16* y; int ldy;
-  int M, N, K;
+  int M, N, K, bt, nst, splits;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t a) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
-}
-__device__ __forceinline__ void mbar_wait(uint32_t a, uint32_t parity) {
-  uint32_t ok;
-  do {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-  } while (!ok);
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-// D[tmem] (+)= A[smem desc] * B[smem desc]
-__device__ __forceinline__ void tc_mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// K-major, no-swizzle shared-memory matrix descriptor (sm_100): core matrix = 8 rows x 16 B, contiguous
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;
-  return d;
-}
-// kind::f16: D = f32, A = B = bf16 (K-major), M = 128, N = 256
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t mbar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
-               "l"(map), "r"(mbar), "r"(c0), "r"(c1), "r"(c2)
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+               "r"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
                : "memory");
 }
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t a, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(a), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_dsmem(uint32_t addr, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
 
-template <int NACC>
-__global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_constant__ Params p) {
-  constexpr int BM = Cfg<NACC>::BM, A_BYTES = Cfg<NACC>::A_BYTES, STAGE_BYTES = Cfg<NACC>::STAGE_BYTES, NSTAGE = Cfg<NACC>::NSTAGE;
-  constexpr int LBO_A = Cfg<NACC>::LBO_A;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const uint32_t sbase = smem_u32(smem);
-  const uint32_t bars = sbase + NSTAGE * STAGE_BYTES;      // full[NSTAGE], empty[NSTAGE], accum
-  const uint32_t bar_full = bars, bar_empty = bars + NSTAGE * 8, bar_acc = bars + 2 * NSTAGE * 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + NSTAGE * STAGE_BYTES + (2 * NSTAGE + 1) * 8);
+__global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant__ Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 2 * NA + 1];
+  __shared__ uint32_t tmem_slot;
+  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;            // 128-byte swizzle atoms are 1024-byte aligned
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
-  const int n_kt = p.K / BK;
+  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, a_full = empty + 8 * MAX_STAGES, a_empty = a_full + 8 * NA, acc_done = a_empty + 8 * NA;
+  const uint32_t stage_bytes = W_BYTES + (uint32_t)p.bt * (BK * 2);
+  const int tile_n = blockIdx.x / p.splits, n0 = tile_n * BN, m0 = blockIdx.y * p.bt;
+  const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
+  const int n_kt = p.K / BK, kt_lo = (int)((long long)rank * n_kt / p.splits), kt_hi = (int)((long long)(rank + 1) * n_kt / p.splits);
+  const uint32_t cols = p.bt > 128 ? 512u : 256u;
+  uint32_t dead = 0;
 
   if (tid == 0) {
-    for (int i = 0; i < NSTAGE; ++i) {
-      mbar_init(bar_full + i * 8, NPROD / 32 + 1);   // one elected arrival per producer warp + the TMA issuer's expect_tx
-      mbar_init(bar_empty + i * 8, 1);           // tcgen05.commit
-    }
-    mbar_init(bar_acc, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < p.nst; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 1); }
+    for (int i = 0; i < NA; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, 1); }
+    mbar_init(acc_done, 1);
+    mbar_init_fence();
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(256 * NACC) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
+  if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), cols);
+  fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  fence_after();
+  const uint32_t tmem = tmem_slot;
 
   if (warp == 0) {
-    // ===================== MMA issuer =====================
     if (lane == 0) {
-      for (int kt = 0; kt < n_kt; ++kt) {
-        const int st = kt % NSTAGE;
-        mbar_wait(bar_full + st * 8, (uint32_t)(kt / NSTAGE) & 1u);
-        tc_fence_after();
-        const uint32_t a_base = sbase + st * STAGE_BYTES, b_base = a_base + A_BYTES;
-#pragma unroll
-        for (int j = 0; j < BK / 16; ++j) {
-          const uint64_t bd = make_desc(b_base + j * 2 * LBO_B, LBO_B, SBO);
-          // token rows 0..127 -> accumulator columns 0..255, rows 128..255 -> columns 256..511
-#pragma unroll
-          for (int h = 0; h < NACC; ++h)
-            tc_mma_ss(tmem + 256 * h, make_desc(a_base + h * 128 * 16 + j * 2 * LBO_A, LBO_A, SBO), bd, IDESC, (kt > 0 || j > 0) ? 1u : 0u);
-        }
-        tc_commit(bar_empty + st * 8);   // the stage may be refilled once these MMAs have read it
+      const uint8_t* wsrc = p.qwt + ((size_t)tile_n * (p.K / 32) + (size_t)kt_lo * 2) * 2048;
+      int st = 0;
+      uint32_t ph = 1;                                       // parity of a stage's previous use: passes at once the first time
+      for (int kt = kt_lo; kt < kt_hi; ++kt, wsrc += W_BYTES) {
+        mbar_wait(empty + 8 * st, ph, dead);
+        if (dead) break;
+        const uint32_t base = sbase + st * stage_bytes;
+        mbar_expect_tx(full + 8 * st, stage_bytes);
+        bulk_load(base, wsrc, W_BYTES, full + 8 * st);
+        tma_load_2d(base + W_BYTES, &p.xmap, kt * BK, m0, full + 8 * st);
+        if (++st == p.nst) { st = 0; ph ^= 1u; }
       }
-      tc_commit(bar_acc);                // accumulators complete
     }
-  } else {
-    // ===================== producers: activations (cp.async) + dequantised weights =====================
-    const int pt = tid - 32;                       // 0..255 = weight row of the tile
-    const int row_n = n0 + pt;
-    const int n_slab = p.K / 32;
-    const bool row_ok = row_n < ((p.N + 127) / 128) * 128;     // rows inside the (128-padded) tiling
-    const uint8_t* wrow = p.qwt + ((size_t)(row_n >> 7) * n_slab * 128 + (row_n & 127)) * 16;   // + slab * 2048
+  } else if (warp == 1) {
+    const uint32_t lead = elect_lane();
+    // kind::f16: D = f32, A = B = bf16 (K-major), 128 x bt
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bt >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
+    int st = 0;
+    uint32_t ph = 0, acc = 0;
+    for (int kt = kt_lo, it = 0; kt < kt_hi; ++kt, ++it) {
+      const int ab = it & (NA - 1);
+      mbar_wait(full + 8 * st, ph, dead);
+      mbar_wait(a_full + 8 * ab, (uint32_t)(it / NA) & 1u, dead);
+      if (dead) break;
+      fence_after();
+      const uint64_t bd = desc_sw128(sbase + st * stage_bytes + W_BYTES);
+      const uint32_t ad = tmem + ab * A_COLS;
+#pragma unroll
+      for (int k = 0; k < BK / 16; ++k) mma_ts(tmem + COL_ACC, ad + 8 * k, bd + 2 * k, idesc, k > 0 ? 1u : acc, lead);
+      acc = 1;
+      if (lead) {
+        commit(empty + 8 * st);
+        commit(a_empty + 8 * ab);
+      }
+      __syncwarp();
+      if (++st == p.nst) { st = 0; ph ^= 1u; }
+    }
+    if (lead) commit(acc_done);
+  } else if (warp >= 4) {
+    const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = n0 + row;
+    const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
     float sc_f = 0.f, z_f = 0.f;
-    if (row_n < p.N) { sc_f = load_sz(p.scales, p.szdt, row_n); z_f = load_sz(p.zeros, p.szdt, row_n); }
-    const __nv_bfloat162 sc2 = __float2bfloat162_rn(sc_f), z2 = __float2bfloat162_rn(z_f);
-    const __nv_bfloat162 c128 = __float2bfloat162_rn(128.f);
-    uint4 wq[2];
-    auto load_w = [&](int kt) {
+    if (n < p.N) { sc_f = load_sz(p.scales, p.szdt, n); z_f = load_sz(p.zeros, p.szdt, n); }
+    const __nv_bfloat162 sc2 = __float2bfloat162_rn(sc_f), z2 = __float2bfloat162_rn(z_f), c128 = __float2bfloat162_rn(128.f);
+    int st = grp;
+    uint32_t ph = 0;
+    if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
+    for (int it = grp; it < kt_hi - kt_lo; it += GROUPS) {
+      const int ab = it & (NA - 1);
+      mbar_wait(full + 8 * st, ph, dead);
+      uint32_t w[8];
+      const uint32_t src = sbase + st * stage_bytes + row * 16;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * h]), "=r"(w[4 * h + 1]), "=r"(w[4 * h + 2]), "=r"(w[4 * h + 3]) : "r"(src + h * 2048) : "memory");
+      if (it >= NA) mbar_wait(a_empty + 8 * ab, (uint32_t)(it / NA - 1) & 1u, dead);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        wq[h] = make_uint4(0, 0, 0, 0);
-        if (row_ok) wq[h] = __ldg(reinterpret_cast<const uint4*>(wrow + (size_t)(kt * 2 + h) * 2048));
-      }
-    };
-    load_w(0);
-    for (int kt = 0; kt < n_kt; ++kt) {
-      const int st = kt % NSTAGE;
-      if (kt >= NSTAGE) mbar_wait(bar_empty + st * 8, (uint32_t)(kt / NSTAGE - 1) & 1u);
-      const uint32_t a_base = sbase + st * STAGE_BYTES, b_base = a_base + A_BYTES;
-      // ---- activations: one tensor-map TMA copy of the whole [8 k chunks][256 rows][16 B] tile
-      if (pt == 0) {
-        mbar_expect_tx(bar_full + st * 8, A_BYTES);
-        tma_load_3d(a_base, &p.xmap, 0, m0, kt * (BK / 8), bar_full + st * 8);
-      }
-      // ---- weights of this stage (loaded one stage ahead), then the next stage's loads
-      const uint4 w0 = wq[0], w1 = wq[1];
-      if (kt + 1 < n_kt) load_w(kt + 1);
-      const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        uint32_t o[16];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {       // word c = 8 consecutive k = one 16-byte core-matrix row
-        uint32_t o[4];
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const uint32_t v = ((ww[c] >> (4 * s)) & 0x000f000fu) | 0x43004300u;          // (128 + level) pair, exact
-          __nv_bfloat162 t = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), c128);   // level, exact
-          t = __hmul2(__hsub2(t, z2), sc2);      // (level - zero) * scale with the reference's bf16 roundings
-          o[s] = *reinterpret_cast<const uint32_t*>(&t);
-        }
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(b_base + c * LBO_B + pt * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_full + st * 8);
-    }
-    // ===================== epilogue: TMEM -> bf16 -> y =====================
-    mbar_wait(bar_acc, 0);
-    tc_fence_after();
-    const int quarter = warp & 3;                 // TMEM lanes 32 * quarter .. + 31 are reachable from this warp
-    // two accumulators: warps 1..4 drain accumulator 0 (tokens 0..127), warps 5..8 accumulator 1, all 256 columns each;
-    // one accumulator: warps 1..4 drain columns 0..127, warps 5..8 columns 128..255
-    const int grp = (warp - 1) >> 2;
-    const int chalf = NACC == 2 ? grp : 0;
-    const int cb_lo = NACC == 2 ? 0 : grp * (BN / 32), cb_hi = NACC == 2 ? BN / 16 : cb_lo + BN / 32;
-    const int m = m0 + chalf * 128 + quarter * 32 + lane;
-#pragma unroll 1
-    for (int cb = cb_lo; cb < cb_hi; ++cb) {
-      uint32_t r[16];
-      tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(chalf * 256 + cb * 16), r);
-      if (m < p.M) {
-        const int n = n0 + cb * 16;
-        __nv_bfloat16* dst = p.y + (size_t)m * p.ldy + n;
-        if (n + 16 <= p.N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-          uint32_t o[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const __nv_bfloat162 t = __floats2bfloat162_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-            o[i] = *reinterpret_cast<const uint32_t*>(&t);
+          for (int s = 0; s < 4; ++s) {
+            const uint32_t v = ((w[4 * h + c] >> (4 * s)) & 0x000f000fu) | 0x43004300u;      // (128 + level) pair, exact
+            __nv_bfloat162 t = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), c128);     // level, exact
+            t = __hmul2(__hsub2(t, z2), sc2);                                                 // the reference's bf16 roundings
+            o[4 * c + s] = *reinterpret_cast<const uint32_t*>(&t);
           }
-          reinterpret_cast<uint4*>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
-          reinterpret_cast<uint4*>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
-        } else {
+        tmem_st16(tmem + lane_at + ab * A_COLS + 16 * h, o);
+      }
+      tmem_wait_st();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(a_full + 8 * ab);
+      st += GROUPS;
+      if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
+    }
+    mbar_wait(acc_done, 0, dead);
+    fence_after();
+  }
+  __syncwarp();
+  // ---- epilogue: a thread owns weight row n, 16 tokens at a time, the two groups in turn; split K: a token group is summed by one CTA
+  const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = n0 + row, nb = p.bt / 16;
+  const uint32_t acc_at = tmem + ((uint32_t)(qtr * 32) << 16) + COL_ACC;
+  if (p.splits > 1) {
+    // stage memory is free (every MMA has completed): f32 [token group][128 rows][16 tokens], the 16-byte pieces of a row rotated
+    if (warp >= 4) {
+      for (int b = grp; b < nb; b += GROUPS) {
+        uint32_t r[16];
+        tmem_ld16(acc_at + 16 * b, r);
+        const uint32_t dst = sbase + (uint32_t)(b * BN + row) * 64;
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (n + i < p.N) dst[i] = f2bf(__uint_as_float(r[i]));
+        for (int c = 0; c < 4; ++c)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16 * ((c + (row >> 1)) & 3)), "r"(r[4 * c]), "r"(r[4 * c + 1]), "r"(r[4 * c + 2]), "r"(r[4 * c + 3]) : "memory");
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+  }
+  if (warp >= 4) {
+    for (int b = (int)rank + grp * p.splits; b < nb; b += GROUPS * p.splits) {
+      __syncwarp();
+      float v[16];
+      if (p.splits == 1) {
+        uint32_t r[16];
+        tmem_ld16(acc_at + 16 * b, r);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+        for (int s = 0; s < p.splits; ++s) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float4 u = ld_dsmem(sbase + (uint32_t)(b * BN + row) * 64 + 16 * ((c + (row >> 1)) & 3), (uint32_t)s);
+            v[4 * c] += u.x; v[4 * c + 1] += u.y; v[4 * c + 2] += u.z; v[4 * c + 3] += u.w;
+          }
         }
+      }
+      const int m = m0 + 16 * b;
+      if (n < p.N) {
+        __nv_bfloat16* dst = p.y + (size_t)m * p.ldy + n;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (m + i < p.M) dst[(size_t)i * p.ldy] = f2bf(dead ? __int_as_float(0x7fc00000) : v[i]);
       }
     }
   }
-  tc_fence_before();
+  __syncwarp();
+  if (p.splits > 1) cluster_sync_all();              // nobody leaves while a peer reads its partial sums
+  fence_before();
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(256 * NACC) : "memory");
+  if (warp == 1) tmem_dealloc(tmem, cols);
+}
+
+struct Plan { int bt, m_tiles, splits, nst; size_t smem; };
+// Tile height and K split by a model of the time in tensor cycles: rounds of CTAs over the SMs times (stages of max(2 bt, the 200 a stage's
+// dequantisation takes) + a fixed part: first copies, epilogue, and the sums of a split).
+static Plan plan_for(int M, int N, int K) {
+  const int sms = sm_count(), n_tiles = (N + BN - 1) / BN, n_kt = K / BK;
+  Plan best{};
+  long long best_cost = -1;
+  const int least = (M + 255) / 256;
+  for (int mt = least; mt <= least + 3; ++mt) {
+    const int bt = ((M + mt - 1) / mt + 15) / 16 * 16, tiles = (M + bt - 1) / bt;
+    for (int sp = 1; sp <= 8; ++sp) {
+      if (sp > 1 && n_kt / sp < 8) break;
+      const long long ctas = (long long)n_tiles * tiles * sp, rounds = (ctas + sms - 1) / sms;
+      const long long stages = (n_kt + sp - 1) / sp, per = bt * 2 > 200 ? bt * 2 : 200;
+      const long long cost = rounds * (stages * per + 3000 + 8 * bt + (sp > 1 ? 1500 + 10 * bt : 0));
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best.bt = bt; best.m_tiles = tiles; best.splits = sp;
+      }
+    }
+  }
+  const size_t stage = W_BYTES + (size_t)best.bt * BK * 2;
+  const size_t budget = best.bt <= 128 ? 110 * 1024 : 216 * 1024;       // two CTAs per SM where tensor memory allows it
+  best.nst = (int)(budget / stage);
+  if (best.nst > MAX_STAGES) best.nst = MAX_STAGES;
+  best.smem = best.nst * stage + 1024;
+  const size_t part = (size_t)BN * best.bt * 4 + 1024;
+  if (best.splits > 1 && part > best.smem) best.smem = part;
+  return best;
 }
 
 }  // namespace q4gm
@@ -276,54 +281,16 @@ extern "C" int b2l_q4_gemm(const b2l_q4_linear_args* a, b2l_stream_t stream) {
   B2L_CHECK_ARG(((uintptr_t)a->x % 16 == 0) && ((uintptr_t)a->qw_tiled % 16 == 0), "b2l_q4_gemm: x / qw_tiled must be 16-byte aligned");
   B2L_CHECK_ARG(a->sz_dtype == B2L_BF16 || a->sz_dtype == B2L_F32, "b2l_q4_gemm: bad sz_dtype");
   B2L_CHECK_SUPPORTED(a->prologue == B2L_PRO_NONE && a->epilogue == B2L_EPI_STORE, "b2l_q4_gemm: plain linear only (no fused prologue / epilogue)");
-  // cuTensorMapEncodeTiled through the runtime (resolved once)
-  typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) fn = nullptr;
-    return (EncodeFn)fn;
-  }();
-  if (encode == nullptr) {
-    set_error("b2l_q4_gemm: cuTensorMapEncodeTiled is not available from this driver");
-    return B2L_E_STATE;
-  }
-  // tile height: 256 token rows unless that tiling would fill the last wave of CTAs less than half (then 128)
-  const long tiles256 = (long)((a->N + BN - 1) / BN) * ((a->M + 255) / 256);
-  const int sms = sm_count();
-  static const int env_nacc = [] { const char* e = getenv("B2L_GEMM_NACC"); return e ? atoi(e) : 0; }();
-  int nacc = (a->M <= 128 || (tiles256 % sms != 0 && tiles256 % sms < sms / 2 && tiles256 < 4 * sms)) ? 1 : 2;
-  if (env_nacc == 1 || env_nacc == 2) nacc = env_nacc;
+  const Plan q = plan_for(a->M, a->N, a->K);
   Params p;
-  {
-    // x[M, K] (leading dimension ldx) as (8 elements | M rows | K/8 chunks): a box of 8 x 256 x 8 is one stage's tile
-    const cuuint64_t dims[3] = {8, (cuuint64_t)a->M, (cuuint64_t)(a->K / 8)};
-    const cuuint64_t strides[2] = {(cuuint64_t)a->ldx * 2, 16};
-    const cuuint32_t box[3] = {8, (cuuint32_t)(128 * nacc), (cuuint32_t)(BK / 8)};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult cr = encode(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(a->x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) {
-      set_error("b2l_q4_gemm: cuTensorMapEncodeTiled failed (%d) for M=%d K=%d ldx=%d", (int)cr, a->M, a->K, a->ldx);
-      return B2L_E_ARG;
-    }
-  }
-  p.x = (const __nv_bfloat16*)a->x; p.ldx = a->ldx;
+  if (int rc = map_sw128(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->x, a->M, a->K, a->ldx, BK, q.bt)) return rc;
   p.qwt = (const uint8_t*)a->qw_tiled;
   p.scales = a->scales; p.zeros = a->zeros; p.szdt = a->sz_dtype;
   p.y = (__nv_bfloat16*)a->y; p.ldy = a->ldy;
-  p.M = a->M; p.N = a->N; p.K = a->K;
-  static DynSmemCache smem_cache[2];
-  if (nacc == 2) {
-    if (int rc = ensure_dyn_smem(q4_gemm_kernel<2>, Cfg<2>::SMEM_BYTES, smem_cache[1])) return rc;
-    dim3 grid((a->N + BN - 1) / BN, (a->M + 255) / 256);
-    q4_gemm_kernel<2><<<grid, NTHREADS, Cfg<2>::SMEM_BYTES, (cudaStream_t)stream>>>(p);
-  } else {
-    if (int rc = ensure_dyn_smem(q4_gemm_kernel<1>, Cfg<1>::SMEM_BYTES, smem_cache[0])) return rc;
-    dim3 grid((a->N + BN - 1) / BN, (a->M + 127) / 128);
-    q4_gemm_kernel<1><<<grid, NTHREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(p);
-  }
-  B2L_LAUNCH_CHECK("q4_gemm_kernel");
+  p.M = a->M; p.N = a->N; p.K = a->K; p.bt = q.bt; p.nst = q.nst; p.splits = q.splits;
+  static DynSmemCache smem_cache;
+  if (int rc = ensure_dyn_smem(q4_gemm_kernel, q.smem, smem_cache)) return rc;
+  LaunchCfg lc(dim3((unsigned)((a->N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, (cudaStream_t)stream, false, q.splits);
+  B2L_CUDA(cudaLaunchKernelEx(&lc.cfg, q4_gemm_kernel, p));
   return 0;
 }
