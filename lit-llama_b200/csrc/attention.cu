@@ -7,7 +7,7 @@
 // does once per layer per token, model.py:214).
 #include <cstdlib>
 
-#include "b2l_common.cuh"
+#include "attn_tc.cuh"
 
 namespace b2l {
 
@@ -755,6 +755,110 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// ----------------------------------------------------------------------------------
+// Longer prompts: the tcgen05 kernel of attn_tc.cuh, 128 query rows of one head per CTA, q in one bf16 part (it is bf16), the weights in three.
+// grid (B * n_head, row tiles), the tiles with the most keys first.  Tiles of 64 slots that neither wrap in the ring nor end early come by
+// tiled TMA copies from the cache (or from qkv without one).
+// ----------------------------------------------------------------------------------
+struct PromptProb {
+  CUtensorMap map_a, map_b, map_v;
+  const __nv_bfloat16* qkv;
+  KvView kv;
+  const int64_t* input_pos;
+  const int32_t* ring_start;
+  __nv_bfloat16* y;
+  int T, n_head, cached;
+  int DK, DV, stages, split8, q_tmem;
+  float scale, softcap;
+  struct Tile {
+    int b, h, t_first, rows, j_begin, j_end, cap, ring, xa, xb, xv;
+    const __nv_bfloat16 *k, *v;
+  };
+  struct Row { const __nv_bfloat16 *ka, *kb, *v; };
+  __device__ __forceinline__ int slots(int t, int cap) const {       // visible slots of query t: 0 .. its position, or all of a full cache
+    const long long p = input_pos ? input_pos[t] : (long long)t;
+    return (int)(p < cap ? p : (long long)cap - 1) + 1;
+  }
+  __device__ __forceinline__ Tile tile() const {
+    Tile t;
+    t.b = blockIdx.x / n_head;
+    t.h = blockIdx.x - t.b * n_head;
+    t.t_first = ((int)gridDim.y - 1 - (int)blockIdx.y) * atc::ROWS;
+    t.rows = min(atc::ROWS, T - t.t_first);
+    t.cap = kv.S > 0 ? kv.S : T;
+    t.ring = (kv.S > 0 && ring_start) ? *ring_start : 0;
+    t.j_begin = 0;
+    float most = 0.f;                                                // the most slots a row of the tile sees (below 2^24: exact)
+    for (int i = threadIdx.x & 31; i < t.rows; i += 32) most = fmaxf(most, (float)slots(t.t_first + i, t.cap));
+    t.j_end = (int)warp_max(most);
+    t.k = kv.k + (size_t)t.b * kv.b_stride + (size_t)t.h * kv.h_stride;
+    t.v = kv.v + (size_t)t.b * kv.b_stride + (size_t)t.h * kv.h_stride;
+    t.xa = cached ? 0 : (n_head + t.h) * 128;
+    t.xv = cached ? 0 : (2 * n_head + t.h) * 128;
+    t.xb = 0;
+    return t;
+  }
+  __device__ __forceinline__ Row row(const Tile& t, int j) const {
+    if (kv.S > 0) { j += t.ring; if (j >= kv.S) j -= kv.S; }
+    Row r;
+    r.ka = t.k + (size_t)j * kv.s_stride;
+    r.kb = nullptr;
+    r.v = t.v + (size_t)j * kv.s_stride;
+    return r;
+  }
+  __device__ __forceinline__ bool bulk(const Tile& t, int j0, int& ra, int& rb, int& rv) const {
+    int p = j0 + t.ring;
+    if (p >= t.cap) p -= t.cap;
+    ra = rv = cached ? (t.b * n_head + t.h) * kv.S + p : t.b * T + j0;
+    rb = 0;
+    return j0 + atc::KEYS <= t.j_end && p + atc::KEYS <= t.cap;
+  }
+  __device__ __forceinline__ void query(const Tile& t, int r, int c, float (&x)[8]) const {
+    const uint4 u = *reinterpret_cast<const uint4*>(qkv + ((size_t)t.b * T + t.t_first + r) * 3 * n_head * 128 + (size_t)t.h * 128 + 8 * c);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[2 * i] = __uint_as_float(w[i] << 16);
+      x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+  __device__ __forceinline__ void range(const Tile& t, int r, int& lo, int& hi) const {
+    lo = 0;
+    hi = r < t.rows ? slots(t.t_first + r, t.cap) - 1 : -1;
+  }
+  __device__ __forceinline__ float sink(const Tile&) const { return -INFINITY; }
+  __device__ __forceinline__ bool partial(const Tile&) const { return false; }
+  __device__ __forceinline__ void store_ml(const Tile&, int, float, float) const {}
+  __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[16]) const {}
+  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
+    uint4* o = reinterpret_cast<uint4*>(y + ((size_t)t.b * T + t.t_first + r) * n_head * 128 + (size_t)t.h * 128 + c0);
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+};
+
+static int launch_prompt_tc(const __nv_bfloat16* qkv, const KvView& kv, const int64_t* input_pos, const int32_t* ring_start, __nv_bfloat16* y, int B, int T,
+                            int n_head, int S, cudaStream_t st) {
+  const atc::Layout l = atc::layout(1, 128, 128);
+  PromptProb p;
+  p.qkv = qkv; p.kv = kv; p.input_pos = input_pos; p.ring_start = ring_start; p.y = y;
+  p.T = T; p.n_head = n_head; p.cached = kv.S > 0;
+  p.DK = p.DV = 128; p.stages = l.stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = 1.0f / sqrtf(128.f); p.softcap = 0.f;
+  const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const long long rows = p.cached ? (long long)B * n_head * S : (long long)B * T, cols = p.cached ? 128 : 3LL * n_head * 128;
+  if (int rc = tc::map_sw128(&p.map_a, bf, 2, p.cached ? kv.k : qkv, rows, cols, cols, 64, atc::KEYS)) return rc;
+  if (int rc = tc::map_sw128(&p.map_v, bf, 2, p.cached ? kv.v : qkv, rows, cols, cols, 64, atc::KEYS)) return rc;
+  p.map_b = p.map_a;
+  static DynSmemCache smem_cache;
+  return atc::launch<PromptProb, 1, 3, false>(p, dim3((unsigned)(B * n_head), (unsigned)((T + atc::ROWS - 1) / atc::ROWS)), l.smem, smem_cache, st);
+}
+
 // debug timeline slot for the next fused-attention launch (set by b2l_decode_step; nullptr = off)
 void* g_attn_timeline = nullptr;
 
@@ -767,6 +871,9 @@ static inline void split_plan(int T, int S, int* n_split, int* chunk) {
 static int launch_attn(const __nv_bfloat16* qkv, KvView kv, const int64_t* input_pos, const int32_t* ring_start,
                        float* work, __nv_bfloat16* y, int B, int T, int n_head, int hs, int cap, cudaStream_t st) {
   static const int env_pf = [] { const char* e = getenv("B2L_ATTN_PREFILL"); return e ? atoi(e) : 1; }();
+  const bool al = (((uintptr_t)qkv | (uintptr_t)kv.k | (uintptr_t)kv.v | (uintptr_t)y) & 15) == 0;
+  if (hs == 128 && T >= 64 && env_pf && al && (T + 127) / 128 <= 65535)      // shorter prompts fill less than half of a 128-row tile
+    return launch_prompt_tc(qkv, kv, input_pos, ring_start, y, B, T, n_head, kv.S, st);
   if (hs == 128 && T > 1 && env_pf) {   // tiled tensor-core kernel (B2L_ATTN_PREFILL=0: the per-query path below)
     static DynSmemCache smem_cache;
     if (int rc = ensure_dyn_smem(attn_prefill_kernel, PF_SMEM_BYTES, smem_cache)) return rc;

@@ -269,32 +269,43 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     // ===================== queries, softmax, output =====================
     const int qtr = warp & 3, b = (warp >> 2) - 1, r = qtr * 32 + lane;      // b: the parity of the group's tiles
     const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
-    for (int g = b; g < pr.DK / 16; g += 2) {                // the groups take turns with 16 entries of a row
-      float x[16];
+    for (int g0 = b; g0 < pr.DK / 16; g0 += 8) {             // the groups take turns with 16 entries of a row; four turns' loads together
+      float x[4][16];
 #pragma unroll
-      for (int e = 0; e < 16; ++e) x[e] = 0.f;
-      if (r < tl.rows) {
-        pr.query(tl, r, 2 * g, *reinterpret_cast<float (*)[8]>(x));
-        pr.query(tl, r, 2 * g + 1, *reinterpret_cast<float (*)[8]>(x + 8));
+      for (int u = 0; u < 4; ++u) {
+        const int g = g0 + 2 * u;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[u][e] = 0.f;
+        if (r < tl.rows && g < pr.DK / 16) {
+          pr.query(tl, r, 2 * g, *reinterpret_cast<float (*)[8]>(x[u]));
+          pr.query(tl, r, 2 * g + 1, *reinterpret_cast<float (*)[8]>(x[u] + 8));
+        }
       }
       __syncwarp();
 #pragma unroll
-      for (int s = 0; s < NQ; ++s) {
-        uint32_t w[8];
+      for (int u = 0; u < 4; ++u) {
+        const int g = g0 + 2 * u;
+        if (g >= pr.DK / 16) break;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = hi_pair(x[2 * e], x[2 * e + 1]);
-        if (s >= nsm) {
-          tmem_st8(tmem + lane_at + COL_Q + (s - nsm) * (pr.DK / 2) + 8 * g, w);
-        } else {
+        for (int s = 0; s < NQ; ++s) {
+          uint32_t w[8];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int c = 2 * g + h;
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sq + (s * ka + (c >> 3)) * Q_ATOM + r * 128 + (((c & 7) ^ (r & 7)) << 4)), "r"(w[4 * h]),
-                         "r"(w[4 * h + 1]), "r"(w[4 * h + 2]), "r"(w[4 * h + 3]) : "memory");
+          for (int e = 0; e < 8; ++e) w[e] = hi_pair(x[u][2 * e], x[u][2 * e + 1]);
+          if (s >= nsm) {
+            tmem_st8(tmem + lane_at + COL_Q + (s - nsm) * (pr.DK / 2) + 8 * g, w);
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int c = 2 * g + h;
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sq + (s * ka + (c >> 3)) * Q_ATOM + r * 128 + (((c & 7) ^ (r & 7)) << 4)), "r"(w[4 * h]),
+                           "r"(w[4 * h + 1]), "r"(w[4 * h + 2]), "r"(w[4 * h + 3]) : "memory");
+            }
+          }
+          if (s + 1 < NQ) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) x[u][e] = fabsf(x[u][e]) < INFINITY ? rest(x[u][e]) : 0.f;
           }
         }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) x[e] = fabsf(x[e]) < INFINITY ? rest(x[e]) : 0.f;
       }
     }
     tmem_wait_st();

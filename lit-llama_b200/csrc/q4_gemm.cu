@@ -7,18 +7,19 @@
 // A CTA computes 128 output features x `bt` tokens (16..256), the WEIGHT as the 128-row operand in tensor memory:
 //   warp 0       TMA: per 64-wide k stage the 4 KB of packed levels (load-time tiling b2l_q4_tile: contiguous) and the activation tile
 //                [bt tokens][64 k] as one 128-byte swizzled box, on one mbarrier; rows beyond M are zero-filled by the TMA unit
-//   warps 4..11  two groups, alternate stages: a thread owns one weight row: LDS.128 of 32 levels, nibble order chosen so that
+//   warps 4..19  four groups, a stage each in turn: a thread owns one weight row: LDS.128 of 32 levels, nibble order chosen so that
 //                (w >> 4s) & 0x000f000f | 0x43004300 IS the bf16 pair (128 + level[k], 128 + level[k+1]), then level - zero and * scale with
 //                get_weight's own bf16 roundings (quantization.py:392-411), so the product sees exactly the matrix the reference's dense
-//                branch multiplies; tcgen05.st into one of four tensor-memory buffers of 32 columns
+//                branch multiplies; tcgen05.st into the stage's 32 columns
 //   warp 1       tcgen05.mma.cta_group::1.kind::f16, A from tensor memory, B from shared memory, M 128, N bt, K 16
-//   afterwards the eight dequantising warps are the epilogue: tcgen05.ld, bf16, a warp writes 32 neighbouring features per token.
+//   afterwards the dequantising warps are the epilogue: tcgen05.ld, bf16, a warp writes 32 neighbouring features per token.
 //
 // Why this form: with both operands in shared memory a 256 x 256 tile moves 160 bytes per cycle through it (dequantised weights written
-// and read, activations written and read) where 128 fit, and held the tensor pipe at 42 % (4096 x 5120 -> 5120: 291 us on the device);
-// a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice.  With the weight in tensor memory 128 bytes
-// per cycle remain for wide tiles, and a tile's height follows the prompt.  Where tiles are few a cluster of up to 8 CTAs splits K
-// and adds its f32 sums through distributed shared memory in rank order (the result does not depend on timing).
+// and read, activations written and read) where 128 fit, and held the tensor pipe at 42 % (4096 x 5120 -> 5120: 291 us on the device,
+// now 153); a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice (4096 -> 11008: 45 us, now 28).
+// What bounds it now is L2: a stage of bt = 240 brings 35 KB to the SM in some 750 cycles (480 of them the tensor pipe's).  Where tiles
+// are few a cluster of up to 8 CTAs splits K and adds its f32 sums through distributed shared memory in rank order (the result does not
+// depend on timing).
 #include "tc_common.cuh"
 
 namespace b2l {
@@ -28,9 +29,9 @@ using namespace tc;
 
 constexpr int BN = 128, BK = 64;
 constexpr int W_BYTES = BN * BK / 2;           // packed levels of a stage
-constexpr int NTHREADS = 384, GROUPS = 2;
-constexpr int NA = 4, A_COLS = BK / 2, COL_ACC = NA * A_COLS;      // tensor memory: four weight buffers, then the accumulator
-constexpr int MAX_STAGES = 8;
+constexpr int GROUPS = 4, NTHREADS = 128 + 128 * GROUPS;
+constexpr int MAX_STAGES = 8, A_COLS = BK / 2;      // a stage owns a weight buffer of 32 tensor-memory columns; the accumulator follows from COL_ACC on
+constexpr int COL_ACC = 512 - 256;
 
 struct Params {
   CUtensorMap xmap;        // x as 2-D, boxes of 64 columns x bt rows; must stay the first member (64-byte alignment)
@@ -72,27 +73,25 @@ __device__ __forceinline__ float4 ld_dsmem(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-__global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 2 * NA + 1];
+  __shared__ __align__(8) uint64_t bars[3 * MAX_STAGES + 1];
   __shared__ uint32_t tmem_slot;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;            // 128-byte swizzle atoms are 1024-byte aligned
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, a_full = empty + 8 * MAX_STAGES, a_empty = a_full + 8 * NA, acc_done = a_empty + 8 * NA;
+  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, a_full = empty + 8 * MAX_STAGES, acc_done = a_full + 8 * MAX_STAGES;
   const uint32_t stage_bytes = W_BYTES + (uint32_t)p.bt * (BK * 2);
   const int tile_n = blockIdx.x / p.splits, n0 = tile_n * BN, m0 = blockIdx.y * p.bt;
   const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
   const int n_kt = p.K / BK, kt_lo = (int)((long long)rank * n_kt / p.splits), kt_hi = (int)((long long)(rank + 1) * n_kt / p.splits);
-  const uint32_t cols = p.bt > 128 ? 512u : 256u;
   uint32_t dead = 0;
 
   if (tid == 0) {
-    for (int i = 0; i < p.nst; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 1); }
-    for (int i = 0; i < NA; ++i) { mbar_init(a_full + 8 * i, 4); mbar_init(a_empty + 8 * i, 1); }
+    for (int i = 0; i < p.nst; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 1); mbar_init(a_full + 8 * i, 4); }
     mbar_init(acc_done, 1);
     mbar_init_fence();
   }
-  if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), cols);
+  if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), 512);
   fence_before();
   __syncthreads();
   fence_after();
@@ -119,21 +118,17 @@ __global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bt >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
     int st = 0;
     uint32_t ph = 0, acc = 0;
-    for (int kt = kt_lo, it = 0; kt < kt_hi; ++kt, ++it) {
-      const int ab = it & (NA - 1);
+    for (int kt = kt_lo; kt < kt_hi; ++kt) {
       mbar_wait(full + 8 * st, ph, dead);
-      mbar_wait(a_full + 8 * ab, (uint32_t)(it / NA) & 1u, dead);
+      mbar_wait(a_full + 8 * st, ph, dead);
       if (dead) break;
       fence_after();
       const uint64_t bd = desc_sw128(sbase + st * stage_bytes + W_BYTES);
-      const uint32_t ad = tmem + ab * A_COLS;
+      const uint32_t ad = tmem + st * A_COLS;
 #pragma unroll
       for (int k = 0; k < BK / 16; ++k) mma_ts(tmem + COL_ACC, ad + 8 * k, bd + 2 * k, idesc, k > 0 ? 1u : acc, lead);
       acc = 1;
-      if (lead) {
-        commit(empty + 8 * st);
-        commit(a_empty + 8 * ab);
-      }
+      if (lead) commit(empty + 8 * st);                      // one per stage: it frees both halves, and each holds the pipe up for 100 cycles
       __syncwarp();
       if (++st == p.nst) { st = 0; ph ^= 1u; }
     }
@@ -148,14 +143,13 @@ __global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant
     uint32_t ph = 0;
     if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
     for (int it = grp; it < kt_hi - kt_lo; it += GROUPS) {
-      const int ab = it & (NA - 1);
-      mbar_wait(full + 8 * st, ph, dead);
+      mbar_wait(full + 8 * st, ph, dead);                    // also: the MMAs of the stage's previous use are done
       uint32_t w[8];
       const uint32_t src = sbase + st * stage_bytes + row * 16;
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * h]), "=r"(w[4 * h + 1]), "=r"(w[4 * h + 2]), "=r"(w[4 * h + 3]) : "r"(src + h * 2048) : "memory");
-      if (it >= NA) mbar_wait(a_empty + 8 * ab, (uint32_t)(it / NA - 1) & 1u, dead);
+      fence_after();
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t o[16];
@@ -168,12 +162,12 @@ __global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant
             t = __hmul2(__hsub2(t, z2), sc2);                                                 // the reference's bf16 roundings
             o[4 * c + s] = *reinterpret_cast<const uint32_t*>(&t);
           }
-        tmem_st16(tmem + lane_at + ab * A_COLS + 16 * h, o);
+        tmem_st16(tmem + lane_at + st * A_COLS + 16 * h, o);
       }
       tmem_wait_st();
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(a_full + 8 * ab);
+      if (lane == 0) mbar_arrive(a_full + 8 * st);
       st += GROUPS;
       if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
     }
@@ -181,7 +175,7 @@ __global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant
     fence_after();
   }
   __syncwarp();
-  // ---- epilogue: a thread owns weight row n, 16 tokens at a time, the two groups in turn; split K: a token group is summed by one CTA
+  // ---- epilogue: a thread owns weight row n, 16 tokens at a time, the groups in turn; split K: a token group is summed by one CTA
   const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = n0 + row, nb = p.bt / 16;
   const uint32_t acc_at = tmem + ((uint32_t)(qtr * 32) << 16) + COL_ACC;
   if (p.splits > 1) {
@@ -232,7 +226,7 @@ __global__ void __launch_bounds__(NTHREADS) q4_gemm_kernel(const __grid_constant
   if (p.splits > 1) cluster_sync_all();              // nobody leaves while a peer reads its partial sums
   fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, cols);
+  if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 struct Plan { int bt, m_tiles, splits, nst; size_t smem; };
@@ -257,8 +251,7 @@ static Plan plan_for(int M, int N, int K) {
     }
   }
   const size_t stage = W_BYTES + (size_t)best.bt * BK * 2;
-  const size_t budget = best.bt <= 128 ? 110 * 1024 : 216 * 1024;       // two CTAs per SM where tensor memory allows it
-  best.nst = (int)(budget / stage);
+  best.nst = (int)(216 * 1024 / stage);
   if (best.nst > MAX_STAGES) best.nst = MAX_STAGES;
   best.smem = best.nst * stage + 1024;
   const size_t part = (size_t)BN * best.bt * 4 + 1024;
