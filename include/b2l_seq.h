@@ -127,6 +127,9 @@ typedef struct {
   int ones; float* state_ones; float* out_ones;
 } b2l_seq_scan_args;
 int b2l_seq_scan_chunks(int T, int delta);
+/* Floats of work_state with which a delta-rule portion (n_chunks 1) runs in chunks of 16 tokens where its sizes allow it; 0: step by step,
+ * as with work_state null. */
+long long b2l_seq_scan_delta_work_floats(int T, int heads);
 int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream);
 
 /* Read-out of a recurrence: groups of `group` consecutive channels of o (f32 [T, n]) are divided by their root
