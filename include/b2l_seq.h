@@ -127,9 +127,9 @@ typedef struct {
   int ones; float* state_ones; float* out_ones;
 } b2l_seq_scan_args;
 int b2l_seq_scan_chunks(int T, int delta);
-/* Floats of work_state with which a delta-rule portion (n_chunks 1) runs in chunks of 16 tokens where its sizes allow it; 0: step by step,
- * as with work_state null. */
-long long b2l_seq_scan_delta_work_floats(int T, int heads);
+/* Floats of work_state with which a portion with n_chunks <= 1 runs 16 tokens at a time where its sizes allow it (0: too short); step by step
+ * with work_state null.  The space of a portion with n_chunks > 1 serves as well where it is as large. */
+long long b2l_seq_scan_work_floats(int T, int heads);
 int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream);
 
 /* Read-out of a recurrence: groups of `group` consecutive channels of o (f32 [T, n]) are divided by their root

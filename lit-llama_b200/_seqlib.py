@@ -150,7 +150,7 @@ _SIGS = {
                               c_void_p]),
     "b2l_seq_scan": (c_int, [C.POINTER(ScanArgs), c_void_p]),
     "b2l_seq_scan_chunks": (c_int, [c_int, c_int]),
-    "b2l_seq_scan_delta_work_floats": (C.c_longlong, [c_int, c_int]),
+    "b2l_seq_scan_work_floats": (C.c_longlong, [c_int, c_int]),
     "b2l_seq_group_norm_gate": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p,
                                         c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "b2l_seq_headnorm_rope": (c_int, [c_void_p, c_int, c_void_p, c_float, c_void_p, c_int, c_float, c_void_p, c_void_p, c_int, c_int,

@@ -325,63 +325,114 @@ __global__ void seq_scan_combine_kernel(b2l_seq_scan_args a) {
   *st = s;
 }
 
-// ---- the delta rule over a portion, 16 tokens at a time.  With G_t the product of the decays of a chunk's tokens up to t (per channel) and
-// D_(t,i) that of the tokens after i up to t, and S_0 the state before the chunk:
-//   P_t = S_0^T (G_t k_t), R_t = S_0^T (G_t q_t);   u = T (v - P),  T = (I + diag(beta) tril(A,-1))^-1 diag(beta),  A[t,i] = k_t . D_(t,i) k_i
-//   o = R + tril(B) u = R + (tril(B) T) (v - P),  B[t,i] = q_t . D_(t,i) k_i;   S_16 = G_16 S_0 + sum_i (D_(16,i) k_i) u_i^T
+// ---- a portion 16 tokens at a time.  With G_t the product of the decays of a chunk's tokens up to t (per channel) and D_(t,i) that of the
+// tokens after i up to t, S_0 the state before the chunk, B[t,i] = q_t . D_(t,i) k_i for i <= t, R_t = S_0^T (G_t q_t):
+//   without the delta rule:  u_i = vscale_i v_i;  o = R + B u
+//   delta rule:  P_t = S_0^T (G_t k_t);  u = T (v - P),  T = (I + diag(beta) A)^-1 diag(beta),  A[t,i] = k_t . D_(t,i) k_i for i < t;
+//                o = R + (B T) (v - P)
+//   S_16 = G_16 S_0 + sum_i (D_(16,i) k_i) u_i^T
 // Decays only ever multiply (no quotient of cumulative products, which overflows where a channel forgets fast).  T is the product of the
 // chunk's transition matrices seen from k: its entries stay below 1 for unit keys.  All f32 on the CUDA cores, like the step-by-step form.
-//   seq_delta_chunk_kernel  a CTA per (chunk, head): T and tril(B) T, 16 x 16 each, into the workspace; all chunks in parallel
-//   seq_delta_scan_kernel   a CTA per (head, 16 value columns) walks the chunks: warps 4..7 (a thread per key channel) form G k, G q, D k of the
-//                           next chunk while warps 0..3 run P / R (K split over the warps, 4 x 4 tiles), u / o, and the state update
-// What bounds it: the walk over T / 16 chunks, 832 FMA cycles per chunk plus four barriers.  The step-by-step kernel spends 0.38 us per token on
-// one dependent chain of FMAs and shuffles, whatever the width.
-constexpr int DL_C = 16, DL_VT = 16, DL_KT = 36;      // tokens per chunk, value columns per CTA, padded row of the transposed operands
+//   seq_chunk_kernel  a CTA per (chunk, head): T and B T (or B), 16 x 16 each, into the workspace; all chunks in parallel
+//   seq_walk_kernel   a CTA per (head, 16 value columns) walks the chunks: warps 4..11 (a thread per key channel, the two groups on
+//                     alternate chunks) load and form G k, G q, D k a chunk ahead, while warps 0..3 run P / R (K split over the warps),
+//                     u / o and the state update in 4 x 4 tiles
+// What bounds it: the walk over T / 16 chunks, 832 FMA cycles per chunk (delta rule) and four barriers.  The step-by-step kernel spends 0.38 us
+// per token on one dependent chain of FMAs and shuffles, whatever the width (16 heads of 128 x 128, 2048 tokens: 780 us).
+constexpr int CH_C = 16, CH_VT = 16, CH_MAT = CH_C * CH_C;      // tokens per chunk, value columns per CTA
 
-template <typename act_t, int K>
-__global__ void __launch_bounds__(128) seq_delta_chunk_kernel(b2l_seq_scan_args a) {
-  __shared__ __align__(16) float sk[DL_C][K], sq[DL_C][K], sg[DL_C][K];
-  __shared__ float sA[DL_C][DL_C + 1], sB[DL_C][DL_C + 1], sT[DL_C][DL_C + 1], sbeta[DL_C];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, chunk = blockIdx.x, h = blockIdx.y, hq = h / (a.heads / a.qk_heads);
-  const int t0 = chunk * DL_C, nt = min(DL_C, a.T - t0);
-  for (int i = tid; i < DL_C * K; i += 128) {
-    const int t = i / K, c = i - t * K;
-    const bool in = t < nt;
-    sk[t][c] = in ? a.k[(size_t)(t0 + t) * a.ldk + (size_t)hq * K + c] : 0.f;
-    sq[t][c] = in ? a.q[(size_t)(t0 + t) * a.ldq + (size_t)hq * K + c] : 0.f;
-    sg[t][c] = in ? a.decay[(size_t)(t0 + t) * a.ldd + (size_t)h * K + c] : 1.f;
+// v[0..7] of every lane summed over the warp: lane l holds sum number ((l >> 4) & 1) * 4 + ((l >> 3) & 1) * 2 + ((l >> 2) & 1)
+__device__ __forceinline__ float warp_sum8(float (&v)[8], int lane) {
+#pragma unroll
+  for (int half = 4, w = 16; half >= 1; half >>= 1, w >>= 1) {
+    const bool up = lane & w;
+#pragma unroll
+    for (int j = 0; j < half; ++j) {
+      const float send = up ? v[j] : v[j + half], keep = up ? v[j + half] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+    }
   }
-  if (tid < DL_C) sbeta[tid] = tid < nt ? sigmoid_f(ld_act((const act_t*)a.beta, (size_t)(t0 + tid) * a.ldb + h)) : 0.f;
-  for (int i = tid; i < DL_C * (DL_C + 1); i += 128) { (&sA[0][0])[i] = 0.f; (&sB[0][0])[i] = 0.f; (&sT[0][0])[i] = 0.f; }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <typename act_t, int K, bool DELTA>
+__global__ void __launch_bounds__(128) seq_chunk_kernel(b2l_seq_scan_args a, int vec) {
+  __shared__ __align__(16) float sk[CH_C][K], sq[CH_C][K], sg[CH_C][K];
+  __shared__ float sA[CH_C][CH_C + 1], sB[CH_C][CH_C + 1], sT[CH_C][CH_C + 1], sbeta[CH_C];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, chunk = blockIdx.x, h = blockIdx.y, hq = h / (a.heads / a.qk_heads);
+  const int t0 = chunk * CH_C, nt = min(CH_C, a.T - t0);
+  const float* gk = a.k + (size_t)t0 * a.ldk + (size_t)hq * K;
+  const float* gq = a.q + (size_t)t0 * a.ldq + (size_t)hq * K;
+  const float* gd = a.decay + (size_t)t0 * a.ldd + (a.decay_per_channel ? (size_t)h * K : (size_t)h);
+  if (vec) {
+#pragma unroll
+    for (int i = tid; i < CH_C * K / 4; i += 128) {
+      const int t = i / (K / 4), c = (i - t * (K / 4)) * 4;
+      const bool in = t < nt;
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(&sk[t][c]) = in ? *reinterpret_cast<const float4*>(gk + (size_t)t * a.ldk + c) : z;
+      *reinterpret_cast<float4*>(&sq[t][c]) = in ? *reinterpret_cast<const float4*>(gq + (size_t)t * a.ldq + c) : z;
+      if (a.decay_per_channel) *reinterpret_cast<float4*>(&sg[t][c]) = in ? *reinterpret_cast<const float4*>(gd + (size_t)t * a.ldd + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+  } else {
+    for (int i = tid; i < CH_C * K; i += 128) {
+      const int t = i / K, c = i - t * K;
+      const bool in = t < nt;
+      sk[t][c] = in ? gk[(size_t)t * a.ldk + c] : 0.f;
+      sq[t][c] = in ? gq[(size_t)t * a.ldq + c] : 0.f;
+      if (a.decay_per_channel) sg[t][c] = in ? gd[(size_t)t * a.ldd + c] : 1.f;
+    }
+  }
+  if (!a.decay_per_channel)
+    for (int i = tid; i < CH_C * K; i += 128) {
+      const int t = i / K;
+      sg[t][i - t * K] = t < nt ? gd[(size_t)t * a.ldd] : 1.f;
+    }
+  if (DELTA && tid < CH_C) sbeta[tid] = tid < nt ? sigmoid_f(ld_act((const act_t*)a.beta, (size_t)(t0 + tid) * a.ldb + h)) : 0.f;
   __syncthreads();
 #pragma unroll 1
-  for (int n = 0; n < 4; ++n) {                        // a warp takes columns w, 7 - w, 8 + w, 15 - w: 34 pairs each
+  for (int n = 0; n < 4; ++n) {                        // a warp takes columns w, 7 - w, 8 + w, 15 - w
     const int i = (n & 2) * 4 + ((n & 1) ? 7 - warp : warp);
     float x[K / 32];
 #pragma unroll
     for (int e = 0; e < K / 32; ++e) x[e] = sk[i][lane + 32 * e];
-#pragma unroll 4
-    for (int t = i; t < DL_C; ++t) {
-      float pk = 0.f, pq = 0.f;
+#pragma unroll 1
+    for (int tb = 0; tb < CH_C; tb += 4) {             // four rows: eight sums in nine shuffles
+      float p[8];
 #pragma unroll
-      for (int e = 0; e < K / 32; ++e) {
-        if (t > i) x[e] *= sg[t][lane + 32 * e];
-        pk = fmaf(sk[t][lane + 32 * e], x[e], pk);
-        pq = fmaf(sq[t][lane + 32 * e], x[e], pq);
+      for (int r = 0; r < 4; ++r) {
+        const int t = tb + r;
+        float pk = 0.f, pq = 0.f;
+        if (t >= i) {
+#pragma unroll
+          for (int e = 0; e < K / 32; ++e) {
+            if (t > i) x[e] *= sg[t][lane + 32 * e];
+            if (DELTA) pk = fmaf(sk[t][lane + 32 * e], x[e], pk);
+            pq = fmaf(sq[t][lane + 32 * e], x[e], pq);
+          }
+        }
+        p[r] = t > i ? pk : 0.f;
+        p[4 + r] = pq;
       }
-      pk = warp_sum(pk);
-      pq = warp_sum(pq);
-      if (lane == 0) {
-        if (t > i) sA[t][i] = pk;
-        sB[t][i] = pq;
+      const float v = warp_sum8(p, lane);
+      if ((lane & 3) == 0) {
+        const int t = tb + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        if (lane & 16) sB[t][i] = v;
+        else if (DELTA) sA[t][i] = v;
       }
     }
   }
   __syncthreads();
-  if (tid < DL_C) {                                    // column tid of T by forward substitution
-    float col[DL_C];
+  float* out = a.work_state + ((size_t)chunk * a.heads + h) * (2 * CH_MAT);
+  if (!DELTA) {
+    for (int e = tid; e < CH_MAT; e += 128) out[CH_MAT + e] = sB[e / CH_C][e % CH_C];
+    return;
+  }
+  if (tid < CH_C) {                                    // column tid of T by forward substitution
+    float col[CH_C];
 #pragma unroll
-    for (int t = 0; t < DL_C; ++t) {
+    for (int t = 0; t < CH_C; ++t) {
       float s0 = 0.f, s1 = 0.f;
 #pragma unroll
       for (int i = 0; i < t; ++i) {
@@ -393,189 +444,253 @@ __global__ void __launch_bounds__(128) seq_delta_chunk_kernel(b2l_seq_scan_args 
     }
   }
   __syncthreads();
-  float* out = a.work_state + ((size_t)chunk * a.heads + h) * (2 * DL_C * DL_C);
-  for (int e = tid; e < DL_C * DL_C; e += 128) {
-    const int t = e / DL_C, j = e - t * DL_C;
+  for (int e = tid; e < CH_MAT; e += 128) {
+    const int t = e / CH_C, j = e - t * CH_C;
     float m = 0.f;
 #pragma unroll
-    for (int i = 0; i < DL_C; ++i) m = fmaf(sB[t][i], sT[i][j], m);
+    for (int i = 0; i < CH_C; ++i) m = fmaf(sB[t][i], sT[i][j], m);
     out[e] = sT[t][j];
-    out[DL_C * DL_C + e] = m;
+    out[CH_MAT + e] = m;
   }
 }
 
-template <int K>
-struct DeltaStage {
-  float kq[K][DL_KT];              // [channel][16 tokens of G k | 16 of G q | padding]
-  float kd[DL_C][K];               // D k
-  float tm[2 * DL_C][DL_C];        // T over tril(B) T
-  float v[DL_C][DL_VT];
+template <int K, bool DELTA>
+struct WalkStage {
+  static constexpr int ROWS = DELTA ? 32 : 16, LD = ROWS + 4;      // padded: 16-byte rows of a channel on distinct banks
+  float kq[K][LD];                 // [channel][(delta: 16 tokens of G k) | 16 of G q | padding]
+  float kd[CH_C][K];               // D k
+  float tm[ROWS][CH_C];            // (T over) B T, or B
+  float v[CH_C][CH_VT], u[CH_C][CH_VT];      // values, and (no delta rule) values times vscale
   float gc[K];                     // G of the whole chunk
 };
-template <int K>
-struct DeltaSmem {
-  DeltaStage<K> st[2];
-  float S[K][DL_VT];
-  float part[4][2 * DL_C][DL_VT + 4];
-  float w[DL_C][DL_VT], u[DL_C][DL_VT];
+template <int K, bool DELTA>
+struct WalkSmem {
+  WalkStage<K, DELTA> st[2];
+  float S[K][CH_VT];
+  float part[4][WalkStage<K, DELTA>::ROWS][CH_VT + 4];
+  float w[CH_C][CH_VT], u[CH_C][CH_VT];
 };
-__device__ __forceinline__ void delta_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void walk_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void fma4(float4& d, float s, const float4& v) {
   d.x = fmaf(s, v.x, d.x); d.y = fmaf(s, v.y, d.y); d.z = fmaf(s, v.z, d.z); d.w = fmaf(s, v.w, d.w);
 }
 
-template <int K>
-__global__ void __launch_bounds__(256) seq_delta_scan_kernel(b2l_seq_scan_args a) {
-  extern __shared__ __align__(16) unsigned char delta_raw[];
-  DeltaSmem<K>& sm = *reinterpret_cast<DeltaSmem<K>*>(delta_raw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, hq = h / (a.heads / a.qk_heads), v0 = blockIdx.x * DL_VT;
-  const int n_chunks = (a.T + DL_C - 1) / DL_C;
+template <typename act_t, int K, bool DELTA>
+__global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
+  extern __shared__ __align__(16) unsigned char walk_raw[];
+  using Stage = WalkStage<K, DELTA>;
+  WalkSmem<K, DELTA>& sm = *reinterpret_cast<WalkSmem<K, DELTA>*>(walk_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, hq = h / (a.heads / a.qk_heads), v0 = blockIdx.x * CH_VT;
+  const int n_chunks = (a.T + CH_C - 1) / CH_C;
   float* st = a.state + ((size_t)a.meta[0] * a.heads + h) * (size_t)a.V * K;
 
-  auto prepare = [&](int n) {                          // threads 128..255
-    DeltaStage<K>& s = sm.st[n & 1];
-    const int c = tid - 128, t0 = n * DL_C, nt = min(DL_C, a.T - t0);
-    const float* tm = a.work_state + ((size_t)n * a.heads + h) * (2 * DL_C * DL_C);
-    reinterpret_cast<float4*>(&s.tm[0][0])[c] = reinterpret_cast<const float4*>(tm)[c];
-    for (int i = c; i < DL_C * DL_VT; i += 128) {
-      const int t = i / DL_VT, e = i - t * DL_VT;
-      s.v[t][e] = t < nt ? a.v[(size_t)(t0 + t) * a.ldv + (size_t)h * a.V + v0 + e] : 0.f;
-    }
-    if (c >= K) return;
-    float k[DL_C], q[DL_C], g[DL_C];
+  if (warp >= 4) {
+    // ===================== operands: warps 4..7 the even chunks, 8..11 the odd ones =====================
+    const int par = warp >= 8, c = tid - 128 - 128 * par;
+    const bool chan = c < K;
+    float k[CH_C], q[CH_C], g[CH_C], v[2], vs[2], G = 1.f;
+    float4 tm;
+    auto load = [&](int n) {
+      if (n >= n_chunks) return;
+      const int t0 = n * CH_C, nt = min(CH_C, a.T - t0);
+      if (c < Stage::ROWS * CH_C / 4)
+        tm = reinterpret_cast<const float4*>(a.work_state + ((size_t)n * a.heads + h) * (2 * CH_MAT) + (DELTA ? 0 : CH_MAT))[c];
 #pragma unroll
-    for (int t = 0; t < DL_C; ++t) {
-      const bool in = t < nt;
-      g[t] = in ? a.decay[(size_t)(t0 + t) * a.ldd + (size_t)h * K + c] : 1.f;
-      k[t] = in ? a.k[(size_t)(t0 + t) * a.ldk + (size_t)hq * K + c] : 0.f;
-      q[t] = in ? a.q[(size_t)(t0 + t) * a.ldq + (size_t)hq * K + c] : 0.f;
-    }
-    float d = 1.f;
+      for (int i = 0; i < 2; ++i) {
+        const int t = c / CH_VT + 8 * i, e = c % CH_VT;
+        v[i] = t < nt ? a.v[(size_t)(t0 + t) * a.ldv + (size_t)h * a.V + v0 + e] : 0.f;
+        vs[i] = (!DELTA && a.vscale && t < nt) ? a.vscale[(size_t)(t0 + t) * a.ldvs + h] : 1.f;
+      }
+      if (!chan) return;
+      const float* pg = a.decay + (size_t)t0 * a.ldd + (a.decay_per_channel ? (size_t)h * K + c : (size_t)h);
+      const float* pk = a.k + (size_t)t0 * a.ldk + (size_t)hq * K + c;
+      const float* pq = a.q + (size_t)t0 * a.ldq + (size_t)hq * K + c;
+      if (nt == CH_C) {
 #pragma unroll
-    for (int t = DL_C - 1; t >= 0; --t) {
-      s.kd[t][c] = d * k[t];
-      d *= g[t];
-    }
-    float G = 1.f;
+        for (int t = 0; t < CH_C; ++t, pg += a.ldd, pk += a.ldk, pq += a.ldq) { g[t] = *pg; k[t] = *pk; q[t] = *pq; }
+      } else {
 #pragma unroll
-    for (int t = 0; t < DL_C; ++t) {
-      G *= g[t];
-      k[t] *= G;
-      q[t] *= G;
-    }
-    s.gc[c] = G;
+        for (int t = 0; t < CH_C; ++t, pg += a.ldd, pk += a.ldk, pq += a.ldq) {
+          const bool in = t < nt;
+          g[t] = in ? *pg : 1.f;
+          k[t] = in ? *pk : 0.f;
+          q[t] = in ? *pq : 0.f;
+        }
+      }
+    };
+    float kd[CH_C];
+    auto form = [&](int n) {                           // in registers: the stage's buffer is still in use
+      if (n >= n_chunks || !chan) return;
+      float d = 1.f;
 #pragma unroll
-    for (int t = 0; t < DL_C; t += 4) {
-      *reinterpret_cast<float4*>(&s.kq[c][t]) = make_float4(k[t], k[t + 1], k[t + 2], k[t + 3]);
-      *reinterpret_cast<float4*>(&s.kq[c][DL_C + t]) = make_float4(q[t], q[t + 1], q[t + 2], q[t + 3]);
+      for (int t = CH_C - 1; t >= 0; --t) {
+        kd[t] = d * k[t];
+        d *= g[t];
+      }
+      G = 1.f;
+#pragma unroll
+      for (int t = 0; t < CH_C; ++t) {
+        G *= g[t];
+        k[t] *= G;
+        q[t] *= G;
+      }
+    };
+    auto store = [&](int n) {
+      if (n >= n_chunks) return;
+      Stage& s = sm.st[n & 1];
+      if (c < Stage::ROWS * CH_C / 4) reinterpret_cast<float4*>(&s.tm[0][0])[c] = tm;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = c / CH_VT + 8 * i, e = c % CH_VT;
+        s.v[t][e] = v[i];
+        if (!DELTA) s.u[t][e] = v[i] * vs[i];
+      }
+      if (!chan) return;
+      s.gc[c] = G;
+#pragma unroll
+      for (int t = 0; t < CH_C; ++t) s.kd[t][c] = kd[t];
+#pragma unroll
+      for (int t = 0; t < CH_C; t += 4) {
+        if (DELTA) *reinterpret_cast<float4*>(&s.kq[c][t]) = make_float4(k[t], k[t + 1], k[t + 2], k[t + 3]);
+        *reinterpret_cast<float4*>(&s.kq[c][Stage::ROWS - CH_C + t]) = make_float4(q[t], q[t + 1], q[t + 2], q[t + 3]);
+      }
+    };
+    load(par);
+    form(par);
+    if (par == 0) {
+      store(0);
+      load(2);
     }
-  };
-
-  const int cg = tid >> 2, vg = tid & 3;               // threads 0..127: channels 4 cg .. + 3 (K = 64: half of them), columns 4 vg .. + 3
+    __syncthreads();
+    for (int n = 0; n < n_chunks; ++n) {
+      if (((n + 1) & 1) == par) {
+        store(n + 1);
+        load(n + 3);
+      } else {
+        form(n + 2);
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  // ===================== the walk =====================
+  const int cg = tid >> 2, vg = tid & 3;               // channels 4 cg .. + 3 (K = 64: half of the threads), columns 4 vg .. + 3
   const bool own = cg < K / 4;
+  const float skip = a.skip ? ld_act((const act_t*)a.skip, h) : 0.f;
   float4 S[4];                                         // S[j]: channel 4 cg + j, the four columns
-  if (warp < 4) {
-    if (own) {
-      float4 col[4];
+  if (own) {
+    float4 col[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) col[e] = *reinterpret_cast<const float4*>(st + (size_t)(v0 + 4 * vg + e) * K + 4 * cg);
-      S[0] = make_float4(col[0].x, col[1].x, col[2].x, col[3].x);
-      S[1] = make_float4(col[0].y, col[1].y, col[2].y, col[3].y);
-      S[2] = make_float4(col[0].z, col[1].z, col[2].z, col[3].z);
-      S[3] = make_float4(col[0].w, col[1].w, col[2].w, col[3].w);
+    for (int e = 0; e < 4; ++e) col[e] = *reinterpret_cast<const float4*>(st + (size_t)(v0 + 4 * vg + e) * K + 4 * cg);
+    S[0] = make_float4(col[0].x, col[1].x, col[2].x, col[3].x);
+    S[1] = make_float4(col[0].y, col[1].y, col[2].y, col[3].y);
+    S[2] = make_float4(col[0].z, col[1].z, col[2].z, col[3].z);
+    S[3] = make_float4(col[0].w, col[1].w, col[2].w, col[3].w);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.S[4 * cg + j][4 * vg]) = S[j];
-    }
-  } else {
-    prepare(0);
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.S[4 * cg + j][4 * vg]) = S[j];
   }
   __syncthreads();
-
   for (int n = 0; n < n_chunks; ++n) {
-    if (warp >= 4) {
-      if (n + 1 < n_chunks) prepare(n + 1);
-    } else {
-      const DeltaStage<K>& s = sm.st[n & 1];
-      // P and R: this warp's quarter of the channels, tokens 4 tg .. + 3 of the 32 rows
-      const int tg = lane >> 2;
-      float4 acc[4] = {};
+    const Stage& s = sm.st[n & 1];
+    constexpr int RT = Stage::ROWS / 8;                // rows per lane
+    // (P and) R: this warp's quarter of the channels
+    const int tg = lane >> 2;
+    float4 acc[RT] = {};
 #pragma unroll 8
-      for (int c = warp * (K / 4); c < (warp + 1) * (K / 4); ++c) {
-        const float4 x = *reinterpret_cast<const float4*>(&s.kq[c][4 * tg]), y = *reinterpret_cast<const float4*>(&sm.S[c][4 * vg]);
-        fma4(acc[0], x.x, y); fma4(acc[1], x.y, y); fma4(acc[2], x.z, y); fma4(acc[3], x.w, y);
+    for (int c = warp * (K / 4); c < (warp + 1) * (K / 4); ++c) {
+      const float4 y = *reinterpret_cast<const float4*>(&sm.S[c][4 * vg]);
+      if (DELTA) {
+        const float4 x = *reinterpret_cast<const float4*>(&s.kq[c][4 * tg]);
+        fma4(acc[0], x.x, y); fma4(acc[1], x.y, y); fma4(acc[RT - 2], x.z, y); fma4(acc[RT - 1], x.w, y);
+      } else {
+        const float2 x = *reinterpret_cast<const float2*>(&s.kq[c][2 * tg]);
+        fma4(acc[0], x.x, y); fma4(acc[1], x.y, y);
       }
+    }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.part[warp][4 * tg + j][4 * vg]) = acc[j];
-      delta_bar();
-      // row cg of the 32: v - P, or R
-      float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < RT; ++j) *reinterpret_cast<float4*>(&sm.part[warp][RT * tg + j][4 * vg]) = acc[j];
+    walk_bar();
+    // row cg: v - P, or R
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (cg < Stage::ROWS) {
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const float4 p = *reinterpret_cast<const float4*>(&sm.part[w][cg][4 * vg]);
         r.x += p.x; r.y += p.y; r.z += p.z; r.w += p.w;
       }
-      if (cg < DL_C) {
+    }
+    if (DELTA) {
+      if (cg < CH_C) {
         const float4 v = *reinterpret_cast<const float4*>(&s.v[cg][4 * vg]);
         *reinterpret_cast<float4*>(&sm.w[cg][4 * vg]) = make_float4(v.x - r.x, v.y - r.y, v.z - r.z, v.w - r.w);
         r = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      delta_bar();
+      walk_bar();
+    }
+    const float (*in)[CH_VT] = DELTA ? sm.w : s.u;
+    if (cg < Stage::ROWS) {
 #pragma unroll
-      for (int i = 0; i < DL_C; i += 4) {
+      for (int i = 0; i < CH_C; i += 4) {
         const float4 m = *reinterpret_cast<const float4*>(&s.tm[cg][i]);
-        fma4(r, m.x, *reinterpret_cast<const float4*>(&sm.w[i][4 * vg]));
-        fma4(r, m.y, *reinterpret_cast<const float4*>(&sm.w[i + 1][4 * vg]));
-        fma4(r, m.z, *reinterpret_cast<const float4*>(&sm.w[i + 2][4 * vg]));
-        fma4(r, m.w, *reinterpret_cast<const float4*>(&sm.w[i + 3][4 * vg]));
+        fma4(r, m.x, *reinterpret_cast<const float4*>(&in[i][4 * vg]));
+        fma4(r, m.y, *reinterpret_cast<const float4*>(&in[i + 1][4 * vg]));
+        fma4(r, m.z, *reinterpret_cast<const float4*>(&in[i + 2][4 * vg]));
+        fma4(r, m.w, *reinterpret_cast<const float4*>(&in[i + 3][4 * vg]));
       }
-      if (cg < DL_C) {
+      if (DELTA && cg < CH_C) {
         *reinterpret_cast<float4*>(&sm.u[cg][4 * vg]) = r;
       } else {
-        const int t = n * DL_C + cg - DL_C;
+        const int tt = cg - (Stage::ROWS - CH_C), t = n * CH_C + tt;
         if (t < a.T) {
+          const float4 v = *reinterpret_cast<const float4*>(&s.v[tt][4 * vg]);
           float* o = a.out + (size_t)t * a.ldo + (size_t)h * a.V + v0 + 4 * vg;
-          o[0] = r.x * a.q_mult; o[1] = r.y * a.q_mult; o[2] = r.z * a.q_mult; o[3] = r.w * a.q_mult;
+          o[0] = r.x * a.q_mult + skip * v.x; o[1] = r.y * a.q_mult + skip * v.y; o[2] = r.z * a.q_mult + skip * v.z; o[3] = r.w * a.q_mult + skip * v.w;
         }
       }
-      delta_bar();
-      if (own) {
-        const float4 g = *reinterpret_cast<const float4*>(&s.gc[4 * cg]);
-        const float gj[4] = {g.x, g.y, g.z, g.w};
+    }
+    if (DELTA) walk_bar();
+    const float (*add)[CH_VT] = DELTA ? sm.u : s.u;
+    if (own) {
+      const float4 g = *reinterpret_cast<const float4*>(&s.gc[4 * cg]);
+      const float gj[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { S[j].x *= gj[j]; S[j].y *= gj[j]; S[j].z *= gj[j]; S[j].w *= gj[j]; }
+      for (int j = 0; j < 4; ++j) { S[j].x *= gj[j]; S[j].y *= gj[j]; S[j].z *= gj[j]; S[j].w *= gj[j]; }
 #pragma unroll 8
-        for (int i = 0; i < DL_C; ++i) {
-          const float4 x = *reinterpret_cast<const float4*>(&s.kd[i][4 * cg]), y = *reinterpret_cast<const float4*>(&sm.u[i][4 * vg]);
-          fma4(S[0], x.x, y); fma4(S[1], x.y, y); fma4(S[2], x.z, y); fma4(S[3], x.w, y);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.S[4 * cg + j][4 * vg]) = S[j];
+      for (int i = 0; i < CH_C; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(&s.kd[i][4 * cg]), y = *reinterpret_cast<const float4*>(&add[i][4 * vg]);
+        fma4(S[0], x.x, y); fma4(S[1], x.y, y); fma4(S[2], x.z, y); fma4(S[3], x.w, y);
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.S[4 * cg + j][4 * vg]) = S[j];
     }
     __syncthreads();                                   // the next chunk's operands and the state are in place
   }
-  if (warp < 4 && own) {
+  if (own) {
     const float s4[4][4] = {{S[0].x, S[1].x, S[2].x, S[3].x}, {S[0].y, S[1].y, S[2].y, S[3].y}, {S[0].z, S[1].z, S[2].z, S[3].z}, {S[0].w, S[1].w, S[2].w, S[3].w}};
 #pragma unroll
     for (int e = 0; e < 4; ++e) *reinterpret_cast<float4*>(st + (size_t)(v0 + 4 * vg + e) * K + 4 * cg) = make_float4(s4[e][0], s4[e][1], s4[e][2], s4[e][3]);
   }
 }
 
-static DynSmemCache g_delta_smem[2];
-
-// Portions of two chunks or more with key sizes 64 or 128 and whole groups of 16 values; other sizes and single tokens go step by step.
-static bool delta_chunks(const b2l_seq_scan_args* a) {
-  return a->delta && a->work_state != nullptr && a->T >= 2 * DL_C && (a->K == 64 || a->K == 128) && a->V % DL_VT == 0 && a->decay_per_channel && !a->skip &&
-         !a->vscale && !a->ones && ((uintptr_t)a->state & 15) == 0 && ((uintptr_t)a->work_state & 15) == 0 && (a->T + DL_C - 1) / DL_C <= (1 << 30) && a->heads <= 65535;
+// Portions of two chunks or more with key sizes 64 or 128 and whole groups of 16 values, given room for the chunks' matrices; other sizes, the
+// column of ones and single tokens go step by step.
+static bool walk_chunks(const b2l_seq_scan_args* a) {
+  const size_t chunks = ((size_t)a->T + CH_C - 1) / CH_C;
+  const bool room = a->n_chunks <= 1 || (size_t)a->n_chunks * a->V * a->K >= chunks * 2 * CH_MAT;      // a caller's space for the three-pass form
+  return a->work_state != nullptr && room && a->T >= 2 * CH_C && (a->K == 64 || a->K == 128) && a->V % CH_VT == 0 && !a->ones &&
+         (!a->delta || (a->decay_per_channel && !a->vscale)) && ((uintptr_t)a->state & 15) == 0 && ((uintptr_t)a->work_state & 15) == 0 && a->heads <= 65535;
 }
 
-template <typename act_t, int K>
-static int launch_delta(const b2l_seq_scan_args* a, DynSmemCache& cache, cudaStream_t s) {
-  if (int rc = ensure_dyn_smem(seq_delta_scan_kernel<K>, sizeof(DeltaSmem<K>), cache)) return rc;
-  seq_delta_chunk_kernel<act_t, K><<<dim3((unsigned)((a->T + DL_C - 1) / DL_C), (unsigned)a->heads), 128, 0, s>>>(*a);
-  B2L_LAUNCH_CHECK("seq_delta_chunk_kernel");
-  seq_delta_scan_kernel<K><<<dim3((unsigned)(a->V / DL_VT), (unsigned)a->heads), 256, sizeof(DeltaSmem<K>), s>>>(*a);
-  B2L_LAUNCH_CHECK("seq_delta_scan_kernel");
+template <typename act_t, int K, bool DELTA>
+static int launch_walk(const b2l_seq_scan_args* a, cudaStream_t s) {
+  static DynSmemCache cache;
+  if (int rc = ensure_dyn_smem(seq_walk_kernel<act_t, K, DELTA>, sizeof(WalkSmem<K, DELTA>), cache)) return rc;
+  auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+  const int vec = a->ldq % 4 == 0 && a->ldk % 4 == 0 && al(a->q) && al(a->k) && (!a->decay_per_channel || (a->ldd % 4 == 0 && al(a->decay)));
+  seq_chunk_kernel<act_t, K, DELTA><<<dim3((unsigned)((a->T + CH_C - 1) / CH_C), (unsigned)a->heads), 128, 0, s>>>(*a, vec);
+  B2L_LAUNCH_CHECK("seq_chunk_kernel");
+  seq_walk_kernel<act_t, K, DELTA><<<dim3((unsigned)(a->V / CH_VT), (unsigned)a->heads), 384, sizeof(WalkSmem<K, DELTA>), s>>>(*a);
+  B2L_LAUNCH_CHECK("seq_walk_kernel");
   return 0;
 }
 
@@ -591,8 +706,8 @@ extern "C" int b2l_seq_scan_chunks(int T, int delta) {
   return (T + SCAN_CHUNK - 1) / SCAN_CHUNK;
 }
 
-extern "C" long long b2l_seq_scan_delta_work_floats(int T, int heads) {
-  return T < 2 * DL_C || heads <= 0 ? 0 : (long long)((T + DL_C - 1) / DL_C) * heads * (2 * DL_C * DL_C);
+extern "C" long long b2l_seq_scan_work_floats(int T, int heads) {
+  return T < 2 * CH_C || heads <= 0 ? 0 : (long long)((T + CH_C - 1) / CH_C) * heads * (2 * CH_MAT);
 }
 
 extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
@@ -606,11 +721,12 @@ extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
                 "b2l_seq_scan: chunked portions need the workspace, no delta rule and n_chunks from b2l_seq_scan_chunks");
   B2L_CHECK_ARG(!a->ones || (a->state_ones && a->out_ones && !a->skip && !a->delta), "b2l_seq_scan: the column of ones needs its state and its output, no skip and no delta rule");
   if (a->T == 0) return 0;
-  if (delta_chunks(a)) {
-    if (a->act_dtype == B2L_BF16)
-      return a->K == 64 ? launch_delta<__nv_bfloat16, 64>(a, g_delta_smem[0], (cudaStream_t)stream) : launch_delta<__nv_bfloat16, 128>(a, g_delta_smem[1], (cudaStream_t)stream);
-    if (a->act_dtype == B2L_F32)
-      return a->K == 64 ? launch_delta<float, 64>(a, g_delta_smem[0], (cudaStream_t)stream) : launch_delta<float, 128>(a, g_delta_smem[1], (cudaStream_t)stream);
+  if (walk_chunks(a) && (a->act_dtype == B2L_BF16 || a->act_dtype == B2L_F32)) {
+    cudaStream_t st = (cudaStream_t)stream;
+    B2L_SEQ_DISPATCH(a->act_dtype, {
+      if (a->delta) return a->K == 64 ? launch_walk<act_t, 64, true>(a, st) : launch_walk<act_t, 128, true>(a, st);
+      return a->K == 64 ? launch_walk<act_t, 64, false>(a, st) : launch_walk<act_t, 128, false>(a, st);
+    });
   }
   const int VT = a->V + (a->ones ? 1 : 0);
   const int n_chunks = a->n_chunks > 1 ? a->n_chunks : 1;

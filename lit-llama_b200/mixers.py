@@ -177,8 +177,8 @@ def _scan(ctx: StepContext, *, q, ldq, k, ldk, v, ldv, q_mult, decay, ldd, per_c
     if n_chunks > 1:      # long portion, no delta rule: chunks in parallel (local states, combine, outputs)
         ws = torch.empty((n_chunks, heads, V + int(state_ones is not None), K), dtype=torch.float32, device=state.device)
         wd = torch.empty((n_chunks, heads, K if per_channel else 1), dtype=torch.float32, device=state.device)
-    elif beta is not None:
-        n = lib.b2l_seq_scan_delta_work_floats(ctx.T, heads)
+    elif state_ones is None:  # 16 tokens at a time
+        n = lib.b2l_seq_scan_work_floats(ctx.T, heads)
         ws = torch.empty((n,), dtype=torch.float32, device=state.device) if n else None
     a = S.ScanArgs(q=q, ldq=ldq, k=k, ldk=ldk, v=v, ldv=ldv, q_mult=float(q_mult), decay=decay, ldd=ldd,
                    decay_per_channel=int(per_channel), beta=beta, ldb=ldb, delta=int(beta is not None), vscale=vscale, ldvs=ldvs,
