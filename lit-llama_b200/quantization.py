@@ -117,7 +117,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         registered buffer itself unless release_reference_layout() freed it: then a TRANSIENT tensor rebuilt from the
         batch-1 kernel's tiling (b2l_q4_untile_i8: a pure nibble permutation, tested bit-exact) or by `_source`."""
         if not self._released:
-            return self.quant_weight
+            return self._buffers["quant_weight"]
         if self._source is not None:
             return self._source()
         out = torch.empty((self.in_features // 2, self.out_features), dtype=torch.uint8, device=self._tiled_i8.device).t()
@@ -182,8 +182,9 @@ class ColBlockQuantizedLinear(torch.nn.Module):
     @property
     def tc_capable(self) -> bool:
         """Eligible for the tcgen05 kernel: 4 bits, one (scale, zero) per row, K % 32 == 0, no bias."""
-        return (self.bits == 4 and self.scales.shape[1] == 1 and self.in_features % 32 == 0 and self.bias is None
-                and self.zeros.dtype == self.scales.dtype)
+        buf = self._buffers
+        scales = buf["scales"]
+        return self.bits == 4 and scales.shape[1] == 1 and self.in_features % 32 == 0 and buf["bias"] is None and buf["zeros"].dtype == scales.dtype
 
     def tiled(self) -> torch.Tensor:
         """The [N/128][K/32][128][16 B] re-tiling (b2l_q4_tile), rebuilt when quant_weight changes."""
@@ -237,11 +238,16 @@ class ColBlockQuantizedLinear(torch.nn.Module):
 
     @property
     def gemv_capable(self) -> bool:
+        """Eligible for the kernels of 1..8 rows."""
         return self.tc_capable and self.in_features % 64 == 0 and self.in_features <= 24576
 
     def forward(self, inp):
+        # the small calls are bound by this function (a one-row product takes the GPU 4 us): module attributes are looked up once, and
+        # argument blocks name only the fields that are not zero
         L.require_cuda_bf16(inp, "ColBlockQuantizedLinear.forward")
-        if self.scales.device != inp.device:
+        buf = self._buffers
+        scales, zeros = buf["scales"], buf["zeros"]
+        if scales.device != inp.device:
             raise RuntimeError("input and quant_weight are on different devices")
         shape = inp.shape
         x = inp.reshape(-1, shape[-1])
@@ -252,42 +258,33 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         y = torch.empty((M, N), device=inp.device, dtype=inp.dtype)
         if M == 0:
             return y.reshape(*shape[:-1], N)
-        aligned = x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0
+        ldx = x.stride(0)
+        aligned = x.data_ptr() % 16 == 0 and ldx % 8 == 0
+        tc = self.tc_capable
+        gemv = tc and K % 64 == 0 and K <= 24576         # gemv_capable
         # `wt` keeps a transient tiling (released layers) alive until its launch is enqueued; the caching allocator
         # hands freed blocks out in stream order, so the kernel has finished before anybody else writes there
-        if self.gemv_capable and aligned and M == 1:
+        if gemv and aligned and M == 1:
             wt = self.tiled_i8()
-            a = L.Q4LinearArgs(
-                x=x.data_ptr(), ldx=x.stride(0), qw_tiled=wt.data_ptr(), scales=self.scales.data_ptr(),
-                zeros=self.zeros.data_ptr(), sz_dtype=L.sz_dtype_of(self.scales), y=y.data_ptr(), ldy=N, M=1, N=N, K=K,
-                prologue=L.PRO_NONE, norm_scale=None, eps=0.0, epilogue=L.EPI_STORE, res=None, ldres=0, split_k=0, flags=0)
+            a = L.Q4LinearArgs(x=x.data_ptr(), ldx=ldx, qw_tiled=wt.data_ptr(), scales=scales.data_ptr(), zeros=zeros.data_ptr(),
+                               sz_dtype=L.sz_dtype_of(scales), y=y.data_ptr(), ldy=N, M=1, N=N, K=K)
             L.check(L.lib().b2l_q4_gemv(C.byref(a), L.stream_ptr()), "b2l_q4_gemv")
-        elif self.gemv_capable and aligned and M <= 8 and BATCH_GEMV:
+        elif gemv and aligned and M <= 8 and BATCH_GEMV:
             # 2..8 rows: the mma.sync tile has 8 columns, one per row (csrc/q4_gemv_batch.cu)
             wt = self.tiled_mma()
-            a = L.Q4LinearArgs(
-                x=x.data_ptr(), ldx=x.stride(0), qw_tiled=wt.data_ptr(), scales=self.scales.data_ptr(),
-                zeros=self.zeros.data_ptr(), sz_dtype=L.sz_dtype_of(self.scales), y=y.data_ptr(), ldy=N, M=M, N=N, K=K,
-                prologue=L.PRO_NONE, norm_scale=None, eps=0.0, epilogue=L.EPI_STORE, res=None, ldres=0, split_k=0, flags=0,
-                workspace=batch_workspace(inp.device, K).data_ptr())
+            a = L.Q4LinearArgs(x=x.data_ptr(), ldx=ldx, qw_tiled=wt.data_ptr(), scales=scales.data_ptr(), zeros=zeros.data_ptr(),
+                               sz_dtype=L.sz_dtype_of(scales), y=y.data_ptr(), ldy=N, M=M, N=N, K=K, workspace=batch_workspace(inp.device, K).data_ptr())
             L.check(L.lib().b2l_q4_gemv_batch(C.byref(a), L.stream_ptr()), "b2l_q4_gemv_batch")
-        elif self.tc_capable and aligned and M <= 16:
+        elif tc and aligned and (M <= 16 or K % 64 == 0):
+            # 9..16 rows: tcgen05 with K split over clusters; prompts: tcgen05 tiles of 128 features, weights dequantised on the fly with
+            # get_weight's roundings
             wt = self.tiled()
-            a = L.Q4LinearArgs(
-                x=x.data_ptr(), ldx=x.stride(0), qw_tiled=wt.data_ptr(), scales=self.scales.data_ptr(),
-                zeros=self.zeros.data_ptr(), sz_dtype=L.sz_dtype_of(self.scales), y=y.data_ptr(), ldy=N,
-                M=M, N=N, K=K, prologue=L.PRO_NONE, norm_scale=None, eps=0.0, epilogue=L.EPI_STORE, res=None,
-                ldres=0, split_k=0, flags=0)
-            L.check(L.lib().b2l_q4_linear_tc(C.byref(a), L.stream_ptr()), "b2l_q4_linear_tc")
-        elif self.tc_capable and aligned and K % 64 == 0:
-            # prefill-shaped: 256 x 256 tcgen05 tiles, weights dequantised on the fly with get_weight's roundings
-            wt = self.tiled()
-            a = L.Q4LinearArgs(
-                x=x.data_ptr(), ldx=x.stride(0), qw_tiled=wt.data_ptr(), scales=self.scales.data_ptr(),
-                zeros=self.zeros.data_ptr(), sz_dtype=L.sz_dtype_of(self.scales), y=y.data_ptr(), ldy=N,
-                M=M, N=N, K=K, prologue=L.PRO_NONE, norm_scale=None, eps=0.0, epilogue=L.EPI_STORE, res=None,
-                ldres=0, split_k=0, flags=0)
-            L.check(L.lib().b2l_q4_gemm(C.byref(a), L.stream_ptr()), "b2l_q4_gemm")
+            a = L.Q4LinearArgs(x=x.data_ptr(), ldx=ldx, qw_tiled=wt.data_ptr(), scales=scales.data_ptr(), zeros=zeros.data_ptr(),
+                               sz_dtype=L.sz_dtype_of(scales), y=y.data_ptr(), ldy=N, M=M, N=N, K=K)
+            if M <= 16:
+                L.check(L.lib().b2l_q4_linear_tc(C.byref(a), L.stream_ptr()), "b2l_q4_linear_tc")
+            else:
+                L.check(L.lib().b2l_q4_gemm(C.byref(a), L.stream_ptr()), "b2l_q4_gemm")
         else:
             self._check_layout()
             qw = self.reference_quant_weight()
