@@ -207,6 +207,66 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
 }
 
 // state <- the last taps-1 inputs after T >= taps-1 new tokens (multi-tile launches only).
+// Four taps over long portions in bf16: a thread owns 8 neighbouring channels (16-byte loads, two 16-byte stores) and CONV_VT tokens, so the
+// bytes in flight suffice for HBM (6144 channels x 2048 tokens: 73 us one channel at a time); sums in the order of the kernel above.
+constexpr int CONV_VT = 16, CONV_V = 8;
+__device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    x[2 * i] = __uint_as_float(w[i] << 16);
+    x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+__global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16* __restrict__ in, int ldin, const __nv_bfloat16* __restrict__ w,
+                                                            const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ state,
+                                                            const int* __restrict__ meta, float* __restrict__ out, int ldout, int T, int C) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * CONV_V;
+  if (c >= C) return;
+  const int t0 = blockIdx.y * CONV_VT, nt = min(CONV_VT, T - t0);
+  const __nv_bfloat16* st = state + (size_t)meta[0] * 3 * C;
+  float wr[4][8], win[3][8], b[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {                         // w is [channel][tap]
+    float x[8];
+    ld8_bf16(w + (size_t)c * 4 + 8 * i, x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) wr[e & 3][2 * i + (e >> 2)] = x[e];
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) b[e] = 0.f;
+  if (bias) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) b[e] = __bfloat162float(bias[c + e]);
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int t = t0 - 3 + j;
+    ld8_bf16(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(3 + t) * C + c, win[j]);
+  }
+#pragma unroll 4
+  for (int r = 0; r < nt; ++r) {
+    float cur[8], y[8];
+    ld8_bf16(in + (size_t)(t0 + r) * ldin + c, cur);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float acc = b[e];
+      acc += wr[0][e] * win[0][e];
+      acc += wr[1][e] * win[1][e];
+      acc += wr[2][e] * win[2][e];
+      acc += wr[3][e] * cur[e];
+      y[e] = silu_f(acc);
+      win[0][e] = win[1][e];
+      win[1][e] = win[2][e];
+      win[2][e] = cur[e];
+    }
+    float4* o = reinterpret_cast<float4*>(out + (size_t)(t0 + r) * ldout + c);
+    o[0] = make_float4(y[0], y[1], y[2], y[3]);
+    o[1] = make_float4(y[4], y[5], y[6], y[7]);
+  }
+}
+
 template <typename act_t>
 __global__ void seq_conv_state_kernel(const act_t* __restrict__ in, int ldin, act_t* __restrict__ state,
                                       const int* __restrict__ meta, int T, int C, int taps) {
@@ -432,6 +492,14 @@ extern "C" int b2l_seq_conv_silu(const void* in, int ldin, const void* w, const 
   if (T == 0) return 0;
   const int tiles = (T + CONV_TT - 1) / CONV_TT;
   dim3 grid((unsigned)((C + 127) / 128), (unsigned)tiles);
+  if (act_dtype == B2L_BF16 && taps == 4 && T > CONV_TT && C % CONV_V == 0 && ldin % 8 == 0 && ldout % 4 == 0 && al16(in) && al16(w) && al16(state) && al16(out) &&
+      (T + CONV_VT - 1) / CONV_VT <= 65535) {
+    seq_conv4_silu_kernel<<<dim3((unsigned)((C / CONV_V + 127) / 128), (unsigned)((T + CONV_VT - 1) / CONV_VT)), 128, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)in, ldin, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)state, meta, out, ldout, T, C);
+    seq_conv_state_kernel<__nv_bfloat16><<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (__nv_bfloat16*)state, meta, T, C, taps);
+    B2L_LAUNCH_CHECK("seq_conv4_silu_kernel");
+    return 0;
+  }
   B2L_SEQ_DISPATCH(act_dtype, {
     seq_conv_silu_kernel<act_t><<<grid, 128, 0, (cudaStream_t)stream>>>((const act_t*)in, ldin, (const act_t*)w, (const act_t*)bias,
                                                                         (act_t*)state, meta, out, ldout, T, C, taps, tiles == 1);

@@ -150,6 +150,15 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
   const float pos = (float)(a.meta[1] + t);
   const int half = a.rot_dims / 2, K = a.K;
   const float temp = a.temp_every > 0 ? 1.0f + a.temp_coef * logf((float)((a.meta[1] + t + 1) / a.temp_every + 1)) : 1.0f;
+  // every head turns by the same angles: once per token instead of once per head (16 + 4 heads, 2048 tokens: 29 us before)
+  extern __shared__ float turn[];                       // cos | sin of the pairs, times rot_mult
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    float s, c;
+    sincosf(pos * a.freq[i], &s, &c);
+    turn[i] = c * a.rot_mult;
+    turn[half + i] = s * a.rot_mult;
+  }
+  __syncthreads();
   for (int which = 0; which < 2; ++which) {
     const act_t* x = row + (which == 0 ? a.q_off : a.k_off);
     const act_t* w = (const act_t*)(which == 0 ? a.q_norm : a.k_norm);
@@ -183,10 +192,7 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
       for (int i = lane; i < half; i += 32) {
         const float u = ld_act(p, i) * r * (wh ? ld_act(wh, i) : 1.f);
         const float v = ld_act(p, i + half) * r * (wh ? ld_act(wh, i + half) : 1.f);
-        float s, c;
-        sincosf(pos * a.freq[i], &s, &c);
-        s *= a.rot_mult;
-        c *= a.rot_mult;
+        const float c = turn[i], s = turn[half + i];
         if (which == 0) {
           qo[i] = (u * c - v * s) * temp;
           qo[i + half] = (v * c + u * s) * temp;
@@ -301,8 +307,9 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   B2L_CHECK_ARG((a->v_first == nullptr) || (a->v_out && a->lambda), "b2l_seq_qkv_prep: value mixing needs lambda and an output");
   B2L_CHECK_ARG(a->temp_every >= 0, "b2l_seq_qkv_prep: negative temperature step");
   B2L_CHECK_ARG(!a->unit_rms || (a->q_norm == nullptr && a->k_norm == nullptr), "b2l_seq_qkv_prep: the norm after the rotation has no weight");
+  B2L_CHECK_SUPPORTED(a->rot_dims <= 8192, "b2l_seq_qkv_prep: %d rotated entries of a head", a->rot_dims);
   if (a->T == 0) return 0;
-  B2L_SEQ_DISPATCH(a->act_dtype, (seq_qkv_prep_kernel<act_t><<<a->T, 256, 0, (cudaStream_t)stream>>>(*a)));
+  B2L_SEQ_DISPATCH(a->act_dtype, (seq_qkv_prep_kernel<act_t><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a)));
   B2L_LAUNCH_CHECK("seq_qkv_prep_kernel");
   return 0;
 }
