@@ -883,15 +883,7 @@ struct PromptProb {
   __device__ __forceinline__ void store_ml(const Tile&, int, float, float) const {}
   __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[16]) const {}
   __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
-    uint4* o = reinterpret_cast<uint4*>(y + ((size_t)t.b * T + t.t_first + r) * n_head * 128 + (size_t)t.h * 128 + c0);
-    uint32_t w[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-      w[i] = *reinterpret_cast<const uint32_t*>(&v);
-    }
-    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    atc::st16_bf16(y + ((size_t)t.b * T + t.t_first + r) * n_head * 128 + (size_t)t.h * 128 + c0, x);
   }
 };
 

@@ -98,6 +98,17 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ uint32_t hi_pair(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
 __device__ __forceinline__ float rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 
+__device__ __forceinline__ void st16_bf16(__nv_bfloat16* p, const float (&y)[16]) {      // 16-byte aligned
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(y[2 * i], y[2 * i + 1]);
+    w[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+  reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
 // Prob: what a family's attention is made of.  Members, all __device__:
 //   Tile tile()                           blockIdx -> {first row, rows, [j_begin, j_end) keys, ...}; per-CTA values in Prob::Tile
 //   Row row(tile, j)                      pointers of key j: ka (score entries 0 .. split8*8), kb (the rest), v

@@ -152,8 +152,16 @@ struct Params {
   int M, N, K, Mp, ldy, bt, nst, splits;
 };
 
-__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+// The whole warp runs the issuing loop, so descriptors stay in uniform registers (issued from one lane's branch an MMA took twice its time).
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a),
+               "l"(b), "r"(idesc), "r"(acc), "r"(lead)
+               : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void cluster_sync_all() {
@@ -195,31 +203,36 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int kb = kb_lo, it = 0; kb < kb_hi; ++kb, ++it) {
-        const int st = it % p.nst;
-        if (it >= p.nst) mbar_wait(bar_empty + 8 * st, (uint32_t)(it / p.nst - 1) & 1u, dead);
+      int st = 0;
+      uint32_t ph = 1;                                       // parity of a stage's previous use: passes at once the first time
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        mbar_wait(bar_empty + 8 * st, ph, dead);
         if (dead) break;
         mbar_expect_tx(bar_full + 8 * st, stage_bytes);
         tma_load_2d(sbase + st * stage_bytes, &p.wmap, kb * BK, n0, bar_full + 8 * st);
         tma_load_2d(sbase + st * stage_bytes + A_BYTES, &p.xmap, kb * BK, m0, bar_full + 8 * st);
+        if (++st == p.nst) { st = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // kind::i8: D = s32, A = B = s8, K-major, 128 x bt
-      const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bt >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
-      for (int kb = kb_lo, it = 0; kb < kb_hi; ++kb, ++it) {
-        const int st = it % p.nst;
-        mbar_wait(bar_full + 8 * st, (uint32_t)(it / p.nst) & 1u, dead);
-        if (dead) break;
-        fence_after();
-        const uint64_t ad = desc_sw128(sbase + st * stage_bytes), bd = desc_sw128(sbase + st * stage_bytes + A_BYTES);
+    const uint32_t lead = elect_lane();
+    // kind::i8: D = s32, A = B = s8, K-major, 128 x bt
+    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bt >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
+    int st = 0;
+    uint32_t ph = 0, acc = 0;
+    for (int kb = kb_lo; kb < kb_hi; ++kb) {
+      mbar_wait(bar_full + 8 * st, ph, dead);
+      if (dead) break;
+      fence_after();
+      const uint64_t ad = desc_sw128(sbase + st * stage_bytes), bd = desc_sw128(sbase + st * stage_bytes + A_BYTES);
 #pragma unroll
-        for (int j = 0; j < BK / 32; ++j) mma_i8(tmem, ad + 2 * j, bd + 2 * j, idesc, (it > 0 || j > 0) ? 1u : 0u);
-        commit(bar_empty + 8 * st);
-      }
-      commit(bar_acc);
+      for (int j = 0; j < BK / 32; ++j) mma_i8(tmem, ad + 2 * j, bd + 2 * j, idesc, j > 0 ? 1u : acc, lead);
+      acc = 1;
+      if (lead) commit(bar_empty + 8 * st);
+      __syncwarp();
+      if (++st == p.nst) { st = 0; ph ^= 1u; }
     }
+    if (lead) commit(bar_acc);
   } else {
     mbar_wait(bar_acc, 0, dead);
     fence_after();
@@ -246,6 +259,11 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
     const int n_out = *p.n_out;
     const float scb = n < p.N ? p.scb[n] : 0.f, wsc = scb / 127.0f;
     const int8_t* cbrow = p.cb + (size_t)min(n, p.N - 1) * p.K;
+    // outlier weights by eights: their loads, and those of the activations below, travel together (one by one the six outlier columns of
+    // 137 x 4096 -> 11008 took 30 of the kernel's 44 us); the first eight stay for all token groups
+    float w_first[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) w_first[u] = u < n_out ? __half2float(__float2half_rn((float)cbrow[p.list[u]] * wsc)) : 0.f;
     for (int b = (int)rank; b < nb; b += p.splits) {
       __syncwarp();
       int t[16];
@@ -270,16 +288,29 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
         float term[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) term[i] = 0.f;
-        for (int j = 0; j < n_out; ++j) {            // ascending k, one fma each: the order of the single-row kernel
-          const float w = __half2float(__float2half_rn((float)cbrow[p.list[j]] * wsc));
-          const uint4* ap = reinterpret_cast<const uint4*>(p.aout + (size_t)j * p.Mp + m);     // the same for the whole warp
-          const uint4 a0 = ap[0], a1 = ap[1];
-          const uint32_t aw[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        for (int j0 = 0; j0 < n_out; j0 += 8) {      // ascending k, one fma each: the order of the single-row kernel
+          float w[8];
+          uint4 act[8][2];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&aw[i]));
-            term[2 * i] = fmaf(f.x, w, term[2 * i]);
-            term[2 * i + 1] = fmaf(f.y, w, term[2 * i + 1]);
+          for (int u = 0; u < 8; ++u) {
+            if (j0 + u < n_out) {
+              const uint4* ap = reinterpret_cast<const uint4*>(p.aout + (size_t)(j0 + u) * p.Mp + m);      // the same for the whole warp
+              act[u][0] = ap[0];
+              act[u][1] = ap[1];
+              w[u] = j0 == 0 ? w_first[u] : __half2float(__float2half_rn((float)cbrow[p.list[j0 + u]] * wsc));
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            if (j0 + u < n_out) {
+              const uint32_t aw[8] = {act[u][0].x, act[u][0].y, act[u][0].z, act[u][0].w, act[u][1].x, act[u][1].y, act[u][1].z, act[u][1].w};
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&aw[i]));
+                term[2 * i] = fmaf(f.x, w[u], term[2 * i]);
+                term[2 * i + 1] = fmaf(f.y, w[u], term[2 * i + 1]);
+              }
+            }
           }
         }
 #pragma unroll

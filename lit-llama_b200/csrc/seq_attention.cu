@@ -642,7 +642,7 @@ static int launch_tile(const b2l_seq_attn_args* a, cudaStream_t s, int cache_slo
 struct LocalProb {
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_attn_args a;
-  int DK, DV, stages, split8, q_tmem;
+  int DK, DV, stages, split8, q_tmem, wide;             // wide: rows of `out` are 16-byte aligned
   float scale, softcap;
   struct Tile {
     int h, t_first, rows, pos0, j_begin, j_end, ring0, sk, sv, xa, xb, xv;
@@ -707,9 +707,29 @@ struct LocalProb {
     const __nv_bfloat16* gate = (const __nv_bfloat16*)a.gate + (size_t)tt * a.ldg;
     const float f = a.out_mult * ((a.gate && !a.gate_per_channel) ? sigmoid_f(ld_act(gate, t.h)) : 1.f);
     const size_t o = (size_t)tt * a.ldo + (size_t)t.h * a.V + c0;
+    float y[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      st_out<__nv_bfloat16>(a, o + i, x[i] * f * ((a.gate && a.gate_per_channel) ? sigmoid_f(ld_act(gate, (size_t)t.h * a.V + c0 + i)) : 1.f));
+    for (int i = 0; i < 16; ++i) y[i] = x[i] * f;
+    if (a.gate && a.gate_per_channel) {                       // 16-byte aligned rows: a condition of the launch
+      const uint4* gp = reinterpret_cast<const uint4*>(gate + (size_t)t.h * a.V + c0);
+      const uint4 g0 = gp[0], g1 = gp[1];
+      const uint32_t w[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        y[2 * i] *= sigmoid_f(__uint_as_float(w[i] << 16));
+        y[2 * i + 1] *= sigmoid_f(__uint_as_float(w[i] & 0xffff0000u));
+      }
+    }
+    if (!wide) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) st_out<__nv_bfloat16>(a, o + i, y[i]);
+    } else if (a.out_f32) {
+      float4* q = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+    } else {
+      atc::st16_bf16(reinterpret_cast<__nv_bfloat16*>(a.out) + o, y);
+    }
   }
 };
 
@@ -723,6 +743,7 @@ static int launch_local_tc(const b2l_seq_attn_args* a, cudaStream_t s) {
   if (int rc = tc::map_sw128(&p.map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->v_new, a->T, (long long)a->kv_heads * a->V, a->ldv, 64, atc::KEYS)) return rc;
   p.map_b = p.map_a;
   p.a = *a; p.DK = a->K; p.DV = a->V; p.stages = l.stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = a->softcap;
+  p.wide = ((uintptr_t)a->out & 15) == 0 && a->ldo % 8 == 0;
   const dim3 grid((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS));
   return a->softcap > 0.f ? atc::launch<LocalProb, 3, 3, true>(p, grid, l.smem, g_local_tc_smem[1], s)
                           : atc::launch<LocalProb, 3, 3, false>(p, grid, l.smem, g_local_tc_smem[0], s);

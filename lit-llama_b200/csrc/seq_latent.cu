@@ -512,7 +512,7 @@ __global__ void seq_head_gate_kernel(const act_t* __restrict__ in, long long ld_
 struct LatentProb {
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_latent_attn_args a;
-  int DK, DV, stages, split8, q_tmem, tiled;
+  int DK, DV, stages, split8, q_tmem, tiled, wide;
   float scale, softcap;
   struct Tile {
     int h, t_first, rows, pos0, j_begin, j_end, xa, xb, xv, row_b;
@@ -577,8 +577,15 @@ struct LatentProb {
   __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
     const int tt = t.t_first + r;
     __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)tt * a.ldo + (size_t)t.h * a.vdim + c0;
+    float y[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) st_act(o, i, x[i] * (a.gate ? sigmoid_f(a.gate[(size_t)tt * a.ldg + (size_t)t.h * a.vdim + c0 + i]) : 1.f));
+    for (int i = 0; i < 16; ++i) y[i] = x[i] * (a.gate ? sigmoid_f(a.gate[(size_t)tt * a.ldg + (size_t)t.h * a.vdim + c0 + i]) : 1.f);
+    if (wide) {
+      atc::st16_bf16(o, y);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) st_act(o, i, y[i]);
+    }
   }
 };
 
@@ -598,6 +605,7 @@ static int launch_latent_tc(const b2l_seq_latent_attn_args* a, int splits, cudaS
   const atc::Layout l = atc::layout(3, dk, a->vdim);
   LatentProb p;
   p.a = *a; p.DK = dk; p.DV = a->vdim; p.stages = l.stages; p.split8 = dn / 8; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = 0.f;
+  p.wide = al16(a->out) && a->ldo % 8 == 0;
   // tiled copies: rows of one slot's keys counted from position 0 (only rows of visible positions are read), whole 64-column steps per part.
   // The shared part lies in the slot that the device names: its rows are reached through the map only when the rows of all slots follow one
   // another, and then from slot 0's first.
