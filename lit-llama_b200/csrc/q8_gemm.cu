@@ -27,6 +27,7 @@ constexpr int BK = 128;                    // k (bytes) per stage: one swizzled 
 constexpr int A_BYTES = BN * BK;           // 16 KB
 constexpr int NTHREADS = 192;              // warp 0: TMA, warp 1: MMA issue and tensor memory, warps 2..5: epilogue
 constexpr int MAX_STAGES = 8;
+constexpr int SM_OUT = 16;                 // outlier columns whose activations wait in shared memory; more are read from the workspace
 
 // ---------------------------------------------------------------- outlier columns: 64 columns per CTA, 32 rows at a time
 __global__ void __launch_bounds__(256) q8_mask_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int M, int K, float threshold, uint32_t* __restrict__ mask) {
@@ -180,6 +181,8 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 1];
   __shared__ uint32_t tmem_slot;
+  __shared__ __align__(16) __half s_act[SM_OUT][256];        // the first outliers' activations of the CTA's tokens
+  __shared__ float s_sca[256];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;            // 128-byte swizzle atoms are 1024-byte aligned
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * MAX_STAGES, bar_acc = bar_full + 16 * MAX_STAGES;
@@ -234,6 +237,14 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
     }
     if (lead) commit(bar_acc);
   } else {
+    // while the product runs: row scales and outlier activations of these tokens (read from the workspace group by group they took 1000 cycles each)
+    const int e = tid - 64, n_sm = min(*p.n_out, SM_OUT);
+    for (int i = e; i < p.bt; i += 128) s_sca[i] = m0 + i < p.M ? p.sca[m0 + i] : 0.f;
+    for (int i = e; i < n_sm * (p.bt / 8); i += 128) {
+      const int j = i / (p.bt / 8), c = (i - j * (p.bt / 8)) * 8;
+      if (m0 + c < p.Mp) *reinterpret_cast<uint4*>(&s_act[j][c]) = *reinterpret_cast<const uint4*>(p.aout + (size_t)j * p.Mp + m0 + c);
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
     mbar_wait(bar_acc, 0, dead);
     fence_after();
   }
@@ -294,7 +305,8 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             if (j0 + u < n_out) {
-              const uint4* ap = reinterpret_cast<const uint4*>(p.aout + (size_t)(j0 + u) * p.Mp + m);      // the same for the whole warp
+              // the same for the whole warp
+              const uint4* ap = reinterpret_cast<const uint4*>(j0 + u < SM_OUT ? &s_act[j0 + u][16 * b] : p.aout + (size_t)(j0 + u) * p.Mp + m);
               act[u][0] = ap[0];
               act[u][1] = ap[1];
               w[u] = j0 == 0 ? w_first[u] : __half2float(__float2half_rn((float)cbrow[p.list[j0 + u]] * wsc));
@@ -316,7 +328,7 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           if (m + i >= p.M) break;
-          const float sca = p.sca[m + i];
+          const float sca = s_sca[16 * b + i];
           float v = __half2float(__float2half_rn((float)t[i] * (sca * scb * (1.0f / (127.0f * 127.0f)))));
           if (n_out > 0) v = __half2float(__float2half_rn(v + __half2float(__float2half_rn(term[i]))));
           if (dead) v = __int_as_float(0x7fc00000);
