@@ -1,0 +1,214 @@
+"""GPU: the kernels of long prompts at the edges of their tiles, each through the C ABI against a float64 restatement on the same operands:
+tensor-core attention (local, expanded latent, LLaMA cache), the scans in chunks of 16 tokens, the four-tap convolution, the int4 GEMM's
+tile heights and K splits.
+
+Tolerances: f32 sums of exact products, relative to the result's norm.  A score is a sum of at most 192 products and a row sums at most some
+hundred weighted values, so errors of about sqrt(192 + keys) 2^-24 of the summed magnitudes reach the result: 2e-6 with weights that
+multiply the score's error by its size (scores up to ~10), 1e-5 allowed.  bf16 outputs add their own rounding, 2^-9 per value: 2.5e-3."""
+import ctypes as C
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF = torch.bfloat16
+
+
+def rel(got, want):
+    return float((got.double() - want.double()).norm() / (want.double().norm() + 1e-30))
+
+
+def attend(q, k, v, scale, seen, sink=None, cap=0.0):
+    """q [T, H, K], k [S, H, K], v [S, H, V] in float64, seen [T, S]; sink [H] scores."""
+    s = torch.einsum("thk,shk->hts", q, k) * scale
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    s = s.masked_fill(~seen[None], -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink[:, None, None].expand(-1, s.shape[1], 1)], dim=2)
+    return torch.einsum("hts,shv->thv", torch.softmax(s, -1)[..., :k.shape[0]], v)
+
+
+@pytest.mark.parametrize("T,H,G,K,V,pos0,window,block,sink,cap", [
+    (64, 8, 2, 128, 128, 0, 0, 512, 1, 0.0),        # half a row tile
+    (127, 6, 2, 192, 16, 0, 33, 40, 0, 0.0),        # one part of the query in shared memory, the narrowest values, a window below a key tile
+    (129, 8, 4, 64, 96, 100, 0, 128, 1, 30.0),      # block-local with history across a block border, score cap, values over one and a half atoms
+    (200, 4, 4, 16, 64, 333, 150, 160, 0, 0.0),     # one MMA step per product, history wraps in the ring
+    (300, 4, 1, 48, 80, 50, 1000, 1024, 1, 0.0),    # key size between atoms
+    (1, 320, 320, 128, 128, 0, 0, 64, 0, 0.0),      # one token of many heads stays on the other kernels
+])
+def test_local_attention_tiles(T, H, G, K, V, pos0, window, block, sink, cap):
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    n = pos0 + T
+    q = torch.randn(T, H, K, generator=g, device=DEV) * 2
+    k = torch.randn(n, G, K, generator=g, device=DEV).to(BF)
+    v = torch.randn(n, G, V, generator=g, device=DEV).to(BF)
+    ring_k, ring_v = torch.zeros(2, block, G, K, dtype=BF, device=DEV), torch.zeros(2, block, G, V, dtype=BF, device=DEV)
+    for j in range(max(0, pos0 - block), pos0):
+        ring_k[1, j % block], ring_v[1, j % block] = k[j], v[j]
+    meta = torch.tensor([1, pos0], dtype=torch.int32, device=DEV)
+    out = torch.empty(T, H * V, device=DEV)
+    kn, vn = k[pos0:].contiguous(), v[pos0:].contiguous()
+    a = S.AttnArgs(q=q.data_ptr(), k_new=kn.data_ptr(), v_new=vn.data_ptr(), ldv=G * V, cache_k=ring_k.data_ptr(), cache_v=ring_v.data_ptr(), meta=meta.data_ptr(),
+                   out=out.data_ptr(), ldo=H * V, scale=K ** -0.5, softcap=cap, out_mult=0.5, has_sink=sink, block=block, T=T, heads=H, kv_heads=G, K=K, V=V,
+                   act_dtype=S.act_code(BF), window=window, out_f32=1)
+    S.check(S.lib().b2l_seq_block_attention(C.byref(a), S.stream_ptr()), "attention")
+    i, j = torch.arange(pos0, n, device=DEV)[:, None], torch.arange(n, device=DEV)[None]
+    seen = (j <= i) & ((i - j < window) if window else (i // block == j // block))
+    rep = H // G
+    want = 0.5 * attend(q.double(), k.double().repeat_interleave(rep, 1), v.double().repeat_interleave(rep, 1), K ** -0.5, seen,
+                        torch.zeros(H, dtype=torch.float64, device=DEV) if sink else None, cap)
+    assert rel(out.view(T, H, V), want) < 1e-5
+    last = n - 1                                        # the ring afterwards: the last token's block or the last `block` tokens
+    for p in range(max(pos0, last - block + 1 if window else last // block * block), n):
+        assert torch.equal(ring_k[1, p % block], k[p]) and torch.equal(ring_v[1, p % block], v[p])
+
+
+@pytest.mark.parametrize("T,H,dn,dr,V,pos0,window,sink,splits", [(32, 3, 128, 64, 128, 0, 0, True, 1), (70, 2, 64, 64, 16, 59, 0, False, 5), (129, 4, 32, 16, 48, 300, 100, True, 3),
+                                                                 (65, 2, 128, 0, 128, 1000, 0, True, 30), (257, 2, 128, 64, 128, 7, 64, False, 2)])
+def test_expanded_latent_attention_tiles(T, H, dn, dr, V, pos0, window, sink, splits):
+    """Key splits (also empty ones), windows, a key part shared by the heads or none; sizes whose columns are not whole 64-column steps."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(T + dn)
+    n = pos0 + T
+    kv = torch.randn(n, H, V + dn, generator=g, device=DEV).to(BF)
+    shared = torch.randn(2, n, 24 + dr, generator=g, device=DEV).to(BF)
+    q = torch.randn(T, H, dn + dr, generator=g, device=DEV)
+    sk = torch.randn(H, generator=g, device=DEV)
+    meta = torch.tensor([1, pos0], dtype=torch.int32, device=DEV)
+    out = torch.empty(T, H * V, dtype=BF, device=DEV)
+    work = torch.full((splits, T * H, V + 2), float("nan"), device=DEV)
+    scale = (dn + dr) ** -0.5
+    a = S.LatentAttnArgs(q_a=q.data_ptr(), ldqa_t=H * (dn + dr), ldqa_h=dn + dr, q_b=q.data_ptr() + 4 * dn, ldqb_t=H * (dn + dr), ldqb_h=dn + dr,
+                         key_a=kv.data_ptr(), ldka=H * (V + dn), hska=V + dn, slot_stride_a=0, key_b=shared.data_ptr() + 48, ldkb=24 + dr,
+                         slot_stride_b=n * (24 + dr), sink=sk.data_ptr() if sink else None, meta=meta.data_ptr(), out=out.data_ptr(), ldo=H * V, work=work.data_ptr(),
+                         scale=scale, T=T, heads=H, heads_per_group=1, n_a=V + dn, n_b=dr, vdim=V, score_off=V, splits=splits, act_dtype=S.act_code(BF), window=window)
+    S.check(S.lib().b2l_seq_latent_attention(C.byref(a), S.stream_ptr()), "latent attention")
+    keys = torch.cat([kv[..., V:].double(), shared[1, :, None, 24:].double().expand(n, H, dr)], dim=2)
+    i, j = torch.arange(pos0, n, device=DEV)[:, None], torch.arange(n, device=DEV)[None]
+    seen = (j <= i) & ((i - j < window) if window else (j >= 0))
+    want = attend(q.double(), keys, kv[..., :V].double(), scale, seen, sk.double() if sink else None)
+    assert rel(out.view(T, H, V), want) < 2.5e-3
+
+
+@pytest.mark.parametrize("B,T,nh,S,ring,start", [(1, 64, 3, 128, 0, 0), (2, 129, 2, 200, 37, 0), (1, 130, 2, 300, 290, 100), (2, 300, 1, None, 0, 0)])
+def test_llama_prompt_attention_tiles(B, T, nh, S, ring, start):
+    """64 rows and more at head size 128: cache with and without a turned ring, a second portion behind earlier slots, no cache."""
+    from lit_llama_b200 import _lib as L
+
+    lib, hs, C_ = L.lib(), 128, nh * 128
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(B, T, 3 * C_, generator=g, device=DEV).to(BF)
+    block = 512
+    theta = 1.0 / (10000.0 ** (torch.arange(0, hs, 2, device=DEV).float() / hs))
+    ang = torch.outer(torch.arange(block, device=DEV).float(), theta)
+    rope = torch.stack([ang.cos(), ang.sin()], -1).contiguous()
+    pos = torch.arange(start, start + T, device=DEV)
+
+    def turn(x):
+        r = rope[pos][None, :, None]
+        u, w = x.float()[..., 0::2], x.float()[..., 1::2]
+        return torch.stack([u * r[..., 0] - w * r[..., 1], w * r[..., 0] + u * r[..., 1]], -1).flatten(-2).to(BF)
+
+    q, k, v = qkv.view(B, T, 3, nh, hs).unbind(2)
+    q, k = turn(q), turn(k)
+    y = torch.empty(B, T, C_, dtype=BF, device=DEV)
+    work = torch.zeros(lib.b2l_attn_workspace_bytes(B, nh, hs, T, S or T) // 4 + 1, device=DEV)
+    mine = qkv.clone()
+    if S is None:
+        L.check(lib.b2l_attention_nocache(mine.data_ptr(), rope.data_ptr(), y.data_ptr(), work.data_ptr(), B, T, nh, hs, block, L.stream_ptr()), "attention")
+        kk, vv, seen = k, v, torch.ones(T, T, dtype=torch.bool, device=DEV).tril()
+    else:
+        kk, vv = (torch.randn(B, S, nh, hs, generator=g, device=DEV).to(BF) for _ in range(2))
+        kk[:, start:start + T], vv[:, start:start + T] = k, v
+        slot = (torch.arange(S, device=DEV) + ring) % S
+        ck, cv = torch.empty(B, nh, S, hs, dtype=BF, device=DEV), torch.empty(B, nh, S, hs, dtype=BF, device=DEV)
+        ck[:, :, slot], cv[:, :, slot] = kk.transpose(1, 2), vv.transpose(1, 2)
+        ck[:, :, slot[start:start + T]] = 0
+        cv[:, :, slot[start:start + T]] = 0
+        ring_start = torch.tensor([ring], dtype=torch.int32, device=DEV)
+        L.check(lib.b2l_attention(mine.data_ptr(), ck.data_ptr(), cv.data_ptr(), rope.data_ptr(), pos.data_ptr(), ring_start.data_ptr(), y.data_ptr(), work.data_ptr(),
+                                  B, T, nh, hs, S, block, 0, L.stream_ptr()), "attention")
+        assert torch.equal(ck[:, :, slot[start:start + T]], k.transpose(1, 2)) and torch.equal(cv[:, :, slot[start:start + T]], v.transpose(1, 2))
+        seen = torch.arange(S, device=DEV)[None] <= pos[:, None]
+    for b in range(B):
+        want = attend(q[b].double(), kk[b].double(), vv[b].double(), hs ** -0.5, seen)
+        assert rel(y[b].view(T, nh, hs), want) < 2.5e-3
+
+
+@pytest.mark.parametrize("T,K,V,H,G,form", [(32, 64, 16, 2, 2, "delta"), (47, 128, 48, 4, 2, "delta"), (100, 128, 32, 3, 1, "channel"), (33, 64, 64, 2, 2, "scalar"), (400, 128, 64, 4, 1, "scalar")])
+def test_scans_sixteen_tokens_at_a_time(T, K, V, H, G, form):
+    """Whole chunks and a remainder, from a state that is not zero; strong and weak decays side by side (a factor of e^-6 per step underflows
+    nothing and overflows no quotient); against the token-by-token recurrence in float64.  Same tolerance as the other recurrence tests."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(T + K + V)
+    q, k = torch.randn(T, G, K, generator=g, device=DEV), torch.randn(T, G, K, generator=g, device=DEV)
+    k = k / k.norm(dim=-1, keepdim=True)
+    v = torch.randn(T, H, V, generator=g, device=DEV)
+    a = torch.exp(-6 * torch.rand(T, H, 1 if form == "scalar" else K, generator=g, device=DEV) ** 3)
+    beta = torch.randn(T, H, generator=g, device=DEV)
+    vs, skip = torch.rand(T, H, generator=g, device=DEV) + 0.1, torch.randn(H, generator=g, device=DEV)
+    state = torch.randn(2, H, V, K, generator=g, device=DEV) * 0.1
+    s64, want = state[1].double().clone(), torch.empty(T, H, V, dtype=torch.float64, device=DEV)
+    rep = H // G
+    for t in range(T):
+        kt, qt = k[t].double().repeat_interleave(rep, 0), q[t].double().repeat_interleave(rep, 0)
+        s64 = s64 * a[t].double()[:, None, :]
+        if form == "delta":
+            u = torch.sigmoid(beta[t].double())[:, None] * (v[t].double() - torch.einsum("hvk,hk->hv", s64, kt))
+        else:
+            u = v[t].double() * (vs[t].double()[:, None] if form == "scalar" else 1.0)
+        s64 = s64 + u[:, :, None] * kt[:, None, :]
+        want[t] = 0.5 * torch.einsum("hvk,hk->hv", s64, qt) + (skip.double()[:, None] * v[t].double() if form == "scalar" else 0)
+    lib, out = S.lib(), torch.empty(T, H * V, device=DEV)
+    meta = torch.tensor([1, 0], dtype=torch.int32, device=DEV)
+    n = lib.b2l_seq_scan_work_floats(T, H)
+    assert n > 0 and lib.b2l_seq_scan_work_floats(31, H) == 0
+    other = state[0].clone()
+    work = torch.empty(n, device=DEV)
+    args = S.ScanArgs(q=q.data_ptr(), ldq=G * K, k=k.data_ptr(), ldk=G * K, v=v.data_ptr(), ldv=H * V, q_mult=0.5, decay=a.data_ptr(), ldd=a.shape[1] * a.shape[2],
+                      decay_per_channel=int(form != "scalar"), beta=beta.data_ptr() if form == "delta" else None, ldb=H, delta=int(form == "delta"),
+                      vscale=vs.data_ptr() if form == "scalar" else None, ldvs=H, skip=skip.data_ptr() if form == "scalar" else None, state=state.data_ptr(),
+                      meta=meta.data_ptr(), out=out.data_ptr(), ldo=H * V, T=T, heads=H, qk_heads=G, K=K, V=V, act_dtype=S.act_code(torch.float32), work_state=work.data_ptr(),
+                      n_chunks=1)
+    S.check(lib.b2l_seq_scan(C.byref(args), S.stream_ptr()), "scan")
+    assert rel(out.view(T, H, V), want) < 2e-5 and rel(state[1], s64) < 2e-5
+    assert torch.equal(state[0], other)
+
+
+@pytest.mark.parametrize("T,Ch,bias", [(33, 8, True), (48, 1032, False), (100, 2304, True)])
+def test_four_tap_convolution_of_long_portions(T, Ch, bias):
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x, w = torch.randn(T, Ch + 8, generator=g, device=DEV).to(BF), torch.randn(Ch, 4, generator=g, device=DEV).to(BF)
+    b, state = torch.randn(Ch, generator=g, device=DEV).to(BF), torch.randn(2, 3, Ch, generator=g, device=DEV).to(BF)
+    full = torch.cat([state[1], x[:, :Ch]]).double()
+    want = sum(full[j:j + T] * w[:, j].double() for j in range(4)) + (b.double() if bias else 0)
+    want = want * torch.sigmoid(want)
+    out, meta = torch.empty(T, Ch, device=DEV), torch.tensor([1, 5], dtype=torch.int32, device=DEV)
+    S.check(S.lib().b2l_seq_conv_silu(x.data_ptr(), Ch + 8, w.data_ptr(), b.data_ptr() if bias else None, state.data_ptr(), meta.data_ptr(), out.data_ptr(), Ch, T, Ch, 4,
+                                      S.act_code(BF), S.stream_ptr()), "convolution")
+    assert rel(out, want) < 1e-6 and torch.equal(state[1], x[-3:, :Ch])
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 130, 11008), (33, 4096, 4096), (203, 11008, 4096), (257, 128, 512), (513, 384, 64)])
+def test_q4_gemm_tile_heights_and_splits(M, N, K):
+    """Token tiles of 16..256 and K split over clusters of 1..8 CTAs: f32 sums of exact bf16 products, one bf16 rounding."""
+    from gpu_util import rand_q4, relerr, tile
+    from lit_llama_b200 import _lib as L
+
+    lv, qw, sc, z = rand_q4(N, K, DEV, seed=M + N + K)
+    qt = tile(L, qw, N, K)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    y = torch.full((M + 1, N), 7.0, device=DEV, dtype=BF)
+    a = L.Q4LinearArgs(x=x.data_ptr(), ldx=K, qw_tiled=qt.data_ptr(), scales=sc.data_ptr(), zeros=z.data_ptr(), sz_dtype=L.sz_dtype_of(sc), y=y.data_ptr(), ldy=N, M=M, N=N, K=K)
+    assert L.lib().b2l_q4_gemm(C.byref(a), L.stream_ptr()) == 0, L.lib().b2l_last_error()
+    want = x.double() @ ((lv.to(BF) - z.to(BF)) * sc.to(BF)).double().t()
+    assert relerr(y[:M], want) < 2.0 ** -9 and bool((y[M] == 7).all())
