@@ -764,6 +764,12 @@ __global__ void seq_ring_append_kernel(b2l_seq_attn_args a) {
   const act_t* vn = (const act_t*)a.v_new + (size_t)t * a.ldv;
   act_t* ck = (act_t*)a.cache_k + ((size_t)slot * a.block + e) * nk;
   act_t* cv = (act_t*)a.cache_v + ((size_t)slot * a.block + e) * nv;
+  constexpr int PER = 16 / (int)sizeof(act_t);              // 16-byte copies where every row starts on a boundary
+  if (nk % PER == 0 && nv % PER == 0 && a.ldv % PER == 0 && ((((uintptr_t)a.k_new | (uintptr_t)a.v_new | (uintptr_t)a.cache_k | (uintptr_t)a.cache_v)) & 15) == 0) {
+    for (int i = threadIdx.x; i < nk / PER; i += blockDim.x) reinterpret_cast<uint4*>(ck)[i] = reinterpret_cast<const uint4*>(kn)[i];
+    for (int i = threadIdx.x; i < nv / PER; i += blockDim.x) reinterpret_cast<uint4*>(cv)[i] = reinterpret_cast<const uint4*>(vn)[i];
+    return;
+  }
   for (int i = threadIdx.x; i < nk; i += blockDim.x) ck[i] = kn[i];
   for (int i = threadIdx.x; i < nv; i += blockDim.x) cv[i] = vn[i];
 }

@@ -162,7 +162,8 @@ class CausalSelfAttention(nn.Module):
                 self._ring = torch.zeros(1, dtype=torch.int32, device=x.device)
             if not self._ring_shared:  # stand-alone use: this module owns the roll state (model.py:214-218)
                 L.check(lib.b2l_ring_advance(pos.data_ptr(), T, self._ring.data_ptr(), S, L.stream_ptr()), "b2l_ring_advance")
-            work = torch.zeros(lib.b2l_attn_workspace_bytes(B, self.n_head, hs, T, S) // 4 + 1, device=x.device, dtype=torch.float32)
+            alloc = torch.zeros if T == 1 else torch.empty      # only the one-token kernel has counters in it that must start at zero
+            work = alloc(lib.b2l_attn_workspace_bytes(B, self.n_head, hs, T, S) // 4 + 1, device=x.device, dtype=torch.float32)
             flags = 0 if _rope_is_table else 4  # B2L_F_ROPE_ROWS
             rc = lib.b2l_attention(qkv.data_ptr(), cache_k.data_ptr(), cache_v.data_ptr(), rope32.data_ptr(), pos.data_ptr(),
                                    self._ring.data_ptr(), y.data_ptr(), work.data_ptr(), B, T, self.n_head, hs, S,
