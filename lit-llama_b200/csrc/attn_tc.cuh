@@ -23,8 +23,9 @@
 // issue.  So a tile is taken in four steps of 16 keys, read from tensor memory once for the maximum and once for the weights.
 //
 // A 128 x 64 tile of head size 128 is 24 MMAs of 32 cycles and 12 of 64; it takes 2640 (3000 cycles of copies, then 5250 of softmax and issue
-// in the first form), bound by the issuing warp's waits between the two products.  Layer of width 2048, 2048 tokens, window 1024:
-// 811 us on the CUDA cores (9-19 TFLOP/s), 204 us so; latent layer 1555 -> 203 us.
+// in the first form), bound by the waits between softmax, the two products and back; with a row tile or two per SM the first copies and
+// query loads (4 us per CTA) and the uneven last round show as well.  Layer of width 2048, 2048 tokens, window 1024:
+// 811 us on the CUDA cores (9-19 TFLOP/s), 149 us so (the kernel 79; with two-byte stores, a row per lane, 126); latent layer 1555 -> 178 us.
 #pragma once
 #include "tc_common.cuh"
 

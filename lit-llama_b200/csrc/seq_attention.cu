@@ -416,7 +416,8 @@ static DynSmemCache g_chunk_smem[2];
 // Scores: thread (ty, tx) holds queries ty + 16 i and keys tx + 8 j (4 x 4) with q and k rows read as float4 from
 // padded shared memory; the 8 lanes of a ty group share their rows' maxima and sums by shuffles; the weights go
 // through shared memory into the value product, where the same thread holds its 4 queries x V/8 value channels.
-// All in f32 on the CUDA cores: the design wants scores and weights in 32-bit, which the tensor cores do not give.
+// All in f32 on the CUDA cores: float32 models, portions below 64 tokens and head sizes that are not whole MMA steps; the others take the
+// tensor-core kernel (width 2048, 2048 tokens, window 1024: 700 us here, 79 there).
 constexpr int TQ = 64, TK = 32, TILE_THREADS = 128;
 
 template <typename act_t>
