@@ -218,3 +218,15 @@ def test_weight_changes_bump_the_generation_and_compact_refuses_what_it_cannot_s
     # state_dict of an untouched module is the registered buffer itself (reference strides)
     sd = grouped.state_dict()
     assert sd["quant_weight"].stride() == (1, 32)
+
+
+def test_int4_linear_takes_parameters_in_place_of_its_buffers():
+    """A program may put Parameters where the constructor registers buffers (trainable scales, a bias added later): the layer finds them."""
+    lin = P.ColBlockQuantizedLinear(64, 32, bias=False, bits=4, tile_cols=-1)
+    assert lin.tc_capable and lin.gemv_capable
+    lin.scales, lin.zeros = torch.nn.Parameter(lin.scales), torch.nn.Parameter(lin.zeros)
+    assert lin.tc_capable and lin.gemv_capable
+    lin.quant_weight = torch.nn.Parameter(lin.quant_weight, requires_grad=False)
+    assert lin.reference_quant_weight() is lin.quant_weight
+    lin.bias = torch.nn.Parameter(torch.zeros(32))
+    assert not lin.tc_capable
