@@ -117,7 +117,8 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         registered buffer itself unless release_reference_layout() freed it: then a TRANSIENT tensor rebuilt from the
         batch-1 kernel's tiling (b2l_q4_untile_i8: a pure nibble permutation, tested bit-exact) or by `_source`."""
         if not self._released:
-            return self._held("quant_weight")
+            buf = self._buffers
+            return buf["quant_weight"] if "quant_weight" in buf else self.quant_weight
         if self._source is not None:
             return self._source()
         out = torch.empty((self.in_features // 2, self.out_features), dtype=torch.uint8, device=self._tiled_i8.device).t()
@@ -179,18 +180,15 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         L.check(rc, "b2l_q_dequant")
         return out
 
-    def _held(self, name: str):
-        """self.<name> without the way through Module.__getattr__ while it is the buffer that the constructor registers (a tenth of a
-        microsecond instead of one); a program may have put a Parameter in its place."""
-        buf = self._buffers
-        return buf[name] if name in buf else getattr(self, name)
-
     @property
     def tc_capable(self) -> bool:
         """Eligible for the tcgen05 kernel: 4 bits, one (scale, zero) per row, K % 32 == 0, no bias."""
-        scales = self._held("scales")
-        return (self.bits == 4 and scales.shape[1] == 1 and self.in_features % 32 == 0 and self._held("bias") is None
-                and self._held("zeros").dtype == scales.dtype)
+        try:                      # the buffers of the constructor, without the way through Module.__getattr__
+            buf = self._buffers
+            scales, zeros, bias = buf["scales"], buf["zeros"], buf["bias"]
+        except KeyError:          # a program has put Parameters in their place
+            scales, zeros, bias = self.scales, self.zeros, self.bias
+        return self.bits == 4 and scales.shape[1] == 1 and self.in_features % 32 == 0 and bias is None and zeros.dtype == scales.dtype
 
     def tiled(self) -> torch.Tensor:
         """The [N/128][K/32][128][16 B] re-tiling (b2l_q4_tile), rebuilt when quant_weight changes."""
@@ -251,7 +249,9 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         # the small calls are bound by this function (a one-row product takes the GPU 4 us): module attributes are looked up once, and
         # argument blocks name only the fields that are not zero
         L.require_cuda_bf16(inp, "ColBlockQuantizedLinear.forward")
-        scales, zeros = self._held("scales"), self._held("zeros")
+        buf = self._buffers
+        scales = buf["scales"] if "scales" in buf else self.scales
+        zeros = buf["zeros"] if "zeros" in buf else self.zeros
         if scales.device != inp.device:
             raise RuntimeError("input and quant_weight are on different devices")
         shape = inp.shape
