@@ -448,7 +448,8 @@ __global__ void __launch_bounds__(128) seq_chunk_kernel(b2l_seq_scan_args a, int
     const int t = e / CH_C, j = e - t * CH_C;
     float m = 0.f;
 #pragma unroll
-    for (int i = 0; i < CH_C; ++i) m = fmaf(sB[t][i], sT[i][j], m);
+    for (int i = 0; i < CH_C; ++i)
+      if (i >= j && i <= t) m = fmaf(sB[t][i], sT[i][j], m);      // the rest is zero times a token that t has not seen, which may be infinite
     out[e] = sT[t][j];
     out[CH_MAT + e] = m;
   }
@@ -629,18 +630,19 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
     }
     const float (*in)[CH_VT] = DELTA ? sm.w : s.u;
     if (cg < Stage::ROWS) {
+      const int tt = cg & (CH_C - 1);                  // tokens up to this row's: a zero weight would turn a later token's infinity into NaN
 #pragma unroll
       for (int i = 0; i < CH_C; i += 4) {
         const float4 m = *reinterpret_cast<const float4*>(&s.tm[cg][i]);
-        fma4(r, m.x, *reinterpret_cast<const float4*>(&in[i][4 * vg]));
-        fma4(r, m.y, *reinterpret_cast<const float4*>(&in[i + 1][4 * vg]));
-        fma4(r, m.z, *reinterpret_cast<const float4*>(&in[i + 2][4 * vg]));
-        fma4(r, m.w, *reinterpret_cast<const float4*>(&in[i + 3][4 * vg]));
+        if (i <= tt) fma4(r, m.x, *reinterpret_cast<const float4*>(&in[i][4 * vg]));
+        if (i + 1 <= tt) fma4(r, m.y, *reinterpret_cast<const float4*>(&in[i + 1][4 * vg]));
+        if (i + 2 <= tt) fma4(r, m.z, *reinterpret_cast<const float4*>(&in[i + 2][4 * vg]));
+        if (i + 3 <= tt) fma4(r, m.w, *reinterpret_cast<const float4*>(&in[i + 3][4 * vg]));
       }
       if (DELTA && cg < CH_C) {
         *reinterpret_cast<float4*>(&sm.u[cg][4 * vg]) = r;
       } else {
-        const int tt = cg - (Stage::ROWS - CH_C), t = n * CH_C + tt;
+        const int t = n * CH_C + tt;
         if (t < a.T) {
           const float4 v = *reinterpret_cast<const float4*>(&s.v[tt][4 * vg]);
           float* o = a.out + (size_t)t * a.ldo + (size_t)h * a.V + v0 + 4 * vg;
