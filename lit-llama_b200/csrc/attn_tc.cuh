@@ -121,6 +121,87 @@ __device__ __forceinline__ void st16_bf16(__nv_bfloat16* p, const float (&y)[16]
 //   bool partial(tile); void store_part(tile, r, c0, x[16]); void store_ml(tile, r, m, l)
 //   void store(tile, r, c0, x[16])        normalised outputs c0 .. c0+15
 // and the tensor maps, the host-visible ints DK, DV, stages, split8, q_tmem, floats scale, softcap.
+// Rows whose result is infinite or NaN, again on the CUDA cores over the keys that they see, one row after the other with the whole CTA (a key
+// per thread for the scores, three threads per value column).  The products above cannot tell an infinite key or value from NaN: the lower
+// parts of a query or weight are often zero, and a key that the row does not see, with its weight of zero, counts as well.  Where all is
+// finite it costs the test alone.
+template <class Prob, bool CAP>
+__device__ __noinline__ void redo_rows(const Prob& pr, const uint32_t* s_bad, float* sm) {
+  constexpr int WARPS = THREADS / 32, GROUPS = THREADS / MAX_DV;
+  float *q = sm, *w = q + MAX_DK, *s_acc = w + THREADS, *red = s_acc + GROUPS * MAX_DV, *red2 = red + WARPS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = tid % MAX_DV, grp = tid / MAX_DV;
+  const typename Prob::Tile tl = pr.tile();
+  for (int r = 0; r < tl.rows; ++r) {
+    if (!((s_bad[r >> 5] >> (r & 31)) & 1u)) continue;
+    __syncthreads();
+    if (tid < pr.DK / 8) {
+      float x[8];
+      pr.query(tl, r, tid, x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[8 * tid + e] = x[e];
+    }
+    int lo, hi;
+    pr.range(tl, r, lo, hi);
+    lo = max(lo, tl.j_begin);
+    hi = min(hi, tl.j_end - 1);
+    float m = -INFINITY, l = 0.f, acc = 0.f;
+    __syncthreads();
+    for (int j0 = lo; j0 <= hi; j0 += THREADS) {
+      const int j = j0 + tid, count = min(THREADS, hi - j0 + 1);
+      float s = -INFINITY;
+      if (j <= hi) {
+        const typename Prob::Row row = pr.row(tl, j);
+        s = 0.f;
+        for (int c = 0; c < pr.DK / 8; ++c) {
+          const uint4 u = *reinterpret_cast<const uint4*>(c < pr.split8 ? row.ka + 8 * c : row.kb + 8 * (c - pr.split8));
+          const uint32_t k[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s = fmaf(q[8 * c + 2 * e], __uint_as_float(k[e] << 16), s);
+            s = fmaf(q[8 * c + 2 * e + 1], __uint_as_float(k[e] & 0xffff0000u), s);
+          }
+        }
+        s *= pr.scale;
+        if (CAP) s = pr.softcap * tanhf(s / pr.softcap);
+      }
+      const float top = warp_max(s);
+      if (lane == 0) red[warp] = top;
+      __syncthreads();
+      float now = m;
+      for (int i = 0; i < WARPS; ++i) now = fmaxf(now, red[i]);
+      const float weight = s == -INFINITY ? 0.f : expf(s - now), corr = m == now ? 1.f : expf(m - now), part = warp_sum(weight);
+      w[tid] = weight;
+      if (lane == 0) red2[warp] = part;
+      __syncthreads();
+      float sum = 0.f;
+      for (int i = 0; i < WARPS; ++i) sum += red2[i];
+      l = l * corr + sum;
+      acc *= corr;
+      m = now;
+      if (grp < GROUPS && d < pr.DV)
+        for (int i = grp; i < count; i += GROUPS) acc = fmaf(w[i], __bfloat162float(pr.row(tl, j0 + i).v[d]), acc);
+      __syncthreads();
+    }
+    if (grp < GROUPS) s_acc[grp * MAX_DV + d] = acc;
+    __syncthreads();
+    const bool part = pr.partial(tl);
+    const float sink = pr.sink(tl), M = fmaxf(m, sink), e = m == -INFINITY ? 0.f : expf(m - M);
+    const float inv = part ? 1.f : e / (l * e + (sink == -INFINITY ? 0.f : expf(sink - M)));
+    if (tid == 0 && part) pr.store_ml(tl, r, m, l);
+    if (tid < pr.DV / 16) {
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float t = 0.f;
+        for (int g = 0; g < GROUPS; ++g) t += s_acc[g * MAX_DV + 16 * tid + i];
+        x[i] = t * inv;
+      }
+      if (part) pr.store_part(tl, r, 16 * tid, x);
+      else pr.store(tl, r, 16 * tid, x);
+    }
+  }
+}
+
 template <class Prob, int NQ, int NP, bool CAP>
 __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_constant__ Prob pr) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -128,6 +209,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   float* s_end = s_ref + ROWS;                               // [2][ROWS] maximum and sum of the other group at the end
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 18
   uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 18);
+  uint32_t* s_bad = &tmem_slot + 1;                          // [ROWS / 32] rows with an infinite or NaN result
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages, nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
   const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
@@ -143,6 +225,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     mbar_init_fence();
   }
   if (tid < ROWS) s_ref[tid] = -INFINITY;
+  if (tid < ROWS / 32) s_bad[tid] = 0u;
   if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 512);
   fence_before();
   __syncthreads();
@@ -415,9 +498,14 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full + 8 * b);
     }
-    // the even group ends with the sum of both (relative to the last reference); each group stores every other 16 columns
-    if (n > 0) mbar_wait(pv_done + 8 * ((n - 1) & 1), (uint32_t)((n - 1) >> 1) & 1u, dead);
-    fence_after();
+    // the even group ends with the sum of both (relative to the last reference); each group stores every other 16 columns.  Only the group of
+    // the last tile waits for its product (the other may not have seen the phase before it, whose parity would let it pass); the barriers
+    // below carry that to the other group.
+    if (n > 0 && b == ((n - 1) & 1)) {
+      mbar_wait(pv_done + 8 * b, (uint32_t)((n - 1) >> 1) & 1u, dead);
+      fence_after();
+    }
+    fence_before();
     if (b == 1) { s_end[r] = m; s_end[ROWS + r] = l; }
     bar_named(10, 2 * ROWS);
     const float ref = s_ref[r];
@@ -428,6 +516,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       tot[r] = l;
     }
     bar_named(10, 2 * ROWS);
+    fence_after();
     l = tot[r];
     m = ref;
     const bool part = pr.partial(tl), live = r < tl.rows;
@@ -436,22 +525,29 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     float inv = e / (l * e + (sink == -INFINITY ? 0.f : expf(sink - M)));
     if (dead) inv = l = __int_as_float(0x7fc00000);
     if (part && live && b == 0) pr.store_ml(tl, r, m, l);
+    float odd = part ? l * 0.f : 0.f;                        // NaN as soon as something infinite or NaN came out
     for (int g = b; g < pr.DV / 16; g += 2) {
       uint32_t o[16];
       __syncwarp();
       tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
       float x[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) x[i] = n > 0 ? __uint_as_float(o[i]) * (part ? 1.f : inv) : 0.f;
+      for (int i = 0; i < 16; ++i) {
+        x[i] = n > 0 ? __uint_as_float(o[i]) * (part ? 1.f : inv) : 0.f;
+        odd = fmaf(x[i], 0.f, odd);
+      }
       if (live) {
         if (part) pr.store_part(tl, r, 16 * g, x);
         else pr.store(tl, r, 16 * g, x);
       }
     }
+    const uint32_t bad = __ballot_sync(0xffffffffu, live && !dead && odd != odd);
+    if (lane == 0 && bad) atomicOr(&s_bad[qtr], bad);
   }
   fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
+  if (s_bad[0] | s_bad[1] | s_bad[2] | s_bad[3]) redo_rows<Prob, CAP>(pr, s_bad, reinterpret_cast<float*>(smem_raw + CONTROL));
 }
 
 template <class Prob, int NQ, int NP, bool CAP>
