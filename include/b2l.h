@@ -131,7 +131,9 @@ enum {
   B2L_F_ROPE_ROWS = 4,  /* b2l_attention: `rope` holds the T rows already selected by
                            input_pos (the reference's call convention, model.py:93)    */
   B2L_F_ATTN_UNFUSED = 8, /* debug: force the three-kernel attention path for T == 1   */
-  B2L_F_DEBUG_NOCOMPUTE = 16 /* debug: b2l_q4_gemv streams the weights but skips the math */
+  B2L_F_DEBUG_NOCOMPUTE = 16, /* debug: b2l_q4_gemv streams the weights but skips the math */
+  B2L_F_EXPIRED_SHIFT = 8 /* debug, b2l_q4_gemm: 1 + r in bits 8..11 lets the CTAs of cluster rank r end, after their
+                           work, as if their last wait had run out (their features become NaN) */
 };
 
 /* Fused [RMSNorm ->] int4 linear [-> residual | SwiGLU] on tcgen05.  Replaces

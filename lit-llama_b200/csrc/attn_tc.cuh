@@ -207,14 +207,15 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   float* s_ref = reinterpret_cast<float*>(smem_raw);         // [ROWS] a row's reference maximum after the latest tile
   float* s_end = s_ref + ROWS;                               // [2][ROWS] maximum and sum of the other group at the end
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 18
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 19
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 19);
   uint32_t* s_bad = &tmem_slot + 1;                          // [ROWS / 32] rows with an infinite or NaN result
+  uint32_t& failed = s_bad[ROWS / 32];                       // a wait of the CTA's softmax groups ran out
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages, nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
   const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
   const uint32_t b0 = smem_u32(bars);
-  const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 112, pv_done = b0 + 128;
+  const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 112, pv_done = b0 + 128, gave_up = b0 + 144;
   uint32_t dead = (sq & 1023u) ? 1u : 0u;                    // swizzle atoms need 1024-byte alignment (shared memory starts on one)
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) {
@@ -222,6 +223,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       mbar_init(v_full + 8 * i, V_THREADS); mbar_init(v_empty + 8 * i, 1);
     }
     for (int i = 0; i < 2; ++i) { mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, 4); mbar_init(pv_done + 8 * i, 1); }
+    mbar_init(gave_up, 1);
+    failed = 0u;
     mbar_init_fence();
   }
   if (tid < ROWS) s_ref[tid] = -INFINITY;
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       uint32_t k_ph = 0, v_ph = 0;
       auto score = [&](int t) {
         const int st = k_st;
-        mbar_wait(k_full + 8 * st, k_ph, dead);
+        mbar_wait_warp(k_full + 8 * st, k_ph, dead);
         if (++k_st == nst) { k_st = 0; k_ph ^= 1u; }
         if (dead) return;
         copied(t);
@@ -296,7 +299,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         const int st = v_st;
         mbar_wait(v_full + 8 * st, v_ph, dead);
         if (++v_st == nst) { v_st = 0; v_ph ^= 1u; }
-        mbar_wait(p_full + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, dead);
+        mbar_wait_warp(p_full + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, dead);
         if (dead) break;
         copied(t);
         fence_after();
@@ -313,6 +316,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         __syncwarp();
         if (t + 2 < n) score(t + 2);                         // over the weights of tile t, which the MMAs before it have read
       }
+      if (dead) {                                            // what was issued ends before tensor memory is given back
+        uint32_t late = 0;
+        if (lead) commit(gave_up);
+        mbar_wait(gave_up, 0, late);
+      }
     }
     __syncwarp();
   } else if (warp < 4 || warp == 12) {
@@ -323,9 +331,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     const uint32_t base = keys ? sk : sv, stage = (uint32_t)(keys ? ka : va) * K_ATOM, full = keys ? k_full : v_full, empty = keys ? k_empty : v_empty;
     int st = -1;
     uint32_t phase = 0;                                      // parity of the stage's previous use
-    for (int t = 0; t < n; ++t) {
+    int t = 0;
+    for (; t < n; ++t) {
       if (++st == nst) { st = 0; phase ^= t > nst ? 1u : 0u; }
       if (t >= nst) mbar_wait(empty + 8 * st, phase, dead);
+      if (dead) break;                                       // the stage may still be read: no copy, no arrival
       const uint32_t dst0 = base + st * stage;
       const int j0 = tl.j_begin + t * KEYS;
       int row_a, row_b, row_v;
@@ -360,6 +370,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       cp_arrive(full + 8 * st);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");         // no copy outlives its thread
+    if (lt == 0) {                                           // nor a tiled one: the latest use of every stage, all landed unless a wait ran out
+      uint32_t late = 0;
+      for (int s = 0; s < nst && s < t; ++s) mbar_wait(full + 8 * s, (uint32_t)((t - 1 - s) / nst) & 1u, late);
+    }
   } else {
     // ===================== queries, softmax, output =====================
     const int qtr = warp & 3, b = (warp >> 2) - 1, r = qtr * 32 + lane;      // b: the parity of the group's tiles
@@ -506,6 +520,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       fence_after();
     }
     fence_before();
+    if (dead) failed = 1u;
     if (b == 1) { s_end[r] = m; s_end[ROWS + r] = l; }
     bar_named(10, 2 * ROWS);
     const float ref = s_ref[r];
@@ -517,6 +532,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     }
     bar_named(10, 2 * ROWS);
     fence_after();
+    dead |= failed;
     l = tot[r];
     m = ref;
     const bool part = pr.partial(tl), live = r < tl.rows;

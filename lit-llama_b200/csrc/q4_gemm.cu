@@ -39,6 +39,7 @@ struct Params {
   const void* scales; const void* zeros; int szdt;
   __nv_bfloat16* y; int ldy;
   int M, N, K, bt, nst, splits;
+  int expired;             // cluster rank that ends as if its last wait had run out, or -1
 };
 
 __device__ __forceinline__ uint32_t elect_lane() {
@@ -73,13 +74,21 @@ __device__ __forceinline__ float4 ld_dsmem(uint32_t addr, uint32_t rank) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t addr, uint32_t rank) {
+  uint32_t a, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
 __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * MAX_STAGES + 1];
-  __shared__ uint32_t tmem_slot;
+  __shared__ __align__(8) uint64_t bars[3 * MAX_STAGES + 2];
+  __shared__ uint32_t tmem_slot, failed;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;            // 128-byte swizzle atoms are 1024-byte aligned
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, a_full = empty + 8 * MAX_STAGES, acc_done = a_full + 8 * MAX_STAGES;
+  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, a_full = empty + 8 * MAX_STAGES, acc_done = a_full + 8 * MAX_STAGES,
+                 gave_up = acc_done + 8;
   const uint32_t stage_bytes = W_BYTES + (uint32_t)p.bt * (BK * 2);
   const int tile_n = blockIdx.x / p.splits, n0 = tile_n * BN, m0 = blockIdx.y * p.bt;
   const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
@@ -89,6 +98,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
   if (tid == 0) {
     for (int i = 0; i < p.nst; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 1); mbar_init(a_full + 8 * i, 4); }
     mbar_init(acc_done, 1);
+    mbar_init(gave_up, 1);
+    failed = 0u;
     mbar_init_fence();
   }
   if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), 512);
@@ -111,6 +122,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
         tma_load_2d(base + W_BYTES, &p.xmap, kt * BK, m0, full + 8 * st);
         if (++st == p.nst) { st = 0; ph ^= 1u; }
       }
+      uint32_t late = 0;
+      for (int i = 0; i < p.nst; ++i) {                      // no copy outlives the CTA; all have landed unless a wait ran out
+        mbar_wait(full + 8 * st, ph, late);
+        if (++st == p.nst) { st = 0; ph ^= 1u; }
+      }
     }
   } else if (warp == 1) {
     const uint32_t lead = elect_lane();
@@ -120,7 +136,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
     uint32_t ph = 0, acc = 0;
     for (int kt = kt_lo; kt < kt_hi; ++kt) {
       mbar_wait(full + 8 * st, ph, dead);
-      mbar_wait(a_full + 8 * st, ph, dead);
+      mbar_wait_warp(a_full + 8 * st, ph, dead);
       if (dead) break;
       fence_after();
       const uint64_t bd = desc_sw128(sbase + st * stage_bytes + W_BYTES);
@@ -132,7 +148,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
       __syncwarp();
       if (++st == p.nst) { st = 0; ph ^= 1u; }
     }
-    if (lead) commit(acc_done);
+    if (lead) commit(dead ? gave_up : acc_done);
+    if (dead) {
+      uint32_t late = 0;
+      mbar_wait(gave_up, 0, late);
+    }
   } else if (warp >= 4) {
     const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = n0 + row;
     const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
@@ -167,12 +187,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
       tmem_wait_st();
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(a_full + 8 * st);
+      if (lane == 0 && !dead) mbar_arrive(a_full + 8 * st);
       st += GROUPS;
       if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
     }
     mbar_wait(acc_done, 0, dead);
     fence_after();
+    if (p.expired == (int)rank) dead = 1u;
+    if (dead) failed = 1u;
   }
   __syncwarp();
   // ---- epilogue: a thread owns weight row n, 16 tokens at a time, the groups in turn; split K: a token group is summed by one CTA
@@ -180,7 +202,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
   const uint32_t acc_at = tmem + ((uint32_t)(qtr * 32) << 16) + COL_ACC;
   if (p.splits > 1) {
     // stage memory is free (every MMA has completed): f32 [token group][128 rows][16 tokens], the 16-byte pieces of a row rotated
-    if (warp >= 4) {
+    if (warp >= 4 && !__any_sync(0xffffffffu, dead)) {
       for (int b = grp; b < nb; b += GROUPS) {
         uint32_t r[16];
         tmem_ld16(acc_at + 16 * b, r);
@@ -194,6 +216,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
     cluster_sync_all();
   }
   if (warp >= 4) {
+    for (int s = 0; s < p.splits; ++s)
+      if (p.splits > 1) dead |= ld_dsmem_u32(smem_u32(&failed), (uint32_t)s);
     for (int b = (int)rank + grp * p.splits; b < nb; b += GROUPS * p.splits) {
       __syncwarp();
       float v[16];
@@ -281,6 +305,7 @@ extern "C" int b2l_q4_gemm(const b2l_q4_linear_args* a, b2l_stream_t stream) {
   p.scales = a->scales; p.zeros = a->zeros; p.szdt = a->sz_dtype;
   p.y = (__nv_bfloat16*)a->y; p.ldy = a->ldy;
   p.M = a->M; p.N = a->N; p.K = a->K; p.bt = q.bt; p.nst = q.nst; p.splits = q.splits;
+  p.expired = (a->flags >> B2L_F_EXPIRED_SHIFT & 15) - 1;
   static DynSmemCache smem_cache;
   if (int rc = ensure_dyn_smem(q4_gemm_kernel, q.smem, smem_cache)) return rc;
   LaunchCfg lc(dim3((unsigned)((a->N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, (cudaStream_t)stream, false, q.splits);

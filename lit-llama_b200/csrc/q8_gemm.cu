@@ -177,15 +177,23 @@ __device__ __forceinline__ int4 ld_dsmem(uint32_t addr, uint32_t rank) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t addr, uint32_t rank) {
+  uint32_t a, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
 __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 1];
-  __shared__ uint32_t tmem_slot;
+  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 2];
+  __shared__ uint32_t tmem_slot, failed;
   __shared__ __align__(16) __half s_act[SM_OUT][256];        // the first outliers' activations of the CTA's tokens
   __shared__ float s_sca[256];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;            // 128-byte swizzle atoms are 1024-byte aligned
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * MAX_STAGES, bar_acc = bar_full + 16 * MAX_STAGES;
+  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * MAX_STAGES, bar_acc = bar_full + 16 * MAX_STAGES,
+                 gave_up = bar_acc + 8;
   const uint32_t stage_bytes = A_BYTES + (uint32_t)p.bt * BK;
   const int n0 = (blockIdx.x / p.splits) * BN, m0 = blockIdx.y * p.bt;
   const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
@@ -196,6 +204,8 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
   if (tid == 0) {
     for (int i = 0; i < p.nst; ++i) { mbar_init(bar_full + 8 * i, 1); mbar_init(bar_empty + 8 * i, 1); }
     mbar_init(bar_acc, 1);
+    mbar_init(gave_up, 1);
+    failed = 0u;
     mbar_init_fence();
   }
   if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), cols);
@@ -216,6 +226,11 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
         tma_load_2d(sbase + st * stage_bytes + A_BYTES, &p.xmap, kb * BK, m0, bar_full + 8 * st);
         if (++st == p.nst) { st = 0; ph ^= 1u; }
       }
+      uint32_t late = 0;
+      for (int i = 0; i < p.nst; ++i) {                      // no copy outlives the CTA; all have landed unless a wait ran out
+        mbar_wait(bar_full + 8 * st, ph, late);
+        if (++st == p.nst) { st = 0; ph ^= 1u; }
+      }
     }
   } else if (warp == 1) {
     const uint32_t lead = elect_lane();
@@ -224,7 +239,7 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
     int st = 0;
     uint32_t ph = 0, acc = 0;
     for (int kb = kb_lo; kb < kb_hi; ++kb) {
-      mbar_wait(bar_full + 8 * st, ph, dead);
+      mbar_wait_warp(bar_full + 8 * st, ph, dead);
       if (dead) break;
       fence_after();
       const uint64_t ad = desc_sw128(sbase + st * stage_bytes), bd = desc_sw128(sbase + st * stage_bytes + A_BYTES);
@@ -235,7 +250,11 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
       __syncwarp();
       if (++st == p.nst) { st = 0; ph ^= 1u; }
     }
-    if (lead) commit(bar_acc);
+    if (lead) commit(dead ? gave_up : bar_acc);
+    if (dead) {
+      uint32_t late = 0;
+      mbar_wait(gave_up, 0, late);
+    }
   } else {
     // while the product runs: row scales and outlier activations of these tokens (read from the workspace group by group they took 1000 cycles each)
     const int e = tid - 64, n_sm = min(*p.n_out, SM_OUT);
@@ -247,6 +266,7 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
     asm volatile("bar.sync 1, 128;" ::: "memory");
     mbar_wait(bar_acc, 0, dead);
     fence_after();
+    if (dead) failed = 1u;
   }
   __syncwarp();
   // ---- epilogue: a thread owns weight row n, 16 tokens at a time; split K: slices of 16 tokens are summed by one CTA each
@@ -254,7 +274,7 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
   if (p.splits > 1) {
     // stage memory is free (every MMA has completed): int32 [token group][128 rows][16 tokens]; rows of 64 bytes, the 16-byte piece
     // rotated by the row so that a warp's stores touch every bank
-    if (warp >= 2) {
+    if (warp >= 2 && !__any_sync(0xffffffffu, dead)) {
       for (int b = 0; b < nb; ++b) {
         uint32_t r[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + 16u * b, r);
@@ -267,6 +287,8 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
     cluster_sync_all();
   }
   if (warp >= 2) {
+    for (int s = 0; s < p.splits; ++s)
+      if (p.splits > 1) dead |= ld_dsmem_u32(smem_u32(&failed), (uint32_t)s);
     const int n_out = *p.n_out;
     const float scb = n < p.N ? p.scb[n] : 0.f, wsc = scb / 127.0f;
     const int8_t* cbrow = p.cb + (size_t)min(n, p.N - 1) * p.K;

@@ -16,7 +16,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
 }
 // Waits for the phase with this parity.  `dead` is the thread's sticky error word: a wait that runs out (about a second; a kernel here
-// takes milliseconds at most) sets it and every later wait of the thread returns at once, so the kernel ends; the caller then stores NaN.
+// takes milliseconds at most) sets it and every later wait of the thread returns at once, so the kernel ends.  A thread whose word is set
+// passes nothing on: it issues no copy and no MMA, and leaves the barriers that follow without their arrival, so the waits of those that depend on it
+// run out too, down to the threads that store the result; they store NaN, and a CTA whose sums others add says so in its `failed` word.
+// Copies and MMAs in flight are waited for (with the same limit) by the warp that issued them, with a word of its own.
 __device__ __forceinline__ void mbar_wait(uint32_t a, uint32_t parity, uint32_t& dead) {
   if (dead) return;
   uint32_t ok = 0;
@@ -25,6 +28,11 @@ __device__ __forceinline__ void mbar_wait(uint32_t a, uint32_t parity, uint32_t&
     if (ok) return;
   }
   dead = 1u;
+}
+// The same for a whole warp that acts on the outcome together (aligned instructions, loops with barriers in them).
+__device__ __forceinline__ void mbar_wait_warp(uint32_t a, uint32_t parity, uint32_t& dead) {
+  mbar_wait(a, parity, dead);
+  dead = __any_sync(0xffffffffu, dead) ? 1u : 0u;
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
