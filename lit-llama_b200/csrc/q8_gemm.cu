@@ -27,7 +27,9 @@ constexpr int BK = 128;                    // k (bytes) per stage: one swizzled 
 constexpr int A_BYTES = BN * BK;           // 16 KB
 constexpr int NTHREADS = 192;              // warp 0: TMA, warp 1: MMA issue and tensor memory, warps 2..5: epilogue
 constexpr int MAX_STAGES = 8;
-constexpr int SM_OUT = 16;                 // outlier columns whose activations wait in shared memory; more are read from the workspace
+constexpr int SM_OUT = 16;                 // outlier columns whose activations wait in shared memory; more are read from the workspace,
+constexpr int WS_OUT = 128;                // and beyond these from x
+constexpr int SLAB = 4096;                 // rows per pass: bounds the workspace (16 tiles of 256 rows fill the chip whatever N)
 
 // ---------------------------------------------------------------- outlier columns: 64 columns per CTA, 32 rows at a time
 __global__ void __launch_bounds__(256) q8_mask_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int M, int K, float threshold, uint32_t* __restrict__ mask) {
@@ -114,8 +116,12 @@ __global__ void __launch_bounds__(ROW_THREADS) q8_rows_kernel(const __nv_bfloat1
         int j = before[k >> 5] + __popc(word & ((1u << (k & 31)) - 1u));
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          if ((mb >> e) & 1u) aout[(size_t)(j++) * Mp + m] = __float2half_rn(av[c][e]);
-          else amax = fmaxf(amax, fabsf(av[c][e]));
+          if ((mb >> e) & 1u) {
+            if (j < WS_OUT) aout[(size_t)j * Mp + m] = __float2half_rn(av[c][e]);
+            ++j;
+          } else {
+            amax = fmaxf(amax, fabsf(av[c][e]));
+          }
         }
       }
     }
@@ -149,8 +155,9 @@ __global__ void __launch_bounds__(ROW_THREADS) q8_rows_kernel(const __nv_bfloat1
 struct Params {
   CUtensorMap wmap, xmap;      // CB [N][K], xq [M][K]: boxes of 128 bytes x 128 / bt rows
   const int8_t* cb; const float* scb; const float* sca; const __half* aout; const int* list; const int* n_out;
+  const __nv_bfloat16* x;
   __nv_bfloat16* y;
-  int M, N, K, Mp, ldy, bt, nst, splits;
+  int M, N, K, Mp, ldx, ldy, bt, nst, splits;
 };
 
 // The whole warp runs the issuing loop, so descriptors stay in uniform registers (issued from one lane's branch an MMA took twice its time).
@@ -184,7 +191,7 @@ __device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-__global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 2];
   __shared__ uint32_t tmem_slot, failed;
@@ -321,12 +328,13 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
         float term[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) term[i] = 0.f;
-        for (int j0 = 0; j0 < n_out; j0 += 8) {      // ascending k, one fma each: the order of the single-row kernel
+        const int n_ws = min(n_out, WS_OUT);
+        for (int j0 = 0; j0 < n_ws; j0 += 8) {       // ascending k, one fma each: the order of the single-row kernel
           float w[8];
           uint4 act[8][2];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
-            if (j0 + u < n_out) {
+            if (j0 + u < n_ws) {
               // the same for the whole warp
               const uint4* ap = reinterpret_cast<const uint4*>(j0 + u < SM_OUT ? &s_act[j0 + u][16 * b] : p.aout + (size_t)(j0 + u) * p.Mp + m);
               act[u][0] = ap[0];
@@ -336,7 +344,7 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
           }
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
-            if (j0 + u < n_out) {
+            if (j0 + u < n_ws) {
               const uint32_t aw[8] = {act[u][0].x, act[u][0].y, act[u][0].z, act[u][0].w, act[u][1].x, act[u][1].y, act[u][1].z, act[u][1].w};
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
@@ -346,6 +354,13 @@ __global__ void __launch_bounds__(NTHREADS) q8_gemm_kernel(const __grid_constant
               }
             }
           }
+        }
+        for (int j = WS_OUT; j < n_out; ++j) {
+          const int k = p.list[j];
+          const float w = __half2float(__float2half_rn((float)cbrow[k] * wsc));
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (m + i < p.M) term[i] = fmaf(__half2float(__float2half_rn(bf2f(p.x[(size_t)(m + i) * p.ldx + k]))), w, term[i]);
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -393,10 +408,13 @@ static size_t up16(size_t v) { return (v + 255) & ~(size_t)255; }
 using namespace b2l;
 using namespace b2l::q8gm;
 
+static inline int slab_rows(int M) { return M < SLAB ? M : SLAB; }
+
+// Of one slab of rows: int8 rows, scales, activations of the first outlier columns; the list of outlier columns and their mask.
 extern "C" size_t b2l_q8_linear_workspace_bytes(int M, int K) {
   if (M <= 0 || K <= 0) return 0;
-  const size_t Mp = (size_t)(M + 15) / 16 * 16;
-  return up16((size_t)M * K) + up16(Mp * 4) + up16((size_t)K * Mp * 2) + up16((size_t)K * 4) + up16((size_t)(K + 31) / 32 * 4) + 256;
+  const size_t R = (size_t)slab_rows(M), Rp = (R + 15) / 16 * 16;
+  return up16(R * K) + up16(Rp * 4) + up16(WS_OUT * Rp * 2) + up16((size_t)K * 4) + up16((size_t)(K + 31) / 32 * 4) + 256;
 }
 
 extern "C" int b2l_q8_linear(const void* x, int ldx, const void* cb, const void* scb, void* y, int ldy, void* workspace, int M, int N, int K, float threshold,
@@ -406,28 +424,32 @@ extern "C" int b2l_q8_linear(const void* x, int ldx, const void* cb, const void*
   B2L_CHECK_SUPPORTED(K > 0 && K % BK == 0 && K <= MAX_K, "b2l_q8_linear: K=%d must be a multiple of %d and <= %d", K, BK, MAX_K);
   B2L_CHECK_ARG((((uintptr_t)x | (uintptr_t)cb | (uintptr_t)workspace) % 16) == 0, "b2l_q8_linear: x, cb and workspace must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
-  const int Mp = (M + 15) / 16 * 16;
+  const int R = slab_rows(M), Rp = (R + 15) / 16 * 16;
   uint8_t* w = (uint8_t*)workspace;
-  int8_t* xq = (int8_t*)w;              w += up16((size_t)M * K);
-  float* sca = (float*)w;               w += up16((size_t)Mp * 4);
-  __half* aout = (__half*)w;            w += up16((size_t)K * Mp * 2);
+  int8_t* xq = (int8_t*)w;              w += up16((size_t)R * K);
+  float* sca = (float*)w;               w += up16((size_t)Rp * 4);
+  __half* aout = (__half*)w;            w += up16((size_t)WS_OUT * Rp * 2);
   int* list = (int*)w;                  w += up16((size_t)K * 4);
   uint32_t* mask = (uint32_t*)w;        w += up16((size_t)(K + 31) / 32 * 4);
   int* n_out = (int*)w;
-  const Plan q = plan_for(M, N, K);
-  Params p;
-  if (int rc = map_sw128(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cb, N, K, K, BK, BN)) return rc;
-  if (int rc = map_sw128(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, M, K, K, BK, q.bt)) return rc;
-  static DynSmemCache smem_cache;
-  if (int rc = ensure_dyn_smem(q8_gemm_kernel, q.smem, smem_cache)) return rc;
-  q8_mask_kernel<<<(K + 63) / 64, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, M, K, threshold, mask);
+  q8_mask_kernel<<<(K + 63) / 64, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, M, K, threshold, mask);      // outlier columns are the whole batch's
   B2L_LAUNCH_CHECK("q8_mask_kernel");
-  q8_rows_kernel<<<M, ROW_THREADS, 0, s>>>((const __nv_bfloat16*)x, ldx, K, Mp, mask, xq, sca, aout, list, n_out);
-  B2L_LAUNCH_CHECK("q8_rows_kernel");
-  p.cb = (const int8_t*)cb; p.scb = (const float*)scb; p.sca = sca; p.aout = aout; p.list = list; p.n_out = n_out;
-  p.y = (__nv_bfloat16*)y;
-  p.M = M; p.N = N; p.K = K; p.Mp = Mp; p.ldy = ldy; p.bt = q.bt; p.nst = q.nst; p.splits = q.splits;
-  LaunchCfg lc(dim3((unsigned)((N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, s, false, q.splits);
-  B2L_CUDA(cudaLaunchKernelEx(&lc.cfg, q8_gemm_kernel, p));
+  for (int at = 0; at < M; at += SLAB) {
+    const int rows = M - at < SLAB ? M - at : SLAB;
+    const Plan q = plan_for(rows, N, K);
+    Params p;
+    if (int rc = map_sw128(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cb, N, K, K, BK, BN)) return rc;
+    if (int rc = map_sw128(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, rows, K, K, BK, q.bt)) return rc;
+    static DynSmemCache smem_cache;
+    if (int rc = ensure_dyn_smem(q8_gemm_kernel, q.smem, smem_cache)) return rc;
+    p.x = (const __nv_bfloat16*)x + (size_t)at * ldx;
+    p.y = (__nv_bfloat16*)y + (size_t)at * ldy;
+    q8_rows_kernel<<<rows, ROW_THREADS, 0, s>>>(p.x, ldx, K, Rp, mask, xq, sca, aout, list, n_out);
+    B2L_LAUNCH_CHECK("q8_rows_kernel");
+    p.cb = (const int8_t*)cb; p.scb = (const float*)scb; p.sca = sca; p.aout = aout; p.list = list; p.n_out = n_out;
+    p.M = rows; p.N = N; p.K = K; p.Mp = Rp; p.ldx = ldx; p.ldy = ldy; p.bt = q.bt; p.nst = q.nst; p.splits = q.splits;
+    LaunchCfg lc(dim3((unsigned)((N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, s, false, q.splits);
+    B2L_CUDA(cudaLaunchKernelEx(&lc.cfg, q8_gemm_kernel, p));
+  }
   return 0;
 }

@@ -389,6 +389,32 @@ def test_int8_rows_at_once_equal_single_rows(dev, M, N, K, outliers):
     assert torch.equal(want, got), int((want != got).sum())
 
 
+def test_int8_long_batches_in_slabs_of_rows(dev):
+    """4096 rows per pass bound the workspace whatever the batch (and 128 outlier columns of it); outlier columns are still the whole batch's:
+    a row of the first slab under the mask that a row of the second one makes gives the single-row kernel's bits."""
+    from lit_llama_b200 import _lib as L
+
+    lib, (M, N, K) = L.lib(), (4133, 130, 256)
+    assert lib.b2l_q8_linear_workspace_bytes(1 << 20, 5120) == lib.b2l_q8_linear_workspace_bytes(4096, 5120) <= 4096 * (5120 + 2 * 128 + 4) + 5120 * 4 + 8192
+    g = torch.Generator().manual_seed(M)
+    cb, scb = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(dev), (torch.rand(N, generator=g) * 0.1 + 0.01).to(dev)
+    x = torch.randn(M, K, generator=g).clamp_(-5, 5)
+    x[4130, 77], x[9, 200] = 9.0, -8.0
+    x = x.bfloat16().to(dev)
+    tiled, mask = torch.empty(lib.b2l_q8_tiled_bytes(N, K), dtype=torch.uint8, device=dev), torch.empty(K // 32, dtype=torch.int32, device=dev)
+    L.check(lib.b2l_q8_tile(cb.data_ptr(), tiled.data_ptr(), N, K, L.stream_ptr()), "tile")
+    L.check(lib.b2l_q8_outlier_mask(x.data_ptr(), K, M, K, 6.0, mask.data_ptr(), L.stream_ptr()), "mask")
+    got = torch.empty(M + 1, N, dtype=torch.bfloat16, device=dev).fill_(3.0)
+    n = lib.b2l_q8_linear_workspace_bytes(M, K)
+    ws = torch.full((n + 256,), 7, dtype=torch.uint8, device=dev)
+    L.check(lib.b2l_q8_linear(x.data_ptr(), K, cb.data_ptr(), scb.data_ptr(), got.data_ptr(), N, ws.data_ptr(), M, N, K, 6.0, L.stream_ptr()), "linear")
+    assert bool((ws[n:] == 7).all()) and bool((got[M] == 3).all())
+    for m in (0, 9, 77, 4095, 4096, 4130, 4132):
+        want = torch.empty(N, dtype=torch.bfloat16, device=dev)
+        L.check(lib.b2l_q8_gemv(x[m].data_ptr(), tiled.data_ptr(), cb.data_ptr(), scb.data_ptr(), mask.data_ptr(), want.data_ptr(), N, K, 6.0, 0, L.stream_ptr()), "gemv")
+        assert torch.equal(want, got[m])
+
+
 @pytest.mark.parametrize("n", [4096, 8192, 130])
 def test_tp_allreduce_single_rank_is_identity(dev, n):
     """b2l_tp_allreduce with world = 1 (no peers): the multi-CTA indexing, the in-place path and the epoch words that
