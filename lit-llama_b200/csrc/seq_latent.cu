@@ -609,7 +609,8 @@ static int launch_latent_tc(const b2l_seq_latent_attn_args* a, int splits, cudaS
   // tiled copies: rows of one slot's keys counted from position 0 (only rows of visible positions are read), whole 64-column steps per part.
   // The shared part lies in the slot that the device names: its rows are reached through the map only when the rows of all slots follow one
   // another, and then from slot 0's first.
-  p.tiled = a->slot_stride_a == 0 && (a->n_b == 0 || (dn % 64 == 0 && a->slot_stride_b % a->ldkb == 0));
+  // A tensor map's rows do not overlap: heads that lie further apart than the positions go by 16-byte copies.
+  p.tiled = a->slot_stride_a == 0 && (a->heads - 1) * a->hska + a->n_a <= a->ldka && (a->n_b == 0 || (dn % 64 == 0 && a->slot_stride_b % a->ldkb == 0));
   if (p.tiled) {
     const long long rows = 1LL << 31;
     if (int rc = tc::map_sw128(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->key_a, rows, (a->heads - 1) * a->hska + a->n_a, a->ldka, 64, atc::KEYS)) return rc;

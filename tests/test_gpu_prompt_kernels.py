@@ -212,3 +212,23 @@ def test_q4_gemm_tile_heights_and_splits(M, N, K):
     assert L.lib().b2l_q4_gemm(C.byref(a), L.stream_ptr()) == 0, L.lib().b2l_last_error()
     want = x.double() @ ((lv.to(BF) - z.to(BF)) * sc.to(BF)).double().t()
     assert relerr(y[:M], want) < 2.0 ** -9 and bool((y[M] == 7).all())
+
+
+def test_expanded_latent_attention_with_heads_apart():
+    """Keys and values head by head ([heads][positions][entries], rows of one head next to each other): the same result as position by position."""
+    from lit_llama_b200 import _seqlib as S
+
+    T, H, dn, V, pos0 = 150, 3, 64, 64, 90
+    n, g = pos0 + T, torch.Generator(device=DEV).manual_seed(5)
+    kv, q = torch.randn(n, H, V + dn, generator=g, device=DEV).to(BF), torch.randn(T, H, dn, generator=g, device=DEV)
+    apart, meta = kv.transpose(0, 1).contiguous(), torch.tensor([0, pos0], dtype=torch.int32, device=DEV)
+    res = []
+    for rows, ldka, hska in ((kv, H * (V + dn), V + dn), (apart, V + dn, n * (V + dn))):
+        out = torch.empty(T, H * V, dtype=BF, device=DEV)
+        a = S.LatentAttnArgs(q_a=q.data_ptr(), ldqa_t=H * dn, ldqa_h=dn, key_a=rows.data_ptr(), ldka=ldka, hska=hska, slot_stride_a=0, meta=meta.data_ptr(), out=out.data_ptr(),
+                             ldo=H * V, scale=dn ** -0.5, T=T, heads=H, heads_per_group=1, n_a=V + dn, n_b=0, vdim=V, score_off=V, splits=1, act_dtype=S.act_code(BF))
+        S.check(S.lib().b2l_seq_latent_attention(C.byref(a), S.stream_ptr()), "latent attention")
+        res.append(out)
+    seen = torch.arange(n, device=DEV)[None] <= torch.arange(pos0, n, device=DEV)[:, None]
+    assert rel(res[0].view(T, H, V), attend(q.double(), kv[..., V:].double(), kv[..., :V].double(), dn ** -0.5, seen)) < 2.5e-3
+    assert torch.equal(res[0], res[1])
