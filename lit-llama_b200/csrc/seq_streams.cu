@@ -134,6 +134,8 @@ __global__ void seq_scale_kernel(float* __restrict__ z, size_t n, float mult) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) z[i] *= mult;
 }
 
+constexpr int MOST_PAIRS = 4096;      // rotated pairs whose cos and sin fit the 48 KB of a launch without an attribute
+
 // Attention operands of one token from the stacked projection row, one CTA per token.
 //   q_out (f32) and k_out (act): RMS norm (whole_row: over all heads*K entries with a weight of that size; else per
 //   head with a weight of K entries shared by the heads; no weight: no norm), then rotation of the first rot_dims
@@ -152,7 +154,8 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
   const float temp = a.temp_every > 0 ? 1.0f + a.temp_coef * logf((float)((a.meta[1] + t + 1) / a.temp_every + 1)) : 1.0f;
   // every head turns by the same angles: once per token instead of once per head (16 + 4 heads, 2048 tokens: 29 -> 27 us)
   extern __shared__ float turn[];                       // cos | sin of the pairs, times rot_mult
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+  const bool table = half <= MOST_PAIRS;
+  for (int i = threadIdx.x; table && i < half; i += blockDim.x) {
     float s, c;
     sincosf(pos * a.freq[i], &s, &c);
     turn[i] = c * a.rot_mult;
@@ -237,7 +240,15 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
       for (int i = lane; i < half; i += 32) {
         const float u = ld_act(p, i) * r * (wh ? ld_act(wh, i) : 1.f);
         const float v = ld_act(p, i + half) * r * (wh ? ld_act(wh, i + half) : 1.f);
-        const float c = turn[i], s = turn[half + i];
+        float s, c;
+        if (table) {
+          c = turn[i];
+          s = turn[half + i];
+        } else {
+          sincosf(pos * a.freq[i], &s, &c);
+          s *= a.rot_mult;
+          c *= a.rot_mult;
+        }
         if (which == 0) {
           qo[i] = (u * c - v * s) * temp;
           qo[i + half] = (v * c + u * s) * temp;
@@ -352,13 +363,13 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   B2L_CHECK_ARG((a->v_first == nullptr) || (a->v_out && a->lambda), "b2l_seq_qkv_prep: value mixing needs lambda and an output");
   B2L_CHECK_ARG(a->temp_every >= 0, "b2l_seq_qkv_prep: negative temperature step");
   B2L_CHECK_ARG(!a->unit_rms || (a->q_norm == nullptr && a->k_norm == nullptr), "b2l_seq_qkv_prep: the norm after the rotation has no weight");
-  B2L_CHECK_SUPPORTED(a->rot_dims <= 8192, "b2l_seq_qkv_prep: %d rotated entries of a head", a->rot_dims);
   if (a->T == 0) return 0;
   auto al8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; };
   // whole heads turn, in groups of four pairs, and no factor per head; both norms or none, so that both rows take the same form
-  const int quads = a->act_dtype == B2L_BF16 && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
+  const bool table = a->rot_dims / 2 <= MOST_PAIRS;
+  const int quads = table && a->act_dtype == B2L_BF16 && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
                     a->k_off % 4 == 0 && a->ld % 4 == 0 && al8(a->proj) && al8(a->q_norm) && al8(a->k_norm) && al16(a->q_out) && al8(a->k_out);
-  B2L_SEQ_DISPATCH(a->act_dtype, (seq_qkv_prep_kernel<act_t><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a, quads)));
+  B2L_SEQ_DISPATCH(a->act_dtype, (seq_qkv_prep_kernel<act_t><<<a->T, 256, table ? sizeof(float) * a->rot_dims : 0, (cudaStream_t)stream>>>(*a, quads)));
   B2L_LAUNCH_CHECK("seq_qkv_prep_kernel");
   return 0;
 }

@@ -232,3 +232,22 @@ def test_expanded_latent_attention_with_heads_apart():
     seen = torch.arange(n, device=DEV)[None] <= torch.arange(pos0, n, device=DEV)[:, None]
     assert rel(res[0].view(T, H, V), attend(q.double(), kv[..., V:].double(), kv[..., :V].double(), dn ** -0.5, seen)) < 2.5e-3
     assert torch.equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("rot", [8192, 8208])
+def test_attention_operands_of_very_wide_heads(rot):
+    """The angles of a token wait in shared memory up to 8192 rotated entries; beyond that every head forms its own.  cos and sin of f32 angles
+    up to 40 are good to 40 * 2^-24, products and sums add a few 2^-24: 1e-5 of the largest entries."""
+    from lit_llama_b200 import _seqlib as S
+
+    T, g = 3, torch.Generator(device=DEV).manual_seed(rot)
+    x, freq = torch.randn(T, 2 * rot, generator=g, device=DEV), torch.rand(rot // 2, generator=g, device=DEV)
+    q, k, meta = torch.empty(T, rot, device=DEV), torch.empty(T, rot, device=DEV), torch.tensor([0, 30], dtype=torch.int32, device=DEV)
+    a = S.QkvPrepArgs(proj=x.data_ptr(), ld=2 * rot, q_off=0, k_off=rot, v_off=0, eps=1e-6, freq=freq.data_ptr(), rot_dims=rot, rot_mult=1.0, meta=meta.data_ptr(),
+                      q_out=q.data_ptr(), k_out=k.data_ptr(), T=T, heads=1, kv_heads=1, K=rot, V=16, act_dtype=S.act_code(torch.float32))
+    S.check(S.lib().b2l_seq_qkv_prep(C.byref(a), S.stream_ptr()), "operands")
+    ang = (torch.arange(30, 30 + T, device=DEV).double()[:, None] * freq.double())
+    for got, src in ((q, x[:, :rot]), (k, x[:, rot:])):
+        u, v = src.double()[:, :rot // 2], src.double()[:, rot // 2:]
+        want = torch.cat([u * ang.cos() - v * ang.sin(), v * ang.cos() + u * ang.sin()], 1)
+        assert float((got - want).abs().max()) < 1e-5 * float(want.abs().max())
