@@ -1,4 +1,4 @@
-"""bench.py - LLaMA-7B gptq.int4 batch-1 decode throughput on B200 (BASELINE.json configs[1]).
+"""bench.py - LLaMA-7B gptq.int4 batch-1 decode throughput on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -18,10 +18,10 @@ positions 16..2047 whatever K is (a stride, not consecutive positions), so `valu
             __graft_entry__.build()) on the host cores, same synthetic weights as the GPU arm, whole tokens through
             all 32 Blocks; the token loop is the golden-pinned restatement of generate.py (oracle/llama_oracle.py).
             Fallback when oracle/_ref is absent: the oracle port (kind "port").
-N > 1: `value` = independent replicas, one process per GPU (the reference has no multi-GPU inference, SURVEY.md section
-2.1; 7B fits one GPU): weak scaling, no data-path collective.  The same run then measures the TENSOR-PARALLEL path on
-the same ranks and reports it under "tp": LLaMA-7B split N ways, and LLaMA-65B gptq.int4 TP = 8 (BASELINE.json
-configs[4]) when N = 8 -- fused per-rank step, two one-shot all-reduces per Block over peer memory (tools/tp_bench.py).
+N > 1: `value` = independent replicas, one process per GPU (the reference has no multi-GPU inference;
+7B fits one GPU): weak scaling, no data-path collective.  The same run then measures the TENSOR-PARALLEL path on
+the same ranks and reports it under "tp": LLaMA-7B split N ways, and LLaMA-65B gptq.int4 TP = 8
+when N = 8 -- fused per-rank step, two one-shot all-reduces per Block over peer memory (tools/tp_bench.py).
 """
 import argparse
 import json
@@ -50,7 +50,7 @@ def n_hidden_for(n_embd: int) -> int:
 
 
 def model_bytes(cfg_name: str):
-    """Algorithmic bytes of SURVEY.md section 8d for batch 1: W (packed int4 linears incl. lm_head, bf16 scales and
+    """Algorithmic bytes for batch 1: W (packed int4 linears incl. lm_head, bf16 scales and
     zeros, RMSNorm scales, one wte row) and KV bytes per position."""
     L, _, C = LLAMA_SHAPES[cfg_name]
     nh, V = n_hidden_for(C), 32000
@@ -62,7 +62,7 @@ def model_bytes(cfg_name: str):
 
 
 def synth_state(name, seed=1234, dev=None):
-    """Random-init gptq.int4 weights of the named size: the direct synthesis of SURVEY.md section 8d (uniform levels,
+    """Random-init gptq.int4 weights of the named size: direct synthesis (uniform levels,
     zero 8, per-row scales).  Drawn with the generator of `dev` (default: cuda:0 when there is one, so that the GPU
     arm and the CPU reference arm -- which moves the tensors to the host -- hold IDENTICAL weights)."""
     import torch
@@ -175,7 +175,7 @@ def sample_next(logits, top_k=TOP_K, temperature=TEMPERATURE):
 def host_threads():
     """Threads for the CPU arm: every core this process may use (torchrun exports OMP_NUM_THREADS=1, which would
     silently turn the baseline into a single-core run), capped at 32 -- the reference's CPU path is a chain of small
-    torch ops per Linear and runs SLOWER beyond that on a 100+-thread host (measured in round 1: 7.4x swings)."""
+    torch ops per Linear and runs SLOWER beyond that on a 100+-thread host (measured: 7.4x swings)."""
     try:
         n = len(os.sched_getaffinity(0))
     except AttributeError:
@@ -508,7 +508,7 @@ def main():
             barrier()
             t_e2e = time.perf_counter() - t0
 
-        # ---- tokens/s at fixed positions (SURVEY 8d): 24 steps each at p = 128, 1024, 2047
+        # ---- tokens/s at fixed positions: 24 steps each at p = 128, 1024, 2047
         points = {}
         for q in (128, 1024, 2047):
             pq = torch.tensor([q], device=dev)
@@ -533,8 +533,8 @@ def main():
     import ctypes as C
     launches = L.lib().b2l_decode_step_launches(C.byref(model._decode.args))
 
-    # ---- N > 1: the tensor-parallel path on the same ranks (SURVEY.md section 8e; `value` stays the replicas metric).
-    # 7B split N ways, and LLaMA-65B gptq.int4 TP = 8 (BASELINE.json configs[4]) when N = 8.  A watchdog ends the run with
+    # ---- N > 1: the tensor-parallel path on the same ranks (`value` stays the replicas metric).
+    # 7B split N ways, and LLaMA-65B gptq.int4 TP = 8 when N = 8.  A watchdog ends the run with
     # the headline line intact should a collective ever hang.
     tp = None
     if world > 1 and not args.no_tp:
@@ -557,7 +557,7 @@ def main():
         import tp_bench
 
         tp = {}
-        # the model that NEEDS the split first (BASELINE.json configs[4]); every model in its own try: shapes are the same
+        # the model that NEEDS the split first; every model in its own try: shapes are the same
         # on every rank, so a failure is symmetric and the next model still runs
         for name, steps in ([("65B", 64)] if world == 8 else []) + [("7B", 96)]:
             try:

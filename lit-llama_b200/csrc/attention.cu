@@ -263,7 +263,7 @@ __global__ void kv_unroll_kernel(const __nv_bfloat16* __restrict__ cache, const 
 // next one as soon as a buffer has been consumed.  A warp handles 4 keys per round: 8 lanes per key, 16 head
 // dims (32 B) per lane, a score needs 3 shuffles.  The new token's key / value never touch the tile: they are
 // rotated, appended to the cache and scored from registers.
-// Round 1 used one 128-key tile per CTA (64 KB, 3 CTAs per SM): at position 2047 its 512 CTAs needed a second
+// With one 128-key tile per CTA (64 KB, 3 CTAs per SM) the 512 CTAs of position 2047 needed a second
 // wave and 16 partials per head had to be merged (profiles/r01_ncu_attn_decode_fused_kernel.txt: 0.19 of HBM
 // peak); 256 keys per CTA keep every position a single wave (<= 8 x n_head CTAs) with half the partials.
 // ----------------------------------------------------------------------------------
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32)
   // K / V ring is idle now: every requested sub-tile has been consumed behind a __syncthreads), one warp turns the 32
   // running maxima into weights, 128 threads add.  Otherwise: the 4 key groups of a warp merge with shuffles first
   // (36 per warp), then the 8 warps through shared memory -- the default: measured 1.1 % faster per token at position
-  // 1030 on the same box (tools/env_sweep.sh "B2L_ATTN_SMEM_MERGE=0 B2L_ATTN_SMEM_MERGE=1").
+  // 1030 on the same box (tools/diag.py bench_ctx under B2L_ATTN_SMEM_MERGE=0 and =1).
   float* part = reinterpret_cast<float*>(fsm);                 // [32][HS]
   float* pm = part + 32 * HS;                                  // [32] running max, [32] sum, [32] weight, M, Ls
   float* pl = pm + 32, *pw = pl + 32;
@@ -610,8 +610,8 @@ __global__ void __launch_bounds__(FD_WARPS * 32)
 
 // ----------------------------------------------------------------------------------
 // Prefill / no-cache attention for head_size 128 and T > 1 (model.py:200-230 over many query positions): a tiled
-// online-softmax kernel on the tensor cores (mma.sync.m16n8k16 bf16, fp32 accumulate).  Round 1 gave every query row
-// its own CTA that re-read all its keys from L2 (13B, 8 x 512 tokens: 153 ms of a 315 ms prefill); here a CTA owns
+// online-softmax kernel on the tensor cores (mma.sync.m16n8k16 bf16, fp32 accumulate).  A CTA per query row
+// re-read all its keys from L2 (13B, 8 x 512 tokens: 153 ms of a 315 ms prefill); here a CTA owns
 // 64 query rows of one head (4 warps x 16 rows), streams 64-key K / V tiles through a double-buffered shared-memory
 // ring (cp.async, rows gathered through the cache ring), computes S = Q K^T and O += P V with ldmatrix-fed MMAs.
 // Scores are scaled and exponentiated in fp32; P enters the second MMA as bf16 hi + lo parts (2^-17 relative), so the

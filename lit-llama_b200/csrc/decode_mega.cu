@@ -5,7 +5,7 @@
 // -> [mlp.c_proj + residual] (model.py:156-168, 171-237, 240-254), ln_f + lm_head; and the roll branch of
 // model.py:214-218 as a ring offset.  The per-op kernels of api.cu remain the path for every other shape.
 //
-// Why one kernel (measured, DESIGN.md section 4): a 2 x 110 KB-per-SM streaming kernel cannot be co-resident with
+// Why one kernel (measured): a 2 x 110 KB-per-SM streaming kernel cannot be co-resident with
 // its successor, so programmatic dependent launch only overlaps kernel TAILS and every one of the 161 launches of a
 // token pays its own ring-fill latency (~2 us of idle HBM per launch at 7B).  Here one CTA per SM stays resident for
 // the whole token:

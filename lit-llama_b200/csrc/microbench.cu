@@ -236,7 +236,7 @@ extern "C" int b2l_debug_hmma_rate(void* out, int warps, int chains, int iters, 
 }
 
 // ---- legacy integer tensor pipe: how often can one SM sub-partition issue mma.sync.m16n8k32 u8 x s8 (IMMA.16832.U8.S8)?
-// Round-2 question: an int8 contraction consumes 512 weight nibbles per MMA (two packed words per lane) with at most
+// An int8 contraction consumes 512 weight nibbles per MMA (two packed words per lane) with at most
 // two LOP3 in front of it, against 256 nibbles and five ALU ops for the fp16 form.  n_alu = ALU ops issued per MMA.
 template <int CH>
 __global__ void __launch_bounds__(1024) imma_rate_kernel(unsigned long long* out, int iters, int n_alu, uint32_t seed) {
@@ -361,8 +361,8 @@ extern "C" int b2l_debug_consumer_rate(void* out, int warps, int iters, int mode
 
 // ---- what does a grid-wide dependency cost without a kernel boundary?  Every CTA (all co-resident) arrives on a
 // global counter with red.release and polls it with ld.acquire until all have arrived; out[r] = max over CTAs of
-// the nanoseconds between its arrival and its release, out[rounds + r] = min.  The persistent-kernel plan of
-// DESIGN.md section 7 replaces five kernel boundaries per Block with five of these.
+// the nanoseconds between its arrival and its release, out[rounds + r] = min.  The persistent kernel
+// (decode_mega.cu) replaces five kernel boundaries per Block with five of these.
 __global__ void __launch_bounds__(128) grid_flag_kernel(unsigned long long* out, unsigned int* counter, int rounds) {
   if (threadIdx.x != 0) return;
   for (int r = 0; r < rounds; ++r) {

@@ -25,10 +25,10 @@
 //
 // Why not tcgen05 here: one thread issues a 128x16x16 tcgen05.mma every ~55 cycles (4 issuing warps: 15 cycles,
 // profiles/r02_micro_issuers_gridflag.txt), but its A operand must first be expanded to 16-bit lanes by the same
-// ALUs (>= 4 LOP3 per packed word) and handed over through tensor memory (300-500 cycles per hand-off, DESIGN.md
-// section 3); the IMMA form needs 1 LOP3 per packed word and no hand-off.  tcgen05 carries the M > 8 shapes.
+// ALUs (>= 4 LOP3 per packed word) and handed over through tensor memory (300-500 cycles per
+// hand-off); the IMMA form needs 1 LOP3 per packed word and no hand-off.  tcgen05 carries the M > 8 shapes.
 //
-// Data movement is unchanged from round 1: a persistent CTA owns 16-row blocks over the FULL K, a producer warp
+// Data movement: a persistent CTA owns 16-row blocks over the FULL K, a producer warp
 // streams 16 KB stages with TMA bulk copies into an mbarrier ring (issued before griddepcontrol.wait, so the
 // weights of this linear stream while the previous kernel drains), 8 consumer warps split K inside a stage.
 //

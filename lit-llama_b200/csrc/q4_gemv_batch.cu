@@ -1,5 +1,5 @@
 // Batched decode kernel: fused [RMSNorm ->] int4 weight-only linear [-> residual | SwiGLU] for 2..8
-// activation rows (batched generation; BASELINE.json configs[3] decodes 8 sequences at once).
+// activation rows (batched generation, for instance 8 sequences at once).
 //
 // Same replacement as q4_gemv.cu (ColBlockQuantizedLinear.forward lit_llama/quantization.py:413-423 with the
 // RMSNorm of lit_llama/model.py:270-277 in front and x + h / silu(a) * b of model.py:166-167, 252 behind) and

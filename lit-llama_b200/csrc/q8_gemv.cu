@@ -16,7 +16,7 @@
 // and 32c + 16 + 4t..+3.
 //
 // parity: the arithmetic restates the published LLM.int8() algorithm (bitsandbytes is not in
-// the reference tree and not installed): parity with the reference is unpinned (DESIGN.md).
+// the reference tree and not installed): parity with the reference is unpinned.
 #include <cuda_fp16.h>
 
 #include "b2l_common.cuh"

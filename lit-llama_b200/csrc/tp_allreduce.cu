@@ -1,6 +1,6 @@
 // One-shot all-reduce (sum) of a bf16 activation row over the GPUs of one node, through peer memory (NVLink).
 //
-// Tensor-parallel decode (lit_llama_b200/tp.py; SURVEY.md section 8e -- the reference has no multi-GPU inference, the
+// Tensor-parallel decode (lit_llama_b200/tp.py -- the reference has no multi-GPU inference, the
 // split dims are those of scripts/convert_checkpoint.py:56-64) needs two sums per Block: after attn.c_proj and after
 // mlp.c_proj (the row-parallel linears), 8..16 KB each.  At that size a collective is pure latency, so this kernel is
 // built like NCCL's LL protocol but for exactly this case:

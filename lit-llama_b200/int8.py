@@ -8,7 +8,7 @@ are attributes of the parameter like in bitsandbytes.  The forward is the LLM.in
 algorithm on the tensor cores (csrc/q8_gemv.cu) - no bitsandbytes, no CPU path.
 
 bitsandbytes is not part of the reference tree (unpinned dependency, pyproject.toml:19), so the
-arithmetic follows the published algorithm (parity with the reference is unpinned, see DESIGN.md).
+arithmetic follows the published algorithm (parity with the reference is unpinned).
 """
 import torch
 

@@ -324,7 +324,7 @@ class LLaMA(nn.Module):
     copy_logits: bool = True
     #: batch-1 decode (head_size 128) as ONE persistent kernel per token (csrc/decode_mega.cu) instead of one kernel
     #: per op.  Opt-in (B2L_PERSISTENT=1): measured on B200 it is correct but slower than the per-op path under
-    #: programmatic dependent launch (DESIGN.md section 4: 1330 vs 964 us per 7B token).
+    #: programmatic dependent launch (1330 vs 964 us per 7B token).
     persistent: bool = os.environ.get("B2L_PERSISTENT", "0") == "1"
 
     def __init__(self, config: LLaMAConfig) -> None:

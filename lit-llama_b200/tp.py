@@ -1,4 +1,4 @@
-"""Tensor-parallel decode across GPUs of one node (SURVEY.md section 8e; new capability - the
+"""Tensor-parallel decode across GPUs of one node (new capability - the
 reference has no multi-GPU inference, every script is `L.Fabric(devices=1)`).
 
 Megatron-style sharding of the reference Block (split dims as recorded by the reference's own
@@ -123,7 +123,7 @@ class _TPDecodeState:
       -> all-reduce -> [rms_2 + c_fc1|c_fc2 (local columns) + SwiGLU] -> [mlp.c_proj (K = local columns) (+ residual on
       rank 0)] -> all-reduce; finally [ln_f + lm_head (local vocabulary rows)] -> all-gather.
     The residual enters the sum exactly once (rank 0's epilogue), so all-reduce(sum) leaves x + sum_r partial_r on every
-    rank (model.py:166-167).  Two all-reduces per Block (SURVEY section 7.6)."""
+    rank (model.py:166-167).  Two all-reduces per Block."""
 
     def __init__(self, m: "TPLLaMA", S: int, dev: torch.device, idx_dtype: torch.dtype) -> None:
         cfg, lib = m.config, L.lib()

@@ -1,13 +1,13 @@
 """CPU oracle for the lit-llama quantized decode path.  TEST INFRASTRUCTURE ONLY.
 
 This module restates, on the CPU, the arithmetic of the reference hot path
- as plain functions over torch CPU tensors.  It exists to
+as plain functions over torch CPU tensors.  It exists to
 *check* the CUDA path; nothing under `lit-llama_b200/` may import it.  Only
 `tests/`, `__graft_entry__.smoke()` and the `cpu_baseline` / `--impl reference`
 legs of `bench.py` use it.
 
-Pinning: the reference's own tests hold no golden vectors for quantization.py
-(SURVEY.md section 8c); the pin is therefore the reference itself, executed in the
+Pinning: the reference's own tests hold no golden vectors for quantization.py;
+the pin is therefore the reference itself, executed in the
 build container by `oracle/make_golden.py`, whose outputs are committed under
 `tests/golden/` and compared against this restatement by
 `tests/test_oracle_golden.py`.  The gptq.int4/int8 + model.py + generate.py part
@@ -367,7 +367,7 @@ def generate(model, idx: Tensor, max_new_tokens: int, *, max_seq_length: Optiona
 
 
 # ----------------------------------------------------------------------------
-# Synthetic weights (SURVEY.md section 8d) - shared by tests, smoke and bench
+# Synthetic weights - shared by tests, smoke and bench
 # ----------------------------------------------------------------------------
 def synth_state_dict(n_layer: int, n_head: int, n_embd: int, vocab_size: int, mode: Optional[str],
                      dtype=torch.bfloat16, seed: int = 1234, tile_cols: int = -1) -> Dict[str, Tensor]:

@@ -251,7 +251,7 @@ def test_7b_shaped_block_vs_oracle(dev):
 
 
 def test_13b_width_batch8_prefill_and_decode_vs_oracle(dev):
-    """BASELINE.json configs[3] in small: two Blocks at the LLaMA-13B widths (n_embd 5120, 40 heads of 128, n_hidden
+    """Batched 13B generation in small: two Blocks at the LLaMA-13B widths (n_embd 5120, 40 heads of 128, n_hidden
     13824), batch 8: prefill 32 tokens per sequence (tcgen05 GEMM at M = 256, tensor-core prefill attention), then 4
     decode steps (2..8-row mma.sync kernel, fused attention, CUDA graph from the third step), every logits tensor and
     the KV cache against the oracle in exact arithmetic."""

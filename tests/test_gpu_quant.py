@@ -1,7 +1,7 @@
 """-m gpu: the quantized linears through the C ABI against the oracle / golden vectors.
 
 Bars: integer work (unpack, dequant in a given dtype, re-tiling) bit-exact; linear outputs
-normwise within 1e-3 of exact arithmetic (north_star) and within the reference's own bf16
+normwise within 1e-3 of exact arithmetic and within the reference's own bf16
 tolerance (tests/test_model.py:133) of the reference's CPU forward."""
 import pytest
 import torch

@@ -183,7 +183,7 @@ def test_empty_init_on_device_and_lazy_load(tmp_path):
 
 
 def test_weight_changes_bump_the_generation_and_compact_refuses_what_it_cannot_serve():
-    """Host logic behind two round-2 features, no kernels involved: (1) load_state_dict / pack_weight / .to() bump the
+    """Host logic behind two features, no kernels involved: (1) load_state_dict / pack_weight / .to() bump the
     generation counter that invalidates baked decode states (lit_llama_b200/model.py); (2) compact() /
     release_reference_layout() refuse models and layers the batch-1 decode tiling cannot represent instead of
     freeing their only copy."""

@@ -442,7 +442,7 @@ def sec_mma_rate():
 
 
 def sec_mma_issuers():
-    """tcgen05.mma issue from 1..4 threads of one CTA at once (round-2 question: does a multi-issuer kernel scale?)."""
+    """tcgen05.mma issue from 1..4 threads of one CTA at once (does a multi-issuer kernel scale?)."""
     import torch
     from lit_llama_b200 import _lib as L
 
@@ -706,7 +706,7 @@ def _decode_us(model, B, S, dev, p0=512, n=24):
 
 
 def sec_bench_13b_b8():
-    """BASELINE.json configs[3]: LLaMA-13B gptq.int4, batch 8, prefill 512 then decode (ctx 2048)."""
+    """LLaMA-13B gptq.int4, batch 8, prefill 512 then decode (ctx 2048)."""
     import torch
     from bench import build_synthetic_model
 

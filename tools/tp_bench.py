@@ -1,4 +1,4 @@
-"""Tensor-parallel batch-1 decode throughput on N GPUs of one node:
+"""Tensor-parallel batch-1 decode throughput on N GPUs of one node (LLaMA-65B split 8 ways, 7B):
 
     python -m torch.distributed.run --nnodes=1 --nproc-per-node 8 --master-addr 127.0.0.1 --master-port 29533 \
         tools/tp_bench.py --model 65B [--steps 64] [--warmup 8]
