@@ -143,9 +143,10 @@ enum {
 int b2l_q4_linear_tc(const b2l_q4_linear_args* args, b2l_stream_t stream);
 
 /* Prefill-shaped linear (any M; meant for M > 16): y[M, N] = x[M, K] . dequant(W)^T on tcgen05 (csrc/q4_gemm.cu):
- * 256 x 256 output tile per CTA, both operands from shared memory (producer warps dequantise the packed levels with
- * the reference's own bf16 roundings, so the tensor core multiplies exactly get_weight()'s matrix), fp32 accumulators
- * in tensor memory.  Same argument block as b2l_q4_linear_tc; qw_tiled from b2l_q4_tile; prologue / epilogue must be
+ * 128 output features x 16..256 tokens per CTA, the weight as the 128-row operand in tensor memory (dequantised with the
+ * reference's own bf16 roundings, so the tensor core multiplies exactly get_weight()'s matrix), fp32 accumulators beside it.
+ * Where the tiles are few a cluster of 2..8 CTAs splits K and adds its f32 sums in rank order; whether depends on M, N
+ * and K, so the last bits of a row may depend on how many rows there are.  Same argument block as b2l_q4_linear_tc; qw_tiled from b2l_q4_tile; prologue / epilogue must be
  * NONE / STORE; K % 64 == 0; ldx % 8 == 0.  Replaces quantization.py:187-333 (Triton tile kernel) / :413-423. */
 int b2l_q4_gemm(const b2l_q4_linear_args* args, b2l_stream_t stream);
 

@@ -206,7 +206,6 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
   }
 }
 
-// state <- the last taps-1 inputs after T >= taps-1 new tokens (multi-tile launches only).
 // Four taps over long portions in bf16: a thread owns 8 neighbouring channels (16-byte loads, two 16-byte stores) and CONV_VT tokens, so the
 // bytes in flight suffice for HBM (6144 channels x 2048 tokens: 39 us, 73 one channel at a time); sums in the order of the kernel above.
 constexpr int CONV_VT = 16, CONV_V = 8;
@@ -267,6 +266,7 @@ __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16
   }
 }
 
+// state <- the last taps-1 inputs after T >= taps-1 new tokens (multi-tile launches only).
 template <typename act_t>
 __global__ void seq_conv_state_kernel(const act_t* __restrict__ in, int ldin, act_t* __restrict__ state,
                                       const int* __restrict__ meta, int T, int C, int taps) {

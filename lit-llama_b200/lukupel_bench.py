@@ -96,7 +96,7 @@ def kernel_table(model, engine, T: int, device, timer, peaks: dict) -> List[dict
                            cache_v=M._p(ctx.state[att.name + ".v"]), meta=M._p(meta), out=M._p(out), ldo=H * V, scale=att.scale, out_mult=1.0, block=ring, T=tt,
                            heads=H, kv_heads=G, K=K, V=V, act_dtype=act, **kw)
             t = timer(lambda: M.local_attention(b, ctx))
-            add(name, tt, t, nb, 2.0 * tt * H * keys * (K + V), f"f32 scores on CUDA cores, {keys:.0f} keys per query")
+            add(name, tt, t, nb, 2.0 * tt * H * keys * (K + V), f"f32 scores, {keys:.0f} keys per query")
         t = timer(lambda: att.forward(hh, ctx))
         wb = (att.w_in.numel() + att.w_o.numel()) * es
         add("LocalAttention whole (2 products + operands + attention)", tt, t, wb + 2 * tt * D * es, 2.0 * tt * H * keys * (K + V) + 2.0 * tt * wb / es)

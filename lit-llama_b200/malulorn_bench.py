@@ -103,7 +103,7 @@ def kernel_table(model, engine, T: int, device, timer, peaks: dict) -> List[dict
             a2 = S.AttnArgs(q=p(q), k_new=p(kn), v_new=p(proj, att.o_v), ldv=ld, cache_k=p(ctx.state[att.name + ".k"]), cache_v=p(ctx.state[att.name + ".v"]),
                             meta=p(meta), gate=p(proj, att.o_g), ldg=ld, out=p(out), ldo=H * V, scale=att.scale, out_mult=1.0, has_sink=1, block=ring, T=tt, heads=H,
                             kv_heads=G, K=K, V=V, act_dtype=act, **kw)
-            add(name, tt, timer(lambda: M.local_attention(a2, ctx)), nb, 2.0 * tt * H * keys * (K + V), f"f32 scores on CUDA cores, {keys:.0f} keys per query")
+            add(name, tt, timer(lambda: M.local_attention(a2, ctx)), nb, 2.0 * tt * H * keys * (K + V), f"f32 scores, {keys:.0f} keys per query")
         wb = (att.w_in.numel() + att.w_o.numel()) * es
         add("LocalAttention whole (2 products + operands + attention)", tt, timer(lambda: att.forward(hh, ctx)), wb + 2 * tt * D * es,
             2.0 * tt * H * keys * (K + V) + 2.0 * tt * wb / es)
@@ -179,7 +179,7 @@ def latent_rows(model, lat, ctx, tt: int, pos0: int, keys: float, timer, hbm: fl
                   n_a=dv + dn, score_off=dv, heads_per_group=1, **shared_b)
         fl, nb = 2.0 * tt * H * keys * (dq + dv), n_keys * (H * (dv + dn) + dr) * es + tt * H * (dq * 4 + dv * es)
         t = timer(lambda: lat._attend(ctx, out, dv, splits, **gate, **kw))
-        add("seq_latent_attention_kernel (expanded form, gate per channel)", t, nb + tt * H * dv * 4, fl, f"f32 scores on CUDA cores, {splits} key split(s)")
+        add("seq_latent_attention_kernel (expanded form, gate per channel)", t, nb + tt * H * dv * 4, fl, f"f32 scores, {splits} key split(s)")
         lat.sink = sink
         t = timer(lambda: lat._attend(ctx, out, dv, splits, **kw))
         lat.sink = None

@@ -4,7 +4,7 @@
 (names, shapes, dtypes, strides) and `state_dict` keys (quantization.py:340-374), so a
 `llama-gptq.4bit.pth` produced by the reference's quantize/gptq.py loads unchanged.
 `forward` runs hand-written sm_100a kernels through the C ABI of include/b2l.h (M = 1: exact int8-digit MMA GEMV;
-2..8: f16 MMA batch kernel; 9..16: tcgen05 from tensor memory; > 16: tcgen05 256 x 256 tile GEMM); there is no
+2..8: f16 MMA batch kernel; 9..16: tcgen05 from tensor memory; > 16: tcgen05 GEMM with the weight in tensor memory); there is no
 Triton, no library GEMM, no dense fallback and no CPU path.
 """
 import ctypes as C

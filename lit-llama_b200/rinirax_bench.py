@@ -130,7 +130,7 @@ def kernel_table(model, engine, T: int, device, timer, peaks: dict) -> List[dict
         t = timer(lambda: M.local_attention(bA, ctx))
         nb = tt * (H * 2 * K * 4 + G * (2 * K + V) * es * 2 + H * V * es) + (keys * G * (2 * K + V) * es if tt == 1 else 0)
         add("seq_block_attention (2 maps per head + differential read-out) + append", tt, t, nb, 2.0 * tt * 2 * H * keys * (K + V),
-            f"f32 scores on CUDA cores, {keys:.0f} keys per query")
+            f"f32 scores, {keys:.0f} keys per query")
         t = timer(lambda: S.check(lib.b2l_seq_diff_combine(M._p(maps), H * 2 * V, att.lam, eps, 1.0 - att.diff, M._p(y), H * V, tt, H, V, ctx.act, ctx.stream), "k"))
         add("  seq_diff_combine_kernel alone (the read-out as a kernel of its own: prompt portions)", tt, t, tt * H * V * (8 + es))
         gate = torch.randn(tt, H, device=device).to(dt)
@@ -176,7 +176,7 @@ def kernel_table(model, engine, T: int, device, timer, peaks: dict) -> List[dict
                                               heads_per_group=Hl, **shared_b))
                 fl, form = 2.0 * tt * Hl * kq * (2 * rk + dr), "latent"
                 nbl = kq * Kd * es + tt * Hl * (Kd * 4 + rk * es)
-            add(f"{name}, {form} form)", tt, t, nbl, fl, f"f32 scores on CUDA cores, {kq:.0f} keys per query, {splits} key split(s)")
+            add(f"{name}, {form} form)", tt, t, nbl, fl, f"f32 scores, {kq:.0f} keys per query, {splits} key split(s)")
         lat.window, lat.sink = Wn, None
         t = timer(lambda: lat.forward(hh, ctx))
         wb = (lat.w_in.numel() + lat.w_uq.numel() + lat.w_uk.numel() + lat.w_uv.numel() + lat.w_o.numel()) * es

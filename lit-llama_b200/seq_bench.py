@@ -250,7 +250,7 @@ def kernel_table(model, engine, T: int, device, timer: _Timer, peaks: dict) -> L
                 nb = tt * (att.H * att.K * (es + 4) + att.G * (att.K + att.V) * es * 3 + att.H * att.V * es) + \
                     (min(T, att.block) * att.G * (att.K + att.V) * es if tt == 1 else 0)
                 add("attention branch (2 x seq_headnorm_rope + seq_block_attention + seq_ring_append)", "b2l_attention (prefill: mma.sync tiles)", t, nb, fl,
-                    "f32 scores on CUDA cores")
+                    "f32 scores")
                 t = timer(lambda: gla.run(proj, mx.offs[4:], ctx, out, mx.widths[0], 1.0))
                 st = gla.H * gla.K * gla.V * 4 * 2
                 add("linear-attention branch (product + seq_decay + seq_scan + seq_group_norm_gate)", "-", t, st + tt * gla.H * (3 * gla.K + 2 * gla.V) * 4,

@@ -124,7 +124,7 @@ def kernel_table(model, engine, T: int, device, timer, peaks: dict) -> List[dict
             nb = n_keys * Kd * es + tt * H * (Kd * 4 + rk * es)
         add("seq_latent_attention_kernel (" + ("expanded" if expanded else "latent") + " form)",
             "seq_block_attention_tile_kernel" if tt > 1 else "seq_block_attention_kernel", tt, t, nb, fl,
-            f"f32 scores on CUDA cores, {splits} key split(s)")
+            f"f32 scores, {splits} key split(s)")
         t = timer(lambda: att.forward(hh, ctx))
         wb = (att.w_in.numel() + att.w_uq.numel() + att.w_uk.numel() + att.w_uv.numel() + att.w_o.numel()) * es
         add("LatentAttention whole (5 products + prep + rotation + attention)", "attention branch", tt, t, wb + nb, fl + 2.0 * tt * wb / es)

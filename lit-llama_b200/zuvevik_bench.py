@@ -147,7 +147,7 @@ def kernel_table(model, engine, T: int, device, timer, peaks: dict) -> List[dict
                            kv_heads=G, K=K, V=V, act_dtype=ctx.act, window=window, gate_per_channel=per_channel)
             t = timer(lambda: M.local_attention(b, ctx))
             nb = tt * (H * K * 4 + G * (K + V) * es * 2 + H * V * es * (2 if per_channel else 1)) + (kq * G * (K + V) * es if tt == 1 else 0)
-            add(name, tt, t, nb, 2.0 * tt * H * kq * (K + V), f"f32 scores on CUDA cores, {kq:.0f} keys per query")
+            add(name, tt, t, nb, 2.0 * tt * H * kq * (K + V), f"f32 scores, {kq:.0f} keys per query")
         t = timer(lambda: att.forward(hh, ctx))
         wb = (att.w_in.numel() + att.w_o.numel()) * es
         add("SlidingWindowAttention whole (2 products + operands + attention)", tt, t, wb + 2 * tt * D * es, 2.0 * tt * H * keys * (K + V) + 2.0 * tt * wb / es)
