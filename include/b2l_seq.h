@@ -130,6 +130,9 @@ int b2l_seq_scan_chunks(int T, int delta);
 /* Floats of work_state with which a portion with n_chunks <= 1 runs 16 tokens at a time where its sizes allow it (0: too short); step by step
  * with work_state null.  The space of a portion with n_chunks > 1 serves as well where it is as large. */
 long long b2l_seq_scan_work_floats(int T, int heads);
+/* The fastest form for these sizes (vscale: whether a value scale is given): sets *n_chunks and returns the floats of work_state it wants (0: none,
+ * step by step).  work_decay is wanted where *n_chunks > 1: n_chunks * heads * (per_channel ? K : 1) floats. */
+long long b2l_seq_scan_plan(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks);
 int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream);
 
 /* Read-out of a recurrence: groups of `group` consecutive channels of o (f32 [T, n]) are divided by their root

@@ -674,12 +674,30 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
   }
 }
 
+constexpr int SCAN_CHUNK = 128;      // tokens per chunk of a chunked portion (a multiple of SCAN_TC)
+
+static bool walk_sizes(int T, int K, int V, int ones) { return T >= 2 * CH_C && (K == 64 || K == 128) && V % CH_VT == 0 && !ones; }
+// Where the walk is the faster form.  Against the step-by-step form (0.35 us per token): from 48 tokens on where every CTA of the walk has an SM
+// of its own (16 heads of 128 x 128, 48 tokens: 20..26 against 27..29 us; 32 tokens: 17..24 against 21..23), from 64 on otherwise (64 heads of
+// 64 x 64, 33 tokens: 26..30 against 21..23; 64 tokens: 28..32 against 35..39).  Against the chunked form without the delta rule, which
+// stays flat until its CTAs fill the SMs while the walk takes 1.3 us (1.0 with 64 keys) per 16 tokens and turn of CTAs whatever the heads:
+// both times from the fits below, in ns (128 x 128, us walk / chunked: 1024 tokens of 4 heads 95 / 103; 2048 of 4 173 / 130, of 8 179 / 240;
+// 4096 of 4 333 / 251, of 8 345 / 388; 8192 of 1 634 / 134, of 8 673 / 667, of 16 710 / 1285).
+static bool walk_pays(int T, int heads, int K, int V, int delta) {
+  const long long sms = sm_count(), ctas = (long long)heads * (V / CH_VT), turns = (ctas + sms - 1) / sms;
+  if (T < (turns <= 1 ? 48 : 64)) return false;
+  if (delta || T < 2 * SCAN_CHUNK) return true;
+  const long long cols = K == 64 ? 64 : 32, chunked = (V + cols - 1) / cols * heads * ((T + SCAN_CHUNK - 1) / SCAN_CHUNK), load = (chunked + sms - 1) / sms;
+  const long long t_chunked = load == 1 ? 104000 : load == 2 ? 131000 : 60000 + 45000 * load, t_walk = 15000 + (long long)(T / CH_C) * (K == 64 ? 1050 : 1350) * turns;
+  return t_walk <= t_chunked;
+}
 // Portions of two chunks or more with key sizes 64 or 128 and whole groups of 16 values, given room for the chunks' matrices; other sizes, the
-// column of ones and single tokens go step by step.
+// column of ones and single tokens go step by step.  A caller that asks for the chunked form gets the walk where it is faster and its space
+// suffices.
 static bool walk_chunks(const b2l_seq_scan_args* a) {
   const size_t chunks = ((size_t)a->T + CH_C - 1) / CH_C;
-  const bool room = a->n_chunks <= 1 || (size_t)a->n_chunks * a->V * a->K >= chunks * 2 * CH_MAT;      // a caller's space for the three-pass form
-  return a->work_state != nullptr && room && a->T >= 2 * CH_C && (a->K == 64 || a->K == 128) && a->V % CH_VT == 0 && !a->ones &&
+  const bool wanted = a->n_chunks <= 1 || ((size_t)a->n_chunks * a->V * a->K >= chunks * 2 * CH_MAT && walk_pays(a->T, a->heads, a->K, a->V, a->delta));
+  return a->work_state != nullptr && wanted && walk_sizes(a->T, a->K, a->V, a->ones) &&
          (!a->delta || (a->decay_per_channel && !a->vscale)) && ((uintptr_t)a->state & 15) == 0 && ((uintptr_t)a->work_state & 15) == 0 && a->heads <= 65535;
 }
 
@@ -697,7 +715,6 @@ static int launch_walk(const b2l_seq_scan_args* a, cudaStream_t s) {
 }
 
 static DynSmemCache g_scan_smem[10];
-constexpr int SCAN_CHUNK = 128;      // tokens per chunk of a chunked portion (a multiple of SCAN_TC)
 
 }  // namespace b2l
 
@@ -710,6 +727,15 @@ extern "C" int b2l_seq_scan_chunks(int T, int delta) {
 
 extern "C" long long b2l_seq_scan_work_floats(int T, int heads) {
   return T < 2 * CH_C || heads <= 0 ? 0 : (long long)((T + CH_C - 1) / CH_C) * heads * (2 * CH_MAT);
+}
+
+extern "C" long long b2l_seq_scan_plan(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks) {
+  if (n_chunks) *n_chunks = 1;
+  if (T <= 0 || heads <= 0 || K <= 0 || V <= 0) return 0;
+  if (walk_sizes(T, K, V, ones) && (!delta || (per_channel && !vscale)) && heads <= 65535 && walk_pays(T, heads, K, V, delta)) return b2l_seq_scan_work_floats(T, heads);
+  const int n = b2l_seq_scan_chunks(T, delta);
+  if (n_chunks) *n_chunks = n;
+  return n > 1 ? (long long)n * heads * (V + (ones ? 1 : 0)) * K : 0;
 }
 
 extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {

@@ -172,14 +172,13 @@ class DenseMLP:
 def _scan(ctx: StepContext, *, q, ldq, k, ldk, v, ldv, q_mult, decay, ldd, per_channel, state, out, ldo, heads, qk_heads,
           K, V, beta=None, ldb=0, vscale=None, ldvs=0, skip=None, state_ones=None, out_ones=None) -> None:
     lib = S.lib()
-    n_chunks = lib.b2l_seq_scan_chunks(ctx.T, int(beta is not None))
-    ws = wd = None
-    if n_chunks > 1:      # long portion, no delta rule: chunks in parallel (local states, combine, outputs)
-        ws = torch.empty((n_chunks, heads, V + int(state_ones is not None), K), dtype=torch.float32, device=state.device)
-        wd = torch.empty((n_chunks, heads, K if per_channel else 1), dtype=torch.float32, device=state.device)
-    elif state_ones is None:  # 16 tokens at a time
-        n = lib.b2l_seq_scan_work_floats(ctx.T, heads)
+    n_chunks, ws, wd = 1, None, None
+    if ctx.T > 1:         # 16 tokens at a time, or (long portion, few heads, no delta rule) chunks in parallel: local states, combine, outputs
+        chunks = C.c_int(1)
+        n = lib.b2l_seq_scan_plan(ctx.T, heads, K, V, int(per_channel), int(beta is not None), int(state_ones is not None), int(vscale is not None), C.byref(chunks))
+        n_chunks = chunks.value
         ws = torch.empty((n,), dtype=torch.float32, device=state.device) if n else None
+        wd = torch.empty((n_chunks, heads, K if per_channel else 1), dtype=torch.float32, device=state.device) if n_chunks > 1 else None
     a = S.ScanArgs(q=q, ldq=ldq, k=k, ldk=ldk, v=v, ldv=ldv, q_mult=float(q_mult), decay=decay, ldd=ldd,
                    decay_per_channel=int(per_channel), beta=beta, ldb=ldb, delta=int(beta is not None), vscale=vscale, ldvs=ldvs,
                    skip=skip, state=_p(state), meta=_p(ctx.meta), out=out, ldo=ldo, T=ctx.T, heads=heads, qk_heads=qk_heads, K=K, V=V,

@@ -251,3 +251,35 @@ def test_attention_operands_of_very_wide_heads(rot):
         u, v = src.double()[:, :rot // 2], src.double()[:, rot // 2:]
         want = torch.cat([u * ang.cos() - v * ang.sin(), v * ang.cos() + u * ang.sin()], 1)
         assert float((got - want).abs().max()) < 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("T,H,K,V,want", [(2048, 4, 128, 128, "chunks"), (2048, 8, 64, 64, "chunks"), (300, 1, 128, 16, "walk"), (2048, 16, 128, 128, "walk"), (257, 64, 128, 64, "walk"),
+                                          (47, 2, 64, 32, "steps"), (48, 2, 64, 32, "walk"), (63, 64, 64, 64, "steps"), (64, 64, 64, 64, "walk")])
+def test_scan_plan_and_its_neighbours(T, H, K, V, want):
+    """The planned form of a scan without the delta rule (148 SMs) and the forms it was chosen over: the same outputs and state up to the order
+    of f32 sums (2048 decayed terms, 1e-6 of the norm)."""
+    from lit_llama_b200 import _seqlib as S
+
+    lib, g = S.lib(), torch.Generator(device=DEV).manual_seed(T + H)
+    q, k, v = (torch.randn(T, H, n, generator=g, device=DEV) for n in (K, K, V))
+    a, state0 = torch.rand(T, H, K, generator=g, device=DEV) * 0.3 + 0.7, torch.randn(1, H, V, K, generator=g, device=DEV)
+    meta, n_chunks = torch.zeros(2, dtype=torch.int32, device=DEV), C.c_int(0)
+    n = lib.b2l_seq_scan_plan(T, H, K, V, 1, 0, 0, 0, C.byref(n_chunks))
+    assert want == ("chunks" if n_chunks.value > 1 else "walk" if n else "steps")
+    assert want != "walk" or n == lib.b2l_seq_scan_work_floats(T, H)
+    assert lib.b2l_seq_scan_plan(T, H, K, V, 0, 1, 0, 0, C.byref(n_chunks)) == 0 and n_chunks.value == 1      # delta rule, one decay per head: step by step
+
+    def run(chunks, floats):
+        out, state, ws = torch.empty(T, H, V, device=DEV), state0.clone(), torch.full((max(floats, 1) + 64,), 3.0, device=DEV)
+        wd = torch.empty(chunks * H * K, device=DEV)
+        args = S.ScanArgs(q=q.data_ptr(), ldq=H * K, k=k.data_ptr(), ldk=H * K, v=v.data_ptr(), ldv=H * V, q_mult=1.0, decay=a.data_ptr(), ldd=H * K, decay_per_channel=1,
+                          state=state.data_ptr(), meta=meta.data_ptr(), out=out.data_ptr(), ldo=H * V, T=T, heads=H, qk_heads=H, K=K, V=V, act_dtype=S.act_code(torch.float32),
+                          work_state=ws.data_ptr() if floats else None, work_decay=wd.data_ptr(), n_chunks=chunks)
+        S.check(lib.b2l_seq_scan(C.byref(args), S.stream_ptr()), "scan")
+        assert bool((ws[floats:] == 3).all()) or not floats
+        return out, state
+
+    out, state = run(1, 0)
+    lib.b2l_seq_scan_plan(T, H, K, V, 1, 0, 0, 0, C.byref(n_chunks))
+    for got, st in (run(n_chunks.value, n), run(1, lib.b2l_seq_scan_work_floats(T, H))):
+        assert rel(got, out) < 1e-6 and rel(st, state) < 1e-6
