@@ -144,7 +144,7 @@ constexpr int MOST_PAIRS = 4096;      // rotated pairs whose cos and sin fit the
 //   the sum of squares is taken from the entries before it.
 //   q_out is multiplied by the query temperature of its position when temp_every > 0.
 //   v_out (act): (1 - lambda) v + lambda v_first when v_first is given (lambda read on the device), else not written.
-template <typename act_t>
+template <typename act_t, bool TABLE>      // TABLE: up to MOST_PAIRS pairs
 __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args a, int quads) {
   __shared__ float red[32];
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -154,8 +154,7 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
   const float temp = a.temp_every > 0 ? 1.0f + a.temp_coef * logf((float)((a.meta[1] + t + 1) / a.temp_every + 1)) : 1.0f;
   // every head turns by the same angles: once per token instead of once per head (16 + 4 heads, 2048 tokens: 29 -> 27 us)
   extern __shared__ float turn[];                       // cos | sin of the pairs, times rot_mult
-  const bool table = half <= MOST_PAIRS;
-  for (int i = threadIdx.x; table && i < half; i += blockDim.x) {
+  for (int i = threadIdx.x; TABLE && i < half; i += blockDim.x) {
     float s, c;
     sincosf(pos * a.freq[i], &s, &c);
     turn[i] = c * a.rot_mult;
@@ -240,8 +239,8 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
       for (int i = lane; i < half; i += 32) {
         const float u = ld_act(p, i) * r * (wh ? ld_act(wh, i) : 1.f);
         const float v = ld_act(p, i + half) * r * (wh ? ld_act(wh, i + half) : 1.f);
-        float s, c;
-        if (table) {
+        float c, s;
+        if constexpr (TABLE) {
           c = turn[i];
           s = turn[half + i];
         } else {
@@ -369,7 +368,10 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   const bool table = a->rot_dims / 2 <= MOST_PAIRS;
   const int quads = table && a->act_dtype == B2L_BF16 && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
                     a->k_off % 4 == 0 && a->ld % 4 == 0 && al8(a->proj) && al8(a->q_norm) && al8(a->k_norm) && al16(a->q_out) && al8(a->k_out);
-  B2L_SEQ_DISPATCH(a->act_dtype, (seq_qkv_prep_kernel<act_t><<<a->T, 256, table ? sizeof(float) * a->rot_dims : 0, (cudaStream_t)stream>>>(*a, quads)));
+  B2L_SEQ_DISPATCH(a->act_dtype, {
+    if (table) seq_qkv_prep_kernel<act_t, true><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a, quads);
+    else seq_qkv_prep_kernel<act_t, false><<<a->T, 256, 0, (cudaStream_t)stream>>>(*a, quads);
+  });
   B2L_LAUNCH_CHECK("seq_qkv_prep_kernel");
   return 0;
 }
