@@ -42,45 +42,9 @@ struct Params {
   int expired;             // cluster rank that ends as if its last wait had run out, or -1
 };
 
-__device__ __forceinline__ uint32_t elect_lane() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t lead) {
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-               "r"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
-               : "memory");
-}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t a, const uint32_t (&r)[16]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(a), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_dsmem(uint32_t addr, uint32_t rank) {
-  uint32_t a;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t addr, uint32_t rank) {
-  uint32_t a, v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-
 __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * MAX_STAGES + 2];
@@ -232,8 +196,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
         for (int s = 0; s < p.splits; ++s) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float4 u = ld_dsmem(sbase + (uint32_t)(b * BN + row) * 64 + 16 * ((c + (row >> 1)) & 3), (uint32_t)s);
-            v[4 * c] += u.x; v[4 * c + 1] += u.y; v[4 * c + 2] += u.z; v[4 * c + 3] += u.w;
+            const uint4 u = ld_dsmem(sbase + (uint32_t)(b * BN + row) * 64 + 16 * ((c + (row >> 1)) & 3), (uint32_t)s);
+            v[4 * c] += __uint_as_float(u.x); v[4 * c + 1] += __uint_as_float(u.y); v[4 * c + 2] += __uint_as_float(u.z); v[4 * c + 3] += __uint_as_float(u.w);
           }
         }
       }

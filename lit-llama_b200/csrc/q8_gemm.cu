@@ -160,37 +160,11 @@ struct Params {
   int M, N, K, Mp, ldx, ldy, bt, nst, splits;
 };
 
-// The whole warp runs the issuing loop, so descriptors stay in uniform registers (issued from one lane's branch an MMA took twice its time).
-__device__ __forceinline__ uint32_t elect_lane() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc, uint32_t lead) {
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a),
                "l"(b), "r"(idesc), "r"(acc), "r"(lead)
                : "memory");
 }
-__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ int4 ld_dsmem(uint32_t addr, uint32_t rank) {
-  uint32_t a;
-  int4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t addr, uint32_t rank) {
-  uint32_t a, v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-
 __global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 2];
@@ -318,8 +292,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_const
         for (int s = 0; s < p.splits; ++s) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const int4 v = ld_dsmem(sbase + (uint32_t)(b * BN + row) * 64 + 16 * ((c + (row >> 1)) & 3), (uint32_t)s);
-            t[4 * c] += v.x; t[4 * c + 1] += v.y; t[4 * c + 2] += v.z; t[4 * c + 3] += v.w;
+            const uint4 v = ld_dsmem(sbase + (uint32_t)(b * BN + row) * 64 + 16 * ((c + (row >> 1)) & 3), (uint32_t)s);
+            t[4 * c] += (int)v.x; t[4 * c + 1] += (int)v.y; t[4 * c + 2] += (int)v.z; t[4 * c + 3] += (int)v.w;
           }
         }
       }
