@@ -244,6 +244,9 @@ static Plan plan_for(int M, int N, int K) {
   best.smem = best.nst * stage + 1024;
   const size_t part = (size_t)BN * best.bt * 4 + 1024;
   if (best.splits > 1 && part > best.smem) best.smem = part;
+  // One CTA per SM by its shared memory, whatever its registers: each takes all of tensor memory, and a CTA of a cluster that waited for another's
+  // would wait for good if that one waits for it at the cluster's barrier.
+  if (best.smem < 120 * 1024) best.smem = 120 * 1024;
   return best;
 }
 
