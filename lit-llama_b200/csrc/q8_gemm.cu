@@ -366,7 +366,10 @@ static Plan plan_for(int M, int N, int K) {
   q.splits = 1;
   while (q.splits < 8 && tiles * q.splits * 2 <= sm_count() && K / BK / (q.splits * 2) >= 4) q.splits *= 2;
   const size_t stage = A_BYTES + (size_t)q.bt * BK;
-  const size_t budget = q.bt <= 128 ? 108 * 1024 : 200 * 1024;       // two CTAs per SM for narrow tiles: one's epilogue under the other's loads
+  // Two CTAs per SM for tiles of up to 128 tokens, one's epilogue under the other's loads: half of an SM's 228 KB less the 1 KB the system
+  // keeps per CTA, the static arrays and the alignment of the stages.  Wider tiles take one.
+  constexpr size_t STATIC = sizeof(__half) * SM_OUT * 256 + sizeof(float) * 256 + 8 * (2 * MAX_STAGES + 4);
+  const size_t budget = q.bt <= 128 ? 114 * 1024 - 1024 - STATIC - 1024 : 200 * 1024;
   q.nst = (int)(budget / stage);
   if (q.nst > MAX_STAGES) q.nst = MAX_STAGES;
   q.smem = q.nst * stage + 1024;
