@@ -1,8 +1,11 @@
 // Prompt attention on tcgen05 with f32 scores and weights: 128 query rows of one head against tiles of 64 keys.
 //
 // Keys and values are bf16.  A query in f32 is cut into NQ = 3 bf16 parts that add up to it exactly (8 bits each, by truncation), and so is
-// every softmax weight (NP = 3): the products of the parts with bf16 keys or values are exact, the tensor core adds them in f32, so
-// the result is that of an f32 kernel up to the order of the sums.  Three bf16 MMAs cost 3 / 16 of what one f32 FMA costs on the CUDA cores.
+// every softmax weight (NP = 3): the products of the parts with bf16 keys or values are exact, and the tensor core adds them in f32, but it
+// truncates where an f32 add rounds: left in the accumulator, the output's error grew with the keys as a bias towards zero (1024 keys 1.6e-6 of
+// the norm, 2048 keys 7e-6, 4096 keys with values of mean 2 2.4e-5; the f32 kernel 4e-7, 9e-7 and 7e-7).  So (REGS) every tile's product
+// starts from zero and is added to f32 registers: 2.3e-7, 3.2e-7 and 1.2e-7 in these cases, below the f32 kernel in every size measured.
+// Three bf16 MMAs cost 3 / 32 of what the f32 FMAs cost on the CUDA cores (4096 against 128 per cycle).
 //
 //   warp 0       issues the MMAs: S(t+2) = Q K^T goes behind O += P(t) V
 //   warps 1, 2   keys, warps 3, 12 values, into 128-byte swizzled rows (keys K-major, values MN-major for the second product), two or three
@@ -12,7 +15,9 @@
 //   warps 4..7   softmax of the even tiles, warps 8..11 of the odd ones: a thread owns one row (tensor-memory lane) of a tile.  The two
 //                groups are half a period apart, so one exponentiates while the other waits for tensor memory.  A row's reference maximum
 //                travels from tile to tile through shared memory and moves only when it is exceeded by more than 8 (weights reach e^8;
-//                nothing is rounded by that), so the output accumulator is rescaled a few times per row instead of once per tile.
+//                nothing is rounded by that), so the output is rescaled a few times per row instead of once per tile.  The output of a row, half of
+//                its columns in each group, is in registers: a group adds tile t's product while it waits for its next scores, and the
+//                other group adds it before it hands over its own weights.
 // Tensor memory: 2 x 96 columns for a tile's scores (the upper 64) and, behind the reader, its weights (24 columns per 16 keys: three
 // parts of 8); O 128; the rest holds query parts (all three
 // of a 128-entry head, two of a 192-entry one, the third stays in shared memory): with the query in shared memory an N = 64 MMA
@@ -22,10 +27,11 @@
 // over 64 keys (26 KB) every role ran into instruction fetches (2.7 stalled warps per issued instruction) and an MMA took 120 cycles to
 // issue.  So a tile is taken in four steps of 16 keys, read from tensor memory once for the maximum and once for the weights.
 //
-// A 128 x 64 tile of head size 128 is 24 MMAs of 32 cycles and 12 of 64; it takes 2640 (3000 cycles of copies, then 5250 of softmax and issue
-// in the first form), bound by the waits between softmax, the two products and back; with a row tile or two per SM the first copies and
+// A 128 x 64 tile of head size 128 is 24 MMAs of 32 cycles and 12 of 64; it takes about 2900 (2640 without the sums in
+// registers; 3000 cycles of copies, then 5250 of softmax and issue in the first form), bound by the waits between softmax, the two products and back; with a row tile or two per SM the first copies and
 // query loads (4 us per CTA) and the uneven last round show as well.  Layer of width 2048, 2048 tokens, window 1024:
-// 811 us on the CUDA cores (9-19 TFLOP/s), 149 us so (the kernel 79; with two-byte stores, a row per lane, 126); latent layer 1555 -> 178 us.
+// 811 us on the CUDA cores (9-19 TFLOP/s), 158 us so (the kernel 90; 82 with the outputs left in tensor memory; with two-byte stores, a row per
+// lane, 47 more); latent layer 1555 -> 191 us (the kernel 115; 103).
 #pragma once
 #include "tc_common.cuh"
 
@@ -72,6 +78,24 @@ __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint3
 __device__ __forceinline__ uint64_t desc_mn(uint32_t addr, uint32_t lbo) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
+// 16 columns on their way; the registers hold them after the wait below, which takes them as operands so that nothing uses them before it
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[16], uint32_t (&b)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]),
+                 "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15])
+               :
+               : "memory");
+  asm volatile("" : "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]), "+r"(b[8]), "+r"(b[9]), "+r"(b[10]), "+r"(b[11]),
+               "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15]) : : "memory");
+}
 __device__ __forceinline__ void tmem_st8(uint32_t a, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]),
                "r"(r[6]), "r"(r[7])
@@ -103,6 +127,8 @@ __device__ __forceinline__ void st16_bf16(__nv_bfloat16* p, const float (&y)[16]
 //   float sink(tile)                      score of the sink, -inf without one
 //   bool partial(tile); void store_part(tile, r, c0, x[16]); void store_ml(tile, r, m, l)
 //   void store(tile, r, c0, x[16])        normalised outputs c0 .. c0+15
+//   REGS                                  every tile's product is added to f32 registers: the tensor core truncates when it adds to its
+//                                         accumulator, which over many tiles is a bias towards zero (see above)
 // and the tensor maps, the host-visible ints DK, DV, stages, split8, q_tmem, floats scale, softcap.
 // Rows whose result is infinite or NaN, again on the CUDA cores over the keys that they see, one row after the other with the whole CTA (a key
 // per thread for the scores, three threads per value column).  The products above cannot tell an infinite key or value from NaN: the lower
@@ -190,15 +216,16 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   float* s_ref = reinterpret_cast<float*>(smem_raw);         // [ROWS] a row's reference maximum after the latest tile
   float* s_end = s_ref + ROWS;                               // [2][ROWS] maximum and sum of the other group at the end
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 19
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 20
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 20);
   uint32_t* s_bad = &tmem_slot + 1;                          // [ROWS / 32] rows with an infinite or NaN result
   uint32_t& failed = s_bad[ROWS / 32];                       // a wait of the CTA's softmax groups ran out
+  constexpr bool REGS = Prob::REGS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages, nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
   const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
   const uint32_t b0 = smem_u32(bars);
-  const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 112, pv_done = b0 + 128, gave_up = b0 + 144;
+  const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 112, pv_done = b0 + 128, gave_up = b0 + 144, o_free = b0 + 152;
   uint32_t dead = (sq & 1023u) ? 1u : 0u;                    // swizzle atoms need 1024-byte alignment (shared memory starts on one)
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) {
@@ -207,6 +234,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     }
     for (int i = 0; i < 2; ++i) { mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, 4); mbar_init(pv_done + 8 * i, 1); }
     mbar_init(gave_up, 1);
+    mbar_init(o_free, 4);
     failed = 0u;
     mbar_init_fence();
   }
@@ -283,6 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         mbar_wait(v_full + 8 * st, v_ph, dead);
         if (++v_st == nst) { v_st = 0; v_ph ^= 1u; }
         mbar_wait_warp(p_full + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, dead);
+        if (REGS && t > 0) mbar_wait_warp(o_free, (uint32_t)(t - 1) & 1u, dead);      // the other group has taken the product before it too
         if (dead) break;
         copied(t);
         fence_after();
@@ -291,7 +320,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
 #pragma unroll 1
         for (int q = NP - 1; q >= 0; --q)
 #pragma unroll
-          for (int k = 0; k < KEYS / 16; ++k) mma_ts(tmem + COL_O, pc + 24 * k + 8 * q, vd + k * (16 * 128 / 16), id_o, (t > 0 || q < NP - 1 || k > 0) ? 1u : 0u, lead);
+          for (int k = 0; k < KEYS / 16; ++k) mma_ts(tmem + COL_O, pc + 24 * k + 8 * q, vd + k * (16 * 128 / 16), id_o, ((!REGS && t > 0) || q < NP - 1 || k > 0) ? 1u : 0u, lead);
         if (lead) {
           commit(v_empty + 8 * st);
           commit(pv_done + 8 * (t & 1));
@@ -409,7 +438,17 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     pr.range(tl, r, lo, hi);
     if (r >= tl.rows) { lo = 1; hi = 0; }
     float m = -INFINITY, l = 0.f;                            // reference maximum, and the sum over this group's tiles relative to it
-    for (int t = b; t < n; t += 2) {
+    float acc[MAX_DV / 32][16], acc_ref = -INFINITY;         // output columns 16 (b + 2 i) .. of the tiles so far, relative to acc_ref
+#pragma unroll
+    for (int i = 0; i < MAX_DV / 32; ++i)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) acc[i][e] = 0.f;
+    for (int t = b; t < n + (REGS ? 1 : 0); t += 2) {        // REGS, tile n: nothing but the product of tile n - 1, for the group that has not taken it
+     float base[2] = {-INFINITY, -INFINITY};                 // the references of tiles t - 1 and t
+     if (REGS && t == n) {
+      if (t > 0) bar_named(1 + 4 * (b ^ 1) + qtr, 64);
+      base[0] = s_ref[r];
+     } else {
       mbar_wait(s_full + 8 * b, (uint32_t)(t >> 1) & 1u, dead);
       fence_after();
       const uint32_t reg = tmem + lane_at + REGION * b;
@@ -449,21 +488,25 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       const bool up = mx > ref + 8.f;                        // also the first key a row sees (ref = -inf)
       const float now = up ? mx : ref;
       if (up) s_ref[r] = now;
-      if (t + 1 < n) bar_named_arrive(1 + 4 * b + qtr, 64);
+      if (REGS || t + 1 < n) bar_named_arrive(1 + 4 * b + qtr, 64);
+      base[0] = ref;
+      base[1] = now;
       if (m != now) {
         l *= m == -INFINITY ? 0.f : expf(m - now);
         m = now;
       }
-      const float f = (up && ref != -INFINITY) ? expf(ref - now) : 1.f;      // nothing was added to a row that saw no key
-      if (__any_sync(0xffffffffu, f != 1.f)) {               // t > 0 here; the scores of this tile came after PV(t - 2)
-        mbar_wait(pv_done + 8 * (b ^ 1), (uint32_t)((t - 1) >> 1) & 1u, dead);
-        fence_after();
-        for (int g = 0; g < pr.DV / 16; ++g) {
-          uint32_t o[16];
-          tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
+      if (!REGS) {                                           // what is in tensor memory follows the reference
+        const float f = (up && ref != -INFINITY) ? expf(ref - now) : 1.f;    // nothing was added to a row that saw no key
+        if (__any_sync(0xffffffffu, f != 1.f)) {             // t > 0 here; the scores of this tile came after PV(t - 2)
+          mbar_wait(pv_done + 8 * (b ^ 1), (uint32_t)((t - 1) >> 1) & 1u, dead);
+          fence_after();
+          for (int g = 0; g < pr.DV / 16; ++g) {
+            uint32_t o[16];
+            tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-          tmem_st16(tmem + lane_at + COL_O + 16 * g, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+            tmem_st16(tmem + lane_at + COL_O + 16 * g, o);
+          }
         }
       }
       const float mm = m == -INFINITY ? 0.f : m;             // a row that has seen no key: every score is -inf, every weight 0
@@ -491,18 +534,56 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       }
       l += sum[0] + sum[1];
       tmem_wait_st();
-      fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full + 8 * b);
+     }
+      if (!REGS) {
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full + 8 * b);
+      }
+      // REGS: the products of tiles t - 1 and t into the registers: the first before PV(t) may overwrite it, the second while S(t + 2) is on its way
+#pragma unroll 1
+      for (int k = 0; REGS && k < 2; ++k) {
+        const int u = t - 1 + k;
+        if (u >= 0 && u < n) {
+          mbar_wait(pv_done + 8 * (u & 1), (uint32_t)(u >> 1) & 1u, dead);
+          fence_after();
+          const float to = k ? base[1] : base[0];
+          if (__any_sync(0xffffffffu, acc_ref != to)) {
+            const float f = acc_ref == to ? 1.f : acc_ref == -INFINITY ? 0.f : expf(acc_ref - to);
+            acc_ref = to;
+#pragma unroll
+            for (int i = 0; i < MAX_DV / 32; ++i)
+#pragma unroll
+              for (int e = 0; e < 16; ++e) acc[i][e] *= f;
+          }
+#pragma unroll
+          for (int i = 0; i < MAX_DV / 32; i += 2) {         // two loads on their way together (columns beyond the head are loaded, not used)
+            if (b + 2 * i >= pr.DV / 16) break;
+            uint32_t o[2][16];
+            tmem_ld16_issue(tmem + lane_at + COL_O + 16 * (b + 2 * i), o[0]);
+            tmem_ld16_issue(tmem + lane_at + COL_O + 16 * (b + 2 * i + 2), o[1]);
+            tmem_wait_ld(o[0], o[1]);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              acc[i][e] += __uint_as_float(o[0][e]);
+              acc[i + 1][e] += __uint_as_float(o[1][e]);
+            }
+          }
+        }
+        if (t == n) break;
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(k ? o_free : p_full + 8 * b);
+      }
     }
-    // the even group ends with the sum of both (relative to the last reference); each group stores every other 16 columns.  Only the group of
-    // the last tile waits for its product (the other may not have seen the phase before it, whose parity would let it pass); the barriers
-    // below carry that to the other group.
-    if (n > 0 && b == ((n - 1) & 1)) {
+    // the even group ends with the sum of both (relative to the last reference); each group stores every other 16 columns.  Without REGS only
+    // the group of the last tile waits for its product (the other may not have seen the phase before it, whose parity would let it pass);
+    // the barriers below carry that to the other group.
+    if (!REGS && n > 0 && b == ((n - 1) & 1)) {
       mbar_wait(pv_done + 8 * b, (uint32_t)((n - 1) >> 1) & 1u, dead);
       fence_after();
     }
-    fence_before();
+    if (!REGS) fence_before();
     if (dead) failed = 1u;
     if (b == 1) { s_end[r] = m; s_end[ROWS + r] = l; }
     bar_named(10, 2 * ROWS);
@@ -514,7 +595,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       tot[r] = l;
     }
     bar_named(10, 2 * ROWS);
-    fence_after();
+    if (!REGS) fence_after();
     dead |= failed;
     l = tot[r];
     m = ref;
@@ -525,6 +606,17 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     if (dead) inv = l = __int_as_float(0x7fc00000);
     if (part && live && b == 0) pr.store_ml(tl, r, m, l);
     float odd = part ? l * 0.f : 0.f;                        // NaN as soon as something infinite or NaN came out
+    if (REGS) {                                              // back to tensor memory: written out from the registers, 64 columns' gates and stores in a
+#pragma unroll                                               // row are more code than the instruction caches hold (10 us per CTA)
+      for (int i = 0; i < MAX_DV / 32; ++i) {
+        uint32_t o[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(acc[i][e]);
+        if (b + 2 * i < pr.DV / 16) tmem_st16(tmem + lane_at + COL_O + 16 * (b + 2 * i), o);
+      }
+      tmem_wait_st();
+    }
+#pragma unroll 1
     for (int g = b; g < pr.DV / 16; g += 2) {
       uint32_t o[16];
       __syncwarp();

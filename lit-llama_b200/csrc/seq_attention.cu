@@ -417,7 +417,7 @@ static DynSmemCache g_chunk_smem[2];
 // padded shared memory; the 8 lanes of a ty group share their rows' maxima and sums by shuffles; the weights go
 // through shared memory into the value product, where the same thread holds its 4 queries x V/8 value channels.
 // All in f32 on the CUDA cores: float32 models, portions below 64 tokens and head sizes that are not whole MMA steps; the others take the
-// tensor-core kernel (width 2048, 2048 tokens, window 1024: 700 us here, 79 there).
+// tensor-core kernel (width 2048, 2048 tokens, window 1024: 700 us here, 90 there).
 constexpr int TQ = 64, TK = 32, TILE_THREADS = 128;
 
 template <typename act_t>
@@ -641,6 +641,7 @@ static int launch_tile(const b2l_seq_attn_args* a, cudaStream_t s, int cache_slo
 // ---- prompt portions with bf16 keys and values: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, 1), the tiles with the
 // most keys first.
 struct LocalProb {
+  static constexpr bool REGS = true;
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_attn_args a;
   int DK, DV, stages, split8, q_tmem, wide;             // wide: rows of `out` are 16-byte aligned

@@ -510,6 +510,7 @@ __global__ void seq_head_gate_kernel(const act_t* __restrict__ in, long long ld_
 // ---- the expanded form of a prompt portion in bf16: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, key splits), the tiles
 // with the most keys first.
 struct LatentProb {
+  static constexpr bool REGS = true;
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_latent_attn_args a;
   int DK, DV, stages, split8, q_tmem, tiled, wide;
