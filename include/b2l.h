@@ -214,7 +214,7 @@ int b2l_q8_outlier_mask(const void* x, int ldx, int M, int K, float threshold, v
                         b2l_stream_t stream);
 /* The same for M activation rows at once (csrc/q8_gemm.cu: tcgen05 kind::i8), outlier columns shared by the batch; reads CB in the
  * checkpoint's layout.  K % 128 == 0, K <= 12288; x, cb and workspace 16-byte aligned; workspace of
- * b2l_q8_linear_workspace_bytes(M, K) bytes. */
+ * b2l_q8_linear_workspace_bytes(M, K) bytes: K + 260 per row, of at most 4096 rows, and some 4 K. */
 size_t b2l_q8_linear_workspace_bytes(int M, int K);
 int b2l_q8_linear(const void* x, int ldx, const void* cb, const void* scb, void* y, int ldy,
                   void* workspace, int M, int N, int K, float threshold, b2l_stream_t stream);

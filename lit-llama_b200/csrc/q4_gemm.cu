@@ -16,7 +16,7 @@
 //
 // Why this form: with both operands in shared memory a 256 x 256 tile moves 160 bytes per cycle through it (dequantised weights written
 // and read, activations written and read) where 128 fit, and held the tensor pipe at 42 % (4096 x 5120 -> 5120: 291 us on the device,
-// now 153); a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice (4096 -> 11008: 45 us, now 28).
+// now 168 under the profiler); a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice (4096 -> 11008: 45 us, now 28).
 // What bounds it now is L2: a stage of bt = 240 brings 35 KB to the SM in some 750 cycles (480 of them the tensor pipe's).  Where tiles
 // are few a cluster of up to 8 CTAs splits K and adds its f32 sums through distributed shared memory in rank order (the result does not
 // depend on timing).

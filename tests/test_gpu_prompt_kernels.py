@@ -200,7 +200,8 @@ def test_four_tap_convolution_of_long_portions(T, Ch, bias):
 
 @pytest.mark.parametrize("M,N,K", [(17, 130, 11008), (33, 4096, 4096), (203, 11008, 4096), (257, 128, 512), (513, 384, 64)])
 def test_q4_gemm_tile_heights_and_splits(M, N, K):
-    """Token tiles of 16..256 and K split over clusters of 1..8 CTAs: f32 sums of exact bf16 products, one bf16 rounding."""
+    """Token tiles of 16, 48, 208, 64 and 96 and K split over clusters of 8, 4 and 1 CTAs (148 SMs): f32 sums of exact bf16 products, one bf16
+    rounding."""
     from gpu_util import rand_q4, relerr, tile
     from lit_llama_b200 import _lib as L
 
@@ -307,3 +308,10 @@ def test_local_attention_rounds_like_f32_over_many_keys(T, pos0, q_scale, v_mean
     want = attend(q.double(), k.double().repeat_interleave(H // G, 1), v.double().repeat_interleave(H // G, 1), K ** -0.5, seen)
     assert rel(out, want) < 8e-7
     assert abs(float(((out.double() - want) * want.sign()).sum() / want.abs().sum())) < 4e-7
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 5120, 13824), (208, 5120, 5120), (350, 4096, 11008), (256, 16384, 1024)])
+def test_q4_gemm_other_plans(M, N, K):
+    """On 148 SMs: splits of three with five token groups and, uneven, with thirteen (some warps sum a second one), of two with eleven,
+    the full tile of 256 tokens."""
+    test_q4_gemm_tile_heights_and_splits(M, N, K)
