@@ -4,22 +4,29 @@
 // Replaces ColBlockQuantizedLinear.forward (lit_llama/quantization.py:413-423) and the Triton kernel linear_kernel_4bit_weight
 // (quantization.py:187-333: tiles up to 256 x 256, dequantise inside the tile loop) for 4-bit weights with one (scale, zero) per row.
 //
-// A CTA computes 128 output features x `bt` tokens (16..256), the WEIGHT as the 128-row operand in tensor memory:
-//   warp 0       TMA: per 64-wide k stage the 4 KB of packed levels (load-time tiling b2l_q4_tile: contiguous) and the activation tile
-//                [bt tokens][64 k] as one 128-byte swizzled box, on one mbarrier; rows beyond M are zero-filled by the TMA unit
-//   warps 4..19  four groups, a stage each in turn: a thread owns one weight row: LDS.128 of 32 levels, nibble order chosen so that
-//                (w >> 4s) & 0x000f000f | 0x43004300 IS the bf16 pair (128 + level[k], 128 + level[k+1]), then level - zero and * scale with
-//                get_weight's own bf16 roundings (quantization.py:392-411), so the product sees exactly the matrix the reference's dense
-//                branch multiplies; tcgen05.st into the stage's 32 columns
-//   warp 1       tcgen05.mma.cta_group::1.kind::f16, A from tensor memory, B from shared memory, M 128, N bt, K 16
-//   afterwards the dequantising warps are the epilogue: tcgen05.ld, bf16, a warp writes 32 neighbouring features per token.
+// Work is in items of 128 output features x `bt` tokens (16..256), the WEIGHT as the 128-row operand in tensor memory; a CTA takes items in turn.
+// Operands move in units of 128 k:
+//   warp 0       TMA: the activation tile [bt tokens][128 k] as two 128-byte swizzled boxes, three or four units in flight; rows beyond M are zero-filled
+//   warp 2       TMA: the 8 KB of packed levels (load-time tiling b2l_q4_tile: contiguous), four or eight units ahead
+//   warps 4..19  four groups, a unit each in turn: a thread owns one weight row: LDS.128 of 32 levels, nibbles as bf16 subnormals, so that one fma gives
+//                level - zero and one product the weight, with get_weight's own bf16 roundings (quantization.py:392-411): the product sees exactly the
+//                matrix the reference's dense branch multiplies; tcgen05.st into the unit's 64 columns
+//   warp 1       tcgen05.mma.cta_group::1.kind::f16, A from tensor memory, B from shared memory, M 128, N bt, K 16: one barrier (activations landed and
+//                weights stored) and one commit per unit
+//   warps 20..27 the epilogue: tcgen05.ld, bf16, a warp writes 32 neighbouring features per token, while the next item's operands are on their way
+//                (two accumulators where bt <= 128); of a CTA's last item the dequantising warps store a share.
 //
 // Why this form: with both operands in shared memory a 256 x 256 tile moves 160 bytes per cycle through it (dequantised weights written
-// and read, activations written and read) where 128 fit, and held the tensor pipe at 42 % (4096 x 5120 -> 5120: 291 us on the device,
-// now 168 under the profiler); a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice (4096 -> 11008: 45 us, now 28).
-// What bounds it now is L2: a stage of bt = 240 brings 35 KB to the SM in some 750 cycles (480 of them the tensor pipe's).  Where tiles
-// are few a cluster of up to 8 CTAs splits K and adds its f32 sums through distributed shared memory in rank order (the result does not
-// depend on timing).
+// and read, activations written and read) where 128 fit, and held the tensor pipe at 42 % (4096 x 5120 -> 5120: 291 us on the device);
+// a prompt of 203 tokens gave 86 CTAs that each dequantised every second weight row twice.
+// What bounds it: from some 200 tokens per tile on the tensor pipe and the power it may draw (148 tiles of 256: 346 ns per 64 k, 512 cycles at the 1.5 GHz
+// the chip then keeps; 4096 x 5120 -> 5120 163 -> 153 us); below that the issuing warp and the dequantisation (64 tokens: 200 ns per 64 k).  A barrier that is
+// complete still costs the issuing warp 120..190 cycles beside four dequantising warps on its scheduler, and a bf16x2 operation takes a scheduler two
+// cycles: units of 128 k instead of 64, one barrier for both operands and two operations per pair of weights instead of three took 64 tokens from 280 to
+// 200 ns per 64 k (device time of 64 / 512 / 777 x 4096 -> 11008: 23.2 / 50.9 / 74.7 -> 16.8 / 41.9 / 55.7 us).  Where tiles are few a cluster of up to
+// 8 CTAs splits K and adds its f32 sums through distributed shared memory in rank order (the result does not depend on timing).
+#include <atomic>
+
 #include "tc_common.cuh"
 
 namespace b2l {
@@ -27,10 +34,10 @@ namespace q4gm {
 
 using namespace tc;
 
-constexpr int BN = 128, BK = 64;
-constexpr int W_BYTES = BN * BK / 2;           // packed levels of a stage
-constexpr int GROUPS = 4, NTHREADS = 128 + 128 * GROUPS;
-constexpr int MAX_STAGES = 8, A_COLS = BK / 2;      // a stage owns a weight buffer of 32 tensor-memory columns; the accumulator follows from COL_ACC on
+constexpr int BN = 128, BK = 64, UNIT = 2 * BK;      // k of an activation box, and of a pipeline unit (the last one of an odd count is half full)
+constexpr int W_BYTES = BN * UNIT / 2;         // packed levels of a unit
+constexpr int GROUPS = 4, EPI = 2, NTHREADS = 128 + 128 * (GROUPS + EPI);
+constexpr int A_BUFS = 4, A_COLS = UNIT / 2, MAX_W = 8;      // a weight buffer is 64 tensor-memory columns; accumulators follow from COL_ACC on
 constexpr int COL_ACC = 512 - 256;
 
 struct Params {
@@ -38,7 +45,7 @@ struct Params {
   const uint8_t* qwt;      // b2l_q4_tile layout: [N/128 tiles][K/32 slabs][128 rows][16 B]
   const void* scales; const void* zeros; int szdt;
   __nv_bfloat16* y; int ldy;
-  int M, N, K, bt, nst, splits;
+  int M, N, K, bt, nx, nw, splits, n_tiles, items;
   int expired;             // cluster rank that ends as if its last wait had run out, or -1
 };
 
@@ -47,22 +54,26 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 }
 __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * MAX_STAGES + 2];
+  __shared__ __align__(8) uint64_t bars[2 * MAX_W + 2 * A_BUFS + 6];
   __shared__ uint32_t tmem_slot, failed;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;            // 128-byte swizzle atoms are 1024-byte aligned
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, a_full = empty + 8 * MAX_STAGES, acc_done = a_full + 8 * MAX_STAGES,
-                 gave_up = acc_done + 8;
-  const uint32_t stage_bytes = W_BYTES + (uint32_t)p.bt * (BK * 2);
-  const int tile_n = blockIdx.x / p.splits, n0 = tile_n * BN, m0 = blockIdx.y * p.bt;
+  const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * MAX_W, full = w_empty + 8 * MAX_W, done = full + 8 * A_BUFS, acc_full = done + 8 * A_BUFS,
+                 acc_empty = acc_full + 16, gave_up = acc_empty + 16, last_full = gave_up + 8;
+  const uint32_t box = (uint32_t)p.bt * (BK * 2), wbase = sbase + p.nx * 2 * box;
   const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
-  const int n_kt = p.K / BK, kt_lo = (int)((long long)rank * n_kt / p.splits), kt_hi = (int)((long long)(rank + 1) * n_kt / p.splits);
+  const int n_kt = p.K / BK, kt_lo = (int)((long long)rank * n_kt / p.splits), kt_hi = (int)((long long)(rank + 1) * n_kt / p.splits), nk = kt_hi - kt_lo;
+  // a CTA takes items blockIdx.x, + gridDim.x, ...; its units are counted through all of them.  Split K: one item for the whole cluster.
+  const int item0 = p.splits > 1 ? (int)(blockIdx.x / p.splits) : (int)blockIdx.x, step = p.splits > 1 ? p.items : (int)gridDim.x;
+  const int accs = p.bt <= 128 ? 2 : 1;                                    // accumulators in turn, or one
   uint32_t dead = 0;
 
   if (tid == 0) {
-    for (int i = 0; i < p.nst; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 1); mbar_init(a_full + 8 * i, 4); }
-    mbar_init(acc_done, 1);
+    for (int i = 0; i < p.nw; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4); }
+    for (int i = 0; i < A_BUFS; ++i) { mbar_init(full + 8 * i, 5); mbar_init(done + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 4 * EPI); }      // nobody waits for the last item's
     mbar_init(gave_up, 1);
+    mbar_init(last_full, 1);
     failed = 0u;
     mbar_init_fence();
   }
@@ -72,104 +83,215 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
   fence_after();
   const uint32_t tmem = tmem_slot;
 
+  // output of the CTA's n-th item, its 16-token groups first, first + stride, ...: a thread owns weight row 32 (warp % 4) + lane
+  auto put = [&](int item, int n, int first, int stride, uint32_t bar, uint32_t parity) {
+    const int qtr = warp & 3, ab = accs == 2 ? n & 1 : 0, row = item % p.n_tiles * BN + qtr * 32 + lane, m0 = item / p.n_tiles * p.bt;
+    mbar_wait_warp(bar, parity, dead);
+    fence_after();
+    const bool lost = dead || p.expired == 0;
+    const uint32_t at = tmem + ((uint32_t)(qtr * 32) << 16) + COL_ACC + 128 * ab;
+#pragma unroll 1
+    for (int b = first; b < p.bt / 16; b += stride) {
+      uint32_t r[16];
+      __syncwarp();
+      tmem_ld16(at + 16 * b, r);
+      const int m = m0 + 16 * b;
+      if (row < p.N) {
+        __nv_bfloat16* dst = p.y + (size_t)m * p.ldy + row;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (m + i < p.M) dst[(size_t)i * p.ldy] = f2bf(lost ? __int_as_float(0x7fc00000) : __uint_as_float(r[i]));
+      }
+    }
+    fence_before();
+    __syncwarp();
+    if (lane == 0 && !dead) mbar_arrive(acc_empty + 8 * ab);
+  };
+
   if (warp == 0) {
-    if (lane == 0) {
-      const uint8_t* wsrc = p.qwt + ((size_t)tile_n * (p.K / 32) + (size_t)kt_lo * 2) * 2048;
-      int st = 0;
-      uint32_t ph = 1;                                       // parity of a stage's previous use: passes at once the first time
-      for (int kt = kt_lo; kt < kt_hi; ++kt, wsrc += W_BYTES) {
-        mbar_wait(empty + 8 * st, ph, dead);
-        if (dead) break;
-        const uint32_t base = sbase + st * stage_bytes;
-        mbar_expect_tx(full + 8 * st, stage_bytes);
-        bulk_load(base, wsrc, W_BYTES, full + 8 * st);
-        tma_load_2d(base + W_BYTES, &p.xmap, kt * BK, m0, full + 8 * st);
-        if (++st == p.nst) { st = 0; ph ^= 1u; }
+    if (lane == 0) {                                         // activations: unit u on the barrier of its weight buffer; its memory is free when the MMAs
+      int u = 0, st = 0;                                     // of unit u - nx are done
+      for (int item = item0; item < p.items && !dead; item += step) {
+        const int m0 = item / p.n_tiles * p.bt;
+        for (int kt = kt_lo; kt < kt_hi; kt += 2, ++u) {
+          if (u >= p.nx) mbar_wait(done + 8 * ((u - p.nx) % A_BUFS), (uint32_t)((u - p.nx) / A_BUFS) & 1u, dead);
+          if (dead) break;
+          const uint32_t bar = full + 8 * (u % A_BUFS), dst = sbase + st * 2 * box;
+          const bool two = kt + 1 < kt_hi;
+          mbar_expect_tx(bar, two ? 2 * box : box);
+          tma_load_2d(dst, &p.xmap, kt * BK, m0, bar);
+          if (two) tma_load_2d(dst + box, &p.xmap, kt * BK + BK, m0, bar);
+          if (++st == p.nx) st = 0;
+        }
+      }
+      uint32_t late = 0;                                     // no copy outlives the CTA: the latest phases of all barriers, complete unless a wait ran out
+      for (int i = max(0, u - A_BUFS); i < u; ++i) mbar_wait(full + 8 * (i % A_BUFS), (uint32_t)(i / A_BUFS) & 1u, late);
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {                                         // packed levels, far ahead: they come from HBM
+      int st = 0, u = 0;
+      uint32_t ph = 1;                                       // parity of a slot's previous use: passes at once the first time
+      for (int item = item0; item < p.items && !dead; item += step) {
+        const uint8_t* wsrc = p.qwt + ((size_t)(item % p.n_tiles) * (p.K / 32) + (size_t)kt_lo * 2) * 2048;
+        for (int left = nk; left > 0; left -= 2, ++u, wsrc += W_BYTES) {
+          const uint32_t bytes = left > 1 ? W_BYTES : W_BYTES / 2;
+          mbar_wait(w_empty + 8 * st, ph, dead);
+          if (dead) break;
+          mbar_expect_tx(w_full + 8 * st, bytes);
+          bulk_load(wbase + st * W_BYTES, wsrc, bytes, w_full + 8 * st);
+          if (++st == p.nw) { st = 0; ph ^= 1u; }
+        }
       }
       uint32_t late = 0;
-      for (int i = 0; i < p.nst; ++i) {                      // no copy outlives the CTA; all have landed unless a wait ran out
-        mbar_wait(full + 8 * st, ph, late);
-        if (++st == p.nst) { st = 0; ph ^= 1u; }
-      }
+      for (int i = max(0, u - p.nw); i < u; ++i) mbar_wait(w_full + 8 * (i % p.nw), (uint32_t)(i / p.nw) & 1u, late);
     }
   } else if (warp == 1) {
     const uint32_t lead = elect_lane();
     // kind::f16: D = f32, A = B = bf16 (K-major), 128 x bt
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bt >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
-    int st = 0;
-    uint32_t ph = 0, acc = 0;
-    for (int kt = kt_lo; kt < kt_hi; ++kt) {
-      mbar_wait(full + 8 * st, ph, dead);
-      mbar_wait_warp(a_full + 8 * st, ph, dead);
-      if (dead) break;
-      fence_after();
-      const uint64_t bd = desc_sw128(sbase + st * stage_bytes + W_BYTES);
-      const uint32_t ad = tmem + st * A_COLS;
+    int st = 0, u = 0, n = 0;
+    uint32_t ready = 0;                                      // the next unit's operands are there: asked while this one's MMAs are issued
+    for (int item = item0; item < p.items; item += step, ++n) {
+      const int ab = accs == 2 ? n & 1 : 0, use = accs == 2 ? n >> 1 : n;
+      if (use > 0) mbar_wait_warp(acc_empty + 8 * ab, (uint32_t)(use - 1) & 1u, dead);
+      const uint32_t d = tmem + COL_ACC + 128 * ab;
+      uint32_t acc = 0;
+      for (int left = nk; left > 0; left -= 2) {
+        const int buf = u % A_BUFS;
+        if (!__all_sync(0xffffffffu, ready)) mbar_wait_warp(full + 8 * buf, (uint32_t)(u / A_BUFS) & 1u, dead);
+        if (dead) break;
+        fence_after();
+        ++u;
+        ready = mbar_test(full + 8 * (u % A_BUFS), (uint32_t)(u / A_BUFS) & 1u);
+        const uint64_t bd = desc_sw128(sbase + st * 2 * box);
+        const uint32_t ad = tmem + buf * A_COLS;
 #pragma unroll
-      for (int k = 0; k < BK / 16; ++k) mma_ts(tmem + COL_ACC, ad + 8 * k, bd + 2 * k, idesc, k > 0 ? 1u : acc, lead);
-      acc = 1;
-      if (lead) commit(empty + 8 * st);                      // one per stage: it frees both halves, and each holds the pipe up for 100 cycles
+        for (int k = 0; k < BK / 16; ++k) mma_ts(d, ad + 8 * k, bd + 2 * k, idesc, k > 0 ? 1u : acc, lead);
+        acc = 1;
+        if (left > 1) {
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) mma_ts(d, ad + A_COLS / 2 + 8 * k, bd + (box >> 4) + 2 * k, idesc, 1u, lead);
+        }
+        if (lead) commit(done + 8 * buf);                    // frees the weight buffer and the activations' memory
+        __syncwarp();
+        if (++st == p.nx) st = 0;
+      }
+      if (dead) break;
+      if (lead) {
+        commit(acc_full + 8 * ab);
+        if (item + step >= p.items) commit(last_full);
+      }
       __syncwarp();
-      if (++st == p.nst) { st = 0; ph ^= 1u; }
     }
-    if (lead) commit(dead ? gave_up : acc_done);
     if (dead) {
       uint32_t late = 0;
+      if (lead) commit(gave_up);
       mbar_wait(gave_up, 0, late);
     }
-  } else if (warp >= 4) {
-    const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = n0 + row;
+  } else if (warp >= 4 && warp < 4 + 4 * GROUPS) {
+    const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane;
     const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
     float sc_f = 0.f, z_f = 0.f;
-    if (n < p.N) { sc_f = load_sz(p.scales, p.szdt, n); z_f = load_sz(p.zeros, p.szdt, n); }
-    const __nv_bfloat162 sc2 = __float2bfloat162_rn(sc_f), z2 = __float2bfloat162_rn(z_f), c128 = __float2bfloat162_rn(128.f);
-    int st = grp;
+    auto row_values = [&](int item) {
+      const int n = item % p.n_tiles * BN + row;
+      const bool in = item < p.items && n < p.N;
+      sc_f = in ? load_sz(p.scales, p.szdt, n) : 0.f;
+      z_f = in ? load_sz(p.zeros, p.szdt, n) : 0.f;
+    };
+    int st = grp, turn = grp, u0 = 0;                        // a group takes every fourth unit, counted through all items
     uint32_t ph = 0;
-    if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
-    for (int it = grp; it < kt_hi - kt_lo; it += GROUPS) {
-      mbar_wait(full + 8 * st, ph, dead);                    // also: the MMAs of the stage's previous use are done
-      uint32_t w[8];
-      const uint32_t src = sbase + st * stage_bytes + row * 16;
+    const int nu = (nk + 1) / 2;
+    row_values(item0);
+    for (int item = item0; item < p.items; item += step, u0 += nu) {
+      // levels as they lie, bf16 subnormals of 2^-133 (low four bits) or 2^-130 (bits 3..6) each, times 2^127: (level - z) 2^-6 or 2^-3 in one fma
+      // with get_weight's rounding, since a power of two changes none; its product with scale 2^6 or 2^3 is rounded as the product with scale.
+      // Rows whose zero point or scale leaves bf16's normal range so go through 128 + level instead.
+      const bool fits = (z_f == 0.f || fabsf(z_f) >= 0x1p-100f) && fabsf(sc_f) <= 0x1p100f, all_fit = __all_sync(0xffffffffu, fits);
+      const __nv_bfloat162 up = __float2bfloat162_rn(0x1p127f), zl = __float2bfloat162_rn(all_fit ? z_f * -0x1p-6f : z_f), zh = __float2bfloat162_rn(z_f * -0x1p-3f),
+                           sl = __float2bfloat162_rn(all_fit ? sc_f * 0x1p6f : sc_f), sh = __float2bfloat162_rn(sc_f * 0x1p3f);
+      row_values(item + step);
+      for (; turn < nu; turn += GROUPS) {
+        mbar_wait(w_full + 8 * st, ph, dead);
+        const int u = u0 + turn, buf = u % A_BUFS, halves = min(2, nk - 2 * turn);
+#pragma unroll 1
+        for (int h = 0; h < halves; ++h) {
+          uint32_t w[8];
+          const uint32_t src = wbase + st * W_BYTES + h * (W_BYTES / 2) + row * 16;
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * h]), "=r"(w[4 * h + 1]), "=r"(w[4 * h + 2]), "=r"(w[4 * h + 3]) : "r"(src + h * 2048) : "memory");
-      fence_after();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t o[16];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const uint32_t v = ((w[4 * h + c] >> (4 * s)) & 0x000f000fu) | 0x43004300u;      // (128 + level) pair, exact
-            __nv_bfloat162 t = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), c128);     // level, exact
-            t = __hmul2(__hsub2(t, z2), sc2);                                                 // the reference's bf16 roundings
-            o[4 * c + s] = *reinterpret_cast<const uint32_t*>(&t);
+          for (int i = 0; i < 2; ++i)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4 * i]), "=r"(w[4 * i + 1]), "=r"(w[4 * i + 2]), "=r"(w[4 * i + 3]) : "r"(src + i * 2048) : "memory");
+          if (h + 1 == halves) {                             // the levels are in registers: their memory is free
+            __syncwarp();
+            if (lane == 0 && !dead) mbar_arrive(w_empty + 8 * st);
           }
-        tmem_st16(tmem + lane_at + st * A_COLS + 16 * h, o);
+          if (h == 0) {
+            if (u >= A_BUFS) mbar_wait(done + 8 * buf, (uint32_t)(u / A_BUFS - 1) & 1u, dead);
+            fence_after();
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            uint32_t o[16];
+            if (all_fit) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const uint32_t v = w[4 * i + c], lo[2] = {v & 0x000f000fu, (v >> 8) & 0x000f000fu}, hi[2] = {(v >> 1) & 0x00780078u, (v >> 9) & 0x00780078u};
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                  const __nv_bfloat162 l = __hmul2(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&lo[s]), up, zl), sl),
+                                       m = __hmul2(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&hi[s]), up, zh), sh);
+                  o[4 * c + 2 * s] = *reinterpret_cast<const uint32_t*>(&l);
+                  o[4 * c + 2 * s + 1] = *reinterpret_cast<const uint32_t*>(&m);
+                }
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                  const uint32_t v = ((w[4 * i + c] >> (4 * s)) & 0x000f000fu) | 0x43004300u;      // (128 + level) pair, exact
+                  __nv_bfloat162 t = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), __float2bfloat162_rn(128.f));
+                  t = __hmul2(__hsub2(t, zl), sl);
+                  o[4 * c + s] = *reinterpret_cast<const uint32_t*>(&t);
+                }
+            }
+            tmem_st16(tmem + lane_at + buf * A_COLS + 32 * h + 16 * i, o);
+          }
+        }
+        tmem_wait_st();
+        fence_before();
+        __syncwarp();
+        if (lane == 0 && !dead) mbar_arrive(full + 8 * buf);
+        st += GROUPS;
+        if (st >= p.nw) { st -= p.nw; ph ^= 1u; }
       }
-      tmem_wait_st();
-      fence_before();
-      __syncwarp();
-      if (lane == 0 && !dead) mbar_arrive(a_full + 8 * st);
-      st += GROUPS;
-      if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
+      turn -= nu;                                            // counted from the next item's first unit
     }
-    mbar_wait(acc_done, 0, dead);
-    fence_after();
-    if (p.expired == (int)rank) dead = 1u;
-    if (dead) failed = 1u;
+    if (p.splits > 1) {
+      mbar_wait(acc_full, 0, dead);
+      fence_after();
+      if (p.expired == (int)rank) dead = 1u;
+      if (dead) failed = 1u;
+    } else {
+      const int n = (p.items - 1 - item0) / step;            // the last item's output together with the other groups
+      put(item0 + n * step, n, EPI + grp, EPI + GROUPS, last_full, 0u);      // a barrier of its own: they have not followed the phases of the others
+    }
+  } else if (warp >= 4 + 4 * GROUPS && p.splits == 1) {
+    // the accumulator of an item while the next item's weights are on their way
+    const int grp = (warp >> 2) - 1 - GROUPS;
+    int n = 0;
+    for (int item = item0; item < p.items; item += step, ++n)
+      put(item, n, grp, item + step < p.items ? EPI : EPI + GROUPS, acc_full + 8 * (accs == 2 ? n & 1 : 0), (uint32_t)(accs == 2 ? n >> 1 : n) & 1u);
   }
   __syncwarp();
-  // ---- epilogue: a thread owns weight row n, 16 tokens at a time, the groups in turn; split K: a token group is summed by one CTA
-  const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = n0 + row, nb = p.bt / 16;
-  const uint32_t acc_at = tmem + ((uint32_t)(qtr * 32) << 16) + COL_ACC;
+  // ---- split K: a thread owns weight row n, 16 tokens at a time, the groups in turn; a token group is summed by one CTA
   if (p.splits > 1) {
+    const int qtr = warp & 3, grp = (warp >> 2) - 1, row = qtr * 32 + lane, n = item0 % p.n_tiles * BN + row, m0 = item0 / p.n_tiles * p.bt, nb = p.bt / 16;
+    const bool mine = warp >= 4 && warp < 4 + 4 * GROUPS;
     // stage memory is free (every MMA has completed): f32 [token group][128 rows][16 tokens], the 16-byte pieces of a row rotated
-    if (warp >= 4 && !__any_sync(0xffffffffu, dead)) {
+    if (mine && !__any_sync(0xffffffffu, dead)) {
       for (int b = grp; b < nb; b += GROUPS) {
         uint32_t r[16];
-        tmem_ld16(acc_at + 16 * b, r);
+        tmem_ld16(tmem + ((uint32_t)(qtr * 32) << 16) + COL_ACC + 16 * b, r);
         const uint32_t dst = sbase + (uint32_t)(b * BN + row) * 64;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -178,19 +300,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
     }
     __syncwarp();
     cluster_sync_all();
-  }
-  if (warp >= 4) {
-    for (int s = 0; s < p.splits; ++s)
-      if (p.splits > 1) dead |= ld_dsmem_u32(smem_u32(&failed), (uint32_t)s);
-    for (int b = (int)rank + grp * p.splits; b < nb; b += GROUPS * p.splits) {
-      __syncwarp();
-      float v[16];
-      if (p.splits == 1) {
-        uint32_t r[16];
-        tmem_ld16(acc_at + 16 * b, r);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-      } else {
+    if (mine) {
+      for (int s = 0; s < p.splits; ++s) dead |= ld_dsmem_u32(smem_u32(&failed), (uint32_t)s);
+      for (int b = (int)rank + grp * p.splits; b < nb; b += GROUPS * p.splits) {
+        __syncwarp();
+        float v[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = 0.f;
         for (int s = 0; s < p.splits; ++s) {
@@ -200,26 +314,44 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
             v[4 * c] += __uint_as_float(u.x); v[4 * c + 1] += __uint_as_float(u.y); v[4 * c + 2] += __uint_as_float(u.z); v[4 * c + 3] += __uint_as_float(u.w);
           }
         }
-      }
-      const int m = m0 + 16 * b;
-      if (n < p.N) {
-        __nv_bfloat16* dst = p.y + (size_t)m * p.ldy + n;
+        const int m = m0 + 16 * b;
+        if (n < p.N) {
+          __nv_bfloat16* dst = p.y + (size_t)m * p.ldy + n;
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (m + i < p.M) dst[(size_t)i * p.ldy] = f2bf(dead ? __int_as_float(0x7fc00000) : v[i]);
+          for (int i = 0; i < 16; ++i)
+            if (m + i < p.M) dst[(size_t)i * p.ldy] = f2bf(dead ? __int_as_float(0x7fc00000) : v[i]);
+        }
       }
     }
+    __syncwarp();
+    cluster_sync_all();                              // nobody leaves while a peer reads its partial sums
   }
-  __syncwarp();
-  if (p.splits > 1) cluster_sync_all();              // nobody leaves while a peer reads its partial sums
   fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-struct Plan { int bt, m_tiles, splits, nst; size_t smem; };
-// Tile height and K split by a model of the time in tensor cycles: rounds of CTAs over the SMs times (stages of max(2 bt, the 200 a stage's
-// dequantisation takes) + a fixed part: first copies, epilogue, and the sums of a split).
+constexpr size_t MOST_SMEM = 226 * 1024;
+struct Plan { int bt, m_tiles, splits, nx, nw; size_t smem; };
+// Clusters of sp CTAs, one per SM, that run at once (B200: 148, 74, 45, 33, 26, 22, 15, 15 of 1..8: clusters do not cross the SM groups).
+static int slots(int sp, int sms) {
+  if (sp == 1) return sms;
+  static std::atomic<int> known[9];
+  int n = known[sp].load(std::memory_order_relaxed);
+  if (n == 0) {
+    LaunchCfg lc(dim3((unsigned)sp), dim3(NTHREADS), 120 * 1024, nullptr, false, sp);
+    if (cudaOccupancyMaxActiveClusters(&n, q4_gemm_kernel, &lc.cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = sms / sp > 0 ? sms / sp : 1;
+    }
+    known[sp].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+// Tile height and K split by a model of the time in ns: a CTA's items one after the other, each of so many 64-wide stages (60 + 1.15 per token of the
+// tile, and no less than the 200 that dequantising and issuing take; 18944 features, 64 / 128 / 208 / 256 tokens: 200 / 209 / 286 / 346) and 1000 for
+// each; first copies and the last output once, 4000 and 15 per token.  A split adds 3500 for its barriers and, for every further rank, 12 per token
+// (partial sums to and from shared memory; seen: 32 tokens in four 4500, 112 in four 7000, 208 in two 5000), and every round of it starts anew.
 static Plan plan_for(int M, int N, int K) {
   const int sms = sm_count(), n_tiles = (N + BN - 1) / BN, n_kt = K / BK;
   Plan best{};
@@ -229,19 +361,21 @@ static Plan plan_for(int M, int N, int K) {
     const int bt = ((M + mt - 1) / mt + 15) / 16 * 16, tiles = (M + bt - 1) / bt;
     for (int sp = 1; sp <= 8; ++sp) {
       if (sp > 1 && n_kt / sp < 8) break;
-      const long long ctas = (long long)n_tiles * tiles * sp, rounds = (ctas + sms - 1) / sms;
-      const long long stages = (n_kt + sp - 1) / sp, per = bt * 2 > 200 ? bt * 2 : 200;
-      const long long cost = rounds * (stages * per + 3000 + 8 * bt + (sp > 1 ? 1500 + 10 * bt : 0));
+      const int at_once = slots(sp, sms);
+      const long long rounds = (n_tiles * tiles + at_once - 1) / at_once, stages = (n_kt + sp - 1) / sp;
+      const long long per = 600 + bt * 23 / 2 > 2000 ? 600 + bt * 23 / 2 : 2000, once = 4000 + 15 * bt;
+      const long long cost = sp == 1 ? rounds * (stages * per / 10 + 1000) + once : rounds * (stages * per / 10 + once + 3500 + (sp - 1) * 12 * bt);
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
         best.bt = bt; best.m_tiles = tiles; best.splits = sp;
       }
     }
   }
-  const size_t stage = W_BYTES + (size_t)best.bt * BK * 2;
-  best.nst = (int)(216 * 1024 / stage);
-  if (best.nst > MAX_STAGES) best.nst = MAX_STAGES;
-  best.smem = best.nst * stage + 1024;
+  // four units of activations where they fit beside eight of weights, three beside four otherwise
+  const size_t x = (size_t)best.bt * UNIT * 2, room = MOST_SMEM - 1024;
+  best.nx = A_BUFS * x + MAX_W * W_BYTES <= room ? A_BUFS : 3;
+  best.nw = best.nx == A_BUFS ? MAX_W : 4;
+  best.smem = best.nx * x + best.nw * W_BYTES + 1024;
   const size_t part = (size_t)BN * best.bt * 4 + 1024;
   if (best.splits > 1 && part > best.smem) best.smem = part;
   // One CTA per SM by its shared memory, whatever its registers: each takes all of tensor memory, and a CTA of a cluster that waited for another's
@@ -265,17 +399,19 @@ extern "C" int b2l_q4_gemm(const b2l_q4_linear_args* a, b2l_stream_t stream) {
   B2L_CHECK_ARG(((uintptr_t)a->x % 16 == 0) && ((uintptr_t)a->qw_tiled % 16 == 0), "b2l_q4_gemm: x / qw_tiled must be 16-byte aligned");
   B2L_CHECK_ARG(a->sz_dtype == B2L_BF16 || a->sz_dtype == B2L_F32, "b2l_q4_gemm: bad sz_dtype");
   B2L_CHECK_SUPPORTED(a->prologue == B2L_PRO_NONE && a->epilogue == B2L_EPI_STORE, "b2l_q4_gemm: plain linear only (no fused prologue / epilogue)");
+  static DynSmemCache smem_cache;
+  if (int rc = ensure_dyn_smem(q4_gemm_kernel, MOST_SMEM, smem_cache)) return rc;
   const Plan q = plan_for(a->M, a->N, a->K);
   Params p;
   if (int rc = map_sw128(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->x, a->M, a->K, a->ldx, BK, q.bt)) return rc;
   p.qwt = (const uint8_t*)a->qw_tiled;
   p.scales = a->scales; p.zeros = a->zeros; p.szdt = a->sz_dtype;
   p.y = (__nv_bfloat16*)a->y; p.ldy = a->ldy;
-  p.M = a->M; p.N = a->N; p.K = a->K; p.bt = q.bt; p.nst = q.nst; p.splits = q.splits;
+  p.M = a->M; p.N = a->N; p.K = a->K; p.bt = q.bt; p.nx = q.nx; p.nw = q.nw; p.splits = q.splits;
+  p.n_tiles = (a->N + BN - 1) / BN; p.items = p.n_tiles * q.m_tiles;
   p.expired = (a->flags >> B2L_F_EXPIRED_SHIFT & 15) - 1;
-  static DynSmemCache smem_cache;
-  if (int rc = ensure_dyn_smem(q4_gemm_kernel, q.smem, smem_cache)) return rc;
-  LaunchCfg lc(dim3((unsigned)((a->N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, (cudaStream_t)stream, false, q.splits);
+  const int ctas = q.splits > 1 ? p.items * q.splits : (p.items < sm_count() ? p.items : sm_count());
+  LaunchCfg lc(dim3((unsigned)ctas), dim3(NTHREADS), q.smem, (cudaStream_t)stream, false, q.splits);
   B2L_CUDA(cudaLaunchKernelEx(&lc.cfg, q4_gemm_kernel, p));
   return 0;
 }

@@ -34,6 +34,13 @@ __device__ __forceinline__ void mbar_wait_warp(uint32_t a, uint32_t parity, uint
   mbar_wait(a, parity, dead);
   dead = __any_sync(0xffffffffu, dead) ? 1u : 0u;
 }
+// Whether the phase with this parity is complete, without waiting: a wait on a barrier that is complete takes 120..300 cycles, so a loop
+// asks for its next barrier before it works on this one.
+__device__ __forceinline__ uint32_t mbar_test(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+  return ok;
+}
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

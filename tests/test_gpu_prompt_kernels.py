@@ -315,3 +315,24 @@ def test_q4_gemm_other_plans(M, N, K):
     """On 148 SMs: splits of three with five token groups and, uneven, with thirteen (some warps sum a second one), of two with eleven,
     the full tile of 256 tokens."""
     test_q4_gemm_tile_heights_and_splits(M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 19300, 192), (300, 9700, 320), (20, 38000, 64), (600, 9600, 128)])
+def test_q4_gemm_several_tiles_per_cta(M, N, K):
+    """More tiles than the 148 SMs: one and two accumulators, k counts that end in half a unit, the second token group without a block; rows whose
+    zero point or scale is outside the range in which levels are taken as subnormals, beside ordinary ones.  Products are exact, sums f32."""
+    from gpu_util import rand_q4, tile
+    from lit_llama_b200 import _lib as L
+
+    lv, qw, sc, z = rand_q4(N, K, DEV, seed=M + N + K)
+    sc, z = sc.to(BF), z.to(BF)
+    z[64:128:5], z[200:230:3], z[300] = 2.0 ** -120, 0.0, -0.0
+    sc[130:160:7], sc[260:270], sc[N - 3] = 2.0 ** 104, 2.0 ** -128, -(2.0 ** 101)
+    qt = tile(L, qw, N, K)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    y = torch.full((M + 1, N), 7.0, device=DEV, dtype=BF)
+    a = L.Q4LinearArgs(x=x.data_ptr(), ldx=K, qw_tiled=qt.data_ptr(), scales=sc.data_ptr(), zeros=z.data_ptr(), sz_dtype=L.sz_dtype_of(sc), y=y.data_ptr(), ldy=N, M=M, N=N, K=K)
+    assert L.lib().b2l_q4_gemm(C.byref(a), L.stream_ptr()) == 0, L.lib().b2l_last_error()
+    want = x.double() @ ((lv.to(BF) - z) * sc).double().t()
+    err = (y[:M].double() - want).norm(dim=0) / want.norm(dim=0)          # per feature: one bf16 rounding
+    assert float(err.max()) < 2.0 ** -8 and bool((y[M] == 7).all())
