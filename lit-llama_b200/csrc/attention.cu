@@ -876,6 +876,10 @@ struct PromptProb {
       x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
   }
+  __device__ __forceinline__ bool pieces() const { return true; }
+  __device__ __forceinline__ const void* piece(const Tile& t, int r, int p) const {
+    return qkv + ((size_t)t.b * T + t.t_first + r) * 3 * n_head * 128 + (size_t)t.h * 128 + 8 * p;
+  }
   __device__ __forceinline__ void range(const Tile& t, int r, int& lo, int& hi) const {
     lo = 0;
     hi = r < t.rows ? slots(t.t_first + r, t.cap) - 1 : -1;
@@ -883,9 +887,14 @@ struct PromptProb {
   __device__ __forceinline__ float sink(const Tile&) const { return -INFINITY; }
   __device__ __forceinline__ bool partial(const Tile&) const { return false; }
   __device__ __forceinline__ void store_ml(const Tile&, int, float, float) const {}
-  __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[16]) const {}
-  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
-    atc::st16_bf16(y + ((size_t)t.b * T + t.t_first + r) * n_head * 128 + (size_t)t.h * 128 + c0, x);
+  __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[4]) const {}
+  struct Gate {};
+  __device__ __forceinline__ bool gate_pieces() const { return false; }
+  __device__ __forceinline__ const void* gate_piece(const Tile&, int, int) const { return nullptr; }
+  __device__ __forceinline__ Gate gate(const Tile&, int, int) const { return {}; }
+  __device__ __forceinline__ float factor(const Tile&, int) const { return 1.f; }
+  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[4], const Gate&) const {
+    atc::st4_bf16(y + ((size_t)t.b * T + t.t_first + r) * n_head * 128 + (size_t)t.h * 128 + c0, x);
   }
 };
 

@@ -7,31 +7,33 @@
 // starts from zero and is added to f32 registers: 2.3e-7, 3.2e-7 and 1.2e-7 in these cases, below the f32 kernel in every size measured.
 // Three bf16 MMAs cost 3 / 32 of what the f32 FMAs cost on the CUDA cores (4096 against 128 per cycle).
 //
-//   warp 0       issues the MMAs: S(t+2) = Q K^T goes behind O += P(t) V
-//   warps 1, 2   keys, warps 3, 12 values, into 128-byte swizzled rows (keys K-major, values MN-major for the second product), two or three
+//   warp 0       issues the MMAs of the scores S(t) = Q K^T, three tiles ahead at most, warp 13 those of the outputs, P(t) V
+//   warps 1, 2   keys, warps 3, 12 values, into 128-byte swizzled rows (keys K-major, values MN-major for the second product), three
 //                stages.  Tiles of 64 consecutive rows (the fresh projections, an expanded latent) come by tiled TMA copies; tiles that touch
 //                the cache ring or end early by 16-byte cp.async, which arrive on the stage's barrier by themselves but take 3000 cycles
-//                to issue, twice what the rest of a tile takes
+//                to issue, more than the rest of a tile takes
 //   warps 4..7   softmax of the even tiles, warps 8..11 of the odd ones: a thread owns one row (tensor-memory lane) of a tile.  The two
 //                groups are half a period apart, so one exponentiates while the other waits for tensor memory.  A row's reference maximum
-//                travels from tile to tile through shared memory and moves only when it is exceeded by more than 8 (weights reach e^8;
+//                travels from tile to tile through shared memory and moves only when it is exceeded by more than 11 (weights reach 2^11;
 //                nothing is rounded by that), so the output is rescaled a few times per row instead of once per tile.  The output of a row, half of
-//                its columns in each group, is in registers: a group adds tile t's product while it waits for its next scores, and the
-//                other group adds it before it hands over its own weights.
-// Tensor memory: 2 x 96 columns for a tile's scores (the upper 64) and, behind the reader, its weights (24 columns per 16 keys: three
-// parts of 8); O 128; the rest holds query parts (all three
-// of a 128-entry head, two of a 192-entry one, the third stays in shared memory): with the query in shared memory an N = 64 MMA
-// reads 6 KB in its 48 cycles, which is all of the shared-memory bandwidth, and everything else on the SM waited for it.  One CTA per SM.
+//                its columns in each group, is in registers: a group adds the product of its tile before when it has the maximum of this one, and the
+//                other group's before it hands over its own weights.
+// Tensor memory: 3 x 96 columns for a tile's scores (the upper 64) and, behind the reader, its weights (24 columns per 16 keys: three
+// parts of 8); O 128; the smallest part of an f32 query (of 64..192 entries) 96.  Its other parts, and a bf16 query as it lies, are in shared
+// memory: an N = 64 MMA then reads 6 KB in its 48 cycles, all that shared memory gives, so nothing else uses it much.  One CTA per SM.
+//
+// Scores are powers of two: an f32 query takes scale * log2(e) with it (two parts, rounded once), so a weight is one subtraction and ex2,
+// and additions go in pairs (f32x2): 9 instructions per score and weight, of which expf and its scaling alone were as many.  f32 outputs
+// against float64 as before or closer (1024 keys 3.1e-7 -> 2.8e-7 of the norm, 2048 keys 3.2e-7 -> 2.9e-7).
 //
 // All roles' loops together stay under the 12 KB or so that an instruction cache next to the schedulers holds: with the softmax written out
 // over 64 keys (26 KB) every role ran into instruction fetches (2.7 stalled warps per issued instruction) and an MMA took 120 cycles to
 // issue.  So a tile is taken in four steps of 16 keys, read from tensor memory once for the maximum and once for the weights.
 //
-// A 128 x 64 tile of head size 128 is 24 MMAs of 32 cycles and 12 of 64; it takes about 2900 (2640 without the sums in
-// registers; 3000 cycles of copies, then 5250 of softmax and issue in the first form), bound by the waits between softmax, the two products and back; with a row tile or two per SM the first copies and
-// query loads (4 us per CTA) and the uneven last round show as well.  Layer of width 2048, 2048 tokens, window 1024:
-// 811 us on the CUDA cores (9-19 TFLOP/s), 158 us so (the kernel 90; 82 with the outputs left in tensor memory; with two-byte stores, a row per
-// lane, 47 more); latent layer 1555 -> 191 us (the kernel 115; 103).
+// What bounds it: a 128 x 64 tile of head size 128 is 24 MMAs of 48 cycles and 12 of 64, 1920 in all; it takes 2400..2700 (2950 with two score
+// regions and one issuing warp, 5250 of softmax and issue in the first form); queries, outputs and the first tile's chain of waits take 12 us per CTA
+// whatever its tiles (16, latent heads 30, with a row per lane in both).  Kernel time in us, before this form and now: 16 heads, window 1024, 2048
+// tokens 85 / 72, latent 16 heads of 192, 128 / 2048 tokens 36 / 16 and 110 / 75, LLaMA's 32 heads, 2048 tokens 111 / 85.
 #pragma once
 #include "tc_common.cuh"
 
@@ -41,9 +43,9 @@ namespace atc {
 using namespace tc;
 
 constexpr int ROWS = 128, KEYS = 64;
-constexpr int K_THREADS = 64, V_THREADS = 64, THREADS = 416;
+constexpr int K_THREADS = 64, V_THREADS = 64, THREADS = 448;
 constexpr int Q_ATOM = ROWS * 128, K_ATOM = KEYS * 128;      // bytes of 64 columns of a query / key / value tile
-constexpr uint32_t REGION = 96, S_AT = 32, COL_O = 192, COL_Q = 320;      // tile parity b: region at 96 b, scores at + 32, weights over them
+constexpr uint32_t REGION = 96, S_AT = 32, COL_O = 288, COL_Q = 416;      // tile t: region at 96 (t % 3), scores at + 32, weights over them
 constexpr int MAX_DK = 192, MAX_DV = 128;
 constexpr int CONTROL = 3072;                                // barriers, tensor-memory address, row maxima
 
@@ -51,8 +53,7 @@ __host__ __device__ inline int atoms(int d) { return (d + 63) / 64; }
 struct Layout { int stages, q_tmem; size_t smem; };
 static inline Layout layout(int nq, int dk, int dv) {
   Layout l;
-  l.q_tmem = (512 - (int)COL_Q) / (dk / 2);                  // query parts in tensor memory, the others in shared memory
-  if (l.q_tmem > nq) l.q_tmem = nq;
+  l.q_tmem = nq > 1 ? 1 : 0;                                 // the smallest part of a query in tensor memory, the others in shared memory
   const size_t q = (size_t)(nq - l.q_tmem) * atoms(dk) * Q_ATOM, st = (size_t)(atoms(dk) + atoms(dv)) * K_ATOM;
   l.stages = CONTROL + q + 3 * st <= 227 * 1024 ? 3 : 2;
   l.smem = CONTROL + q + l.stages * st;
@@ -104,17 +105,33 @@ __device__ __forceinline__ void tmem_st8(uint32_t a, const uint32_t (&r)[8]) {
 
 // The upper halves of x and y as a bf16 pair (truncation), x in the low half
 __device__ __forceinline__ uint32_t hi_pair(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
-__device__ __forceinline__ float rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+// Two f32 operations in one instruction: half the issue slots at the same rate.  a += c, b += d
+__device__ __forceinline__ void add2(float& a, float& b, float c, float d) {
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+f"(a), "+f"(b) : "f"(c), "f"(d));
+}
+__device__ __forceinline__ void sub2(float& a, float& b, float c, float d) {
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tsub.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}" : "+f"(a), "+f"(b) : "f"(c), "f"(d));
+}
+// a = a * f + c, b = b * f + d
+__device__ __forceinline__ void fma2(float& a, float& b, float f, float c, float d) {
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmov.b64 z, {%3, %4};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(a), "+f"(b) : "f"(f), "f"(c), "f"(d));
+}
+__device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+// 2^x; what CUDA's expf ends with as well, so as a weight it is no less exact than expf of the score
+__device__ __forceinline__ float exp2_f(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+constexpr float LOG2E = 1.44269502162933349609375f, LOG2E_LO = 1.925963033500011e-8f, LN2 = 0.693147180559945309f;      // log2(e) in two parts
 
-__device__ __forceinline__ void st16_bf16(__nv_bfloat16* p, const float (&y)[16]) {      // 16-byte aligned
-  uint32_t w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(y[2 * i], y[2 * i + 1]);
-    w[i] = *reinterpret_cast<const uint32_t*>(&v);
-  }
-  reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+__device__ __forceinline__ void st4_bf16(__nv_bfloat16* p, const float (&y)[4]) {      // 8-byte aligned
+  const __nv_bfloat162 u = __floats2bfloat162_rn(y[0], y[1]), v = __floats2bfloat162_rn(y[2], y[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&u), *reinterpret_cast<const uint32_t*>(&v));
+}
+__device__ __forceinline__ void tmem_st4(uint32_t a, const uint32_t (&r)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 
 // Prob: what a family's attention is made of.  Members, all __device__:
@@ -123,10 +140,14 @@ __device__ __forceinline__ void st16_bf16(__nv_bfloat16* p, const float (&y)[16]
 //   bool bulk(tile, j0, ra, rb, rv)       keys j0 .. j0+63 are rows ra.. of map_a (64-column boxes from column tile.xa; the columns from
 //                                         split8*8 on: rows rb.. of map_b from tile.xb) and values rows rv.. of map_v from tile.xv
 //   void query(tile, r, c, float x[8])    query entries 8c .. 8c+7 of row r
+//   bool pieces(); const void* piece(tile, r, p)      the same by 16-byte aligned pieces (4 f32 or, one part, 8 bf16), where they are
 //   void range(tile, r, lo, hi)           keys lo .. hi are visible to row r
 //   float sink(tile)                      score of the sink, -inf without one
-//   bool partial(tile); void store_part(tile, r, c0, x[16]); void store_ml(tile, r, m, l)
-//   void store(tile, r, c0, x[16])        normalised outputs c0 .. c0+15
+//   bool partial(tile); void store_part(tile, r, c0, x[4]); void store_ml(tile, r, m, l)
+//   float factor(tile, r)                 what the row's outputs are multiplied with
+//   Gate gate(tile, r, c0)                and what outputs c0 .. c0+3 are, as it lies in memory
+//   bool gate_pieces(); const void* gate_piece(tile, r, p)      the same by 16-byte aligned pieces, where it is
+//   void store(tile, r, c0, x[4], gate)   normalised outputs c0 .. c0+3, already with the factor
 //   REGS                                  every tile's product is added to f32 registers: the tensor core truncates when it adds to its
 //                                         accumulator, which over many tiles is a bias towards zero (see above)
 // and the tensor maps, the host-visible ints DK, DV, stages, split8, q_tmem, floats scale, softcap.
@@ -197,16 +218,16 @@ __device__ __noinline__ void redo_rows(const Prob& pr, const uint32_t* s_bad, fl
     const float sink = pr.sink(tl), M = fmaxf(m, sink), e = m == -INFINITY ? 0.f : expf(m - M);
     const float inv = part ? 1.f : e / (l * e + (sink == -INFINITY ? 0.f : expf(sink - M)));
     if (tid == 0 && part) pr.store_ml(tl, r, m, l);
-    if (tid < pr.DV / 16) {
-      float x[16];
+    if (tid < pr.DV / 4) {
+      float x[4];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
+      for (int i = 0; i < 4; ++i) {
         float t = 0.f;
-        for (int g = 0; g < GROUPS; ++g) t += s_acc[g * MAX_DV + 16 * tid + i];
-        x[i] = t * inv;
+        for (int g = 0; g < GROUPS; ++g) t += s_acc[g * MAX_DV + 4 * tid + i];
+        x[i] = t * inv * (part ? 1.f : pr.factor(tl, r));
       }
-      if (part) pr.store_part(tl, r, 16 * tid, x);
-      else pr.store(tl, r, 16 * tid, x);
+      if (part) pr.store_part(tl, r, 4 * tid, x);
+      else pr.store(tl, r, 4 * tid, x, pr.gate(tl, r, 4 * tid));
     }
   }
 }
@@ -216,8 +237,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   float* s_ref = reinterpret_cast<float*>(smem_raw);         // [ROWS] a row's reference maximum after the latest tile
   float* s_end = s_ref + ROWS;                               // [2][ROWS] maximum and sum of the other group at the end
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 20
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_end + 2 * ROWS);      // 23
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 23);
   uint32_t* s_bad = &tmem_slot + 1;                          // [ROWS / 32] rows with an infinite or NaN result
   uint32_t& failed = s_bad[ROWS / 32];                       // a wait of the CTA's softmax groups ran out
   constexpr bool REGS = Prob::REGS;
@@ -225,15 +246,18 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages, nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
   const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
   const uint32_t b0 = smem_u32(bars);
-  const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 112, pv_done = b0 + 128, gave_up = b0 + 144, o_free = b0 + 152;
+  const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 120, pv_done = b0 + 136, gave_up = b0 + 160, o_free = b0 + 176;
   uint32_t dead = (sq & 1023u) ? 1u : 0u;                    // swizzle atoms need 1024-byte alignment (shared memory starts on one)
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) {
       mbar_init(k_full + 8 * i, K_THREADS); mbar_init(k_empty + 8 * i, 1);
       mbar_init(v_full + 8 * i, V_THREADS); mbar_init(v_empty + 8 * i, 1);
+      mbar_init(s_full + 8 * i, 1);
+      mbar_init(pv_done + 8 * i, 1);
     }
-    for (int i = 0; i < 2; ++i) { mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, 4); mbar_init(pv_done + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) mbar_init(p_full + 8 * i, 4);
     mbar_init(gave_up, 1);
+    mbar_init(gave_up + 8, 1);
     mbar_init(o_free, 4);
     failed = 0u;
     mbar_init_fence();
@@ -241,36 +265,36 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   if (tid < ROWS) s_ref[tid] = -INFINITY;
   if (tid < ROWS / 32) s_bad[tid] = 0u;
   if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 512);
+  const typename Prob::Tile tl = pr.tile();
+  const int n = (tl.j_end - tl.j_begin + KEYS - 1) / KEYS;
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
-  const typename Prob::Tile tl = pr.tile();
-  const int n = (tl.j_end - tl.j_begin + KEYS - 1) / KEYS;
-
-  if (warp == 0) {
-    // ===================== MMA issue =====================
-    bar_named(9, 32 + 2 * ROWS);                             // the queries are in place
-    {
-      const uint32_t lead = elect_lane();
+  if (warp == 0 || warp == 13) {
+    // ===================== MMA issue: warp 0 the scores, warp 13 the outputs =====================
+    // One warp for both spent 2800 cycles on a tile: a batch is issued about as fast as it is executed (some 50 cycles an MMA), so every wait, 65..240
+    // cycles even on a barrier that is complete, left the tensor pipe idle.
+    const uint32_t lead = elect_lane();
+    auto copied = [&](int t) {                               // cp.async writes through the generic proxy; the fence costs some 300 cycles
+      int ra, rb, rv;
+      if (!pr.bulk(tl, tl.j_begin + t * KEYS, ra, rb, rv)) fence_proxy_async();
+    };
+    int st = 0, reg = 0;                                     // stage and region, counted instead of divided out
+    uint32_t ph = 0;
+    if (warp == 0) {
+      bar_named(9, 32 + 2 * ROWS);                           // the queries are in place
       fence_after();
       const uint32_t id_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KEYS >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
-      const uint32_t id_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(pr.DV >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
       const int full = pr.DK / 64, odd = pr.DK / 16 % 4;      // steps of 16 entries: four per 64, and the rest
-      auto copied = [&](int t) {                             // cp.async writes through the generic proxy; the fence costs some 300 cycles
-        int ra, rb, rv;
-        if (!pr.bulk(tl, tl.j_begin + t * KEYS, ra, rb, rv)) fence_proxy_async();
-      };
-      int k_st = 0, v_st = 0;                                // stages and their phases, counted instead of divided out
-      uint32_t k_ph = 0, v_ph = 0;
-      auto score = [&](int t) {
-        const int st = k_st;
-        mbar_wait_warp(k_full + 8 * st, k_ph, dead);
-        if (++k_st == nst) { k_st = 0; k_ph ^= 1u; }
-        if (dead) return;
+      for (int t = 0; t < n; ++t) {
+        mbar_wait(k_full + 8 * st, ph, dead);
+        if (t >= 3) mbar_wait(pv_done + 8 * reg, (uint32_t)(t / 3 - 1) & 1u, dead);      // over the weights of tile t - 3
+        dead = __any_sync(0xffffffffu, dead) ? 1u : 0u;
+        if (dead) break;
         copied(t);
         fence_after();
-        const uint32_t kb = sk + st * ka * K_ATOM, d = tmem + REGION * (t & 1) + S_AT;
+        const uint32_t kb = sk + st * ka * K_ATOM, d = tmem + REGION * reg + S_AT;
         const uint64_t kd0 = desc_sw128(kb);
         uint32_t acc = 0;
 #pragma unroll 1
@@ -299,40 +323,42 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
           }
         }
         if (lead) {
-          commit(s_full + 8 * (t & 1));
+          commit(s_full + 8 * reg);
           commit(k_empty + 8 * st);
         }
+        if (++reg == 3) reg = 0;
+        if (++st == nst) { st = 0; ph ^= 1u; }
         __syncwarp();
-      };
-      if (n > 0) score(0);                                   // an empty key split has no tile
-      if (n > 1) score(1);
-      for (int t = 0; t < n && !dead; ++t) {
-        const int st = v_st;
-        mbar_wait(v_full + 8 * st, v_ph, dead);
-        if (++v_st == nst) { v_st = 0; v_ph ^= 1u; }
-        mbar_wait_warp(p_full + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, dead);
-        if (REGS && t > 0) mbar_wait_warp(o_free, (uint32_t)(t - 1) & 1u, dead);      // the other group has taken the product before it too
+      }
+    } else {
+      const uint32_t id_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(pr.DV >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
+      for (int t = 0; t < n; ++t) {
+        mbar_wait(v_full + 8 * st, ph, dead);
+        if (REGS && t > 0) mbar_wait(o_free, (uint32_t)(t - 1) & 1u, dead);      // the group of the tile before has taken that product
+        mbar_wait_warp(p_full + 8 * (t & 1), (uint32_t)(t >> 1) & 1u, dead);     // and so has this tile's
         if (dead) break;
         copied(t);
         fence_after();
         const uint64_t vd = desc_mn(sv + st * va * K_ATOM, K_ATOM);
-        const uint32_t pc = tmem + REGION * (t & 1);
+        const uint32_t pc = tmem + REGION * reg;
 #pragma unroll 1
         for (int q = NP - 1; q >= 0; --q)
 #pragma unroll
           for (int k = 0; k < KEYS / 16; ++k) mma_ts(tmem + COL_O, pc + 24 * k + 8 * q, vd + k * (16 * 128 / 16), id_o, ((!REGS && t > 0) || q < NP - 1 || k > 0) ? 1u : 0u, lead);
         if (lead) {
+          commit(pv_done + 8 * reg);
           commit(v_empty + 8 * st);
-          commit(pv_done + 8 * (t & 1));
         }
+        if (++reg == 3) reg = 0;
+        if (++st == nst) { st = 0; ph ^= 1u; }
         __syncwarp();
-        if (t + 2 < n) score(t + 2);                         // over the weights of tile t, which the MMAs before it have read
       }
-      if (dead) {                                            // what was issued ends before tensor memory is given back
-        uint32_t late = 0;
-        if (lead) commit(gave_up);
-        mbar_wait(gave_up, 0, late);
-      }
+    }
+    if (dead) {                                              // what was issued ends before tensor memory is given back
+      const uint32_t bar = gave_up + (warp ? 8 : 0);
+      uint32_t late = 0;
+      if (lead) commit(bar);
+      mbar_wait(bar, 0, late);
     }
     __syncwarp();
   } else if (warp < 4 || warp == 12) {
@@ -390,42 +416,51 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     // ===================== queries, softmax, output =====================
     const int qtr = warp & 3, b = (warp >> 2) - 1, r = qtr * 32 + lane;      // b: the parity of the group's tiles
     const uint32_t lane_at = (uint32_t)(qtr * 32) << 16;
-    for (int g0 = b; g0 < pr.DK / 16; g0 += 8) {             // the groups take turns with 16 entries of a row; four turns' loads together
-      float x[4][16];
+    // Queries: 16-byte pieces, a warp on one row after the other, to where the parts go that the row's threads make of them (of 8 f32 entries in two
+    // pieces: to the places of the two parts in shared memory).  A row per lane kept the load unit busy with 32 lines for every instruction.
+    const int sw = warp - 4, pieces = pr.DK / (NQ > 1 ? 4 : 8);
+    auto slot = [&](int s, int c, int row) { return sq + (s * ka + (c >> 3)) * Q_ATOM + row * 128 + (((c & 7) ^ (row & 7)) << 4); };
+    if (pr.pieces()) {
+      for (int p = lane; p < pieces; p += 32)
+#pragma unroll 4
+        for (int q = sw; q < ROWS; q += 2 * ROWS / 32)
+          cp16(NQ > 1 ? slot(p & 1, p >> 1, q) : slot(0, p, q), pr.piece(tl, q < tl.rows ? q : 0, p), q < tl.rows);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      bar_named(10, 2 * ROWS);
+    }
+    // f32 queries take the scale with them, as a factor in two parts; a bf16 query, which is one part as it lies, leaves it to the weights.
+    constexpr bool FOLD = NQ > 1;
+    const float by = CAP ? pr.scale / pr.softcap : pr.scale * LOG2E, by_lo = CAP ? fmaf(-by, pr.softcap, pr.scale) / pr.softcap : fmaf(pr.scale, LOG2E, -by) + pr.scale * LOG2E_LO;
+    const float after = FOLD ? 1.f : CAP ? 1.f : by;
+#pragma unroll 1
+    for (int c = b; NQ > 1 && c < pr.DK / 8; c += 2) {        // rolled up: code that runs once is fetched at some 12 cycles an instruction
+      float x[8];
+      if (pr.pieces()) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int g = g0 + 2 * u;
+        for (int h = 0; h < 2; ++h)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[4 * h]), "=f"(x[4 * h + 1]), "=f"(x[4 * h + 2]), "=f"(x[4 * h + 3]) : "r"(slot(h, c, r)) : "memory");
+      } else {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) x[u][e] = 0.f;
-        if (r < tl.rows && g < pr.DK / 16) {
-          pr.query(tl, r, 2 * g, *reinterpret_cast<float (*)[8]>(x[u]));
-          pr.query(tl, r, 2 * g + 1, *reinterpret_cast<float (*)[8]>(x[u] + 8));
-        }
+        for (int e = 0; e < 8; ++e) x[e] = 0.f;
+        if (r < tl.rows) pr.query(tl, r, c, x);
+        __syncwarp();
       }
-      __syncwarp();
+      // scores come out in powers of two (with a cap: as its argument); rounded once
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int g = g0 + 2 * u;
-        if (g >= pr.DK / 16) break;
+      for (int e = 0; e < 8; e += 2) {
+        float lo[2] = {x[e] * by_lo, x[e + 1] * by_lo};
+        fma2(x[e], x[e + 1], by, lo[0], lo[1]);
+      }
 #pragma unroll
-        for (int s = 0; s < NQ; ++s) {
-          uint32_t w[8];
+      for (int s = 0; s < NQ; ++s) {
+        uint32_t w[4];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) w[e] = hi_pair(x[u][2 * e], x[u][2 * e + 1]);
-          if (s >= nsm) {
-            tmem_st8(tmem + lane_at + COL_Q + (s - nsm) * (pr.DK / 2) + 8 * g, w);
-          } else {
+        for (int e = 0; e < 4; ++e) w[e] = hi_pair(x[2 * e], x[2 * e + 1]);
+        if (s >= nsm) tmem_st4(tmem + lane_at + COL_Q + (s - nsm) * (pr.DK / 2) + 4 * c, w);
+        else asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slot(s, c, r)), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+        if (s + 1 < NQ) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int c = 2 * g + h;
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sq + (s * ka + (c >> 3)) * Q_ATOM + r * 128 + (((c & 7) ^ (r & 7)) << 4)), "r"(w[4 * h]),
-                           "r"(w[4 * h + 1]), "r"(w[4 * h + 2]), "r"(w[4 * h + 3]) : "memory");
-            }
-          }
-          if (s + 1 < NQ) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) x[u][e] = fabsf(x[u][e]) < INFINITY ? rest(x[u][e]) : 0.f;
-          }
+          for (int e = 0; e < 8; e += 2) sub2(x[e], x[e + 1], high_part(x[e]), high_part(x[e + 1]));      // an infinite entry: NaN, and the row is taken again
         }
       }
     }
@@ -443,15 +478,19 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     for (int i = 0; i < MAX_DV / 32; ++i)
 #pragma unroll
       for (int e = 0; e < 16; ++e) acc[i][e] = 0.f;
-    for (int t = b; t < n + (REGS ? 1 : 0); t += 2) {        // REGS, tile n: nothing but the product of tile n - 1, for the group that has not taken it
-     float base[2] = {-INFINITY, -INFINITY};                 // the references of tiles t - 1 and t
-     if (REGS && t == n) {
-      if (t > 0) bar_named(1 + 4 * (b ^ 1) + qtr, 64);
-      base[0] = s_ref[r];
-     } else {
-      mbar_wait(s_full + 8 * b, (uint32_t)(t >> 1) & 1u, dead);
+    int s_reg = b;                                           // tile t's region, and the phase of its barrier (this group meets every second one; the one
+    uint32_t s_ph = 0;                                       // between, tile t - 3, came before the scores of this group's tile before)
+    float base[2] = {-INFINITY, -INFINITY};                  // the references of tiles t - 2 and t - 1
+    uint32_t d_bar = 0, d_ph = 0;                            // REGS: barrier and phase of the next product; a group adds all of them in order
+    for (int t = b; t < n + (REGS ? 2 : 0); t += 2) {        // REGS, tiles n and n + 1: nothing but the products still to be added
+     float now = -INFINITY;
+     float mm = 0.f, scale = 1.f;
+     const uint32_t reg = tmem + lane_at + REGION * s_reg;
+     if (t < n) {
+      mbar_wait(s_full + 8 * s_reg, s_ph, dead);
       fence_after();
-      const uint32_t reg = tmem + lane_at + REGION * b;
+      s_reg += 2;
+      if (s_reg >= 3) { s_reg -= 3; s_ph ^= 1u; }
       const int at = tl.j_begin + t * KEYS, first = lo - at, last = hi - at;      // keys first .. last of these 64 are seen
       const bool cut = __any_sync(0xffffffffu, first > 0 || last < KEYS - 1);
       float mx = -INFINITY;
@@ -461,10 +500,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         tmem_ld16(reg + S_AT + 16 * c, u);
         float s[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) s[i] = __uint_as_float(u[i]) * pr.scale;
-        if (CAP) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) s[i] = pr.softcap * tanhf(s[i] / pr.softcap);
+        for (int i = 0; i < 16; ++i) {
+          s[i] = __uint_as_float(u[i]);
+          if (CAP) s[i] = pr.softcap * LOG2E * tanhf(FOLD ? s[i] : s[i] * by);
+          else if (!FOLD) s[i] *= by;
         }
         if (cut) {
 #pragma unroll
@@ -480,25 +519,24 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         for (int i = 1; i < 16; ++i) m2[i & 1] = fmaxf(m2[i & 1], s[i]);
         mx = fmaxf(m2[0], m2[1]);
       }
-      const float scale = (CAP || cut) ? 1.f : pr.scale;
+      scale = (CAP || cut) ? 1.f : after;
       if (CAP || cut) tmem_wait_st();
       // the row's reference after tile t - 1, from the other group; this tile's goes to it (barriers 1..4 even -> odd, 5..8 odd -> even)
       if (t > 0) bar_named(1 + 4 * (b ^ 1) + qtr, 64);
       const float ref = s_ref[r];
-      const bool up = mx > ref + 8.f;                        // also the first key a row sees (ref = -inf)
-      const float now = up ? mx : ref;
+      const bool up = mx > ref + 11.f;                       // also the first key a row sees (ref = -inf)
+      now = up ? mx : ref;
       if (up) s_ref[r] = now;
       if (REGS || t + 1 < n) bar_named_arrive(1 + 4 * b + qtr, 64);
-      base[0] = ref;
-      base[1] = now;
+      base[1] = ref;
       if (m != now) {
-        l *= m == -INFINITY ? 0.f : expf(m - now);
+        l *= m == -INFINITY ? 0.f : exp2_f(m - now);
         m = now;
       }
       if (!REGS) {                                           // what is in tensor memory follows the reference
-        const float f = (up && ref != -INFINITY) ? expf(ref - now) : 1.f;    // nothing was added to a row that saw no key
-        if (__any_sync(0xffffffffu, f != 1.f)) {             // t > 0 here; the scores of this tile came after PV(t - 2)
-          mbar_wait(pv_done + 8 * (b ^ 1), (uint32_t)((t - 1) >> 1) & 1u, dead);
+        const float f = (up && ref != -INFINITY) ? exp2_f(ref - now) : 1.f;    // nothing was added to a row that saw no key
+        if (__any_sync(0xffffffffu, f != 1.f)) {             // t > 0 here; the scores of this tile came after PV(t - 3), the phase before on this barrier is complete
+          mbar_wait(pv_done + 8 * ((t - 1) % 3), (uint32_t)((t - 1) / 3) & 1u, dead);
           fence_after();
           for (int g = 0; g < pr.DV / 16; ++g) {
             uint32_t o[16];
@@ -509,47 +547,25 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
           }
         }
       }
-      const float mm = m == -INFINITY ? 0.f : m;             // a row that has seen no key: every score is -inf, every weight 0
-      float sum[2] = {0.f, 0.f};
-#pragma unroll 1
-      for (int c = 0; c < KEYS / 16; ++c) {
-        uint32_t u[16];
-        tmem_ld16(reg + S_AT + 16 * c, u);
-        float s[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          s[i] = expf(__uint_as_float(u[i]) * scale - mm);
-          sum[i & 1] += s[i];
-        }
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-          uint32_t w[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            w[i] = hi_pair(s[2 * i], s[2 * i + 1]);
-            if (q + 1 < NP) { s[2 * i] = rest(s[2 * i]); s[2 * i + 1] = rest(s[2 * i + 1]); }
-          }
-          tmem_st8(reg + 24 * c + 8 * q, w);
-        }
-      }
-      l += sum[0] + sum[1];
-      tmem_wait_st();
+      mm = m == -INFINITY ? 0.f : m;                         // a row that has seen no key: every score is -inf, every weight 0
      }
-      if (!REGS) {
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_full + 8 * b);
-      }
-      // REGS: the products of tiles t - 1 and t into the registers: the first before PV(t) may overwrite it, the second while S(t + 2) is on its way
+     // REGS: the product of tile t - 2 into the registers, then this tile's weights, then the product of tile t - 1 before PV(t) may overwrite it.
+     // The product of this group's tile before comes while the other group exponentiates, and the scores of tile t + 2 need none of it.
 #pragma unroll 1
-      for (int k = 0; REGS && k < 2; ++k) {
-        const int u = t - 1 + k;
+     for (int k = 0; k < 2; ++k) {
+      if (REGS) {
+        const int u = t - 2 + k;
+        if (k == 1 && t == n && n > 0) {
+          bar_named(1 + 4 * (b ^ 1) + qtr, 64);
+          base[1] = s_ref[r];
+        }
         if (u >= 0 && u < n) {
-          mbar_wait(pv_done + 8 * (u & 1), (uint32_t)(u >> 1) & 1u, dead);
+          mbar_wait(pv_done + 8 * d_bar, d_ph, dead);
+          if (++d_bar == 3) { d_bar = 0; d_ph ^= 1u; }
           fence_after();
           const float to = k ? base[1] : base[0];
           if (__any_sync(0xffffffffu, acc_ref != to)) {
-            const float f = acc_ref == to ? 1.f : acc_ref == -INFINITY ? 0.f : expf(acc_ref - to);
+            const float f = acc_ref == to ? 1.f : acc_ref == -INFINITY ? 0.f : exp2_f(acc_ref - to);
             acc_ref = to;
 #pragma unroll
             for (int i = 0; i < MAX_DV / 32; ++i)
@@ -564,26 +580,75 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
             tmem_ld16_issue(tmem + lane_at + COL_O + 16 * (b + 2 * i + 2), o[1]);
             tmem_wait_ld(o[0], o[1]);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              acc[i][e] += __uint_as_float(o[0][e]);
-              acc[i + 1][e] += __uint_as_float(o[1][e]);
+            for (int e = 0; e < 16; e += 2) {
+              add2(acc[i][e], acc[i][e + 1], __uint_as_float(o[0][e]), __uint_as_float(o[0][e + 1]));
+              add2(acc[i + 1][e], acc[i + 1][e + 1], __uint_as_float(o[1][e]), __uint_as_float(o[1][e + 1]));
             }
           }
+          if (k == 0) {
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(o_free);
+          }
         }
-        if (t == n) break;
+      }
+      if (t >= n) continue;
+      if (k == 1) {
         fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(k ? o_free : p_full + 8 * b);
+        if (lane == 0) mbar_arrive(p_full + 8 * b);
+        continue;
       }
+      float sum[2] = {0.f, 0.f};
+#pragma unroll 1
+      for (int c = 0; c < KEYS / 16; ++c) {
+        uint32_t u[16];
+        tmem_ld16(reg + S_AT + 16 * c, u);
+        float s[16];
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          s[i] = __uint_as_float(u[i]);
+          s[i + 1] = __uint_as_float(u[i + 1]);
+          if (FOLD) sub2(s[i], s[i + 1], mm, mm);
+          else fma2(s[i], s[i + 1], scale, -mm, -mm);
+          s[i] = exp2_f(s[i]);
+          s[i + 1] = exp2_f(s[i + 1]);
+          add2(sum[0], sum[1], s[i], s[i + 1]);
+        }
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          uint32_t w[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            w[i] = hi_pair(s[2 * i], s[2 * i + 1]);
+            if (q + 1 < NP) sub2(s[2 * i], s[2 * i + 1], high_part(s[2 * i]), high_part(s[2 * i + 1]));
+          }
+          tmem_st8(reg + 24 * c + 8 * q, w);
+        }
+      }
+      l += sum[0] + sum[1];
+      tmem_wait_st();
+     }
+     base[0] = now;
     }
     // the even group ends with the sum of both (relative to the last reference); each group stores every other 16 columns.  Without REGS only
     // the group of the last tile waits for its product (the other may not have seen the phase before it, whose parity would let it pass);
     // the barriers below carry that to the other group.
     if (!REGS && n > 0 && b == ((n - 1) & 1)) {
-      mbar_wait(pv_done + 8 * b, (uint32_t)((n - 1) >> 1) & 1u, dead);
+      mbar_wait(pv_done + 8 * ((n - 1) % 3), (uint32_t)((n - 1) / 3) & 1u, dead);
       fence_after();
     }
     if (!REGS) fence_before();
+    // Gates along the rows into the memory of the queries, which every score has read by now
+    const bool staged = REGS && !pr.partial(tl) && pr.gate_pieces();
+    const uint32_t gate_row = pr.DV / 4 * sizeof(typename Prob::Gate);
+    if (staged) {
+      const int per = gate_row / 16, at_once = 32 / per, sub = lane / per, p = lane - sub * per;
+      if (sub < at_once) {
+#pragma unroll 4
+        for (int q = (warp - 4) * at_once + sub; q < tl.rows; q += 2 * ROWS / 32 * at_once) cp16(sq + q * gate_row + 16 * p, pr.gate_piece(tl, q, p), true);
+      }
+    }
     if (dead) failed = 1u;
     if (b == 1) { s_end[r] = m; s_end[ROWS + r] = l; }
     bar_named(10, 2 * ROWS);
@@ -591,7 +656,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     float* tot = s_end;                                      // [ROWS]: the sum, for both groups
     if (b == 0) {
       const float m1 = s_end[r], l1 = s_end[ROWS + r];
-      l = (m == -INFINITY ? 0.f : l * expf(m - ref)) + (m1 == -INFINITY ? 0.f : l1 * expf(m1 - ref));
+      l = (m == -INFINITY ? 0.f : l * exp2_f(m - ref)) + (m1 == -INFINITY ? 0.f : l1 * exp2_f(m1 - ref));
       tot[r] = l;
     }
     bar_named(10, 2 * ROWS);
@@ -600,36 +665,60 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     l = tot[r];
     m = ref;
     const bool part = pr.partial(tl), live = r < tl.rows;
-    const float sink = pr.sink(tl), M = fmaxf(m, sink);
-    const float e = m == -INFINITY ? 0.f : expf(m - M);
-    float inv = e / (l * e + (sink == -INFINITY ? 0.f : expf(sink - M)));
+    const float sink = pr.sink(tl), M = fmaxf(m, sink * LOG2E);
+    const float e = m == -INFINITY ? 0.f : exp2_f(m - M);
+    float inv = e / (l * e + (sink == -INFINITY ? 0.f : exp2_f(fmaf(sink, LOG2E, fmaf(sink, LOG2E_LO, -M)))));
+    if (part) {                                              // maxima outside are in powers of e: what rounding changes about this one goes into the sums
+      const float me = m == -INFINITY ? m : m * LN2;
+      inv = fabsf(me) < INFINITY ? exp2_f(fmaf(-me, LOG2E_LO, fmaf(-me, LOG2E, m))) : 1.f;
+      m = me;
+      l *= inv;
+    }
     if (dead) inv = l = __int_as_float(0x7fc00000);
     if (part && live && b == 0) pr.store_ml(tl, r, m, l);
+    if (!part && live) inv *= pr.factor(tl, r);
     float odd = part ? l * 0.f : 0.f;                        // NaN as soon as something infinite or NaN came out
-    if (REGS) {                                              // back to tensor memory: written out from the registers, 64 columns' gates and stores in a
-#pragma unroll                                               // row are more code than the instruction caches hold (10 us per CTA)
-      for (int i = 0; i < MAX_DV / 32; ++i) {
-        uint32_t o[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(acc[i][e]);
-        if (b + 2 * i < pr.DV / 16) tmem_st16(tmem + lane_at + COL_O + 16 * (b + 2 * i), o);
-      }
-      tmem_wait_st();
-    }
-#pragma unroll 1
-    for (int g = b; g < pr.DV / 16; g += 2) {
-      uint32_t o[16];
-      __syncwarp();
-      tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
-      float x[16];
+    // Outputs through shared memory (the stages are free: every product is done), rows apart by 16 bytes more than they take; then lanes side by side
+    // along a row.
+    const uint32_t row_bytes = pr.DV * 4 + 16, mine = sk + r * row_bytes;
+    auto keep = [&](int c0, float (&x)[16]) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        x[i] = n > 0 ? __uint_as_float(o[i]) * (part ? 1.f : inv) : 0.f;
+        x[i] = n > 0 ? x[i] * inv : 0.f;
         odd = fmaf(x[i], 0.f, odd);
       }
-      if (live) {
-        if (part) pr.store_part(tl, r, 16 * g, x);
-        else pr.store(tl, r, 16 * g, x);
+#pragma unroll
+      for (int i = 0; i < 16; i += 4)
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(mine + 4 * (c0 + i)), "f"(x[i]), "f"(x[i + 1]), "f"(x[i + 2]), "f"(x[i + 3]) : "memory");
+    };
+    if (REGS) {
+#pragma unroll
+      for (int i = 0; i < MAX_DV / 32; ++i)
+        if (b + 2 * i < pr.DV / 16) keep(16 * (b + 2 * i), acc[i]);
+    } else {
+#pragma unroll 1
+      for (int g = b; g < pr.DV / 16; g += 2) {
+        uint32_t o[16];
+        tmem_ld16(tmem + lane_at + COL_O + 16 * g, o);
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(o[i]);
+        keep(16 * g, x);
+      }
+    }
+    if (staged) asm volatile("cp.async.wait_all;" ::: "memory");
+    bar_named(10, 2 * ROWS);
+    const int per = pr.DV / 4, at_once = 32 / per, sub = lane / per, c0 = 4 * (lane - sub * per), stride = 2 * ROWS / 32 * at_once;      // rows a turn
+    const int first_row = sub < at_once ? sw * at_once + sub : ROWS;
+#pragma unroll 1
+    for (int k = first_row; k < tl.rows; k += stride) {
+      float x[4];
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(sk + k * row_bytes + 4 * c0) : "memory");
+      if (part) {
+        pr.store_part(tl, k, c0, x);
+      } else {
+        const typename Prob::Gate g = staged ? *reinterpret_cast<const typename Prob::Gate*>(smem_raw + CONTROL + k * gate_row + c0 / 4 * sizeof(typename Prob::Gate)) : pr.gate(tl, k, c0);
+        pr.store(tl, k, c0, x, g);
       }
     }
     const uint32_t bad = __ballot_sync(0xffffffffu, live && !dead && odd != odd);

@@ -696,6 +696,8 @@ struct LocalProb {
     const float4 u = q[0], v = q[1];
     x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
   }
+  __device__ __forceinline__ bool pieces() const { return true; }
+  __device__ __forceinline__ const void* piece(const Tile& t, int r, int p) const { return a.q + ((size_t)(t.t_first + r) * a.heads + t.h) * a.K + 4 * p; }
   __device__ __forceinline__ void range(const Tile& t, int r, int& lo, int& hi) const {
     hi = t.pos0 + t.t_first + r;
     lo = first_visible(a, hi);
@@ -703,34 +705,37 @@ struct LocalProb {
   __device__ __forceinline__ float sink(const Tile&) const { return a.has_sink ? 0.f : -INFINITY; }
   __device__ __forceinline__ bool partial(const Tile&) const { return false; }
   __device__ __forceinline__ void store_ml(const Tile&, int, float, float) const {}
-  __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[16]) const {}
-  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
-    const int tt = t.t_first + r;
-    const __nv_bfloat16* gate = (const __nv_bfloat16*)a.gate + (size_t)tt * a.ldg;
-    const float f = a.out_mult * ((a.gate && !a.gate_per_channel) ? sigmoid_f(ld_act(gate, t.h)) : 1.f);
-    const size_t o = (size_t)tt * a.ldo + (size_t)t.h * a.V + c0;
-    float y[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) y[i] = x[i] * f;
-    if (a.gate && a.gate_per_channel) {                       // 16-byte aligned rows: a condition of the launch
-      const uint4* gp = reinterpret_cast<const uint4*>(gate + (size_t)t.h * a.V + c0);
-      const uint4 g0 = gp[0], g1 = gp[1];
-      const uint32_t w[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        y[2 * i] *= sigmoid_f(__uint_as_float(w[i] << 16));
-        y[2 * i + 1] *= sigmoid_f(__uint_as_float(w[i] & 0xffff0000u));
-      }
+  __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[4]) const {}
+  struct Gate { uint2 w; };                                   // four channels' (16-byte aligned rows: a condition of the launch)
+  __device__ __forceinline__ const __nv_bfloat16* gate_at(const Tile& t, int r, int c0) const {
+    return (const __nv_bfloat16*)a.gate + (size_t)(t.t_first + r) * a.ldg + (size_t)t.h * a.V + c0;
+  }
+  __device__ __forceinline__ bool gate_pieces() const { return a.gate && a.gate_per_channel; }
+  __device__ __forceinline__ const void* gate_piece(const Tile& t, int r, int p) const { return gate_at(t, r, 8 * p); }
+  __device__ __forceinline__ Gate gate(const Tile& t, int r, int c0) const {
+    Gate g = {};
+    if (gate_pieces()) g.w = *reinterpret_cast<const uint2*>(gate_at(t, r, c0));
+    return g;
+  }
+  __device__ __forceinline__ float factor(const Tile& t, int r) const {
+    return a.out_mult * ((a.gate && !a.gate_per_channel) ? sigmoid_f(ld_act((const __nv_bfloat16*)a.gate + (size_t)(t.t_first + r) * a.ldg, t.h)) : 1.f);
+  }
+  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[4], const Gate& g) const {
+    const size_t o = (size_t)(t.t_first + r) * a.ldo + (size_t)t.h * a.V + c0;
+    float y[4] = {x[0], x[1], x[2], x[3]};
+    if (gate_pieces()) {
+      y[0] *= sigmoid_f(__uint_as_float(g.w.x << 16));
+      y[1] *= sigmoid_f(__uint_as_float(g.w.x & 0xffff0000u));
+      y[2] *= sigmoid_f(__uint_as_float(g.w.y << 16));
+      y[3] *= sigmoid_f(__uint_as_float(g.w.y & 0xffff0000u));
     }
     if (!wide) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) st_out<__nv_bfloat16>(a, o + i, y[i]);
+      for (int i = 0; i < 4; ++i) st_out<__nv_bfloat16>(a, o + i, y[i]);
     } else if (a.out_f32) {
-      float4* q = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o) = make_float4(y[0], y[1], y[2], y[3]);
     } else {
-      atc::st16_bf16(reinterpret_cast<__nv_bfloat16*>(a.out) + o, y);
+      atc::st4_bf16(reinterpret_cast<__nv_bfloat16*>(a.out) + o, y);
     }
   }
 };

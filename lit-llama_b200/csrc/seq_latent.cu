@@ -513,7 +513,7 @@ struct LatentProb {
   static constexpr bool REGS = true;
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_latent_attn_args a;
-  int DK, DV, stages, split8, q_tmem, tiled, wide;
+  int DK, DV, stages, split8, q_tmem, tiled, wide, q_wide;      // wide: rows of `out`, q_wide: pieces of the queries are 16-byte aligned
   float scale, softcap;
   struct Tile {
     int h, t_first, rows, pos0, j_begin, j_end, xa, xb, xv, row_b;
@@ -558,6 +558,11 @@ struct LatentProb {
 #pragma unroll
     for (int e = 0; e < 8; ++e) x[e] = p[e];
   }
+  __device__ __forceinline__ bool pieces() const { return q_wide; }
+  __device__ __forceinline__ const void* piece(const Tile& t, int r, int p) const {
+    const long long tt = t.t_first + r;
+    return p < 2 * split8 ? a.q_a + tt * a.ldqa_t + t.h * a.ldqa_h + 4 * p : a.q_b + tt * a.ldqb_t + t.h * a.ldqb_h + 4 * (p - 2 * split8);
+  }
   __device__ __forceinline__ void range(const Tile& t, int r, int& lo, int& hi) const {
     hi = min(t.pos0 + t.t_first + r, t.j_end - 1);
     lo = a.window > 0 ? max(0, t.pos0 + t.t_first + r - a.window + 1) : 0;
@@ -571,21 +576,39 @@ struct LatentProb {
     part(t, r)[0] = m;
     part(t, r)[1] = l;
   }
-  __device__ __forceinline__ void store_part(const Tile& t, int r, int c0, const float (&x)[16]) const {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) part(t, r)[2 + c0 + i] = x[i];
-  }
-  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[16]) const {
-    const int tt = t.t_first + r;
-    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)tt * a.ldo + (size_t)t.h * a.vdim + c0;
-    float y[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) y[i] = x[i] * (a.gate ? sigmoid_f(a.gate[(size_t)tt * a.ldg + (size_t)t.h * a.vdim + c0 + i]) : 1.f);
-    if (wide) {
-      atc::st16_bf16(o, y);
+  __device__ __forceinline__ void store_part(const Tile& t, int r, int c0, const float (&x)[4]) const {      // rows of vdim + 2 floats
+    float* q = part(t, r) + 2 + c0;
+    if (((uintptr_t)a.work & 7) == 0) {
+      reinterpret_cast<float2*>(q)[0] = make_float2(x[0], x[1]);
+      reinterpret_cast<float2*>(q)[1] = make_float2(x[2], x[3]);
     } else {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) st_act(o, i, y[i]);
+      for (int i = 0; i < 4; ++i) q[i] = x[i];
+    }
+  }
+  struct Gate { float v[4]; };
+  __device__ __forceinline__ const float* gate_at(const Tile& t, int r, int c0) const { return a.gate + (size_t)(t.t_first + r) * a.ldg + (size_t)t.h * a.vdim + c0; }
+  __device__ __forceinline__ bool gate_pieces() const { return a.gate && ((uintptr_t)a.gate & 15) == 0 && a.ldg % 4 == 0; }
+  __device__ __forceinline__ const void* gate_piece(const Tile& t, int r, int p) const { return gate_at(t, r, 4 * p); }
+  __device__ __forceinline__ Gate gate(const Tile& t, int r, int c0) const {
+    Gate g = {};
+    if (a.gate) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g.v[i] = gate_at(t, r, c0)[i];
+    }
+    return g;
+  }
+  __device__ __forceinline__ float factor(const Tile&, int) const { return 1.f; }
+  __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[4], const Gate& g) const {
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)(t.t_first + r) * a.ldo + (size_t)t.h * a.vdim + c0;
+    float y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[i] = x[i] * (a.gate ? sigmoid_f(g.v[i]) : 1.f);
+    if (wide) {
+      atc::st4_bf16(o, y);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) st_act(o, i, y[i]);
     }
   }
 };
@@ -607,6 +630,7 @@ static int launch_latent_tc(const b2l_seq_latent_attn_args* a, int splits, cudaS
   LatentProb p;
   p.a = *a; p.DK = dk; p.DV = a->vdim; p.stages = l.stages; p.split8 = dn / 8; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = 0.f;
   p.wide = al16(a->out) && a->ldo % 8 == 0;
+  p.q_wide = al16(a->q_a) && a->ldqa_t % 4 == 0 && a->ldqa_h % 4 == 0 && (a->n_b == 0 || (al16(a->q_b) && a->ldqb_t % 4 == 0 && a->ldqb_h % 4 == 0));
   // tiled copies: rows of one slot's keys counted from position 0 (only rows of visible positions are read), whole 64-column steps per part.
   // The shared part lies in the slot that the device names: its rows are reached through the map only when the rows of all slots follow one
   // another, and then from slot 0's first.

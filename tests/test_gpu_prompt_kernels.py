@@ -336,3 +336,45 @@ def test_q4_gemm_several_tiles_per_cta(M, N, K):
     want = x.double() @ ((lv.to(BF) - z) * sc).double().t()
     err = (y[:M].double() - want).norm(dim=0) / want.norm(dim=0)          # per feature: one bf16 rounding
     assert float(err.max()) < 2.0 ** -8 and bool((y[M] == 7).all())
+
+
+@pytest.mark.parametrize("T,K,V,per_channel", [(65, 128, 48, True), (130, 192, 112, True), (129, 64, 16, False), (200, 80, 128, False)])
+def test_local_attention_gates_along_the_rows(T, K, V, per_channel):
+    """Outputs stored several rows at a time (2, 1, 8 and 1 of them), gates through shared memory or one per row, rows that end within a turn."""
+    from lit_llama_b200 import _seqlib as S
+
+    H, G, win = 4, 2, 96
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    q, k, v = torch.randn(T, H, K, generator=g, device=DEV), torch.randn(T, G, K, generator=g, device=DEV).to(BF), torch.randn(T, G, V, generator=g, device=DEV).to(BF)
+    n_gate = H * V if per_channel else 8
+    gate = (torch.randn(T, n_gate, generator=g, device=DEV) * 3).to(BF)
+    gate[1, 0], gate[2, 1] = 100.0, -100.0
+    ring_k, ring_v = k.new_zeros(1, win, G, K), v.new_zeros(1, win, G, V)
+    out, meta = torch.full((T + 1, H * V), 7.0, device=DEV, dtype=BF), torch.zeros(2, dtype=torch.int32, device=DEV)
+    a = S.AttnArgs(q=q.data_ptr(), k_new=k.data_ptr(), v_new=v.data_ptr(), ldv=G * V, cache_k=ring_k.data_ptr(), cache_v=ring_v.data_ptr(), meta=meta.data_ptr(),
+                   gate=gate.data_ptr(), ldg=n_gate, gate_per_channel=int(per_channel), out=out.data_ptr(), ldo=H * V, scale=K ** -0.5, out_mult=0.5, block=win, T=T,
+                   heads=H, kv_heads=G, K=K, V=V, act_dtype=S.act_code(BF), window=win)
+    S.check(S.lib().b2l_seq_block_attention(C.byref(a), S.stream_ptr()), "attention")
+    i, j = torch.arange(T, device=DEV)[None], torch.arange(T, device=DEV)[:, None]
+    want = attend(q.double(), k.double().repeat_interleave(H // G, 1), v.double().repeat_interleave(H // G, 1), K ** -0.5, (i <= j) & (j - i < win))
+    gd = torch.sigmoid(gate.double()).view(T, H, V) if per_channel else torch.sigmoid(gate.double())[:, :H, None]
+    assert rel(out[:T].view(T, H, V), want * gd * 0.5) < 2.5e-3 and bool((out[T] == 7).all())
+
+
+def test_expanded_latent_attention_with_unaligned_queries():
+    """Queries whose rows start on 4-byte boundaries only are read entry by entry: the same bits as aligned ones."""
+    from lit_llama_b200 import _seqlib as S
+
+    T, H, dn, V = 140, 3, 64, 64
+    g = torch.Generator(device=DEV).manual_seed(9)
+    kv, q = torch.randn(T, H, V + dn, generator=g, device=DEV).to(BF), torch.randn(T, H, dn, generator=g, device=DEV)
+    odd = torch.zeros(T, H * dn + 1, device=DEV)
+    odd[:, 1:] = q.view(T, H * dn)
+    meta, outs = torch.zeros(2, dtype=torch.int32, device=DEV), []
+    for at, ld in ((q.data_ptr(), H * dn), (odd.data_ptr() + 4, H * dn + 1)):
+        out = torch.empty(T, H * V, device=DEV, dtype=BF)
+        a = S.LatentAttnArgs(q_a=at, ldqa_t=ld, ldqa_h=dn, key_a=kv.data_ptr(), ldka=H * (V + dn), hska=V + dn, meta=meta.data_ptr(), out=out.data_ptr(), ldo=H * V,
+                             scale=dn ** -0.5, T=T, heads=H, heads_per_group=1, n_a=V + dn, n_b=0, vdim=V, score_off=V, splits=1, act_dtype=S.act_code(BF))
+        S.check(S.lib().b2l_seq_latent_attention(C.byref(a), S.stream_ptr()), "latent attention")
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
