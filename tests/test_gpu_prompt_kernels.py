@@ -378,3 +378,21 @@ def test_expanded_latent_attention_with_unaligned_queries():
         S.check(S.lib().b2l_seq_latent_attention(C.byref(a), S.stream_ptr()), "latent attention")
         outs.append(out)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("act", ["sigmoid", "silu"])
+def test_gates_are_within_rounding_of_float64(act):
+    """Logistic gates in f32 from -120 to 120, infinities and NaN: expf (2 ulp), one addition and a quotient within one rounding, so 4 * 2^-24 relative
+    (negative arguments add expf's argument rounding, none: expf reduces it exactly); results below 2^-100 may be zero."""
+    from lit_llama_b200 import _seqlib as S
+
+    x = torch.cat([torch.linspace(-120, 120, 40001, device=DEV), torch.tensor([math.inf, -math.inf, math.nan, 0.0, -0.0], device=DEV)])
+    y = torch.empty_like(x)
+    S.check(S.lib().b2l_seq_unary_act(x.data_ptr(), x.numel(), y.data_ptr(), x.numel(), 1, x.numel(), S.ACT_SIGMOID if act == "sigmoid" else S.ACT_SILU, None,
+                                      S.act_code(torch.float32), S.stream_ptr()), "b2l_seq_unary_act")
+    xd = x.double()
+    want = torch.sigmoid(xd) * (1 if act == "sigmoid" else xd)
+    big = want.isfinite() & (want.abs() > 2.0 ** -100)
+    assert float(((y.double() - want).abs() / want.abs())[big].max()) < 4 * 2.0 ** -24 * 1.5
+    assert bool((y[want.isfinite() & ~big].abs() < 2.0 ** -99).all()) and float(y[-5]) == (1.0 if act == "sigmoid" else math.inf) and math.isnan(float(y[-3]))
+    assert float(y[-4]) == 0.0 if act == "sigmoid" else math.isnan(float(y[-4]))
