@@ -187,8 +187,9 @@ typedef struct {
 } b2l_seq_attn_args;
 int b2l_seq_block_attention(const b2l_seq_attn_args* a, b2l_stream_t stream);
 /* With few queries (decoding) the keys of a query are cut into chunks that run in parallel and are merged afterwards;
- * that form needs a work space of this many floats (0: this call does not use one).  Without `work` the call runs a
- * slower form that needs none.  The count depends on T, the head counts, V and the window or block, not on positions. */
+ * that form needs a work space of this many floats (0: this call does not use one).  Portions in f32 are taken by the tensor cores when they have
+ * room for keys and values as three bf16 parts each (`work` 16-byte aligned; none is asked for above 128 MB).  Without `work` the call runs a
+ * slower form that needs none.  The count depends on T, the head counts, K, V and the window or block, not on positions. */
 long long b2l_seq_block_attention_work_floats(const b2l_seq_attn_args* a);
 
 /* Differential read-out of two attention maps per head: a f32 [T, lda] holds per head [map 0 (V) | map 1 (V)];

@@ -815,6 +815,7 @@ __global__ void __launch_bounds__(128)
 struct PromptProb {
   // bf16 outputs, and the mma.sync kernel below adds in its accumulators as well (weights to 2^-17): 2048 tokens 136 us so, 161 through registers
   static constexpr bool REGS = false;
+  static constexpr int KP = 1;
   CUtensorMap map_a, map_b, map_v;
   const __nv_bfloat16* qkv;
   KvView kv;
@@ -822,7 +823,7 @@ struct PromptProb {
   const int32_t* ring_start;
   __nv_bfloat16* y;
   int T, n_head, cached;
-  int DK, DV, stages, split8, q_tmem;
+  int DK, DV, stages, v_stages, split8, q_tmem;
   float scale, softcap;
   struct Tile {
     int b, h, t_first, rows, j_begin, j_end, cap, ring, xa, xb, xv;
@@ -904,7 +905,7 @@ static int launch_prompt_tc(const __nv_bfloat16* qkv, const KvView& kv, const in
   PromptProb p;
   p.qkv = qkv; p.kv = kv; p.input_pos = input_pos; p.ring_start = ring_start; p.y = y;
   p.T = T; p.n_head = n_head; p.cached = kv.S > 0;
-  p.DK = p.DV = 128; p.stages = l.stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = 1.0f / sqrtf(128.f); p.softcap = 0.f;
+  p.DK = p.DV = 128; p.stages = l.stages; p.v_stages = l.v_stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = 1.0f / sqrtf(128.f); p.softcap = 0.f;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const long long rows = p.cached ? (long long)B * n_head * S : (long long)B * T, cols = p.cached ? 128 : 3LL * n_head * 128;
   if (int rc = tc::map_sw128(&p.map_a, bf, 2, p.cached ? kv.k : qkv, rows, cols, cols, 64, atc::KEYS)) return rc;

@@ -7,6 +7,10 @@
 // starts from zero and is added to f32 registers: 2.3e-7, 3.2e-7 and 1.2e-7 in these cases, below the f32 kernel in every size measured.
 // Three bf16 MMAs cost 3 / 32 of what the f32 FMAs cost on the CUDA cores (4096 against 128 per cycle).
 //
+// f32 keys and values (KP = 3) are cut into three rounded parts beforehand, and of the nine products the six above 2^-24 are taken: twice the MMAs
+// of bf16 keys; against the f32 FMAs on the CUDA cores 777 tokens of 8 heads, window 512, take 40 us instead of 217, with errors of 2.1e-7 instead of
+// 3.8e-7 against float64 (between a quarter and two thirds of the FMAs' in all sizes measured).
+//
 //   warp 0       issues the MMAs of the scores S(t) = Q K^T, three tiles ahead at most, warp 13 those of the outputs, P(t) V
 //   warps 1, 2   keys, warps 3, 12 values, into 128-byte swizzled rows (keys K-major, values MN-major for the second product), three
 //                stages.  Tiles of 64 consecutive rows (the fresh projections, an expanded latent) come by tiled TMA copies; tiles that touch
@@ -50,13 +54,17 @@ constexpr int MAX_DK = 192, MAX_DV = 128;
 constexpr int CONTROL = 3072;                                // barriers, tensor-memory address, row maxima
 
 __host__ __device__ inline int atoms(int d) { return (d + 63) / 64; }
-struct Layout { int stages, q_tmem; size_t smem; };
-static inline Layout layout(int nq, int dk, int dv) {
+struct Layout { int stages, v_stages, q_tmem; size_t smem; };      // no stages: the sizes do not fit
+static inline Layout layout(int nq, int dk, int dv, int kp = 1) {
   Layout l;
   l.q_tmem = nq > 1 ? 1 : 0;                                 // the smallest part of a query in tensor memory, the others in shared memory
-  const size_t q = (size_t)(nq - l.q_tmem) * atoms(dk) * Q_ATOM, st = (size_t)(atoms(dk) + atoms(dv)) * K_ATOM;
-  l.stages = CONTROL + q + 3 * st <= 227 * 1024 ? 3 : 2;
-  l.smem = CONTROL + q + l.stages * st;
+  const size_t room = 227 * 1024 - CONTROL - (size_t)(nq - l.q_tmem) * atoms(dk) * Q_ATOM, k = (size_t)kp * atoms(dk) * K_ATOM, v = (size_t)kp * atoms(dv) * K_ATOM;
+  l.stages = l.v_stages = 0;
+  while (l.stages < 3 && (l.stages + 1) * k + (l.v_stages ? l.v_stages : 1) * v <= room) {      // keys first: their products run three tiles ahead
+    ++l.stages;
+    if (l.v_stages < 3 && l.stages * k + (l.v_stages + 1) * v <= room) ++l.v_stages;
+  }
+  l.smem = 227 * 1024 - room + l.stages * k + l.v_stages * v;
   if (l.smem < 120 * 1024) l.smem = 120 * 1024;              // one CTA per SM: each takes all of tensor memory
   return l;
 }
@@ -148,9 +156,11 @@ __device__ __forceinline__ void tmem_st4(uint32_t a, const uint32_t (&r)[4]) {
 //   Gate gate(tile, r, c0)                and what outputs c0 .. c0+3 are, as it lies in memory
 //   bool gate_pieces(); const void* gate_piece(tile, r, p)      the same by 16-byte aligned pieces, where it is
 //   void store(tile, r, c0, x[4], gate)   normalised outputs c0 .. c0+3, already with the factor
+//   KP                                    parts of a key or value: 1, bf16 as they lie; 3, f32 cut beforehand, the parts `plane` rows apart in map_a and map_v
+//                                         (keys and values in Row are f32 then, and bulk() is always true)
 //   REGS                                  every tile's product is added to f32 registers: the tensor core truncates when it adds to its
 //                                         accumulator, which over many tiles is a bias towards zero (see above)
-// and the tensor maps, the host-visible ints DK, DV, stages, split8, q_tmem, floats scale, softcap.
+// and the tensor maps, the host-visible ints DK, DV, stages, v_stages, split8, q_tmem, floats scale, softcap.
 // Rows whose result is infinite or NaN, again on the CUDA cores over the keys that they see, one row after the other with the whole CTA (a key
 // per thread for the scores, three threads per value column).  The products above cannot tell an infinite key or value from NaN: the lower
 // parts of a query or weight are often zero, and a key that the row does not see, with its weight of zero, counts as well.  Where all is
@@ -183,13 +193,9 @@ __device__ __noinline__ void redo_rows(const Prob& pr, const uint32_t* s_bad, fl
         const typename Prob::Row row = pr.row(tl, j);
         s = 0.f;
         for (int c = 0; c < pr.DK / 8; ++c) {
-          const uint4 u = *reinterpret_cast<const uint4*>(c < pr.split8 ? row.ka + 8 * c : row.kb + 8 * (c - pr.split8));
-          const uint32_t k[4] = {u.x, u.y, u.z, u.w};
+          const auto* k = c < pr.split8 ? row.ka + 8 * c : row.kb + 8 * (c - pr.split8);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s = fmaf(q[8 * c + 2 * e], __uint_as_float(k[e] << 16), s);
-            s = fmaf(q[8 * c + 2 * e + 1], __uint_as_float(k[e] & 0xffff0000u), s);
-          }
+          for (int e = 0; e < 8; ++e) s = fmaf(q[8 * c + e], (float)k[e], s);
         }
         s *= pr.scale;
         if (CAP) s = pr.softcap * tanhf(s / pr.softcap);
@@ -209,7 +215,7 @@ __device__ __noinline__ void redo_rows(const Prob& pr, const uint32_t* s_bad, fl
       acc *= corr;
       m = now;
       if (grp < GROUPS && d < pr.DV)
-        for (int i = grp; i < count; i += GROUPS) acc = fmaf(w[i], __bfloat162float(pr.row(tl, j0 + i).v[d]), acc);
+        for (int i = grp; i < count; i += GROUPS) acc = fmaf(w[i], (float)pr.row(tl, j0 + i).v[d], acc);
       __syncthreads();
     }
     if (grp < GROUPS) s_acc[grp * MAX_DV + d] = acc;
@@ -243,8 +249,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   uint32_t& failed = s_bad[ROWS / 32];                       // a wait of the CTA's softmax groups ran out
   constexpr bool REGS = Prob::REGS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ka = atoms(pr.DK), va = atoms(pr.DV), nst = pr.stages, nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
-  const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + nst * ka * K_ATOM;
+  constexpr int KP = Prob::KP;
+  const int ka = atoms(pr.DK), va = atoms(pr.DV), nsm = NQ - pr.q_tmem;      // query parts 0 .. nsm-1 lie in shared memory
+  const uint32_t sq = smem_u32(smem_raw) + CONTROL, sk = sq + nsm * ka * Q_ATOM, sv = sk + pr.stages * KP * ka * K_ATOM;
   const uint32_t b0 = smem_u32(bars);
   const uint32_t k_full = b0, k_empty = b0 + 24, v_full = b0 + 48, v_empty = b0 + 72, s_full = b0 + 96, p_full = b0 + 120, pv_done = b0 + 136, gave_up = b0 + 160, o_free = b0 + 176;
   uint32_t dead = (sq & 1023u) ? 1u : 0u;                    // swizzle atoms need 1024-byte alignment (shared memory starts on one)
@@ -280,7 +287,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       int ra, rb, rv;
       if (!pr.bulk(tl, tl.j_begin + t * KEYS, ra, rb, rv)) fence_proxy_async();
     };
+    const int nst = warp ? pr.v_stages : pr.stages;
     int st = 0, reg = 0;                                     // stage and region, counted instead of divided out
+    // Keys and values of one part meet every part of a query or weight; of three parts, the products above 2^-24 (indexes two bits each)
+    static_assert(KP == 1 || (NQ == 3 && NP == 3), "three parts meet three parts");
+    constexpr int PAIRS = KP == 3 ? 6 : NQ, QS = 0x046, KS = 0x124;
     uint32_t ph = 0;
     if (warp == 0) {
       bar_named(9, 32 + 2 * ROWS);                           // the queries are in place
@@ -294,12 +305,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         if (dead) break;
         copied(t);
         fence_after();
-        const uint32_t kb = sk + st * ka * K_ATOM, d = tmem + REGION * reg + S_AT;
+        const uint32_t kb = sk + st * KP * ka * K_ATOM, d = tmem + REGION * reg + S_AT;
         const uint64_t kd0 = desc_sw128(kb);
         uint32_t acc = 0;
 #pragma unroll 1
-        for (int s = NQ - 1; s >= 0; --s) {                  // the smallest parts first
-          uint64_t kd = kd0;
+        for (int i = 0; i < PAIRS; ++i) {                    // the smallest parts first
+          const int s = KP == 3 ? QS >> 2 * i & 3 : NQ - 1 - i;
+          uint64_t kd = kd0 + (KP == 3 ? (uint32_t)((KS >> 2 * i & 3) * ka * K_ATOM) >> 4 : 0u);
           if (s >= nsm) {
             uint32_t qa = tmem + COL_Q + (s - nsm) * (pr.DK / 2);
 #pragma unroll 1
@@ -339,12 +351,15 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         if (dead) break;
         copied(t);
         fence_after();
-        const uint64_t vd = desc_mn(sv + st * va * K_ATOM, K_ATOM);
+        const uint64_t vd0 = desc_mn(sv + st * KP * va * K_ATOM, K_ATOM);
         const uint32_t pc = tmem + REGION * reg;
 #pragma unroll 1
-        for (int q = NP - 1; q >= 0; --q)
+        for (int i = 0; i < (KP == 3 ? 6 : NP); ++i) {
+          const int q = KP == 3 ? QS >> 2 * i & 3 : NP - 1 - i;
+          const uint64_t vd = vd0 + (KP == 3 ? (uint32_t)((KS >> 2 * i & 3) * va * K_ATOM) >> 4 : 0u);
 #pragma unroll
-          for (int k = 0; k < KEYS / 16; ++k) mma_ts(tmem + COL_O, pc + 24 * k + 8 * q, vd + k * (16 * 128 / 16), id_o, ((!REGS && t > 0) || q < NP - 1 || k > 0) ? 1u : 0u, lead);
+          for (int k = 0; k < KEYS / 16; ++k) mma_ts(tmem + COL_O, pc + 24 * k + 8 * q, vd + k * (16 * 128 / 16), id_o, ((!REGS && t > 0) || i > 0 || k > 0) ? 1u : 0u, lead);
+        }
         if (lead) {
           commit(pv_done + 8 * reg);
           commit(v_empty + 8 * st);
@@ -366,7 +381,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     const bool keys = warp < 3;
     const int lt = keys ? tid - 32 : (warp == 12 ? 32 : 0) + lane, r0 = lt >> 3, c0 = lt & 7;
     const int chunks = (keys ? pr.DK : pr.DV) / 8;
-    const uint32_t base = keys ? sk : sv, stage = (uint32_t)(keys ? ka : va) * K_ATOM, full = keys ? k_full : v_full, empty = keys ? k_empty : v_empty;
+    const uint32_t base = keys ? sk : sv, stage = (uint32_t)(KP * (keys ? ka : va)) * K_ATOM, full = keys ? k_full : v_full, empty = keys ? k_empty : v_empty;
+    const int nst = keys ? pr.stages : pr.v_stages;
     int st = -1;
     uint32_t phase = 0;                                      // parity of the stage's previous use
     int t = 0;
@@ -380,19 +396,25 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
       if (pr.bulk(tl, j0, row_a, row_b, row_v)) {            // 64 consecutive rows: a tiled copy per 64 columns
         if (lt == 0) {
           mbar_expect_tx(full + 8 * st, stage);
-          if (keys) {
-            for (int a = 0; a < ka; ++a) {
-              if (8 * a < pr.split8) tma_load_2d(dst0 + a * K_ATOM, &pr.map_a, tl.xa + 64 * a, row_a, full + 8 * st);
-              else tma_load_2d(dst0 + a * K_ATOM, &pr.map_b, tl.xb + 64 * a - 8 * pr.split8, row_b, full + 8 * st);
+          for (int part = 0; part < KP; ++part) {
+            const uint32_t dst = dst0 + part * (keys ? ka : va) * K_ATOM;
+            int below = 0;
+            if constexpr (KP > 1) below = part * pr.plane;
+            if (keys) {
+              for (int a = 0; a < ka; ++a) {
+                if (8 * a < pr.split8) tma_load_2d(dst + a * K_ATOM, &pr.map_a, tl.xa + 64 * a, row_a + below, full + 8 * st);
+                else tma_load_2d(dst + a * K_ATOM, &pr.map_b, tl.xb + 64 * a - 8 * pr.split8, row_b + below, full + 8 * st);
+              }
+            } else {
+              for (int a = 0; a < va; ++a) tma_load_2d(dst + a * K_ATOM, &pr.map_v, tl.xv + 64 * a, row_v + below, full + 8 * st);
             }
-          } else {
-            for (int a = 0; a < va; ++a) tma_load_2d(dst0 + a * K_ATOM, &pr.map_v, tl.xv + 64 * a, row_v, full + 8 * st);
           }
         } else {
           mbar_arrive(full + 8 * st);
         }
         continue;
       }
+      if constexpr (KP == 1) {
 #pragma unroll 2
       for (int i = 0; i < KEYS / 8; ++i) {
         const int r = r0 + 8 * i, j = j0 + r;
@@ -406,6 +428,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
         }
       }
       cp_arrive(full + 8 * st);
+      }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");         // no copy outlives its thread
     if (lt == 0) {                                           // nor a tiled one: the latest use of every stage, all landed unless a wait ran out
@@ -640,8 +663,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
     }
     if (!REGS) fence_before();
     // Gates along the rows into the memory of the queries, which every score has read by now
-    const bool staged = REGS && !pr.partial(tl) && pr.gate_pieces();
     const uint32_t gate_row = pr.DV / 4 * sizeof(typename Prob::Gate);
+    const bool staged = REGS && !pr.partial(tl) && pr.gate_pieces() && ROWS * gate_row <= nsm * ka * Q_ATOM;
     if (staged) {
       const int per = gate_row / 16, at_once = 32 / per, sub = lane / per, p = lane - sub * per;
       if (sub < at_once) {

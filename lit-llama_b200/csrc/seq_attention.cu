@@ -640,17 +640,19 @@ static int launch_tile(const b2l_seq_attn_args* a, cudaStream_t s, int cache_slo
 
 // ---- prompt portions with bf16 keys and values: the tensor-core kernel of attn_tc.cuh.  grid (heads, row tiles, 1), the tiles with the
 // most keys first.
+template <typename E>
 struct LocalProb {
   static constexpr bool REGS = true;
+  static constexpr int KP = sizeof(E) == 4 ? 3 : 1;
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_attn_args a;
-  int DK, DV, stages, split8, q_tmem, wide;             // wide: rows of `out` are 16-byte aligned
+  int DK, DV, stages, v_stages, split8, q_tmem, wide, plane;      // wide: rows of `out` are 16-byte aligned; plane: rows of a part (f32)
   float scale, softcap;
   struct Tile {
-    int h, t_first, rows, pos0, j_begin, j_end, ring0, sk, sv, xa, xb, xv;
-    const __nv_bfloat16 *kn, *vn, *ck, *cv;
+    int h, t_first, rows, pos0, j_begin, j_end, ring0, sk, sv, xa, xb, xv, j_first;
+    const E *kn, *vn, *ck, *cv;
   };
-  struct Row { const __nv_bfloat16 *ka, *kb, *v; };
+  struct Row { const E *ka, *kb, *v; };
   __device__ __forceinline__ Tile tile() const {
     Tile t;
     t.h = blockIdx.x;
@@ -668,10 +670,11 @@ struct LocalProb {
     t.xa = gk * a.K;
     t.xb = 0;
     t.xv = gv * a.V;
-    t.kn = (const __nv_bfloat16*)a.k_new + (size_t)gk * a.K;
-    t.vn = (const __nv_bfloat16*)a.v_new + (size_t)gv * a.V;
-    t.ck = (const __nv_bfloat16*)a.cache_k + (size_t)slot * a.block * t.sk + (size_t)gk * a.K;
-    t.cv = (const __nv_bfloat16*)a.cache_v + (size_t)slot * a.block * t.sv + (size_t)gv * a.V;
+    t.j_first = KP > 1 ? first_visible(a, t.pos0) : t.pos0;  // the position of map row 0
+    t.kn = (const E*)a.k_new + (size_t)gk * a.K;
+    t.vn = (const E*)a.v_new + (size_t)gv * a.V;
+    t.ck = (const E*)a.cache_k + (size_t)slot * a.block * t.sk + (size_t)gk * a.K;
+    t.cv = (const E*)a.cache_v + (size_t)slot * a.block * t.sv + (size_t)gv * a.V;
     return t;
   }
   __device__ __forceinline__ Row row(const Tile& t, int j) const {
@@ -687,9 +690,9 @@ struct LocalProb {
     return r;
   }
   __device__ __forceinline__ bool bulk(const Tile& t, int j0, int& ra, int& rb, int& rv) const {
-    ra = rv = j0 - t.pos0;                                    // rows past the portion's last read as zeros
+    ra = rv = j0 - t.j_first;                                 // rows past the portion's last read as zeros
     rb = 0;
-    return j0 >= t.pos0;
+    return KP > 1 || j0 >= t.pos0;
   }
   __device__ __forceinline__ void query(const Tile& t, int r, int c, float (&x)[8]) const {
     const float4* q = reinterpret_cast<const float4*>(a.q + ((size_t)(t.t_first + r) * a.heads + t.h) * a.K + 8 * c);
@@ -706,33 +709,31 @@ struct LocalProb {
   __device__ __forceinline__ bool partial(const Tile&) const { return false; }
   __device__ __forceinline__ void store_ml(const Tile&, int, float, float) const {}
   __device__ __forceinline__ void store_part(const Tile&, int, int, const float (&)[4]) const {}
-  struct Gate { uint2 w; };                                   // four channels' (16-byte aligned rows: a condition of the launch)
-  __device__ __forceinline__ const __nv_bfloat16* gate_at(const Tile& t, int r, int c0) const {
-    return (const __nv_bfloat16*)a.gate + (size_t)(t.t_first + r) * a.ldg + (size_t)t.h * a.V + c0;
+  struct alignas(4 * sizeof(E)) Gate { E e[4]; };              // four channels' (16-byte aligned rows: a condition of the launch)
+  __device__ __forceinline__ const E* gate_at(const Tile& t, int r, int c0) const {
+    return (const E*)a.gate + (size_t)(t.t_first + r) * a.ldg + (size_t)t.h * a.V + c0;
   }
   __device__ __forceinline__ bool gate_pieces() const { return a.gate && a.gate_per_channel; }
-  __device__ __forceinline__ const void* gate_piece(const Tile& t, int r, int p) const { return gate_at(t, r, 8 * p); }
+  __device__ __forceinline__ const void* gate_piece(const Tile& t, int r, int p) const { return gate_at(t, r, 16 / (int)sizeof(E) * p); }
   __device__ __forceinline__ Gate gate(const Tile& t, int r, int c0) const {
     Gate g = {};
-    if (gate_pieces()) g.w = *reinterpret_cast<const uint2*>(gate_at(t, r, c0));
+    if (gate_pieces()) g = *reinterpret_cast<const Gate*>(gate_at(t, r, c0));
     return g;
   }
   __device__ __forceinline__ float factor(const Tile& t, int r) const {
-    return a.out_mult * ((a.gate && !a.gate_per_channel) ? sigmoid_f(ld_act((const __nv_bfloat16*)a.gate + (size_t)(t.t_first + r) * a.ldg, t.h)) : 1.f);
+    return a.out_mult * ((a.gate && !a.gate_per_channel) ? sigmoid_f(ld_act((const E*)a.gate + (size_t)(t.t_first + r) * a.ldg, t.h)) : 1.f);
   }
   __device__ __forceinline__ void store(const Tile& t, int r, int c0, const float (&x)[4], const Gate& g) const {
     const size_t o = (size_t)(t.t_first + r) * a.ldo + (size_t)t.h * a.V + c0;
     float y[4] = {x[0], x[1], x[2], x[3]};
     if (gate_pieces()) {
-      y[0] *= sigmoid_f(__uint_as_float(g.w.x << 16));
-      y[1] *= sigmoid_f(__uint_as_float(g.w.x & 0xffff0000u));
-      y[2] *= sigmoid_f(__uint_as_float(g.w.y << 16));
-      y[3] *= sigmoid_f(__uint_as_float(g.w.y & 0xffff0000u));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y[i] *= sigmoid_f((float)g.e[i]);
     }
     if (!wide) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) st_out<__nv_bfloat16>(a, o + i, y[i]);
-    } else if (a.out_f32) {
+      for (int i = 0; i < 4; ++i) st_out<E>(a, o + i, y[i]);
+    } else if (KP > 1 || a.out_f32) {
       *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o) = make_float4(y[0], y[1], y[2], y[3]);
     } else {
       atc::st4_bf16(reinterpret_cast<__nv_bfloat16*>(a.out) + o, y);
@@ -740,20 +741,79 @@ struct LocalProb {
   }
 };
 
-static DynSmemCache g_local_tc_smem[2];
+static DynSmemCache g_local_tc_smem[4];
 
+// f32 keys and values for the tensor cores: x = hi + mid + lo, each rounded to bf16 (24 bits in three times eight), in planes of `rows` rows: row i is
+// position first_visible(pos0) + i, from the ring or the portion; 64 rows of zeros behind the last (a tile's rows end where it does).
+static int plane_rows(const b2l_seq_attn_args* a) { return a->T + (a->window > 0 ? a->window : a->block) + atc::KEYS; }
+static size_t plane_cols(const b2l_seq_attn_args* a) { return (size_t)a->kv_heads * ((a->maps > 1 ? a->maps : 1) * a->K + a->V); }
+__global__ void __launch_bounds__(128) seq_attention_planes_kernel(b2l_seq_attn_args a, __nv_bfloat16* planes, int rows) {
+  const int pos0 = a.meta[1], j0 = first_visible(a, pos0), j = j0 + (int)blockIdx.x, end = pos0 + a.T;
+  if (j >= end + atc::KEYS) return;
+  const int nk = a.kv_heads * (a.maps > 1 ? a.maps : 1) * a.K, nv = a.kv_heads * a.V;
+  const bool fresh = j >= pos0;
+  const size_t ring = (size_t)a.meta[0] * a.block + j % a.block;
+  const float* k = fresh ? (const float*)a.k_new + (size_t)(j - pos0) * nk : (const float*)a.cache_k + ring * nk;
+  const float* v = fresh ? (const float*)a.v_new + (size_t)(j - pos0) * a.ldv : (const float*)a.cache_v + ring * nv;
+  __nv_bfloat16* pv = planes + (size_t)3 * rows * nk;
+  for (int c = 8 * (int)threadIdx.x; c < nk + nv; c += 8 * 128) {
+    const bool key = c < nk;
+    const float* src = key ? k + c : v + (c - nk);
+    float x[8] = {};
+    if (j < end) {
+      *reinterpret_cast<float4*>(x) = reinterpret_cast<const float4*>(src)[0];
+      *reinterpret_cast<float4*>(x + 4) = reinterpret_cast<const float4*>(src)[1];
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+        x[2 * e] -= __uint_as_float(w[e] << 16);
+        x[2 * e + 1] -= __uint_as_float(w[e] & 0xffff0000u);
+      }
+      __nv_bfloat16* dst = key ? planes + ((size_t)p * rows + blockIdx.x) * nk + c : pv + ((size_t)p * rows + blockIdx.x) * nv + (c - nk);
+      *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+template <typename E>
 static int launch_local_tc(const b2l_seq_attn_args* a, cudaStream_t s) {
-  const atc::Layout l = atc::layout(3, a->K, a->V);
-  LocalProb p;
-  const int sk = a->kv_heads * (a->maps > 1 ? a->maps : 1) * a->K;
-  if (int rc = tc::map_sw128(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->k_new, a->T, sk, sk, 64, atc::KEYS)) return rc;
-  if (int rc = tc::map_sw128(&p.map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->v_new, a->T, (long long)a->kv_heads * a->V, a->ldv, 64, atc::KEYS)) return rc;
+  const atc::Layout l = atc::layout(3, a->K, a->V, LocalProb<E>::KP);
+  LocalProb<E> p;
+  const int sk = a->kv_heads * (a->maps > 1 ? a->maps : 1) * a->K, sv = a->kv_heads * a->V;
+  const void *keys = a->k_new, *values = a->v_new;
+  long long rows = a->T, ldv = a->ldv;
+  p.plane = 0;
+  if (sizeof(E) == 4) {
+    p.plane = plane_rows(a);
+    rows = 3LL * p.plane;
+    keys = a->work;
+    values = (const __nv_bfloat16*)a->work + rows * sk;
+    ldv = sv;
+    seq_attention_planes_kernel<<<p.plane, 128, 0, s>>>(*a, (__nv_bfloat16*)a->work, p.plane);
+    B2L_LAUNCH_CHECK("seq_attention_planes_kernel");
+  }
+  if (int rc = tc::map_sw128(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, keys, rows, sk, sk, 64, atc::KEYS)) return rc;
+  if (int rc = tc::map_sw128(&p.map_v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, values, rows, sv, ldv, 64, atc::KEYS)) return rc;
   p.map_b = p.map_a;
-  p.a = *a; p.DK = a->K; p.DV = a->V; p.stages = l.stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = a->softcap;
+  p.a = *a; p.DK = a->K; p.DV = a->V; p.stages = l.stages; p.v_stages = l.v_stages; p.split8 = 1 << 20; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = a->softcap;
   p.wide = ((uintptr_t)a->out & 15) == 0 && a->ldo % 8 == 0;
   const dim3 grid((unsigned)a->heads, (unsigned)((a->T + atc::ROWS - 1) / atc::ROWS));
-  return a->softcap > 0.f ? atc::launch<LocalProb, 3, 3, true>(p, grid, l.smem, g_local_tc_smem[1], s)
-                          : atc::launch<LocalProb, 3, 3, false>(p, grid, l.smem, g_local_tc_smem[0], s);
+  DynSmemCache* cache = g_local_tc_smem + (sizeof(E) == 4 ? 2 : 0);
+  return a->softcap > 0.f ? atc::launch<LocalProb<E>, 3, 3, true>(p, grid, l.smem, cache[1], s) : atc::launch<LocalProb<E>, 3, 3, false>(p, grid, l.smem, cache[0], s);
+}
+// Sizes the tensor-core form takes; f32 needs the planes' room (at most 128 MB: the ring of a layer that sees everything is as long as the longest sequence).
+static bool tensor_sizes(const b2l_seq_attn_args* a) {
+  return a->T >= 64 && a->K % 16 == 0 && a->K <= atc::MAX_DK && a->V % 16 == 0 && a->V <= atc::MAX_DV && (a->T + atc::ROWS - 1) / atc::ROWS <= 65535;
+}
+static long long plane_floats(const b2l_seq_attn_args* a) {
+  if (a->act_dtype != B2L_F32 || !tensor_sizes(a) || atc::layout(3, a->K, a->V, 3).stages == 0) return 0;
+  const long long n = ((long long)plane_rows(a) * (long long)plane_cols(a) * 3 + 1) / 2;
+  return n <= 32LL << 20 ? n : 0;
 }
 
 // ring[p % block] <- token p for the portion's tokens in the block of its last token (block-local) or for its last
@@ -880,9 +940,12 @@ extern "C" int b2l_seq_block_attention(const b2l_seq_attn_args* a, b2l_stream_t 
   const bool tile = !split && a->T >= 16 && al && (a->K * esz) % 16 == 0 && (a->V * esz) % 16 == 0 && a->V % 4 == 0 && a->V <= 128 &&
                     (a->ldv * esz) % 16 == 0 && gate_ok && tile_smem <= 200 * 1024;
   // bf16 keys and values of sizes the MMA takes (16 entries per step): tensor cores; else the f32 tiles
-  const bool tens = tile && a->T >= 64 && a->act_dtype == B2L_BF16 && a->K % 16 == 0 && a->K <= atc::MAX_DK && a->V % 16 == 0 && (a->T + atc::ROWS - 1) / atc::ROWS <= 65535;
-  if (tens) {
-    if (int rc = launch_local_tc(a, s)) return rc;
+  const bool tens = tile && tensor_sizes(a);
+  const long long planes = plane_floats(a);
+  if (tens && a->act_dtype == B2L_BF16) {
+    if (int rc = launch_local_tc<__nv_bfloat16>(a, s)) return rc;
+  } else if (tens && planes > 0 && a->work != nullptr && ((uintptr_t)a->work & 15) == 0 && a->work_floats >= planes) {
+    if (int rc = launch_local_tc<float>(a, s)) return rc;
   } else if (tile) {
     const int vc = (a->V + 31) / 32;
     int rc = 0;
@@ -917,6 +980,6 @@ extern "C" int b2l_seq_block_attention(const b2l_seq_attn_args* a, b2l_stream_t 
 
 extern "C" long long b2l_seq_block_attention_work_floats(const b2l_seq_attn_args* a) {
   if (a == nullptr || a->T <= 0 || a->heads <= 0 || a->kv_heads <= 0 || a->V <= 0 || a->block <= 0) return 0;
-  if (!few_queries(a)) return 0;
+  if (!few_queries(a)) return plane_floats(a);
   return (long long)a->T * a->heads * chunk_count(a) * (a->V + 2);
 }

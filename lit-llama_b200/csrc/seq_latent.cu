@@ -511,9 +511,10 @@ __global__ void seq_head_gate_kernel(const act_t* __restrict__ in, long long ld_
 // with the most keys first.
 struct LatentProb {
   static constexpr bool REGS = true;
+  static constexpr int KP = 1;
   CUtensorMap map_a, map_b, map_v;
   b2l_seq_latent_attn_args a;
-  int DK, DV, stages, split8, q_tmem, tiled, wide, q_wide;      // wide: rows of `out`, q_wide: pieces of the queries are 16-byte aligned
+  int DK, DV, stages, v_stages, split8, q_tmem, tiled, wide, q_wide;      // wide: rows of `out`, q_wide: pieces of the queries are 16-byte aligned
   float scale, softcap;
   struct Tile {
     int h, t_first, rows, pos0, j_begin, j_end, xa, xb, xv, row_b;
@@ -628,7 +629,7 @@ static int launch_latent_tc(const b2l_seq_latent_attn_args* a, int splits, cudaS
   const int dn = a->n_a - a->score_off, dk = dn + a->n_b;
   const atc::Layout l = atc::layout(3, dk, a->vdim);
   LatentProb p;
-  p.a = *a; p.DK = dk; p.DV = a->vdim; p.stages = l.stages; p.split8 = dn / 8; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = 0.f;
+  p.a = *a; p.DK = dk; p.DV = a->vdim; p.stages = l.stages; p.v_stages = l.v_stages; p.split8 = dn / 8; p.q_tmem = l.q_tmem; p.scale = a->scale; p.softcap = 0.f;
   p.wide = al16(a->out) && a->ldo % 8 == 0;
   p.q_wide = al16(a->q_a) && a->ldqa_t % 4 == 0 && a->ldqa_h % 4 == 0 && (a->n_b == 0 || (al16(a->q_b) && a->ldqb_t % 4 == 0 && a->ldqb_h % 4 == 0));
   // tiled copies: rows of one slot's keys counted from position 0 (only rows of visible positions are read), whole 64-column steps per part.

@@ -396,3 +396,35 @@ def test_gates_are_within_rounding_of_float64(act):
     assert float(((y.double() - want).abs() / want.abs())[big].max()) < 4 * 2.0 ** -24 * 1.5
     assert bool((y[want.isfinite() & ~big].abs() < 2.0 ** -99).all()) and float(y[-5]) == (1.0 if act == "sigmoid" else math.inf) and math.isnan(float(y[-3]))
     assert float(y[-4]) == 0.0 if act == "sigmoid" else math.isnan(float(y[-4]))
+
+
+@pytest.mark.parametrize("T,H,G,K,V,pos0,window,block,sink,cap", [
+    (64, 8, 2, 128, 128, 0, 512, 512, 0, 0.0), (130, 4, 1, 192, 16, 300, 96, 100, 1, 0.0), (257, 4, 2, 64, 112, 90, 0, 128, 0, 30.0), (200, 8, 8, 16, 64, 1000, 333, 333, 1, 0.0)])
+def test_f32_local_attention_in_three_parts(T, H, G, K, V, pos0, window, block, sink, cap):
+    """f32 keys and values as three bf16 parts each: older keys from the ring (entries nobody sees are NaN), windows and blocks, room that nothing has
+    written yet, and the f32 tiles without room.  Products above 2^-24 are kept and every tile's sum is rounded: the bound of f32 sums at the top."""
+    from lit_llama_b200 import _seqlib as S
+
+    n, g, f32 = pos0 + T, torch.Generator(device=DEV).manual_seed(T + K), torch.float32
+    q, k, v = torch.randn(T, H, K, generator=g, device=DEV), torch.randn(n, G, K, generator=g, device=DEV), torch.randn(n, G, V, generator=g, device=DEV)
+    ring_k, ring_v = k.new_full((1, block, G, K), math.nan), v.new_full((1, block, G, V), math.nan)
+    old = torch.arange(max(0, pos0 - window + 1) if window else pos0 // block * block, pos0, device=DEV)
+    ring_k[0, old % block], ring_v[0, old % block] = k[old], v[old]
+    kn, vn, meta = k[pos0:].contiguous(), v[pos0:].contiguous(), torch.tensor([0, pos0], dtype=torch.int32, device=DEV)
+    gate = torch.randn(T, H * V, generator=g, device=DEV)
+    i, j = torch.arange(n, device=DEV)[None], torch.arange(pos0, n, device=DEV)[:, None]
+    seen = (i <= j) & ((j - i < window) if window else (i // block == j // block))
+    want = attend(q.double(), k.double().repeat_interleave(H // G, 1), v.double().repeat_interleave(H // G, 1), K ** -0.5, seen,
+                  torch.zeros(H, device=DEV, dtype=torch.float64) if sink else None, cap) * torch.sigmoid(gate.double()).view(T, H, V)
+    for room in (True, False):
+        out = torch.full((T + 1, H * V), 7.0, device=DEV)
+        a = S.AttnArgs(q=q.data_ptr(), k_new=kn.data_ptr(), v_new=vn.data_ptr(), ldv=G * V, cache_k=ring_k.data_ptr(), cache_v=ring_v.data_ptr(), meta=meta.data_ptr(),
+                       gate=gate.data_ptr(), ldg=H * V, gate_per_channel=1, out=out.data_ptr(), ldo=H * V, scale=K ** -0.5, softcap=cap, has_sink=sink, out_mult=1.0,
+                       block=block, T=T, heads=H, kv_heads=G, K=K, V=V, act_dtype=S.act_code(f32), window=window, no_append=1)
+        floats = S.lib().b2l_seq_block_attention_work_floats(C.byref(a))
+        work = torch.full((floats,), math.nan, device=DEV)
+        if room:
+            assert floats > 0
+            a.work, a.work_floats = work.data_ptr(), floats
+        S.check(S.lib().b2l_seq_block_attention(C.byref(a), S.stream_ptr()), "attention")
+        assert rel(out[:T].view(T, H, V), want) < 2e-6 and bool((out[T] == 7).all())
