@@ -58,6 +58,10 @@ int b2l_seq_gated_act(const void* gu, int ldgu, void* out, int T, int F, int act
 int b2l_seq_unary_act(const void* in, int ldin, void* out, int ldout, int T, int F, int act, const float* coef, int act_dtype,
                       b2l_stream_t stream);
 
+/* y[M, N] = x[M, K] . w[N, K]^T, operands, sums and results f32, on the tensor cores (three bf16 parts per operand).  K a multiple of 8, rows of x
+ * and w 16-byte aligned (leading dimensions multiples of 4). */
+int b2l_seq_linear_f32(const float* x, long long ldx, const float* w, long long ldw, float* y, long long ldy, int M, int N, int K, b2l_stream_t stream);
+
 /* Short causal convolution over time per channel, then silu, with the last taps-1 inputs of the sequence carried
  * in `state` ([n_slots][taps-1][C] act, oldest first; a fresh slot holds zeros):
  *   out[t, c] = silu(bias[c] + sum_j w[c, taps-1-j] * in[t-j, c]),  in[<0] from the state.

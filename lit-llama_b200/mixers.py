@@ -106,14 +106,34 @@ def share_weights(mixer, name: str):
 FEW_TOKENS = 4          # up to this many tokens a mechanism may run its products in its own kernels, without the library
 
 
+#: rows x outputs from which an f32 product runs on the tensor cores: below, too few tiles for the SMs and the library is as fast
+#: (us here / library: 64 x 1024 -> 1024 32 / 31, 64 x 1024 -> 2560 33 / 34, 256 x 1024 -> 1024 32 / 34, 128 x 1024 -> 2560 33 / 45, 64 x 2048 -> 5120 49 / 75)
+LINEAR_F32_FROM = 1 << 18
+
+
+def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether b2l_seq_linear_f32 takes x W^T: plain f32 matrices with 16-byte aligned rows, and a caller who asked for full f32 products without autograd."""
+    return (x.shape[0] * w.shape[0] >= LINEAR_F32_FROM and x.dim() == 2 and w.dim() == 2 and x.is_cuda and w.device == x.device and w.dtype == torch.float32
+            and x.shape[1] == w.shape[1] and x.shape[1] % 8 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0
+            and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter)
+            and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
+            and not torch.is_autocast_enabled() and not torch.backends.cuda.matmul.allow_tf32)
+
+
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    if x.dtype == torch.float32 and _f32_product(x, w):
+        y = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
+        S.check(S.lib().b2l_seq_linear_f32(_p(x), x.stride(0), _p(w), w.stride(0), _p(y), w.shape[0], x.shape[0], w.shape[0], x.shape[1], S.stream_ptr()),
+                "b2l_seq_linear_f32")
+        return y
     return F.linear(x, w)
 
 
 def linear_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """x W^T with the f32 accumulator kept (bf16 operands), or the plain f32 product."""
     if x.dtype == torch.float32:
-        return F.linear(x, w)
+        return linear(x, w)
     return torch.mm(x, w.t(), out_dtype=torch.float32)
 
 

@@ -428,3 +428,25 @@ def test_f32_local_attention_in_three_parts(T, H, G, K, V, pos0, window, block, 
             a.work, a.work_floats = work.data_ptr(), floats
         S.check(S.lib().b2l_seq_block_attention(C.byref(a), S.stream_ptr()), "attention")
         assert rel(out[:T].view(T, H, V), want) < 2e-6 and bool((out[T] == 7).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 8), (17, 130, 72), (113, 300, 64), (70, 2200, 1000), (300, 1025, 200)])
+def test_f32_linear_in_three_parts(M, N, K):
+    """Token tiles of 16 to 112, ragged features, k that ends within a stage, rows apart; infinite and NaN operands come out as FMAs give them.
+    Sums of 64 products of 2^-24 relative error each, rounded once per 64 k: far below sqrt(K) 2^-24."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x, w = torch.randn(M, K + 4, generator=g, device=DEV)[:, :K], torch.randn(N, K + 8, generator=g, device=DEV)[:, :K]
+    y = torch.full((M + 1, N + 1), 7.0, device=DEV)
+
+    def run():
+        S.check(S.lib().b2l_seq_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), y.data_ptr(), N + 1, M, N, K, S.stream_ptr()), "b2l_seq_linear_f32")
+        assert bool((y[M] == 7).all()) and bool((y[:, N] == 7).all())
+        return y[:M, :N]
+
+    assert rel(run(), x.double() @ w.double().t()) < 4e-7
+    x[0, 1], w[N // 2, 2], w[N - 1] = math.inf, math.nan, w[N - 1] * 1e30
+    x[M - 1] *= 1e12
+    want, got = torch.nn.functional.linear(x, w), run()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got == math.inf, want == math.inf) and torch.equal(got == -math.inf, want == -math.inf)
