@@ -87,6 +87,8 @@ class Lugovik:
     """The model over a dict of device tensors in the activation dtype (torch.bfloat16, or torch.float32 for true
     32-bit arithmetic throughout)."""
 
+    portion_graph_safe = True      # every launch of a portion follows from its length
+
     def __init__(self, config: LugovikConfig, weights: Dict[str, torch.Tensor], max_positions: int = 0) -> None:
         self.config = config
         self.embed = weights["embed"].contiguous()

@@ -585,3 +585,25 @@ def test_llama_is_served_by_the_same_engine():
     model.reset_cache()
     engine = P.Engine(LLaMASequenceModel(model, 32), n_slots=1)
     assert engine.generate(prompt, 8) == want
+
+
+@pytest.mark.parametrize("keep", [1, 4])
+def test_portions_of_a_recurring_length_are_replayed(keep):
+    """Two lengths and numbers of places in turn, at starts and in slots that change: recorded after two eager portions each, and logits and states are the
+    same bits as an engine's that never records; with room for one graph each new length drops the other."""
+    from lit_llama_b200 import Engine
+
+    cfg = cfg_b()
+    a, _ = build(cfg, torch.bfloat16, n_slots=2)
+    b = Engine(a.model, n_slots=2)
+    a.portion_graphs, b.portion_graph_after = keep, 0
+    toks = tokens_for(cfg, 200, seed=3)
+    for turn in range(6):
+        for rid, n, want in (("x", 17, [16]), ("y", 33, [0, 5, 31]), ("x", 17, []), ("y", 33, [30, 31, 32])):
+            part = toks[7 * turn: 7 * turn + n]
+            end = [rid] if turn in (2, 4) and len(want) in (0, 3) else []
+            one, two = (e.step([{"id": rid, "tokens": part, "want": want}], end=end)[0] for e in (a, b))
+            assert torch.equal(one, two)
+        assert all(torch.equal(a.pool.tensors[k], b.pool.tensors[k]) for k in b.pool.tensors)
+    graphs = [e for e in a._portions.values() if not isinstance(e, int)]
+    assert len(graphs) == min(keep, 3) and not b._portions
