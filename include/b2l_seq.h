@@ -89,6 +89,11 @@ typedef struct {
 } b2l_seq_conv_rope_args;
 int b2l_seq_conv_rope(const b2l_seq_conv_rope_args* a, b2l_stream_t stream);
 
+/* b2l_seq_conv_silu, then b2l_seq_unit_norm over the heads at channel q_at (times q_mult) and at k_at (times k_mult): in one pass where the long bf16
+ * form runs and a head's channels lie in one warp. */
+int b2l_seq_conv_silu_unit(const void* in, int ldin, const void* w, const void* bias, void* state, const int* meta, float* out, int ldout, int T, int C, int taps,
+                           int q_at, int k_at, int heads, int size, float eps, float q_mult, float k_mult, int act_dtype, b2l_stream_t stream);
+
 /* In place on f32: every block of `size` becomes x * mult / sqrt(sum(x^2) + eps). */
 int b2l_seq_unit_norm(float* x, int ld, int T, int heads, int size, float eps, float mult, b2l_stream_t stream);
 

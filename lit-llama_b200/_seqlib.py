@@ -146,6 +146,8 @@ _SIGS = {
     "b2l_seq_linear_f32": (c_int, [c_void_p, C.c_longlong, c_void_p, C.c_longlong, c_void_p, C.c_longlong, c_int, c_int, c_int, c_void_p]),
     "b2l_seq_conv_silu": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                   c_void_p]),
+    "b2l_seq_conv_silu_unit": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                       c_float, c_float, c_float, c_int, c_void_p]),
     "b2l_seq_unit_norm": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p]),
     "b2l_seq_decay": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                               c_void_p]),

@@ -26,7 +26,19 @@ __device__ __forceinline__ float over_f(float x, float y) {
 }
 __device__ __forceinline__ float sigmoid_f(float z) { return over_f(1.0f, 1.0f + expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return over_f(z, 1.0f + expf(-z)); }
-__device__ __forceinline__ float softplus_f(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
+// log(1 + e^z) = max(z, 0) + log(1 + u), u = e^-|z| <= 1, and log(1 + u) = 2 atanh(s), s = u / (2 + u) <= 1/3, by atanh's series to s^15 (the next term is
+// below 2e-9 of the sum): no branch and some 20 operations, where log1pf(expf(z)) took twice as many.
+__device__ __forceinline__ float softplus_f(float z) {
+  const float u = expf(-fabsf(z)), s = over_f(u, 2.0f + u), t = s * s;
+  float p = 1.0f / 15.0f;
+  p = fmaf(p, t, 1.0f / 13.0f);
+  p = fmaf(p, t, 1.0f / 11.0f);
+  p = fmaf(p, t, 1.0f / 9.0f);
+  p = fmaf(p, t, 1.0f / 7.0f);
+  p = fmaf(p, t, 1.0f / 5.0f);
+  p = fmaf(p, t, 1.0f / 3.0f);
+  return fmaxf(z, 0.0f) + 2.0f * fmaf(p * t, s, s);
+}
 __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }

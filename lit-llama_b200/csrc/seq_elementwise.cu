@@ -207,8 +207,8 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
 }
 
 // Four taps over long portions in bf16: a thread owns 8 neighbouring channels (16-byte loads, two 16-byte stores) and CONV_VT tokens, so the
-// bytes in flight suffice for HBM (6144 channels x 2048 tokens: 39 us, 73 one channel at a time); sums in the order of the kernel above.
-constexpr int CONV_VT = 16, CONV_V = 8;
+// bytes in flight suffice for HBM (6144 channels x 2048 tokens: 30 us with the unit heads, 35 with 16 tokens a thread, 73 one channel at a time); sums in the order of the kernel above.
+constexpr int CONV_VT = 8, CONV_V = 8;
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -218,11 +218,15 @@ __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) 
     x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
 }
+// UNIT: the heads of `size` channels at a0 .. and at b0 .. become unit vectors times ma or mb on the way (size / 8 neighbouring lanes hold a head).
+struct UnitHeads { int a0, a1, b0, b1, size; float eps, ma, mb; };
+template <bool UNIT>
 __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16* __restrict__ in, int ldin, const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ state,
-                                                            const int* __restrict__ meta, float* __restrict__ out, int ldout, int T, int C) {
-  const int c = (blockIdx.x * 128 + threadIdx.x) * CONV_V;
-  if (c >= C) return;
+                                                            const int* __restrict__ meta, float* __restrict__ out, int ldout, int T, int C, UnitHeads u) {
+  const int c0 = (blockIdx.x * 128 + threadIdx.x) * CONV_V, c = min(c0, C - CONV_V);      // lanes past the last channel repeat it
+  const float mult = !UNIT ? 0.f : c >= u.a0 && c < u.a1 ? u.ma : c >= u.b0 && c < u.b1 ? u.mb : 0.f;
+  const bool any = UNIT && __any_sync(0xffffffffu, mult != 0.f);
   const int t0 = blockIdx.y * CONV_VT, nt = min(CONV_VT, T - t0);
   const __nv_bfloat16* st = state + (size_t)meta[0] * 3 * C;
   float wr[4][8], win[3][8], b[8];
@@ -260,7 +264,17 @@ __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16
       win[1][e] = win[2][e];
       win[2][e] = cur[e];
     }
+    if (any) {
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += y[e] * y[e];
+      for (int d = 1; d < u.size / CONV_V; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+      const float f = mult != 0.f ? mult / sqrtf(ss + u.eps) : 1.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) y[e] *= f;
+    }
     float4* o = reinterpret_cast<float4*>(out + (size_t)(t0 + r) * ldout + c);
+    if (c0 >= C) continue;
     o[0] = make_float4(y[0], y[1], y[2], y[3]);
     o[1] = make_float4(y[4], y[5], y[6], y[7]);
   }
@@ -316,6 +330,34 @@ __global__ void seq_decay_kernel(const act_t* __restrict__ a, int lda, const act
   }
 }
 
+// The same for bf16 layers whose heads are whole groups of 8 channels: a thread owns 8 channels (one 16-byte load, two stores), so a head's coefficient is
+// formed once for them (2048 channels x 2048 tokens: 23 us one channel at a time, now 8; 24 MB move).
+__device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]);
+__global__ void __launch_bounds__(256) seq_decay8_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ bias,
+                                                        const __nv_bfloat16* __restrict__ A_log, int mode, float inv_tau, float* __restrict__ out,
+                                                        float* __restrict__ dt_out, int n, int size) {
+  const int j = 8 * (blockIdx.y * blockDim.x + threadIdx.x);
+  if (j >= n) return;
+  float z[8], b[8] = {}, r[8], dt[8];
+  ld8_bf16(a + (size_t)blockIdx.x * lda + j, z);
+  if (bias) ld8_bf16(bias + j, b);
+  const float coef = mode == B2L_SEQ_DECAY_EXP_SOFTPLUS ? -expf(__bfloat162float(A_log[j / size])) : 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    z[e] += b[e];
+    dt[e] = softplus_f(mode == B2L_SEQ_DECAY_EXP_SOFTPLUS ? z[e] : -z[e]);
+    r[e] = expf(mode == B2L_SEQ_DECAY_EXP_SOFTPLUS ? coef * dt[e] : -dt[e] * inv_tau);
+  }
+  float4* o = reinterpret_cast<float4*>(out + (size_t)blockIdx.x * n + j);
+  o[0] = make_float4(r[0], r[1], r[2], r[3]);
+  o[1] = make_float4(r[4], r[5], r[6], r[7]);
+  if (dt_out && mode == B2L_SEQ_DECAY_EXP_SOFTPLUS) {
+    float4* d = reinterpret_cast<float4*>(dt_out + (size_t)blockIdx.x * n + j);
+    d[0] = make_float4(dt[0], dt[1], dt[2], dt[3]);
+    d[1] = make_float4(dt[4], dt[5], dt[6], dt[7]);
+  }
+}
+
 // One warp per (token, group).
 template <typename act_t>
 __global__ void seq_group_norm_gate_kernel(const float* __restrict__ o, int ldo, const act_t* __restrict__ w, int w_shared,
@@ -346,6 +388,43 @@ __global__ void seq_group_norm_gate_kernel(const float* __restrict__ o, int ldo,
     if (gp && !gate_first) v *= gate_of(i);
     st_act(q, i, v);
   }
+}
+
+// The same for bf16 groups of 32 PER channels: a lane owns PER neighbouring ones and keeps them in registers (2048 tokens of 16 groups of 128: 16 us
+// with two-byte accesses, now 7; 32 MB move).
+template <int PER>
+__global__ void __launch_bounds__(128) seq_group_norm_gate_vec_kernel(const float* __restrict__ o, int ldo, const __nv_bfloat16* __restrict__ w, int w_shared,
+                                                                     const __nv_bfloat16* __restrict__ gate, int ldg, int gate_act, int gate_first, float eps,
+                                                                     float out_mult, __nv_bfloat16* __restrict__ out, int ldout, int n_rows, int groups) {
+  const int id = blockIdx.x * 4 + (threadIdx.x >> 5), c = (threadIdx.x & 31) * PER;
+  if (id >= n_rows * groups) return;
+  const int t = id / groups, at = (id - t * groups) * (32 * PER) + c;
+  struct alignas(2 * PER) Row { __nv_bfloat16 e[PER]; };
+  float v[PER], g[PER];
+#pragma unroll
+  for (int i = 0; i < PER; i += 4) *reinterpret_cast<float4*>(&v[i]) = *reinterpret_cast<const float4*>(o + (size_t)t * ldo + at + i);
+  const Row wr = *reinterpret_cast<const Row*>(w + (w_shared ? c : at));
+  if (gate) {
+    const Row gr = *reinterpret_cast<const Row*>(gate + (size_t)t * ldg + at);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const float z = __bfloat162float(gr.e[i]);
+      g[i] = gate_act == B2L_SEQ_ACT_SILU ? silu_f(z) : (gate_act == B2L_SEQ_ACT_SIGMOID ? sigmoid_f(z) : gelu_tanh_f(z));
+      if (gate_first) v[i] *= g[i];
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) ss += v[i] * v[i];
+  const float r = out_mult / sqrtf(warp_sum(ss) / (float)(32 * PER) + eps);
+  Row y;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    float x = v[i] * r * __bfloat162float(wr.e[i]);
+    if (gate && !gate_first) x *= g[i];
+    y.e[i] = __float2bfloat16_rn(x);
+  }
+  *reinterpret_cast<Row*>(out + (size_t)t * ldout + at) = y;
 }
 
 // The same for large groups (a whole layer's channels normalised together): one CTA per (token, group).
@@ -484,8 +563,9 @@ extern "C" int b2l_seq_gated_act(const void* gu, int ldgu, void* out, int T, int
   return 0;
 }
 
-extern "C" int b2l_seq_conv_silu(const void* in, int ldin, const void* w, const void* bias, void* state, const int* meta,
-                                 float* out, int ldout, int T, int C, int taps, int act_dtype, b2l_stream_t stream) {
+// `unit`: heads to normalise; done here where the four-tap kernel runs (*unit_done), left to the caller otherwise
+static int conv_silu(const void* in, int ldin, const void* w, const void* bias, void* state, const int* meta, float* out, int ldout, int T, int C, int taps, int act_dtype,
+                     const UnitHeads* unit, bool* unit_done, b2l_stream_t stream) {
   B2L_CHECK_ARG(in && w && (state || taps == 1) && meta && out, "b2l_seq_conv_silu: null pointer");
   B2L_CHECK_ARG(T >= 0 && C > 0 && ldin >= C && ldout >= C, "b2l_seq_conv_silu: bad size");
   B2L_CHECK_SUPPORTED(taps >= 1 && taps <= CONV_MAX_TAPS, "b2l_seq_conv_silu: taps %d outside 1..%d", taps, CONV_MAX_TAPS);
@@ -494,8 +574,14 @@ extern "C" int b2l_seq_conv_silu(const void* in, int ldin, const void* w, const 
   dim3 grid((unsigned)((C + 127) / 128), (unsigned)tiles);
   if (act_dtype == B2L_BF16 && taps == 4 && T > CONV_TT && C % CONV_V == 0 && ldin % 8 == 0 && ldout % 4 == 0 && al16(in) && al16(w) && al16(state) && al16(out) &&
       (T + CONV_VT - 1) / CONV_VT <= 65535) {
-    seq_conv4_silu_kernel<<<dim3((unsigned)((C / CONV_V + 127) / 128), (unsigned)((T + CONV_VT - 1) / CONV_VT)), 128, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)in, ldin, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)state, meta, out, ldout, T, C);
+    const dim3 grid4((unsigned)((C / CONV_V + 127) / 128), (unsigned)((T + CONV_VT - 1) / CONV_VT));
+    const int lanes = unit ? unit->size / CONV_V : 0;
+    const bool fits = unit && unit->size % CONV_V == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && unit->a0 % unit->size == 0 && unit->b0 % unit->size == 0 &&
+                      unit->ma != 0.f && unit->mb != 0.f;
+    auto kernel = fits ? seq_conv4_silu_kernel<true> : seq_conv4_silu_kernel<false>;
+    kernel<<<grid4, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)state, meta, out, ldout,
+                                                    T, C, fits ? *unit : UnitHeads{});
+    if (unit_done) *unit_done = fits;
     seq_conv_state_kernel<__nv_bfloat16><<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (__nv_bfloat16*)state, meta, T, C, taps);
     B2L_LAUNCH_CHECK("seq_conv4_silu_kernel");
     return 0;
@@ -508,6 +594,22 @@ extern "C" int b2l_seq_conv_silu(const void* in, int ldin, const void* w, const 
   });
   B2L_LAUNCH_CHECK("seq_conv_silu_kernel");
   return 0;
+}
+
+extern "C" int b2l_seq_conv_silu(const void* in, int ldin, const void* w, const void* bias, void* state, const int* meta,
+                                 float* out, int ldout, int T, int C, int taps, int act_dtype, b2l_stream_t stream) {
+  return conv_silu(in, ldin, w, bias, state, meta, out, ldout, T, C, taps, act_dtype, nullptr, nullptr, stream);
+}
+
+extern "C" int b2l_seq_conv_silu_unit(const void* in, int ldin, const void* w, const void* bias, void* state, const int* meta, float* out, int ldout, int T, int C, int taps,
+                                      int q_at, int k_at, int heads, int size, float eps, float q_mult, float k_mult, int act_dtype, b2l_stream_t stream) {
+  B2L_CHECK_ARG(heads > 0 && size > 0 && q_at >= 0 && k_at >= 0 && q_at + heads * size <= C && k_at + heads * size <= C, "b2l_seq_conv_silu_unit: heads outside the channels");
+  const UnitHeads u{q_at, q_at + heads * size, k_at, k_at + heads * size, size, eps, q_mult, k_mult};
+  bool done = false;
+  if (int rc = conv_silu(in, ldin, w, bias, state, meta, out, ldout, T, C, taps, act_dtype, &u, &done, stream)) return rc;
+  if (done || T == 0) return 0;
+  if (int rc = b2l_seq_unit_norm(out + q_at, ldout, T, heads, size, eps, q_mult, stream)) return rc;
+  return b2l_seq_unit_norm(out + k_at, ldout, T, heads, size, eps, k_mult, stream);
 }
 
 extern "C" int b2l_seq_cast_f32(const void* in, int ldin, float* out, int ldout, int T, int n, int act_dtype, b2l_stream_t stream) {
@@ -538,6 +640,13 @@ extern "C" int b2l_seq_decay(const void* a, int lda, const void* bias, const voi
   B2L_CHECK_ARG(mode != B2L_SEQ_DECAY_SIGMOID_ROOT || tau > 0.f, "b2l_seq_decay: tau must be positive");
   if (T == 0) return 0;
   const int n = heads * size;
+  if (act_dtype == B2L_BF16 && size % 8 == 0 && lda % 8 == 0 && al16(a) && al16(out) && (!bias || al16(bias)) && (!dt_out || al16(dt_out))) {
+    const int threads = n >= 2048 ? 256 : 64;
+    seq_decay8_kernel<<<dim3((unsigned)T, (unsigned)((n / 8 + threads - 1) / threads)), threads, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)A_log, mode, mode == B2L_SEQ_DECAY_SIGMOID_ROOT ? 1.0f / tau : 0.f, out, dt_out, n, size);
+    B2L_LAUNCH_CHECK("seq_decay8_kernel");
+    return 0;
+  }
   dim3 grid((unsigned)T, (unsigned)std::min((n + 255) / 256, 64));
   B2L_SEQ_DISPATCH(act_dtype, (seq_decay_kernel<act_t><<<grid, 256, 0, (cudaStream_t)stream>>>(
                                   (const act_t*)a, lda, (const act_t*)bias, (const act_t*)A_log, mode, mode == B2L_SEQ_DECAY_SIGMOID_ROOT ? 1.0f / tau : 0.f,
@@ -553,6 +662,17 @@ extern "C" int b2l_seq_group_norm_gate(const float* o, int ldo, const void* w, i
   B2L_CHECK_ARG(T >= 0 && n > 0 && group > 0 && n % group == 0 && ldo >= n && ldout >= n, "b2l_seq_group_norm_gate: bad size");
   if (T == 0) return 0;
   const int ids = T * (n / group);
+  auto al = [](const void* p, int bytes) { return ((uintptr_t)p & (bytes - 1)) == 0; };
+  if (act_dtype == B2L_BF16 && (group == 128 || group == 256) && ldo % 4 == 0 && al16(o)) {
+    const int per = group / 32;
+    if (ldout % per == 0 && al(out, 2 * per) && al(w, 2 * per) && (!gate || (ldg % per == 0 && al(gate, 2 * per)))) {
+      auto kernel = per == 4 ? seq_group_norm_gate_vec_kernel<4> : seq_group_norm_gate_vec_kernel<8>;
+      kernel<<<(ids + 3) / 4, 128, 0, (cudaStream_t)stream>>>(o, ldo, (const __nv_bfloat16*)w, w_shared, (const __nv_bfloat16*)gate, ldg, gate_act, gate_first, eps, out_mult,
+                                                              (__nv_bfloat16*)out, ldout, T, n / group);
+      B2L_LAUNCH_CHECK("seq_group_norm_gate_vec_kernel");
+      return 0;
+    }
+  }
   B2L_SEQ_DISPATCH(act_dtype, {
     if (group >= 512)
       seq_group_norm_gate_block_kernel<act_t><<<ids, 256, 0, (cudaStream_t)stream>>>(

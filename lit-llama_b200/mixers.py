@@ -240,10 +240,9 @@ class ChannelDeltaMixer:
         a = linear(proj[:, self.o_a1:self.o_a1 + self.rank_a], self.w_a2)    # [T, H*K]
         gate = linear(proj[:, self.o_g1:self.o_g1 + self.rank_g], self.w_g2)  # [T, H*V]
         qkv = torch.empty((T, self.C), dtype=torch.float32, device=dev)
-        S.check(lib.b2l_seq_conv_silu(_p(proj), self.n_in, _p(self.w_conv), None, _p(ctx.state[self.name + ".conv"]), _p(ctx.meta),
-                                      _p(qkv), self.C, T, self.C, self.taps, ctx.act, ctx.stream), "b2l_seq_conv_silu")
-        S.check(lib.b2l_seq_unit_norm(_p(qkv, self.o_q), self.C, T, self.G, self.K, self.unit_eps, self.K ** -0.5, ctx.stream), "b2l_seq_unit_norm")
-        S.check(lib.b2l_seq_unit_norm(_p(qkv, self.o_k), self.C, T, self.G, self.K, self.unit_eps, 1.0, ctx.stream), "b2l_seq_unit_norm")
+        S.check(lib.b2l_seq_conv_silu_unit(_p(proj), self.n_in, _p(self.w_conv), None, _p(ctx.state[self.name + ".conv"]), _p(ctx.meta), _p(qkv), self.C, T,
+                                           self.C, self.taps, self.o_q, self.o_k, self.G, self.K, self.unit_eps, self.K ** -0.5, 1.0, ctx.act, ctx.stream),
+                "b2l_seq_conv_silu_unit")
         g = torch.empty((T, self.H * self.K), dtype=torch.float32, device=dev)
         S.check(lib.b2l_seq_decay(_p(a), self.H * self.K, _p(self.dt_bias), _p(self.A_log), S.DECAY_EXP_SOFTPLUS, 0.0, _p(g), None, T,
                                   self.H, self.K, ctx.act, ctx.stream), "b2l_seq_decay")

@@ -450,3 +450,52 @@ def test_f32_linear_in_three_parts(M, N, K):
     x[M - 1] *= 1e12
     want, got = torch.nn.functional.linear(x, w), run()
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got == math.inf, want == math.inf) and torch.equal(got == -math.inf, want == -math.inf)
+
+
+@pytest.mark.parametrize("T,G,K,bias", [(33, 3, 64, True), (50, 2, 128, False), (20, 2, 128, False), (40, 1, 256, True), (35, 2, 48, False)])
+def test_convolution_with_unit_heads(T, G, K, bias):
+    """Unit q and k heads out of the convolution's own pass (16, 8 and 32 lanes a head) or after it (short portions, heads of 48): values, gaps between
+    the parts, the state.  f32 sums of at most 256 squares."""
+    from lit_llama_b200 import _seqlib as S
+
+    k_at = G * K if K != 48 else 104
+    v_at, Ch = 2 * k_at, 2 * k_at + 40
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    x, w, b = torch.randn(T, Ch + 8, generator=g, device=DEV).to(BF), torch.randn(Ch, 4, generator=g, device=DEV).to(BF), torch.randn(Ch, generator=g, device=DEV).to(BF)
+    state = torch.randn(2, 3, Ch, generator=g, device=DEV).to(BF)
+    xs = torch.cat([state[1], x[:, :Ch]]).double()
+    y = sum(xs[j:j + T] * w[:, j].double() for j in range(4)) + (b.double() if bias else 0.0)
+    want = torch.nn.functional.silu(y)
+    for at, m in ((0, K ** -0.5), (k_at, 1.0)):
+        h = want[:, at:at + G * K].view(T, G, K)
+        want[:, at:at + G * K] = (h / torch.sqrt((h * h).sum(-1, keepdim=True) + 1e-6) * m).view(T, G * K)
+    out, meta = torch.full((T, Ch), 7.0, device=DEV), torch.tensor([1, 9], dtype=torch.int32, device=DEV)
+    S.check(S.lib().b2l_seq_conv_silu_unit(x.data_ptr(), Ch + 8, w.data_ptr(), b.data_ptr() if bias else None, state.data_ptr(), meta.data_ptr(), out.data_ptr(), Ch, T, Ch, 4,
+                                           0, k_at, G, K, 1e-6, K ** -0.5, 1.0, S.act_code(BF), S.stream_ptr()), "convolution")
+    for lo, hi in ((0, k_at), (k_at, v_at), (v_at, Ch)):
+        assert rel(out[:, lo:hi], want[:, lo:hi]) < 1e-6
+    assert torch.equal(state[1], xs[-3:].to(BF))
+
+
+@pytest.mark.parametrize("size,mode", [(8, 0), (24, 1), (128, 0), (128, 1)])
+def test_decays_of_eight_channels(size, mode):
+    """exp(-exp(A) softplus(z + b)) and sigmoid(z)^(1/tau) in groups of 8 channels, from -100 to 100 and at infinity.  The exponent e carries the sum's
+    rounding, the softplus (3 * 2^-24), the coefficient (2 * 2^-24) and the product, 7 * 2^-24 in all, and e multiplies that; expf adds 2 * 2^-24."""
+    from lit_llama_b200 import _seqlib as S
+
+    T, H = 37, 3
+    g = torch.Generator(device=DEV).manual_seed(size)
+    a, bias, A = (torch.randn(T, H * size, generator=g, device=DEV) * 30).to(BF), torch.randn(H * size, generator=g, device=DEV).to(BF), torch.randn(H, generator=g, device=DEV).to(BF)
+    a[0, 0], a[1, 1] = math.inf, -math.inf
+    out, dt = torch.empty(T, H * size, device=DEV), torch.empty(T, H * size, device=DEV)
+    S.check(S.lib().b2l_seq_decay(a.data_ptr(), H * size, bias.data_ptr(), A.data_ptr(), mode, 16.0 if mode else 0.0, out.data_ptr(), None if mode else dt.data_ptr(), T, H, size,
+                                  S.act_code(BF), S.stream_ptr()), "decay")
+    z = a.double() + bias.double()
+    sp = torch.nn.functional.softplus(-z if mode else z, threshold=1e9)
+    e = sp / 16.0 if mode else sp * torch.exp(A.double()).repeat_interleave(size)
+    want = torch.exp(-e)
+    ok = e < 80
+    assert bool((((out.double() - want).abs() / want) < (7 * e + 2) * 2.0 ** -24)[ok].all()) and bool((out[~ok] < 1e-30).all())
+    if not mode:
+        fin = sp.isfinite() & (sp > 1e-35)
+        assert float(((dt.double() - sp).abs() / sp)[fin].max()) < 4e-7 and float(dt[0, 0]) == math.inf and float(dt[1, 1]) == 0.0
