@@ -356,15 +356,29 @@ __global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_const
 }
 
 struct Plan { int bt, m_tiles, splits, nst; size_t smem; };
-// Tokens per tile: the rows in equal tiles of at most 256.  K is split over a cluster while the grid leaves more than half of the SMs
-// idle and a part keeps at least four stages.
+// Tiles of equal height and a split of K over clusters, by a model of the time in ns.  A CTA takes 4400, 210 per stage of 128 k, and per token of its tile
+// 85 for the epilogue's roundings (a rank of a split stores its share) and 1.6 per stage; two CTAs on an SM (tiles of up to 128 tokens) take 1.2 times
+// one's time, a last one alone 0.95; a split in 2, 4, 8 adds 3000, 3900, 4800 for its barriers and 3 per token and rank.  Device time in us, one row of
+// tiles and the plan so: 137 x 4096 -> 12288 29 / 21, 300 x 4096 -> 12288 58 / 32, 512 x 4096 -> 11008 88 / 58, 256 x 5120 -> 5120 31 / 22, 1000 x 4096 ->
+// 4096 46 / 34; up to 64 tokens the plans are mostly the same (16 x 4096 -> 11008 13.3).
 static Plan plan_for(int M, int N, int K) {
-  Plan q;
-  q.m_tiles = (M + 255) / 256;
-  q.bt = ((M + q.m_tiles - 1) / q.m_tiles + 15) / 16 * 16;
-  const int tiles = (N + BN - 1) / BN * q.m_tiles;
-  q.splits = 1;
-  while (q.splits < 8 && tiles * q.splits * 2 <= sm_count() && K / BK / (q.splits * 2) >= 4) q.splits *= 2;
+  static const int clusters[9] = {0, 148, 74, 0, 33, 0, 0, 0, 15};      // of so many CTAs, one per SM, that run at once on 148 SMs
+  const int sms = sm_count(), n_tiles = (N + BN - 1) / BN, least = (M + 255) / 256;
+  Plan q{};
+  long long best = -1;
+  for (int mt = least; mt <= least + 4; ++mt) {
+    const int bt = ((M + mt - 1) / mt + 15) / 16 * 16, tiles = n_tiles * ((M + bt - 1) / bt), two = bt <= 128;
+    for (int sp = 1; sp <= 8; sp *= 2) {
+      const int stages = (K / BK + sp - 1) / sp, at_once = clusters[sp] * sms / 148;
+      if (sp > 1 && (K / BK / sp < 4 || tiles > at_once * (two && sp == 2 ? 2 : 1))) break;      // a split only where its clusters run at once; four and eight alone on their SMs
+      const long long one = 4400 + 210 * stages + bt * (85 / sp + 16 * stages / 10), deep = ((long long)tiles * sp + sms - 1) / sms;
+      const long long cost = (deep == 1 ? one : two ? one * (deep / 2 * 24 + deep % 2 * 19) / 20 : one * deep) + (sp == 1 ? 0 : (sp == 2 ? 3000 : sp == 4 ? 3900 : 4800) + 3 * bt * sp);
+      if (best < 0 || cost < best) {
+        best = cost;
+        q.bt = bt; q.m_tiles = (M + bt - 1) / bt; q.splits = sp;
+      }
+    }
+  }
   const size_t stage = A_BYTES + (size_t)q.bt * BK;
   // Two CTAs per SM for tiles of up to 128 tokens, one's epilogue under the other's loads: half of an SM's 228 KB less the 1 KB the system
   // keeps per CTA, the static arrays and the alignment of the stages.  Wider tiles take one.
