@@ -5,6 +5,7 @@ first use of a model builds what that model needs and nothing else."""
 import os
 import subprocess
 import sys
+import sysconfig
 import tempfile
 
 PKG = os.path.dirname(os.path.abspath(__file__))
@@ -18,6 +19,8 @@ LIBRARIES = {
     "llama": dict(out=os.path.join(PKG, "libb200llama.so"),
                   sources=["api.cu", "q_generic.cu", "elementwise.cu", "attention.cu", "q4_tc.cu", "q4_gemv.cu", "q4_gemv_batch.cu",
                            "q8_gemv.cu", "q8_gemm.cu", "sampling.cu", "decode_mega.cu", "q4_gemm.cu", "tp_allreduce.cu"]),
+    # the quantized linears' entry points as Python functions (a CPython extension, host code only)
+    "pycall": dict(out=os.path.join(PKG, "_pycall.so"), sources=["pycall.cpp"]),
     # sequence-mixer kernels: recurrences, local and latent attention, expert routing, f32 residual streams (include/b2l_seq.h)
     "seq": dict(out=os.path.join(PKG, "libb200seq.so"),
                 sources=["seq_api.cu", "seq_elementwise.cu", "seq_scan.cu", "seq_attention.cu", "seq_latent.cu", "seq_moe.cu", "seq_streams.cu",
@@ -51,7 +54,7 @@ def compile_unit(src: str, force: bool = False, obj_dir: str = OBJ_DIR) -> str:
         t = os.path.getmtime(obj)
         if all(os.path.getmtime(d) <= t for d in [path] + _headers()):
             return obj
-    cmd = [nvcc_path()] + NVCC_FLAGS + ["-c", path, "-o", obj]
+    cmd = [nvcc_path()] + NVCC_FLAGS + (["-I" + sysconfig.get_paths()["include"]] if src.endswith(".cpp") else []) + ["-c", path, "-o", obj]
     print("[build]", " ".join(cmd), file=sys.stderr)
     subprocess.run(cmd, check=True, stdout=sys.stderr)
     return obj

@@ -132,8 +132,28 @@ def lib():
                     fn = getattr(handle, name)
                     fn.restype = res
                     fn.argtypes = args
+                _bind(handle)
                 _lib = handle
     return _lib
+
+
+#: q4 / q8 of csrc/pycall.cpp, set with the library
+pycall = None
+Q4_GEMV, Q4_GEMV_BATCH, Q4_LINEAR_TC, Q4_GEMM = range(4)
+
+
+def _bind(handle) -> None:
+    global pycall
+    import importlib.machinery
+    import importlib.util
+
+    from . import _build
+
+    spec = importlib.util.spec_from_loader("_pycall", importlib.machinery.ExtensionFileLoader("_pycall", _build.ensure("pycall")))
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind(*(C.cast(getattr(handle, n), c_void_p).value for n in ("b2l_q4_gemv", "b2l_q4_gemv_batch", "b2l_q4_linear_tc", "b2l_q4_gemm", "b2l_q8_linear")))
+    pycall = module
 
 
 def check(rc: int, what: str) -> None:

@@ -94,22 +94,28 @@ class Linear8bitLt(torch.nn.Module):
         return self._tiled
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        L.require_cuda_bf16(x, "Linear8bitLt.forward")
-        if self.in_features % 128 != 0 or self.in_features > 12288:
-            raise RuntimeError(f"Linear8bitLt: in_features {self.in_features} unsupported (multiple of 128, <= 12288)")
+        if x.dtype is not torch.bfloat16 or not x.is_cuda:
+            L.require_cuda_bf16(x, "Linear8bitLt.forward")
+        K, N = self.in_features, self.out_features
+        if K % 128 != 0 or K > 12288:
+            raise RuntimeError(f"Linear8bitLt: in_features {K} unsupported (multiple of 128, <= 12288)")
         shape = x.shape
-        x2 = x.reshape(-1, shape[-1]).contiguous()
-        M, K, N = x2.shape[0], self.in_features, self.out_features
+        x2 = (x if len(shape) == 2 else x.reshape(-1, shape[-1])).contiguous()
+        M = x2.shape[0]
         y = torch.empty((M, N), device=x.device, dtype=x.dtype)
         lib = L.lib()
-        cb, scb = self.weight.data, self.weight.SCB
-        if M > 1 and cb.data_ptr() % 16 == 0:        # all rows in one product: the weight is read once (TMA wants 16-byte aligned rows)
+        par = self._parameters
+        weight, bias = par["weight"] if "weight" in par else self.weight, par["bias"] if "bias" in par else self.bias
+        cbp = weight.data_ptr()
+        if M > 1 and cbp % 16 == 0:                  # all rows in one product: the weight is read once (TMA wants 16-byte aligned rows)
             ws = torch.empty(lib.b2l_q8_linear_workspace_bytes(M, K), dtype=torch.uint8, device=x.device)
-            L.check(lib.b2l_q8_linear(x2.data_ptr(), K, cb.data_ptr(), scb.data_ptr(), y.data_ptr(), N, ws.data_ptr(), M, N, K, self.threshold,
-                                      L.stream_ptr()), "b2l_q8_linear")
-            if self.bias is not None:
-                y = y + self.bias.to(y.dtype)
-            return y.reshape(*shape[:-1], N)
+            rc = L.pycall.q8(x2.data_ptr(), K, cbp, weight.SCB.data_ptr(), y.data_ptr(), N, ws.data_ptr(), M, N, K, self.threshold, L.stream_ptr())
+            if rc != 0:
+                L.check(rc, "b2l_q8_linear")
+            if bias is not None:
+                y = y + bias.to(y.dtype)
+            return y if len(shape) == 2 else y.reshape(*shape[:-1], N)
+        cb, scb = weight.data, weight.SCB
         wt = self.tiled()
         mask = None
         if M > 1:  # outlier columns are a property of the whole batch (any row over the threshold)

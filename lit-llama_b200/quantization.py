@@ -246,50 +246,53 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         return self.tc_capable and self.in_features % 64 == 0 and self.in_features <= 24576
 
     def forward(self, inp):
-        # the small calls are bound by this function (a one-row product takes the GPU 4 us): module attributes are looked up once, and
-        # argument blocks name only the fields that are not zero
-        L.require_cuda_bf16(inp, "ColBlockQuantizedLinear.forward")
+        # the small calls are bound by this function (a one-row product takes the GPU 4 us): module attributes are looked up once, nothing is
+        # reshaped that is two-dimensional, and the launch goes through csrc/pycall.cpp
+        if inp.dtype is not torch.bfloat16 or not inp.is_cuda:
+            L.require_cuda_bf16(inp, "ColBlockQuantizedLinear.forward")
         buf = self._buffers
-        scales = buf["scales"] if "scales" in buf else self.scales
-        zeros = buf["zeros"] if "zeros" in buf else self.zeros
-        if scales.device != inp.device:
+        if "scales" in buf and "zeros" in buf and "bias" in buf:
+            scales, zeros, bias = buf["scales"], buf["zeros"], buf["bias"]
+        else:                                            # a program has put Parameters in their place
+            scales, zeros, bias = self.scales, self.zeros, self.bias
+        device = inp.device
+        if scales.device != device:
             raise RuntimeError("input and quant_weight are on different devices")
         shape = inp.shape
-        x = inp.reshape(-1, shape[-1])
-        if x.stride(-1) != 1:
-            x = x.contiguous()
-        M, K, N = x.shape[0], self.in_features, self.out_features
+        K, N = self.in_features, self.out_features
         assert shape[-1] == K, "incompatible dimensions"
-        y = torch.empty((M, N), device=inp.device, dtype=inp.dtype)
+        x = inp if len(shape) == 2 else inp.reshape(-1, K)
+        ldx, step = x.stride()
+        if step != 1:
+            x = x.contiguous()
+            ldx = x.stride(0)
+        M = x.shape[0]
+        y = torch.empty((M, N), device=device, dtype=torch.bfloat16)
         if M == 0:
             return y.reshape(*shape[:-1], N)
-        ldx = x.stride(0)
-        aligned = x.data_ptr() % 16 == 0 and ldx % 8 == 0
-        tc = self.tc_capable
+        xp = x.data_ptr()
+        aligned = xp % 16 == 0 and ldx % 8 == 0
+        tc = self.bits == 4 and K % 32 == 0 and bias is None and scales.shape[1] == 1 and zeros.dtype == scales.dtype      # tc_capable
         gemv = tc and K % 64 == 0 and K <= 24576         # gemv_capable
+        if L.pycall is None:
+            L.lib()
         # `wt` keeps a transient tiling (released layers) alive until its launch is enqueued; the caching allocator
         # hands freed blocks out in stream order, so the kernel has finished before anybody else writes there
+        which, ws = -1, None
         if gemv and aligned and M == 1:
-            wt = self.tiled_i8()
-            a = L.Q4LinearArgs(x=x.data_ptr(), ldx=ldx, qw_tiled=wt.data_ptr(), scales=scales.data_ptr(), zeros=zeros.data_ptr(),
-                               sz_dtype=L.sz_dtype_of(scales), y=y.data_ptr(), ldy=N, M=1, N=N, K=K)
-            L.check(L.lib().b2l_q4_gemv(C.byref(a), L.stream_ptr()), "b2l_q4_gemv")
+            which, wt = L.Q4_GEMV, self.tiled_i8()
         elif gemv and aligned and M <= 8 and BATCH_GEMV:
             # 2..8 rows: the mma.sync tile has 8 columns, one per row (csrc/q4_gemv_batch.cu)
-            wt = self.tiled_mma()
-            a = L.Q4LinearArgs(x=x.data_ptr(), ldx=ldx, qw_tiled=wt.data_ptr(), scales=scales.data_ptr(), zeros=zeros.data_ptr(),
-                               sz_dtype=L.sz_dtype_of(scales), y=y.data_ptr(), ldy=N, M=M, N=N, K=K, workspace=batch_workspace(inp.device, K).data_ptr())
-            L.check(L.lib().b2l_q4_gemv_batch(C.byref(a), L.stream_ptr()), "b2l_q4_gemv_batch")
+            which, wt, ws = L.Q4_GEMV_BATCH, self.tiled_mma(), batch_workspace(device, K).data_ptr()
         elif tc and aligned and (M <= 16 or K % 64 == 0):
             # 9..16 rows: tcgen05 with K split over clusters; prompts: tcgen05 tiles of 128 features, weights dequantised on the fly with
             # get_weight's roundings
-            wt = self.tiled()
-            a = L.Q4LinearArgs(x=x.data_ptr(), ldx=ldx, qw_tiled=wt.data_ptr(), scales=scales.data_ptr(), zeros=zeros.data_ptr(),
-                               sz_dtype=L.sz_dtype_of(scales), y=y.data_ptr(), ldy=N, M=M, N=N, K=K)
-            if M <= 16:
-                L.check(L.lib().b2l_q4_linear_tc(C.byref(a), L.stream_ptr()), "b2l_q4_linear_tc")
-            else:
-                L.check(L.lib().b2l_q4_gemm(C.byref(a), L.stream_ptr()), "b2l_q4_gemm")
+            which, wt = L.Q4_LINEAR_TC if M <= 16 else L.Q4_GEMM, self.tiled()
+        if which >= 0:
+            rc = L.pycall.q4(which, xp, ldx, wt.data_ptr(), scales.data_ptr(), zeros.data_ptr(), 0 if scales.dtype is torch.bfloat16 else L.sz_dtype_of(scales),
+                             y.data_ptr(), N, M, N, K, ws, L.stream_ptr())
+            if rc != 0:
+                L.check(rc, ("b2l_q4_gemv", "b2l_q4_gemv_batch", "b2l_q4_linear_tc", "b2l_q4_gemm")[which])
         else:
             self._check_layout()
             qw = self.reference_quant_weight()
@@ -298,7 +301,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
                                       None if self.bias is None else self.bias.to(inp.dtype).data_ptr(), y.data_ptr(), N,
                                       M, N, K, self.bits, self.tile_cols, L.stream_ptr())
             L.check(rc, "b2l_q_linear")
-        return y.reshape(*shape[:-1], N)
+        return y if len(shape) == 2 else y.reshape(*shape[:-1], N)
 
 
 def qlinear_4bit_weight(inp, weight, scales, zeros):
