@@ -12,7 +12,8 @@
 // box is 128 rows x 128 k.  Where N / 128 tiles do not fill the chip a cluster of 2, 4 or 8 CTAs splits K; the partial sums are integers,
 // so adding them through distributed shared memory changes nothing in the result.
 // One row at a time through the single-row kernel took 3956 us for 137 x 4096 -> 11008 (137 launches that each stream the weight); the
-// three launches take 45 us with the call's host side (5 + 5 + 33 on the device), and the results have the same bits.
+// three launches took 36.5 us with the call's host side one after the other, and 30.7 each launched while the one before it runs (the rows wait for
+// the mask after loading their x, the product for the rows after requesting its first weights); the results have the same bits.
 #include <cuda_fp16.h>
 
 #include "tc_common.cuh"
@@ -33,6 +34,7 @@ constexpr int SLAB = 4096;                 // rows per pass: bounds the workspac
 
 // ---------------------------------------------------------------- outlier columns: 64 columns per CTA, 32 rows at a time
 __global__ void __launch_bounds__(256) q8_mask_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int M, int K, float threshold, uint32_t* __restrict__ mask) {
+  pdl_launch_dependents();                            // the rows' kernel loads its row meanwhile
   __shared__ uint32_t bits[2];
   const int tid = threadIdx.x, k = blockIdx.x * 64 + (tid & 7) * 8;
   if (tid < 2) bits[tid] = 0u;
@@ -67,16 +69,7 @@ __global__ void __launch_bounds__(ROW_THREADS) q8_rows_kernel(const __nv_bfloat1
   __shared__ int wsum[ROW_THREADS / 32];
   constexpr int MAXC = MAX_K / (ROW_THREADS * 8);
   const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, words = K / 32;
-  // two neighbouring words per thread (K <= 12288: at most 384 words), an exclusive scan of their outlier counts
-  const uint32_t w0 = 2 * tid < words ? mask_g[2 * tid] : 0u, w1 = 2 * tid + 1 < words ? mask_g[2 * tid + 1] : 0u;
-  const int mine = __popc(w0) + __popc(w1);
-  int sum = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, sum, o);
-    if (lane >= o) sum += v;
-  }
-  if (lane == 31) wsum[warp] = sum;
+  pdl_launch_dependents();                            // the product starts on its weights
   float av[MAXC][8];
 #pragma unroll
   for (int c = 0; c < MAXC; ++c) {
@@ -91,6 +84,22 @@ __global__ void __launch_bounds__(ROW_THREADS) q8_rows_kernel(const __nv_bfloat1
       }
     }
   }
+  pdl_wait();                                         // the mask is complete; read by coherent loads only (x was there before the mask's kernel began)
+  // two neighbouring words per thread (K <= 12288: at most 384 words), an exclusive scan of their outlier counts
+  auto word = [&](int i) {
+    uint32_t v = 0u;
+    if (i < words) asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(mask_g + i) : "memory");
+    return v;
+  };
+  const uint32_t w0 = word(2 * tid), w1 = word(2 * tid + 1);
+  const int mine = __popc(w0) + __popc(w1);
+  int sum = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += v;
+  }
+  if (lane == 31) wsum[warp] = sum;
   __syncthreads();
   int at = sum - mine;
   for (int w = 0; w < warp; ++w) at += wsum[w];
@@ -199,11 +208,20 @@ __global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_const
     if (lane == 0) {
       int st = 0;
       uint32_t ph = 1;                                       // parity of a stage's previous use: passes at once the first time
+      const int early = min(kb_lo + p.nst, kb_hi);           // weights of the first stages on their way while the rows' kernel still runs
+      for (int kb = kb_lo; kb < early; ++kb) {
+        mbar_expect_tx(bar_full + 8 * (kb - kb_lo), stage_bytes);
+        tma_load_2d(sbase + (kb - kb_lo) * stage_bytes, &p.wmap, kb * BK, n0, bar_full + 8 * (kb - kb_lo));
+      }
+      pdl_wait();
+      asm volatile("fence.proxy.async;" ::: "memory");         // ordinary stores of the kernel before, read by the async proxy
       for (int kb = kb_lo; kb < kb_hi; ++kb) {
         mbar_wait(bar_empty + 8 * st, ph, dead);
         if (dead) break;
-        mbar_expect_tx(bar_full + 8 * st, stage_bytes);
-        tma_load_2d(sbase + st * stage_bytes, &p.wmap, kb * BK, n0, bar_full + 8 * st);
+        if (kb >= early) {
+          mbar_expect_tx(bar_full + 8 * st, stage_bytes);
+          tma_load_2d(sbase + st * stage_bytes, &p.wmap, kb * BK, n0, bar_full + 8 * st);
+        }
         tma_load_2d(sbase + st * stage_bytes + A_BYTES, &p.xmap, kb * BK, m0, bar_full + 8 * st);
         if (++st == p.nst) { st = 0; ph ^= 1u; }
       }
@@ -238,6 +256,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_const
     }
   } else {
     // while the product runs: row scales and outlier activations of these tokens (read from the workspace group by group they took 1000 cycles each)
+    pdl_wait();
     const int e = tid - 64, n_sm = min(*p.n_out, SM_OUT);
     for (int i = e; i < p.bt; i += 128) s_sca[i] = m0 + i < p.M ? p.sca[m0 + i] : 0.f;
     for (int i = e; i < n_sm * (p.bt / 8); i += 128) {
@@ -435,11 +454,11 @@ extern "C" int b2l_q8_linear(const void* x, int ldx, const void* cb, const void*
     if (int rc = ensure_dyn_smem(q8_gemm_kernel, q.smem, smem_cache)) return rc;
     p.x = (const __nv_bfloat16*)x + (size_t)at * ldx;
     p.y = (__nv_bfloat16*)y + (size_t)at * ldy;
-    q8_rows_kernel<<<rows, ROW_THREADS, 0, s>>>(p.x, ldx, K, Rp, mask, xq, sca, aout, list, n_out);
-    B2L_LAUNCH_CHECK("q8_rows_kernel");
+    LaunchCfg lr(dim3((unsigned)rows), dim3(ROW_THREADS), 0, s, true, 1);      // each kernel is launched while the one before it runs, and waits for it where it reads its results
+    B2L_CUDA(cudaLaunchKernelEx(&lr.cfg, q8_rows_kernel, p.x, ldx, K, (int)Rp, (const uint32_t*)mask, xq, sca, aout, list, n_out));
     p.cb = (const int8_t*)cb; p.scb = (const float*)scb; p.sca = sca; p.aout = aout; p.list = list; p.n_out = n_out;
     p.M = rows; p.N = N; p.K = K; p.Mp = Rp; p.ldx = ldx; p.ldy = ldy; p.bt = q.bt; p.nst = q.nst; p.splits = q.splits;
-    LaunchCfg lc(dim3((unsigned)((N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, s, false, q.splits);
+    LaunchCfg lc(dim3((unsigned)((N + BN - 1) / BN * q.splits), (unsigned)q.m_tiles), dim3(NTHREADS), q.smem, s, true, q.splits);
     B2L_CUDA(cudaLaunchKernelEx(&lc.cfg, q8_gemm_kernel, p));
   }
   return 0;

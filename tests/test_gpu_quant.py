@@ -362,6 +362,30 @@ def test_int8_linear_vs_oracle(dev, N, K, M, outliers):
     assert (y - exact).norm() / exact.norm() < 3e-2  # the int8 scheme itself is ~1% accurate
 
 
+@pytest.mark.parametrize("M", [2, 8, 137, 300])
+def test_calls_enqueued_behind_one_another(dev, M):
+    """The launches of a call overlap: calls in one workspace, enqueued without a wait, give the bits of each call by itself."""
+    from lit_llama_b200.quantization import ColBlockQuantizedLinear
+    import lit_llama_b200 as P
+
+    g = torch.Generator().manual_seed(M)
+    N, K = 640, 4096
+    xs = [(torch.randn(M, K, generator=g) * (1 + i / 4)).to(dev, torch.bfloat16) for i in range(6)]   # other scales, other outlier columns
+    int8, int4 = P.Linear8bitLt(K, N, bias=False), ColBlockQuantizedLinear(K, N, bias=False, bits=4, tile_cols=-1)
+    int8.load_state_dict({"weight": torch.randn(N, K, generator=g) * 0.03})
+    int4.quant_weight.copy_(torch.randint(0, 256, int4.quant_weight.shape, generator=g))
+    int4.scales.copy_(torch.rand(int4.scales.shape, generator=g) * 0.01 + 0.001)
+    int4.zeros.copy_(torch.rand(int4.zeros.shape, generator=g) * 15)
+    for lin in (int8.to(dev), int4.to(dev)):
+        alone = []
+        for x in xs:
+            alone.append(lin(x))
+            torch.cuda.synchronize()
+        for _ in range(3):
+            for want, got in zip(alone, [lin(x) for x in xs]):
+                assert torch.equal(want, got)
+
+
 @pytest.mark.parametrize("M,N,K,outliers", [(2, 48, 128, 0), (16, 130, 256, 1), (17, 128, 1024, 3), (33, 4096, 4096, 5), (137, 11008, 4096, 6), (256, 300, 12288, 2),
                                             (257, 272, 1024, 40), (5, 512, 512, 512)])
 def test_int8_rows_at_once_equal_single_rows(dev, M, N, K, outliers):
