@@ -356,27 +356,35 @@ __device__ __forceinline__ float warp_sum8(float (&v)[8], int lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// Two warps: warp 0 the columns 0..3 and 12..15 of A and B, warp 1 the columns 4..11 (20 rows of four columns each).  A row of k, q and decays is
+// read from shared memory once for four columns: with a column at a time those reads were what bounded the kernel (1632 warp reads a chunk, 480 so),
+// 16 heads of 128 x 128, 2048 tokens: 34 us then.
+constexpr int CHUNK_THREADS = 64;
 template <typename act_t, int K, bool DELTA>
-__global__ void __launch_bounds__(128) seq_chunk_kernel(b2l_seq_scan_args a, int vec) {
+__global__ void __launch_bounds__(CHUNK_THREADS) seq_chunk_kernel(b2l_seq_scan_args a, int vec) {
   __shared__ __align__(16) float sk[CH_C][K], sq[CH_C][K], sg[CH_C][K];
-  __shared__ float sA[CH_C][CH_C + 1], sB[CH_C][CH_C + 1], sT[CH_C][CH_C + 1], sbeta[CH_C];
+  __shared__ float sA[CH_C][CH_C + 1], sB[CH_C][CH_C + 1], sbeta[CH_C];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, chunk = blockIdx.x, h = blockIdx.y, hq = h / (a.heads / a.qk_heads);
   const int t0 = chunk * CH_C, nt = min(CH_C, a.T - t0);
   const float* gk = a.k + (size_t)t0 * a.ldk + (size_t)hq * K;
   const float* gq = a.q + (size_t)t0 * a.ldq + (size_t)hq * K;
   const float* gd = a.decay + (size_t)t0 * a.ldd + (a.decay_per_channel ? (size_t)h * K : (size_t)h);
   if (vec) {
-#pragma unroll
-    for (int i = tid; i < CH_C * K / 4; i += 128) {
+#pragma unroll 4
+    for (int i = tid; i < CH_C * K / 4; i += CHUNK_THREADS) {
       const int t = i / (K / 4), c = (i - t * (K / 4)) * 4;
-      const bool in = t < nt;
-      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(&sk[t][c]) = in ? *reinterpret_cast<const float4*>(gk + (size_t)t * a.ldk + c) : z;
-      *reinterpret_cast<float4*>(&sq[t][c]) = in ? *reinterpret_cast<const float4*>(gq + (size_t)t * a.ldq + c) : z;
-      if (a.decay_per_channel) *reinterpret_cast<float4*>(&sg[t][c]) = in ? *reinterpret_cast<const float4*>(gd + (size_t)t * a.ldd + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+      if (t < nt) {
+        cp_async16(&sk[t][c], gk + (size_t)t * a.ldk + c);
+        cp_async16(&sq[t][c], gq + (size_t)t * a.ldq + c);
+        if (a.decay_per_channel) cp_async16(&sg[t][c], gd + (size_t)t * a.ldd + c);
+      } else {
+        *reinterpret_cast<float4*>(&sk[t][c]) = *reinterpret_cast<float4*>(&sq[t][c]) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a.decay_per_channel) *reinterpret_cast<float4*>(&sg[t][c]) = make_float4(1.f, 1.f, 1.f, 1.f);
+      }
     }
+    cp_async_commit();
   } else {
-    for (int i = tid; i < CH_C * K; i += 128) {
+    for (int i = tid; i < CH_C * K; i += CHUNK_THREADS) {
       const int t = i / K, c = i - t * K;
       const bool in = t < nt;
       sk[t][c] = in ? gk[(size_t)t * a.ldk + c] : 0.f;
@@ -385,73 +393,88 @@ __global__ void __launch_bounds__(128) seq_chunk_kernel(b2l_seq_scan_args a, int
     }
   }
   if (!a.decay_per_channel)
-    for (int i = tid; i < CH_C * K; i += 128) {
+    for (int i = tid; i < CH_C * K; i += CHUNK_THREADS) {
       const int t = i / K;
       sg[t][i - t * K] = t < nt ? gd[(size_t)t * a.ldd] : 1.f;
     }
   if (DELTA && tid < CH_C) sbeta[tid] = tid < nt ? sigmoid_f(ld_act((const act_t*)a.beta, (size_t)(t0 + tid) * a.ldb + h)) : 0.f;
+  cp_async_wait<0>();
   __syncthreads();
+  // the eight sums of row t: k_t and q_t with the decayed keys of columns i0 .. i0 + 3
+  const int col = ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+  auto put = [&](float (&p)[8], int t, int i0) {
+    const float v = warp_sum8(p, lane);
+    if ((lane & 3) == 0) {
+      if (lane & 16) sB[t][i0 + col] = v;
+      else if (DELTA) sA[t][i0 + col] = v;
+    }
+  };
 #pragma unroll 1
-  for (int n = 0; n < 4; ++n) {                        // a warp takes columns w, 7 - w, 8 + w, 15 - w
-    const int i = (n & 2) * 4 + ((n & 1) ? 7 - warp : warp);
-    float x[K / 32];
+  for (int n = 0; n < 2; ++n) {
+    const int i0 = 4 * (warp ? 1 + n : 3 * n);
+    float x[4][K / 32];
 #pragma unroll
-    for (int e = 0; e < K / 32; ++e) x[e] = sk[i][lane + 32 * e];
-#pragma unroll 1
-    for (int tb = 0; tb < CH_C; tb += 4) {             // four rows: eight sums in nine shuffles
-      float p[8];
+    for (int r = 0; r < 4; ++r) {                      // rows of the diagonal's 4 x 4
+      const int t = i0 + r;
+      float p[8] = {};
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int t = tb + r;
-        float pk = 0.f, pq = 0.f;
-        if (t >= i) {
+      for (int e = 0; e < K / 32; ++e) {
+        const float kv = sk[t][lane + 32 * e], qv = sq[t][lane + 32 * e], gv = sg[t][lane + 32 * e];
 #pragma unroll
-          for (int e = 0; e < K / 32; ++e) {
-            if (t > i) x[e] *= sg[t][lane + 32 * e];
-            if (DELTA) pk = fmaf(sk[t][lane + 32 * e], x[e], pk);
-            pq = fmaf(sq[t][lane + 32 * e], x[e], pq);
-          }
+        for (int c = 0; c < r; ++c) {
+          x[c][e] *= gv;
+          if (DELTA) p[c] = fmaf(kv, x[c][e], p[c]);
+          p[4 + c] = fmaf(qv, x[c][e], p[4 + c]);
         }
-        p[r] = t > i ? pk : 0.f;
-        p[4 + r] = pq;
+        x[r][e] = kv;
+        p[4 + r] = fmaf(qv, kv, p[4 + r]);
       }
-      const float v = warp_sum8(p, lane);
-      if ((lane & 3) == 0) {
-        const int t = tb + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-        if (lane & 16) sB[t][i] = v;
-        else if (DELTA) sA[t][i] = v;
+      put(p, t, i0);
+    }
+#pragma unroll 2
+    for (int t = i0 + 4; t < CH_C; ++t) {
+      float p[8] = {};
+#pragma unroll
+      for (int e = 0; e < K / 32; ++e) {
+        const float kv = sk[t][lane + 32 * e], qv = sq[t][lane + 32 * e], gv = sg[t][lane + 32 * e];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          x[c][e] *= gv;
+          if (DELTA) p[c] = fmaf(kv, x[c][e], p[c]);
+          p[4 + c] = fmaf(qv, x[c][e], p[4 + c]);
+        }
       }
+      put(p, t, i0);
     }
   }
   __syncthreads();
   float* out = a.work_state + ((size_t)chunk * a.heads + h) * (2 * CH_MAT);
   if (!DELTA) {
-    for (int e = tid; e < CH_MAT; e += 128) out[CH_MAT + e] = sB[e / CH_C][e % CH_C];
+    for (int e = tid; e < CH_MAT; e += CHUNK_THREADS) out[CH_MAT + e] = e % CH_C <= e / CH_C ? sB[e / CH_C][e % CH_C] : 0.f;
     return;
   }
-  if (tid < CH_C) {                                    // column tid of T by forward substitution
-    float col[CH_C];
+  if (warp) return;
+  const int j = lane & (CH_C - 1), half = lane >> 4;   // column j of T by forward substitution, in both halves of the warp; B T: a half the even rows, the other the odd ones
+  float c[CH_C];
 #pragma unroll
-    for (int t = 0; t < CH_C; ++t) {
-      float s0 = 0.f, s1 = 0.f;
+  for (int t = 0; t < CH_C; ++t) {
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-      for (int i = 0; i < t; ++i) {
-        if (i & 1) s1 = fmaf(sA[t][i], col[i], s1);
-        else s0 = fmaf(sA[t][i], col[i], s0);
-      }
-      col[t] = t < tid ? 0.f : (t == tid ? sbeta[t] : -sbeta[t] * (s0 + s1));
-      sT[t][tid] = col[t];
+    for (int i = 0; i < t; ++i) {
+      if (i & 1) s1 = fmaf(sA[t][i], c[i], s1);
+      else s0 = fmaf(sA[t][i], c[i], s0);
     }
+    c[t] = t < j ? 0.f : (t == j ? sbeta[t] : -sbeta[t] * (s0 + s1));
+    if ((t & 1) == half) out[t * CH_C + j] = c[t];
   }
-  __syncthreads();
-  for (int e = tid; e < CH_MAT; e += 128) {
-    const int t = e / CH_C, j = e - t * CH_C;
+#pragma unroll
+  for (int s = 0; s < CH_C; s += 2) {
+    const int t = s + half;
     float m = 0.f;
 #pragma unroll
-    for (int i = 0; i < CH_C; ++i)
-      if (i >= j && i <= t) m = fmaf(sB[t][i], sT[i][j], m);      // the rest is zero times a token that t has not seen, which may be infinite
-    out[e] = sT[t][j];
-    out[CH_MAT + e] = m;
+    for (int i = 0; i <= s + 1; ++i)
+      if (i >= j && i <= t) m = fmaf(sB[t][i], c[i], m);          // the rest is zero times a token that t has not seen, which may be infinite
+    out[CH_MAT + t * CH_C + j] = m;
   }
 }
 
@@ -707,7 +730,7 @@ static int launch_walk(const b2l_seq_scan_args* a, cudaStream_t s) {
   if (int rc = ensure_dyn_smem(seq_walk_kernel<act_t, K, DELTA>, sizeof(WalkSmem<K, DELTA>), cache)) return rc;
   auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   const int vec = a->ldq % 4 == 0 && a->ldk % 4 == 0 && al(a->q) && al(a->k) && (!a->decay_per_channel || (a->ldd % 4 == 0 && al(a->decay)));
-  seq_chunk_kernel<act_t, K, DELTA><<<dim3((unsigned)((a->T + CH_C - 1) / CH_C), (unsigned)a->heads), 128, 0, s>>>(*a, vec);
+  seq_chunk_kernel<act_t, K, DELTA><<<dim3((unsigned)((a->T + CH_C - 1) / CH_C), (unsigned)a->heads), CHUNK_THREADS, 0, s>>>(*a, vec);
   B2L_LAUNCH_CHECK("seq_chunk_kernel");
   seq_walk_kernel<act_t, K, DELTA><<<dim3((unsigned)(a->V / CH_VT), (unsigned)a->heads), 384, sizeof(WalkSmem<K, DELTA>), s>>>(*a);
   B2L_LAUNCH_CHECK("seq_walk_kernel");
