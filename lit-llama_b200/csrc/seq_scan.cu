@@ -7,6 +7,8 @@
 // lanes of a column read consecutive 16-byte words).  With `ones` the state has one column more whose value is 1 at every
 // step (a normaliser: the decayed sum of the keys), kept and read out beside the others.  Inputs of SCAN_TC steps are staged in shared memory by the
 // whole CTA with asynchronous copies, one stage ahead of the recurrence.  All arithmetic is f32.
+#include <type_traits>
+
 #include "seq_common.cuh"
 
 namespace b2l {
@@ -334,12 +336,14 @@ __global__ void seq_scan_combine_kernel(b2l_seq_scan_args a) {
 // Decays only ever multiply (no quotient of cumulative products, which overflows where a channel forgets fast).  T is the product of the
 // chunk's transition matrices seen from k: its entries stay below 1 for unit keys.  All f32 on the CUDA cores, like the step-by-step form.
 //   seq_chunk_kernel  a CTA per (chunk, head): T and B T (or B), 16 x 16 each, into the workspace; all chunks in parallel
-//   seq_walk_kernel   a CTA per (head, 16 value columns) walks the chunks: warps 4..11 (a thread per key channel, the two groups on
+//   seq_walk_kernel   a CTA per (head, VT = 16 or 8 value columns) walks the chunks: warps 4..11 (a thread per key channel, the two groups on
 //                     alternate chunks) load and form G k, G q, D k a chunk ahead, while warps 0..3 run P / R (K split over the warps),
 //                     u / o and the state update in 4 x 4 tiles
 // What bounds it: the walk over T / 16 chunks, 832 FMA cycles per chunk (delta rule) and four barriers.  The step-by-step kernel spends 0.38 us
 // per token on one dependent chain of FMAs and shuffles, whatever the width (16 heads of 128 x 128, 2048 tokens: 780 us).
-constexpr int CH_C = 16, CH_VT = 16, CH_MAT = CH_C * CH_C;      // tokens per chunk, value columns per CTA
+// With 8 columns per CTA, where the chip has SMs for twice the CTAs, a chunk's products halve (8 heads of 128 x 128, 2048 tokens, us with 16 / 8
+// columns: 171 / 128 without the delta rule, 211 / 163 with it); with more CTAs than SMs two would share an SM's shared-memory reads, which bound it.
+constexpr int CH_C = 16, CH_VT = 16, CH_NARROW = 8, CH_MAT = CH_C * CH_C;      // tokens per chunk, value columns per CTA
 
 // v[0..7] of every lane summed over the warp: lane l holds sum number ((l >> 4) & 1) * 4 + ((l >> 3) & 1) * 2 + ((l >> 2) & 1)
 __device__ __forceinline__ float warp_sum8(float (&v)[8], int lane) {
@@ -478,33 +482,42 @@ __global__ void __launch_bounds__(CHUNK_THREADS) seq_chunk_kernel(b2l_seq_scan_a
   }
 }
 
-template <int K, bool DELTA>
+template <int K, bool DELTA, int VT>
 struct WalkStage {
   static constexpr int ROWS = DELTA ? 32 : 16, LD = ROWS + 4;      // padded: 16-byte rows of a channel on distinct banks
   float kq[K][LD];                 // [channel][(delta: 16 tokens of G k) | 16 of G q | padding]
   float kd[CH_C][K];               // D k
   float tm[ROWS][CH_C];            // (T over) B T, or B
-  float v[CH_C][CH_VT], u[CH_C][CH_VT];      // values, and (no delta rule) values times vscale
+  float v[CH_C][VT], u[CH_C][VT];            // values, and (no delta rule) values times vscale
   float gc[K];                     // G of the whole chunk
 };
-template <int K, bool DELTA>
+template <int K, bool DELTA, int VT>
 struct WalkSmem {
-  WalkStage<K, DELTA> st[2];
-  float S[K][CH_VT];
-  float part[4][WalkStage<K, DELTA>::ROWS][CH_VT + 4];
-  float w[CH_C][CH_VT], u[CH_C][CH_VT];
+  WalkStage<K, DELTA, VT> st[2];
+  float S[K][VT];
+  float part[64 / VT][WalkStage<K, DELTA, VT>::ROWS][VT + 4];
+  float w[CH_C][VT], u[CH_C][VT];
 };
 __device__ __forceinline__ void walk_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void fma4(float4& d, float s, const float4& v) {
   d.x = fmaf(s, v.x, d.x); d.y = fmaf(s, v.y, d.y); d.z = fmaf(s, v.z, d.z); d.w = fmaf(s, v.w, d.w);
 }
+template <int N> struct alignas(4 * N) Cols {           // neighbouring value columns of a thread
+  float v[N];
+  __device__ __forceinline__ void fma(float s, const Cols& o) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = fmaf(s, o.v[e], v[e]);
+  }
+};
 
-template <typename act_t, int K, bool DELTA>
+template <typename act_t, int K, bool DELTA, int VT>
 __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
   extern __shared__ __align__(16) unsigned char walk_raw[];
-  using Stage = WalkStage<K, DELTA>;
-  WalkSmem<K, DELTA>& sm = *reinterpret_cast<WalkSmem<K, DELTA>*>(walk_raw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, hq = h / (a.heads / a.qk_heads), v0 = blockIdx.x * CH_VT;
+  using Stage = WalkStage<K, DELTA, VT>;
+  constexpr int VW = VT / 4;                           // columns per thread of the walk, but in its product P / R
+  using Vec = Cols<VW>;
+  WalkSmem<K, DELTA, VT>& sm = *reinterpret_cast<WalkSmem<K, DELTA, VT>*>(walk_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, hq = h / (a.heads / a.qk_heads), v0 = blockIdx.x * VT;
   const int n_chunks = (a.T + CH_C - 1) / CH_C;
   float* st = a.state + ((size_t)a.meta[0] * a.heads + h) * (size_t)a.V * K;
 
@@ -512,7 +525,7 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
     // ===================== operands: warps 4..7 the even chunks, 8..11 the odd ones =====================
     const int par = warp >= 8, c = tid - 128 - 128 * par;
     const bool chan = c < K;
-    float k[CH_C], q[CH_C], g[CH_C], v[2], vs[2], G = 1.f;
+    float k[CH_C], q[CH_C], g[CH_C], v[VT / 8], vs[VT / 8], G = 1.f;
     float4 tm;
     auto load = [&](int n) {
       if (n >= n_chunks) return;
@@ -520,8 +533,8 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
       if (c < Stage::ROWS * CH_C / 4)
         tm = reinterpret_cast<const float4*>(a.work_state + ((size_t)n * a.heads + h) * (2 * CH_MAT) + (DELTA ? 0 : CH_MAT))[c];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int t = c / CH_VT + 8 * i, e = c % CH_VT;
+      for (int i = 0; i < VT / 8; ++i) {
+        const int t = c / VT + 8 * i, e = c % VT;
         v[i] = t < nt ? a.v[(size_t)(t0 + t) * a.ldv + (size_t)h * a.V + v0 + e] : 0.f;
         vs[i] = (!DELTA && a.vscale && t < nt) ? a.vscale[(size_t)(t0 + t) * a.ldvs + h] : 1.f;
       }
@@ -564,8 +577,8 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
       Stage& s = sm.st[n & 1];
       if (c < Stage::ROWS * CH_C / 4) reinterpret_cast<float4*>(&s.tm[0][0])[c] = tm;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int t = c / CH_VT + 8 * i, e = c % CH_VT;
+      for (int i = 0; i < VT / 8; ++i) {
+        const int t = c / VT + 8 * i, e = c % VT;
         s.v[t][e] = v[i];
         if (!DELTA) s.u[t][e] = v[i] * vs[i];
       }
@@ -598,31 +611,32 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
     return;
   }
   // ===================== the walk =====================
-  const int cg = tid >> 2, vg = tid & 3;               // channels 4 cg .. + 3 (K = 64: half of the threads), columns 4 vg .. + 3
+  const int cg = tid >> 2, vg = tid & 3;               // channels 4 cg .. + 3 (K = 64: half of the threads), columns VW vg .. + VW - 1
   const bool own = cg < K / 4;
   const float skip = a.skip ? ld_act((const act_t*)a.skip, h) : 0.f;
-  float4 S[4];                                         // S[j]: channel 4 cg + j, the four columns
+  auto at = [&](auto& row) -> Vec& { return *reinterpret_cast<Vec*>(&row[VW * vg]); };            // this thread's columns of a row in shared memory
+  auto of = [&](const auto& row) -> const Vec& { return *reinterpret_cast<const Vec*>(&row[VW * vg]); };
+  Vec S[4];                                            // S[j]: channel 4 cg + j
   if (own) {
-    float4 col[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) col[e] = *reinterpret_cast<const float4*>(st + (size_t)(v0 + 4 * vg + e) * K + 4 * cg);
-    S[0] = make_float4(col[0].x, col[1].x, col[2].x, col[3].x);
-    S[1] = make_float4(col[0].y, col[1].y, col[2].y, col[3].y);
-    S[2] = make_float4(col[0].z, col[1].z, col[2].z, col[3].z);
-    S[3] = make_float4(col[0].w, col[1].w, col[2].w, col[3].w);
+    for (int e = 0; e < VW; ++e) {
+      const float4 c = *reinterpret_cast<const float4*>(st + (size_t)(v0 + VW * vg + e) * K + 4 * cg);
+      S[0].v[e] = c.x; S[1].v[e] = c.y; S[2].v[e] = c.z; S[3].v[e] = c.w;
+    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.S[4 * cg + j][4 * vg]) = S[j];
+    for (int j = 0; j < 4; ++j) at(sm.S[4 * cg + j]) = S[j];
   }
   __syncthreads();
   for (int n = 0; n < n_chunks; ++n) {
     const Stage& s = sm.st[n & 1];
     constexpr int RT = Stage::ROWS / 8;                // rows per lane
-    // (P and) R: this warp's quarter of the channels
-    const int tg = lane >> 2;
+    // (P and) R in tiles of RT rows x 4 columns: a quarter of the channels per warp, with 8 columns an eighth per half warp
+    constexpr int SLICES = 64 / VT;
+    const int slice = VT == 16 ? warp : 2 * warp + (lane >> 4), tg = VT == 16 ? lane >> 2 : (lane >> 1) & 7, c4 = 4 * (VT == 16 ? vg : lane & 1);
     float4 acc[RT] = {};
 #pragma unroll 8
-    for (int c = warp * (K / 4); c < (warp + 1) * (K / 4); ++c) {
-      const float4 y = *reinterpret_cast<const float4*>(&sm.S[c][4 * vg]);
+    for (int c = slice * (K / SLICES); c < (slice + 1) * (K / SLICES); ++c) {
+      const float4 y = *reinterpret_cast<const float4*>(&sm.S[c][c4]);
       if (DELTA) {
         const float4 x = *reinterpret_cast<const float4*>(&s.kq[c][4 * tg]);
         fma4(acc[0], x.x, y); fma4(acc[1], x.y, y); fma4(acc[RT - 2], x.z, y); fma4(acc[RT - 1], x.w, y);
@@ -632,68 +646,75 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
       }
     }
 #pragma unroll
-    for (int j = 0; j < RT; ++j) *reinterpret_cast<float4*>(&sm.part[warp][RT * tg + j][4 * vg]) = acc[j];
+    for (int j = 0; j < RT; ++j) *reinterpret_cast<float4*>(&sm.part[slice][RT * tg + j][c4]) = acc[j];
     walk_bar();
     // row cg: v - P, or R
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    Vec r = {};
     if (cg < Stage::ROWS) {
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const float4 p = *reinterpret_cast<const float4*>(&sm.part[w][cg][4 * vg]);
-        r.x += p.x; r.y += p.y; r.z += p.z; r.w += p.w;
+      for (int w = 0; w < SLICES; ++w) {
+        const Vec p = of(sm.part[w][cg]);
+#pragma unroll
+        for (int e = 0; e < VW; ++e) r.v[e] += p.v[e];
       }
     }
     if (DELTA) {
       if (cg < CH_C) {
-        const float4 v = *reinterpret_cast<const float4*>(&s.v[cg][4 * vg]);
-        *reinterpret_cast<float4*>(&sm.w[cg][4 * vg]) = make_float4(v.x - r.x, v.y - r.y, v.z - r.z, v.w - r.w);
-        r = make_float4(0.f, 0.f, 0.f, 0.f);
+        const Vec v = of(s.v[cg]);
+#pragma unroll
+        for (int e = 0; e < VW; ++e) r.v[e] = v.v[e] - r.v[e];
+        at(sm.w[cg]) = r;
+        r = Vec{};
       }
       walk_bar();
     }
-    const float (*in)[CH_VT] = DELTA ? sm.w : s.u;
+    const float (*in)[VT] = DELTA ? sm.w : s.u;
     if (cg < Stage::ROWS) {
       const int tt = cg & (CH_C - 1);                  // tokens up to this row's: a zero weight would turn a later token's infinity into NaN
 #pragma unroll
       for (int i = 0; i < CH_C; i += 4) {
         const float4 m = *reinterpret_cast<const float4*>(&s.tm[cg][i]);
-        if (i <= tt) fma4(r, m.x, *reinterpret_cast<const float4*>(&in[i][4 * vg]));
-        if (i + 1 <= tt) fma4(r, m.y, *reinterpret_cast<const float4*>(&in[i + 1][4 * vg]));
-        if (i + 2 <= tt) fma4(r, m.z, *reinterpret_cast<const float4*>(&in[i + 2][4 * vg]));
-        if (i + 3 <= tt) fma4(r, m.w, *reinterpret_cast<const float4*>(&in[i + 3][4 * vg]));
+        if (i <= tt) r.fma(m.x, of(in[i]));
+        if (i + 1 <= tt) r.fma(m.y, of(in[i + 1]));
+        if (i + 2 <= tt) r.fma(m.z, of(in[i + 2]));
+        if (i + 3 <= tt) r.fma(m.w, of(in[i + 3]));
       }
       if (DELTA && cg < CH_C) {
-        *reinterpret_cast<float4*>(&sm.u[cg][4 * vg]) = r;
+        at(sm.u[cg]) = r;
       } else {
         const int t = n * CH_C + tt;
         if (t < a.T) {
-          const float4 v = *reinterpret_cast<const float4*>(&s.v[tt][4 * vg]);
-          float* o = a.out + (size_t)t * a.ldo + (size_t)h * a.V + v0 + 4 * vg;
-          o[0] = r.x * a.q_mult + skip * v.x; o[1] = r.y * a.q_mult + skip * v.y; o[2] = r.z * a.q_mult + skip * v.z; o[3] = r.w * a.q_mult + skip * v.w;
+          const Vec v = of(s.v[tt]);
+          float* o = a.out + (size_t)t * a.ldo + (size_t)h * a.V + v0 + VW * vg;
+#pragma unroll
+          for (int e = 0; e < VW; ++e) o[e] = r.v[e] * a.q_mult + skip * v.v[e];
         }
       }
     }
     if (DELTA) walk_bar();
-    const float (*add)[CH_VT] = DELTA ? sm.u : s.u;
+    const float (*add)[VT] = DELTA ? sm.u : s.u;
     if (own) {
       const float4 g = *reinterpret_cast<const float4*>(&s.gc[4 * cg]);
       const float gj[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) { S[j].x *= gj[j]; S[j].y *= gj[j]; S[j].z *= gj[j]; S[j].w *= gj[j]; }
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < VW; ++e) S[j].v[e] *= gj[j];
 #pragma unroll 8
       for (int i = 0; i < CH_C; ++i) {
-        const float4 x = *reinterpret_cast<const float4*>(&s.kd[i][4 * cg]), y = *reinterpret_cast<const float4*>(&add[i][4 * vg]);
-        fma4(S[0], x.x, y); fma4(S[1], x.y, y); fma4(S[2], x.z, y); fma4(S[3], x.w, y);
+        const float4 x = *reinterpret_cast<const float4*>(&s.kd[i][4 * cg]);
+        const Vec y = of(add[i]);
+        S[0].fma(x.x, y); S[1].fma(x.y, y); S[2].fma(x.z, y); S[3].fma(x.w, y);
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(&sm.S[4 * cg + j][4 * vg]) = S[j];
+      for (int j = 0; j < 4; ++j) at(sm.S[4 * cg + j]) = S[j];
     }
     __syncthreads();                                   // the next chunk's operands and the state are in place
   }
   if (own) {
-    const float s4[4][4] = {{S[0].x, S[1].x, S[2].x, S[3].x}, {S[0].y, S[1].y, S[2].y, S[3].y}, {S[0].z, S[1].z, S[2].z, S[3].z}, {S[0].w, S[1].w, S[2].w, S[3].w}};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) *reinterpret_cast<float4*>(st + (size_t)(v0 + 4 * vg + e) * K + 4 * cg) = make_float4(s4[e][0], s4[e][1], s4[e][2], s4[e][3]);
+    for (int e = 0; e < VW; ++e)
+      *reinterpret_cast<float4*>(st + (size_t)(v0 + VW * vg + e) * K + 4 * cg) = make_float4(S[0].v[e], S[1].v[e], S[2].v[e], S[3].v[e]);
   }
 }
 
@@ -704,14 +725,16 @@ static bool walk_sizes(int T, int K, int V, int ones) { return T >= 2 * CH_C && 
 // of its own (16 heads of 128 x 128, 48 tokens: 20..26 against 27..29 us; 32 tokens: 17..24 against 21..23), from 64 on otherwise (64 heads of
 // 64 x 64, 33 tokens: 26..30 against 21..23; 64 tokens: 28..32 against 35..39).  Against the chunked form without the delta rule, which
 // stays flat until its CTAs fill the SMs while the walk takes 1.3 us (1.0 with 64 keys) per 16 tokens and turn of CTAs whatever the heads:
-// both times from the fits below, in ns (128 x 128, us walk / chunked: 1024 tokens of 4 heads 95 / 103; 2048 of 4 173 / 130, of 8 179 / 240;
-// 4096 of 4 333 / 251, of 8 345 / 388; 8192 of 1 634 / 134, of 8 673 / 667, of 16 710 / 1285).
+// both times from the fits below, in ns (128 x 128, us walk with 16 columns per CTA / chunked: 1024 tokens of 4 heads 95 / 103; 2048 of 4 173 / 130,
+// of 8 179 / 240; 4096 of 4 333 / 251, of 8 345 / 388; 8192 of 1 634 / 134, of 8 673 / 667, of 16 710 / 1285; walk with 8 columns: 512 tokens of 4
+// and 8 43, 2048 of 4 124, of 8 128; with 64 keys 512 tokens 38, 1024 of 18 63).
+static bool walk_narrow(int heads, int V) { return (long long)heads * (V / CH_NARROW) <= sm_count(); }
 static bool walk_pays(int T, int heads, int K, int V, int delta) {
   const long long sms = sm_count(), ctas = (long long)heads * (V / CH_VT), turns = (ctas + sms - 1) / sms;
   if (T < (turns <= 1 ? 48 : 64)) return false;
   if (delta || T < 2 * SCAN_CHUNK) return true;
   const long long cols = K == 64 ? 64 : 32, chunked = (V + cols - 1) / cols * heads * ((T + SCAN_CHUNK - 1) / SCAN_CHUNK), load = (chunked + sms - 1) / sms;
-  const long long t_chunked = load == 1 ? 104000 : load == 2 ? 131000 : 60000 + 45000 * load, t_walk = 15000 + (long long)(T / CH_C) * (K == 64 ? 1050 : 1350) * turns;
+  const long long t_chunked = load == 1 ? 104000 : load == 2 ? 131000 : 60000 + 45000 * load, t_walk = 15000 + (long long)(T / CH_C) * (walk_narrow(heads, V) ? (K == 64 ? 800 : 920) : (K == 64 ? 1050 : 1350)) * turns;
   return t_walk <= t_chunked;
 }
 // Portions of two chunks or more with key sizes 64 or 128 and whole groups of 16 values, given room for the chunks' matrices; other sizes, the
@@ -726,15 +749,19 @@ static bool walk_chunks(const b2l_seq_scan_args* a) {
 
 template <typename act_t, int K, bool DELTA>
 static int launch_walk(const b2l_seq_scan_args* a, cudaStream_t s) {
-  static DynSmemCache cache;
-  if (int rc = ensure_dyn_smem(seq_walk_kernel<act_t, K, DELTA>, sizeof(WalkSmem<K, DELTA>), cache)) return rc;
   auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   const int vec = a->ldq % 4 == 0 && a->ldk % 4 == 0 && al(a->q) && al(a->k) && (!a->decay_per_channel || (a->ldd % 4 == 0 && al(a->decay)));
   seq_chunk_kernel<act_t, K, DELTA><<<dim3((unsigned)((a->T + CH_C - 1) / CH_C), (unsigned)a->heads), CHUNK_THREADS, 0, s>>>(*a, vec);
   B2L_LAUNCH_CHECK("seq_chunk_kernel");
-  seq_walk_kernel<act_t, K, DELTA><<<dim3((unsigned)(a->V / CH_VT), (unsigned)a->heads), 384, sizeof(WalkSmem<K, DELTA>), s>>>(*a);
-  B2L_LAUNCH_CHECK("seq_walk_kernel");
-  return 0;
+  auto walk = [&](auto vt) {
+    constexpr int VT = decltype(vt)::value;
+    static DynSmemCache cache;
+    if (int rc = ensure_dyn_smem(seq_walk_kernel<act_t, K, DELTA, VT>, sizeof(WalkSmem<K, DELTA, VT>), cache)) return rc;
+    seq_walk_kernel<act_t, K, DELTA, VT><<<dim3((unsigned)(a->V / VT), (unsigned)a->heads), 384, sizeof(WalkSmem<K, DELTA, VT>), s>>>(*a);
+    B2L_LAUNCH_CHECK("seq_walk_kernel");
+    return 0;
+  };
+  return walk_narrow(a->heads, a->V) ? walk(std::integral_constant<int, CH_NARROW>{}) : walk(std::integral_constant<int, CH_VT>{});
 }
 
 static DynSmemCache g_scan_smem[10];

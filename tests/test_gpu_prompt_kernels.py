@@ -286,6 +286,13 @@ def test_scan_plan_and_its_neighbours(T, H, K, V, want):
         assert rel(got, out) < 1e-6 and rel(st, state) < 1e-6
 
 
+@pytest.mark.parametrize("T,K,V,H,G,form", [(47, 128, 48, 24, 2, "delta"), (47, 128, 48, 25, 5, "delta"), (70, 64, 64, 18, 3, "scalar"), (70, 64, 64, 20, 4, "scalar"),
+                                            (33, 128, 128, 9, 9, "channel"), (33, 128, 128, 10, 5, "channel")])
+def test_scans_by_columns_per_cta(T, K, V, H, G, form):
+    """Eight value columns per CTA up to 148 CTAs and sixteen beyond: both sides of the rule."""
+    test_scans_sixteen_tokens_at_a_time(T, K, V, H, G, form)
+
+
 @pytest.mark.parametrize("T,pos0,q_scale,v_mean", [(130, 1900, 1.0, 0.0), (130, 1900, 1.0, 2.0), (200, 900, 4.0, 0.0), (64, 4000, 0.1, 2.0)])
 def test_local_attention_rounds_like_f32_over_many_keys(T, pos0, q_scale, v_mean):
     """Sums over thousands of keys carry no bias of the tensor core's truncating adds: relative error below 8e-7 = 13 * 2^-24 (rounded adds of 32
