@@ -206,9 +206,11 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
   }
 }
 
-// Four taps over long portions in bf16: a thread owns 8 neighbouring channels (16-byte loads, two 16-byte stores) and CONV_VT tokens, so the
-// bytes in flight suffice for HBM (6144 channels x 2048 tokens: 30 us with the unit heads, 35 with 16 tokens a thread, 73 one channel at a time); sums in the order of the kernel above.
-constexpr int CONV_VT = 8, CONV_V = 8;
+// Four taps over long portions in bf16: a thread owns V neighbouring channels and CONV_VT tokens, so the bytes in flight suffice for HBM.  Four
+// channels (8-byte loads, one 16-byte store, 64 registers) keep twice the warps of eight on an SM: 6144 channels x 2048 tokens with the unit
+// heads 26.5 us against 30.3 (73 one channel at a time, 35 with eight channels and 16 tokens).  Eight only where a head of more than 128
+// channels is to lie in one warp.  Sums in the order of the kernel above.
+constexpr int CONV_VT = 8;
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -218,42 +220,51 @@ __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) 
     x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
 }
-// UNIT: the heads of `size` channels at a0 .. and at b0 .. become unit vectors times ma or mb on the way (size / 8 neighbouring lanes hold a head).
+// UNIT: the heads of `size` channels at a0 .. and at b0 .. become unit vectors times ma or mb on the way (size / V neighbouring lanes hold a head).
 struct UnitHeads { int a0, a1, b0, b1, size; float eps, ma, mb; };
-template <bool UNIT>
+template <int V> __device__ __forceinline__ void ldv_bf16(const __nv_bfloat16* p, float (&x)[V]) {
+  if constexpr (V == 8) {
+    ld8_bf16(p, x);
+  } else {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
+    x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
+  }
+}
+template <bool UNIT, int V>
 __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16* __restrict__ in, int ldin, const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ state,
                                                             const int* __restrict__ meta, float* __restrict__ out, int ldout, int T, int C, UnitHeads u) {
-  const int c0 = (blockIdx.x * 128 + threadIdx.x) * CONV_V, c = min(c0, C - CONV_V);      // lanes past the last channel repeat it
+  const int c0 = (blockIdx.x * 128 + threadIdx.x) * V, c = min(c0, C - V);      // lanes past the last channel repeat it
   const float mult = !UNIT ? 0.f : c >= u.a0 && c < u.a1 ? u.ma : c >= u.b0 && c < u.b1 ? u.mb : 0.f;
   const bool any = UNIT && __any_sync(0xffffffffu, mult != 0.f);
   const int t0 = blockIdx.y * CONV_VT, nt = min(CONV_VT, T - t0);
   const __nv_bfloat16* st = state + (size_t)meta[0] * 3 * C;
-  float wr[4][8], win[3][8], b[8];
+  float wr[4][V], win[3][V], b[V];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {                         // w is [channel][tap]
+  for (int i = 0; i < V / 2; ++i) {                         // w is [channel][tap]
     float x[8];
     ld8_bf16(w + (size_t)c * 4 + 8 * i, x);
 #pragma unroll
     for (int e = 0; e < 8; ++e) wr[e & 3][2 * i + (e >> 2)] = x[e];
   }
 #pragma unroll
-  for (int e = 0; e < 8; ++e) b[e] = 0.f;
+  for (int e = 0; e < V; ++e) b[e] = 0.f;
   if (bias) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) b[e] = __bfloat162float(bias[c + e]);
+    for (int e = 0; e < V; ++e) b[e] = __bfloat162float(bias[c + e]);
   }
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const int t = t0 - 3 + j;
-    ld8_bf16(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(3 + t) * C + c, win[j]);
+    ldv_bf16<V>(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(3 + t) * C + c, win[j]);
   }
 #pragma unroll 4
   for (int r = 0; r < nt; ++r) {
-    float cur[8], y[8];
-    ld8_bf16(in + (size_t)(t0 + r) * ldin + c, cur);
+    float cur[V], y[V];
+    ldv_bf16<V>(in + (size_t)(t0 + r) * ldin + c, cur);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < V; ++e) {
       float acc = b[e];
       acc += wr[0][e] * win[0][e];
       acc += wr[1][e] * win[1][e];
@@ -267,16 +278,16 @@ __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16
     if (any) {
       float ss = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += y[e] * y[e];
-      for (int d = 1; d < u.size / CONV_V; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+      for (int e = 0; e < V; ++e) ss += y[e] * y[e];
+      for (int d = 1; d < u.size / V; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
       const float f = mult != 0.f ? mult / sqrtf(ss + u.eps) : 1.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] *= f;
+      for (int e = 0; e < V; ++e) y[e] *= f;
     }
     float4* o = reinterpret_cast<float4*>(out + (size_t)(t0 + r) * ldout + c);
     if (c0 >= C) continue;
     o[0] = make_float4(y[0], y[1], y[2], y[3]);
-    o[1] = make_float4(y[4], y[5], y[6], y[7]);
+    if constexpr (V == 8) o[1] = make_float4(y[4], y[5], y[6], y[7]);
   }
 }
 
@@ -572,13 +583,13 @@ static int conv_silu(const void* in, int ldin, const void* w, const void* bias, 
   if (T == 0) return 0;
   const int tiles = (T + CONV_TT - 1) / CONV_TT;
   dim3 grid((unsigned)((C + 127) / 128), (unsigned)tiles);
-  if (act_dtype == B2L_BF16 && taps == 4 && T > CONV_TT && C % CONV_V == 0 && ldin % 8 == 0 && ldout % 4 == 0 && al16(in) && al16(w) && al16(state) && al16(out) &&
+  if (act_dtype == B2L_BF16 && taps == 4 && T > CONV_TT && C % 8 == 0 && ldin % 8 == 0 && ldout % 4 == 0 && al16(in) && al16(w) && al16(state) && al16(out) &&
       (T + CONV_VT - 1) / CONV_VT <= 65535) {
-    const dim3 grid4((unsigned)((C / CONV_V + 127) / 128), (unsigned)((T + CONV_VT - 1) / CONV_VT));
-    const int lanes = unit ? unit->size / CONV_V : 0;
-    const bool fits = unit && unit->size % CONV_V == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && unit->a0 % unit->size == 0 && unit->b0 % unit->size == 0 &&
+    const int wide = unit && unit->size > 128 ? 8 : 4, lanes = unit ? unit->size / wide : 0;       // a head of the unit vectors lies in one warp
+    const bool fits = unit && unit->size % wide == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && unit->a0 % unit->size == 0 && unit->b0 % unit->size == 0 &&
                       unit->ma != 0.f && unit->mb != 0.f;
-    auto kernel = fits ? seq_conv4_silu_kernel<true> : seq_conv4_silu_kernel<false>;
+    const dim3 grid4((unsigned)((C / (fits ? wide : 4) + 127) / 128), (unsigned)((T + CONV_VT - 1) / CONV_VT));
+    auto kernel = !fits ? seq_conv4_silu_kernel<false, 4> : wide == 8 ? seq_conv4_silu_kernel<true, 8> : seq_conv4_silu_kernel<true, 4>;
     kernel<<<grid4, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)state, meta, out, ldout,
                                                     T, C, fits ? *unit : UnitHeads{});
     if (unit_done) *unit_done = fits;
