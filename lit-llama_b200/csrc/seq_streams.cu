@@ -145,7 +145,7 @@ constexpr int MOST_PAIRS = 4096;      // rotated pairs whose cos and sin fit the
 //   q_out is multiplied by the query temperature of its position when temp_every > 0.
 //   v_out (act): (1 - lambda) v + lambda v_first when v_first is given (lambda read on the device), else not written.
 template <typename act_t, bool TABLE>      // TABLE: up to MOST_PAIRS pairs
-__global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args a, int quads) {
+__global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args a) {
   __shared__ float red[32];
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const act_t* row = (const act_t*)a.proj + (size_t)t * a.ld;
@@ -168,57 +168,12 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
     float r_row = 1.f;
     if (w && a.whole_row) {
       float ss = 0.f;
-      if (quads && sizeof(act_t) == 2) {
-        for (int i = threadIdx.x * 4; i < heads * K; i += blockDim.x * 4) {
-          const uint2 u = *reinterpret_cast<const uint2*>(x + i);
-          const float v0 = __uint_as_float(u.x << 16), v1 = __uint_as_float(u.x & 0xffff0000u), v2 = __uint_as_float(u.y << 16), v3 = __uint_as_float(u.y & 0xffff0000u);
-          ss += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
-        }
-      } else {
-        for (int i = threadIdx.x; i < heads * K; i += blockDim.x) {
-          const float v = ld_act(x, i);
-          ss += v * v;
-        }
+      for (int i = threadIdx.x; i < heads * K; i += blockDim.x) {
+        const float v = ld_act(x, i);
+        ss += v * v;
       }
       ss = block_sum(ss, red);
       r_row = 1.0f / sqrtf(ss / (float)(heads * K) + a.eps);
-    }
-    if (quads && sizeof(act_t) == 2) {
-      // one factor for the whole row: four neighbouring pairs per thread, 8-byte loads (a lane per pair with 2-byte loads took 27 us for 2048 tokens of 16 + 4 heads, so 17)
-      const int per = half / 4;
-      for (int u = threadIdx.x; u < heads * per; u += blockDim.x) {
-        const int hd = u / per, i = (u - hd * per) * 4;
-        const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(x) + (size_t)hd * K + i;
-        const __nv_bfloat16* pw = reinterpret_cast<const __nv_bfloat16*>(w) + (size_t)hd * K + i;
-        const uint2 a0 = *reinterpret_cast<const uint2*>(p), a1 = *reinterpret_cast<const uint2*>(p + half);
-        const uint2 w0 = w ? *reinterpret_cast<const uint2*>(pw) : make_uint2(0x3f803f80u, 0x3f803f80u);
-        const uint2 w1 = w ? *reinterpret_cast<const uint2*>(pw + half) : make_uint2(0x3f803f80u, 0x3f803f80u);
-        const uint32_t ua[4] = {a0.x, a0.y, a1.x, a1.y}, uw[4] = {w0.x, w0.y, w1.x, w1.y};
-        float lo[4], hi[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = e >> 1;
-          const float xu = __uint_as_float(e & 1 ? ua[j] & 0xffff0000u : ua[j] << 16), wu = __uint_as_float(e & 1 ? uw[j] & 0xffff0000u : uw[j] << 16);
-          const float xv = __uint_as_float(e & 1 ? ua[2 + j] & 0xffff0000u : ua[2 + j] << 16), wv = __uint_as_float(e & 1 ? uw[2 + j] & 0xffff0000u : uw[2 + j] << 16);
-          const float pu = xu * r_row * wu, pv = xv * r_row * wv, c = turn[i + e], s = turn[half + i + e];
-          lo[e] = pu * c - pv * s;
-          hi[e] = pv * c + pu * s;
-        }
-        if (which == 0) {
-          float* qo = a.q_out + ((size_t)t * heads + hd) * K + i;
-          *reinterpret_cast<float4*>(qo) = make_float4(lo[0] * temp, lo[1] * temp, lo[2] * temp, lo[3] * temp);
-          *reinterpret_cast<float4*>(qo + half) = make_float4(hi[0] * temp, hi[1] * temp, hi[2] * temp, hi[3] * temp);
-        } else {
-          __nv_bfloat16* ko = (__nv_bfloat16*)a.k_out + ((size_t)t * heads + hd) * K + i;
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            const float (&y)[4] = b ? hi : lo;
-            const __nv_bfloat162 y0 = __floats2bfloat162_rn(y[0], y[1]), y1 = __floats2bfloat162_rn(y[2], y[3]);
-            *reinterpret_cast<uint2*>(ko + b * half) = make_uint2(*reinterpret_cast<const uint32_t*>(&y0), *reinterpret_cast<const uint32_t*>(&y1));
-          }
-        }
-      }
-      continue;
     }
     for (int hd = warp; hd < heads; hd += nw) {
       const act_t* p = x + (size_t)hd * K;
@@ -269,6 +224,125 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
     const act_t* vf = (const act_t*)a.v_first + (size_t)t * a.ldvf;
     act_t* vo = (act_t*)a.v_out + (size_t)t * a.kv_heads * a.V;
     for (int i = threadIdx.x; i < a.kv_heads * a.V; i += blockDim.x) st_act(vo, i, (1.f - lam) * ld_act(v, i) + lam * ld_act(vf, i));
+  }
+}
+
+// The same in bf16 where whole heads turn and a row has one factor: four neighbouring pairs (u: 16 bytes of x) are a unit, a thread holds NU of the
+// token's units in registers, so x is read once, with its norm weights for all of the CTA's tokens, and the next token's x travels meanwhile.
+// Bound by the chain from launch to store: a token per CTA, each waiting for its angles and then for x, took 14.3 us for 2048 tokens of 16 + 4
+// heads of 128 with norms; four tokens per CTA 10.0.
+constexpr int QUAD_THREADS = 512;
+template <int NU>
+__global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_seq_qkv_prep_args a, int tokens) {
+  __shared__ float red[2][2][QUAD_THREADS / 32];
+  extern __shared__ __align__(16) float turn_quads[];   // per token: cos | sin of the pairs, times rot_mult
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+  const int K = a.K, half = K / 2, per = half / 4, units_q = a.heads * per, units = units_q + a.kv_heads * per;
+  const int t0 = blockIdx.x * tokens, nt = min(tokens, a.T - t0);
+  const __nv_bfloat16* qw = (const __nv_bfloat16*)a.q_norm;
+  const __nv_bfloat16* kw = (const __nv_bfloat16*)a.k_norm;
+  uint2 x0[NU], x1[NU], w0[NU], w1[NU];
+  int at[NU], xat[NU];                                  // first entry of the unit: in its row of heads, in the projection's row
+#pragma unroll
+  for (int i = 0; i < NU; ++i) {
+    const int u = min(tid + i * (int)blockDim.x, units - 1), uu = u < units_q ? u : u - units_q, hd = uu / per;
+    at[i] = hd * K + (uu - hd * per) * 4;
+    xat[i] = at[i] + (u < units_q ? a.q_off : a.k_off);
+  }
+  auto load = [&](int t) {
+    const __nv_bfloat16* row = (const __nv_bfloat16*)a.proj + (size_t)t * a.ld;
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      x0[i] = *reinterpret_cast<const uint2*>(row + xat[i]);
+      x1[i] = *reinterpret_cast<const uint2*>(row + xat[i] + half);
+    }
+  };
+  load(t0);
+#pragma unroll
+  for (int i = 0; i < NU; ++i) {
+    const __nv_bfloat16* w = tid + i * (int)blockDim.x < units_q ? qw : kw;
+    w0[i] = w ? *reinterpret_cast<const uint2*>(w + at[i]) : make_uint2(0x3f803f80u, 0x3f803f80u);
+    w1[i] = w ? *reinterpret_cast<const uint2*>(w + at[i] + half) : make_uint2(0x3f803f80u, 0x3f803f80u);
+  }
+  const int pos0 = a.meta[1] + t0;
+  for (int i = tid; i < nt * half; i += blockDim.x) {
+    const int n = i / half, j = i - n * half;
+    float s, c;
+    sincosf((float)(pos0 + n) * a.freq[j], &s, &c);
+    turn_quads[n * K + j] = c * a.rot_mult;
+    turn_quads[n * K + half + j] = s * a.rot_mult;
+  }
+  auto lo16 = [](uint32_t v) { return __uint_as_float(v << 16); };
+  auto hi16 = [](uint32_t v) { return __uint_as_float(v & 0xffff0000u); };
+  for (int n = 0; n < nt; ++n) {
+    const int t = t0 + n;
+    float rq = 1.f, rk = 1.f;
+    if (qw || kw) {
+      float sq = 0.f, sk = 0.f;
+#pragma unroll
+      for (int i = 0; i < NU; ++i) {
+        const int u = tid + i * (int)blockDim.x;
+        const uint32_t w[4] = {x0[i].x, x0[i].y, x1[i].x, x1[i].y};
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss += lo16(w[e]) * lo16(w[e]) + hi16(w[e]) * hi16(w[e]);
+        if (u < units_q) sq += ss;
+        else if (u < units) sk += ss;
+      }
+      sq = warp_sum(sq);
+      sk = warp_sum(sk);
+      if (lane == 0) { red[n & 1][0][warp] = sq; red[n & 1][1][warp] = sk; }
+    }
+    if (n == 0 || qw || kw) __syncthreads();            // the angles; the sums (the other buffer is read until the next token's barrier)
+    if (qw || kw) {
+      float sq = 0.f, sk = 0.f;
+      for (int w = 0; w < nw; ++w) { sq += red[n & 1][0][w]; sk += red[n & 1][1][w]; }
+      if (qw) rq = 1.0f / sqrtf(sq / (float)(a.heads * K) + a.eps);
+      if (kw) rk = 1.0f / sqrtf(sk / (float)(a.kv_heads * K) + a.eps);
+    }
+    const float temp = a.temp_every > 0 ? 1.0f + a.temp_coef * logf((float)((pos0 + n + 1) / a.temp_every + 1)) : 1.0f;
+    const float* tn = turn_quads + n * K;
+    float y[NU][8];
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      const bool is_q = tid + i * (int)blockDim.x < units_q;
+      const float r = is_q ? rq : rk;
+      const int j = at[i] % K;                          // the unit's first pair
+      const float4 c4 = *reinterpret_cast<const float4*>(tn + j), s4 = *reinterpret_cast<const float4*>(tn + half + j);
+      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+      const uint32_t ux[4] = {x0[i].x, x0[i].y, x1[i].x, x1[i].y}, uw[4] = {w0[i].x, w0[i].y, w1[i].x, w1[i].y};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t xu = ux[e >> 1], wu = uw[e >> 1], xv = ux[2 + (e >> 1)], wv = uw[2 + (e >> 1)];
+        const float pu = (e & 1 ? hi16(xu) : lo16(xu)) * r * (e & 1 ? hi16(wu) : lo16(wu)), pv = (e & 1 ? hi16(xv) : lo16(xv)) * r * (e & 1 ? hi16(wv) : lo16(wv));
+        y[i][e] = pu * c[e] - pv * s[e];
+        y[i][4 + e] = pv * c[e] + pu * s[e];
+      }
+    }
+    if (n + 1 < nt) load(t + 1);
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      const int u = tid + i * (int)blockDim.x;
+      if (u < units_q) {
+        float* qo = a.q_out + (size_t)t * a.heads * K + at[i];
+        *reinterpret_cast<float4*>(qo) = make_float4(y[i][0] * temp, y[i][1] * temp, y[i][2] * temp, y[i][3] * temp);
+        *reinterpret_cast<float4*>(qo + half) = make_float4(y[i][4] * temp, y[i][5] * temp, y[i][6] * temp, y[i][7] * temp);
+      } else if (u < units) {
+        __nv_bfloat16* ko = (__nv_bfloat16*)a.k_out + (size_t)t * a.kv_heads * K + at[i];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const __nv_bfloat162 y0 = __floats2bfloat162_rn(y[i][4 * b], y[i][4 * b + 1]), y1 = __floats2bfloat162_rn(y[i][4 * b + 2], y[i][4 * b + 3]);
+          *reinterpret_cast<uint2*>(ko + b * half) = make_uint2(*reinterpret_cast<const uint32_t*>(&y0), *reinterpret_cast<const uint32_t*>(&y1));
+        }
+      }
+    }
+    if (a.v_first != nullptr) {
+      const float lam = ld_act((const __nv_bfloat16*)a.lambda, 0);
+      const __nv_bfloat16* v = (const __nv_bfloat16*)a.proj + (size_t)t * a.ld + a.v_off;
+      const __nv_bfloat16* vf = (const __nv_bfloat16*)a.v_first + (size_t)t * a.ldvf;
+      __nv_bfloat16* vo = (__nv_bfloat16*)a.v_out + (size_t)t * a.kv_heads * a.V;
+      for (int i = tid; i < a.kv_heads * a.V; i += blockDim.x) st_act(vo, i, (1.f - lam) * ld_act(v, i) + lam * ld_act(vf, i));
+    }
   }
 }
 
@@ -368,9 +442,20 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   const bool table = a->rot_dims / 2 <= MOST_PAIRS;
   const int quads = table && a->act_dtype == B2L_BF16 && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
                     a->k_off % 4 == 0 && a->ld % 4 == 0 && al8(a->proj) && al8(a->q_norm) && al8(a->k_norm) && al16(a->q_out) && al8(a->k_out);
+  const long long units = (long long)(a->heads + a->kv_heads) * (a->K / 8);
+  if (quads && units <= 8 * QUAD_THREADS) {
+    // tokens per CTA: up to four where two CTAs per SM are left (the angles of a CTA come at once, its tokens' x one ahead), as far as their angles fit
+    const int fill = a->T / (2 * sm_count()), tokens = a->K > 2048 ? 1 : fill < 1 ? 1 : fill > 4 ? 4 : fill;
+    const int nu = units <= QUAD_THREADS / 2 ? 1 : units <= QUAD_THREADS ? 2 : units <= 4 * QUAD_THREADS ? 4 : 8;
+    const int threads = (int)((units + 32 * nu - 1) / (32 * nu)) * 32;
+    auto kernel = nu == 1 ? seq_qkv_prep_quads_kernel<1> : nu == 2 ? seq_qkv_prep_quads_kernel<2> : nu == 4 ? seq_qkv_prep_quads_kernel<4> : seq_qkv_prep_quads_kernel<8>;
+    kernel<<<(a->T + tokens - 1) / tokens, threads, sizeof(float) * a->K * tokens, (cudaStream_t)stream>>>(*a, tokens);
+    B2L_LAUNCH_CHECK("seq_qkv_prep_quads_kernel");
+    return 0;
+  }
   B2L_SEQ_DISPATCH(a->act_dtype, {
-    if (table) seq_qkv_prep_kernel<act_t, true><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a, quads);
-    else seq_qkv_prep_kernel<act_t, false><<<a->T, 256, 0, (cudaStream_t)stream>>>(*a, quads);
+    if (table) seq_qkv_prep_kernel<act_t, true><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a);
+    else seq_qkv_prep_kernel<act_t, false><<<a->T, 256, 0, (cudaStream_t)stream>>>(*a);
   });
   B2L_LAUNCH_CHECK("seq_qkv_prep_kernel");
   return 0;

@@ -254,6 +254,43 @@ def test_attention_operands_of_very_wide_heads(rot):
         assert float((got - want).abs().max()) < 1e-5 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("T,H,G,K,norms,mix", [(1, 16, 4, 128, "qk", True), (1187, 2, 1, 16, "qk", False), (700, 16, 4, 128, "", True), (900, 3, 2, 24, "k", True), (5, 130, 6, 128, "qk", False),
+                                               (9, 40, 8, 128, "q", True)])
+def test_attention_operands_by_quads_of_pairs(T, H, G, K, norms, mix):
+    """One to eight units per thread, one to four tokens per CTA with a remainder, either row's norm, the query temperature, mixed values.  Angles up to 40 are good to
+    40 * 2^-24, products and sums add a few 2^-24: 1e-5 of the largest entry; k and v are rounded to bf16 on top (2^-9 of an entry)."""
+    from lit_llama_b200 import _seqlib as S
+
+    V, pos0, g = 40, 30, torch.Generator(device=DEV).manual_seed(T + H)
+    n = (H + G) * K + G * V + 12
+    x = torch.randn(T, n, generator=g, device=DEV).to(BF)
+    o_k, o_v = H * K + 4, (H + G) * K + 4
+    w = {c: (torch.randn(m * K, generator=g, device=DEV) * 0.1 + 1).to(BF) for c, m in (("q", H), ("k", G))}
+    freq, vf, lam = torch.rand(K // 2, generator=g, device=DEV) * 40 / (pos0 + T), torch.randn(T, G * V, generator=g, device=DEV).to(BF), torch.tensor([0.3], device=DEV).to(BF)
+    meta, q, k, v = torch.tensor([0, pos0], dtype=torch.int32, device=DEV), torch.full((T + 1, H * K), 7.0, device=DEV), torch.full((T + 1, G * K), 7.0, device=DEV).to(BF), torch.empty(T, G * V, device=DEV).to(BF)
+    a = S.QkvPrepArgs(proj=x.data_ptr(), ld=n, q_off=0, k_off=o_k, v_off=o_v, q_norm=w["q"].data_ptr() if "q" in norms else None, k_norm=w["k"].data_ptr() if "k" in norms else None,
+                      whole_row=int(bool(norms)), eps=1e-6, freq=freq.data_ptr(), rot_dims=K, rot_mult=1.1, meta=meta.data_ptr(), q_out=q.data_ptr(), k_out=k.data_ptr(),
+                      v_first=vf.data_ptr() if mix else None, ldvf=G * V, lambda_=lam.data_ptr() if mix else None, v_out=v.data_ptr() if mix else None, T=T, heads=H, kv_heads=G, K=K, V=V,
+                      act_dtype=S.act_code(BF), temp_coef=0.2, temp_every=64)
+    assert n % 4 == 0
+    S.check(S.lib().b2l_seq_qkv_prep(C.byref(a), S.stream_ptr()), "operands")
+    pos = torch.arange(pos0, pos0 + T, device=DEV).double()
+    ang = pos[:, None] * freq.double()
+    temp = 1 + 0.2 * torch.log(torch.floor((pos + 1) / 64) + 1)
+    for got, at, m, c in ((q, 0, H, "q"), (k, o_k, G, "k")):
+        r = x[:, at:at + m * K].double()
+        if c in norms:
+            r = r / torch.sqrt((r * r).mean(-1, keepdim=True) + 1e-6) * w[c].double()
+        r = r.view(T, m, K)
+        u, z, co, si = r[..., :K // 2], r[..., K // 2:], ang.cos()[:, None] * 1.1, ang.sin()[:, None] * 1.1
+        want = torch.cat([u * co - z * si, z * co + u * si], -1).view(T, m * K) * (temp[:, None] if c == "q" else 1.0)
+        err, top = (got[:T].double() - want).abs(), float(want.abs().max())
+        assert bool((err <= 1e-5 * top + (2.0 ** -8 * want.abs() if c == "k" else 0)).all()) and bool((got[T] == 7).all())
+    if mix:
+        want = (1 - lam.double()) * x[:, o_v:o_v + G * V].double() + lam.double() * vf.double()
+        assert bool(((v.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+
+
 @pytest.mark.parametrize("T,H,K,V,want", [(2048, 4, 128, 128, "chunks"), (2048, 8, 64, 64, "chunks"), (300, 1, 128, 16, "walk"), (2048, 16, 128, 128, "walk"), (257, 64, 128, 64, "walk"),
                                           (47, 2, 64, 32, "steps"), (48, 2, 64, 32, "walk"), (63, 64, 64, 64, "steps"), (64, 64, 64, 64, "walk")])
 def test_scan_plan_and_its_neighbours(T, H, K, V, want):
