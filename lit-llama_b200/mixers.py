@@ -35,8 +35,8 @@ constants are constructor parameters.
     share_weights        the same mixer over the same weights with a state of its own (a layer that runs again)
 
 A mixer is built from a dict of weight tensors (`from_weights`) and runs one portion of one sequence:
-`forward(h, ctx)` with h [T, width] in the model's activation dtype.  Products go through torch (cuBLAS), as the
-dense linears of the package's LLaMA do; everything else is a kernel of libb200seq.  What a mixer carries between
+`forward(h, ctx)` with h [T, width] in the model's activation dtype.  Products in bf16, and small ones in f32, go
+through torch (cuBLAS), as the dense linears of the package's LLaMA do; everything else is a kernel of libb200seq.  What a mixer carries between
 tokens is declared by `state_specs()` and lives in a `SequenceStatePool`.  CUDA only; no CPU fallback."""
 import copy
 import ctypes as C
