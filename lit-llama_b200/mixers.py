@@ -111,6 +111,12 @@ FEW_TOKENS = 4          # up to this many tokens a mechanism may run its product
 LINEAR_F32_FROM = 1 << 18
 
 
+def _tf32_products() -> bool:
+    """Whether the program lets f32 products run in TF32.  `allow_tf32` raises once a program has used both of torch's interfaces to this setting;
+    `fp32_precision` is what either of them has set."""
+    return torch.backends.cuda.matmul.fp32_precision == "tf32"
+
+
 def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether b2l_seq_linear_f32 takes x W^T: plain f32 matrices with 16-byte aligned rows, and a caller who asked for full f32 products without autograd."""
     return (x.shape[0] * w.shape[0] >= LINEAR_F32_FROM and x.dim() == 2 and w.dim() == 2 and x.is_cuda and w.device == x.device and w.dtype == torch.float32
@@ -118,7 +124,7 @@ def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
             and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter)
             and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
-            and not torch.is_autocast_enabled() and not torch.backends.cuda.matmul.allow_tf32)
+            and not torch.is_autocast_enabled() and not _tf32_products())
 
 
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:

@@ -1,0 +1,21 @@
+"""CPU: the rules that pick a form for a call, and what they take into account besides sizes."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def in_a_process_of_its_own(code):
+    """Settings of torch that cannot be taken back stay out of the other tests."""
+    done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("setting,tf32", [
+    ("m.fp32_precision = 'tf32'", True), ("m.allow_tf32 = True", True), ("torch.backends.fp32_precision = 'tf32'", True), ("m.allow_tf32 = True; m.fp32_precision = 'ieee'", False)])
+def test_tf32_is_read_through_either_interface(setting, tf32):
+    """The rule for f32 products reads the precision however a program has set it; torch's older getter raises after some of these."""
+    in_a_process_of_its_own(f"import torch; from lit_llama_b200 import mixers; m = torch.backends.cuda.matmul\n{setting}\nassert mixers._tf32_products() is {tf32}")
