@@ -117,12 +117,17 @@ def _tf32_products() -> bool:
     return torch.backends.cuda.matmul.fp32_precision == "tf32"
 
 
+def _f32_sizes(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Sizes and layouts b2l_seq_linear_f32 takes: f32 matrices with 16-byte aligned rows; an empty sum is the library's, and so are more rows than the
+    grid has tiles of 16 for."""
+    return (x.shape[0] * w.shape[0] >= LINEAR_F32_FROM and x.dim() == 2 and w.dim() == 2 and w.dtype == torch.float32 and 0 < x.shape[1] == w.shape[1]
+            and x.shape[0] <= 16 * 65535 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0
+            and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether b2l_seq_linear_f32 takes x W^T: plain f32 matrices with 16-byte aligned rows, and a caller who asked for full f32 products without autograd."""
-    return (x.shape[0] * w.shape[0] >= LINEAR_F32_FROM and x.dim() == 2 and w.dim() == 2 and x.is_cuda and w.device == x.device and w.dtype == torch.float32
-            and x.shape[1] == w.shape[1] and x.shape[1] % 8 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0
-            and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter)
+    """Whether b2l_seq_linear_f32 takes x W^T: plain tensors, and a caller who asked for full f32 products without autograd."""
+    return (x.is_cuda and w.device == x.device and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and _f32_sizes(x, w)
             and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
             and not torch.is_autocast_enabled() and not _tf32_products())
 

@@ -19,3 +19,14 @@ def in_a_process_of_its_own(code):
 def test_tf32_is_read_through_either_interface(setting, tf32):
     """The rule for f32 products reads the precision however a program has set it; torch's older getter raises after some of these."""
     in_a_process_of_its_own(f"import torch; from lit_llama_b200 import mixers; m = torch.backends.cuda.matmul\n{setting}\nassert mixers._tf32_products() is {tf32}")
+
+
+def test_f32_products_of_no_entries_or_too_many_rows_stay_with_the_library():
+    """Products that the tensor-core kernel refuses: a sum over nothing is zeros, and rows past its grid (16 * 65535) are products like others."""
+    import torch
+    from lit_llama_b200 import mixers
+
+    w, rows = torch.empty(1024, 8), 16 * 65535
+    assert mixers._f32_sizes(torch.empty(1024, 8), w) and mixers._f32_sizes(torch.empty(rows, 8), w)
+    assert not mixers._f32_sizes(torch.empty(1024, 0), torch.empty(1024, 0)) and not mixers._f32_sizes(torch.empty(rows + 1, 8), w)
+    assert not mixers._f32_sizes(torch.empty(1024, 16), w)
