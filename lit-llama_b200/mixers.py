@@ -45,6 +45,8 @@ from typing import Dict, List, Optional, Tuple
 
 import torch
 import torch.nn.functional as F
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _seqlib as S
 from .state import StateSpec
@@ -125,9 +127,17 @@ def _f32_sizes(x: torch.Tensor, w: torch.Tensor) -> bool:
             and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def _followed() -> bool:
+    """Whether something follows torch's calls that a launch past them would not reach: forward-mode derivatives, a tracer or compiler, a function
+    transform, a mode that a program has entered (the default device is one as well, and does not count)."""
+    return (torch.autograd.forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()
+            or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() > 0
+            or torch._C._len_torch_function_stack() > 0 and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack()))
+
+
 def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether b2l_seq_linear_f32 takes x W^T: plain tensors, and a caller who asked for full f32 products without autograd."""
-    return (x.is_cuda and w.device == x.device and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and _f32_sizes(x, w)
+    """Whether b2l_seq_linear_f32 takes x W^T: plain tensors, and a caller who asked for full f32 products without derivatives."""
+    return (x.is_cuda and w.device == x.device and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and not _followed() and _f32_sizes(x, w)
             and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
             and not torch.is_autocast_enabled() and not _tf32_products())
 

@@ -30,3 +30,28 @@ def test_f32_products_of_no_entries_or_too_many_rows_stay_with_the_library():
     assert mixers._f32_sizes(torch.empty(1024, 8), w) and mixers._f32_sizes(torch.empty(rows, 8), w)
     assert not mixers._f32_sizes(torch.empty(1024, 0), torch.empty(1024, 0)) and not mixers._f32_sizes(torch.empty(rows + 1, 8), w)
     assert not mixers._f32_sizes(torch.empty(1024, 16), w)
+
+
+def test_calls_that_torch_follows_stay_with_torch():
+    """Forward-mode derivatives, function transforms, tracing and modes see a product only where it is torch's; a default device does not count."""
+    import torch
+    from lit_llama_b200 import mixers
+    from torch.utils.flop_counter import FlopCounterMode
+
+    x, seen = torch.zeros(2, 2), []
+
+    def look(t):
+        seen.append(mixers._followed())
+        return t + 1
+
+    look(x)
+    with torch.device("cpu"):
+        look(x)
+    assert seen == [False, False]
+    with torch.autograd.forward_ad.dual_level():
+        look(x)
+    torch.vmap(look)(x)
+    torch.jit.trace(look, x, check_trace=False)
+    with FlopCounterMode(display=False):
+        look(x)
+    assert seen[2:] and all(seen[2:])
