@@ -112,20 +112,21 @@ class Engine:
         if isinstance(entry, int):
             if entry < self.portion_graph_after:
                 self._portions[key] = entry + 1
-                while len(self._portions) > 16 * self.portion_graphs:       # counts of lengths long past
-                    self._portions.popitem(last=False)
+                counts = [k for k, e in self._portions.items() if isinstance(e, int)]
+                for k in counts[:max(0, len(counts) - 16 * self.portion_graphs)]:       # of lengths long past
+                    del self._portions[k]
                 return None
             kept = [k for k, e in self._portions.items() if not isinstance(e, int)]
-            torch.cuda.synchronize(self.device)              # also: a graph that goes has run
-            for k in kept[:max(0, len(kept) + 1 - self.portion_graphs)]:
-                del self._portions[k]
-            if self._portion_pool is None:
+            torch.cuda.synchronize(self.device)              # a graph that goes has run
+            if not kept:                                     # a pool that no graph uses is not taken up again, for all that still lies in it
                 self._portion_pool = torch.cuda.graph_pool_handle()
             static_tok, static_want = tok.to(self.device), want.to(self.device)
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, pool=self._portion_pool):
                 logits = m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want)
             entry = (g, static_tok, static_want, logits)
+            for k in kept[:max(0, len(kept) + 1 - self.portion_graphs)]:       # only now: the pool has been in use throughout
+                del self._portions[k]
         else:
             entry[1].copy_(tok)
             entry[2].copy_(want)

@@ -4,6 +4,7 @@ token-by-token decoding and portions of many sizes, interleaved requests, reused
 decoding, greedy generation through the engine's scheduler."""
 import ctypes as C
 import math
+import os
 
 import pytest
 import torch
@@ -607,3 +608,30 @@ def test_portions_of_a_recurring_length_are_replayed(keep):
         assert all(torch.equal(a.pool.tensors[k], b.pool.tensors[k]) for k in b.pool.tensors)
     graphs = [e for e in a._portions.values() if not isinstance(e, int)]
     assert len(graphs) == min(keep, 3) and not b._portions
+
+
+@pytest.mark.parametrize("keep,lengths", [(1, [(17, 3)] * 2 + [(33, 3)] * 2), (2, [(17, 3)] + [(100 + i, 1) for i in range(40)] + [(17, 3), (33, 3)])])
+def test_recording_where_no_graph_is_left(keep, lengths):
+    """A recording after the graphs of its memory pool have gone, or are about to, and more lengths than are counted: in a process where nothing has been
+    recorded before."""
+    import subprocess
+    import sys
+
+    code = f"""
+import sys
+sys.path.insert(0, {os.path.dirname(os.path.abspath(__file__))!r})
+import torch, test_gpu_lugovik as L
+from lit_llama_b200 import Engine
+a, _ = L.build(L.cfg_b(), torch.bfloat16, n_slots=2)
+b = Engine(a.model, n_slots=2)
+a.portion_graphs, b.portion_graph_after = {keep}, 0
+toks, recorded = L.tokens_for(L.cfg_b(), 200, seed=3), 0
+for n, times in {lengths!r}:
+    for _ in range(times):
+        one, two = (e.step([{{"id": "r", "tokens": toks[:n], "want": [n - 1]}}], end=["r"])[0] for e in (a, b))
+        assert torch.equal(one, two)
+        recorded = max(recorded, sum(not isinstance(e, int) for e in a._portions.values()))
+assert 0 < recorded <= {keep}
+"""
+    done = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
