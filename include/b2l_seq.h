@@ -224,6 +224,9 @@ int b2l_seq_cast_f32(const void* in, int ldin, float* out, int ldout, int T, int
 /* Zero one slot of a state tensor laid out [n_slots][slot_bytes]. */
 int b2l_seq_zero_slot(void* state, size_t slot_bytes, int slot, b2l_stream_t stream);
 
+/* A stream of the current device that nothing else uses (torch hands out 32 in turn): what a graph is recorded on. */
+int b2l_seq_stream_create(void** stream);
+
 /* ---- two sublayers on the same input ----
  * x[r] += y1[r] + y2[r] (act, either may be null; the sum is f32), then up to two RMS norms of the new row with weights
  * stored around w_offset: h[r] = x[r] / sqrt(mean(x[r]^2) + eps) * (w_offset + w).  w2 / h2 may be null, and so may

@@ -162,6 +162,7 @@ _SIGS = {
     "b2l_seq_block_attention": (c_int, [C.POINTER(AttnArgs), c_void_p]),
     "b2l_seq_block_attention_work_floats": (C.c_longlong, [C.POINTER(AttnArgs)]),
     "b2l_seq_cast_f32": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
+    "b2l_seq_stream_create": (c_int, [C.POINTER(c_void_p)]),
     "b2l_seq_zero_slot": (c_int, [c_void_p, c_size_t, c_int, c_void_p]),
     "b2l_seq_add_norm2": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_float, c_void_p, c_int,
                                   c_int, c_int, c_void_p]),

@@ -36,3 +36,11 @@ extern "C" int b2l_seq_zero_slot(void* state, size_t slot_bytes, int slot, b2l_s
   B2L_CUDA(cudaMemsetAsync(static_cast<char*>(state) + (size_t)slot * slot_bytes, 0, slot_bytes, (cudaStream_t)stream));
   return 0;
 }
+
+extern "C" int b2l_seq_stream_create(void** stream) {
+  B2L_CHECK_ARG(stream != nullptr, "b2l_seq_stream_create: null pointer");
+  cudaStream_t s = nullptr;
+  B2L_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  *stream = s;
+  return 0;
+}

@@ -20,6 +20,7 @@ from typing import Dict, Hashable, List, Optional, Sequence
 
 import torch
 
+from . import replay
 from .mixers import StepContext
 from .state import PoolFull, SequenceStatePool
 
@@ -61,6 +62,7 @@ class Engine:
         self._single_calls = 0
         self._portions: "OrderedDict[tuple, object]" = OrderedDict()      # (T, places) -> eager portions so far, or (graph, tokens, places, logits)
         self._portion_pool = None
+        self._stream: Optional[torch.cuda.Stream] = None                  # what this engine's graphs are recorded on
         self.steps = 0
 
     # ------------------------------------------------------------------ one portion of one request
@@ -121,9 +123,7 @@ class Engine:
             if not kept:                                     # a pool that no graph uses is not taken up again, for all that still lies in it
                 self._portion_pool = torch.cuda.graph_pool_handle()
             static_tok, static_want = tok.to(self.device), want.to(self.device)
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, pool=self._portion_pool):
-                logits = m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want)
+            g, logits = self._record(self._portion_pool, lambda: m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want))
             entry = (g, static_tok, static_want, logits)
             for k in kept[:max(0, len(kept) + 1 - self.portion_graphs)]:       # only now: the pool has been in use throughout
                 del self._portions[k]
@@ -134,6 +134,11 @@ class Engine:
         entry[0].replay()
         return entry[3].clone()
 
+    def _record(self, pool, body):
+        if self._stream is None:
+            self._stream = replay.recording_stream(self, self.device)
+        return replay.record(self._stream, pool, body)
+
     def _single_token(self) -> torch.Tensor:
         if self._graph is not None:
             self._graph.replay()
@@ -141,12 +146,9 @@ class Engine:
         self._single_calls += 1
         if self._single_calls > self.graph_after:
             torch.cuda.synchronize(self.device)
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                ctx = StepContext(1, self._meta, self.pool.tensors, self.model.dtype)    # inside: it records the capturing stream
-                self._graph_out = self.model.forward_portion(self._tok1, ctx, self._want0)
-            self._graph = g
-            g.replay()            # capture does not run the kernels: this replay is the step itself
+            self._graph, self._graph_out = self._record(None, lambda: self.model.forward_portion(
+                self._tok1, StepContext(1, self._meta, self.pool.tensors, self.model.dtype), self._want0))
+            self._graph.replay()            # capture does not run the kernels: this replay is the step itself
             return self._graph_out.clone()
         ctx = StepContext(1, self._meta, self.pool.tensors, self.model.dtype)
         return self.model.forward_portion(self._tok1, ctx, self._want0)

@@ -635,3 +635,32 @@ assert 0 < recorded <= {keep}
 """
     done = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+def test_engines_on_two_streams_share_no_recording_stream():
+    """Two engines that one thread drives on two streams replay at the same time: each has recorded on a stream (so with a workspace of the library) of its
+    own, and both give the bits of an engine that never records.  An engine that is gone leaves its stream to the next."""
+    import gc
+
+    from lit_llama_b200 import Engine, replay
+
+    cfg = cfg_b()
+    a, _ = build(cfg, torch.bfloat16, n_slots=2)
+    b, still = Engine(a.model, n_slots=2), Engine(a.model, n_slots=2)
+    still.graph_after = still.portion_graph_after = 0
+    toks, streams = tokens_for(cfg, 400, seed=5), [torch.cuda.Stream(), torch.cuda.Stream()]
+    want = [still.step([{"id": "r", "tokens": toks[33 * i: 33 * i + 33], "want": [32]}, {"id": "r", "tokens": [toks[i]], "want": [0]}]) for i in range(10)]
+    torch.cuda.synchronize()
+    got = {0: [], 1: []}
+    for i in range(10):
+        for n, e in enumerate((a, b)):
+            with torch.cuda.stream(streams[n]):
+                got[n].append(e.step([{"id": "r", "tokens": toks[33 * i: 33 * i + 33], "want": [32]}, {"id": "r", "tokens": [toks[i]], "want": [0]}]))
+    torch.cuda.synchronize()
+    for n in got:
+        assert all(torch.equal(x, y) for g, w in zip(got[n], want) for x, y in zip(g, w))
+    own = {a._stream.cuda_stream, b._stream.cuda_stream}
+    assert len(own) == 2 and a._portions and a._graph is not None and not own & {at for free in replay._free.values() for at in free}
+    del a, b, e
+    gc.collect()
+    assert own <= {at for free in replay._free.values() for at in free}
