@@ -41,8 +41,9 @@ class Request:
 class Engine:
     #: replay single-token steps as a CUDA graph after this many eager ones (0 = never)
     graph_after: int = 2
-    #: the same for portions: after this many eager ones of a length and a number of wanted places (0 = never); at most `portion_graphs` lengths are
-    #: kept, the least recently used goes first.  They share one memory pool, as large as the largest portion's temporaries.
+    #: the same for portions: after this many eager ones of a length and a number of wanted places (0 = never); at most `portion_graphs` of them have a
+    #: graph at a time, and one gives way only to another that comes much more often (replay.Sightings).  They share one memory pool, as large as the
+    #: largest portion's temporaries.
     portion_graph_after: int = 2
     portion_graphs: int = 4
 
@@ -60,7 +61,8 @@ class Engine:
         self._graph = None
         self._graph_out: Optional[torch.Tensor] = None
         self._single_calls = 0
-        self._portions: "OrderedDict[tuple, object]" = OrderedDict()      # (T, places) -> eager portions so far, or (graph, tokens, places, logits)
+        self._portions: Dict[tuple, tuple] = {}                           # (T, places) -> (graph, tokens, places, logits)
+        self._sightings = replay.Sightings()
         self._portion_pool = None
         self._stream: Optional[torch.cuda.Stream] = None                  # what this engine's graphs are recorded on
         self.steps = 0
@@ -110,27 +112,22 @@ class Engine:
                 or torch.cuda.is_current_stream_capturing()):
             return None
         key = (T, want.numel())
-        entry = self._portions.pop(key, 0)
-        if isinstance(entry, int):
-            if entry < self.portion_graph_after:
-                self._portions[key] = entry + 1
-                counts = [k for k, e in self._portions.items() if isinstance(e, int)]
-                for k in counts[:max(0, len(counts) - 16 * self.portion_graphs)]:       # of lengths long past
-                    del self._portions[k]
+        entry = self._portions.get(key)
+        record, goes = self._sightings.worth(key, self._portions, self.portion_graph_after, self.portion_graphs)
+        if entry is None:
+            if not record:
                 return None
-            kept = [k for k, e in self._portions.items() if not isinstance(e, int)]
-            torch.cuda.synchronize(self.device)              # a graph that goes has run
-            if not kept:                                     # a pool that no graph uses is not taken up again, for all that still lies in it
+            if not self._portions:                           # a pool that no graph uses is not taken up again, for all that still lies in it
                 self._portion_pool = torch.cuda.graph_pool_handle()
             static_tok, static_want = tok.to(self.device), want.to(self.device)
             g, logits = self._record(self._portion_pool, lambda: m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want))
-            entry = (g, static_tok, static_want, logits)
-            for k in kept[:max(0, len(kept) + 1 - self.portion_graphs)]:       # only now: the pool has been in use throughout
-                del self._portions[k]
+            entry = self._portions[key] = (g, static_tok, static_want, logits)
+            if goes is not None:                             # only now: the pool has been in use throughout
+                torch.cuda.synchronize(self.device)          # and the graph has run
+                del self._portions[goes]
         else:
             entry[1].copy_(tok)
             entry[2].copy_(want)
-        self._portions[key] = entry                          # the most recently used last
         entry[0].replay()
         return entry[3].clone()
 

@@ -1,8 +1,8 @@
-"""Steps recorded as CUDA graphs: the stream they are recorded on, and the recording."""
+"""Steps recorded as CUDA graphs: the stream they are recorded on, the recording, and which portions are worth one."""
 import ctypes as C
 import threading
 import weakref
-from typing import Callable, Dict, List, Tuple
+from typing import Callable, Collection, Dict, Hashable, List, Optional, Tuple
 
 import torch
 
@@ -47,3 +47,29 @@ def record(stream: torch.cuda.Stream, pool, body: Callable[[], torch.Tensor]) ->
         finally:
             g.capture_end()
     return g, out
+
+
+class Sightings:
+    """How often portions of a kind have come lately, and from that which are recorded.  A recording takes 0.5 ms more than its portion run eagerly and
+    saves 0.4 ms whenever it is replayed (four layers of width 1024; both grow with the layers).  While there is room a kind is recorded once it has
+    come `after` times; then only one that comes more than twice as often as the rarest that has a graph, and LEAD times more: lengths that take turns
+    keep the graphs they have, and a recording is spread over more than LEAD portions.  Counts outlive the graphs and are halved every HALF portions."""
+
+    HALF, LEAD = 256, 32
+
+    def __init__(self) -> None:
+        self.counts: Dict[Hashable, int] = {}
+        self.total = 0
+
+    def worth(self, key: Hashable, kept: Collection[Hashable], after: int, room: int) -> Tuple[bool, Optional[Hashable]]:
+        """One more portion of kind `key`, while those of `kept` have graphs: whether it is recorded now, and the graph that goes for it."""
+        self.total += 1
+        if self.total % self.HALF == 0:
+            self.counts = {k: n // 2 for k, n in self.counts.items() if n > 1}
+        n = self.counts[key] = self.counts.get(key, 0) + 1
+        if key in kept or n <= after or room <= 0:
+            return False, None
+        if len(kept) < room:
+            return True, None
+        rarest = min(kept, key=lambda k: self.counts.get(k, 0))
+        return n > 2 * self.counts.get(rarest, 0) + self.LEAD, rarest

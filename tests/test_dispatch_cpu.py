@@ -55,3 +55,80 @@ def test_calls_that_torch_follows_stay_with_torch():
     with FlopCounterMode(display=False):
         look(x)
     assert seen[2:] and all(seen[2:])
+
+
+# ---------------------------------------------------------------------------- the engine's recorded portions, with the graph and the device stubbed
+class _Model:
+    vocab, dtype, portion_graph_safe, capture_layers = 8, None, True, None
+
+    def __init__(self):
+        import torch
+
+        self.dtype, self.device, self.eager = torch.float32, torch.device("cpu"), 0
+        self.weight = torch.ones(2)
+
+    def state_specs(self):
+        return {}
+
+    def forward_portion(self, tokens, ctx, want=None):
+        import torch
+
+        self.eager += 1
+        return torch.full((0 if want is None else want.numel(), self.vocab), float(tokens.sum()) * float(self.weight[0]))
+
+
+class _Graph:
+    def __init__(self, body, log):
+        self.body, self.log, self.out = body, log, body()
+        log.append("recorded")
+
+    def replay(self):
+        self.log.append("replayed")
+        self.out.copy_(self.body())
+
+
+@pytest.fixture
+def stubbed(monkeypatch):
+    import torch
+    from lit_llama_b200 import Engine
+
+    log = []
+
+    def record(self, pool, body):
+        g = _Graph(body, log)
+        return g, g.out
+
+    monkeypatch.setattr(Engine, "_record", record)
+    for name, value in (("is_current_stream_capturing", False), ("synchronize", None), ("graph_pool_handle", (0, 1))):
+        monkeypatch.setattr(torch.cuda, name, lambda *a, value=value, **k: value)
+    return Engine(_Model(), n_slots=1, device="cpu"), log
+
+
+def _feed(engine, T):
+    out = engine.step([{"id": "r", "tokens": [1] * T, "want": [T - 1]}], end=["r"])[0]
+    assert float(out[0, 0]) == T * float(engine.model.weight[0])
+
+
+@pytest.mark.parametrize("lengths,random,recordings,replays", [(4, False, 4, 2980), (8, False, 4, 1480), (20, False, 4, 560), (50, False, 4, 200), (50, True, 6, 150)])
+def test_mixed_lengths_are_not_recorded_again_and_again(stubbed, lengths, random, recordings, replays):
+    """3000 portions of lengths in rotation or at random: a few recordings, and every portion of a length that has one is a replay."""
+    import random as R
+
+    engine, log = stubbed
+    rng = R.Random(1)
+    for i in range(3000):
+        _feed(engine, 2 + (rng.randrange(lengths) if random else i % lengths))
+    assert log.count("recorded") <= recordings and log.count("replayed") >= replays and len(engine._sightings.counts) <= 512
+
+
+def test_a_length_that_comes_much_more_often_takes_a_graph_over(stubbed):
+    """Four lengths with graphs, then one other alone: it has a graph within 200 portions, and the least frequent of the four has none."""
+    engine, log = stubbed
+    for i in range(100):
+        _feed(engine, 2 + i % 4 if i % 5 else 2)
+    assert log.count("recorded") == 4
+    for _ in range(200):
+        _feed(engine, 9)
+    assert log.count("recorded") == 5 and (9, 1) in engine._portions and len(engine._portions) == 4
+    engine.portion_graphs = 0
+    _feed(engine, 11)

@@ -591,7 +591,7 @@ def test_llama_is_served_by_the_same_engine():
 @pytest.mark.parametrize("keep", [1, 4])
 def test_portions_of_a_recurring_length_are_replayed(keep):
     """Two lengths and numbers of places in turn, at starts and in slots that change: recorded after two eager portions each, and logits and states are the
-    same bits as an engine's that never records; with room for one graph each new length drops the other."""
+    same bits as an engine's that never records; with room for one graph the first kind keeps it, since none comes much more often."""
     from lit_llama_b200 import Engine
 
     cfg = cfg_b()
