@@ -65,6 +65,7 @@ class Engine:
         self._sightings = replay.Sightings()
         self._portion_pool = None
         self._stream: Optional[torch.cuda.Stream] = None                  # what this engine's graphs are recorded on
+        self._failed_recordings = 0
         self.steps = 0
 
     # ------------------------------------------------------------------ one portion of one request
@@ -120,8 +121,10 @@ class Engine:
             if not self._portions:                           # a pool that no graph uses is not taken up again, for all that still lies in it
                 self._portion_pool = torch.cuda.graph_pool_handle()
             static_tok, static_want = tok.to(self.device), want.to(self.device)
-            g, logits = self._record(self._portion_pool, lambda: m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want))
-            entry = self._portions[key] = (g, static_tok, static_want, logits)
+            made = self._record(self._portion_pool, lambda: m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want))
+            if made is None:
+                return None
+            entry = self._portions[key] = (made[0], static_tok, static_want, made[1])
             if goes is not None:                             # only now: the pool has been in use throughout
                 torch.cuda.synchronize(self.device)          # and the graph has run
                 del self._portions[goes]
@@ -132,20 +135,29 @@ class Engine:
         return entry[3].clone()
 
     def _record(self, pool, body):
+        """(graph, result), or None where the recording failed (memory ran out, a call that cannot be recorded): the step runs eagerly then, and reports what is
+        wrong with it by itself.  After three failures nothing is recorded any more."""
+        if self._failed_recordings >= 3:
+            return None
         if self._stream is None:
             self._stream = replay.recording_stream(self, self.device)
-        return replay.record(self._stream, pool, body)
+        try:
+            return replay.record(self._stream, pool, body)
+        except RuntimeError:
+            self._failed_recordings += 1
+            return None
 
     def _single_token(self) -> torch.Tensor:
+        if self._graph is None:
+            self._single_calls += 1
+            if self._single_calls > self.graph_after and self._failed_recordings < 3:
+                torch.cuda.synchronize(self.device)
+                made = self._record(None, lambda: self.model.forward_portion(
+                    self._tok1, StepContext(1, self._meta, self.pool.tensors, self.model.dtype), self._want0))
+                if made is not None:
+                    self._graph, self._graph_out = made
         if self._graph is not None:
-            self._graph.replay()
-            return self._graph_out.clone()
-        self._single_calls += 1
-        if self._single_calls > self.graph_after:
-            torch.cuda.synchronize(self.device)
-            self._graph, self._graph_out = self._record(None, lambda: self.model.forward_portion(
-                self._tok1, StepContext(1, self._meta, self.pool.tensors, self.model.dtype), self._want0))
-            self._graph.replay()            # capture does not run the kernels: this replay is the step itself
+            self._graph.replay()            # capture does not run the kernels: the first replay is the step itself
             return self._graph_out.clone()
         ctx = StepContext(1, self._meta, self.pool.tensors, self.model.dtype)
         return self.model.forward_portion(self._tok1, ctx, self._want0)

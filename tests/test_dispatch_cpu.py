@@ -90,15 +90,22 @@ class _Graph:
 @pytest.fixture
 def stubbed(monkeypatch):
     import torch
-    from lit_llama_b200 import Engine
+    from lit_llama_b200 import Engine, replay
 
-    log = []
+    class Log(list):
+        pass
 
-    def record(self, pool, body):
+    log = Log()
+
+    def record(stream, pool, body):
+        log.fails = getattr(log, "fails", 0) - 1
+        if log.fails >= 0:
+            raise RuntimeError("out of memory")
         g = _Graph(body, log)
         return g, g.out
 
-    monkeypatch.setattr(Engine, "_record", record)
+    monkeypatch.setattr(replay, "record", record)
+    monkeypatch.setattr(replay, "recording_stream", lambda *a: None)
     for name, value in (("is_current_stream_capturing", False), ("synchronize", None), ("graph_pool_handle", (0, 1))):
         monkeypatch.setattr(torch.cuda, name, lambda *a, value=value, **k: value)
     return Engine(_Model(), n_slots=1, device="cpu"), log
@@ -132,3 +139,15 @@ def test_a_length_that_comes_much_more_often_takes_a_graph_over(stubbed):
     assert log.count("recorded") == 5 and (9, 1) in engine._portions and len(engine._portions) == 4
     engine.portion_graphs = 0
     _feed(engine, 11)
+
+
+@pytest.mark.parametrize("T", [1, 7])
+@pytest.mark.parametrize("fails", [1, 3])
+def test_a_step_that_cannot_be_recorded_runs_eagerly(stubbed, T, fails):
+    """A recording that fails leaves the eager step in its place, is tried again, and after three times no more."""
+    engine, log = stubbed
+    log.fails = fails
+    for _ in range(12):
+        _feed(engine, T)
+    assert log.count("recorded") == (1 if fails == 1 else 0) and engine._failed_recordings == fails
+    assert log.count("replayed") == (9 if fails == 1 else 0)
