@@ -112,7 +112,7 @@ class Engine:
         if (not getattr(m, "portion_graph_safe", False) or self.portion_graph_after <= 0 or T > self.prefill_chunk or getattr(m, "capture_layers", None) is not None
                 or torch.cuda.is_current_stream_capturing()):
             return None
-        key = (T, want.numel())
+        key = (T, want.numel(), *replay.settings())          # under other settings: recorded again, or refused as the model refuses it
         entry = self._portions.get(key)
         record, goes = self._sightings.worth(key, self._portions, self.portion_graph_after, self.portion_graphs)
         if entry is None:

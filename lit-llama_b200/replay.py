@@ -49,6 +49,13 @@ def record(stream: torch.cuda.Stream, pool, body: Callable[[], torch.Tensor]) ->
     return g, out
 
 
+def settings() -> tuple:
+    """What torch's products look at besides their operands: a recording has the forms that were chosen under the settings of its time."""
+    m = torch.backends.cuda.matmul
+    return (m.fp32_precision == "tf32", m.allow_bf16_reduced_precision_reduction, m.allow_fp16_accumulation, torch.backends.cuda.preferred_blas_library(),
+            torch.are_deterministic_algorithms_enabled(), torch.is_autocast_enabled("cuda"))
+
+
 class Sightings:
     """How often portions of a kind have come lately, and from that which are recorded.  A recording takes 0.5 ms more than its portion run eagerly and
     saves 0.4 ms whenever it is replayed (four layers of width 1024; both grow with the layers).  While there is room a kind is recorded once it has

@@ -106,6 +106,7 @@ def stubbed(monkeypatch):
 
     monkeypatch.setattr(replay, "record", record)
     monkeypatch.setattr(replay, "recording_stream", lambda *a: None)
+    monkeypatch.setattr(torch.backends.cuda, "preferred_blas_library", lambda: 0)      # asks the driver
     for name, value in (("is_current_stream_capturing", False), ("synchronize", None), ("graph_pool_handle", (0, 1))):
         monkeypatch.setattr(torch.cuda, name, lambda *a, value=value, **k: value)
     return Engine(_Model(), n_slots=1, device="cpu"), log
@@ -136,7 +137,7 @@ def test_a_length_that_comes_much_more_often_takes_a_graph_over(stubbed):
     assert log.count("recorded") == 4
     for _ in range(200):
         _feed(engine, 9)
-    assert log.count("recorded") == 5 and (9, 1) in engine._portions and len(engine._portions) == 4
+    assert log.count("recorded") == 5 and (9, 1) in {k[:2] for k in engine._portions} and len(engine._portions) == 4
     engine.portion_graphs = 0
     _feed(engine, 11)
 
@@ -151,3 +152,30 @@ def test_a_step_that_cannot_be_recorded_runs_eagerly(stubbed, T, fails):
         _feed(engine, T)
     assert log.count("recorded") == (1 if fails == 1 else 0) and engine._failed_recordings == fails
     assert log.count("replayed") == (9 if fails == 1 else 0)
+
+
+def test_portions_under_other_settings_are_not_replayed(stubbed, monkeypatch):
+    """A model that refuses TF32 refuses it where its portion has a graph as well, and has the graph again when the setting is taken back."""
+    import torch
+
+    engine, log = stubbed
+    run, m = type(engine.model).forward_portion, torch.backends.cuda.matmul
+
+    def refusing(self, *a):
+        if torch.backends.cuda.matmul.allow_tf32:
+            raise RuntimeError("TF32")
+        return run(self, *a)
+
+    monkeypatch.setattr(_Model, "forward_portion", refusing)
+    for _ in range(5):
+        _feed(engine, 7)
+    m.allow_tf32 = True
+    try:
+        with pytest.raises(RuntimeError, match="TF32"):
+            _feed(engine, 7)
+    finally:
+        m.allow_tf32 = False
+    before = log.count("replayed")
+    engine.step([], end=["r"])
+    _feed(engine, 7)
+    assert before == 3 and log.count("replayed") == 4 and log.count("recorded") == 1
