@@ -63,6 +63,7 @@ class Engine:
         self._single_calls = 0
         self._portions: Dict[tuple, tuple] = {}                           # (T, places) -> (graph, tokens, places, logits)
         self._sightings = replay.Sightings()
+        self._held: Optional[replay.Held] = None                          # what the graphs of _portions have taken from the model
         self._portion_pool = None
         self._stream: Optional[torch.cuda.Stream] = None                  # what this engine's graphs are recorded on
         self._failed_recordings = 0
@@ -115,17 +116,23 @@ class Engine:
         key = (T, want.numel(), *replay.settings())          # under other settings: recorded again, or refused as the model refuses it
         entry = self._portions.get(key)
         record, goes = self._sightings.worth(key, self._portions, self.portion_graph_after, self.portion_graphs)
+        if (entry is not None or record) and self._portions and not self._held.unchanged():      # other weights than the graphs have
+            torch.cuda.synchronize(self.device)              # a graph that goes has run
+            self._portions.clear()
+            self._graph, self._sightings = None, replay.Sightings()
+            return None
         if entry is None:
             if not record:
                 return None
             if not self._portions:                           # a pool that no graph uses is not taken up again, for all that still lies in it
                 self._portion_pool = torch.cuda.graph_pool_handle()
+                self._held = replay.Held(m, self.pool.tensors)
             static_tok, static_want = tok.to(self.device), want.to(self.device)
             made = self._record(self._portion_pool, lambda: m.forward_portion(static_tok, StepContext(T, self._meta, self.pool.tensors, m.dtype), static_want))
             if made is None:
                 return None
             entry = self._portions[key] = (made[0], static_tok, static_want, made[1])
-            if goes is not None:                             # only now: the pool has been in use throughout
+            if goes in self._portions:                       # only now: the pool has been in use throughout
                 torch.cuda.synchronize(self.device)          # and the graph has run
                 del self._portions[goes]
         else:

@@ -64,7 +64,7 @@ class _Model:
     def __init__(self):
         import torch
 
-        self.dtype, self.device, self.eager = torch.float32, torch.device("cpu"), 0
+        self.dtype, self.device = torch.float32, torch.device("cpu")
         self.weight = torch.ones(2)
 
     def state_specs(self):
@@ -73,7 +73,6 @@ class _Model:
     def forward_portion(self, tokens, ctx, want=None):
         import torch
 
-        self.eager += 1
         return torch.full((0 if want is None else want.numel(), self.vocab), float(tokens.sum()) * float(self.weight[0]))
 
 
@@ -179,3 +178,28 @@ def test_portions_under_other_settings_are_not_replayed(stubbed, monkeypatch):
     engine.step([], end=["r"])
     _feed(engine, 7)
     assert before == 3 and log.count("replayed") == 4 and log.count("recorded") == 1
+
+
+@pytest.mark.parametrize("change", ["m.weight = torch.full((2,), 3.0)", "m.weight.data = torch.full((2,), 3.0)", "m.layers[0].scale = 3.0", "m.layers[0] = m.Layer(3.0)",
+                                    "m.layers[0].table['b'] = (torch.full((2,), 3.0),)", "m.layers.append(m.Layer(1.0))"])
+def test_portions_with_other_weights_are_recorded_again(stubbed, change):
+    """Tensors and values that a program has put in the place of those the model had, at any depth: the next portion has them, and recording begins anew.  New contents
+    of the same tensor are no reason for one."""
+    import torch
+
+    class Layer:
+        def __init__(self, scale):
+            self.scale, self.table = scale, {"b": (torch.ones(2),)}
+
+    engine, log = stubbed
+    m = engine.model
+    m.Layer, m.layers = Layer, [Layer(1.0)]
+    for _ in range(5):
+        _feed(engine, 7)
+    m.weight.fill_(2.0)
+    _feed(engine, 7)
+    assert log.count("recorded") == 1 and log.count("replayed") == 4
+    exec(change)
+    for _ in range(5):
+        _feed(engine, 7)
+    assert log.count("recorded") == 2 and log.count("replayed") == 6
