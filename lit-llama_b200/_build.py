@@ -19,8 +19,9 @@ LIBRARIES = {
     "llama": dict(out=os.path.join(PKG, "libb200llama.so"),
                   sources=["api.cu", "q_generic.cu", "elementwise.cu", "attention.cu", "q4_tc.cu", "q4_gemv.cu", "q4_gemv_batch.cu",
                            "q8_gemv.cu", "q8_gemm.cu", "sampling.cu", "decode_mega.cu", "q4_gemm.cu", "tp_allreduce.cu"]),
-    # the quantized linears' entry points as Python functions (a CPython extension, host code only)
-    "pycall": dict(out=os.path.join(PKG, "_pycall.so"), sources=["pycall.cpp"]),
+    # the quantized linears' entry points as Python functions (a CPython extension, host code only; the stable ABI of 3.10 on, so one file for every
+    # interpreter).  The package runs without it, see _lib.py
+    "pycall": dict(out=os.path.join(PKG, "_pycall.abi3.so"), sources=["pycall.cpp"], headers=[os.path.join(ROOT, "include", "b2l.h")]),
     # sequence-mixer kernels: recurrences, local and latent attention, expert routing, f32 residual streams (include/b2l_seq.h)
     "seq": dict(out=os.path.join(PKG, "libb200seq.so"),
                 sources=["seq_api.cu", "seq_elementwise.cu", "seq_scan.cu", "seq_attention.cu", "seq_latent.cu", "seq_moe.cu", "seq_streams.cu",
@@ -39,24 +40,34 @@ def nvcc_path() -> str:
     return "nvcc"
 
 
-def _headers():
+def _headers(spec=None):
+    if spec is not None and "headers" in spec:
+        return spec["headers"]
     inc = os.path.join(ROOT, "include")
     return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + \
            [os.path.join(inc, f) for f in os.listdir(inc)]
 
 
-def compile_unit(src: str, force: bool = False, obj_dir: str = OBJ_DIR) -> str:
+def compile_unit(src: str, force: bool = False, obj_dir: str = OBJ_DIR, spec=None) -> str:
     """csrc/<src> -> <obj_dir>/<name>.o (skipped when newer than the source and every header)."""
     os.makedirs(obj_dir, exist_ok=True)
     obj = os.path.join(obj_dir, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
     if not force and os.path.exists(obj):
         t = os.path.getmtime(obj)
-        if all(os.path.getmtime(d) <= t for d in [path] + _headers()):
+        if all(os.path.getmtime(d) <= t for d in [path] + _headers(spec)):
             return obj
-    cmd = [nvcc_path()] + NVCC_FLAGS + (["-I" + sysconfig.get_paths()["include"]] if src.endswith(".cpp") else []) + ["-c", path, "-o", obj]
+    fd, tmp = tempfile.mkstemp(dir=obj_dir, prefix=".compile-", suffix=".o")
+    os.close(fd)
+    flags = ["-I" + sysconfig.get_paths()["include"], "-DPy_LIMITED_API=0x030A0000"] if src.endswith(".cpp") else []
+    cmd = [nvcc_path()] + NVCC_FLAGS + flags + ["-c", path, "-o", tmp]
     print("[build]", " ".join(cmd), file=sys.stderr)
-    subprocess.run(cmd, check=True, stdout=sys.stderr)
+    try:
+        subprocess.run(cmd, check=True, stdout=sys.stderr)
+        os.replace(tmp, obj)   # processes that build at the same time never link a half-written object
+    finally:
+        if os.path.exists(tmp):
+            os.unlink(tmp)
     return obj
 
 
@@ -81,7 +92,7 @@ def build_library(name: str, force: bool = False) -> str:
 
     spec = LIBRARIES[name]
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        objs = list(ex.map(lambda s: compile_unit(s, force), spec["sources"]))
+        objs = list(ex.map(lambda s: compile_unit(s, force, spec=spec), spec["sources"]))
     link(objs, spec["out"])
     return spec["out"]
 
@@ -91,7 +102,7 @@ def is_stale(name: str) -> bool:
     if not os.path.exists(spec["out"]):
         return True
     t = os.path.getmtime(spec["out"])
-    return any(os.path.getmtime(p) > t for p in [os.path.join(CSRC, s) for s in spec["sources"]] + _headers())
+    return any(os.path.getmtime(p) > t for p in [os.path.join(CSRC, s) for s in spec["sources"]] + _headers(spec))
 
 
 def ensure(name: str) -> str:

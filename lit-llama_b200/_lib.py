@@ -137,21 +137,38 @@ def lib():
     return _lib
 
 
-#: q4 / q8 of csrc/pycall.cpp, set with the library
+#: q4 / q8 of csrc/pycall.cpp or, where that is not built or does not load, of _Foreign; set with the library
 pycall = None
 Q4_GEMV, Q4_GEMV_BATCH, Q4_LINEAR_TC, Q4_GEMM = range(4)
 
 
+class _Foreign:
+    """What csrc/pycall.cpp does, through ctypes: 3 us more a call."""
+
+    def __init__(self, handle) -> None:
+        self._q4 = (handle.b2l_q4_gemv, handle.b2l_q4_gemv_batch, handle.b2l_q4_linear_tc, handle.b2l_q4_gemm)
+        self.q8 = handle.b2l_q8_linear
+
+    def q4(self, which, x, ldx, qw_tiled, scales, zeros, sz_dtype, y, ldy, M, N, K, workspace, stream) -> int:
+        return self._q4[which](C.byref(Q4LinearArgs(x=x, ldx=ldx, qw_tiled=qw_tiled, scales=scales, zeros=zeros, sz_dtype=sz_dtype, y=y, ldy=ldy, M=M, N=N, K=K,
+                                                    workspace=workspace)), stream)
+
+
 def _bind(handle) -> None:
+    """The extension is loaded as it lies there, like the library itself, and never built here: everything but the time of a call is the same without it."""
     global pycall
     import importlib.machinery
     import importlib.util
 
     from . import _build
 
-    spec = importlib.util.spec_from_loader("_pycall", importlib.machinery.ExtensionFileLoader("_pycall", _build.ensure("pycall")))
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
+    try:
+        spec = importlib.util.spec_from_loader("_pycall", importlib.machinery.ExtensionFileLoader("_pycall", _build.LIBRARIES["pycall"]["out"]))
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except ImportError:
+        pycall = _Foreign(handle)
+        return
     module.bind(*(C.cast(getattr(handle, n), c_void_p).value for n in ("b2l_q4_gemv", "b2l_q4_gemv_batch", "b2l_q4_linear_tc", "b2l_q4_gemm", "b2l_q8_linear")))
     pycall = module
 

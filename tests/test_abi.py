@@ -69,3 +69,23 @@ def test_errors_are_reported_not_swallowed(L):
     comm.rank, comm.world, comm.max_elems = 3, 2, 4096
     assert lib.b2l_tp_allreduce(C.byref(comm), C.c_void_p(16), C.c_void_p(16), 4096, 0, None) == -1
     assert b"bad rank" in lib.b2l_last_error()
+
+
+def test_the_extension_is_optional_and_never_built_by_a_call(L, monkeypatch):
+    """Without csrc/pycall.cpp's file the same functions are called through ctypes, with the same answers; no compiler runs for it, however new the headers."""
+    from lit_llama_b200 import _build
+
+    handle, built = L.lib(), L.pycall
+    calls = [("q4", (which, None, 64, None, None, None, 0, None, 1, 1, 1, 64, None, 0)) for which in range(4)] + [("q8", (None, 64, None, None, None, 1, None, 2, 1, 64, 6.0, 0))]
+    answers = [getattr(built, n)(*a) for n, a in calls]
+    assert all(a != 0 for a in answers)
+    monkeypatch.setenv("NVCC", "/nonexistent/nvcc")
+    monkeypatch.setitem(_build.LIBRARIES["pycall"], "out", "/nonexistent/_pycall.abi3.so")
+    try:
+        L._bind(handle)
+        assert isinstance(L.pycall, L._Foreign) and [getattr(L.pycall, n)(*a) for n, a in calls] == answers
+    finally:
+        monkeypatch.undo()
+        L._bind(handle)
+    assert type(L.pycall) is type(built)
+    assert _build._headers(_build.LIBRARIES["pycall"]) == [HEADER] and _build.LIBRARIES["pycall"]["out"].endswith(".abi3.so")
