@@ -108,9 +108,14 @@ def share_weights(mixer, name: str):
 FEW_TOKENS = 4          # up to this many tokens a mechanism may run its products in its own kernels, without the library
 
 
-#: rows x outputs from which an f32 product runs on the tensor cores: below, too few tiles for the SMs and the library is as fast
-#: (us here / library: 64 x 1024 -> 1024 32 / 31, 64 x 1024 -> 2560 33 / 34, 256 x 1024 -> 1024 32 / 34, 128 x 1024 -> 2560 33 / 45, 64 x 2048 -> 5120 49 / 75)
-LINEAR_F32_FROM = 1 << 18
+#: Where an f32 product runs on the tensor cores: below these the tiles are too few for the SMs, or too short for what a tile costs beside its sums, and the
+#: library is as fast or faster.  Device time in us, here / library, over 1024..131072 outputs; from the line on none measured is slower here:
+#:   rows x outputs    128 x 1024 x 1024 (k) 31 / 31, 256 x 1024 x 1024 31 / 31, 512 x 1024 x 1024 31 / 35, 777 x 2560 x 1024 43 / 90
+#:   and times k       256 x 1024 x 512 20.5 / 19.4, 512 x 1024 x 512 20.5 / 22.5, 64 x 8192 x 384 18 / 20
+#:   rows              2 x 131072 x 2048 277 / 203, 4 x 131072 x 1024 160 / 175 (with larger errors: up to 8 rows the library adds more finely), 9 rows 162 / 205,
+#:                     9 x 32000 x 4096 164 / 219; with k below 384, 32 x 131072 x 256 77 / 72, 48 rows 80 / 106
+#:   k                 64: 16 x 32000 18 / 12, 777 x 32000 117 / 104; 128: 32 x 32000 21 / 16, 777 x 2560 16 / 20; 256: 777 x 8192 55 / 80
+LINEAR_F32_FROM, LINEAR_F32_WORK, LINEAR_F32_ROWS, LINEAR_F32_K = 1 << 18, 3 << 26, 9, 256
 
 
 def _tf32_products() -> bool:
@@ -120,11 +125,16 @@ def _tf32_products() -> bool:
 
 
 def _f32_sizes(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Sizes and layouts b2l_seq_linear_f32 takes: f32 matrices with 16-byte aligned rows; an empty sum is the library's, and so are more rows than the
-    grid has tiles of 16 for."""
-    return (x.shape[0] * w.shape[0] >= LINEAR_F32_FROM and x.dim() == 2 and w.dim() == 2 and w.dtype == torch.float32 and 0 < x.shape[1] == w.shape[1]
-            and x.shape[0] <= 16 * 65535 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0
-            and x.stride(0) >= x.shape[1] and w.stride(0) >= w.shape[1] and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    """Sizes and layouts that b2l_seq_linear_f32 is used for: f32 matrices with 16-byte aligned rows; more rows than the grid has tiles of 16 for are the
+    library's."""
+    if x.dim() != 2 or w.dim() != 2 or w.dtype is not torch.float32:
+        return False
+    (rows, k), (n, kw) = x.shape, w.shape
+    if (k != kw or k % 8 != 0 or k < LINEAR_F32_K or rows < (LINEAR_F32_ROWS if k >= 384 else 48) or rows * n < LINEAR_F32_FROM or rows * n * k < LINEAR_F32_WORK
+            or rows > 16 * 65535):
+        return False
+    (ldx, step_x), (ldw, step_w) = x.stride(), w.stride()
+    return (step_x == 1 and step_w == 1 and ldx % 4 == 0 and ldw % 4 == 0 and ldx >= k and ldw >= k and x.storage_offset() % 4 == 0 and w.storage_offset() % 4 == 0)
 
 
 def _followed() -> bool:
@@ -137,9 +147,9 @@ def _followed() -> bool:
 
 def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether b2l_seq_linear_f32 takes x W^T: plain tensors, and a caller who asked for full f32 products without derivatives."""
-    return (x.is_cuda and w.device == x.device and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and not _followed() and _f32_sizes(x, w)
+    return (_f32_sizes(x, w) and x.is_cuda and w.device == x.device and type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and not _followed()
             and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
-            and not torch.is_autocast_enabled() and not _tf32_products())
+            and not torch.is_autocast_enabled() and not _tf32_products() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:

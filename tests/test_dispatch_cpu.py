@@ -26,10 +26,34 @@ def test_f32_products_of_no_entries_or_too_many_rows_stay_with_the_library():
     import torch
     from lit_llama_b200 import mixers
 
-    w, rows = torch.empty(1024, 8), 16 * 65535
-    assert mixers._f32_sizes(torch.empty(1024, 8), w) and mixers._f32_sizes(torch.empty(rows, 8), w)
-    assert not mixers._f32_sizes(torch.empty(1024, 0), torch.empty(1024, 0)) and not mixers._f32_sizes(torch.empty(rows + 1, 8), w)
-    assert not mixers._f32_sizes(torch.empty(1024, 16), w)
+    w, rows = torch.empty(64, 256), 16 * 65535
+    assert mixers._f32_sizes(torch.empty(rows, 256), w) and not mixers._f32_sizes(torch.empty(rows + 1, 256), w)
+    assert not mixers._f32_sizes(torch.empty(1024, 0), torch.empty(1024, 0))
+
+
+@pytest.mark.parametrize("rows,outputs,k,taken", [
+    (256, 1024, 1024, True), (255, 1024, 1024, False), (9, 32000, 1024, True), (8, 65536, 1024, False), (256, 1024, 768, True), (256, 1024, 760, False),
+    (384, 1024, 512, True), (9, 65536, 384, True), (9, 65536, 376, False), (48, 32000, 256, True), (47, 32000, 256, False), (4096, 4096, 248, False)])
+def test_f32_products_on_both_sides_of_the_line(rows, outputs, k, taken):
+    """Rows, k, results and products from which the tensor-core form is the faster one."""
+    import torch
+    from lit_llama_b200 import mixers
+
+    assert mixers._f32_sizes(torch.empty(rows, k), torch.empty(outputs, k)) is taken
+
+
+@pytest.mark.parametrize("x,w,taken", [
+    ("wide[:, :1024]", "w", True), ("wide[:, 4:1028]", "w", True), ("wide[:, 2:1026]", "w", False), ("wide[:, :1020]", "w[:, :1020]", False),
+    ("wide[:, :1024]", "w.t()", False), ("wide.t()[:300, :1024]", "w", False), ("odd[:, :1024]", "w", False), ("wide[:, :1024]", "odd[:, :1024]", False),
+    ("wide[:1, :1024].expand(300, 1024)", "w", False), ("wide[:, :1024].double()", "w.double()", False), ("wide[:, :1024]", "w.bfloat16()", False), ("wide[0, :1024]", "w", False),
+    ("wide[None, :, :1024]", "w", False), ("wide[:, :512]", "w", False)])
+def test_f32_products_by_layout(x, w, taken):
+    """Column slices on 16-byte boundaries are taken; other offsets, k not in groups of 8, transposed, repeated, broadcast and narrower operands are not."""
+    import torch
+    from lit_llama_b200 import mixers
+
+    names = {"wide": torch.empty(1200, 1200), "w": torch.empty(1024, 1024), "odd": torch.empty(1024, 1029)}
+    assert mixers._f32_sizes(eval(x, names), eval(w, names)) is taken
 
 
 def test_calls_that_torch_follows_stay_with_torch():

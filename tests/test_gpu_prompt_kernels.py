@@ -543,3 +543,32 @@ def test_decays_of_eight_channels(size, mode):
     if not mode:
         fin = sp.isfinite() & (sp > 1e-35)
         assert float(((dt.double() - sp).abs() / sp)[fin].max()) < 4e-7 and float(dt[0, 0]) == math.inf and float(dt[1, 1]) == 0.0
+
+
+@pytest.mark.parametrize("M,N,K,own", [(300, 1024, 1024, True), (9, 32000, 1024, True), (8, 65536, 1024, False), (255, 1024, 1024, False), (600, 1024, 512, True)])
+def test_f32_linear_takes_the_form_its_rule_says(M, N, K, own):
+    """Through the entry point of the mixers: sizes on both sides of the line, and callers whom only the library's product serves (derivatives, TF32, rows off a
+    16-byte boundary).  Which one ran shows in the bits.  f32 sums of K products: 4 sqrt(K) 2^-24 of the norm."""
+    from lit_llama_b200 import _seqlib as S
+    from lit_llama_b200 import mixers
+
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    wide, w = torch.randn(M, K + 12, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV) * K ** -0.5
+    x, library = wide[:, 4:K + 4], torch.nn.functional.linear
+    y, here = mixers.linear(x, w), torch.empty(M, N, device=DEV)
+    S.check(S.lib().b2l_seq_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), K, here.data_ptr(), N, M, N, K, S.stream_ptr()), "b2l_seq_linear_f32")
+    assert torch.equal(y, here if own else library(x, w)) and not torch.equal(here, library(x, w))
+    assert rel(y, x.double() @ w.double().t()) < 4 * K ** 0.5 * 2.0 ** -24
+    off = wide[:, 3:K + 3]
+    assert torch.equal(mixers.linear(off, w), library(off, w))
+    wg = w.clone().requires_grad_()
+    mixers.linear(x, wg).sum().backward()
+    assert wg.grad is not None
+    with torch.autograd.forward_ad.dual_level():
+        out = mixers.linear(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)), w)
+        assert torch.autograd.forward_ad.unpack_dual(out).tangent is not None
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        assert torch.equal(mixers.linear(x, w), library(x, w))
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = False
