@@ -136,7 +136,8 @@ __global__ void seq_scale_kernel(float* __restrict__ z, size_t n, float mult) {
 
 constexpr int MOST_PAIRS = 4096;      // rotated pairs whose cos and sin fit the 48 KB of a launch without an attribute
 
-// Attention operands of one token from the stacked projection row, one CTA per token.
+// Attention operands of one token from the stacked projection row, one CTA per token.  `quads`: four neighbouring pairs per thread with 8-byte loads, where
+// whole heads turn and a row has one factor (40960 entries with norms, us with them and a pair of two bytes at a time: one token 41 / 115, 2048 tokens 153 / 351).
 //   q_out (f32) and k_out (act): RMS norm (whole_row: over all heads*K entries with a weight of that size; else per
 //   head with a weight of K entries shared by the heads; no weight: no norm), then rotation of the first rot_dims
 //   entries of every head (entry i with entry i + rot_dims/2) by the angle (pos0 + t) * freq[i]; unit_rms (no weights): the
@@ -145,7 +146,7 @@ constexpr int MOST_PAIRS = 4096;      // rotated pairs whose cos and sin fit the
 //   q_out is multiplied by the query temperature of its position when temp_every > 0.
 //   v_out (act): (1 - lambda) v + lambda v_first when v_first is given (lambda read on the device), else not written.
 template <typename act_t, bool TABLE>      // TABLE: up to MOST_PAIRS pairs
-__global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args a) {
+__global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args a, int quads) {
   __shared__ float red[32];
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const act_t* row = (const act_t*)a.proj + (size_t)t * a.ld;
@@ -168,12 +169,57 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
     float r_row = 1.f;
     if (w && a.whole_row) {
       float ss = 0.f;
-      for (int i = threadIdx.x; i < heads * K; i += blockDim.x) {
-        const float v = ld_act(x, i);
-        ss += v * v;
+      if (quads && sizeof(act_t) == 2) {
+        for (int i = threadIdx.x * 4; i < heads * K; i += blockDim.x * 4) {
+          const uint2 u = *reinterpret_cast<const uint2*>(x + i);
+          const float v0 = __uint_as_float(u.x << 16), v1 = __uint_as_float(u.x & 0xffff0000u), v2 = __uint_as_float(u.y << 16), v3 = __uint_as_float(u.y & 0xffff0000u);
+          ss += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
+        }
+      } else {
+        for (int i = threadIdx.x; i < heads * K; i += blockDim.x) {
+          const float v = ld_act(x, i);
+          ss += v * v;
+        }
       }
       ss = block_sum(ss, red);
       r_row = 1.0f / sqrtf(ss / (float)(heads * K) + a.eps);
+    }
+    if (quads && sizeof(act_t) == 2) {
+      // one factor for the whole row: four neighbouring pairs per thread, 8-byte loads (a lane per pair with 2-byte loads took 27 us for 2048 tokens of 16 + 4 heads, so 17)
+      const int per = half / 4;
+      for (int u = threadIdx.x; u < heads * per; u += blockDim.x) {
+        const int hd = u / per, i = (u - hd * per) * 4;
+        const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(x) + (size_t)hd * K + i;
+        const __nv_bfloat16* pw = reinterpret_cast<const __nv_bfloat16*>(w) + (size_t)hd * K + i;
+        const uint2 a0 = *reinterpret_cast<const uint2*>(p), a1 = *reinterpret_cast<const uint2*>(p + half);
+        const uint2 w0 = w ? *reinterpret_cast<const uint2*>(pw) : make_uint2(0x3f803f80u, 0x3f803f80u);
+        const uint2 w1 = w ? *reinterpret_cast<const uint2*>(pw + half) : make_uint2(0x3f803f80u, 0x3f803f80u);
+        const uint32_t ua[4] = {a0.x, a0.y, a1.x, a1.y}, uw[4] = {w0.x, w0.y, w1.x, w1.y};
+        float lo[4], hi[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = e >> 1;
+          const float xu = __uint_as_float(e & 1 ? ua[j] & 0xffff0000u : ua[j] << 16), wu = __uint_as_float(e & 1 ? uw[j] & 0xffff0000u : uw[j] << 16);
+          const float xv = __uint_as_float(e & 1 ? ua[2 + j] & 0xffff0000u : ua[2 + j] << 16), wv = __uint_as_float(e & 1 ? uw[2 + j] & 0xffff0000u : uw[2 + j] << 16);
+          const float pu = xu * r_row * wu, pv = xv * r_row * wv, c = turn[i + e], s = turn[half + i + e];
+          lo[e] = pu * c - pv * s;
+          hi[e] = pv * c + pu * s;
+        }
+        if (which == 0) {
+          float* qo = a.q_out + ((size_t)t * heads + hd) * K + i;
+          *reinterpret_cast<float4*>(qo) = make_float4(lo[0] * temp, lo[1] * temp, lo[2] * temp, lo[3] * temp);
+          *reinterpret_cast<float4*>(qo + half) = make_float4(hi[0] * temp, hi[1] * temp, hi[2] * temp, hi[3] * temp);
+        } else {
+          __nv_bfloat16* ko = (__nv_bfloat16*)a.k_out + ((size_t)t * heads + hd) * K + i;
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const float (&y)[4] = b ? hi : lo;
+            const __nv_bfloat162 y0 = __floats2bfloat162_rn(y[0], y[1]), y1 = __floats2bfloat162_rn(y[2], y[3]);
+            *reinterpret_cast<uint2*>(ko + b * half) = make_uint2(*reinterpret_cast<const uint32_t*>(&y0), *reinterpret_cast<const uint32_t*>(&y1));
+          }
+        }
+      }
+      continue;
     }
     for (int hd = warp; hd < heads; hd += nw) {
       const act_t* p = x + (size_t)hd * K;
@@ -443,7 +489,11 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   const int quads = table && a->act_dtype == B2L_BF16 && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
                     a->k_off % 4 == 0 && a->ld % 4 == 0 && al8(a->proj) && al8(a->q_norm) && al8(a->k_norm) && al16(a->q_out) && al8(a->k_out);
   const long long units = (long long)(a->heads + a->kv_heads) * (a->K / 8);
-  if (quads && units <= 8 * QUAD_THREADS) {
+  // Rows of more than 32768 entries do not fit a CTA's registers.  From 16384 on they take eight units a thread, at 128 registers with spills: faster where
+  // few CTAs wait for one another's loads (us, registers / a pass per row: 17408 entries with norms, 1 token 12 / 23, 256 18 / 23, 2048 82 / 68; without, 16
+  // tokens 10 / 14, 256 17 / 16, 2048 65 / 47; 32768 with norms, 2048 tokens 114 / 122).
+  const bool norms = a->q_norm || a->k_norm, held = units <= 4 * QUAD_THREADS || (units <= 8 * QUAD_THREADS && (a->T <= sm_count() * (norms ? 2 : 1) || (norms && units >= 7 * QUAD_THREADS)));
+  if (quads && held) {
     // tokens per CTA: up to four where two CTAs per SM are left (the angles of a CTA come at once, its tokens' x one ahead), as far as their angles fit
     const int fill = a->T / (2 * sm_count()), tokens = a->K > 2048 ? 1 : fill < 1 ? 1 : fill > 4 ? 4 : fill;
     const int nu = units <= QUAD_THREADS / 2 ? 1 : units <= QUAD_THREADS ? 2 : units <= 4 * QUAD_THREADS ? 4 : 8;
@@ -454,8 +504,8 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
     return 0;
   }
   B2L_SEQ_DISPATCH(a->act_dtype, {
-    if (table) seq_qkv_prep_kernel<act_t, true><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a);
-    else seq_qkv_prep_kernel<act_t, false><<<a->T, 256, 0, (cudaStream_t)stream>>>(*a);
+    if (table) seq_qkv_prep_kernel<act_t, true><<<a->T, 256, sizeof(float) * a->rot_dims, (cudaStream_t)stream>>>(*a, quads);
+    else seq_qkv_prep_kernel<act_t, false><<<a->T, 256, 0, (cudaStream_t)stream>>>(*a, quads);
   });
   B2L_LAUNCH_CHECK("seq_qkv_prep_kernel");
   return 0;

@@ -255,9 +255,9 @@ def test_attention_operands_of_very_wide_heads(rot):
 
 
 @pytest.mark.parametrize("T,H,G,K,norms,mix", [(1, 16, 4, 128, "qk", True), (1187, 2, 1, 16, "qk", False), (700, 16, 4, 128, "", True), (900, 3, 2, 24, "k", True), (5, 130, 6, 128, "qk", False),
-                                               (9, 40, 8, 128, "q", True)])
+                                               (9, 40, 8, 128, "q", True), (3, 300, 20, 128, "qk", True), (300, 130, 6, 128, "k", False), (150, 126, 4, 128, "", True), (4, 256, 10, 128, "", False)])
 def test_attention_operands_by_quads_of_pairs(T, H, G, K, norms, mix):
-    """One to eight units per thread, one to four tokens per CTA with a remainder, either row's norm, the query temperature, mixed values.  Angles up to 40 are good to
+    """One to eight units per thread, one to four tokens per CTA with a remainder, rows too long for that, either row's norm, the query temperature, mixed values.  Angles up to 40 are good to
     40 * 2^-24, products and sums add a few 2^-24: 1e-5 of the largest entry; k and v are rounded to bf16 on top (2^-9 of an entry)."""
     from lit_llama_b200 import _seqlib as S
 
