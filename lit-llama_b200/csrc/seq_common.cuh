@@ -13,19 +13,21 @@ template <typename T> __device__ __forceinline__ void st_act(T* p, size_t i, flo
 template <> __device__ __forceinline__ void st_act<__nv_bfloat16>(__nv_bfloat16* p, size_t i, float v) { p[i] = __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ void st_act<float>(float* p, size_t i, float v) { p[i] = v; }
 
-// x / y for y >= 1 (also +inf) without a branch: the approximate reciprocal and Markstein's steps (one Newton step for 1/y, then the quotient
-// corrected by its own remainder), within one rounding of the exact quotient.  The division operator's range test makes every use a branch of its own,
-// some 130 cycles that nothing overlaps: four gated outputs took 730 cycles, now 190.
+// x / y for y >= 1/4 without a branch: the approximate reciprocal (at most 1 ulp off, as documented), one Newton step, and the quotient corrected by its own
+// remainder (Markstein).  While 1/y is a normal number, so for y up to 2^126, that is the correctly rounded quotient, subnormal ones as well: 2 in 10^8 are 1
+// ulp off, over all mantissas of y and reciprocals off by up to 1 ulp.  Four gated outputs in a row took the attention kernel 730 cycles with the
+// division operator, 190 so.
 __device__ __forceinline__ float over_f(float x, float y) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   r = fmaf(r, fmaf(-y, r, 1.0f), r);
   const float q = x * r, d = fmaf(fmaf(-y, q, x), r, q);
-  if (y > 0x1p120f) return x * 0.0f;                  // 1/y below what keeps the remainder exact, or zero
+  if (y == INFINITY) return x * 0.0f;
   return fabsf(q) < INFINITY ? d : q;                 // an infinite quotient has no remainder
 }
-__device__ __forceinline__ float sigmoid_f(float z) { return over_f(1.0f, 1.0f + expf(-z)); }
-__device__ __forceinline__ float silu_f(float z) { return over_f(z, 1.0f + expf(-z)); }
+// a quarter of both sides of the fraction: 1 + e^-z up to the largest f32 then has a normal reciprocal (down to z = -88.7), and no rounding changes
+__device__ __forceinline__ float sigmoid_f(float z) { return over_f(0.25f, fmaf(expf(-z), 0.25f, 0.25f)); }
+__device__ __forceinline__ float silu_f(float z) { return over_f(0.25f * z, fmaf(expf(-z), 0.25f, 0.25f)); }
 // log(1 + e^z) = max(z, 0) + log(1 + u), u = e^-|z| <= 1, and log(1 + u) = 2 atanh(s), s = u / (2 + u) <= 1/3, by atanh's series to s^15 (the next term is
 // below 2e-9 of the sum): no branch and some 20 operations, where log1pf(expf(z)) took twice as many.
 __device__ __forceinline__ float softplus_f(float z) {

@@ -442,6 +442,20 @@ def test_gates_are_within_rounding_of_float64(act):
     assert float(y[-4]) == 0.0 if act == "sigmoid" else math.isnan(float(y[-4]))
 
 
+@pytest.mark.parametrize("act", ["sigmoid", "silu"])
+def test_small_gates_are_not_lost(act):
+    """Down to where 1 + e^-x leaves f32 (x = -88.72) a gate keeps its value: the bound above while the result is normal, and one subnormal step (2^-149) more
+    below."""
+    from lit_llama_b200 import _seqlib as S
+
+    x = torch.linspace(-88.7, -40, 20001, device=DEV)
+    y = torch.empty_like(x)
+    S.check(S.lib().b2l_seq_unary_act(x.data_ptr(), x.numel(), y.data_ptr(), x.numel(), 1, x.numel(), S.ACT_SIGMOID if act == "sigmoid" else S.ACT_SILU, None,
+                                      S.act_code(torch.float32), S.stream_ptr()), "b2l_seq_unary_act")
+    want = torch.sigmoid(x.double()) * (1 if act == "sigmoid" else x.double())
+    assert bool(((y.double() - want).abs() <= 6 * 2.0 ** -24 * want.abs() + 2.0 ** -149).all())
+
+
 @pytest.mark.parametrize("T,H,G,K,V,pos0,window,block,sink,cap", [
     (64, 8, 2, 128, 128, 0, 512, 512, 0, 0.0), (130, 4, 1, 192, 16, 300, 96, 100, 1, 0.0), (257, 4, 2, 64, 112, 90, 0, 128, 0, 30.0), (200, 8, 8, 16, 64, 1000, 333, 333, 1, 0.0)])
 def test_f32_local_attention_in_three_parts(T, H, G, K, V, pos0, window, block, sink, cap):
