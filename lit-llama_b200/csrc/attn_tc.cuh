@@ -126,13 +126,13 @@ __device__ __forceinline__ void fma2(float& a, float& b, float f, float c, float
       : "+f"(a), "+f"(b) : "f"(f), "f"(c), "f"(d));
 }
 __device__ __forceinline__ float high_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
-// 2^x; what CUDA's expf ends with as well, so as a weight it is no less exact than expf of the score
+// 2^x, documented to 2^-22 of the result and without subnormals: as a weight that leaves out what is below 2^-126 of the largest
 __device__ __forceinline__ float exp2_f(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-constexpr float LOG2E = 1.44269502162933349609375f, LOG2E_LO = 1.925963033500011e-8f, LN2 = 0.693147180559945309f;      // log2(e) in two parts
+constexpr float LOG2E = 1.44269502162933349609375f, LOG2E_LO = 1.925963033500011e-8f, LN2 = 0.693147180559945309f;      // log2(e): the nearest f32 and its remainder
 
 __device__ __forceinline__ void st4_bf16(__nv_bfloat16* p, const float (&y)[4]) {      // 8-byte aligned
   const __nv_bfloat162 u = __floats2bfloat162_rn(y[0], y[1]), v = __floats2bfloat162_rn(y[2], y[3]);

@@ -426,8 +426,8 @@ def test_expanded_latent_attention_with_unaligned_queries():
 
 @pytest.mark.parametrize("act", ["sigmoid", "silu"])
 def test_gates_are_within_rounding_of_float64(act):
-    """Logistic gates in f32 from -120 to 120, infinities and NaN: expf (2 ulp), one addition and a quotient within one rounding, so 4 * 2^-24 relative
-    (negative arguments add expf's argument rounding, none: expf reduces it exactly); results below 2^-100 may be zero."""
+    """Logistic gates in f32 from -120 to 120, infinities and NaN: expf within its documented 2 ulp (4 * 2^-24 of its value), one addition and one quotient
+    (2^-24 each)."""
     from lit_llama_b200 import _seqlib as S
 
     x = torch.cat([torch.linspace(-120, 120, 40001, device=DEV), torch.tensor([math.inf, -math.inf, math.nan, 0.0, -0.0], device=DEV)])
