@@ -82,7 +82,7 @@ class Engine:
         cap = getattr(self.model, "max_positions", 0)          # models that cache every position say how many fit a slot
         if cap and pos0 + T > cap:
             raise PoolFull(f"request {request_id!r} would reach position {pos0 + T}, a slot holds {cap}")
-        self._meta.copy_(torch.tensor([slot, pos0], dtype=torch.int32))
+        self._meta.copy_(torch.tensor([slot, pos0], dtype=torch.int32), non_blocking=True)
         want = [T - 1] if want is None else list(want)
         if any(w < 0 or w >= T for w in want):
             raise IndexError(f"wanted places {want} outside a portion of {T} tokens")
@@ -136,8 +136,8 @@ class Engine:
                 torch.cuda.synchronize(self.device)          # and the graph has run
                 del self._portions[goes]
         else:
-            entry[1].copy_(tok)
-            entry[2].copy_(want)
+            entry[1].copy_(tok, non_blocking=True)           # out of pageable memory, so it is read before the call returns
+            entry[2].copy_(want, non_blocking=True)
         entry[0].replay()
         return entry[3].clone()
 
