@@ -25,8 +25,6 @@
 // cycles: units of 128 k instead of 64, one barrier for both operands and two operations per pair of weights instead of three took 64 tokens from 280 to
 // 200 ns per 64 k (device time of 64 / 512 / 777 x 4096 -> 11008: 23.2 / 50.9 / 74.7 -> 16.8 / 41.9 / 55.7 us).  Where tiles are few a cluster of up to
 // 8 CTAs splits K and adds its f32 sums through distributed shared memory in rank order (the result does not depend on timing).
-#include <atomic>
-
 #include "tc_common.cuh"
 
 namespace b2l {
@@ -333,26 +331,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
 
 constexpr size_t MOST_SMEM = 226 * 1024;
 struct Plan { int bt, m_tiles, splits, nx, nw; size_t smem; };
-// Clusters of sp CTAs, one per SM, that run at once (B200: 148, 74, 45, 33, 26, 22, 15, 15 of 1..8: clusters do not cross the SM groups).
-static int slots(int sp, int sms) {
-  if (sp == 1) return sms;
-  static std::atomic<int> known[9];
-  int n = known[sp].load(std::memory_order_relaxed);
-  if (n == 0) {
-    LaunchCfg lc(dim3((unsigned)sp), dim3(NTHREADS), 120 * 1024, nullptr, false, sp);
-    if (cudaOccupancyMaxActiveClusters(&n, q4_gemm_kernel, &lc.cfg) != cudaSuccess || n <= 0) {
-      (void)cudaGetLastError();
-      n = sms / sp > 0 ? sms / sp : 1;
-    }
-    known[sp].store(n, std::memory_order_relaxed);
-  }
-  return n;
-}
 // Tile height and K split by a model of the time in ns: a CTA's items one after the other, each of so many 64-wide stages (60 + 1.15 per token of the
 // tile, and no less than the 200 that dequantising and issuing take; 18944 features, 64 / 128 / 208 / 256 tokens: 200 / 209 / 286 / 346) and 1000 for
 // each; first copies and the last output once, 4000 and 15 per token.  A split adds 3500 for its barriers and, for every further rank, 12 per token
 // (partial sums to and from shared memory; seen: 32 tokens in four 4500, 112 in four 7000, 208 in two 5000), and every round of it starts anew.
 static Plan plan_for(int M, int N, int K) {
+  static std::atomic<int> known[9];
   const int sms = sm_count(), n_tiles = (N + BN - 1) / BN, n_kt = K / BK;
   Plan best{};
   long long best_cost = -1;
@@ -361,7 +345,7 @@ static Plan plan_for(int M, int N, int K) {
     const int bt = ((M + mt - 1) / mt + 15) / 16 * 16, tiles = (M + bt - 1) / bt;
     for (int sp = 1; sp <= 8; ++sp) {
       if (sp > 1 && n_kt / sp < 8) break;
-      const int at_once = slots(sp, sms);
+      const int at_once = clusters_at_once(q4_gemm_kernel, NTHREADS, sp, sms, known);
       const long long rounds = (n_tiles * tiles + at_once - 1) / at_once, stages = (n_kt + sp - 1) / sp;
       const long long per = 600 + bt * 23 / 2 > 2000 ? 600 + bt * 23 / 2 : 2000, once = 4000 + 15 * bt;
       const long long cost = sp == 1 ? rounds * (stages * per / 10 + 1000) + once : rounds * (stages * per / 10 + once + 3500 + (sp - 1) * 12 * bt);

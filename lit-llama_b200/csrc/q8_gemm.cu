@@ -374,6 +374,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) q8_gemm_kernel(const __grid_const
   if (warp == 1) tmem_dealloc(tmem, cols);
 }
 
+constexpr size_t MOST_SMEM = 201 * 1024;
 struct Plan { int bt, m_tiles, splits, nst; size_t smem; };
 // Tiles of equal height and a split of K over clusters, by a model of the time in ns.  A CTA takes 4400, 210 per stage of 128 k, and per token of its tile
 // 85 for the epilogue's roundings (a rank of a split stores its share) and 1.6 per stage; two CTAs on an SM (tiles of up to 128 tokens) take 1.2 times
@@ -381,14 +382,14 @@ struct Plan { int bt, m_tiles, splits, nst; size_t smem; };
 // tiles and the plan so: 137 x 4096 -> 12288 29 / 21, 300 x 4096 -> 12288 58 / 32, 512 x 4096 -> 11008 88 / 58, 256 x 5120 -> 5120 31 / 22, 1000 x 4096 ->
 // 4096 46 / 34; up to 64 tokens the plans are mostly the same (16 x 4096 -> 11008 13.3).
 static Plan plan_for(int M, int N, int K) {
-  static const int clusters[9] = {0, 148, 74, 0, 33, 0, 0, 0, 15};      // of so many CTAs, one per SM, that run at once on 148 SMs
+  static std::atomic<int> known[9];
   const int sms = sm_count(), n_tiles = (N + BN - 1) / BN, least = (M + 255) / 256;
   Plan q{};
   long long best = -1;
   for (int mt = least; mt <= least + 4; ++mt) {
     const int bt = ((M + mt - 1) / mt + 15) / 16 * 16, tiles = n_tiles * ((M + bt - 1) / bt), two = bt <= 128;
     for (int sp = 1; sp <= 8; sp *= 2) {
-      const int stages = (K / BK + sp - 1) / sp, at_once = clusters[sp] * sms / 148;
+      const int stages = (K / BK + sp - 1) / sp, at_once = clusters_at_once(q8_gemm_kernel, NTHREADS, sp, sms, known);
       if (sp > 1 && (K / BK / sp < 4 || tiles > at_once * (two && sp == 2 ? 2 : 1))) break;      // a split only where its clusters run at once; four and eight alone on their SMs
       const long long one = 4400 + 210 * stages + bt * (85 / sp + 16 * stages / 10), deep = ((long long)tiles * sp + sms - 1) / sms;
       const long long cost = (deep == 1 ? one : two ? one * (deep / 2 * 24 + deep % 2 * 19) / 20 : one * deep) + (sp == 1 ? 0 : (sp == 2 ? 3000 : sp == 4 ? 3900 : 4800) + 3 * bt * sp);
@@ -402,7 +403,7 @@ static Plan plan_for(int M, int N, int K) {
   // Two CTAs per SM for tiles of up to 128 tokens, one's epilogue under the other's loads: half of an SM's 228 KB less the 1 KB the system
   // keeps per CTA, the static arrays and the alignment of the stages.  Wider tiles take one.
   constexpr size_t STATIC = sizeof(__half) * SM_OUT * 256 + sizeof(float) * 256 + 8 * (2 * MAX_STAGES + 4);
-  const size_t budget = q.bt <= 128 ? 114 * 1024 - 1024 - STATIC - 1024 : 200 * 1024;
+  const size_t budget = q.bt <= 128 ? 114 * 1024 - 1024 - STATIC - 1024 : MOST_SMEM - 1024;
   q.nst = (int)(budget / stage);
   if (q.nst > MAX_STAGES) q.nst = MAX_STAGES;
   q.smem = q.nst * stage + 1024;
@@ -444,14 +445,14 @@ extern "C" int b2l_q8_linear(const void* x, int ldx, const void* cb, const void*
   int* n_out = (int*)w;
   q8_mask_kernel<<<(K + 63) / 64, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, M, K, threshold, mask);      // outlier columns are the whole batch's
   B2L_LAUNCH_CHECK("q8_mask_kernel");
+  static DynSmemCache smem_cache;
+  if (int rc = ensure_dyn_smem(q8_gemm_kernel, MOST_SMEM, smem_cache)) return rc;
   for (int at = 0; at < M; at += SLAB) {
     const int rows = M - at < SLAB ? M - at : SLAB;
     const Plan q = plan_for(rows, N, K);
     Params p;
     if (int rc = map_sw128(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cb, N, K, K, BK, BN)) return rc;
     if (int rc = map_sw128(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, rows, K, K, BK, q.bt)) return rc;
-    static DynSmemCache smem_cache;
-    if (int rc = ensure_dyn_smem(q8_gemm_kernel, q.smem, smem_cache)) return rc;
     p.x = (const __nv_bfloat16*)x + (size_t)at * ldx;
     p.y = (__nv_bfloat16*)y + (size_t)at * ldy;
     LaunchCfg lr(dim3((unsigned)rows), dim3(ROW_THREADS), 0, s, true, 1);      // each kernel is launched while the one before it runs, and waits for it where it reads its results

@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda.h>   // CUtensorMap and its enums only: the encoder is fetched with cudaGetDriverEntryPoint (no libcuda link)
 
+#include <atomic>
+
 #include "b2l_common.cuh"
 
 namespace b2l {
@@ -148,6 +150,22 @@ inline int map_sw128(CUtensorMap* m, CUtensorMapDataType type, int esize, const 
     return B2L_E_ARG;
   }
   return 0;
+}
+
+// Clusters of `size` (1..8) CTAs of a kernel, one per SM by 120 KB of shared memory, that run at once (B200: 148, 74, 45, 33, 26, 22, 15, 15: clusters do not
+// cross the SM groups).  Asked of the driver once; the kernel's limit of dynamic shared memory has been raised before.
+template <class Kernel> inline int clusters_at_once(Kernel kernel, int threads, int size, int sms, std::atomic<int> (&known)[9]) {
+  if (size == 1) return sms;
+  int n = known[size].load(std::memory_order_relaxed);
+  if (n == 0) {
+    LaunchCfg lc(dim3((unsigned)size), dim3((unsigned)threads), 120 * 1024, nullptr, false, size);
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc.cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = sms / size > 0 ? sms / size : 1;
+    }
+    known[size].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 }  // namespace tc
