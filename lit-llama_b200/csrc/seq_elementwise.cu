@@ -615,6 +615,7 @@ extern "C" int b2l_seq_conv_silu(const void* in, int ldin, const void* w, const 
 extern "C" int b2l_seq_conv_silu_unit(const void* in, int ldin, const void* w, const void* bias, void* state, const int* meta, float* out, int ldout, int T, int C, int taps,
                                       int q_at, int k_at, int heads, int size, float eps, float q_mult, float k_mult, int act_dtype, b2l_stream_t stream) {
   B2L_CHECK_ARG(heads > 0 && size > 0 && q_at >= 0 && k_at >= 0 && q_at + heads * size <= C && k_at + heads * size <= C, "b2l_seq_conv_silu_unit: heads outside the channels");
+  B2L_CHECK_ARG(q_at + heads * size <= k_at || k_at + heads * size <= q_at, "b2l_seq_conv_silu_unit: the two rows of heads overlap");
   const UnitHeads u{q_at, q_at + heads * size, k_at, k_at + heads * size, size, eps, q_mult, k_mult};
   bool done = false;
   if (int rc = conv_silu(in, ldin, w, bias, state, meta, out, ldout, T, C, taps, act_dtype, &u, &done, stream)) return rc;

@@ -172,3 +172,12 @@ def test_scheduler_portions_turns_slots_and_budget():
     e2.add_request("big", [1] * 20, 1)
     with pytest.raises(PoolFull):
         e2.run()
+
+
+def test_unit_heads_that_overlap_are_refused():
+    """One pass would scale an entry by one of the two factors, two passes by both: neither is asked for."""
+    from lit_llama_b200 import _seqlib as S
+
+    for q_at, k_at in ((0, 0), (64, 0), (0, 127)):
+        assert S.lib().b2l_seq_conv_silu_unit(8, 256, 8, None, 8, 8, 8, 256, 0, 256, 4, q_at, k_at, 2, 64, 1e-6, 1.0, 1.0, S.act_code(torch.bfloat16), None) != 0
+    assert S.lib().b2l_seq_conv_silu_unit(8, 256, 8, None, 8, 8, 8, 256, 0, 256, 4, 128, 0, 2, 64, 1e-6, 1.0, 1.0, S.act_code(torch.bfloat16), None) == 0
