@@ -446,13 +446,16 @@ def rope_frequencies(dims: int, base: float, scaling: Optional[dict]) -> Tuple[t
 
 # ------------------------------------------------------------------------------------------------ attention
 def local_attention(a: "S.AttnArgs", ctx: StepContext) -> None:
-    """b2l_seq_block_attention with the work space its few-query form asks for."""
+    """b2l_seq_block_attention with the work space its forms for few queries and for f32 portions ask for; where no memory is left, the forms that need none."""
     lib = S.lib()
     n = lib.b2l_seq_block_attention_work_floats(C.byref(a))
     work = None
     if n:
-        work = torch.empty((n,), dtype=torch.float32, device=ctx.meta.device)
-        a.work, a.work_floats = _p(work), n
+        try:
+            work = torch.empty((n,), dtype=torch.float32, device=ctx.meta.device)
+            a.work, a.work_floats = _p(work), n
+        except torch.OutOfMemoryError:
+            a.work, a.work_floats = None, 0
     S.check(lib.b2l_seq_block_attention(C.byref(a), ctx.stream), "b2l_seq_block_attention")
 
 

@@ -227,3 +227,23 @@ def test_portions_with_other_weights_are_recorded_again(stubbed, change):
     for _ in range(5):
         _feed(engine, 7)
     assert log.count("recorded") == 2 and log.count("replayed") == 6
+
+
+def test_attention_without_room_runs_the_form_that_needs_none(monkeypatch):
+    """A portion in f32 asks for up to 128 MB it can do without: where that does not fit, the call is made without it."""
+    import types
+
+    import torch
+    from lit_llama_b200 import _seqlib as S
+    from lit_llama_b200 import mixers
+
+    seen = []
+    monkeypatch.setattr(S, "lib", lambda: types.SimpleNamespace(b2l_seq_block_attention_work_floats=lambda a: 1 << 20,
+                                                                b2l_seq_block_attention=lambda a, s: seen.append((a._obj.work, a._obj.work_floats)) or 0))
+
+    def none_left(*a, **k):
+        raise torch.OutOfMemoryError("CUDA out of memory")
+
+    monkeypatch.setattr(torch, "empty", none_left)
+    mixers.local_attention(S.AttnArgs(), types.SimpleNamespace(meta=torch.zeros(2), stream=None))
+    assert seen == [(None, 0)]
