@@ -118,10 +118,15 @@ FEW_TOKENS = 4          # up to this many tokens a mechanism may run its product
 LINEAR_F32_FROM, LINEAR_F32_WORK, LINEAR_F32_ROWS, LINEAR_F32_K = 1 << 18, 3 << 26, 9, 256
 
 
+#: looked up once: a product of the size of the line takes 20 us, and asking through torch's modules took 2 of them
+_precision, _tracing, _transforms = torch._C._get_fp32_precision_getter, torch._C._get_tracing_state, torch._C._functorch.peek_interpreter_stack
+_dispatch_modes, _function_modes, _forward_ad = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack, torch.autograd.forward_ad
+
+
 def _tf32_products() -> bool:
-    """Whether the program lets f32 products run in TF32.  `allow_tf32` raises once a program has used both of torch's interfaces to this setting;
-    `fp32_precision` is what either of them has set."""
-    return torch.backends.cuda.matmul.fp32_precision == "tf32"
+    """Whether the program lets f32 products run in TF32 (torch.backends.cuda.matmul.fp32_precision): what either of torch's interfaces to this setting has
+    set, where `allow_tf32` raises once a program has used both."""
+    return _precision("cuda", "matmul") == "tf32"
 
 
 def _f32_sizes(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -140,9 +145,8 @@ def _f32_sizes(x: torch.Tensor, w: torch.Tensor) -> bool:
 def _followed() -> bool:
     """Whether something follows torch's calls that a launch past them would not reach: forward-mode derivatives, a tracer or compiler, a function
     transform, a mode that a program has entered (the default device is one as well, and does not count)."""
-    return (torch.autograd.forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling()
-            or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() > 0
-            or torch._C._len_torch_function_stack() > 0 and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack()))
+    return (_forward_ad._current_level >= 0 or _tracing() is not None or _transforms() is not None or _dispatch_modes() > 0 or torch.compiler.is_compiling()
+            or _function_modes() > 0 and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack()))
 
 
 def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
