@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(128)
 // tiled TMA copies from the cache (or from qkv without one).
 // ----------------------------------------------------------------------------------
 struct PromptProb {
-  // bf16 outputs, and the mma.sync kernel below adds in its accumulators as well (weights to 2^-17): 2048 tokens 115 us so; 136 against 161 through registers before its present pipeline
+  // bf16 outputs, and the mma.sync kernel below adds in its accumulators as well (weights to 2^-17): 2048 tokens 86 us so; before its present pipeline 136, and 161 through registers
   static constexpr bool REGS = false;
   static constexpr int KP = 1;
   CUtensorMap map_a, map_b, map_v;

@@ -8,7 +8,7 @@
 // Three bf16 MMAs cost 3 / 32 of what the f32 FMAs cost on the CUDA cores (4096 against 128 per cycle).
 //
 // f32 keys and values (KP = 3) are cut into three rounded parts beforehand, and of the nine products the six above 2^-24 are taken: twice the MMAs
-// of bf16 keys; against the f32 FMAs on the CUDA cores 777 tokens of 8 heads, window 512, take 40 us instead of 217, with errors of 2.1e-7 instead of
+// of bf16 keys (entries below 2^-109 keep fewer than 24 bits: the parts have f32's exponents and no more); against the f32 FMAs on the CUDA cores 777 tokens of 8 heads, window 512, take 40 us instead of 217, with errors of 2.1e-7 instead of
 // 3.8e-7 against float64 (between a quarter and two thirds of the FMAs' in all sizes measured).
 //
 //   warp 0       issues the MMAs of the scores S(t) = Q K^T, three tiles ahead at most, warp 13 those of the outputs, P(t) V
@@ -37,7 +37,7 @@
 // What bounds it: a 128 x 64 tile of head size 128 is 24 MMAs of 48 cycles and 12 of 64, 1920 in all; it takes 2400..2700 (2950 with two score
 // regions and one issuing warp, 5250 of softmax and issue in the first form); queries, outputs and the first tile's chain of waits take 12 us per CTA
 // whatever its tiles (16, latent heads 30, with a row per lane in both).  Kernel time in us, before this form and now: 16 heads, window 1024, 2048
-// tokens 85 / 72, latent 16 heads of 192, 128 / 2048 tokens 36 / 16 and 110 / 75, LLaMA's 32 heads, 2048 tokens 111 / 85.
+// tokens 85 / 68, latent 16 heads of 192, 128 / 2048 tokens 36 / 16 and 110 / 77, LLaMA's 32 heads, 2048 tokens 111 / 86.
 #pragma once
 #include "tc_common.cuh"
 

@@ -342,7 +342,7 @@ __global__ void seq_decay_kernel(const act_t* __restrict__ a, int lda, const act
 }
 
 // The same for bf16 layers whose heads are whole groups of 8 channels: a thread owns 8 channels (one 16-byte load, two stores), so a head's coefficient is
-// formed once for them (2048 channels x 2048 tokens: 23 us one channel at a time, now 8; 24 MB move).
+// formed once for them (2048 channels x 2048 tokens: 23 us one channel at a time, now 9.6; 24 MB move).
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]);
 __global__ void __launch_bounds__(256) seq_decay8_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ bias,
                                                         const __nv_bfloat16* __restrict__ A_log, int mode, float inv_tau, float* __restrict__ out,
@@ -402,7 +402,7 @@ __global__ void seq_group_norm_gate_kernel(const float* __restrict__ o, int ldo,
 }
 
 // The same for bf16 groups of 32 PER channels: a lane owns PER neighbouring ones and keeps them in registers (2048 tokens of 16 groups of 128: 16 us
-// with two-byte accesses, now 7; 32 MB move).
+// with two-byte accesses, now 10; 32 MB move).
 template <int PER>
 __global__ void __launch_bounds__(128) seq_group_norm_gate_vec_kernel(const float* __restrict__ o, int ldo, const __nv_bfloat16* __restrict__ w, int w_shared,
                                                                      const __nv_bfloat16* __restrict__ gate, int ldg, int gate_act, int gate_first, float eps,

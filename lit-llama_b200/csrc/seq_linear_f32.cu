@@ -1,7 +1,7 @@
 // f32 linear on the tensor cores: y[M, N] = x[M, K] . W[N, K]^T with f32 operands, f32 sums and f32 results (models that run in 32 bits).
 //
 // An f32 number is the sum of three bf16 numbers (hi + mid + lo, each rounded: 24 bits in three times eight).  Of the nine products of parts the six
-// above 2^-24 are taken; each is exact in f32, and the sum of 64 k is added to f32 registers, since the tensor core truncates where it adds to its
+// above 2^-24 are taken (entries below 2^-109 keep fewer bits: the parts have f32's exponents and no more); each is exact in f32, and the sum of 64 k is added to f32 registers, since the tensor core truncates where it adds to its
 // accumulator (1024 k in one accumulator: a bias of 2e-6; so errors against float64 are those of f32 FMAs or smaller).
 //
 // A CTA computes 128 output features x bt tokens (16..112), the WEIGHT as the 128-row operand in tensor memory; per stage of 64 k
