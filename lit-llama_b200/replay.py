@@ -9,7 +9,7 @@ import torch
 
 from . import _seqlib as S
 
-_lock = threading.Lock()
+_lock = threading.RLock()                 # an owner may be collected, and give back, while its thread is inside
 _free: Dict[int, List[int]] = {}          # device -> recording streams whose owners are gone
 
 
@@ -27,7 +27,7 @@ def recording_stream(owner, device: torch.device) -> torch.cuda.Stream:
             at = p.value
         else:
             torch.cuda.synchronize(index)
-    weakref.finalize(owner, _give_back, index, at)
+    weakref.finalize(owner, _give_back, index, at).atexit = False
     return torch.cuda.ExternalStream(at, device=torch.device("cuda", index))
 
 

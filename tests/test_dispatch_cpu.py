@@ -247,3 +247,37 @@ def test_attention_without_room_runs_the_form_that_needs_none(monkeypatch):
     monkeypatch.setattr(torch, "empty", none_left)
     mixers.local_attention(S.AttnArgs(), types.SimpleNamespace(meta=torch.zeros(2), stream=None))
     assert seen == [(None, 0)]
+
+
+def test_an_owner_collected_while_a_stream_is_handed_out(monkeypatch):
+    """Engines are collected at any moment, also while their thread takes a stream from the list: its stream is given back without waiting for itself."""
+    import contextlib
+    import threading
+
+    import torch
+    from lit_llama_b200 import replay
+
+    class Owner:
+        pass
+
+    class Streams(dict):
+        def get(self, key):
+            gone.clear()                                     # the collector runs here
+            return dict.get(self, key)
+
+    gone, free = [Owner()], Streams()
+    monkeypatch.setattr(replay, "_free", free)
+    monkeypatch.setattr(torch.cuda, "device", lambda i: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda i: None)
+    monkeypatch.setattr(torch.cuda, "ExternalStream", lambda at, device: at)
+    free[0] = [11]
+    first, taken = Owner(), []
+    kept = gone[0]
+    assert replay.recording_stream(kept, torch.device("cuda", 0)) == 11
+    gone[:] = [kept]
+    del kept
+    free[0] = [12]
+    t = threading.Thread(target=lambda: taken.append(replay.recording_stream(first, torch.device("cuda", 0))), daemon=True)
+    t.start()
+    t.join(20)
+    assert not t.is_alive() and taken and sorted(free[0] + taken) == [11, 12]
