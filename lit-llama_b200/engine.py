@@ -146,9 +146,9 @@ class Engine:
         wrong with it by itself.  After three failures nothing is recorded any more."""
         if self._failed_recordings >= 3:
             return None
-        if self._stream is None:
-            self._stream = replay.recording_stream(self, self.device)
         try:
+            if self._stream is None:
+                self._stream = replay.recording_stream(self, self.device)
             return replay.record(self._stream, pool, body)
         except RuntimeError:
             self._failed_recordings += 1

@@ -39,14 +39,23 @@ def _give_back(index: int, at: int) -> None:
 def record(stream: torch.cuda.Stream, pool, body: Callable[[], torch.Tensor]) -> Tuple[torch.cuda.CUDAGraph, torch.Tensor]:
     """What body() launches as a graph (not run), with its temporaries in `pool` (None: one of its own), and body()'s result.  Only this thread's calls count
     as part of the recording: another thread may allocate, launch or record meanwhile."""
-    g = torch.cuda.CUDAGraph()
     with torch.cuda.device(stream.device), torch.cuda.stream(stream):
         torch.cuda.current_blas_handle()                 # the thread's handle and its workspace for this stream are there before the recording
-        g.capture_begin(pool=pool, capture_error_mode="thread_local")
         try:
-            out = body()
-        finally:
-            g.capture_end()
+            return _recorded(pool, body)
+        except RuntimeError:
+            # a recording that a call has broken off leaves torch's random numbers waiting for its end; one that ends takes them out of that
+            _recorded(None, lambda: torch.zeros(1, device=stream.device))
+            raise
+
+
+def _recorded(pool, body):
+    g = torch.cuda.CUDAGraph()
+    g.capture_begin(pool=pool, capture_error_mode="thread_local")
+    try:
+        out = body()
+    finally:
+        g.capture_end()
     return g, out
 
 

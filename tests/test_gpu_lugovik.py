@@ -664,3 +664,35 @@ def test_engines_on_two_streams_share_no_recording_stream():
     del a, b, e
     gc.collect()
     assert own <= {at for free in replay._free.values() for at in free}
+
+
+def test_a_recording_that_fails_leaves_everything_usable():
+    """A forward pass that waits for the device cannot be recorded: its steps run eagerly with the bits of an engine that never records, and random numbers,
+    other engines' recordings and allocations go on as before."""
+    from lit_llama_b200 import Engine
+
+    cfg = cfg_b()
+    a, _ = build(cfg, torch.bfloat16, n_slots=2)
+    b, good = Engine(a.model, n_slots=2), Engine(a.model, n_slots=2)
+    b.graph_after = b.portion_graph_after = 0
+    toks = tokens_for(cfg, 400, seed=9)
+
+    class Waiting(type(a.model)):
+        def forward_portion(self, *args):
+            out = super().forward_portion(*args)
+            torch.cuda.synchronize()
+            return out
+
+    a.model.__class__, plain = Waiting, type(a.model)
+    for i in range(8):
+        for part in (toks[33 * i: 33 * i + 33], [toks[i]]):
+            one = a.step([{"id": "r", "tokens": part, "want": [len(part) - 1]}])[0]
+            two = b.step([{"id": "r", "tokens": part, "want": [len(part) - 1]}])[0]
+            assert torch.equal(one, two)
+    assert a._failed_recordings == 3 and a._graph is None and not a._portions
+    a.model.__class__ = plain
+    assert torch.isfinite(torch.randn(1000, device=DEV)).all() and torch.zeros(1 << 20, device=DEV).sum() == 0
+    for i in range(5):
+        good.step([{"id": "r", "tokens": toks[33 * i: 33 * i + 33], "want": [32]}])
+    assert good._portions and good._failed_recordings == 0
+    assert all(torch.equal(a.pool.tensors[k], b.pool.tensors[k]) for k in b.pool.tensors)
