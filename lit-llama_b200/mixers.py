@@ -108,14 +108,20 @@ def share_weights(mixer, name: str):
 FEW_TOKENS = 4          # up to this many tokens a mechanism may run its products in its own kernels, without the library
 
 
-#: Where an f32 product runs on the tensor cores: below these the tiles are too few for the SMs, or too short for what a tile costs beside its sums, and the
-#: library is as fast or faster.  Device time in us, here / library, over 1024..131072 outputs; from the line on none measured is slower here:
-#:   rows x outputs    128 x 1024 x 1024 (k) 31 / 31, 256 x 1024 x 1024 31 / 31, 512 x 1024 x 1024 31 / 35, 777 x 2560 x 1024 43 / 90
-#:   and times k       256 x 1024 x 512 20.5 / 19.4, 512 x 1024 x 512 20.5 / 22.5, 64 x 8192 x 384 18 / 20
-#:   rows              2 x 131072 x 2048 277 / 203, 4 x 131072 x 1024 160 / 175 (with larger errors: up to 8 rows the library adds more finely), 9 rows 162 / 205,
-#:                     9 x 32000 x 4096 164 / 219; with k below 384, 32 x 131072 x 256 77 / 72, 48 rows 80 / 106
-#:   k                 64: 16 x 32000 18 / 12, 777 x 32000 117 / 104; 128: 32 x 32000 21 / 16, 777 x 2560 16 / 20; 256: 777 x 8192 55 / 80
-LINEAR_F32_FROM, LINEAR_F32_WORK, LINEAR_F32_ROWS, LINEAR_F32_K = 1 << 18, 3 << 26, 9, 256
+def _f32_pays(rows: int, n: int, k: int) -> bool:
+    """Where an f32 product of these sizes runs on the tensor cores: below, tiles are too few for the SMs or too short for what they cost beside their sums,
+    and the library is as fast or faster.  Device time in us, here / library; of 310 measured sizes above the line (rows 8..2048, n 1024..131072, k 128..4096)
+    none is slower here:
+      results    128 x 1024 x 1024 (k) 31 / 31, 256 x 1024 x 1024 31 / 31, 777 x 2560 x 1024 43 / 90; with shorter sums 256 x 1024 x 512 20.5 / 19.4,
+                 128 x 2560 x 512 20.5 / 22.5
+      rows       2 x 131072 x 2048 277 / 203; 4 rows 279 / 323, but up to 4 rows the library adds in more parts (k 4096: error 1.3e-7, here 1.7e-7; 8 rows 4.1e-7
+                 and 1.7e-7); 8 x 131072 x 1024 162 / 179; k 256: 32 x 131072 77 / 72, 48 x 131072 80 / 106
+      k          128: 256 x 1024 12 / 10, 777 x 2560 16 / 20, 9 x 32000 20 / 16, 256 x 131072 197 / 190; 64: 16 x 32000 18 / 12, 777 x 32000 117 / 104"""
+    if k >= 384:
+        return rows >= 8 and rows * n >= (1 << 18 if k >= 768 else 17 << 14)
+    if k >= 256:
+        return rows >= 48 and rows * n >= 17 << 14
+    return k >= 128 and rows >= 48 and n <= 8192 and rows * n >= 600000
 
 
 #: looked up once: a product of the size of the line takes 20 us, and asking through torch's modules took 2 of them
@@ -135,8 +141,7 @@ def _f32_sizes(x: torch.Tensor, w: torch.Tensor) -> bool:
     if x.dim() != 2 or w.dim() != 2 or w.dtype is not torch.float32:
         return False
     (rows, k), (n, kw) = x.shape, w.shape
-    if (k != kw or k % 8 != 0 or k < LINEAR_F32_K or rows < (LINEAR_F32_ROWS if k >= 384 else 48) or rows * n < LINEAR_F32_FROM or rows * n * k < LINEAR_F32_WORK
-            or rows > 16 * 65535):
+    if k != kw or k % 8 != 0 or rows > 16 * 65535 or not _f32_pays(rows, n, k):
         return False
     (ldx, step_x), (ldw, step_w) = x.stride(), w.stride()
     return (step_x == 1 and step_w == 1 and ldx % 4 == 0 and ldw % 4 == 0 and ldx >= k and ldw >= k and x.storage_offset() % 4 == 0 and w.storage_offset() % 4 == 0)

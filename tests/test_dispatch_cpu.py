@@ -32,8 +32,9 @@ def test_f32_products_of_no_entries_or_too_many_rows_stay_with_the_library():
 
 
 @pytest.mark.parametrize("rows,outputs,k,taken", [
-    (256, 1024, 1024, True), (255, 1024, 1024, False), (9, 32000, 1024, True), (8, 65536, 1024, False), (256, 1024, 768, True), (256, 1024, 760, False),
-    (384, 1024, 512, True), (9, 65536, 384, True), (9, 65536, 376, False), (48, 32000, 256, True), (47, 32000, 256, False), (4096, 4096, 248, False)])
+    (256, 1024, 1024, True), (255, 1024, 1024, False), (8, 32768, 1024, True), (7, 65536, 1024, False), (256, 1024, 768, True), (256, 1024, 760, False),
+    (272, 1024, 384, True), (8, 65536, 384, True), (8, 65536, 376, False), (48, 32000, 256, True), (47, 32000, 256, False), (272, 1024, 256, True),
+    (74, 8192, 248, True), (73, 8192, 128, False), (100, 8200, 128, False), (586, 1024, 128, True), (4096, 4096, 120, False)])
 def test_f32_products_on_both_sides_of_the_line(rows, outputs, k, taken):
     """Rows, k, results and products from which the tensor-core form is the faster one."""
     import torch
