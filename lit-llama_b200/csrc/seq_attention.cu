@@ -747,35 +747,39 @@ static DynSmemCache g_local_tc_smem[4];
 // position first_visible(pos0) + i, from the ring or the portion; 64 rows of zeros behind the last (a tile's rows end where it does).
 static int plane_rows(const b2l_seq_attn_args* a) { return a->T + (a->window > 0 ? a->window : a->block) + atc::KEYS; }
 static size_t plane_cols(const b2l_seq_attn_args* a) { return (size_t)a->kv_heads * ((a->maps > 1 ? a->maps : 1) * a->K + a->V); }
+// A CTA takes rows in turn: the ring may be as long as the longest sequence, and the rows in use are known on the device only (8 heads of 32, ring of 16384,
+// first 64 tokens: 29 us with a CTA for every row there might be, 21 so, 20..21 with FMAs; second half of the ring, 8 heads of 128: 319 / 314).
+constexpr int PLANE_CTAS = 8;      // per SM
 __global__ void __launch_bounds__(128) seq_attention_planes_kernel(b2l_seq_attn_args a, __nv_bfloat16* planes, int rows) {
-  const int pos0 = a.meta[1], j0 = first_visible(a, pos0), j = j0 + (int)blockIdx.x, end = pos0 + a.T;
-  if (j >= end + atc::KEYS) return;
+  const int pos0 = a.meta[1], j0 = first_visible(a, pos0), end = pos0 + a.T;
   const int nk = a.kv_heads * (a.maps > 1 ? a.maps : 1) * a.K, nv = a.kv_heads * a.V;
-  const bool fresh = j >= pos0;
-  const size_t ring = (size_t)a.meta[0] * a.block + j % a.block;
-  const float* k = fresh ? (const float*)a.k_new + (size_t)(j - pos0) * nk : (const float*)a.cache_k + ring * nk;
-  const float* v = fresh ? (const float*)a.v_new + (size_t)(j - pos0) * a.ldv : (const float*)a.cache_v + ring * nv;
   __nv_bfloat16* pv = planes + (size_t)3 * rows * nk;
-  for (int c = 8 * (int)threadIdx.x; c < nk + nv; c += 8 * 128) {
-    const bool key = c < nk;
-    const float* src = key ? k + c : v + (c - nk);
-    float x[8] = {};
-    if (j < end) {
-      *reinterpret_cast<float4*>(x) = reinterpret_cast<const float4*>(src)[0];
-      *reinterpret_cast<float4*>(x + 4) = reinterpret_cast<const float4*>(src)[1];
-    }
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      uint32_t w[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
-        w[e] = *reinterpret_cast<const uint32_t*>(&h);
-        x[2 * e] -= __uint_as_float(w[e] << 16);
-        x[2 * e + 1] -= __uint_as_float(w[e] & 0xffff0000u);
+  for (int row = blockIdx.x, j = j0 + row; j < end + atc::KEYS; row += gridDim.x, j += gridDim.x) {
+    const bool fresh = j >= pos0;
+    const size_t ring = (size_t)a.meta[0] * a.block + j % a.block;
+    const float* k = fresh ? (const float*)a.k_new + (size_t)(j - pos0) * nk : (const float*)a.cache_k + ring * nk;
+    const float* v = fresh ? (const float*)a.v_new + (size_t)(j - pos0) * a.ldv : (const float*)a.cache_v + ring * nv;
+    for (int c = 8 * (int)threadIdx.x; c < nk + nv; c += 8 * 128) {
+      const bool key = c < nk;
+      const float* src = key ? k + c : v + (c - nk);
+      float x[8] = {};
+      if (j < end) {
+        *reinterpret_cast<float4*>(x) = reinterpret_cast<const float4*>(src)[0];
+        *reinterpret_cast<float4*>(x + 4) = reinterpret_cast<const float4*>(src)[1];
       }
-      __nv_bfloat16* dst = key ? planes + ((size_t)p * rows + blockIdx.x) * nk + c : pv + ((size_t)p * rows + blockIdx.x) * nv + (c - nk);
-      *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+          w[e] = *reinterpret_cast<const uint32_t*>(&h);
+          x[2 * e] -= __uint_as_float(w[e] << 16);
+          x[2 * e + 1] -= __uint_as_float(w[e] & 0xffff0000u);
+        }
+        __nv_bfloat16* dst = key ? planes + ((size_t)p * rows + row) * nk + c : pv + ((size_t)p * rows + row) * nv + (c - nk);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
     }
   }
 }
@@ -794,7 +798,7 @@ static int launch_local_tc(const b2l_seq_attn_args* a, cudaStream_t s) {
     keys = a->work;
     values = (const __nv_bfloat16*)a->work + rows * sk;
     ldv = sv;
-    seq_attention_planes_kernel<<<p.plane, 128, 0, s>>>(*a, (__nv_bfloat16*)a->work, p.plane);
+    seq_attention_planes_kernel<<<std::min(p.plane, PLANE_CTAS * sm_count()), 128, 0, s>>>(*a, (__nv_bfloat16*)a->work, p.plane);
     B2L_LAUNCH_CHECK("seq_attention_planes_kernel");
   }
   if (int rc = tc::map_sw128(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, keys, rows, sk, sk, 64, atc::KEYS)) return rc;

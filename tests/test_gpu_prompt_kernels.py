@@ -457,10 +457,10 @@ def test_small_gates_are_not_lost(act):
 
 
 @pytest.mark.parametrize("T,H,G,K,V,pos0,window,block,sink,cap", [
-    (64, 8, 2, 128, 128, 0, 512, 512, 0, 0.0), (130, 4, 1, 192, 16, 300, 96, 100, 1, 0.0), (257, 4, 2, 64, 112, 90, 0, 128, 0, 30.0), (200, 8, 8, 16, 64, 1000, 333, 333, 1, 0.0)])
+    (64, 8, 2, 128, 128, 0, 512, 512, 0, 0.0), (130, 4, 1, 192, 16, 300, 96, 100, 1, 0.0), (257, 4, 2, 64, 112, 90, 0, 128, 0, 30.0), (200, 8, 8, 16, 64, 1000, 333, 333, 1, 0.0), (777, 4, 2, 64, 64, 1300, 1250, 1250, 0, 0.0)])
 def test_f32_local_attention_in_three_parts(T, H, G, K, V, pos0, window, block, sink, cap):
     """f32 keys and values as three bf16 parts each: older keys from the ring (entries nobody sees are NaN), windows and blocks, room that nothing has
-    written yet, and the f32 tiles without room.  Products above 2^-24 are kept and every tile's sum is rounded: the bound of f32 sums at the top."""
+    written yet, more rows than a CTA's one, and the f32 tiles without room.  Products above 2^-24 are kept and every tile's sum is rounded: the bound of f32 sums at the top."""
     from lit_llama_b200 import _seqlib as S
 
     n, g, f32 = pos0 + T, torch.Generator(device=DEV).manual_seed(T + K), torch.float32
