@@ -162,7 +162,7 @@ def _f32_product(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    if x.dtype == torch.float32 and _f32_product(x, w):
+    if x.dtype == torch.float32 and x.shape[0] >= 8 and _f32_product(x, w):
         y = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
         S.check(S.lib().b2l_seq_linear_f32(_p(x), x.stride(0), _p(w), w.stride(0), _p(y), w.shape[0], x.shape[0], w.shape[0], x.shape[1], S.stream_ptr()),
                 "b2l_seq_linear_f32")
