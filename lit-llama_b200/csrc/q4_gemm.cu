@@ -1,5 +1,5 @@
-// Prompt-shaped int4 weight-only GEMM on the 5th-generation tensor cores: y[M, N] = x[M, K] . dequant(W)[N, K]^T for M > 16 (prompt
-// processing, no-cache forward, evaluation).
+// Prompt-shaped int4 weight-only GEMM on the 5th-generation tensor cores: y[M, N] = x[M, K] . dequant(W)[N, K]^T for M > 8 (prompt
+// processing, no-cache forward, evaluation, linears of 9..16 sequences; a tile has 16 tokens or more, so 9..16 rows take as long as 17 less the extra tile).
 //
 // Replaces ColBlockQuantizedLinear.forward (lit_llama/quantization.py:413-423) and the Triton kernel linear_kernel_4bit_weight
 // (quantization.py:187-333: tiles up to 256 x 256, dequantise inside the tile loop) for 4-bit weights with one (scale, zero) per row.

@@ -4,7 +4,7 @@
 (names, shapes, dtypes, strides) and `state_dict` keys (quantization.py:340-374), so a
 `llama-gptq.4bit.pth` produced by the reference's quantize/gptq.py loads unchanged.
 `forward` runs hand-written sm_100a kernels through the C ABI of include/b2l.h (M = 1: exact int8-digit MMA GEMV;
-2..8: f16 MMA batch kernel; 9..16: tcgen05 from tensor memory; > 16: tcgen05 GEMM with the weight in tensor memory); there is no
+2..8: f16 MMA batch kernel; > 8: tcgen05 GEMM with the weight in tensor memory; 9..16 where the input is no multiple of 64 wide: q4_linear_tc); there is no
 Triton, no library GEMM, no dense fallback and no CPU path.
 """
 import ctypes as C
@@ -285,9 +285,11 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             # 2..8 rows: the mma.sync tile has 8 columns, one per row (csrc/q4_gemv_batch.cu)
             which, wt, ws = L.Q4_GEMV_BATCH, self.tiled_mma(), batch_workspace(device, K).data_ptr()
         elif tc and aligned and (M <= 16 or K % 64 == 0):
-            # 9..16 rows: tcgen05 with K split over clusters; prompts: tcgen05 tiles of 128 features, weights dequantised on the fly with
-            # get_weight's roundings
-            which, wt = L.Q4_LINEAR_TC if M <= 16 else L.Q4_GEMM, self.tiled()
+            # more than 8 rows: tcgen05 tiles of 128 features, weights dequantised on the fly with get_weight's roundings.  Up to 16 rows q4_linear_tc
+            # (K split over clusters) takes inputs that are no multiple of 64 wide, and no others: 9 / 16 rows of 4096 -> 4096 take it 23 / 30 us and the
+            # GEMM 11.4 / 11.6, 4096 -> 11008 36 / 46 and 15.8, 13824 -> 5120 49 / 63 and 20, 64 -> 64 10 / 14 and 5.0; 1.7 to 3.2 times in all 14 shapes
+            # measured, and 0.0017 off the product of get_weight's matrix in 64 bits instead of 0.0024
+            which, wt = L.Q4_GEMM if K % 64 == 0 else L.Q4_LINEAR_TC, self.tiled()
         if which >= 0:
             rc = L.pycall.q4(which, xp, ldx, wt.data_ptr(), scales.data_ptr(), zeros.data_ptr(), 0 if scales.dtype is torch.bfloat16 else L.sz_dtype_of(scales),
                              y.data_ptr(), N, M, N, K, ws, L.stream_ptr())

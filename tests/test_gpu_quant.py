@@ -259,6 +259,25 @@ def test_q4_gemm_prefill_shapes(dev, M, N, K):
         assert torch.equal(lin.get_weight(torch.bfloat16), wb)
 
 
+@pytest.mark.parametrize("M", [9, 15, 16])
+@pytest.mark.parametrize("N,K,sz", [(130, 64, torch.bfloat16), (300, 192, torch.float32), (5120, 1024, torch.bfloat16), (300, 96, torch.bfloat16)])
+def test_linear_of_9_to_16_rows(dev, M, N, K, sz):
+    """Through forward(): the GEMM, which multiplies get_weight's matrix, where K is a multiple of 64, the older kernel otherwise (its weights are not rounded
+    to bf16: within the sum of both roundings).  Rows apart in memory."""
+    from gpu_util import rand_q4
+    from lit_llama_b200.quantization import ColBlockQuantizedLinear
+
+    lv, qw, sc, z = rand_q4(N, K, dev, seed=M + N + K)
+    lin = ColBlockQuantizedLinear(K, N, bias=False, bits=4, tile_cols=-1).to(dev)
+    lin.quant_weight.copy_(qw); lin.scales = sc.to(sz); lin.zeros = z.to(sz)
+    x = torch.randn(M, K + 8, device=dev).bfloat16()[:, :K]
+    y, wb = lin(x).double(), lin.get_weight(torch.bfloat16).double()
+    want, mag = x.double() @ wb.t(), x.double().abs() @ wb.abs().t()
+    # one bf16 rounding of the result and f32 sums; without get_weight's roundings of level - zero and of the product, 2^-9 each, as well
+    room = want.abs() * 2.0 ** -8 + mag * (2.0 ** -20 if K % 64 == 0 else 2.0 ** -8) + 1e-30
+    assert bool(((y - want).abs() <= room).all())
+
+
 @pytest.mark.parametrize("name,N,K", [("c_attn", 12288, 4096), ("c_proj", 4096, 4096), ("c_fc12", 22016, 4096),
                                       ("mlp_proj", 4096, 11008), ("lm_head", 32000, 4096)])
 def test_tc_linear_7b_shapes(dev, name, N, K):
