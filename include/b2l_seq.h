@@ -137,7 +137,8 @@ typedef struct {
 } b2l_seq_scan_args;
 int b2l_seq_scan_chunks(int T, int delta);
 /* Floats of work_state with which a portion with n_chunks <= 1 runs 16 tokens at a time where its sizes allow it (0: too short); step by step
- * with work_state null.  The space of a portion with n_chunks > 1 serves as well where it is as large. */
+ * with work_state null.  The space of a portion with n_chunks > 1 serves as well where it is as large.  It holds the chunks' matrices, and from 64 tokens
+ * on (up to 256 heads) the operands of the form on the tensor cores, 50 KB a chunk and head, of at most 2048 of them at a time. */
 long long b2l_seq_scan_work_floats(int T, int heads);
 /* The fastest form for these sizes (vscale: whether a value scale is given): sets *n_chunks and returns the floats of work_state it wants (0: none,
  * step by step).  work_decay is wanted where *n_chunks > 1: n_chunks * heads * (per_channel ? K : 1) floats. */

@@ -334,7 +334,8 @@ __global__ void seq_scan_combine_kernel(b2l_seq_scan_args a) {
 //                o = R + (B T) (v - P)
 //   S_16 = G_16 S_0 + sum_i (D_(16,i) k_i) u_i^T
 // Decays only ever multiply (no quotient of cumulative products, which overflows where a channel forgets fast).  T is the product of the
-// chunk's transition matrices seen from k: its entries stay below 1 for unit keys.  All f32 on the CUDA cores, like the step-by-step form.
+// chunk's transition matrices seen from k: its entries stay below 1 for unit keys.  Long portions with 128 keys take the form on the tensor cores
+// (seq_scan_mma.cuh); here all is f32 on the CUDA cores, like the step-by-step form.
 //   seq_chunk_kernel  a CTA per (chunk, head): T and B T (or B), 16 x 16 each, into the workspace; all chunks in parallel
 //   seq_walk_kernel   a CTA per (head, VT = 16 or 8 value columns) walks the chunks: warps 4..11 (a thread per key channel, the two groups on
 //                     alternate chunks) load and form G k, G q, D k a chunk ahead, while warps 0..3 run P / R (K split over the warps),
@@ -718,6 +719,12 @@ __global__ void __launch_bounds__(384) seq_walk_kernel(b2l_seq_scan_args a) {
   }
 }
 
+}  // namespace b2l
+
+#include "seq_scan_mma.cuh"
+
+namespace b2l {
+
 constexpr int SCAN_CHUNK = 128;      // tokens per chunk of a chunked portion (a multiple of SCAN_TC)
 
 static bool walk_sizes(int T, int K, int V, int ones) { return T >= 2 * CH_C && (K == 64 || K == 128) && V % CH_VT == 0 && !ones; }
@@ -727,7 +734,8 @@ static bool walk_sizes(int T, int K, int V, int ones) { return T >= 2 * CH_C && 
 // stays flat until its CTAs fill the SMs while the walk takes 1.3 us (1.0 with 64 keys) per 16 tokens and turn of CTAs whatever the heads:
 // both times from the fits below, in ns (128 x 128, us walk with 16 columns per CTA / chunked: 1024 tokens of 4 heads 95 / 103; 2048 of 4 173 / 130,
 // of 8 179 / 240; 4096 of 4 333 / 251, of 8 345 / 388; 8192 of 1 634 / 134, of 8 673 / 667, of 16 710 / 1285; walk with 8 columns: 512 tokens of 4
-// and 8 43, 2048 of 4 124, of 8 128; with 64 keys 512 tokens 38, 1024 of 18 63).
+// and 8 43, 2048 of 4 124, of 8 128; with 64 keys 512 tokens 38, 1024 of 18 63).  The fits are the FMA walk's also where the tensor cores walk (2048 and 4096 tokens of 4
+// heads 81 and 153, 4096 and 8192 of 8 221 and 432, 8192 of 1 261): a chunked form's workspace, which callers bring by its size, is too small for that walk's operands.
 static bool walk_narrow(int heads, int V) { return (long long)heads * (V / CH_NARROW) <= sm_count(); }
 static bool walk_pays(int T, int heads, int K, int V, int delta) {
   const long long sms = sm_count(), ctas = (long long)heads * (V / CH_VT), turns = (ctas + sms - 1) / sms;
@@ -737,14 +745,18 @@ static bool walk_pays(int T, int heads, int K, int V, int delta) {
   const long long t_chunked = load == 1 ? 104000 : load == 2 ? 131000 : 60000 + 45000 * load, t_walk = 15000 + (long long)(T / CH_C) * (walk_narrow(heads, V) ? (K == 64 ? 800 : 920) : (K == 64 ? 1050 : 1350)) * turns;
   return t_walk <= t_chunked;
 }
-// Portions of two chunks or more with key sizes 64 or 128 and whole groups of 16 values, given room for the chunks' matrices; other sizes, the
-// column of ones and single tokens go step by step.  A caller that asks for the chunked form gets the walk where it is faster and its space
-// suffices.
-static bool walk_chunks(const b2l_seq_scan_args* a) {
-  const size_t chunks = ((size_t)a->T + CH_C - 1) / CH_C;
-  const bool wanted = a->n_chunks <= 1 || ((size_t)a->n_chunks * a->V * a->K >= chunks * 2 * CH_MAT && walk_pays(a->T, a->heads, a->K, a->V, a->delta));
-  return a->work_state != nullptr && wanted && walk_sizes(a->T, a->K, a->V, a->ones) &&
-         (!a->delta || (a->decay_per_channel && !a->vscale)) && ((uintptr_t)a->state & 15) == 0 && ((uintptr_t)a->work_state & 15) == 0 && a->heads <= 65535;
+// Portions of two chunks or more with key sizes 64 or 128 and whole groups of 16 values, given room for the chunks' matrices (or operands); other sizes, the
+// column of ones and single tokens go step by step.  A caller that asks for the chunked form gets a walk where it is faster and its space suffices.
+static long long walk_floats(int T, int heads) { return (long long)((T + CH_C - 1) / CH_C) * heads * (2 * CH_MAT); }
+enum { WALK_NONE, WALK_FMA, WALK_MMA };
+static int walk_form(const b2l_seq_scan_args* a) {
+  if (a->work_state == nullptr || !walk_sizes(a->T, a->K, a->V, a->ones) || (a->delta && (!a->decay_per_channel || a->vscale)) || ((uintptr_t)a->state & 15) != 0 ||
+      ((uintptr_t)a->work_state & 15) != 0 || a->heads > 65535)
+    return WALK_NONE;
+  if (a->n_chunks > 1 && !walk_pays(a->T, a->heads, a->K, a->V, a->delta)) return WALK_NONE;
+  auto fits = [&](long long floats) { return a->n_chunks <= 1 || (long long)a->n_chunks * a->heads * a->V * a->K >= floats; };
+  if (mma_walk(a->T, a->heads, a->K, a->V, a->delta) && fits(mma_walk_floats(a->T, a->heads))) return WALK_MMA;
+  return fits(walk_floats(a->T, a->heads)) ? WALK_FMA : WALK_NONE;
 }
 
 template <typename act_t, int K, bool DELTA>
@@ -776,7 +788,9 @@ extern "C" int b2l_seq_scan_chunks(int T, int delta) {
 }
 
 extern "C" long long b2l_seq_scan_work_floats(int T, int heads) {
-  return T < 2 * CH_C || heads <= 0 ? 0 : (long long)((T + CH_C - 1) / CH_C) * heads * (2 * CH_MAT);
+  if (T < 2 * CH_C || heads <= 0) return 0;
+  const long long fma = walk_floats(T, heads), mma = T >= MW_LEAST && heads <= MW_HEADS ? mma_walk_floats(T, heads) : 0;
+  return fma > mma ? fma : mma;                        // for either, whatever the key size
 }
 
 extern "C" long long b2l_seq_scan_plan(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks) {
@@ -799,9 +813,14 @@ extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
                 "b2l_seq_scan: chunked portions need the workspace, no delta rule and n_chunks from b2l_seq_scan_chunks");
   B2L_CHECK_ARG(!a->ones || (a->state_ones && a->out_ones && !a->skip && !a->delta), "b2l_seq_scan: the column of ones needs its state and its output, no skip and no delta rule");
   if (a->T == 0) return 0;
-  if (walk_chunks(a) && (a->act_dtype == B2L_BF16 || a->act_dtype == B2L_F32)) {
+  const int form = walk_form(a);
+  if (form != WALK_NONE && (a->act_dtype == B2L_BF16 || a->act_dtype == B2L_F32)) {
     cudaStream_t st = (cudaStream_t)stream;
     B2L_SEQ_DISPATCH(a->act_dtype, {
+      if (form == WALK_MMA) {
+        if (a->delta) return launch_mma_walk<act_t, 128, true>(a, st);
+        return a->K == 64 ? launch_mma_walk<act_t, 64, false>(a, st) : launch_mma_walk<act_t, 128, false>(a, st);
+      }
       if (a->delta) return a->K == 64 ? launch_walk<act_t, 64, true>(a, st) : launch_walk<act_t, 128, true>(a, st);
       return a->K == 64 ? launch_walk<act_t, 64, false>(a, st) : launch_walk<act_t, 128, false>(a, st);
     });

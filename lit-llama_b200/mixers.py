@@ -237,7 +237,12 @@ def _scan(ctx: StepContext, *, q, ldq, k, ldk, v, ldv, q_mult, decay, ldd, per_c
         chunks = C.c_int(1)
         n = lib.b2l_seq_scan_plan(ctx.T, heads, K, V, int(per_channel), int(beta is not None), int(state_ones is not None), int(vscale is not None), C.byref(chunks))
         n_chunks = chunks.value
-        ws = torch.empty((n,), dtype=torch.float32, device=state.device) if n else None
+        try:
+            ws = torch.empty((n,), dtype=torch.float32, device=state.device) if n else None
+        except torch.OutOfMemoryError:
+            if n_chunks > 1:
+                raise
+            ws = None                                    # up to 102 MB: without it the portion goes token by token
         wd = torch.empty((n_chunks, heads, K if per_channel else 1), dtype=torch.float32, device=state.device) if n_chunks > 1 else None
     a = S.ScanArgs(q=q, ldq=ldq, k=k, ldk=ldk, v=v, ldv=ldv, q_mult=float(q_mult), decay=decay, ldd=ldd,
                    decay_per_channel=int(per_channel), beta=beta, ldb=ldb, delta=int(beta is not None), vscale=vscale, ldvs=ldvs,

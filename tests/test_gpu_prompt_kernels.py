@@ -182,6 +182,87 @@ def test_scans_sixteen_tokens_at_a_time(T, K, V, H, G, form):
     assert torch.equal(state[0], other)
 
 
+@pytest.mark.parametrize("T,K,V,H,G,form", [(64, 128, 128, 9, 3, "delta"), (79, 128, 16, 65, 13, "delta"), (144, 128, 48, 2, 1, "delta"), (161, 128, 128, 5, 5, "channel"),
+                                            (65, 128, 64, 18, 1, "scalar"), (175, 128, 16, 1, 1, "scalar"), (512, 64, 16, 4, 2, "channel"), (527, 64, 128, 2, 2, "scalar"),
+                                            (208, 128, 16, 160, 160, "delta"), (145, 128, 32, 256, 2, "scalar")])
+def test_scans_on_the_tensor_cores(T, K, V, H, G, form):
+    """The least portions by either side of the rule, last chunks of 1, 15 and 16 tokens, one tile of value columns and all eight, heads that share q and k, and
+    portions in two and more segments (2048 chunks times heads each)."""
+    test_scans_sixteen_tokens_at_a_time(T, K, V, H, G, form)
+
+
+@pytest.mark.parametrize("delta", [0, 1])
+@pytest.mark.parametrize("T", [144, 777])
+def test_scan_on_the_tensor_cores_is_as_near_as_token_by_token(T, delta):
+    """Rows apart by 3 entries (no 16-byte copies), one head, against float64 and against the form that walks token by token: 16-token sums of three bf16 parts are no
+    further off than twice its error (measured: 0.6 to 1.0 of it)."""
+    from lit_llama_b200 import _seqlib as S
+
+    H, K, V, ld = 3, 128, 32, 3 * 128 + 3
+    lib, g = S.lib(), torch.Generator(device=DEV).manual_seed(T + delta)
+    q, k, v = (torch.randn(T, ld, generator=g, device=DEV) for _ in range(3))
+    k[:, :H * K] = torch.nn.functional.normalize(k[:, :H * K].view(T, H, K), dim=-1).view(T, H * K)
+    a, beta, state0 = torch.rand(T, H, K, generator=g, device=DEV) * 0.5 + 0.5, torch.randn(T, H, generator=g, device=DEV), torch.randn(1, H, V, K, generator=g, device=DEV)
+    meta = torch.zeros(2, dtype=torch.int32, device=DEV)
+    s64, want = state0[0].double(), torch.empty(T, H, V, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        kt, qt, vt = (x[t, :H * n].double().view(H, n) for x, n in ((k, K), (q, K), (v, V)))
+        s64 = s64 * a[t].double()[:, None, :]
+        u = torch.sigmoid(beta[t].double())[:, None] * (vt - torch.einsum("hvk,hk->hv", s64, kt)) if delta else vt
+        s64 = s64 + u[:, :, None] * kt[:, None, :]
+        want[t] = torch.einsum("hvk,hk->hv", s64, qt)
+    errs = []
+    for work in (torch.empty(lib.b2l_seq_scan_work_floats(T, H), device=DEV), None):
+        out, state = torch.empty(T, H, V, device=DEV), state0.clone()
+        args = S.ScanArgs(q=q.data_ptr(), ldq=ld, k=k.data_ptr(), ldk=ld, v=v.data_ptr(), ldv=ld, q_mult=1.0, decay=a.data_ptr(), ldd=H * K, decay_per_channel=1,
+                          beta=beta.data_ptr() if delta else None, ldb=H, delta=delta, state=state.data_ptr(), meta=meta.data_ptr(), out=out.data_ptr(), ldo=H * V, T=T, heads=H,
+                          qk_heads=H, K=K, V=V, act_dtype=S.act_code(torch.float32), work_state=work.data_ptr() if work is not None else None, n_chunks=1)
+        S.check(lib.b2l_seq_scan(C.byref(args), S.stream_ptr()), "scan")
+        errs.append((rel(out, want), rel(state[0], s64)))
+    assert errs[0][0] < 2 * errs[1][0] and errs[0][1] < 2 * errs[1][1] and max(errs[0]) < 1e-6
+
+
+@pytest.mark.parametrize("what,bad", [("v", math.inf), ("k", math.nan), ("k", -math.inf), ("q", math.inf), ("decay", math.nan), ("beta", math.nan), ("state", math.inf)])
+@pytest.mark.parametrize("delta", [0, 1])
+def test_scan_on_the_tensor_cores_with_infinities(delta, what, bad):
+    """Tokens before a bad one, other heads and (values) other columns keep their bits; the rest is what the form that walks token by token gives: infinities and NaN in
+    the same places, finite results to 1e-5 of their row (f32 sums in two orders)."""
+    from lit_llama_b200 import _seqlib as S
+
+    T, H, K, V, at = 161, 2, 128, 32, 70
+    g = torch.Generator(device=DEV).manual_seed(11)
+    ops = {"q": torch.randn(T, H, K, generator=g, device=DEV), "k": torch.randn(T, H, K, generator=g, device=DEV) / 12, "v": torch.randn(T, H, V, generator=g, device=DEV),
+           "beta": torch.randn(T, H, generator=g, device=DEV), "decay": torch.rand(T, H, K, generator=g, device=DEV) * 0.5 + 0.5, "state": torch.randn(1, H, V, K, generator=g, device=DEV)}
+    meta, lib = torch.zeros(2, dtype=torch.int32, device=DEV), S.lib()
+    work = torch.empty(lib.b2l_seq_scan_work_floats(T, H), device=DEV)
+
+    def run(space):
+        out, state = torch.empty(T, H, V, device=DEV), ops["state"].clone()
+        a = S.ScanArgs(q=ops["q"].data_ptr(), ldq=H * K, k=ops["k"].data_ptr(), ldk=H * K, v=ops["v"].data_ptr(), ldv=H * V, q_mult=1.0, decay=ops["decay"].data_ptr(), ldd=H * K,
+                       decay_per_channel=1, beta=ops["beta"].data_ptr() if delta else None, ldb=H, delta=delta, state=state.data_ptr(), meta=meta.data_ptr(),
+                       out=out.data_ptr(), ldo=H * V, T=T, heads=H, qk_heads=H, K=K, V=V, act_dtype=S.act_code(torch.float32), work_state=space, n_chunks=1)
+        S.check(lib.b2l_seq_scan(C.byref(a), S.stream_ptr()), "scan")
+        return out, state
+
+    clean, clean_state = run(work.data_ptr())
+    if what == "state":
+        ops["state"][0, 1, 3, 5] = bad
+    else:
+        ops[what][at, 1, *([5] if what != "beta" else [])] = bad
+    (got, st), (want, st_want) = run(work.data_ptr()), run(None)
+    assert torch.equal(got[:, 0], clean[:, 0]) and torch.equal(st[0, 0], clean_state[0, 0])
+    if what != "state":
+        assert torch.equal(got[:at], clean[:at])
+    if what in ("v", "state"):
+        c = 5 if what == "v" else 3
+        assert torch.equal(got[:, :, :c], clean[:, :, :c]) and torch.equal(got[:, :, c + 1:], clean[:, :, c + 1:]) and torch.equal(st[0, 1, c + 1:], clean_state[0, 1, c + 1:])
+    for x, y in ((got, want), (st, st_want)):
+        fin = y.isfinite()
+        assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x[~fin & ~y.isnan()], y[~fin & ~y.isnan()])
+        x, y = x.double().where(fin, 0.0), y.double().where(fin, 0.0)
+        assert bool(((x - y).abs() <= 1e-5 * y.norm(dim=-1, keepdim=True)).all())
+
+
 @pytest.mark.parametrize("T,Ch,bias", [(33, 8, True), (48, 1032, False), (100, 2304, True)])
 def test_four_tap_convolution_of_long_portions(T, Ch, bias):
     from lit_llama_b200 import _seqlib as S
