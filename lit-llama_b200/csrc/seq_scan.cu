@@ -818,8 +818,9 @@ extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
     cudaStream_t st = (cudaStream_t)stream;
     B2L_SEQ_DISPATCH(a->act_dtype, {
       if (form == WALK_MMA) {
-        if (a->delta) return launch_mma_walk<act_t, 128, true>(a, st);
-        return a->K == 64 ? launch_mma_walk<act_t, 64, false>(a, st) : launch_mma_walk<act_t, 128, false>(a, st);
+        if (a->delta) return launch_mma_walk<act_t, 128, true, false>(a, st);
+        if (!a->decay_per_channel) return a->K == 64 ? launch_mma_walk<act_t, 64, false, true>(a, st) : launch_mma_walk<act_t, 128, false, true>(a, st);
+        return a->K == 64 ? launch_mma_walk<act_t, 64, false, false>(a, st) : launch_mma_walk<act_t, 128, false, false>(a, st);
       }
       if (a->delta) return a->K == 64 ? launch_walk<act_t, 64, true>(a, st) : launch_walk<act_t, 128, true>(a, st);
       return a->K == 64 ? launch_walk<act_t, 64, false>(a, st) : launch_walk<act_t, 128, false>(a, st);

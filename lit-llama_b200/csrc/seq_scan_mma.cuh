@@ -128,10 +128,12 @@ struct alignas(16) ChunkOps {
   uint32_t kd[K / 8 * 192];        // [8 channels][lane][part][8 tokens]
   float gc[K];                     // G of the whole chunk
 };
-constexpr int MW_TILE = 384;     // words per chunk and 16 value columns: T v (256), without the delta rule the parts of v vscale
+// Words per chunk, head and 16 value columns: T v (256), or without the delta rule the parts of v vscale; with one decay per head the parts of D v vscale, and G of
+// the 16 tokens behind them.
+constexpr int MW_TILE = 384, MW_TILE_G = MW_TILE + CH_C;
 
-struct MwWork { void* ops; uint32_t* tile; };   // of a segment: [chunk][head] ChunkOps, then [chunk][head][16 value columns] tiles
-// What a chunk gives by itself, a CTA per chunk and head.
+struct MwWork { void* ops; uint32_t* tile; };   // of a segment: [chunk][head, or head of q and k] ChunkOps, then [chunk][head][16 value columns] tiles
+// What a chunk gives by itself, a CTA per chunk and head; a decay per channel.
 constexpr int MW_CHUNK_THREADS = 256;
 template <typename act_t, int K, bool DELTA>
 __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_seq_scan_args a, int vec, int t_lo, int t_hi, MwWork work) {
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_
   const int t0 = t_lo + chunk * CH_C, nt = min(CH_C, t_hi - t0);
   const float* gk = a.k + (size_t)t0 * a.ldk + (size_t)hq * K;
   const float* gq = a.q + (size_t)t0 * a.ldq + (size_t)hq * K;
-  const float* gd = a.decay + (size_t)t0 * a.ldd + (a.decay_per_channel ? (size_t)h * K : (size_t)h);
+  const float* gd = a.decay + (size_t)t0 * a.ldd + (size_t)h * K;
   if (vec) {
 #pragma unroll 2
     for (int i = tid; i < CH_C * K / 4; i += MW_CHUNK_THREADS) {
@@ -154,10 +156,10 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_
       if (t < nt) {
         cp_async16(&sk[t][c], gk + (size_t)t * a.ldk + c);
         cp_async16(&sq[t][c], gq + (size_t)t * a.ldq + c);
-        if (a.decay_per_channel) cp_async16(&sg[t][c], gd + (size_t)t * a.ldd + c);
+        cp_async16(&sg[t][c], gd + (size_t)t * a.ldd + c);
       } else {
         *reinterpret_cast<float4*>(&sk[t][c]) = *reinterpret_cast<float4*>(&sq[t][c]) = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a.decay_per_channel) *reinterpret_cast<float4*>(&sg[t][c]) = make_float4(1.f, 1.f, 1.f, 1.f);
+        *reinterpret_cast<float4*>(&sg[t][c]) = make_float4(1.f, 1.f, 1.f, 1.f);
       }
     }
     cp_async_commit();
@@ -167,14 +169,9 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_
       const bool in = t < nt;
       sk[t][c] = in ? gk[(size_t)t * a.ldk + c] : 0.f;
       sq[t][c] = in ? gq[(size_t)t * a.ldq + c] : 0.f;
-      if (a.decay_per_channel) sg[t][c] = in ? gd[(size_t)t * a.ldd + c] : 1.f;
+      sg[t][c] = in ? gd[(size_t)t * a.ldd + c] : 1.f;
     }
   }
-  if (!a.decay_per_channel)
-    for (int i = tid; i < CH_C * K; i += MW_CHUNK_THREADS) {
-      const int t = i / K;
-      sg[t][i - t * K] = t < nt ? gd[(size_t)t * a.ldd] : 1.f;
-    }
   if (DELTA && tid < CH_C) sbeta[tid] = tid < nt ? sigmoid_f(ld_act((const act_t*)a.beta, (size_t)(t0 + tid) * a.ldb + h)) : 0.f;
   const bool values = warp * CH_VT < a.V;              // 16 value columns a warp: columns g, g + 8; tokens 2 t4, + 1, + 8, + 9
   float v[2][4] = {}, vs[2][2];
@@ -422,11 +419,173 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_
   }
 }
 
+// The same with one decay per head and no delta rule: q, k and their products are those of all heads that share them, and a head's decays weight outputs, values and the
+// 16 x 16 matrix.  So a CTA per (chunk, head of q and k, up to eight heads) multiplies q and k once, and the first of them leaves the walk one set of operands for all
+// heads, which the L2 then holds once.  us, both kernels, a CTA per head / this form: 32 heads of 128 x 64 over one q and k, 512 and 2048 tokens 44 / 34, 184 / 102; over 32 of
+// their own 44 / 46 and 197 / 195; 8 heads of 128 x 128 over one, 2048 tokens 93 / 83.
+template <typename act_t, int K>
+__global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_shared_kernel(b2l_seq_scan_args a, int vec, int t_lo, int t_hi, int per, MwWork work) {
+  using Ops = ChunkOps<K, false>;
+  constexpr int LD = K + 4, TILES = K / 64;
+  extern __shared__ __align__(16) unsigned char chunk_raw[];
+  float (*sq)[LD] = reinterpret_cast<float (*)[LD]>(chunk_raw), (*sk)[LD] = sq + CH_C;
+  Ops& ops = *reinterpret_cast<Ops*>(chunk_raw + sizeof(float) * 2 * CH_C * LD);
+  __shared__ __align__(16) float sB[8][CH_C][24];
+  __shared__ float sqk[CH_C][CH_C + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, chunk = blockIdx.x, hq = blockIdx.y;
+  // a warp takes a head; where a CTA has fewer than eight, several take one, and its value columns in turn
+  const int rep = a.heads / a.qk_heads, here = min(per, rep - per * (int)blockIdx.z), share = 8 / here, h = hq * rep + per * blockIdx.z + warp % here;
+  const int t0 = t_lo + chunk * CH_C, nt = min(CH_C, t_hi - t0);
+  const float* gk = a.k + (size_t)t0 * a.ldk + (size_t)hq * K;
+  const float* gq = a.q + (size_t)t0 * a.ldq + (size_t)hq * K;
+  if (vec) {
+#pragma unroll 2
+    for (int i = tid; i < CH_C * K / 4; i += MW_CHUNK_THREADS) {
+      const int t = i / (K / 4), c = (i - t * (K / 4)) * 4;
+      if (t < nt) {
+        cp_async16(&sk[t][c], gk + (size_t)t * a.ldk + c);
+        cp_async16(&sq[t][c], gq + (size_t)t * a.ldq + c);
+      } else {
+        *reinterpret_cast<float4*>(&sk[t][c]) = *reinterpret_cast<float4*>(&sq[t][c]) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    cp_async_commit();
+  } else {
+    for (int i = tid; i < CH_C * K; i += MW_CHUNK_THREADS) {
+      const int t = i / K, c = i - t * K;
+      sk[t][c] = t < nt ? gk[(size_t)t * a.ldk + c] : 0.f;
+      sq[t][c] = t < nt ? gq[(size_t)t * a.ldq + c] : 0.f;
+    }
+  }
+  const bool live = warp < share * here;
+  const int tt = lane & 15;
+  const float d = live && tt < nt ? a.decay[(size_t)(t0 + tt) * a.ldd + h] : 1.f, scale = live && a.vscale && tt < nt ? a.vscale[(size_t)(t0 + tt) * a.ldvs + h] : 1.f;
+  cp_async_wait<0>();
+  __syncthreads();
+  {
+    const int t = tid >> 4, i = tid & 15;              // q_t . k_i; of later tokens k_i nothing is used
+    float s[4] = {};
+#pragma unroll 8
+    for (int c = 0; c < K; c += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(&sq[t][c]), y = *reinterpret_cast<const float4*>(&sk[i][c]);
+      s[0] = fmaf(x.x, y.x, s[0]); s[1] = fmaf(x.y, y.y, s[1]); s[2] = fmaf(x.z, y.z, s[2]); s[3] = fmaf(x.w, y.w, s[3]);
+    }
+    sqk[t][i] = (s[0] + s[1]) + (s[2] + s[3]);
+  }
+  if (blockIdx.z == 0) {
+#pragma unroll 1
+    for (int tile = warp * TILES; tile < (warp + 1) * TILES; ++tile) {
+      uint32_t p[3][2];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) split2(sk[2 * t4 + 8 * hf][8 * tile + g], sk[2 * t4 + 8 * hf + 1][8 * tile + g], p[0][hf], p[1][hf], p[2][hf]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(ops.kd + tile * 192 + lane * 6 + 2 * i) = make_uint2(p[i][0], p[i][1]);
+      uint32_t* at = ops.wq + (tile >> 1) * (Ops::NT * 192) + lane * 6 + (tile & 1);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float2 y = *reinterpret_cast<const float2*>(&sq[g + 8 * r][8 * tile + 2 * t4]);
+        uint32_t w[3];
+        split2(y.x, y.y, w[0], w[1], w[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) at[r * 192 + 2 * i] = w[i];
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  if (blockIdx.z == 0 && tid == 0) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(reinterpret_cast<Ops*>(work.ops) + (size_t)chunk * a.qk_heads + hq),
+                 "r"((uint32_t)__cvta_generic_to_shared(&ops)), "r"((uint32_t)sizeof(Ops)) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+  __syncwarp();
+  if (live) {
+    float G = d, D = d;                                // products of the decays up to a token, after it
+#pragma unroll
+    for (int o = 1; o < CH_C; o <<= 1) {
+      const float p = __shfl_up_sync(0xffffffffu, G, o, 16), n = __shfl_down_sync(0xffffffffu, D, o, 16);
+      if (tt >= o) G *= p;
+      if (tt + o < CH_C) D *= n;
+    }
+    D = __shfl_down_sync(0xffffffffu, D, 1, 16);
+    if (tt == CH_C - 1) D = 1.f;
+    float x = 1.f;                                     // column tt of B, the upper half of the warp the odd rows
+#pragma unroll 4
+    for (int t = 0; t < CH_C; ++t) {
+      const float dt = __shfl_sync(0xffffffffu, d, t);
+      if (t > tt) x *= dt;
+      if ((t & 1) == lane >> 4) sB[warp][t][tt] = t >= tt ? x * sqk[t][tt] : 0.f;
+    }
+    __syncwarp();
+    PartsB b[2];                                       // B transposed
+    float dec[2][2], vs[2][2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float2 y = *reinterpret_cast<const float2*>(&sB[warp][g + 8 * j][2 * t4 + 8 * r]);
+        split2(y.x, y.y, b[j].b[0][r], b[j].b[1][r], b[j].b[2][r]);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        dec[j][e] = __shfl_sync(0xffffffffu, D, 8 * j + 2 * t4 + e);
+        vs[j][e] = __shfl_sync(0xffffffffu, scale, 8 * j + 2 * t4 + e);
+      }
+    }
+    const float skip = a.skip ? ld_act((const act_t*)a.skip, h) : 0.f;
+#pragma unroll 1
+    for (int vt = warp / here; vt < a.V / CH_VT; vt += share) {
+      uint32_t* tile = work.tile + (((size_t)chunk * a.heads + h) * (a.V / CH_VT) + vt) * MW_TILE_G;
+      const size_t col = (size_t)h * a.V + vt * CH_VT + g;
+      float v[2][4] = {}, u[2][4], y[2][4], ys[2][4];
+      Parts ua;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = 8 * j + 2 * t4 + (e & 1);
+          if (t < nt) v[j][e] = a.v[(size_t)(t0 + t) * a.ldv + col + 8 * (e >> 1)];
+        }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[j][e] = v[j][e] * vs[j][e & 1] * dec[j][e & 1];
+      split_pair(y, ua);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(tile + 128 * i + 4 * lane) = make_uint4(ua.a[i][0], ua.a[i][1], ua.a[i][2], ua.a[i][3]);
+      if (lane < CH_C) tile[MW_TILE + lane] = __float_as_uint(G);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[j][e] = v[j][e] * vs[j][e & 1];
+      int first[2];
+      const bool bad = __any_sync(0xffffffffu, !(finite4(u[0]) && finite4(u[1])));
+      if (bad) leave_out(u, lane, first);
+      split_pair(u, ua);
+      mma_parts<2, true>(y, ys, ua, b);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[j][e] += ys[j][e];
+      if (bad) lose_from(y, lane, first);
+      float* out = a.out + (size_t)t0 * a.ldo + col;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = 8 * j + 2 * t4 + (e & 1);
+          if (t < nt) out[(size_t)t * a.ldo + 8 * (e >> 1)] = fmaf(y[j][e], a.q_mult, skip * v[j][e]);
+        }
+    }
+  }
+  if (blockIdx.z == 0 && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
 constexpr int MW_WARPS = 8, MW_THREADS = 32 * (MW_WARPS + 4);      // the walk, warp 8 operands, 9 and 10 outputs
 template <int K, bool DELTA>
 struct MwStage {
   ChunkOps<K, DELTA> ops;
-  uint32_t tile[MW_TILE];
+  uint32_t tile[MW_TILE_G];
   float4 rx[MW_WARPS][2][32];    // R of the walk's warps, tokens 0..7 and 8..15
 };
 template <int K, bool DELTA>
@@ -501,8 +660,8 @@ __device__ __noinline__ void walk_redo(const b2l_seq_scan_args& a, int t_lo, int
 
 
 
-// tokens t_lo .. t_hi - 1
-template <typename act_t, int K, bool DELTA>
+// tokens t_lo .. t_hi - 1.  SHARED: operands of seq_chunk_shared_kernel; a head's decays are in its tiles
+template <typename act_t, int K, bool DELTA, bool SHARED>
 __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_args a, int t_lo, int t_hi, MwWork work) {
   using namespace tc;
   extern __shared__ __align__(16) unsigned char walk_raw[];
@@ -529,7 +688,7 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
   if (warp < MW_WARPS) {
     // ===================== the walk: channels WC warp .. of S =====================
     const int c0 = warp * WC, at0 = UN == 1 ? warp & 1 : 0;
-      Parts sa;
+    Parts sa;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
       if (j >= at0 && j < at0 + UN) {
@@ -592,7 +751,9 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
       mma_parts<UN, DELTA>(d, ds, ua, bd);
 #pragma unroll
       for (int j = 0; j < UN; ++j) {
-        const float2 gc = *reinterpret_cast<const float2*>(&s.ops.gc[c0 + 8 * j + 2 * t4]);
+        float2 gc;
+        if (SHARED) gc.x = gc.y = __uint_as_float(s.tile[MW_TILE_G - 1]);
+        else gc = *reinterpret_cast<const float2*>(&s.ops.gc[c0 + 8 * j + 2 * t4]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) d[j][e] += fmaf(UN == 1 ? S[0][e] + S[1][e] : S[j][e], e & 1 ? gc.y : gc.x, ds[j][e]);
       }
@@ -609,16 +770,18 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
     odd = !(finite4(S[0]) && finite4(S[1]));
   } else if (warp == MW_WARPS) {
     // ===================== operands, as the chunk kernel wrote them: STAGES - 1 copies ahead of the chunk that is handed over =====================
-    const Ops* ops = reinterpret_cast<const Ops*>(work.ops) + h;
-    const uint32_t* tile = work.tile + ((size_t)h * gridDim.x + blockIdx.x) * MW_TILE;
+    constexpr int WORDS = SHARED ? MW_TILE_G : MW_TILE;
+    const int sets = SHARED ? a.qk_heads : a.heads;    // of operands, of a chunk
+    const Ops* ops = reinterpret_cast<const Ops*>(work.ops) + (SHARED ? h / (a.heads / a.qk_heads) : h);
+    const uint32_t* tile = work.tile + ((size_t)h * gridDim.x + blockIdx.x) * WORDS;
     auto copy = [&](int n, int to) {
       if (lane == 0) {
         const uint32_t bar = smem_u32(sm.bars + to);
-        mbar_expect_tx(bar, sizeof(Ops) + 4 * MW_TILE);
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(&sm.st[to].ops)), "l"(ops + (size_t)n * a.heads),
+        mbar_expect_tx(bar, sizeof(Ops) + 4 * WORDS);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(&sm.st[to].ops)), "l"(ops + (size_t)n * sets),
                      "r"((uint32_t)sizeof(Ops)), "r"(bar) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(sm.st[to].tile)),
-                     "l"(tile + (size_t)n * a.heads * gridDim.x * MW_TILE), "r"((uint32_t)(4 * MW_TILE)), "r"(bar) : "memory");
+                     "l"(tile + (size_t)n * a.heads * gridDim.x * WORDS), "r"((uint32_t)(4 * WORDS)), "r"(bar) : "memory");
       }
     };
     int ahead = 0, sta = 0, sti = 0;
@@ -654,6 +817,10 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
       as4(r, s.rx[0][ow][lane]);
 #pragma unroll
       for (int w = 1; w < MW_WARPS; ++w) plus4(r, s.rx[w][ow][lane]);
+      if (SHARED) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] *= __uint_as_float(s.tile[MW_TILE + 8 * ow + 2 * t4 + (e & 1)]);
+      }
       bar_arrive(EMPTY + sti, 96);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -698,25 +865,35 @@ static bool mma_walk(int T, int heads, int K, int V, int delta) {
 static int mma_segment(int heads) { return MW_SEGMENT / heads * CH_C; }
 static long long mma_walk_floats(int T, int heads) {
   const long long chunks = ((T < mma_segment(heads) ? T : mma_segment(heads)) + CH_C - 1) / CH_C;
-  return chunks * heads * (long long)(sizeof(ChunkOps<128, true>) / 4 + MW_V / CH_VT * MW_TILE);
+  return chunks * heads * (long long)(sizeof(ChunkOps<128, true>) / 4 + MW_V / CH_VT * MW_TILE_G);
 }
 
-template <typename act_t, int K, bool DELTA>
+template <typename act_t, int K, bool DELTA, bool SHARED>
 static int launch_mma_walk(const b2l_seq_scan_args* a, cudaStream_t s) {
   using Ops = ChunkOps<K, DELTA>;
   auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   const int vec = a->ldq % 4 == 0 && a->ldk % 4 == 0 && al(a->q) && al(a->k) && (!a->decay_per_channel || (a->ldd % 4 == 0 && al(a->decay)));
   static DynSmemCache chunk_cache, walk_cache;
-  const size_t chunk_smem = sizeof(Ops) + sizeof(float) * 3 * CH_C * (K + 4), walk_smem = sizeof(MwSmem<K, DELTA>);
-  if (int rc = ensure_dyn_smem(seq_chunk_ops_kernel<act_t, K, DELTA>, chunk_smem, chunk_cache)) return rc;
-  if (int rc = ensure_dyn_smem(seq_walk_mma_kernel<act_t, K, DELTA>, walk_smem, walk_cache)) return rc;
-  const int seg = mma_segment(a->heads);
+  const size_t chunk_smem = sizeof(Ops) + sizeof(float) * (SHARED ? 2 : 3) * CH_C * (K + 4), walk_smem = sizeof(MwSmem<K, DELTA>);
+  if constexpr (SHARED) {
+    if (int rc = ensure_dyn_smem(seq_chunk_shared_kernel<act_t, K>, chunk_smem, chunk_cache)) return rc;
+  } else {
+    if (int rc = ensure_dyn_smem(seq_chunk_ops_kernel<act_t, K, DELTA>, chunk_smem, chunk_cache)) return rc;
+  }
+  if (int rc = ensure_dyn_smem(seq_walk_mma_kernel<act_t, K, DELTA, SHARED>, walk_smem, walk_cache)) return rc;
+  const int seg = mma_segment(a->heads), rep = a->heads / a->qk_heads, sms = sm_count();
   for (int t = 0; t < a->T; t += seg) {
     const int hi = a->T - t < seg ? a->T : t + seg, chunks = (hi - t + CH_C - 1) / CH_C;
-    const MwWork work{a->work_state, reinterpret_cast<uint32_t*>(reinterpret_cast<Ops*>(a->work_state) + (size_t)chunks * a->heads)};
-    seq_chunk_ops_kernel<act_t, K, DELTA><<<dim3((unsigned)chunks, (unsigned)a->heads), MW_CHUNK_THREADS, chunk_smem, s>>>(*a, vec, t, hi, work);
+    const MwWork work{a->work_state, reinterpret_cast<uint32_t*>(reinterpret_cast<Ops*>(a->work_state) + (size_t)chunks * (SHARED ? a->qk_heads : a->heads))};
+    if constexpr (SHARED) {
+      int per = 8;                                       // heads of a CTA: fewer where CTAs of eight leave SMs idle (8 heads, 512 tokens: 35 us with eight, 32 with two)
+      while (per > 1 && (long long)chunks * a->qk_heads * ((rep + per - 1) / per) * 8 < 7LL * sms) per /= 2;
+      seq_chunk_shared_kernel<act_t, K><<<dim3((unsigned)chunks, (unsigned)a->qk_heads, (unsigned)((rep + per - 1) / per)), MW_CHUNK_THREADS, chunk_smem, s>>>(*a, vec, t, hi, per,
+                                                                                                                                                             work);
+    } else
+      seq_chunk_ops_kernel<act_t, K, DELTA><<<dim3((unsigned)chunks, (unsigned)a->heads), MW_CHUNK_THREADS, chunk_smem, s>>>(*a, vec, t, hi, work);
     B2L_LAUNCH_CHECK("seq_chunk_ops_kernel");
-    seq_walk_mma_kernel<act_t, K, DELTA><<<dim3((unsigned)(a->V / CH_VT), (unsigned)a->heads), MW_THREADS, walk_smem, s>>>(*a, t, hi, work);
+    seq_walk_mma_kernel<act_t, K, DELTA, SHARED><<<dim3((unsigned)(a->V / CH_VT), (unsigned)a->heads), MW_THREADS, walk_smem, s>>>(*a, t, hi, work);
     B2L_LAUNCH_CHECK("seq_walk_mma_kernel");
   }
   return 0;
