@@ -2,6 +2,8 @@
 // (pre, post + residual + next pre fused), gated activations, short causal convolution with carried inputs, unit
 // norms, decay factors, grouped read-out norm with its gate.  All arithmetic is f32; `act_t` is only the storage
 // type of projection outputs and weights.
+#include <type_traits>
+
 #include "seq_common.cuh"
 
 namespace b2l {
@@ -153,14 +155,14 @@ __global__ void seq_gated_act_kernel(const act_t* __restrict__ gu, int ldgu, act
 }
 
 // Causal convolution + silu.  Thread = one channel over a tile of CONV_TT tokens with a sliding window in registers.
-// Tile 0 reads the carried inputs; with a single tile the same thread also advances the state (no race); with
-// several tiles seq_conv_state_kernel advances it in a second launch.
+// Tile 0 reads the carried inputs, and the thread that has read a channel's advances them: to its last inputs, or, where
+// the portion has several tiles (and so more tokens than taps), to the portion's (no second launch: 2.5 us of a portion).
 constexpr int CONV_TT = 32;
 constexpr int CONV_MAX_TAPS = 8;
 template <typename act_t>
 __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, const act_t* __restrict__ w,
-                                     const act_t* __restrict__ bias, act_t* __restrict__ state, const int* __restrict__ meta,
-                                     float* __restrict__ out, int ldout, int T, int C, int taps, int update_state) {
+                                     const act_t* __restrict__ bias, act_t* state, const int* __restrict__ meta,
+                                     float* __restrict__ out, int ldout, int T, int C, int taps) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const int t0 = blockIdx.y * CONV_TT, t1 = min(T, t0 + CONV_TT);
@@ -198,10 +200,10 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
       if (j == taps - 2) win[j] = cur;
     }
   }
-  if (update_state) {   // single tile: win[] now holds the last taps-1 inputs of the sequence
+  if (blockIdx.y == 0) {   // single tile: win[] now holds the last taps-1 inputs of the sequence
 #pragma unroll
     for (int j = 0; j < CONV_MAX_TAPS; ++j) {
-      if (j < taps - 1) st_act(st, (size_t)j * C + c, win[j]);
+      if (j < taps - 1) st_act(st, (size_t)j * C + c, gridDim.y == 1 ? win[j] : ld_act(in, (size_t)(T - (taps - 1) + j) * ldin + c));
     }
   }
 }
@@ -210,7 +212,8 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
 // channels (8-byte loads, one 16-byte store, 64 registers) keep twice the warps of eight on an SM: 6144 channels x 2048 tokens with the unit
 // heads 26.5 us against 30.3 (73 one channel at a time, 35 with eight channels and 16 tokens).  Eight only where a head of more than 128
 // channels is to lie in one warp.  Sums in the order of the kernel above.
-constexpr int CONV_VT = 8;
+// Portions that give the SMs fewer than eight CTAs of eight tokens go by four tokens a thread: their time is a thread's chain of loads and gates.
+constexpr int CONV_VT = 8, CONV_VT_FEW = 4;
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -231,15 +234,16 @@ template <int V> __device__ __forceinline__ void ldv_bf16(const __nv_bfloat16* p
     x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
   }
 }
-template <bool UNIT, int V>
+template <bool UNIT, int V, int VT>
 __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16* __restrict__ in, int ldin, const __nv_bfloat16* __restrict__ w,
-                                                            const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ state,
+                                                            const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* state,
                                                             const int* __restrict__ meta, float* __restrict__ out, int ldout, int T, int C, UnitHeads u) {
   const int c0 = (blockIdx.x * 128 + threadIdx.x) * V, c = min(c0, C - V);      // lanes past the last channel repeat it
   const float mult = !UNIT ? 0.f : c >= u.a0 && c < u.a1 ? u.ma : c >= u.b0 && c < u.b1 ? u.mb : 0.f;
   const bool any = UNIT && __any_sync(0xffffffffu, mult != 0.f);
-  const int t0 = blockIdx.y * CONV_VT, nt = min(CONV_VT, T - t0);
-  const __nv_bfloat16* st = state + (size_t)meta[0] * 3 * C;
+  static_assert(VT >= 3, "only the first tile may read the carried inputs, which it overwrites");
+  const int t0 = blockIdx.y * VT, nt = min(VT, T - t0);
+  __nv_bfloat16* st = state + (size_t)meta[0] * 3 * C;
   float wr[4][V], win[3][V], b[V];
 #pragma unroll
   for (int i = 0; i < V / 2; ++i) {                         // w is [channel][tap]
@@ -257,7 +261,18 @@ __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const int t = t0 - 3 + j;
-    ldv_bf16<V>(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(3 + t) * C + c, win[j]);
+    if (t >= 0 || c0 < C) ldv_bf16<V>(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(3 + t) * C + c, win[j]);
+    else                                                    // a lane that repeats the last channels stays off what their own lane writes below
+#pragma unroll
+      for (int e = 0; e < V; ++e) win[j][e] = 0.f;
+  }
+  if (blockIdx.y == 0 && c0 < C) {                          // the thread that has read the carried inputs of its channels leaves the portion's last ones
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      using Word = std::conditional_t<V == 8, uint4, uint2>;
+      const int t = T - 3 + j;                              // of fewer than three tokens: a carried input, row j is written after row T + j is read
+      *reinterpret_cast<Word*>(st + (size_t)j * C + c) = *reinterpret_cast<const Word*>(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(T + j) * C + c);
+    }
   }
 #pragma unroll 4
   for (int r = 0; r < nt; ++r) {
@@ -289,16 +304,6 @@ __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16
     o[0] = make_float4(y[0], y[1], y[2], y[3]);
     if constexpr (V == 8) o[1] = make_float4(y[4], y[5], y[6], y[7]);
   }
-}
-
-// state <- the last taps-1 inputs after T >= taps-1 new tokens (multi-tile launches only).
-template <typename act_t>
-__global__ void seq_conv_state_kernel(const act_t* __restrict__ in, int ldin, act_t* __restrict__ state,
-                                      const int* __restrict__ meta, int T, int C, int taps) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  act_t* st = state + (size_t)meta[0] * (taps - 1) * C;
-  for (int j = 0; j < taps - 1; ++j) st[(size_t)j * C + c] = in[(size_t)(T - (taps - 1) + j) * ldin + c];
 }
 
 template <typename act_t>
@@ -583,25 +588,29 @@ static int conv_silu(const void* in, int ldin, const void* w, const void* bias, 
   if (T == 0) return 0;
   const int tiles = (T + CONV_TT - 1) / CONV_TT;
   dim3 grid((unsigned)((C + 127) / 128), (unsigned)tiles);
-  if (act_dtype == B2L_BF16 && taps == 4 && T > CONV_TT && C % 8 == 0 && ldin % 8 == 0 && ldout % 4 == 0 && al16(in) && al16(w) && al16(state) && al16(out) &&
-      (T + CONV_VT - 1) / CONV_VT <= 65535) {
+  if (act_dtype == B2L_BF16 && taps == 4 && C % 8 == 0 && ldin % 8 == 0 && ldout % 4 == 0 && al16(in) && al16(w) && al16(state) && al16(out) &&
+      (T + CONV_VT - 1) / CONV_VT <= 65535) {      // with fewer CTAs than eight an SM, four tokens a thread stay below as well
     const int wide = unit && unit->size > 128 ? 8 : 4, lanes = unit ? unit->size / wide : 0;       // a head of the unit vectors lies in one warp
     const bool fits = unit && unit->size % wide == 0 && lanes >= 1 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && unit->a0 % unit->size == 0 && unit->b0 % unit->size == 0 &&
                       unit->ma != 0.f && unit->mb != 0.f;
-    const dim3 grid4((unsigned)((C / (fits ? wide : 4) + 127) / 128), (unsigned)((T + CONV_VT - 1) / CONV_VT));
-    auto kernel = !fits ? seq_conv4_silu_kernel<false, 4> : wide == 8 ? seq_conv4_silu_kernel<true, 8> : seq_conv4_silu_kernel<true, 4>;
-    kernel<<<grid4, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)state, meta, out, ldout,
+    const long long across = (C / (fits ? wide : 4) + 127) / 128;
+    const bool few = across * ((T + CONV_VT - 1) / CONV_VT) < 8LL * sm_count();
+    const int vt = few ? CONV_VT_FEW : CONV_VT;
+    const dim3 grid4((unsigned)across, (unsigned)((T + vt - 1) / vt));
+    auto pick = [&](auto n) {
+      constexpr int N = decltype(n)::value;
+      return !fits ? seq_conv4_silu_kernel<false, 4, N> : wide == 8 ? seq_conv4_silu_kernel<true, 8, N> : seq_conv4_silu_kernel<true, 4, N>;
+    };
+    auto kernel = few ? pick(std::integral_constant<int, CONV_VT_FEW>{}) : pick(std::integral_constant<int, CONV_VT>{});
+    kernel<<<grid4, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)state, meta, out, ldout,
                                                     T, C, fits ? *unit : UnitHeads{});
     if (unit_done) *unit_done = fits;
-    seq_conv_state_kernel<__nv_bfloat16><<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldin, (__nv_bfloat16*)state, meta, T, C, taps);
     B2L_LAUNCH_CHECK("seq_conv4_silu_kernel");
     return 0;
   }
   B2L_SEQ_DISPATCH(act_dtype, {
     seq_conv_silu_kernel<act_t><<<grid, 128, 0, (cudaStream_t)stream>>>((const act_t*)in, ldin, (const act_t*)w, (const act_t*)bias,
-                                                                        (act_t*)state, meta, out, ldout, T, C, taps, tiles == 1);
-    if (tiles > 1 && taps > 1)   // T > CONV_TT >= taps - 1: the new state comes from the portion alone
-      seq_conv_state_kernel<act_t><<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const act_t*)in, ldin, (act_t*)state, meta, T, C, taps);
+                                                                        (act_t*)state, meta, out, ldout, T, C, taps);
   });
   B2L_LAUNCH_CHECK("seq_conv_silu_kernel");
   return 0;
