@@ -475,6 +475,52 @@ __global__ void __launch_bounds__(256) seq_group_norm_gate_block_kernel(const fl
   }
 }
 
+// The same in bf16 where every row starts on 16 bytes: eight neighbouring channels a thread and step, NV steps kept in registers, so each gate is taken once and
+// nothing is read twice (512 tokens of 2048 channels with silu gates, device time 11.5 -> 5.6 us; their 8 MB take 1.3).
+template <int NV>
+__global__ void __launch_bounds__(256) seq_group_norm_gate_wide_kernel(const float* __restrict__ o, int ldo, const __nv_bfloat16* __restrict__ w, int w_shared,
+                                                                       const __nv_bfloat16* __restrict__ gate, int ldg, int gate_act, int gate_first, float eps,
+                                                                       float out_mult, __nv_bfloat16* __restrict__ out, int ldout, int groups, int group) {
+  __shared__ float red[32];
+  const int t = blockIdx.x / groups, g = blockIdx.x % groups;
+  const size_t at = (size_t)g * group;
+  float v[NV][8], z[NV][8], ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    const int i = (c * 256 + threadIdx.x) * 8;
+    if (i >= group) continue;
+    const float4 a = *reinterpret_cast<const float4*>(o + (size_t)t * ldo + at + i), b = *reinterpret_cast<const float4*>(o + (size_t)t * ldo + at + i + 4);
+    v[c][0] = a.x; v[c][1] = a.y; v[c][2] = a.z; v[c][3] = a.w; v[c][4] = b.x; v[c][5] = b.y; v[c][6] = b.z; v[c][7] = b.w;
+    if (gate) {
+      ld8_bf16(gate + (size_t)t * ldg + at + i, z[c]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        z[c][e] = gate_act == B2L_SEQ_ACT_SILU ? silu_f(z[c][e]) : gate_act == B2L_SEQ_ACT_SIGMOID ? sigmoid_f(z[c][e]) : gelu_tanh_f(z[c][e]);
+        if (gate_first) v[c][e] *= z[c][e];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += v[c][e] * v[c][e];
+  }
+  ss = block_sum(ss, red);
+  const float r = out_mult / sqrtf(ss / (float)group + eps);
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    const int i = (c * 256 + threadIdx.x) * 8;
+    if (i >= group) continue;
+    float x[8];
+    ld8_bf16(w + (w_shared ? 0 : at) + i, x);
+    __nv_bfloat162 y[4];
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      float p[2] = {v[c][e] * r * x[e], v[c][e + 1] * r * x[e + 1]};
+      if (gate && !gate_first) { p[0] *= z[c][e]; p[1] *= z[c][e + 1]; }
+      y[e / 2] = __floats2bfloat162_rn(p[0], p[1]);
+    }
+    *reinterpret_cast<uint4*>(out + (size_t)t * ldout + at + i) = *reinterpret_cast<const uint4*>(y);
+  }
+}
+
 // Per-head RMS norm + partial rotation.  One warp per (token, head).
 template <typename act_t, typename out_t>
 __global__ void seq_headnorm_rope_kernel(const act_t* __restrict__ x, int ldx, const act_t* __restrict__ w, float eps,
@@ -693,6 +739,14 @@ extern "C" int b2l_seq_group_norm_gate(const float* o, int ldo, const void* w, i
       B2L_LAUNCH_CHECK("seq_group_norm_gate_vec_kernel");
       return 0;
     }
+  }
+  if (act_dtype == B2L_BF16 && group >= 512 && group <= 8192 && group % 8 == 0 && ldo % 4 == 0 && ldout % 8 == 0 && al16(o) && al16(w) && al16(out) &&
+      (!gate || (ldg % 8 == 0 && al16(gate)))) {
+    auto kernel = group <= 2048 ? seq_group_norm_gate_wide_kernel<1> : group <= 4096 ? seq_group_norm_gate_wide_kernel<2> : seq_group_norm_gate_wide_kernel<4>;
+    kernel<<<ids, 256, 0, (cudaStream_t)stream>>>(o, ldo, (const __nv_bfloat16*)w, w_shared, (const __nv_bfloat16*)gate, ldg, gate_act, gate_first, eps, out_mult,
+                                                  (__nv_bfloat16*)out, ldout, n / group, group);
+    B2L_LAUNCH_CHECK("seq_group_norm_gate_wide_kernel");
+    return 0;
   }
   B2L_SEQ_DISPATCH(act_dtype, {
     if (group >= 512)

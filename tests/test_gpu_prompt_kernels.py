@@ -569,6 +569,24 @@ def test_f32_local_attention_in_three_parts(T, H, G, K, V, pos0, window, block, 
         assert rel(out[:T].view(T, H, V), want) < 2e-6 and bool((out[T] == 7).all())
 
 
+@pytest.mark.parametrize("T,n,group,gate_first,act", [(3, 2048, 2048, 1, "silu"), (2, 1032, 1032, 0, "sigmoid"), (5, 8192, 4096, 1, None), (2, 6400, 6400, 0, "silu"), (3, 1544, 772, 1, "silu")])
+def test_gated_norm_of_wide_groups(T, n, group, gate_first, act):
+    """One, two and four steps of 2048 channels, a last step that ends within the CTA, groups that do not start on 16 bytes (the form for those); one bf16 rounding of f32 sums."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(n)
+    o, w = torch.randn(T, n + 4, generator=g, device=DEV), torch.randn(group, generator=g, device=DEV).to(BF)
+    gate, out = torch.randn(T, n + 8, generator=g, device=DEV).to(BF), torch.full((T, n + 8), 7.0, device=DEV, dtype=BF)
+    S.check(S.lib().b2l_seq_group_norm_gate(o.data_ptr(), n + 4, w.data_ptr(), 1, gate.data_ptr() if act else None, n + 8, S.ACT_SILU if act == "silu" else S.ACT_SIGMOID, gate_first,
+                                            1e-6, 1.5, out.data_ptr(), n + 8, T, n, group, S.act_code(BF), S.stream_ptr()), "norm")
+    x, z = o[:, :n].double().view(T, -1, group), gate[:, :n].double().view(T, -1, group)
+    z = torch.sigmoid(z) * (z if act == "silu" else 1.0) if act else torch.ones_like(z)
+    x = x * z if gate_first else x
+    want = 1.5 * x / (x.pow(2).mean(-1, keepdim=True) + 1e-6).sqrt() * w.double() * (1.0 if gate_first else z)
+    got = out[:, :n].double().view(T, -1, group)
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()) and bool((out[:, n:] == 7).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 128, 8), (17, 130, 72), (113, 300, 64), (70, 2200, 1000), (300, 1025, 200)])
 def test_f32_linear_in_three_parts(M, N, K):
     """Token tiles of 16 to 112, ragged features, k that ends within a stage, rows apart; infinite and NaN operands come out as FMAs give them.
@@ -589,6 +607,37 @@ def test_f32_linear_in_three_parts(M, N, K):
     x[M - 1] *= 1e12
     want, got = torch.nn.functional.linear(x, w), run()
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got == math.inf, want == math.inf) and torch.equal(got == -math.inf, want == -math.inf)
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 7])
+def test_convolution_of_few_tokens_carries_its_inputs(T):
+    """Portions of fewer tokens than taps keep some of the inputs carried so far; a portion in two halves gives the same bits as in one."""
+    from lit_llama_b200 import _seqlib as S
+
+    Ch, g = 520, torch.Generator(device=DEV).manual_seed(T)
+    x, w = torch.randn(2 * T, Ch, generator=g, device=DEV).to(BF), torch.randn(Ch, 4, generator=g, device=DEV).to(BF)
+    first, meta = torch.randn(2, 3, Ch, generator=g, device=DEV).to(BF), torch.tensor([1, 0], dtype=torch.int32, device=DEV)
+
+    def run(parts):
+        state, outs = first.clone(), []
+        for p in parts:
+            out = torch.empty(p.shape[0], Ch, device=DEV)
+            S.check(S.lib().b2l_seq_conv_silu_unit(p.data_ptr(), Ch, w.data_ptr(), None, state.data_ptr(), meta.data_ptr(), out.data_ptr(), Ch, p.shape[0], Ch, 4, 0, 128, 2, 64, 1e-6,
+                                                   0.5, 1.0, S.act_code(BF), S.stream_ptr()), "convolution")
+            outs.append(out)
+        return torch.cat(outs), state
+
+    whole, state = run([x])
+    halves, state2 = run([x[:T], x[T:]])
+    assert torch.equal(whole, halves) and torch.equal(state, state2) and torch.equal(state[0], first[0])
+    assert torch.equal(state[1], torch.cat([first[1], x])[-3:])
+    full = torch.cat([first[1], x]).double()
+    want = sum(full[j:j + 2 * T] * w[:, j].double() for j in range(4))
+    want = want * torch.sigmoid(want)
+    for at, m in ((0, 0.5), (128, 1.0)):
+        h = want[:, at:at + 128].view(2 * T, 2, 64)
+        want[:, at:at + 128] = (m * h / (h.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()).view(2 * T, 128)
+    assert rel(whole, want) < 1e-6
 
 
 @pytest.mark.parametrize("T,G,K,bias", [(33, 3, 64, True), (50, 2, 128, False), (20, 2, 128, False), (40, 1, 256, True), (35, 2, 48, False)])
