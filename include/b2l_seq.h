@@ -224,6 +224,8 @@ int b2l_seq_cast_f32(const void* in, int ldin, float* out, int ldout, int T, int
 
 /* Zero one slot of a state tensor laid out [n_slots][slot_bytes]. */
 int b2l_seq_zero_slot(void* state, size_t slot_bytes, int slot, b2l_stream_t stream);
+/* The same for n tensors, in one launch for every 16 of them (host arrays, read before the call returns). */
+int b2l_seq_zero_slots(void* const* states, const size_t* slot_bytes, int n, int slot, b2l_stream_t stream);
 
 /* A stream of the current device that nothing else uses (torch hands out 32 in turn): what a graph is recorded on. */
 int b2l_seq_stream_create(void** stream);

@@ -164,6 +164,7 @@ _SIGS = {
     "b2l_seq_cast_f32": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "b2l_seq_stream_create": (c_int, [C.POINTER(c_void_p)]),
     "b2l_seq_zero_slot": (c_int, [c_void_p, c_size_t, c_int, c_void_p]),
+    "b2l_seq_zero_slots": (c_int, [C.POINTER(c_void_p), C.POINTER(c_size_t), c_int, c_int, c_void_p]),
     "b2l_seq_add_norm2": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_float, c_void_p, c_int,
                                   c_int, c_int, c_void_p]),
     "b2l_seq_softcap": (c_int, [c_void_p, c_size_t, c_float, c_void_p]),

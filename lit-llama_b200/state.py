@@ -6,6 +6,7 @@ tensor `[n_slots, *shape]` per spec, hands slots to requests, zeroes what must s
 taken (a slot that another request used before is as good as a fresh one), and keeps the position of every
 sequence.  Kernels address a slot through the device int32 pair {slot, position} (`meta`), so a captured step
 replays for any slot."""
+import ctypes as C
 from dataclasses import dataclass
 from typing import Dict, Hashable, List, Tuple
 
@@ -58,10 +59,11 @@ class SequenceStatePool:
         if not self._free:
             raise PoolFull(f"all {self.n_slots} state slots are in use")
         slot = self._free.pop()
-        for name, sp in self.specs.items():
-            if sp.zero_on_acquire:
-                t = self.tensors[name]
-                S.check(S.lib().b2l_seq_zero_slot(t.data_ptr(), t[0].numel() * t.element_size(), slot, S.stream_ptr()), "b2l_seq_zero_slot")
+        zeroed = [self.tensors[name] for name, sp in self.specs.items() if sp.zero_on_acquire]
+        if zeroed:
+            n = len(zeroed)
+            S.check(S.lib().b2l_seq_zero_slots((C.c_void_p * n)(*[t.data_ptr() for t in zeroed]), (C.c_size_t * n)(*[t.nbytes // self.n_slots for t in zeroed]), n, slot,
+                                               S.stream_ptr()), "b2l_seq_zero_slots")
         self._slot_of[request_id] = slot
         self._pos[slot] = 0
         self.acquired += 1

@@ -587,6 +587,18 @@ def test_gated_norm_of_wide_groups(T, n, group, gate_first, act):
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()) and bool((out[:, n:] == 7).all())
 
 
+def test_slots_are_zeroed_at_once():
+    """Seventeen tensors of a slot: more than a launch takes, words and odd sizes, empty ones; the neighbouring slots stay."""
+    from lit_llama_b200 import _seqlib as S
+
+    sizes = [16, 48, 33, 0, 4096 * 16, 2, 1 << 20] + [32 * (i + 1) for i in range(12)]
+    pools = [torch.full((3, n), 5, dtype=torch.uint8, device=DEV) for n in sizes]
+    n = len(pools)
+    S.check(S.lib().b2l_seq_zero_slots((C.c_void_p * n)(*[t.data_ptr() or None for t in pools]), (C.c_size_t * n)(*sizes), n, 1, S.stream_ptr()), "zero")
+    for t in pools:
+        assert bool((t[1] == 0).all()) and bool((t[0] == 5).all()) and bool((t[2] == 5).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 128, 8), (17, 130, 72), (113, 300, 64), (70, 2200, 1000), (300, 1025, 200)])
 def test_f32_linear_in_three_parts(M, N, K):
     """Token tiles of 16 to 112, ragged features, k that ends within a stage, rows apart; infinite and NaN operands come out as FMAs give them.
