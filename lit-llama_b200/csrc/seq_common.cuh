@@ -13,6 +13,18 @@ template <typename T> __device__ __forceinline__ void st_act(T* p, size_t i, flo
 template <> __device__ __forceinline__ void st_act<__nv_bfloat16>(__nv_bfloat16* p, size_t i, float v) { p[i] = __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ void st_act<float>(float* p, size_t i, float v) { p[i] = v; }
 
+// Four elements at once, p aligned to all four of them.
+__device__ __forceinline__ float4 ld_act4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ld_act4(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void st_act4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void st_act4(__nv_bfloat16* p, float4 v) {
+  const __nv_bfloat162 y[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+  *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(y);
+}
+
 // x / y for y >= 1/4 without a branch: the approximate reciprocal (at most 1 ulp off, as documented), one Newton step, and the quotient corrected by its own
 // remainder (Markstein).  While 1/y is a normal number, so for y up to 2^126, that is the correctly rounded quotient, subnormal ones as well: 2 in 10^8 are 1
 // ulp off, over all mantissas of y and reciprocals off by up to 1 ulp.  Four gated outputs in a row took the attention kernel 730 cycles with the
@@ -83,6 +95,8 @@ __device__ __forceinline__ float row_dot(const act_t* __restrict__ w, const floa
   return warp_sum(acc);
 }
 
+// whether p may be read by fours of elements of `size` bytes
+static inline bool al4(const void* p, size_t size) { return (reinterpret_cast<uintptr_t>(p) & (4 * size - 1)) == 0; }
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Calls `fn.template operator()<T>()` with the element type of act_dtype.

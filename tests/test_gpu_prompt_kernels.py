@@ -587,6 +587,79 @@ def test_gated_norm_of_wide_groups(T, n, group, gate_first, act):
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()) and bool((out[:, n:] == 7).all())
 
 
+@pytest.mark.parametrize("D,off", [(4, 0), (1020, 0), (1024, 4), (1028, 0), (2052, 0), (4096, 0), (4100, 0), (1022, 0), (1024, 1)])
+@pytest.mark.parametrize("dt", [BF, torch.float32])
+def test_rows_by_fours(D, off, dt):
+    """Embedding, norms and cast: fours at the end of each width, widths and starts (`off` elements in) that have none (the other forms).  One rounding of f32
+    sums of D squares: 2^-8 of a bf16 output, D 2^-24 at most of an f32 one (4e-6 for the rounding of its square root and products below that)."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(D + off)
+    T, V, code, st, lib = 5, 11, S.act_code(dt), S.stream_ptr(), S.lib()
+
+    def rows(n, t=dt):
+        return torch.randn(n * D + off, generator=g, device=DEV).to(t)[off:].view(n, D)
+
+    def near(got, want, mag=None):
+        tol = (2.0 ** -8 if got.dtype == BF else max(4e-6, D * 2.0 ** -24)) * (want.abs() if mag is None else mag)
+        return bool(((got.double() - want).abs() <= tol + 1e-6).all())
+
+    def norm(t):
+        return t * (t.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt()
+
+    table, tok = rows(V), torch.tensor([3, 0, 10, 7, 3], device=DEV)
+    x, h = rows(T, torch.float32), rows(T)
+    S.check(lib.b2l_seq_embed(tok.data_ptr(), 1, table.data_ptr(), code, 1.5, x.data_ptr(), h.data_ptr(), T, D, V, st), "embed")
+    want = table[tok].float() * 1.5
+    assert torch.equal(x, want) and torch.equal(h, want.to(dt))
+    w, wn, y, pick = rows(1)[0], rows(1)[0], rows(T), torch.tensor([4, 1], dtype=torch.int32, device=DEV)
+    S.check(lib.b2l_seq_rmsnorm(x.data_ptr(), w.data_ptr(), 1e-6, h.data_ptr(), pick.data_ptr(), 2, D, code, st), "rmsnorm")
+    assert near(h[:2], norm(x[pick.long()].double()) * w.double())
+    x0, add = x.double(), 0.7 * norm(y.double()) * w.double()
+    S.check(lib.b2l_seq_norm_add_norm(y.data_ptr(), w.data_ptr(), 1e-6, 0.7, x.data_ptr(), wn.data_ptr(), h.data_ptr(), T, D, code, st), "norm_add_norm")
+    assert near(x, x0 + add, x0.abs() + add.abs()) and near(h, norm(x0 + add) * wn.double(), (norm(x0.abs() + add.abs()) * wn.double()).abs() * 1.5)
+    out = torch.full((T, D + 4), 7.0, device=DEV)
+    S.check(lib.b2l_seq_cast_f32(y.data_ptr(), D, out.data_ptr(), D + 4, T, D, code, st), "cast")
+    assert torch.equal(out[:, :D], y.float()) and bool((out[:, D:] == 7).all())
+
+
+@pytest.mark.parametrize("rq,rk,dr,rot,inter,off", [(4, 512, 0, 0, 0, 0), (516, 20, 8, 4, 1, 0), (1028, 512, 64, 64, 0, 0), (2048, 2048, 4, 2, 1, 0), (2052, 4, 4, 4, 0, 0), (768, 510, 64, 64, 1, 0), (768, 512, 64, 64, 1, 1)])
+@pytest.mark.parametrize("dt", [BF, torch.float32])
+def test_latent_rows_by_fours(rq, rk, dr, rot, inter, off, dt):
+    """Each number of fours a thread, ranks and starts that have none (the other form), positions past the cache left alone.  Tolerances as for the norms
+    above; a rotated entry is two products of angles below 400, themselves 2^-15 off as f32 (256 <= angle < 512): 4e-5 of the pair."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(rq + rk)
+    T, pos0, max_pos, ld = 6, 300, 304, rq + rk + dr + 4
+    proj = torch.randn(T * ld + off, generator=g, device=DEV)[off:].view(T, ld)
+    wq, wk = torch.randn(rq, generator=g, device=DEV).to(dt), torch.randn(rk, generator=g, device=DEV).to(dt)
+    freq, meta = torch.rand(max(rot // 2, 1), generator=g, device=DEV), torch.tensor([1, pos0], dtype=torch.int32, device=DEV)
+    cq, cache = torch.full((T, rq), 7.0, device=DEV, dtype=dt), torch.full((3, max_pos, rk + dr), 7.0, device=DEV, dtype=dt)
+    S.check(S.lib().b2l_seq_latent_prep(proj.data_ptr(), ld, 0, rq, wq.data_ptr(), cq.data_ptr(), rq, rk, wk.data_ptr(), dr, freq.data_ptr(), rot, inter, 1.25, 1e-6,
+                                        meta.data_ptr(), cache.data_ptr(), max_pos, T, S.act_code(dt), S.stream_ptr()), "latent_prep")
+    p, n = proj.double(), max_pos - pos0
+
+    def near(got, want, mag, eps):
+        return bool(((got.double() - want).abs() <= (2.0 ** -8 if dt == BF else 0.0) * want.abs() + eps * mag + 1e-6).all())
+
+    def norm(t):
+        return t * (t.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt()
+
+    want = norm(p[:, :rq]) * wq.double()
+    assert near(cq, want, want.abs(), max(4e-6, rq * 2.0 ** -24))
+    want = (norm(p[:, rq:rq + rk]) * wk.double())[:n]
+    assert near(cache[1, pos0:, :rk], want, want.abs(), max(4e-6, rk * 2.0 ** -24))
+    k = p[:n, rq + rk:rq + rk + dr].clone()
+    if rot:
+        a, b = (slice(0, rot, 2), slice(1, rot, 2)) if inter else (slice(0, rot // 2), slice(rot // 2, rot))
+        ang = torch.arange(pos0, max_pos, device=DEV, dtype=torch.float64)[:, None] * freq[:rot // 2].double()
+        u, v = k[:, a].clone(), k[:, b].clone()
+        k[:, a], k[:, b] = 1.25 * (u * ang.cos() - v * ang.sin()), 1.25 * (v * ang.cos() + u * ang.sin())
+    assert near(cache[1, pos0:, rk:], k, 8.0, 4e-5)
+    assert bool((cache[0] == 7).all() and (cache[2] == 7).all() and (cache[1, :pos0] == 7).all())
+
+
 def test_slots_are_zeroed_at_once():
     """Seventeen tensors of a slot: more than a launch takes, words and odd sizes, empty ones; the neighbouring slots stay."""
     from lit_llama_b200 import _seqlib as S
