@@ -22,6 +22,8 @@ LIBRARIES = {
     # the quantized linears' entry points as Python functions (a CPython extension, host code only; the stable ABI of 3.10 on, so one file for every
     # interpreter).  The package runs without it, see _lib.py
     "pycall": dict(out=os.path.join(PKG, "_pycall.abi3.so"), sources=["pycall.cpp"], headers=[os.path.join(ROOT, "include", "b2l.h")]),
+    # the same for the sequence kernels' functions, see _seqlib.py
+    "seqcall": dict(out=os.path.join(PKG, "_seqcall.abi3.so"), sources=["seqcall.cpp"], headers=[os.path.join(ROOT, "include", h) for h in ("b2l_seq.h", "b2l.h")]),
     # sequence-mixer kernels: recurrences, local and latent attention, expert routing, f32 residual streams (include/b2l_seq.h)
     "seq": dict(out=os.path.join(PKG, "libb200seq.so"),
                 sources=["seq_api.cu", "seq_elementwise.cu", "seq_scan.cu", "seq_attention.cu", "seq_latent.cu", "seq_moe.cu", "seq_streams.cu",

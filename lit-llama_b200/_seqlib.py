@@ -2,6 +2,7 @@
 first use when it is missing (only this library, not the quantized-LLaMA one).  No CPU or PyTorch fallback."""
 import ctypes as C
 import threading
+import types
 
 import torch
 
@@ -227,8 +228,29 @@ def lib():
                     fn = getattr(handle, name)
                     fn.restype = res
                     fn.argtypes = args
-                _lib = handle
+                _lib = _functions(handle)
     return _lib
+
+
+def _functions(handle) -> types.SimpleNamespace:
+    """The library's functions by name: those of csrc/seqcall.cpp where its file lies there and knows them, else ctypes' (some 3 us more a call).  Like the
+    quantized linears' extension it is never built here."""
+    import importlib.machinery
+    import importlib.util
+
+    out = {name: getattr(handle, name) for name in _SIGS}
+    try:
+        spec = importlib.util.spec_from_loader("_seqcall", importlib.machinery.ExtensionFileLoader("_seqcall", _build.LIBRARIES["seqcall"]["out"]))
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except ImportError:
+        return types.SimpleNamespace(**out)
+    codes = {c_void_p: "p", c_int: "i", c_float: "f", C.c_longlong: "q", c_size_t: "z"}
+    for name, (res, args) in _SIGS.items():
+        if res is c_int and all(a in codes for a in args):
+            made = module.make(name, C.cast(out[name], c_void_p).value, out[name], "".join(codes[a] for a in args))
+            out[name] = made if made is not None else out[name]
+    return types.SimpleNamespace(**out)
 
 
 def check(rc: int, what: str) -> None:

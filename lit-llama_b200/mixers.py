@@ -73,7 +73,7 @@ def _p(t: Optional[torch.Tensor], offset: int = 0) -> Optional[int]:
     """Device address of element `offset` of a tensor's storage view."""
     if t is None:
         return None
-    return S.ptr(t) + offset * t.element_size()
+    return S.ptr(t) + offset * t.element_size() if offset else S.ptr(t)
 
 
 def pad8(n: int) -> int:

@@ -89,3 +89,41 @@ def test_the_extension_is_optional_and_never_built_by_a_call(L, monkeypatch):
         L._bind(handle)
     assert type(L.pycall) is type(built)
     assert _build._headers(_build.LIBRARIES["pycall"]) == [HEADER] and _build.LIBRARIES["pycall"]["out"].endswith(".abi3.so")
+
+
+def test_sequence_functions_take_what_ctypes_takes(monkeypatch):
+    """csrc/seqcall.cpp's functions against the ctypes functions they stand for: the same answers and messages for arguments that convert, that ctypes truncates
+    or unwraps, and the same refusals; without the file, and with another signature, ctypes'.  No call gets as far as a launch."""
+    from lit_llama_b200 import _build
+    from lit_llama_b200 import _seqlib as S
+
+    lib, handle = S.lib(), C.CDLL(_build.LIBRARIES["seq"]["out"])
+    made = [n for n in S.EXPORTS if type(getattr(lib, n)).__name__ == "builtin_function_or_method"]
+    if not os.path.exists(_build.LIBRARIES["seqcall"]["out"]):
+        assert not made
+        pytest.skip("the extension is not built")
+    assert len(made) == sum(S._SIGS[n][0] is C.c_int and bool(S._SIGS[n][1]) and all(a in (C.c_void_p, C.c_int, C.c_float, C.c_longlong, C.c_size_t) for a in S._SIGS[n][1])
+                            for n in S.EXPORTS if n not in ("b2l_seq_scan_chunks", "b2l_seq_latent_attention_warps", "b2l_seq_mingru_chunks"))
+    for n in made:
+        slow, (slow.restype, slow.argtypes) = getattr(handle, n), S._SIGS[n]
+
+        def outcome(f, args):
+            try:
+                return f(*args), lib.b2l_seq_last_error()
+            except (TypeError, C.ArgumentError) as e:
+                return type(e)
+
+        args = [None if a is C.c_void_p else 0.5 if a is C.c_float else 0 for a in S._SIGS[n][1]]
+        first, ints = S._SIGS[n][1].index(C.c_void_p), [i for i, a in enumerate(S._SIGS[n][1]) if a is C.c_int]
+        calls = [args, args[:-1], args + [0], [C.c_void_p(None) if i == first else a for i, a in enumerate(args)], ["x" if i == first else a for i, a in enumerate(args)]]
+        for v in (-1, True, 2 ** 31 - 1, 2 ** 32, -2 ** 40, 2 ** 70, 1.0, None):
+            calls.append([v if ints and i == ints[-1] else a for i, a in enumerate(args)])
+        calls.append([1 if a == 0.5 else a for a in args])
+        for c in calls:
+            assert outcome(getattr(lib, n), c) == outcome(slow, c), (n, c)
+        with pytest.raises(TypeError):
+            getattr(lib, n)(*args[:-1], stream=0)
+    monkeypatch.setitem(S._SIGS, "b2l_seq_norm", (C.c_int, S._SIGS["b2l_seq_norm"][1] + [C.c_int]))
+    assert type(S._functions(handle).b2l_seq_norm) is not type(lib.b2l_seq_norm)
+    monkeypatch.setitem(_build.LIBRARIES["seqcall"], "out", "/nonexistent/_seqcall.abi3.so")
+    assert type(S._functions(handle).b2l_seq_rope) is not type(lib.b2l_seq_rope)
