@@ -309,6 +309,10 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
 // heads 26.5 us against 30.3 (73 one channel at a time, 35 with eight channels and 16 tokens).  Eight only where a head of more than 128
 // channels is to lie in one warp.  Sums in the order of the kernel above.
 // Portions that give the SMs fewer than eight CTAs of eight tokens go by four tokens a thread: their time is a thread's chain of loads and gates.
+// A thread takes four tokens at once, the next four requested before: each token by itself waited for its load, its gates and, with unit heads, five
+// exchanges, a root and a quotient in every lane; for four tokens together a lane adds up one token's squares and takes its root alone.  us, token by token /
+// by fours, unit heads of 128: 6144 channels x 2048 tokens 25.4 / 22.6, 3072 x 512 6.1 / 5.2, x 9 4.9 / 3.6; without heads 3072 x 9 3.7 / 3.2, but
+// 6144 x 2048 19.2 / 19.9 (80 registers), so those go token by token, as do heads of fewer than four lanes.
 constexpr int CONV_VT = 8, CONV_VT_FEW = 4;
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
@@ -370,35 +374,103 @@ __global__ void __launch_bounds__(128) seq_conv4_silu_kernel(const __nv_bfloat16
       *reinterpret_cast<Word*>(st + (size_t)j * C + c) = *reinterpret_cast<const Word*>(t >= 0 ? in + (size_t)t * ldin + c : st + (size_t)(T + j) * C + c);
     }
   }
+  if (UNIT ? u.size < 4 * V : VT == CONV_VT) {               // token by token: heads of one or two lanes, and long portions without heads
 #pragma unroll 4
-  for (int r = 0; r < nt; ++r) {
-    float cur[V], y[V];
-    ldv_bf16<V>(in + (size_t)(t0 + r) * ldin + c, cur);
+    for (int r = 0; r < nt; ++r) {
+      float cur[V], y[V];
+      ldv_bf16<V>(in + (size_t)(t0 + r) * ldin + c, cur);
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      float acc = b[e];
-      acc += wr[0][e] * win[0][e];
-      acc += wr[1][e] * win[1][e];
-      acc += wr[2][e] * win[2][e];
-      acc += wr[3][e] * cur[e];
-      y[e] = silu_f(acc);
-      win[0][e] = win[1][e];
-      win[1][e] = win[2][e];
-      win[2][e] = cur[e];
+      for (int e = 0; e < V; ++e) {
+        float acc = b[e];
+        acc += wr[0][e] * win[0][e];
+        acc += wr[1][e] * win[1][e];
+        acc += wr[2][e] * win[2][e];
+        acc += wr[3][e] * cur[e];
+        y[e] = silu_f(acc);
+        win[0][e] = win[1][e];
+        win[1][e] = win[2][e];
+        win[2][e] = cur[e];
+      }
+      if (any) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < V; ++e) ss += y[e] * y[e];
+        if (u.size > V) ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        const float f = mult != 0.f ? mult / sqrtf(ss + u.eps) : 1.f;
+#pragma unroll
+        for (int e = 0; e < V; ++e) y[e] *= f;
+      }
+      float4* o = reinterpret_cast<float4*>(out + (size_t)(t0 + r) * ldout + c);
+      if (c0 >= C) continue;
+      o[0] = make_float4(y[0], y[1], y[2], y[3]);
+      if constexpr (V == 8) o[1] = make_float4(y[4], y[5], y[6], y[7]);
     }
+    return;
+  }
+  // four tokens at a time, the next four on their way meanwhile
+  using Word = std::conditional_t<V == 8, uint4, uint2>;
+  const __nv_bfloat16* row = in + (size_t)t0 * ldin + c;
+  float* o = out + (size_t)t0 * ldout + c;
+  Word raw[4];
+  auto fetch = [&](int from) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      raw[r] = from + r < nt ? *reinterpret_cast<const Word*>(row + (size_t)(from + r) * ldin) : Word{};
+  };
+  fetch(0);
+#pragma unroll 1
+  for (int r0 = 0; r0 < nt; r0 += 4) {
+    float cur[4][V], y[4][V] = {};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) ldv_bf16<V>(reinterpret_cast<const __nv_bfloat16*>(&raw[r]), cur[r]);
+    fetch(r0 + 4);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (VT == CONV_VT_FEW && (r == 1 || r == 2) && nt == r) break;
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        float acc = b[e];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc += wr[j][e] * (r + j < 3 ? win[r + j][e] : cur[r + j - 3][e]);
+        y[r][e] = silu_f(acc);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) win[j][e] = cur[1 + j][e];
     if (any) {
-      float ss = 0.f;
+      float ss[4];
 #pragma unroll
-      for (int e = 0; e < V; ++e) ss += y[e] * y[e];
-      for (int d = 1; d < u.size / V; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-      const float f = mult != 0.f ? mult / sqrtf(ss + u.eps) : 1.f;
+      for (int r = 0; r < 4; ++r) {
+        ss[r] = 0.f;
 #pragma unroll
-      for (int e = 0; e < V; ++e) y[e] *= f;
+        for (int e = 0; e < V; ++e) ss[r] += y[r][e] * y[r][e];
+      }
+      float f[4];
+      // a lane adds up one token's squares, and takes its root
+      const bool odd = threadIdx.x & 1, high = threadIdx.x & 2;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) ss[r] = (odd ? ss[r + 2] : ss[r]) + __shfl_xor_sync(0xffffffffu, odd ? ss[r] : ss[r + 2], 1);
+      float all = (high ? ss[1] : ss[0]) + __shfl_xor_sync(0xffffffffu, high ? ss[0] : ss[1], 2);
+      for (int d = 4; d < u.size / V; d <<= 1) all += __shfl_xor_sync(0xffffffffu, all, d);
+      all = mult != 0.f ? mult / sqrtf(all + u.eps) : 1.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) f[r] = __shfl_sync(0xffffffffu, all, (r >> 1) | (r & 1) << 1, 4);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int e = 0; e < V; ++e) y[r][e] *= f[r];
     }
-    float4* o = reinterpret_cast<float4*>(out + (size_t)(t0 + r) * ldout + c);
-    if (c0 >= C) continue;
-    o[0] = make_float4(y[0], y[1], y[2], y[3]);
-    if constexpr (V == 8) o[1] = make_float4(y[4], y[5], y[6], y[7]);
+    if (c0 < C) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (r0 + r < nt) {
+          float4* q = reinterpret_cast<float4*>(o + (size_t)(r0 + r) * ldout);
+          q[0] = make_float4(y[r][0], y[r][1], y[r][2], y[r][3]);
+          if constexpr (V == 8) q[1] = make_float4(y[r][4], y[r][5], y[r][6], y[r][7]);
+        }
+    }
   }
 }
 

@@ -750,6 +750,13 @@ def test_convolution_with_unit_heads(T, G, K, bias):
     assert torch.equal(state[1], xs[-3:].to(BF))
 
 
+@pytest.mark.parametrize("T,G,K,bias", [(1, 2, 16, True), (2, 3, 64, False), (3, 2, 128, True), (6, 3, 8, True), (9, 5, 4, False), (1597, 16, 64, True), (1602, 12, 128, False), (1599, 8, 256, True),
+                                        (3003, 100, 8, False)])
+def test_convolution_of_unit_heads_by_fours(T, G, K, bias):
+    """Tiles of four and of eight tokens with every remainder, heads of four lanes and more (their roots shared out) and of fewer (token by token)."""
+    test_convolution_with_unit_heads(T, G, K, bias)
+
+
 @pytest.mark.parametrize("size,mode", [(8, 0), (24, 1), (128, 0), (128, 1)])
 def test_decays_of_eight_channels(size, mode):
     """exp(-exp(A) softplus(z + b)) and sigmoid(z)^(1/tau) in groups of 8 channels, from -100 to 100 and at infinity.  The exponent e carries the sum's
