@@ -623,6 +623,19 @@ def test_rows_by_fours(D, off, dt):
     assert torch.equal(out[:, :D], y.float()) and bool((out[:, D:] == 7).all())
 
 
+@pytest.mark.parametrize("C_,off", [(8, 0), (2040, 0), (2048, 8), (4104, 0), (12288, 0), (2044, 0), (13, 0), (4096, 1)])
+@pytest.mark.parametrize("wide", [torch.int64, torch.int32])
+def test_embedding_rows_are_copied(C_, off, wide):
+    """Rows of one and several 16-byte rounds a thread, rows and starts that have none; tokens outside the table read row 0."""
+    from lit_llama_b200 import _lib as L
+
+    V, idx = 9, torch.tensor([3, 8, 0, -1, 9, 3], device=DEV, dtype=wide)
+    table = torch.randn(V * C_ + off, device=DEV).to(BF)[off:].view(V, C_)
+    out = torch.full((7 * C_ + off,), 7.0, device=DEV, dtype=BF)[off:].view(7, C_)
+    L.check(L.lib().b2l_embedding(idx.data_ptr(), int(wide is torch.int64), table.data_ptr(), out.data_ptr(), 6, C_, V, L.stream_ptr()), "embedding")
+    assert torch.equal(out[:6], table[[3, 8, 0, 0, 0, 3]]) and bool((out[6] == 7).all())
+
+
 @pytest.mark.parametrize("rq,rk,dr,rot,inter,off", [(4, 512, 0, 0, 0, 0), (516, 20, 8, 4, 1, 0), (1028, 512, 64, 64, 0, 0), (2048, 2048, 4, 2, 1, 0), (2052, 4, 4, 4, 0, 0), (768, 510, 64, 64, 1, 0), (768, 512, 64, 64, 1, 1)])
 @pytest.mark.parametrize("dt", [BF, torch.float32])
 def test_latent_rows_by_fours(rq, rk, dr, rot, inter, off, dt):
