@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
 
 // The same in bf16 where whole heads turn and a row has one factor: four neighbouring pairs (u: 16 bytes of x) are a unit, a thread holds NU of the
 // token's units in registers, so x is read once, with its norm weights for all of the CTA's tokens, and the next token's x travels meanwhile.
-// Bound by the chain from launch to store: a token per CTA, each waiting for its angles and then for x, took 14.3 us for 2048 tokens of 16 + 4
-// heads of 128 with norms; four tokens per CTA 10.0.
+// Bound by the chain from launch to store, a barrier for the norms and the angles in it: 2048 tokens of 16 + 4 heads of 128 with norms take 9.1 us, their bytes
+// 4.8.
 constexpr int QUAD_THREADS = 512;
 template <int NU>
 __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_seq_qkv_prep_args a, int tokens) {
@@ -494,9 +494,16 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   // tokens 10 / 14, 256 17 / 16, 2048 65 / 47; 32768 with norms, 2048 tokens 114 / 122).
   const bool norms = a->q_norm || a->k_norm, held = units <= 4 * QUAD_THREADS || (units <= 8 * QUAD_THREADS && (a->T <= sm_count() * (norms ? 2 : 1) || (norms && units >= 7 * QUAD_THREADS)));
   if (quads && held) {
-    // tokens per CTA: up to four where two CTAs per SM are left (the angles of a CTA come at once, its tokens' x one ahead), as far as their angles fit
-    const int fill = a->T / (2 * sm_count()), tokens = a->K > 2048 ? 1 : fill < 1 ? 1 : fill > 4 ? 4 : fill;
-    const int nu = units <= QUAD_THREADS / 2 ? 1 : units <= QUAD_THREADS ? 2 : units <= 4 * QUAD_THREADS ? 4 : 8;
+    // Tokens per CTA: one until the tokens' threads no longer fit the SMs at once (some 1000 an SM, two units each), then two, whose angles come together and the
+    // second of which is on its way early; four only for rows of more than 768 units, of which an SM holds two CTAs.  As far as their angles fit, and two CTAs
+    // an SM.  us by 1 / 2 / 4 tokens, heads of 128 with norms: 600 tokens of 16 + 4 heads 4.3 / 5.1 / 7.2, 1024 6.0 / 5.7 / 7.5, 2048 9.1 / 9.1 / 9.4; 1024 of 8 + 2
+    // 4.0 / 4.9 / 6.7, 4096 10.2 / 9.9 / 10.3; 2048 of 32 + 8 15.1 / 14.1 / 16.2, of 40 + 8 20.2 / 18.6 / 18.0.
+    const int fill = a->T / (2 * sm_count());
+    const bool many = a->T * units > 2000LL * sm_count();
+    const int tokens = a->K > 2048 || fill < 2 || !many ? 1 : units > 768 && fill >= 4 ? 4 : 2;
+    // Units per thread: two, but one for the shortest rows and few tokens (160 units: 512 tokens 3.4 / 3.5, 600 3.8 / 3.6, 4096 11.2 / 9.9; 40: 3.9 / 4.2); four
+    // from 384 on where tokens are many (480, 2048 tokens: 11.9 / 10.6; 320 9.1 / 10.0) and otherwise where they have to.
+    const int nu = units <= 64 || (units <= QUAD_THREADS / 2 && a->T < 4 * sm_count()) ? 1 : units <= (many ? 384 : QUAD_THREADS) ? 2 : units <= 4 * QUAD_THREADS ? 4 : 8;
     const int threads = (int)((units + 32 * nu - 1) / (32 * nu)) * 32;
     auto kernel = nu == 1 ? seq_qkv_prep_quads_kernel<1> : nu == 2 ? seq_qkv_prep_quads_kernel<2> : nu == 4 ? seq_qkv_prep_quads_kernel<4> : seq_qkv_prep_quads_kernel<8>;
     kernel<<<(a->T + tokens - 1) / tokens, threads, sizeof(float) * a->K * tokens, (cudaStream_t)stream>>>(*a, tokens);
