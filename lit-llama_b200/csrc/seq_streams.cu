@@ -273,21 +273,38 @@ __global__ void __launch_bounds__(256) seq_qkv_prep_kernel(b2l_seq_qkv_prep_args
   }
 }
 
-// The same in bf16 where whole heads turn and a row has one factor: four neighbouring pairs (u: 16 bytes of x) are a unit, a thread holds NU of the
+// The same where whole heads turn and a row has one factor: four neighbouring pairs (u: 16 bytes of x in bf16) are a unit, a thread holds NU of the
 // token's units in registers, so x is read once, with its norm weights for all of the CTA's tokens, and the next token's x travels meanwhile.
 // Bound by the chain from launch to store, a barrier for the norms and the angles in it: 2048 tokens of 16 + 4 heads of 128 with norms take 9.1 us, their bytes
 // 4.8.
 constexpr int QUAD_THREADS = 512;
-template <int NU>
+// four elements as they lie in memory
+template <typename act_t> struct Quad;
+template <> struct Quad<__nv_bfloat16> {
+  uint2 v;
+  __device__ __forceinline__ void ones() { v = make_uint2(0x3f803f80u, 0x3f803f80u); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ float operator[](int e) const {
+    const uint32_t w = e & 2 ? v.y : v.x;
+    return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
+  }
+};
+template <> struct Quad<float> {
+  float4 v;
+  __device__ __forceinline__ void ones() { v = make_float4(1.f, 1.f, 1.f, 1.f); }
+  __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ float operator[](int e) const { return e & 2 ? (e & 1 ? v.w : v.z) : (e & 1 ? v.y : v.x); }
+};
+template <typename act_t, int NU>
 __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_seq_qkv_prep_args a, int tokens) {
   __shared__ float red[2][2][QUAD_THREADS / 32];
   extern __shared__ __align__(16) float turn_quads[];   // per token: cos | sin of the pairs, times rot_mult
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
   const int K = a.K, half = K / 2, per = half / 4, units_q = a.heads * per, units = units_q + a.kv_heads * per;
   const int t0 = blockIdx.x * tokens, nt = min(tokens, a.T - t0);
-  const __nv_bfloat16* qw = (const __nv_bfloat16*)a.q_norm;
-  const __nv_bfloat16* kw = (const __nv_bfloat16*)a.k_norm;
-  uint2 x0[NU], x1[NU], w0[NU], w1[NU];
+  const act_t* qw = (const act_t*)a.q_norm;
+  const act_t* kw = (const act_t*)a.k_norm;
+  Quad<act_t> x0[NU], x1[NU], w0[NU], w1[NU];
   int at[NU], xat[NU];                                  // first entry of the unit: in its row of heads, in the projection's row
 #pragma unroll
   for (int i = 0; i < NU; ++i) {
@@ -296,19 +313,24 @@ __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_se
     xat[i] = at[i] + (u < units_q ? a.q_off : a.k_off);
   }
   auto load = [&](int t) {
-    const __nv_bfloat16* row = (const __nv_bfloat16*)a.proj + (size_t)t * a.ld;
+    const act_t* row = (const act_t*)a.proj + (size_t)t * a.ld;
 #pragma unroll
     for (int i = 0; i < NU; ++i) {
-      x0[i] = *reinterpret_cast<const uint2*>(row + xat[i]);
-      x1[i] = *reinterpret_cast<const uint2*>(row + xat[i] + half);
+      x0[i].load(row + xat[i]);
+      x1[i].load(row + xat[i] + half);
     }
   };
   load(t0);
 #pragma unroll
   for (int i = 0; i < NU; ++i) {
-    const __nv_bfloat16* w = tid + i * (int)blockDim.x < units_q ? qw : kw;
-    w0[i] = w ? *reinterpret_cast<const uint2*>(w + at[i]) : make_uint2(0x3f803f80u, 0x3f803f80u);
-    w1[i] = w ? *reinterpret_cast<const uint2*>(w + at[i] + half) : make_uint2(0x3f803f80u, 0x3f803f80u);
+    const act_t* w = tid + i * (int)blockDim.x < units_q ? qw : kw;
+    if (w) {
+      w0[i].load(w + at[i]);
+      w1[i].load(w + at[i] + half);
+    } else {
+      w0[i].ones();
+      w1[i].ones();
+    }
   }
   const int pos0 = a.meta[1] + t0;
   for (int i = tid; i < nt * half; i += blockDim.x) {
@@ -318,8 +340,6 @@ __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_se
     turn_quads[n * K + j] = c * a.rot_mult;
     turn_quads[n * K + half + j] = s * a.rot_mult;
   }
-  auto lo16 = [](uint32_t v) { return __uint_as_float(v << 16); };
-  auto hi16 = [](uint32_t v) { return __uint_as_float(v & 0xffff0000u); };
   for (int n = 0; n < nt; ++n) {
     const int t = t0 + n;
     float rq = 1.f, rk = 1.f;
@@ -328,10 +348,11 @@ __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_se
 #pragma unroll
       for (int i = 0; i < NU; ++i) {
         const int u = tid + i * (int)blockDim.x;
-        const uint32_t w[4] = {x0[i].x, x0[i].y, x1[i].x, x1[i].y};
         float ss = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ss += lo16(w[e]) * lo16(w[e]) + hi16(w[e]) * hi16(w[e]);
+        for (int e = 0; e < 4; e += 2) ss += x0[i][e] * x0[i][e] + x0[i][e + 1] * x0[i][e + 1];
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) ss += x1[i][e] * x1[i][e] + x1[i][e + 1] * x1[i][e + 1];
         if (u < units_q) sq += ss;
         else if (u < units) sk += ss;
       }
@@ -356,11 +377,9 @@ __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_se
       const int j = at[i] % K;                          // the unit's first pair
       const float4 c4 = *reinterpret_cast<const float4*>(tn + j), s4 = *reinterpret_cast<const float4*>(tn + half + j);
       const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
-      const uint32_t ux[4] = {x0[i].x, x0[i].y, x1[i].x, x1[i].y}, uw[4] = {w0[i].x, w0[i].y, w1[i].x, w1[i].y};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const uint32_t xu = ux[e >> 1], wu = uw[e >> 1], xv = ux[2 + (e >> 1)], wv = uw[2 + (e >> 1)];
-        const float pu = (e & 1 ? hi16(xu) : lo16(xu)) * r * (e & 1 ? hi16(wu) : lo16(wu)), pv = (e & 1 ? hi16(xv) : lo16(xv)) * r * (e & 1 ? hi16(wv) : lo16(wv));
+        const float pu = x0[i][e] * r * w0[i][e], pv = x1[i][e] * r * w1[i][e];
         y[i][e] = pu * c[e] - pv * s[e];
         y[i][4 + e] = pv * c[e] + pu * s[e];
       }
@@ -374,19 +393,16 @@ __global__ void __launch_bounds__(QUAD_THREADS) seq_qkv_prep_quads_kernel(b2l_se
         *reinterpret_cast<float4*>(qo) = make_float4(y[i][0] * temp, y[i][1] * temp, y[i][2] * temp, y[i][3] * temp);
         *reinterpret_cast<float4*>(qo + half) = make_float4(y[i][4] * temp, y[i][5] * temp, y[i][6] * temp, y[i][7] * temp);
       } else if (u < units) {
-        __nv_bfloat16* ko = (__nv_bfloat16*)a.k_out + (size_t)t * a.kv_heads * K + at[i];
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const __nv_bfloat162 y0 = __floats2bfloat162_rn(y[i][4 * b], y[i][4 * b + 1]), y1 = __floats2bfloat162_rn(y[i][4 * b + 2], y[i][4 * b + 3]);
-          *reinterpret_cast<uint2*>(ko + b * half) = make_uint2(*reinterpret_cast<const uint32_t*>(&y0), *reinterpret_cast<const uint32_t*>(&y1));
-        }
+        act_t* ko = (act_t*)a.k_out + (size_t)t * a.kv_heads * K + at[i];
+        st_act4(ko, make_float4(y[i][0], y[i][1], y[i][2], y[i][3]));
+        st_act4(ko + half, make_float4(y[i][4], y[i][5], y[i][6], y[i][7]));
       }
     }
     if (a.v_first != nullptr) {
-      const float lam = ld_act((const __nv_bfloat16*)a.lambda, 0);
-      const __nv_bfloat16* v = (const __nv_bfloat16*)a.proj + (size_t)t * a.ld + a.v_off;
-      const __nv_bfloat16* vf = (const __nv_bfloat16*)a.v_first + (size_t)t * a.ldvf;
-      __nv_bfloat16* vo = (__nv_bfloat16*)a.v_out + (size_t)t * a.kv_heads * a.V;
+      const float lam = ld_act((const act_t*)a.lambda, 0);
+      const act_t* v = (const act_t*)a.proj + (size_t)t * a.ld + a.v_off;
+      const act_t* vf = (const act_t*)a.v_first + (size_t)t * a.ldvf;
+      act_t* vo = (act_t*)a.v_out + (size_t)t * a.kv_heads * a.V;
       for (int i = tid; i < a.kv_heads * a.V; i += blockDim.x) st_act(vo, i, (1.f - lam) * ld_act(v, i) + lam * ld_act(vf, i));
     }
   }
@@ -483,16 +499,18 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
   B2L_CHECK_ARG(a->temp_every >= 0, "b2l_seq_qkv_prep: negative temperature step");
   B2L_CHECK_ARG(!a->unit_rms || (a->q_norm == nullptr && a->k_norm == nullptr), "b2l_seq_qkv_prep: the norm after the rotation has no weight");
   if (a->T == 0) return 0;
-  auto al8 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; };
+  const size_t es = a->act_dtype == B2L_F32 ? 4 : 2;
   // whole heads turn, in groups of four pairs, and no factor per head; both norms or none, so that both rows take the same form
   const bool table = a->rot_dims / 2 <= MOST_PAIRS;
-  const int quads = table && a->act_dtype == B2L_BF16 && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
-                    a->k_off % 4 == 0 && a->ld % 4 == 0 && al8(a->proj) && al8(a->q_norm) && al8(a->k_norm) && al16(a->q_out) && al8(a->k_out);
+  const int quads = table && (a->act_dtype == B2L_BF16 || a->act_dtype == B2L_F32) && a->rot_dims == a->K && a->K % 8 == 0 && !a->unit_rms && (a->whole_row || (!a->q_norm && !a->k_norm)) && a->q_off % 4 == 0 &&
+                    a->k_off % 4 == 0 && a->ld % 4 == 0 && al4(a->proj, es) && al4(a->q_norm, es) && al4(a->k_norm, es) && al16(a->q_out) && al4(a->k_out, es);
   const long long units = (long long)(a->heads + a->kv_heads) * (a->K / 8);
   // Rows of more than 32768 entries do not fit a CTA's registers.  From 16384 on they take eight units a thread, at 128 registers with spills: faster where
   // few CTAs wait for one another's loads (us, registers / a pass per row: 17408 entries with norms, 1 token 12 / 23, 256 18 / 23, 2048 82 / 68; without, 16
   // tokens 10 / 14, 256 17 / 16, 2048 65 / 47; 32768 with norms, 2048 tokens 114 / 122).
-  const bool norms = a->q_norm || a->k_norm, held = units <= 4 * QUAD_THREADS || (units <= 8 * QUAD_THREADS && (a->T <= sm_count() * (norms ? 2 : 1) || (norms && units >= 7 * QUAD_THREADS)));
+  // In f32 a unit takes twice the registers: rows of up to 8192 entries.  us, a pass per row / so, 8 + 2 heads of 128 with norms: 1 token
+  // 4.6 / 2.8, 777 6.6 / 3.8, 2048 12.5 / 8.1; 2048 of 48 + 8 64 / 40.
+  const bool norms = a->q_norm || a->k_norm, held = a->act_dtype == B2L_F32 ? units <= 2 * QUAD_THREADS : units <= 4 * QUAD_THREADS || (units <= 8 * QUAD_THREADS && (a->T <= sm_count() * (norms ? 2 : 1) || (norms && units >= 7 * QUAD_THREADS)));
   if (quads && held) {
     // Tokens per CTA: one until the tokens' threads no longer fit the SMs at once (some 1000 an SM, two units each), then two, whose angles come together and the
     // second of which is on its way early; four only for rows of more than 768 units, of which an SM holds two CTAs.  As far as their angles fit, and two CTAs
@@ -503,9 +521,11 @@ extern "C" int b2l_seq_qkv_prep(const b2l_seq_qkv_prep_args* a, b2l_stream_t str
     const int tokens = a->K > 2048 || fill < 2 || !many ? 1 : units > 768 && fill >= 4 ? 4 : 2;
     // Units per thread: two, but one for the shortest rows and few tokens (160 units: 512 tokens 3.4 / 3.5, 600 3.8 / 3.6, 4096 11.2 / 9.9; 40: 3.9 / 4.2); four
     // from 384 on where tokens are many (480, 2048 tokens: 11.9 / 10.6; 320 9.1 / 10.0) and otherwise where they have to.
-    const int nu = units <= 64 || (units <= QUAD_THREADS / 2 && a->T < 4 * sm_count()) ? 1 : units <= (many ? 384 : QUAD_THREADS) ? 2 : units <= 4 * QUAD_THREADS ? 4 : 8;
+    const int nu = units <= 64 || (units <= QUAD_THREADS / 2 && a->T < 4 * sm_count()) ? 1 : units <= (many ? 384 : QUAD_THREADS) || a->act_dtype == B2L_F32 ? 2 : units <= 4 * QUAD_THREADS ? 4 : 8;
     const int threads = (int)((units + 32 * nu - 1) / (32 * nu)) * 32;
-    auto kernel = nu == 1 ? seq_qkv_prep_quads_kernel<1> : nu == 2 ? seq_qkv_prep_quads_kernel<2> : nu == 4 ? seq_qkv_prep_quads_kernel<4> : seq_qkv_prep_quads_kernel<8>;
+    auto kernel = nu == 1 ? seq_qkv_prep_quads_kernel<__nv_bfloat16, 1> : nu == 2 ? seq_qkv_prep_quads_kernel<__nv_bfloat16, 2>
+                  : nu == 4 ? seq_qkv_prep_quads_kernel<__nv_bfloat16, 4> : seq_qkv_prep_quads_kernel<__nv_bfloat16, 8>;
+    if (a->act_dtype == B2L_F32) kernel = nu == 1 ? seq_qkv_prep_quads_kernel<float, 1> : seq_qkv_prep_quads_kernel<float, 2>;
     kernel<<<(a->T + tokens - 1) / tokens, threads, sizeof(float) * a->K * tokens, (cudaStream_t)stream>>>(*a, tokens);
     B2L_LAUNCH_CHECK("seq_qkv_prep_quads_kernel");
     return 0;

@@ -372,6 +372,16 @@ def test_attention_operands_by_quads_of_pairs(T, H, G, K, norms, mix):
         assert bool(((v.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
 
 
+@pytest.mark.parametrize("T,H,G,K,norms,mix", [(1, 16, 4, 128, "qk", True), (1187, 2, 1, 16, "qk", False), (777, 8, 2, 128, "qk", True), (900, 3, 2, 24, "k", True), (700, 16, 4, 128, "", True),
+                                               (9, 40, 8, 128, "q", True), (5, 130, 6, 128, "qk", False)])
+def test_attention_operands_by_quads_of_pairs_in_f32(T, H, G, K, norms, mix, monkeypatch):
+    """The same in float32: one and two units per thread, rows too long for that; the queries hold the tolerance above without a bf16 rounding."""
+    import sys
+
+    monkeypatch.setattr(sys.modules[__name__], "BF", torch.float32)
+    test_attention_operands_by_quads_of_pairs(T, H, G, K, norms, mix)
+
+
 @pytest.mark.parametrize("T,H,K,V,want", [(2048, 4, 128, 128, "chunks"), (2048, 8, 64, 64, "chunks"), (300, 1, 128, 16, "walk"), (2048, 16, 128, 128, "walk"), (257, 64, 128, 64, "walk"),
                                           (47, 2, 64, 32, "steps"), (48, 2, 64, 32, "walk"), (63, 64, 64, 64, "steps"), (64, 64, 64, 64, "walk")])
 def test_scan_plan_and_its_neighbours(T, H, K, V, want):
