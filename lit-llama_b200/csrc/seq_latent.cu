@@ -46,6 +46,60 @@ __global__ void seq_rope_kernel(const in_t* __restrict__ x, int ldx, const float
   for (int i = off + rot_dims + lane; i < size; i += 32) st_act(q, i, ld_act(p, i) * mult);
 }
 
+// The same where a lane has one or two (P) of the pairs: a warp takes four heads of a token, its angles once and all loads of the four before them, what does not
+// turn by fours of entries.  The form above is bound by its issue slots, an angle per pair and head among them: 2048 tokens of 16 heads of 128 + 64 turned entries
+// 8.1 us, 5.6 so, of 8 heads 4.9 / 3.6, of 32 heads of 64 turned 12.1 / 6.3; with few heads and tokens its shorter chain is what counts (16 heads of 128 + 64, 1
+// token 1.7 / 2.0, 300 2.6 / 2.7, 777 4.2 / 3.3; 8 heads, 300 tokens 2.2 / 2.5, 777 2.9 / 2.7), hence the launch's line of 40 heads an SM.
+template <typename in_t, typename out_t, int P>
+__global__ void __launch_bounds__(128) seq_rope_heads_kernel(const in_t* x, int ldx, const float* __restrict__ freq, int rot_dims, int interleaved, int off, float mult,
+                                                             float rot_mult, const int* __restrict__ meta, out_t* out, int ldo, int n_rows, int heads, int size,
+                                                             int hsx, int hso) {
+  const int groups = (heads + 3) / 4, id = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, t = id / groups, h0 = (id - t * groups) * 4;
+  if (t >= n_rows) return;
+  const int half = rot_dims / 2, n = min(4, heads - h0), plain = (size - rot_dims) / 4;
+  const in_t* p = x + (size_t)t * ldx + (size_t)h0 * hsx;
+  out_t* q = out + (size_t)t * ldo + (size_t)h0 * hso;
+  float u[4][P], v[4][P], c[P], s[P];
+  int iu[P], iv[P];
+#pragma unroll
+  for (int j = 0; j < P; ++j) {
+    const int i = min(lane + 32 * j, half - 1);
+    iu[j] = off + (interleaved ? 2 * i : i);
+    iv[j] = off + (interleaved ? 2 * i + 1 : i + half);
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (h < n) {
+        u[h][j] = ld_act(p + (size_t)h * hsx, iu[j]);
+        v[h][j] = ld_act(p + (size_t)h * hsx, iv[j]);
+      }
+  }
+  for (int f = lane; f < plain; f += 32) {
+    const int e = 4 * f < off ? 4 * f : 4 * f + rot_dims;
+    float4 y[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (h < n) y[h] = ld_act4(p + (size_t)h * hsx + e);
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (h < n) st_act4(q + (size_t)h * hso + e, make_float4(y[h].x * mult, y[h].y * mult, y[h].z * mult, y[h].w * mult));
+  }
+  const float pos = (float)(meta[1] + t);
+#pragma unroll
+  for (int j = 0; j < P; ++j) {
+    const int i = lane + 32 * j;
+    if (i >= half) break;
+    sincosf(pos * freq[i], &s[j], &c[j]);
+    s[j] *= rot_mult;
+    c[j] *= rot_mult;
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (h < n) {
+        st_act(q + (size_t)h * hso, iu[j], (u[h][j] * c[j] - v[h][j] * s[j]) * mult);
+        st_act(q + (size_t)h * hso, iv[j], (v[h][j] * c[j] + u[h][j] * s[j]) * mult);
+      }
+  }
+}
+
 // One CTA per token of the portion, on the f32 product [W_dq ; W_dkv] h:
 //   cq  = rmsnorm(proj[q_off : q_off + q_rank]) * wq                       -> cq (act), input of the query up-projection
 //   c   = rmsnorm(proj[kv_off : kv_off + rank]) * wkv                      -> cache[slot][pos][0 : rank]
@@ -743,15 +797,23 @@ extern "C" int b2l_seq_rope(const void* x, int ldx, int in_f32, const float* fre
   if (T == 0) return 0;
   const int ids = T * heads, grid = (ids + 3) / 4;
   cudaStream_t st = (cudaStream_t)stream;
+  const size_t isz = in_f32 || act_dtype == B2L_F32 ? 4 : 2, osz = out_f32 || act_dtype == B2L_F32 ? 4 : 2;
+  const bool by_heads = (long long)T * heads >= 40LL * sm_count() && rot_dims >= 2 && rot_dims <= 128 && rot_dims % 4 == 0 && rot_off % 4 == 0 && size % 4 == 0 && hsx % 4 == 0 && hso % 4 == 0 && ldx % 4 == 0 &&
+                        ldo % 4 == 0 && al4(x, isz) && al4(out, osz) && (size_t)T * ((heads + 3) / 4) < (1ull << 31);
+  const int warps = (int)(by_heads ? (size_t)T * ((heads + 3) / 4) : 0);
+#define B2L_ROPE_ARGS(IN, OUT) (const IN*)x, ldx, freq, rot_dims, interleaved, rot_off, mult, rot_mult, meta, (OUT*)out, ldo, T, heads, size, hsx, hso
 #define B2L_ROPE_GO(IN, OUT) \
-  seq_rope_kernel<IN, OUT><<<grid, 128, 0, st>>>((const IN*)x, ldx, freq, rot_dims, interleaved, rot_off, mult, rot_mult, meta, (OUT*)out, ldo, T, heads, size, hsx, hso)
+  if (by_heads && rot_dims <= 64) seq_rope_heads_kernel<IN, OUT, 1><<<(warps + 3) / 4, 128, 0, st>>>(B2L_ROPE_ARGS(IN, OUT)); \
+  else if (by_heads) seq_rope_heads_kernel<IN, OUT, 2><<<(warps + 3) / 4, 128, 0, st>>>(B2L_ROPE_ARGS(IN, OUT)); \
+  else seq_rope_kernel<IN, OUT><<<grid, 128, 0, st>>>(B2L_ROPE_ARGS(IN, OUT))
   B2L_SEQ_DISPATCH(act_dtype, {
-    if (in_f32 && out_f32) B2L_ROPE_GO(float, float);
-    else if (in_f32) B2L_ROPE_GO(float, act_t);
-    else if (out_f32) B2L_ROPE_GO(act_t, float);
-    else B2L_ROPE_GO(act_t, act_t);
+    if (in_f32 && out_f32) { B2L_ROPE_GO(float, float); }
+    else if (in_f32) { B2L_ROPE_GO(float, act_t); }
+    else if (out_f32) { B2L_ROPE_GO(act_t, float); }
+    else { B2L_ROPE_GO(act_t, act_t); }
   });
 #undef B2L_ROPE_GO
+#undef B2L_ROPE_ARGS
   B2L_LAUNCH_CHECK("seq_rope_kernel");
   return 0;
 }

@@ -683,6 +683,31 @@ def test_latent_rows_by_fours(rq, rk, dr, rot, inter, off, dt):
     assert bool((cache[0] == 7).all() and (cache[2] == 7).all() and (cache[1, :pos0] == 7).all())
 
 
+@pytest.mark.parametrize("T,H,size,off,rot,inter,apart", [(1200, 5, 192, 128, 64, 0, 0), (1000, 7, 132, 4, 128, 1, 4), (6000, 1, 64, 0, 60, 0, 0), (1500, 4, 72, 64, 4, 1, 8), (900, 8, 136, 0, 132, 0, 0),
+                                                          (1500, 4, 72, 2, 64, 0, 0), (30, 4, 192, 128, 64, 1, 0)])
+@pytest.mark.parametrize("src,dst", [(BF, torch.float32), (torch.float32, torch.float32), (BF, BF)])
+def test_rotation_of_four_heads_a_warp(T, H, size, off, rot, inter, apart, src, dst):
+    """One and two pairs a lane, entries before and after the turned ones, the last warp's fewer heads; more pairs, odd offsets and few tokens (the other form).
+    Angles below 0.1 (T + 10) rounded to 2^-24 of themselves, products and sums 2^-22: 1e-5 and T 2^-27 of the largest entry, and a bf16 output's rounding."""
+    from lit_llama_b200 import _seqlib as S
+
+    g = torch.Generator(device=DEV).manual_seed(T + size)
+    hs = size + apart
+    x, freq = torch.randn(T, H * hs, generator=g, device=DEV).to(src), torch.rand(rot // 2, generator=g, device=DEV) * 0.1
+    meta, out = torch.tensor([0, 10], dtype=torch.int32, device=DEV), torch.full((T, H * hs), 7.0, device=DEV, dtype=dst)
+    S.check(S.lib().b2l_seq_rope(x.data_ptr(), H * hs, int(src is torch.float32), freq.data_ptr(), rot, inter, off, 0.5, 1.1, meta.data_ptr(), out.data_ptr(), H * hs,
+                                 int(dst is torch.float32), T, H, size, hs, hs, S.act_code(BF), S.stream_ptr()), "rope")
+    want = x.double().view(T, H, hs)[..., :size].clone()
+    a, b = (slice(off, off + rot, 2), slice(off + 1, off + rot, 2)) if inter else (slice(off, off + rot // 2), slice(off + rot // 2, off + rot))
+    ang = torch.arange(10, T + 10, device=DEV).double()[:, None, None] * freq.double()
+    u, v = want[..., a].clone(), want[..., b].clone()
+    want[..., a], want[..., b] = 1.1 * (u * ang.cos() - v * ang.sin()), 1.1 * (v * ang.cos() + u * ang.sin())
+    want *= 0.5
+    got = out.view(T, H, hs)
+    tol = (1e-5 + T * 2.0 ** -27) * float(want.abs().max()) + (2.0 ** -8 * want.abs() if dst is BF else 0.0)
+    assert bool(((got[..., :size].double() - want).abs() <= tol).all()) and bool((got[..., size:] == 7).all())
+
+
 def test_slots_are_zeroed_at_once():
     """Seventeen tensors of a slot: more than a launch takes, words and odd sizes, empty ones; the neighbouring slots stay."""
     from lit_llama_b200 import _seqlib as S
