@@ -597,6 +597,12 @@ def test_gated_norm_of_wide_groups(T, n, group, gate_first, act):
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()) and bool((out[:, n:] == 7).all())
 
 
+@pytest.mark.parametrize("T,n,gate_first,act", [(2100, 512, 1, "silu"), (1037, 1024, 0, "sigmoid"), (700, 2048, 1, None), (1500, 768, 0, "silu")])
+def test_gated_norm_of_four_groups_a_warp(T, n, gate_first, act):
+    """Four, eight and sixteen groups of 128 a token, the last CTA's fewer warps; six groups (the form of one a warp); the tolerance of the wide groups."""
+    test_gated_norm_of_wide_groups(T, n, 128, gate_first, act)
+
+
 @pytest.mark.parametrize("D,off", [(4, 0), (1020, 0), (1024, 4), (1028, 0), (2052, 0), (4096, 0), (4100, 0), (1022, 0), (1024, 1)])
 @pytest.mark.parametrize("dt", [BF, torch.float32])
 def test_rows_by_fours(D, off, dt):
