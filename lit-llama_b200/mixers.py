@@ -272,12 +272,6 @@ class ChannelDeltaMixer:
         self.w_conv, _ = stack_rows([W[p + "q.conv"], W[p + "k.conv"], W[p + "v.conv"]])
         assert self.w_conv.shape == (self.C, conv)
         self.w_a2, self.w_g2 = W[p + "a2"].contiguous(), W[p + "g2"].contiguous()
-        # both low-rank products in one, [a2 0; 0 g2] over the columns from a1 to the end of g1, while that is as cheap as two launches: 2048 tokens of 16 heads
-        # of 128, ranks of 64: 12 us as two products, 9 as one; 512 tokens of 8 heads 8 and 5
-        self.n_low, self.w_low = self.o_g1 - self.o_a1 + self.rank_g, None
-        if self.n_low <= 256:
-            self.w_low = self.w_a2.new_zeros((heads * dim + heads * vdim, self.n_low))
-            self.w_low[:heads * dim, :self.rank_a], self.w_low[heads * dim:, self.o_g1 - self.o_a1:] = self.w_a2, self.w_g2
         self.dt_bias, self.A_log, self.w_norm = W[p + "dt_bias"].contiguous(), W[p + "A_log"].contiguous(), W[p + "norm"].contiguous()
         self.w_o = W[p + "o"].contiguous()
 
@@ -288,27 +282,21 @@ class ChannelDeltaMixer:
     def forward(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         lib, T, dev = S.lib(), ctx.T, h.device
         proj = linear(h, self.w_in)                                         # [T, n_in]
-        if self.w_low is not None:
-            a = gate = linear(proj[:, self.o_a1:self.o_a1 + self.n_low], self.w_low)      # [T, H*K + H*V]
-            lda, gate_at = self.H * (self.K + self.V), self.H * self.K
-            ldg = lda
-        else:
-            a = linear(proj[:, self.o_a1:self.o_a1 + self.rank_a], self.w_a2)             # [T, H*K]
-            gate = linear(proj[:, self.o_g1:self.o_g1 + self.rank_g], self.w_g2)          # [T, H*V]
-            lda, ldg, gate_at = self.H * self.K, self.H * self.V, 0
+        a = linear(proj[:, self.o_a1:self.o_a1 + self.rank_a], self.w_a2)    # [T, H*K]
+        gate = linear(proj[:, self.o_g1:self.o_g1 + self.rank_g], self.w_g2)  # [T, H*V]
         qkv = torch.empty((T, self.C), dtype=torch.float32, device=dev)
         S.check(lib.b2l_seq_conv_silu_unit(_p(proj), self.n_in, _p(self.w_conv), None, _p(ctx.state[self.name + ".conv"]), _p(ctx.meta), _p(qkv), self.C, T,
                                            self.C, self.taps, self.o_q, self.o_k, self.G, self.K, self.unit_eps, self.K ** -0.5, 1.0, ctx.act, ctx.stream),
                 "b2l_seq_conv_silu_unit")
         g = torch.empty((T, self.H * self.K), dtype=torch.float32, device=dev)
-        S.check(lib.b2l_seq_decay(_p(a), lda, _p(self.dt_bias), _p(self.A_log), S.DECAY_EXP_SOFTPLUS, 0.0, _p(g), None, T,
+        S.check(lib.b2l_seq_decay(_p(a), self.H * self.K, _p(self.dt_bias), _p(self.A_log), S.DECAY_EXP_SOFTPLUS, 0.0, _p(g), None, T,
                                   self.H, self.K, ctx.act, ctx.stream), "b2l_seq_decay")
         o = torch.empty((T, self.H * self.V), dtype=torch.float32, device=dev)
         _scan(ctx, q=_p(qkv, self.o_q), ldq=self.C, k=_p(qkv, self.o_k), ldk=self.C, v=_p(qkv, self.o_v), ldv=self.C,
               q_mult=1.0, decay=_p(g), ldd=self.H * self.K, per_channel=True, beta=_p(proj, self.o_b), ldb=self.n_in,
               state=ctx.state[self.name + ".S"], out=_p(o), ldo=self.H * self.V, heads=self.H, qk_heads=self.G, K=self.K, V=self.V)
         y = torch.empty((T, self.H * self.V), dtype=h.dtype, device=dev)
-        S.check(lib.b2l_seq_group_norm_gate(_p(o), self.H * self.V, _p(self.w_norm), 1, _p(gate, gate_at), ldg, S.ACT_SIGMOID, 0, self.eps,
+        S.check(lib.b2l_seq_group_norm_gate(_p(o), self.H * self.V, _p(self.w_norm), 1, _p(gate), self.H * self.V, S.ACT_SIGMOID, 0, self.eps,
                                             1.0, _p(y), self.H * self.V, T, self.H * self.V, self.V, ctx.act, ctx.stream), "b2l_seq_group_norm_gate")
         return linear(y, self.w_o)
 

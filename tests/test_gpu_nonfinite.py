@@ -128,3 +128,66 @@ def test_llama_prompt_attention(bad):
     L.check(lib.b2l_attention(mine.data_ptr(), ck.data_ptr(), cv.data_ptr(), rope.data_ptr(), pos.data_ptr(), ring.data_ptr(), y.data_ptr(), work.data_ptr(), 1, T, nh, hs, S, S, 0,
                               L.stream_ptr()), "attention")
     same(y, attend_seen(q, k, v, hs ** -0.5, pos[None] <= pos[:, None]), 2.0 ** -8)
+
+
+def _delta_layer(W, h, D, H, K):
+    from lit_llama_b200 import mixers as X
+    from lit_llama_b200.state import SequenceStatePool
+
+    m = X.ChannelDeltaMixer("a", W, "a.", heads=H, kv_heads=H, dim=K, vdim=K, conv=4, eps=1e-6)
+    pool = SequenceStatePool(m.state_specs(), 1, torch.device(DEV))
+
+    def run():
+        slot = pool.acquire("r")
+        y = m.forward(h, X.StepContext(h.shape[0], torch.zeros(2, dtype=torch.int32, device=DEV), pool.tensors, BF, pos_hint=0, slot_hint=slot))
+        pool.release("r")
+        return y, {n: t.clone() for n, t in pool.tensors.items()}
+
+    return run
+
+
+def _delta_weights(g, D, H, K, rank_a, rank_g):
+    def lin(o, i):
+        return (torch.randn(o, i, generator=g, device=DEV) * i ** -0.5).to(BF)
+
+    W = {"a." + n: lin(o, i) for n, o, i in (("q", H * K, D), ("k", H * K, D), ("v", H * K, D), ("b", H, D), ("a1", rank_a, D), ("a2", H * K, rank_a), ("g1", rank_g, D),
+                                             ("g2", H * K, rank_g), ("o", D, H * K))}
+    for n in "qkv":
+        W[f"a.{n}.conv"] = lin(H * K, 4)
+    W["a.A_log"], W["a.dt_bias"], W["a.norm"] = lin(H, 4)[:, 0].contiguous(), lin(H * K, 4)[:, 0].contiguous(), lin(K, 4)[:, 0] + 1
+    return W
+
+
+@pytest.mark.parametrize("path,ranks", [("g1", (64, 64)), ("a1", (64, 64)), ("g1", (20, 36)), ("a1", (36, 20)), ("a1", (160, 136))])
+def test_delta_layer_keeps_decay_and_gate_apart(path, ranks):
+    """An infinite entry of the gate's inner projection reaches that token's gate only: the state and every other token keep their bits.  One of the decays'
+    makes decays of 0 and 1, and no gate NaN."""
+    D, H, K, T, at = 256, 2, 64, 90, 40
+    g = torch.Generator(device=DEV).manual_seed(ranks[0])
+    W, h = _delta_weights(g, D, H, K, *ranks), torch.randn(T, D, generator=g, device=DEV).to(BF)
+    for n in ("q", "k", "v", "b", "a1", "g1"):
+        W["a." + n][:, 0] = 0                                           # channel 0 feeds the bad entry alone
+    for n in ("a2", "g2"):
+        W["a." + n][W["a." + n] == 0] = 0.5                             # infinity times zero would be NaN by right
+    h[:, 0] = 0
+    h[at, 0] = 1e4
+    clean, state = _delta_layer(W, h, D, H, K)()
+    W["a." + path][3, 0] = 3e38                                         # the product's only infinite entry: token `at`, number 3
+    got, st = _delta_layer(W, h, D, H, K)()
+    assert bool(clean.isfinite().all()) and bool(got.isfinite().all()) and bool(st["a.S"].isfinite().all())
+    assert torch.equal(got[:at], clean[:at]) and not torch.equal(got[at], clean[at])
+    if path == "g1":
+        assert torch.equal(got[at + 1:], clean[at + 1:]) and all(torch.equal(st[n], state[n]) for n in st)
+
+
+def test_delta_layer_follows_its_second_factors():
+    """a2 and g2 are read where the caller keeps them: changed in place, the next call sees them."""
+    D, H, K = 256, 2, 64
+    g = torch.Generator(device=DEV).manual_seed(5)
+    W, h = _delta_weights(g, D, H, K, 64, 64), torch.randn(20, D, generator=g, device=DEV).to(BF)
+    run = _delta_layer(W, h, D, H, K)
+    before, _ = run()
+    for n in ("a2", "g2"):
+        W["a." + n].mul_(-2)
+    (got, st), (want, st_want) = run(), _delta_layer(W, h, D, H, K)()
+    assert torch.equal(got, want) and torch.equal(st["a.S"], st_want["a.S"]) and not torch.equal(got, before)
