@@ -20,6 +20,7 @@
 // 128 x 64 with one decay per head and no delta rule 56 / 44; 2048 and 4096 tokens of 4 heads without it 118 / 81, 224 / 153.
 // With both in f32 FMAs a chunk's products read 0.5 words of shared memory per FMA, 1300 + 750 cycles where the FMAs are 770.
 #pragma once
+#include "seq_walk_schedule.h"
 #include "tc_common.cuh"
 
 namespace b2l {
@@ -658,8 +659,6 @@ __device__ __noinline__ void walk_redo(const b2l_seq_scan_args& a, int t_lo, int
 }
 
 
-
-
 // tokens t_lo .. t_hi - 1.  SHARED: operands of seq_chunk_shared_kernel; a head's decays are in its tiles
 template <typename act_t, int K, bool DELTA, bool SHARED>
 __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_args a, int t_lo, int t_hi, MwWork work) {
@@ -784,24 +783,17 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
                      "l"(tile + (size_t)n * a.heads * gridDim.x * WORDS), "r"((uint32_t)(4 * WORDS)), "r"(bar) : "memory");
       }
     };
-    int ahead = 0, sta = 0, sti = 0;
-    uint32_t ph = 0;
-    for (; ahead < STAGES - 1 && ahead < n_chunks; ++ahead, ++sta) copy(ahead, sta);
-    for (int n = 0; n < n_chunks; ++n) {
-      mbar_wait_warp(smem_u32(sm.bars + sti), ph, dead);
-      bar_arrive(FULL + sti, WT + 32);
-      if (++sti == STAGES) { sti = 0; ph ^= 1u; }
-      if (ahead < n_chunks) {
-        if (ahead >= STAGES) bar_sync(EMPTY + sta, 96);
-        copy(ahead, sta);
-        ++ahead;
-        if (++sta == STAGES) sta = 0;
-      }
-    }
-    for (int n = max(0, ahead - STAGES); dead && n < ahead; ++n) {      // no copy outlives the CTA
-      uint32_t late = 0;
-      mbar_wait(smem_u32(sm.bars + n % STAGES), (uint32_t)(n / STAGES) & 1u, late);
-    }
+    walk_operands<STAGES>(
+        n_chunks, [&](int n) { copy(n, n % STAGES); },
+        [&](int n) {
+          mbar_wait_warp(smem_u32(sm.bars + n % STAGES), (uint32_t)(n / STAGES) & 1u, dead);
+          return !dead;
+        },
+        [&](int n) { bar_arrive(FULL + n % STAGES, WT + 32); }, [&](int n) { bar_sync(EMPTY + n % STAGES, 96); },
+        [&](int n) {
+          uint32_t late = 0;
+          mbar_wait(smem_u32(sm.bars + n % STAGES), (uint32_t)(n / STAGES) & 1u, late);
+        });
   } else if (warp < MW_WARPS + 3) {
     // ===================== outputs: 8 tokens of a chunk each, beside what the chunk kernel wrote =====================
     const int ow = warp - MW_WARPS - 1;
@@ -841,7 +833,7 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
       for (int r = 0; r < 2; ++r)
         if (j >= at0 && j < at0 + UN) {
           const int col = g + 8 * r, ch = warp * WC + 8 * (j - at0) + 2 * t4;
-          *reinterpret_cast<float2*>(redo ? fin + col * K + ch : st + (size_t)(v0 + col) * K + ch) = gone ? make_float2(lost, lost) : make_float2(S[j][2 * r], S[j][2 * r + 1]);
+          *reinterpret_cast<float2*>(walk_state_to_scratch(redo, gone) ? fin + col * K + ch : st + (size_t)(v0 + col) * K + ch) = gone ? make_float2(lost, lost) : make_float2(S[j][2 * r], S[j][2 * r + 1]);
         }
   }
   if (gone) {
