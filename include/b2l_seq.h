@@ -138,12 +138,18 @@ typedef struct {
 int b2l_seq_scan_chunks(int T, int delta);
 /* Floats of work_state with which a portion with n_chunks <= 1 runs 16 tokens at a time where its sizes allow it (0: too short); step by step
  * with work_state null.  The space of a portion with n_chunks > 1 serves as well where it is as large.  It holds the chunks' matrices, and from 64 tokens
- * on (up to 256 heads) the operands of the form on the tensor cores, 50 KB a chunk and head, of at most 2048 of them at a time. */
+ * on (up to 256 heads) the operands of the form on the tensor cores, 50 KB a chunk and head, of at most 2048 of them at a time.  Enough for every key and value
+ * size, and growing with both numbers (up to 256 heads): space for the most serves all. */
 long long b2l_seq_scan_work_floats(int T, int heads);
 /* The fastest form for these sizes (vscale: whether a value scale is given): sets *n_chunks and returns the floats of work_state it wants (0: none,
  * step by step).  work_decay is wanted where *n_chunks > 1: n_chunks * heads * (per_channel ? K : 1) floats. */
 long long b2l_seq_scan_plan(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks);
 int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream);
+/* The same with the space counted exactly for these sizes, for b2l_seq_scan_within: returns the floats that the fastest form writes, and sets *least to the fewer
+ * floats with which the portion still runs 16 tokens at a time (0: there is no such form; with none it runs step by step). */
+long long b2l_seq_scan_space(int T, int heads, int qk_heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks, long long* least);
+/* b2l_seq_scan where work_state holds work_floats floats: the fastest form that finds room there. */
+int b2l_seq_scan_within(const b2l_seq_scan_args* a, long long work_floats, b2l_stream_t stream);
 
 /* Read-out of a recurrence: groups of `group` consecutive channels of o (f32 [T, n]) are divided by their root
  * mean square, multiplied by w (act; `w_shared` != 0: w has `group` entries used by every group, else n) and by

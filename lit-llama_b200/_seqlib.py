@@ -155,6 +155,8 @@ _SIGS = {
     "b2l_seq_scan": (c_int, [C.POINTER(ScanArgs), c_void_p]),
     "b2l_seq_scan_chunks": (c_int, [c_int, c_int]),
     "b2l_seq_scan_work_floats": (C.c_longlong, [c_int, c_int]),
+    "b2l_seq_scan_space": (C.c_longlong, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, C.POINTER(c_int), C.POINTER(C.c_longlong)]),
+    "b2l_seq_scan_within": (c_int, [C.POINTER(ScanArgs), C.c_longlong, c_void_p]),
     "b2l_seq_scan_plan": (C.c_longlong, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, C.POINTER(c_int)]),
     "b2l_seq_group_norm_gate": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p,
                                         c_int, c_int, c_int, c_int, c_int, c_void_p]),

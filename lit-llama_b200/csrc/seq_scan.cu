@@ -7,6 +7,7 @@
 // lanes of a column read consecutive 16-byte words).  With `ones` the state has one column more whose value is 1 at every
 // step (a normaliser: the decayed sum of the keys), kept and read out beside the others.  Inputs of SCAN_TC steps are staged in shared memory by the
 // whole CTA with asynchronous copies, one stage ahead of the recurrence.  All arithmetic is f32.
+#include <climits>
 #include <type_traits>
 
 #include "seq_common.cuh"
@@ -735,7 +736,7 @@ static bool walk_sizes(int T, int K, int V, int ones) { return T >= 2 * CH_C && 
 // both times from the fits below, in ns (128 x 128, us walk with 16 columns per CTA / chunked: 1024 tokens of 4 heads 95 / 103; 2048 of 4 173 / 130,
 // of 8 179 / 240; 4096 of 4 333 / 251, of 8 345 / 388; 8192 of 1 634 / 134, of 8 673 / 667, of 16 710 / 1285; walk with 8 columns: 512 tokens of 4
 // and 8 43, 2048 of 4 124, of 8 128; with 64 keys 512 tokens 38, 1024 of 18 63).  The fits are the FMA walk's also where the tensor cores walk (2048 and 4096 tokens of 4
-// heads 81 and 153, 4096 and 8192 of 8 221 and 432, 8192 of 1 261): a chunked form's workspace, which callers bring by its size, is too small for that walk's operands.
+// heads 81 and 153, 4096 and 8192 of 8 221 and 432, 8192 of 1 261): those portions still go in chunks, 130 and 240 us, until the rule weighs that walk by its own times.
 static bool walk_narrow(int heads, int V) { return (long long)heads * (V / CH_NARROW) <= sm_count(); }
 static bool walk_pays(int T, int heads, int K, int V, int delta) {
   const long long sms = sm_count(), ctas = (long long)heads * (V / CH_VT), turns = (ctas + sms - 1) / sms;
@@ -749,14 +750,13 @@ static bool walk_pays(int T, int heads, int K, int V, int delta) {
 // column of ones and single tokens go step by step.  A caller that asks for the chunked form gets a walk where it is faster and its space suffices.
 static long long walk_floats(int T, int heads) { return (long long)((T + CH_C - 1) / CH_C) * heads * (2 * CH_MAT); }
 enum { WALK_NONE, WALK_FMA, WALK_MMA };
-static int walk_form(const b2l_seq_scan_args* a) {
+static int walk_form(const b2l_seq_scan_args* a, long long room) {      // room: floats of work_state
   if (a->work_state == nullptr || !walk_sizes(a->T, a->K, a->V, a->ones) || (a->delta && (!a->decay_per_channel || a->vscale)) || ((uintptr_t)a->state & 15) != 0 ||
       ((uintptr_t)a->work_state & 15) != 0 || a->heads > 65535)
     return WALK_NONE;
   if (a->n_chunks > 1 && !walk_pays(a->T, a->heads, a->K, a->V, a->delta)) return WALK_NONE;
-  auto fits = [&](long long floats) { return a->n_chunks <= 1 || (long long)a->n_chunks * a->heads * a->V * a->K >= floats; };
-  if (mma_walk(a->T, a->heads, a->K, a->V, a->delta) && fits(mma_walk_floats(a->T, a->heads))) return WALK_MMA;
-  return fits(walk_floats(a->T, a->heads)) ? WALK_FMA : WALK_NONE;
+  if (mma_walk(a->T, a->heads, a->K, a->V, a->delta) && mma_walk_floats(a->T, a->heads, a->qk_heads, a->K, a->V, a->delta, a->decay_per_channel) <= room) return WALK_MMA;
+  return walk_floats(a->T, a->heads) <= room ? WALK_FMA : WALK_NONE;
 }
 
 template <typename act_t, int K, bool DELTA>
@@ -789,20 +789,39 @@ extern "C" int b2l_seq_scan_chunks(int T, int delta) {
 
 extern "C" long long b2l_seq_scan_work_floats(int T, int heads) {
   if (T < 2 * CH_C || heads <= 0) return 0;
-  const long long fma = walk_floats(T, heads), mma = T >= MW_LEAST && heads <= MW_HEADS ? mma_walk_floats(T, heads) : 0;
+  const long long fma = walk_floats(T, heads), mma = T >= MW_LEAST && heads <= MW_HEADS ? mma_walk_most_floats(T, heads) : 0;
   return fma > mma ? fma : mma;                        // for either, whatever the key size
 }
 
-extern "C" long long b2l_seq_scan_plan(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks) {
-  if (n_chunks) *n_chunks = 1;
-  if (T <= 0 || heads <= 0 || K <= 0 || V <= 0) return 0;
-  if (walk_sizes(T, K, V, ones) && (!delta || (per_channel && !vscale)) && heads <= 65535 && walk_pays(T, heads, K, V, delta)) return b2l_seq_scan_work_floats(T, heads);
+static bool plan_walks(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale) {
+  return walk_sizes(T, K, V, ones) && (!delta || (per_channel && !vscale)) && heads <= 65535 && walk_pays(T, heads, K, V, delta);
+}
+static long long plan_chunks(int T, int heads, int K, int V, int delta, int ones, int* n_chunks) {
   const int n = b2l_seq_scan_chunks(T, delta);
   if (n_chunks) *n_chunks = n;
   return n > 1 ? (long long)n * heads * (V + (ones ? 1 : 0)) * K : 0;
 }
 
-extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
+extern "C" long long b2l_seq_scan_plan(int T, int heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks) {
+  if (n_chunks) *n_chunks = 1;
+  if (T <= 0 || heads <= 0 || K <= 0 || V <= 0) return 0;
+  if (plan_walks(T, heads, K, V, per_channel, delta, ones, vscale)) return b2l_seq_scan_work_floats(T, heads);
+  return plan_chunks(T, heads, K, V, delta, ones, n_chunks);
+}
+
+extern "C" long long b2l_seq_scan_space(int T, int heads, int qk_heads, int K, int V, int per_channel, int delta, int ones, int vscale, int* n_chunks, long long* least) {
+  if (n_chunks) *n_chunks = 1;
+  if (least) *least = 0;
+  if (T <= 0 || heads <= 0 || qk_heads <= 0 || K <= 0 || V <= 0) return 0;
+  if (!plan_walks(T, heads, K, V, per_channel, delta, ones, vscale)) return plan_chunks(T, heads, K, V, delta, ones, n_chunks);
+  const long long fma = walk_floats(T, heads);
+  if (!mma_walk(T, heads, K, V, delta)) return fma;
+  const long long mma = mma_walk_floats(T, heads, qk_heads, K, V, delta, per_channel);
+  if (least && fma < mma) *least = fma;
+  return mma;
+}
+
+static int scan(const b2l_seq_scan_args* a, long long room, b2l_stream_t stream) {
   B2L_CHECK_ARG(a != nullptr, "b2l_seq_scan: null argument block");
   B2L_CHECK_ARG(a->q && a->k && a->v && a->decay && a->state && a->meta && a->out, "b2l_seq_scan: null pointer");
   B2L_CHECK_ARG(!a->delta || a->beta, "b2l_seq_scan: the delta rule needs beta");
@@ -813,7 +832,7 @@ extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
                 "b2l_seq_scan: chunked portions need the workspace, no delta rule and n_chunks from b2l_seq_scan_chunks");
   B2L_CHECK_ARG(!a->ones || (a->state_ones && a->out_ones && !a->skip && !a->delta), "b2l_seq_scan: the column of ones needs its state and its output, no skip and no delta rule");
   if (a->T == 0) return 0;
-  const int form = walk_form(a);
+  const int form = walk_form(a, room);
   if (form != WALK_NONE && (a->act_dtype == B2L_BF16 || a->act_dtype == B2L_F32)) {
     cudaStream_t st = (cudaStream_t)stream;
     B2L_SEQ_DISPATCH(a->act_dtype, {
@@ -865,4 +884,15 @@ extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
 #undef B2L_SCAN_LAUNCH
   B2L_LAUNCH_CHECK("seq_scan_kernel");
   return 0;
+}
+
+extern "C" int b2l_seq_scan(const b2l_seq_scan_args* a, b2l_stream_t stream) {
+  // the space that the declarations ask for: a chunked portion's end states, else b2l_seq_scan_work_floats
+  return scan(a, a && a->n_chunks > 1 ? (long long)a->n_chunks * a->heads * a->V * a->K : LLONG_MAX, stream);
+}
+
+extern "C" int b2l_seq_scan_within(const b2l_seq_scan_args* a, long long work_floats, b2l_stream_t stream) {
+  B2L_CHECK_ARG(!a || a->n_chunks <= 1 || work_floats >= (long long)a->n_chunks * a->heads * (a->V + (a->ones ? 1 : 0)) * a->K,
+                "b2l_seq_scan_within: %lld floats do not hold the chunks' end states", work_floats);
+  return scan(a, work_floats, stream);
 }

@@ -852,12 +852,19 @@ static bool mma_walk(int T, int heads, int K, int V, int delta) {
   if (heads > MW_HEADS || V > MW_V || V % CH_VT) return false;
   return K == 128 ? T >= (heads * (V / CH_VT) > 64 ? MW_LEAST : 144) : K == 64 && !delta && T >= 512;
 }
-// Tokens of a segment.  A portion goes through the two kernels by segments so that the workspace stays below 102 MB, most of which the L2 keeps; a segment more costs
-// some 8 us beside 160 or more.
+// Tokens of a segment.  A portion goes through the two kernels by segments so that the workspace stays below 103 MB (2048 chunks and heads of 50 KB with the delta rule
+// and 128 value columns), most of which the L2 keeps; a segment more costs some 8 us beside 160 or more.
 static int mma_segment(int heads) { return MW_SEGMENT / heads * CH_C; }
-static long long mma_walk_floats(int T, int heads) {
+// Floats of the workspace: of the largest segment, each chunk's operands once for every head (or, with one decay per head, every head of q and k), then its tiles.
+static long long mma_walk_floats(int T, int heads, int qk_heads, int K, int V, int delta, int per_channel) {
   const long long chunks = ((T < mma_segment(heads) ? T : mma_segment(heads)) + CH_C - 1) / CH_C;
-  return chunks * heads * (long long)(sizeof(ChunkOps<128, true>) / 4 + MW_V / CH_VT * MW_TILE_G);
+  const long long ops = (K == 64 ? sizeof(ChunkOps<64, false>) : delta ? sizeof(ChunkOps<128, true>) : sizeof(ChunkOps<128, false>)) / 4;
+  return chunks * ((per_channel ? heads : qk_heads) * ops + (long long)heads * (V / CH_VT) * (per_channel ? MW_TILE : MW_TILE_G));
+}
+// At least that, whatever the sizes but these two; grows with both of them.
+static long long mma_walk_most_floats(int T, int heads) {
+  const long long all = (long long)((T + CH_C - 1) / CH_C) * heads;
+  return (all < MW_SEGMENT ? all : MW_SEGMENT) * (long long)(sizeof(ChunkOps<128, true>) / 4 + MW_V / CH_VT * MW_TILE_G);
 }
 
 template <typename act_t, int K, bool DELTA, bool SHARED>

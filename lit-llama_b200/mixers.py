@@ -234,22 +234,24 @@ def _scan(ctx: StepContext, *, q, ldq, k, ldk, v, ldv, q_mult, decay, ldd, per_c
     lib = S.lib()
     n_chunks, ws, wd = 1, None, None
     if ctx.T > 1:         # 16 tokens at a time, or (long portion, few heads, no delta rule) chunks in parallel: local states, combine, outputs
-        chunks = C.c_int(1)
-        n = lib.b2l_seq_scan_plan(ctx.T, heads, K, V, int(per_channel), int(beta is not None), int(state_ones is not None), int(vscale is not None), C.byref(chunks))
+        chunks, least = C.c_int(1), C.c_longlong(0)
+        n = lib.b2l_seq_scan_space(ctx.T, heads, qk_heads, K, V, int(per_channel), int(beta is not None), int(state_ones is not None), int(vscale is not None),
+                                   C.byref(chunks), C.byref(least))
         n_chunks = chunks.value
-        try:
-            ws = torch.empty((n,), dtype=torch.float32, device=state.device) if n else None
-        except torch.OutOfMemoryError:
-            if n_chunks > 1:
-                raise
-            ws = None                                    # up to 102 MB: without it the portion goes token by token
+        for n_ws in (n, least.value):                    # up to 103 MB for the tensor cores, a few for the same 16 tokens at a time without them, none token by token
+            if n_ws and ws is None:
+                try:
+                    ws = torch.empty((n_ws,), dtype=torch.float32, device=state.device)
+                except torch.OutOfMemoryError:
+                    if n_chunks > 1:
+                        raise
         wd = torch.empty((n_chunks, heads, K if per_channel else 1), dtype=torch.float32, device=state.device) if n_chunks > 1 else None
     a = S.ScanArgs(q=q, ldq=ldq, k=k, ldk=ldk, v=v, ldv=ldv, q_mult=float(q_mult), decay=decay, ldd=ldd,
                    decay_per_channel=int(per_channel), beta=beta, ldb=ldb, delta=int(beta is not None), vscale=vscale, ldvs=ldvs,
                    skip=skip, state=_p(state), meta=_p(ctx.meta), out=out, ldo=ldo, T=ctx.T, heads=heads, qk_heads=qk_heads, K=K, V=V,
                    act_dtype=ctx.act, work_state=_p(ws), work_decay=_p(wd), n_chunks=n_chunks, ones=int(state_ones is not None), state_ones=_p(state_ones),
                    out_ones=out_ones)
-    S.check(lib.b2l_seq_scan(C.byref(a), ctx.stream), "b2l_seq_scan")
+    S.check(lib.b2l_seq_scan_within(C.byref(a), 0 if ws is None else ws.numel(), ctx.stream), "b2l_seq_scan_within")
 
 
 class ChannelDeltaMixer:

@@ -414,6 +414,44 @@ def test_scan_plan_and_its_neighbours(T, H, K, V, want):
         assert rel(got, out) < 1e-6 and rel(st, state) < 1e-6
 
 
+@pytest.mark.parametrize("T,K,V,H,G,form", [(2048, 128, 128, 16, 16, "delta"), (70, 128, 128, 9, 3, "delta"), (401, 128, 16, 160, 160, "delta"), (512, 128, 64, 32, 1, "scalar"),
+                                            (2100, 128, 48, 18, 3, "scalar"), (530, 64, 112, 6, 2, "channel"), (48, 64, 32, 3, 3, "delta")])
+def test_scan_in_the_space_it_has(T, K, V, H, G, form):
+    """The space counted exactly for the sizes (nothing behind it is written), the fewer floats of the form in f32, and one less, which goes token by token with the
+    bits of a call without space.  Sums in another order: 1e-6 of the norm."""
+    from lit_llama_b200 import _seqlib as S
+
+    lib, g = S.lib(), torch.Generator(device=DEV).manual_seed(T + V)
+    delta, per = int(form == "delta"), int(form != "scalar")
+    q, k, v = torch.randn(T, G, K, generator=g, device=DEV), torch.randn(T, G, K, generator=g, device=DEV), torch.randn(T, H, V, generator=g, device=DEV)
+    k = k / k.norm(dim=-1, keepdim=True)
+    a, beta = torch.rand(T, H, K if per else 1, generator=g, device=DEV) * 0.3 + 0.7, torch.randn(T, H, generator=g, device=DEV)
+    state0, meta = torch.randn(1, H, V, K, generator=g, device=DEV), torch.zeros(2, dtype=torch.int32, device=DEV)
+    n_chunks, least = C.c_int(0), C.c_longlong(0)
+    fast = lib.b2l_seq_scan_space(T, H, G, K, V, per, delta, 0, 0, C.byref(n_chunks), C.byref(least))
+    assert n_chunks.value == 1 and 0 < fast <= lib.b2l_seq_scan_work_floats(T, H)
+
+    def run(floats):
+        out, state, ws = torch.empty(T, H, V, device=DEV), state0.clone(), torch.full((floats + 4096,), 3.0, device=DEV)
+        args = S.ScanArgs(q=q.data_ptr(), ldq=G * K, k=k.data_ptr(), ldk=G * K, v=v.data_ptr(), ldv=H * V, q_mult=1.0, decay=a.data_ptr(), ldd=a.shape[1] * a.shape[2],
+                          decay_per_channel=per, beta=beta.data_ptr() if delta else None, ldb=H, delta=delta, state=state.data_ptr(), meta=meta.data_ptr(), out=out.data_ptr(),
+                          ldo=H * V, T=T, heads=H, qk_heads=G, K=K, V=V, act_dtype=S.act_code(torch.float32), work_state=ws.data_ptr() if floats else None, n_chunks=1)
+        S.check(lib.b2l_seq_scan_within(C.byref(args), floats, S.stream_ptr()), "scan")
+        assert bool((ws[floats:] == 3).all())
+        return out, state, bool((ws != 3).any())
+
+    out, state, _ = run(0)
+    got, st, used = run(fast)
+    assert used and rel(got, out) < 1e-6 and rel(st, state) < 1e-6
+    if least.value:
+        slow, st_slow, used = run(fast - 1)
+        assert used and rel(slow, out) < 1e-6 and rel(st_slow, state) < 1e-6 and not torch.equal(slow, got)
+        small, st_small, used = run(least.value)
+        assert used and torch.equal(small, slow) and torch.equal(st_small, st_slow)
+    none, st_none, used = run((least.value or fast) - 1)
+    assert not used and torch.equal(none, out) and torch.equal(st_none, state)
+
+
 @pytest.mark.parametrize("T,K,V,H,G,form", [(47, 128, 48, 24, 2, "delta"), (47, 128, 48, 25, 5, "delta"), (70, 64, 64, 18, 3, "scalar"), (70, 64, 64, 20, 4, "scalar"),
                                             (33, 128, 128, 9, 9, "channel"), (33, 128, 128, 10, 5, "channel")])
 def test_scans_by_columns_per_cta(T, K, V, H, G, form):

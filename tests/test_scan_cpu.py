@@ -1,6 +1,12 @@
-"""CPU: what the host can check of the recurrences' kernels: the order of the walk's copies when a wait runs out."""
+"""CPU: what the host can check of the recurrences' kernels: the order of the walk's copies when a wait runs out, the space that a portion asks for, and what it
+does with less."""
+import ctypes as C
 import os
 import subprocess
+import types
+
+import pytest
+import torch
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -68,3 +74,84 @@ def test_walk_starts_no_copy_after_a_wait_that_ran_out(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "lit-llama_b200", "csrc"), str(src), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def _space(T, heads, qk_heads, K, V, per_channel, delta, vscale=0):
+    from lit_llama_b200 import _seqlib as S
+
+    n_chunks, least = C.c_int(0), C.c_longlong(-1)
+    n = S.lib().b2l_seq_scan_space(T, heads, qk_heads, K, V, per_channel, delta, 0, vscale, C.byref(n_chunks), C.byref(least))
+    return n, least.value, n_chunks.value
+
+
+def test_scan_space_is_what_the_form_writes():
+    """Floats: 2 matrices of 16 x 16 a chunk and head for the form in f32; for the tensor cores a chunk's operands, 6 (12 with the delta rule: W and Q) 16-bit words a
+    key channel and token for W | Q and 6 for the decayed keys, the decays, and 384 words for every 16 value columns (400 with one decay per head)."""
+    from lit_llama_b200 import _seqlib as S
+
+    def ops(K, delta):
+        return 16 * K * 3 // 2 * (2 if delta else 1) + 16 * K * 3 // 2 + K
+
+    assert _space(2048, 16, 16, 64, 128, 1, 1) == (128 * 16 * 512, 0, 1)                                  # the delta rule with 64 keys stays in f32
+    assert _space(300, 16, 16, 128, 256, 1, 1) == (19 * 16 * 512, 0, 1)                                   # more value columns than the tensor cores' form takes
+    assert _space(2048, 16, 16, 128, 128, 1, 1) == (128 * 16 * (ops(128, 1) + 8 * 384), 128 * 16 * 512, 1)
+    assert _space(512, 32, 1, 128, 64, 0, 0, 1) == (32 * (ops(128, 0) + 32 * 4 * 400), 32 * 32 * 512, 1)      # operands of q and k once for all heads
+    assert _space(4096, 160, 160, 128, 16, 1, 1)[0] == 12 * 160 * (ops(128, 1) + 384)                     # twelve chunks of 160 heads a segment
+    assert _space(2048, 4, 4, 128, 128, 1, 0) == (16 * 4 * 128 * 128, 0, 16) and _space(31, 4, 4, 128, 128, 1, 1) == (0, 0, 1)
+    for T in (33, 64, 79, 512, 2047, 40000):
+        for H in (1, 4, 18, 65, 160, 256):
+            for K, V, per_channel, delta in ((64, 16, 1, 0), (128, 128, 1, 1), (128, 48, 0, 0), (128, 64, 1, 0), (64, 64, 1, 1)):
+                n, least, n_chunks = _space(T, H, H, K, V, per_channel, delta)
+                assert n_chunks > 1 or (least < max(n, 1) and n <= S.lib().b2l_seq_scan_work_floats(T, H))
+
+
+def test_scan_space_for_the_most_serves_all():
+    from lit_llama_b200 import _seqlib as S
+
+    f = S.lib().b2l_seq_scan_work_floats
+    for T in (31, 32, 63, 64, 500, 2048, 30000):
+        n = [f(T, H) for H in range(1, 257)]
+        assert n == sorted(n)
+    for H in (1, 7, 65, 100, 256):
+        n = [f(T, H) for T in range(16, 6000, 5)]
+        assert n == sorted(n)
+
+
+@pytest.mark.parametrize("delta,T,H,memory,want", [(1, 2048, 16, "all", "fast"), (1, 2048, 16, "little", "least"), (1, 2048, 16, "none", "none"), (1, 70, 2, "little", "fast"),
+                                                   (0, 2048, 4, "none", "raises")])
+def test_scan_without_memory_takes_the_form_that_fits(monkeypatch, delta, T, H, memory, want):
+    """No room for the tensor cores' operands: the walk in f32 has what it needs; without that, token by token.  A portion that was to run in chunks says so."""
+    from lit_llama_b200 import _seqlib as S, mixers as X
+
+    K = V = 128
+    fast, least, _ = _space(T, H, H, K, V, 1, delta)
+    limit = {"all": fast, "little": max(least, H * 3000), "none": 100}[memory]
+    real, asked, calls = torch.empty, [], []
+
+    def empty(shape, **kw):
+        n = 1
+        for d in shape:
+            n *= d
+        asked.append(n)
+        if n > limit:
+            raise torch.OutOfMemoryError("no memory (the test's)")
+        return real((n,), dtype=kw["dtype"], device="meta")
+
+    monkeypatch.setattr(X, "_p", lambda t, offset=0: None if t is None else 64)
+    monkeypatch.setattr(X.torch, "empty", empty)
+    lib = types.SimpleNamespace(b2l_seq_scan_space=S.lib().b2l_seq_scan_space, b2l_seq_scan_within=lambda a, floats, stream: calls.append((a._obj.work_state, a._obj.n_chunks, floats)) or 0)
+    monkeypatch.setattr(S, "lib", lambda: lib)
+    ctx = types.SimpleNamespace(T=T, meta=None, act=0, stream=None)
+
+    def scan():
+        X._scan(ctx, q=64, ldq=H * K, k=64, ldk=H * K, v=64, ldv=H * V, q_mult=1.0, decay=64, ldd=H * K, per_channel=True, state=types.SimpleNamespace(device="meta"), out=64,
+                ldo=H * V, heads=H, qk_heads=H, K=K, V=V, beta=64 if delta else None, ldb=H)
+
+    if want == "raises":
+        with pytest.raises(torch.OutOfMemoryError):
+            scan()
+        assert not calls
+        return
+    scan()
+    floats = {"fast": fast, "least": least, "none": 0}[want]
+    assert calls == [(64 if floats else None, 1, floats)] and asked[0] == fast and asked[-1] == (floats or least)
