@@ -58,12 +58,14 @@ class SequenceStatePool:
             raise KeyError(f"request {request_id!r} already holds slot {self._slot_of[request_id]}")
         if not self._free:
             raise PoolFull(f"all {self.n_slots} state slots are in use")
-        slot = self._free.pop()
         zeroed = [self.tensors[name] for name, sp in self.specs.items() if sp.zero_on_acquire]
+        pointers, slot = [S.ptr(t) for t in zeroed], self._free.pop()      # a kernel writes there: device memory only
         if zeroed:
-            n = len(zeroed)
-            S.check(S.lib().b2l_seq_zero_slots((C.c_void_p * n)(*[t.data_ptr() for t in zeroed]), (C.c_size_t * n)(*[t.nbytes // self.n_slots for t in zeroed]), n, slot,
-                                               S.stream_ptr()), "b2l_seq_zero_slots")
+            if torch._C._cuda_getDevice() == zeroed[0].device.index:
+                self._zero(zeroed, pointers, slot)
+            else:
+                with torch.cuda.device(zeroed[0].device):                 # ... of the device that it runs on
+                    self._zero(zeroed, pointers, slot)
         self._slot_of[request_id] = slot
         self._pos[slot] = 0
         self.acquired += 1
@@ -71,6 +73,10 @@ class SequenceStatePool:
             self.reused += 1
         self._used_before.add(slot)
         return slot
+
+    def _zero(self, tensors: List[torch.Tensor], pointers: List[int], slot: int) -> None:
+        n = len(tensors)
+        S.check(S.lib().b2l_seq_zero_slots((C.c_void_p * n)(*pointers), (C.c_size_t * n)(*[t.nbytes // self.n_slots for t in tensors]), n, slot, S.stream_ptr()), "b2l_seq_zero_slots")
 
     def release(self, request_id: Hashable) -> None:
         slot = self._slot_of.pop(request_id)

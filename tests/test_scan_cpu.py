@@ -155,3 +155,35 @@ def test_scan_without_memory_takes_the_form_that_fits(monkeypatch, delta, T, H, 
     scan()
     floats = {"fast": fast, "least": least, "none": 0}[want]
     assert calls == [(64 if floats else None, 1, floats)] and asked[0] == fast and asked[-1] == (floats or least)
+
+
+def test_slots_are_zeroed_on_the_pools_device(monkeypatch):
+    """The zeroing is a kernel: a pool in host memory is refused before it starts and loses no slot, one on another device than the current one is zeroed there."""
+    from lit_llama_b200 import _seqlib as S, state as P
+
+    pool = P.SequenceStatePool({"S": P.StateSpec((4, 8), torch.float32)}, 3, torch.device("cpu"))
+    monkeypatch.setattr(S, "lib", lambda: pytest.fail("no launch"))
+    with pytest.raises(RuntimeError, match="tensor on cpu"):
+        pool.acquire("r")
+    assert pool.free_slots() == 3 and not pool.has("r")
+    current, calls = [0], []
+
+    class Device:
+        def __init__(self, device):
+            self.device = device
+
+        def __enter__(self):
+            self.before, current[0] = current[0], self.device.index
+
+        def __exit__(self, *exc):
+            current[0] = self.before
+
+    monkeypatch.setattr(P.torch.cuda, "device", Device)
+    monkeypatch.setattr(P.torch._C, "_cuda_getDevice", lambda: current[0], raising=False)
+    monkeypatch.setattr(S, "stream_ptr", lambda: 100 + current[0])
+    monkeypatch.setattr(S, "lib", lambda: types.SimpleNamespace(
+        b2l_seq_zero_slots=lambda p, n, k, slot, stream: calls.append((current[0], list(p), list(n), k, slot, stream)) or 0))
+    for index in (1, 0):
+        pool.tensors = {"S": types.SimpleNamespace(is_cuda=True, device=torch.device("cuda", index), nbytes=3 * 128, data_ptr=lambda: 4096)}
+        slot = pool.acquire(index)
+        assert calls.pop() == (index, [4096], [128], 1, slot, 100 + index) and current[0] == 0
