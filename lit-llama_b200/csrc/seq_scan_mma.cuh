@@ -8,9 +8,14 @@
 //                          parts, in the order in which the walk's products take them; B T v goes to the output
 //   seq_walk_mma_kernel    a CTA per (head, 16 value columns) walks the chunks: [W; Q] S, the difference, the update.  S^T lies in registers, 16 columns by 16
 //                          channels a warp, as the result of one product and, cut into parts, the first operand of the next
-// Decays only multiply, as there.  Every product is six bf16 products of parts (those above 2^-24); what the tensor core truncates of T v's off-diagonal part, of W S and of the
-// update is kept below the FMAs' roundings (the update by a seventh product, beta v by an FMA): relative error against float64 over 2048 tokens of 16 heads of 128 x 128,
-// outputs / state, FMAs 1.08e-7 / 6.97e-8, here 1.02e-7 / 6.82e-8; without the delta rule 2.4e-7 / 2.1e-7 and 1.5e-7 / 1.4e-7.
+// Decays only multiply, as there.  Every product is six bf16 products of parts (those above 2^-24).  The tensor core truncates its sums: a seventh product takes that back
+// where it showed beside the FMAs' roundings, in T v, in a chunk's own outputs (B T v, or B u) and in the update; in W S, Q S and the operands it does not show.
+// Relative errors against float64, outputs / state, 2048 tokens of 4 heads of 128 x 128, unit keys, the FMA form and this one: delta rule, decays of 0.5 to 1 1.07e-7 / 7.3e-8
+// and 1.02e-7 / 6.5e-8, values of mean 2 with decays of 0.99 to 1 2.8e-7 / 2.7e-7 and 1.9e-7 / 1.8e-7, keys that share half of themselves 8.0e-8 / 1.2e-7 and 5.8e-8 / 9.5e-8;
+// without it 8.9e-8 / 4.9e-8 and 8.6e-8 / 4.1e-8, with one decay per head 8.9e-8 / 4.8e-8 and 8.9e-8 / 3.9e-8.  Where all is forgotten within a few tokens (decays uniform
+// from 0) a result is one or two roundings in either form: 8.1e-8 / 3.5e-8 and 8.4e-8 / 4.6e-8.  Decays within 0.001 of 1 round their products low, here by 16 at
+// once: outputs 1.8e-7 and 2.6e-7, state 7.1e-7 and 5.5e-7.  W grows with the keys, and T v - W S loses what T (v - k S) keeps: keys of norm 2 5.5e-7 and 4.2e-7, of norm 3, whose
+// recurrence is no longer stable, 512 tokens 1.4e-6 and 2.4e-6.
 //
 // What bounds it: the walk's chain per chunk, 1500 cycles with the delta rule and 940 without, of which the products are 615 and 390 (m16n8k16 every 8 cycles a
 // scheduler): products 370, W S through shared memory 20 + 300 + 40, the update 500, cutting S 150.  An instruction cache next to the schedulers holds a fraction of the
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_
 #pragma unroll
           for (int i = 0; i < 3; ++i) b[j].b[i][j] &= g & 1 ? 0x0000ffffu : 0xffff0000u;
       }
-      mma_parts<2, false>(y, ys, va, b);
+      mma_parts<2, true>(y, ys, va, b);
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -465,13 +470,17 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_shared_kernel(b
   __syncthreads();
   {
     const int t = tid >> 4, i = tid & 15;              // q_t . k_i; of later tokens k_i nothing is used
-    float s[4] = {};
-#pragma unroll 8
-    for (int c = 0; c < K; c += 4) {
-      const float4 x = *reinterpret_cast<const float4*>(&sq[t][c]), y = *reinterpret_cast<const float4*>(&sk[i][c]);
-      s[0] = fmaf(x.x, y.x, s[0]); s[1] = fmaf(x.y, y.y, s[1]); s[2] = fmaf(x.z, y.z, s[2]); s[3] = fmaf(x.w, y.w, s[3]);
-    }
-    sqk[t][i] = (s[0] + s[1]) + (s[2] + s[3]);
+    float s[4][4] = {};                                // short chains: a sum's error is that of all value columns
+#pragma unroll 2
+    for (int c = 0; c < K; c += 16)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 x = *reinterpret_cast<const float4*>(&sq[t][c + 4 * j]), y = *reinterpret_cast<const float4*>(&sk[i][c + 4 * j]);
+        s[j][0] = fmaf(x.x, y.x, s[j][0]); s[j][1] = fmaf(x.y, y.y, s[j][1]); s[j][2] = fmaf(x.z, y.z, s[j][2]); s[j][3] = fmaf(x.w, y.w, s[j][3]);
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[j][0] = (s[j][0] + s[j][1]) + (s[j][2] + s[j][3]);
+    sqk[t][i] = (s[0][0] + s[1][0]) + (s[2][0] + s[3][0]);
   }
   if (blockIdx.z == 0) {
 #pragma unroll 1
@@ -747,7 +756,7 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
         }
       }
       float d[UN][4], ds[UN][4];
-      mma_parts<UN, DELTA>(d, ds, ua, bd);
+      mma_parts<UN, true>(d, ds, ua, bd);
 #pragma unroll
       for (int j = 0; j < UN; ++j) {
         float2 gc;
