@@ -203,10 +203,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
     for (int item = item0; item < p.items; item += step, u0 += nu) {
       // levels as they lie, bf16 subnormals of 2^-133 (low four bits) or 2^-130 (bits 3..6) each, times 2^127: (level - z) 2^-6 or 2^-3 in one fma
       // with get_weight's rounding, since a power of two changes none; its product with scale 2^6 or 2^3 is rounded as the product with scale.
-      // Rows whose zero point or scale leaves bf16's normal range so go through 128 + level instead.
-      const bool fits = (z_f == 0.f || fabsf(z_f) >= 0x1p-100f) && fabsf(sc_f) <= 0x1p100f, all_fit = __all_sync(0xffffffffu, fits);
-      const __nv_bfloat162 up = __float2bfloat162_rn(0x1p127f), zl = __float2bfloat162_rn(all_fit ? z_f * -0x1p-6f : z_f), zh = __float2bfloat162_rn(z_f * -0x1p-3f),
-                           sl = __float2bfloat162_rn(all_fit ? sc_f * 0x1p6f : sc_f), sh = __float2bfloat162_rn(sc_f * 0x1p3f);
+      // Rows whose zero point or scale leaves bf16's normal range so, or is no bf16 number (kept in f32: rounding it first gave sums 0.0037 off, 0.0017 so), look
+      // their 16 weights up: get_weight's two roundings of each, low and high bytes in registers.  27 operations for 8 weights where the products take 12: us, bf16 / f32
+      // scales, 9 rows of 4096 -> 11008 19 / 28, 203 25 / 31, 2048 135 / 147; 512 rows of 13824 -> 5120 58 / 78.
+      const bool fits = (z_f == 0.f || fabsf(z_f) >= 0x1p-100f) && fabsf(sc_f) <= 0x1p100f && rbf(z_f) == z_f && rbf(sc_f) == sc_f, all_fit = __all_sync(0xffffffffu, fits);
+      const __nv_bfloat162 up = __float2bfloat162_rn(0x1p127f);
+      uint32_t row_w[8];                                     // zero point and scale for levels in the low four bits and in bits 3..6, or the weights' bytes
+      if (all_fit) {
+        auto pair = [](float v) { const __nv_bfloat162 b = __float2bfloat162_rn(v); return *reinterpret_cast<const uint32_t*>(&b); };
+        row_w[0] = pair(z_f * -0x1p-6f); row_w[1] = pair(z_f * -0x1p-3f); row_w[2] = pair(sc_f * 0x1p6f); row_w[3] = pair(sc_f * 0x1p3f);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t b[4];
+#pragma unroll
+          for (int l = 0; l < 4; ++l) b[l] = __float_as_uint(rbf(rbf((float)(4 * q + l) - z_f) * sc_f)) >> 16;
+          row_w[q] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+          row_w[4 + q] = __byte_perm(__byte_perm(b[0], b[1], 0x0051), __byte_perm(b[2], b[3], 0x0051), 0x5410);
+        }
+      }
       row_values(item + step);
       for (; turn < nu; turn += GROUPS) {
         mbar_wait(w_full + 8 * st, ph, dead);
@@ -230,27 +245,37 @@ __global__ void __launch_bounds__(NTHREADS, 1) q4_gemm_kernel(const __grid_const
           for (int i = 0; i < 2; ++i) {
             uint32_t o[16];
             if (all_fit) {
+              const __nv_bfloat162 *zl = reinterpret_cast<const __nv_bfloat162*>(row_w), *zh = zl + 1, *sl = zl + 2, *sh = zl + 3;
 #pragma unroll
               for (int c = 0; c < 4; ++c) {
                 const uint32_t v = w[4 * i + c], lo[2] = {v & 0x000f000fu, (v >> 8) & 0x000f000fu}, hi[2] = {(v >> 1) & 0x00780078u, (v >> 9) & 0x00780078u};
 #pragma unroll
                 for (int s = 0; s < 2; ++s) {
-                  const __nv_bfloat162 l = __hmul2(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&lo[s]), up, zl), sl),
-                                       m = __hmul2(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&hi[s]), up, zh), sh);
+                  const __nv_bfloat162 l = __hmul2(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&lo[s]), up, *zl), *sl),
+                                       m = __hmul2(__hfma2(*reinterpret_cast<const __nv_bfloat162*>(&hi[s]), up, *zh), *sh);
                   o[4 * c + 2 * s] = *reinterpret_cast<const uint32_t*>(&l);
                   o[4 * c + 2 * s + 1] = *reinterpret_cast<const uint32_t*>(&m);
                 }
               }
             } else {
 #pragma unroll
-              for (int c = 0; c < 4; ++c)
+              for (int c = 0; c < 4; ++c) {
+                const uint32_t v = w[4 * i + c];
+                uint32_t e[2][2];                            // the even k's pairs of levels (low half of the word), then the odd k's
 #pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                  const uint32_t v = ((w[4 * i + c] >> (4 * s)) & 0x000f000fu) | 0x43004300u;      // (128 + level) pair, exact
-                  __nv_bfloat162 t = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), __float2bfloat162_rn(128.f));
-                  t = __hmul2(__hsub2(t, zl), sl);
-                  o[4 * c + s] = *reinterpret_cast<const uint32_t*>(&t);
+                for (int s = 0; s < 2; ++s) {
+                  const uint32_t at = v >> (16 * s) & 0x7777u, top = __byte_perm(0x0000ff00u, 0u, v >> (16 * s + 3) & 0x1111u);      // levels 8..15: all bits of the byte
+                  const uint32_t lo = (__byte_perm(row_w[0], row_w[1], at) & ~top) | (__byte_perm(row_w[2], row_w[3], at) & top),
+                                 hi = (__byte_perm(row_w[4], row_w[5], at) & ~top) | (__byte_perm(row_w[6], row_w[7], at) & top);
+                  e[s][0] = __byte_perm(lo, hi, 0x5140);
+                  e[s][1] = __byte_perm(lo, hi, 0x7362);
                 }
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                  o[4 * c + 2 * s] = __byte_perm(e[0][s], e[1][s], 0x5410);
+                  o[4 * c + 2 * s + 1] = __byte_perm(e[0][s], e[1][s], 0x7632);
+                }
+              }
             }
             tmem_st16(tmem + lane_at + buf * A_COLS + 32 * h + 16 * i, o);
           }

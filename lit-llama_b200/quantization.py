@@ -288,7 +288,9 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             # more than 8 rows: tcgen05 tiles of 128 features, weights dequantised on the fly with get_weight's roundings.  Up to 16 rows q4_linear_tc
             # (K split over clusters) takes inputs that are no multiple of 64 wide, and no others: 9 / 16 rows of 4096 -> 4096 take it 23 / 30 us and the
             # GEMM 11.4 / 11.6, 4096 -> 11008 36 / 46 and 15.8, 13824 -> 5120 49 / 63 and 20, 64 -> 64 10 / 14 and 5.0; 1.7 to 3.2 times in all 14 shapes
-            # measured, and 0.0017 off the product of get_weight's matrix in 64 bits instead of 0.0024
+            # measured.  The two multiply different matrices: q4_linear_tc, as the kernels of up to 8 rows, the levels themselves with scale and zero point
+            # applied to the sums, the GEMM get_weight's, whose two bf16 roundings a weight the reference's dense branch has too.  Off the product of
+            # get_weight's matrix in 64 bits 0.0024 and 0.0017 (f32 scales 0.0027 and 0.0017), off that of the unrounded one 0.0017 and 0.0024
             which, wt = L.Q4_GEMM if K % 64 == 0 else L.Q4_LINEAR_TC, self.tiled()
         if which >= 0:
             rc = L.pycall.q4(which, xp, ldx, wt.data_ptr(), scales.data_ptr(), zeros.data_ptr(), 0 if scales.dtype is torch.bfloat16 else L.sz_dtype_of(scales),

@@ -259,6 +259,29 @@ def test_q4_gemm_prefill_shapes(dev, M, N, K):
         assert torch.equal(lin.get_weight(torch.bfloat16), wb)
 
 
+@pytest.mark.parametrize("M", [9, 16, 17, 150, 300])
+@pytest.mark.parametrize("N,K", [(130, 64), (300, 192), (5120, 1024)])
+def test_linear_multiplies_get_weights_matrix_with_f32_scales(dev, M, N, K):
+    """Scales and zero points that bf16 would round, among them one below and one above its range for the products: the weights are get_weight's, all 16 levels of
+    every row.  Sums in f32 and one bf16 rounding of the result."""
+    from gpu_util import rand_q4
+    from lit_llama_b200.quantization import ColBlockQuantizedLinear
+
+    lv, qw, sc, z = rand_q4(N, K, dev, seed=M + N + K)
+    g = torch.Generator(device=dev).manual_seed(N)
+    sc = sc.float() * (1 + torch.randn(N, 1, generator=g, device=dev) * 0.01)
+    z = z.float() + torch.randn(N, 1, generator=g, device=dev) * 0.01
+    z[5], z[7], z[40] = 1e-33, 0.0, 1e20
+    sc[40] *= 1e-20
+    lin = ColBlockQuantizedLinear(K, N, bias=False, bits=4, tile_cols=-1).to(dev)
+    lin.quant_weight.copy_(qw); lin.scales = sc; lin.zeros = z
+    wb = lin.get_weight(torch.bfloat16).double()
+    assert torch.equal(wb, ((lv.float() - z).bfloat16().float() * sc).bfloat16().double())
+    x = torch.randn(M, K, generator=g, device=dev).bfloat16()
+    y, want, mag = lin(x).double(), x.double() @ wb.t(), x.double().abs() @ wb.abs().t()
+    assert bool(((y - want).abs() <= want.abs() * 2.0 ** -8 + mag * 2.0 ** -20 + 1e-30).all())
+
+
 @pytest.mark.parametrize("M", [9, 15, 16])
 @pytest.mark.parametrize("N,K,sz", [(130, 64, torch.bfloat16), (300, 192, torch.float32), (5120, 1024, torch.bfloat16), (300, 96, torch.bfloat16)])
 def test_linear_of_9_to_16_rows(dev, M, N, K, sz):
