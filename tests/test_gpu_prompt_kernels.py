@@ -191,6 +191,13 @@ def test_scans_on_the_tensor_cores(T, K, V, H, G, form):
     test_scans_sixteen_tokens_at_a_time(T, K, V, H, G, form)
 
 
+@pytest.mark.parametrize("T,K,V,H,G", [(300, 128, 48, 13, 1), (512, 128, 64, 32, 1), (576, 128, 64, 13, 1), (700, 128, 128, 11, 1), (1040, 128, 48, 13, 1), (1041, 128, 16, 11, 1),
+                                       (1047, 64, 80, 15, 1), (1056, 128, 32, 28, 2)])
+def test_scans_of_heads_that_share_a_cta(T, K, V, H, G):
+    """One decay per head: two, four and eight heads a CTA (148 SMs), last groups of 1, 3, 5, 6 and 7 heads whose warps take value columns in turn or nothing."""
+    test_scans_sixteen_tokens_at_a_time(T, K, V, H, G, "scalar")
+
+
 @pytest.mark.parametrize("delta", [0, 1])
 @pytest.mark.parametrize("T", [144, 777])
 def test_scan_on_the_tensor_cores_is_as_near_as_token_by_token(T, delta):
@@ -289,6 +296,46 @@ def test_scan_on_the_tensor_cores_with_infinities(delta, what, bad):
     if what in ("v", "state"):
         c = 5 if what == "v" else 3
         assert torch.equal(got[:, :, :c], clean[:, :, :c]) and torch.equal(got[:, :, c + 1:], clean[:, :, c + 1:]) and torch.equal(st[0, 1, c + 1:], clean_state[0, 1, c + 1:])
+    for x, y in ((got, want), (st, st_want)):
+        fin = y.isfinite()
+        assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x[~fin & ~y.isnan()], y[~fin & ~y.isnan()])
+        x, y = x.double().where(fin, 0.0), y.double().where(fin, 0.0)
+        assert bool(((x - y).abs() <= 1e-5 * y.norm(dim=-1, keepdim=True)).all())
+
+
+@pytest.mark.parametrize("what,bad", [("v", math.inf), ("v", math.nan), ("vscale", math.inf), ("vscale", math.nan), ("decay", math.inf), ("decay", math.nan), ("k", -math.inf), ("k", math.nan),
+                                      ("q", math.inf), ("state", -math.inf)])
+@pytest.mark.parametrize("T,H", [(700, 11), (200, 5)])
+def test_scan_of_heads_that_share_a_cta_with_infinities(T, H, what, bad):
+    """The same for one decay per head and q and k shared by all heads: earlier tokens and (but for q and k) other heads keep their bits, the rest has its infinities and NaN
+    where the form that walks token by token has them, and is within 1e-5 of the row elsewhere (f32 sums in two orders)."""
+    from lit_llama_b200 import _seqlib as S
+
+    K, V, at, head = 128, 32, 70, 3
+    g = torch.Generator(device=DEV).manual_seed(T)
+    ops = {"q": torch.randn(T, 1, K, generator=g, device=DEV), "k": torch.randn(T, 1, K, generator=g, device=DEV) / 12, "v": torch.randn(T, H, V, generator=g, device=DEV),
+           "vscale": torch.rand(T, H, generator=g, device=DEV) + 0.5, "decay": torch.rand(T, H, generator=g, device=DEV) * 0.5 + 0.5,
+           "state": torch.randn(1, H, V, K, generator=g, device=DEV)}
+    meta, lib = torch.zeros(2, dtype=torch.int32, device=DEV), S.lib()
+    work = torch.empty(lib.b2l_seq_scan_work_floats(T, H), device=DEV)
+
+    def run(space):
+        out, state = torch.empty(T, H, V, device=DEV), ops["state"].clone()
+        a = S.ScanArgs(q=ops["q"].data_ptr(), ldq=K, k=ops["k"].data_ptr(), ldk=K, v=ops["v"].data_ptr(), ldv=H * V, q_mult=1.0, decay=ops["decay"].data_ptr(), ldd=H,
+                       decay_per_channel=0, vscale=ops["vscale"].data_ptr(), ldvs=H, delta=0, state=state.data_ptr(), meta=meta.data_ptr(), out=out.data_ptr(), ldo=H * V, T=T,
+                       heads=H, qk_heads=1, K=K, V=V, act_dtype=S.act_code(torch.float32), work_state=space, n_chunks=1)
+        S.check(lib.b2l_seq_scan(C.byref(a), S.stream_ptr()), "scan")
+        return out, state
+
+    clean, clean_state = run(work.data_ptr())
+    ops[what][(0, head, 4, 5) if what == "state" else (at, 0, 5) if what in "qk" else (at, head, 5) if what == "v" else (at, head)] = bad
+    (got, st), (want, st_want) = run(work.data_ptr()), run(None)
+    others = [h for h in range(H) if h != head]
+    if what not in "qk":
+        assert torch.equal(got[:, others], clean[:, others]) and torch.equal(st[0, others], clean_state[0, others])
+    if what != "state":
+        assert torch.equal(got[:at], clean[:at])
+    assert not bool(got.isfinite().all())
     for x, y in ((got, want), (st, st_want)):
         fin = y.isfinite()
         assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x[~fin & ~y.isnan()], y[~fin & ~y.isnan()])
@@ -785,16 +832,20 @@ def test_rotation_of_four_heads_a_warp(T, H, size, off, rot, inter, apart, src, 
     assert bool(((got[..., :size].double() - want).abs() <= tol).all()) and bool((got[..., size:] == 7).all())
 
 
-def test_slots_are_zeroed_at_once():
-    """Seventeen tensors of a slot: more than a launch takes, words and odd sizes, empty ones; the neighbouring slots stay."""
+@pytest.mark.parametrize("n", [14, 12, 3, 1])
+def test_slots_are_zeroed_at_once(n):
+    """18, 16, 7 and 5 ranges of whole words (a launch takes 16, so two, one and part of one), odd sizes and empty ones; the neighbouring slots stay."""
     from lit_llama_b200 import _seqlib as S
 
-    sizes = [16, 48, 33, 0, 4096 * 16, 2, 1 << 20] + [32 * (i + 1) for i in range(12)]
+    sizes = [16, 48, 33, 0, 4096 * 16, 2, 1 << 20] + [32 * (i + 1) for i in range(n)]
     pools = [torch.full((3, n), 5, dtype=torch.uint8, device=DEV) for n in sizes]
-    n = len(pools)
-    S.check(S.lib().b2l_seq_zero_slots((C.c_void_p * n)(*[t.data_ptr() or None for t in pools]), (C.c_size_t * n)(*sizes), n, 1, S.stream_ptr()), "zero")
-    for t in pools:
-        assert bool((t[1] == 0).all()) and bool((t[0] == 5).all()) and bool((t[2] == 5).all())
+    for some in (range(len(sizes)), [3, len(sizes) - 1], [5]):           # all of them, one word range beside an empty one, one odd size
+        picked, n = [pools[i] for i in some], len(some)
+        for t in picked:
+            t.fill_(5)
+        S.check(S.lib().b2l_seq_zero_slots((C.c_void_p * n)(*[t.data_ptr() or None for t in picked]), (C.c_size_t * n)(*[sizes[i] for i in some]), n, 1, S.stream_ptr()), "zero")
+        for t in picked:
+            assert bool((t[1] == 0).all()) and bool((t[0] == 5).all()) and bool((t[2] == 5).all())
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 8), (17, 130, 72), (113, 300, 64), (70, 2200, 1000), (300, 1025, 200)])
