@@ -605,6 +605,7 @@ struct MwSmem {
   float4 px[DELTA ? MW_WARPS : 1][2][32];      // W S of the walk's warps
   uint32_t u[MW_TILE];           // parts of u
   uint64_t bars[STAGES];
+  uint32_t bad_columns;          // value columns with something infinite or NaN in them
 };
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
@@ -612,31 +613,44 @@ __device__ __forceinline__ void as4(float (&d)[4], const float4& v) { d[0] = v.x
 __device__ __forceinline__ void plus4(float (&d)[4], const float4& v) { d[0] += v.x; d[1] += v.y; d[2] += v.z; d[3] += v.w; }
 __device__ __forceinline__ float4 sum4(const float (&a)[4], const float (&b)[4]) { return make_float4(a[0] + b[0], a[1] + b[1], a[2] + b[2], a[3] + b[3]); }
 
-// Columns whose results are infinite or NaN, token by token in f32 from the state before the portion: what came out finite stays.  `fin` [16][K]: the walk's state.
+// Columns whose results are infinite or NaN (bits of `bad`), token by token in f32 from the state before the segment: what came out finite stays.  `fin` [16][K]: the
+// walk's state.  A column is settled once its state holds a NaN and all that is to be replaced in it is one: every later output is NaN then.  us, 2048 tokens of 16
+// heads of 128 x 128, delta rule: 169 without anything infinite, 1050 with one infinite value in the middle (2880 before columns settled), 240 with a NaN key at the start.
+// Inlined: as a function of its own it cost the walk's loop up to 4 % of its time by where it lay.
 template <typename act_t, int K, bool DELTA>
-__device__ __noinline__ void walk_redo(const b2l_seq_scan_args& a, int t_lo, int t_hi, const float* fin) {
+__device__ __forceinline__ void walk_redo(const b2l_seq_scan_args& a, int t_lo, int t_hi, const float* fin, uint32_t bad) {
   constexpr int L = 16, PER = K / L;                   // lanes per column
   const int tid = threadIdx.x;
   if (tid >= CH_VT * L) return;
   const int h = blockIdx.y, hq = h / (a.heads / a.qk_heads), col = blockIdx.x * CH_VT + tid / L, l = tid % L;
+  const bool mine = bad >> (tid / L) & 1;
   float* st = a.state + ((size_t)a.meta[0] * a.heads + h) * (size_t)a.V * K + (size_t)col * K;
+  fin += (tid / L) * K + l;
   const float skip = a.skip ? ld_act((const act_t*)a.skip, h) : 0.f;
   float S[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) S[i] = st[l + L * i];
-  for (int t = t_lo; t < t_hi; ++t) {
-    const float* k = a.k + (size_t)t * a.ldk + (size_t)hq * K + l;
-    const float* q = a.q + (size_t)t * a.ldq + (size_t)hq * K + l;
-    const float* d = a.decay + (size_t)t * a.ldd + (a.decay_per_channel ? (size_t)h * K + l : (size_t)h);
-    const float v = a.v[(size_t)t * a.ldv + (size_t)h * a.V + col];
-    float p = 0.f, kq = 0.f, o = 0.f, u = v;          // delta rule: o = S'^T q + u (k . q), as the step by step form takes it
+  int t = __any_sync(0xffffffffu, mine) ? t_lo : t_hi;
+#pragma unroll 1
+  while (t < t_hi) {
+    float k[PER], q[PER], d[PER];                      // all loads before the first store, which they might alias
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-      S[i] *= d[a.decay_per_channel ? L * i : 0];
+      k[i] = a.k[(size_t)t * a.ldk + (size_t)hq * K + l + L * i];
+      q[i] = a.q[(size_t)t * a.ldq + (size_t)hq * K + l + L * i];
+      d[i] = a.decay[(size_t)t * a.ldd + (a.decay_per_channel ? (size_t)h * K + l + L * i : (size_t)h)];
+    }
+    float* out = a.out + (size_t)t * a.ldo + (size_t)h * a.V + col;
+    const float v = a.v[(size_t)t * a.ldv + (size_t)h * a.V + col], was = *out,
+                gate = DELTA ? sigmoid_f(ld_act((const act_t*)a.beta, (size_t)t * a.ldb + h)) : a.vscale ? a.vscale[(size_t)t * a.ldvs + h] : 1.f;
+    float p = 0.f, kq = 0.f, o = 0.f, u = v;           // delta rule: o = S'^T q + u (k . q), as the step by step form takes it
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      S[i] *= d[i];
       if (DELTA) {
-        p = fmaf(S[i], k[L * i], p);
-        o = fmaf(S[i], q[L * i], o);
-        kq = fmaf(k[L * i], q[L * i], kq);
+        p = fmaf(S[i], k[i], p);
+        o = fmaf(S[i], q[i], o);
+        kq = fmaf(k[i], q[i], kq);
       }
     }
     if (DELTA) {
@@ -645,28 +659,37 @@ __device__ __noinline__ void walk_redo(const b2l_seq_scan_args& a, int t_lo, int
         p += __shfl_xor_sync(0xffffffffu, p, w);
         kq += __shfl_xor_sync(0xffffffffu, kq, w);
       }
-      u = sigmoid_f(ld_act((const act_t*)a.beta, (size_t)t * a.ldb + h)) * (v - p);
+      u = gate * (v - p);
     } else if (a.vscale) {
-      u *= a.vscale[(size_t)t * a.ldvs + h];
+      u *= gate;
     }
+    bool held = false, open = false;                   // a NaN in the state; something to be replaced that is none yet
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-      S[i] = fmaf(k[L * i], u, S[i]);
-      if (!DELTA) o = fmaf(S[i], q[L * i], o);
+      S[i] = fmaf(k[i], u, S[i]);
+      if (!DELTA) o = fmaf(S[i], q[i], o);
+      const bool nan = S[i] != S[i];
+      held |= nan;
+      open |= !nan && !(fabsf(fin[L * i]) < INFINITY);
     }
 #pragma unroll
     for (int w = 1; w < L; w <<= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
     if (DELTA) o = fmaf(u, kq, o);
+    if (mine && l == 0 && !(fabsf(was) < INFINITY)) *out = o * a.q_mult + skip * v;
+    const uint32_t half = 0xffffu << (tid & 16), holds = __ballot_sync(0xffffffffu, held) & half, opens = __ballot_sync(0xffffffffu, open) & half;
+    ++t;
+    if (__all_sync(0xffffffffu, !mine || (holds && !opens))) break;
+  }
+  for (t += l; mine && t < t_hi; t += L) {
     float* out = a.out + (size_t)t * a.ldo + (size_t)h * a.V + col;
-    if (l == 0 && !(fabsf(*out) < INFINITY)) *out = o * a.q_mult + skip * v;
+    if (!(fabsf(*out) < INFINITY)) *out = __int_as_float(0x7fc00000);
   }
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    const float x = fin[(tid / L) * K + l + L * i];
+    const float x = fin[L * i];
     st[l + L * i] = fabsf(x) < INFINITY ? x : S[i];
   }
 }
-
 
 // tokens t_lo .. t_hi - 1.  SHARED: operands of seq_chunk_shared_kernel; a head's decays are in its tiles
 template <typename act_t, int K, bool DELTA, bool SHARED>
@@ -683,12 +706,13 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
   float* st = a.state + ((size_t)a.meta[0] * a.heads + h) * (size_t)a.V * K;
   enum { PX = 1, UX = 2, FULL = 3, DONE = FULL + STAGES, EMPTY = DONE + STAGES };      // barriers: W S and u exchanged; operands of a stage there, walked, read out
   if (tid == 0) {
+    sm.bad_columns = 0u;
     for (int i = 0; i < STAGES; ++i) mbar_init(smem_u32(sm.bars + i), 1);
     mbar_init_fence();
   }
   __syncthreads();
   uint32_t dead = 0;
-  bool odd = false;
+  bool odd[2] = {};                                    // this thread saw something infinite or NaN in value column g, g + 8
   constexpr int WC = K / MW_WARPS, UN = WC / 8;      // channels of a warp of the walk: 16, or 8 (the other half of the products' 16 is zero), groups of 8
   float S[2][4] = {};                                  // value columns lane / 4, + 8; channels 2 (lane % 4), + 1 of the group
   const float lost = __int_as_float(0x7fc00000);
@@ -775,7 +799,7 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
       split_pair(S, sa);
       if (++sti == STAGES) sti = 0;
     }
-    odd = !(finite4(S[0]) && finite4(S[1]));
+    for (int e = 0; e < 4; ++e) odd[e >> 1] |= !(fabsf(S[0][e]) < INFINITY && fabsf(S[1][e]) < INFINITY);
   } else if (warp == MW_WARPS) {
     // ===================== operands, as the chunk kernel wrote them: STAGES - 1 copies ahead of the chunk that is handed over =====================
     constexpr int WORDS = SHARED ? MW_TILE_G : MW_TILE;
@@ -826,13 +850,14 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         y[e] = fmaf(r[e], a.q_mult, y[e]);
-        odd |= !(fabsf(y[e]) < INFINITY);
+        odd[e >> 1] |= !(fabsf(y[e]) < INFINITY);
         if (t0 + (e & 1) < t_hi) out[(e & 1) * (size_t)a.ldo + 8 * (e >> 1)] = y[e];
       }
       if (++sti == STAGES) sti = 0;
     }
   }
-  const int redo = __syncthreads_or((int)odd), gone = __syncthreads_or((int)dead);
+  if (odd[0] || odd[1]) atomicOr(&sm.bad_columns, (uint32_t)odd[0] << g | (uint32_t)odd[1] << (g + 8));
+  const int gone = __syncthreads_or((int)dead), redo = (int)sm.bad_columns;
   if (warp < MW_WARPS) {
     float* fin = reinterpret_cast<float*>(&sm.st[0]);  // [16][K]
     const int at0 = UN == 1 ? warp & 1 : 0;
@@ -849,7 +874,7 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
     for (int i = tid; i < (t_hi - t_lo) * CH_VT; i += MW_THREADS) a.out[(size_t)(t_lo + i / CH_VT) * a.ldo + (size_t)h * a.V + v0 + i % CH_VT] = lost;
   } else if (redo) {
     __syncthreads();
-    walk_redo<act_t, K, DELTA>(a, t_lo, t_hi, reinterpret_cast<const float*>(&sm.st[0]));
+    walk_redo<act_t, K, DELTA>(a, t_lo, t_hi, reinterpret_cast<const float*>(&sm.st[0]), (uint32_t)redo);
   }
 }
 

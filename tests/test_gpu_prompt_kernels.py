@@ -262,7 +262,7 @@ def test_scan_on_the_tensor_cores_keeps_what_the_f32_form_keeps(form, G, v_mean,
     assert errs[0] != errs[1] and all(x < 1.125 * y for x, y in zip(*errs)), errs
 
 
-@pytest.mark.parametrize("what,bad", [("v", math.inf), ("k", math.nan), ("k", -math.inf), ("q", math.inf), ("decay", math.nan), ("beta", math.nan), ("state", math.inf)])
+@pytest.mark.parametrize("what,bad", [("v", math.inf), ("k", math.nan), ("k", -math.inf), ("q", math.inf), ("decay", math.nan), ("beta", math.nan), ("state", math.inf), ("state", math.nan)])
 @pytest.mark.parametrize("delta", [0, 1])
 def test_scan_on_the_tensor_cores_with_infinities(delta, what, bad):
     """Tokens before a bad one, other heads and (values) other columns keep their bits; the rest is what the form that walks token by token gives: infinities and NaN in
@@ -304,7 +304,7 @@ def test_scan_on_the_tensor_cores_with_infinities(delta, what, bad):
 
 
 @pytest.mark.parametrize("what,bad", [("v", math.inf), ("v", math.nan), ("vscale", math.inf), ("vscale", math.nan), ("decay", math.inf), ("decay", math.nan), ("k", -math.inf), ("k", math.nan),
-                                      ("q", math.inf), ("state", -math.inf)])
+                                      ("q", math.inf), ("state", -math.inf), ("state", math.nan)])
 @pytest.mark.parametrize("T,H", [(700, 11), (200, 5)])
 def test_scan_of_heads_that_share_a_cta_with_infinities(T, H, what, bad):
     """The same for one decay per head and q and k shared by all heads: earlier tokens and (but for q and k) other heads keep their bits, the rest has its infinities and NaN
