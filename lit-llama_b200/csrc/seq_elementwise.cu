@@ -311,7 +311,8 @@ __global__ void seq_conv_silu_kernel(const act_t* __restrict__ in, int ldin, con
 // Portions that give the SMs fewer than eight CTAs of eight tokens go by four tokens a thread: their time is a thread's chain of loads and gates.
 // A thread takes four tokens at once, the next four requested before: each token by itself waited for its load, its gates and, with unit heads, five
 // exchanges, a root and a quotient in every lane; for four tokens together a lane adds up one token's squares and takes its root alone.  us, token by token /
-// by fours, unit heads of 128: 6144 channels x 2048 tokens 25.4 / 22.6, 3072 x 512 6.1 / 5.2, x 9 4.9 / 3.6; without heads 3072 x 9 3.7 / 3.2, but
+// by fours, unit heads of 128, calls back to back on inputs that the L2 holds: 6144 channels x 2048 tokens 27.1 / 24.9, 3072 x 512 8.5 / 6.6; each call by itself on inputs
+// from memory 37.8 / 33.8, 13.3 / 11.2, 3072 x 9 11.3 / 9.6; in the delta layer of 2048 tokens the kernel takes 26.  Without heads 3072 x 9 3.7 / 3.2, but
 // 6144 x 2048 19.2 / 19.9 (80 registers), so those go token by token, as do heads of fewer than four lanes.
 constexpr int CONV_VT = 8, CONV_VT_FEW = 4;
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float (&x)[8]) {

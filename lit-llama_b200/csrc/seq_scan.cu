@@ -736,7 +736,7 @@ static bool walk_sizes(int T, int K, int V, int ones) { return T >= 2 * CH_C && 
 // both times from the fits below, in ns (128 x 128, us walk with 16 columns per CTA / chunked: 1024 tokens of 4 heads 95 / 103; 2048 of 4 173 / 130,
 // of 8 179 / 240; 4096 of 4 333 / 251, of 8 345 / 388; 8192 of 1 634 / 134, of 8 673 / 667, of 16 710 / 1285; walk with 8 columns: 512 tokens of 4
 // and 8 43, 2048 of 4 124, of 8 128; with 64 keys 512 tokens 38, 1024 of 18 63).  The fits are the FMA walk's also where the tensor cores walk (2048 and 4096 tokens of 4
-// heads 81 and 153, 4096 and 8192 of 8 221 and 432, 8192 of 1 261): those portions still go in chunks, 130 and 240 us, until the rule weighs that walk by its own times.
+// heads 84 and 162): those portions still go in chunks, 130 and 240 us, until the rule weighs that walk by its own times.
 static bool walk_narrow(int heads, int V) { return (long long)heads * (V / CH_NARROW) <= sm_count(); }
 static bool walk_pays(int T, int heads, int K, int V, int delta) {
   const long long sms = sm_count(), ctas = (long long)heads * (V / CH_VT), turns = (ctas + sms - 1) / sms;

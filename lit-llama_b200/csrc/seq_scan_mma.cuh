@@ -21,8 +21,8 @@
 // scheduler): products 370, W S through shared memory 20 + 300 + 40, the update 500, cutting S 150.  An instruction cache next to the schedulers holds a fraction of the
 // loop, which is why the operands are made by another kernel (in the same CTAs they cost as much again: 2900 cycles).  At 128 CTAs without the delta rule the operands' way
 // from the L2 shows as well (27 KB a chunk and CTA, 5 TB/s: 1280 cycles).  The chunk kernel: 20000 cycles a CTA, three on an SM, instruction fetches and its 58 KB of
-// results.  us, FMA form / this one: 2048 tokens, delta rule, 8 / 16 / 32 heads of 128 x 128 155 / 136, 214 / 165, 426 / 314; 512 tokens of 8 heads 49 / 42, of 32 heads of
-// 128 x 64 with one decay per head and no delta rule 56 / 44; 2048 and 4096 tokens of 4 heads without it 118 / 81, 224 / 153.
+// results.  us, FMA form / this one: 2048 tokens, delta rule, 8 / 16 / 32 heads of 128 x 128 156 / 133, 213 / 158, 426 / 321; 512 tokens of 8 heads 49 / 41, of 32 heads of
+// 128 x 64 with one decay per head and no delta rule 56 / 44; 2048 and 4096 tokens of 4 heads without it 119 / 84, 226 / 162 (calls back to back).
 // With both in f32 FMAs a chunk's products read 0.5 words of shared memory per FMA, 1300 + 750 cycles where the FMAs are 770.
 #pragma once
 #include "seq_walk_schedule.h"
@@ -427,8 +427,8 @@ __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_ops_kernel(b2l_
 
 // The same with one decay per head and no delta rule: q, k and their products are those of all heads that share them, and a head's decays weight outputs, values and the
 // 16 x 16 matrix.  So a CTA per (chunk, head of q and k, up to eight heads) multiplies q and k once, and the first of them leaves the walk one set of operands for all
-// heads, which the L2 then holds once.  us, both kernels, a CTA per head / this form: 32 heads of 128 x 64 over one q and k, 512 and 2048 tokens 44 / 34, 184 / 102; over 32 of
-// their own 44 / 46 and 197 / 195; 8 heads of 128 x 128 over one, 2048 tokens 93 / 83.
+// heads, which the L2 then holds once.  us, both kernels, a CTA per head / this form: 32 heads of 128 x 64 over one q and k, 512 and 2048 tokens 44 / 32, 184 / 103; over 32 of
+// their own 44 / 44 and 197 / 188; 8 heads of 128 x 128 over one, 2048 tokens 93 / 84.
 template <typename act_t, int K>
 __global__ void __launch_bounds__(MW_CHUNK_THREADS, 3) seq_chunk_shared_kernel(b2l_seq_scan_args a, int vec, int t_lo, int t_hi, int per, MwWork work) {
   using Ops = ChunkOps<K, false>;
@@ -878,9 +878,9 @@ __global__ void __launch_bounds__(MW_THREADS) seq_walk_mma_kernel(b2l_seq_scan_a
   }
 }
 
-// Where this form is taken: key size 128 (64 without the delta rule: 16 heads of 64 x 64, 512 tokens 34 us both, 64 heads, 2048 tokens 284 / 217 us; with it 42 / 44
+// Where this form is taken: key size 128 (64 without the delta rule: 16 heads of 64 x 64, 512 tokens 33 / 29 us, 64 heads, 2048 tokens 281 / 221 us; with it 42 / 44
 // and 166 / 177), a CTA's worth of value columns, and portions long enough for the second kernel's launch and the chunks' operands to pay: 64 tokens where the walk
-// has more than 64 CTAs (16 heads of 128 x 128 19.5 / 18.8 us; 32 of 128 x 64 20.4 / 17.4), 144 otherwise (8 heads, 96 / 128 / 192 tokens: 20.1 / 20.6, 22.1 / 22.5, 27.0 / 24.9).
+// has more than 64 CTAs (16 heads of 128 x 128 19.8 / 17.7 us with the delta rule, 15.7 / 14.5 without; 32 of 128 x 64 15.8 / 13.6), 144 otherwise (8 heads, 128 / 144 / 192 tokens: 16.7 / 16.7, 18.8 / 16.6, 20.8 / 18.6).
 constexpr int MW_HEADS = 256, MW_V = 128, MW_LEAST = 64, MW_SEGMENT = 2048;      // most heads, value columns; least tokens; chunks times heads of a segment
 static bool mma_walk(int T, int heads, int K, int V, int delta) {
   if (heads > MW_HEADS || V > MW_V || V % CH_VT) return false;
