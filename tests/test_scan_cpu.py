@@ -117,6 +117,18 @@ def test_scan_space_for_the_most_serves_all():
         assert n == sorted(n)
 
 
+def test_scan_within_refuses_what_the_scan_refuses():
+    from lit_llama_b200 import _seqlib as S
+
+    lib, said = S.lib(), lambda: S.lib().b2l_seq_last_error()
+    assert lib.b2l_seq_scan_within(None, 10, None) == -1 and b"null argument block" in said()
+    a = S.ScanArgs(T=512, heads=2, qk_heads=2, K=64, V=64, n_chunks=4)
+    assert lib.b2l_seq_scan_within(C.byref(a), 4 * 2 * 64 * 64 - 1, None) == -1 and b"end states" in said()
+    assert lib.b2l_seq_scan_within(C.byref(a), 4 * 2 * 64 * 64, None) == -1 and b"null pointer" in said()
+    a = S.ScanArgs(T=0, heads=2, qk_heads=2, K=64, V=64, n_chunks=1, q=64, k=64, v=64, decay=64, state=64, meta=64, out=64)
+    assert lib.b2l_seq_scan_within(C.byref(a), 0, None) == 0 and lib.b2l_seq_scan(C.byref(a), None) == 0       # no tokens: no launch
+
+
 @pytest.mark.parametrize("delta,T,H,memory,want", [(1, 2048, 16, "all", "fast"), (1, 2048, 16, "little", "least"), (1, 2048, 16, "none", "none"), (1, 70, 2, "little", "fast"),
                                                    (0, 2048, 4, "none", "raises")])
 def test_scan_without_memory_takes_the_form_that_fits(monkeypatch, delta, T, H, memory, want):
